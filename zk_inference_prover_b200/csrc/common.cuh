@@ -35,6 +35,7 @@ struct zkb_ctx {
     // and a pinned landing buffer for the per-item results; both allocated on first use.
     unsigned int* batch_tickets = nullptr;
     uint32_t* h_batch = nullptr;
+    bool res_ready = false;        // gkr_resident.cu: its kernels' attributes are set on this device
     unsigned int batch_round = 0;  // sequence number of the last batched round launched
     cudaEvent_t events[64] = {nullptr};
     // A second stream for host-to-device copies that overlap compute, and the fences between the two.
@@ -54,7 +55,7 @@ namespace zk {
 
 constexpr int RING_SLOTS = 1 << 18;        // pointer-table staging capacity (2 MiB of pointers)
 constexpr size_t SCRATCH_WORDS = 1 << 22;  // 16 MiB of scratch words
-constexpr int SMALL_WORDS = 4096;
+constexpr int SMALL_WORDS = 1 << 15;
 
 int set_error(zkb_ctx* ctx, int code, const char* fmt, ...);
 

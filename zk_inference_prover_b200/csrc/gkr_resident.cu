@@ -1,18 +1,29 @@
-// GKR prove_batch with the Fiat-Shamir transcript resident on the device.
+// GKR prove_batch with the Fiat-Shamir transcript resident on the device, for one or a few instances.
 //
-// The reference's prover (nitroo/crates/stwo/src/prover/lookups/gkr_prover.rs:657-882 with
-// sumcheck.rs:96-176) returns to the host channel after every sum-check round: 276 round trips for one
-// instance of 2^24 fractions, each a launch, a 32-byte copy and a synchronisation. Which kernels run, on
-// which sizes, in which order depends only on the instances' sizes, never on the transcript. So the host
-// enqueues the whole proof without waiting: small single-thread kernels keep the channel, the claims and the
-// round polynomials in device memory (layer_begin, round_step, layer_end below restate the host code of
-// prover.cpp line for line), and the data-parallel kernels read their challenges from that state. One copy
-// brings the proof back.
+// The reference's prover (nitroo/crates/stwo/src/prover/lookups/gkr_prover.rs:657-882 with sumcheck.rs:96-176) returns to the
+// host channel after every sum-check round: 276 round trips for one instance of 2^24 fractions. Which kernels run, on which
+// sizes, in which order depends only on the instances' sizes, never on the transcript, so the host enqueues the whole proof
+// without waiting and one copy brings it back.
+//
+// What bounds a proof is the chain of its rounds: each is three dependent Blake2s compressions (two to mix the round polynomial
+// in, one to draw the challenge, some 0.8 us each, channel.cuh) between a pass over the layer and the next. Everything else is
+// kept off that chain:
+//   * Layers of at most 2^13 entries run in ONE CTA (res_chain_kernel): from the first fold on they live in its shared memory,
+//     and as many whole layers as are small follow one another in the same launch, so a round costs no launch and no trip to L2.
+//   * What a round polynomial depends on beside the two sums is prepared while the data warps work on the layer: the basis
+//     polynomials of all rounds of a layer while its claims are mixed in, the claims, the corrections and the coefficients' share
+//     that does not depend on the sums (one warp) while the others fold. Between the sums and the hash there is one
+//     multiplication.
+//   * Rounds on larger layers are one launch each (res_round_kernel): the fold by the round before's challenge, the sums of the
+//     result, and, by the CTA that finishes last, the transcript step; the next launch is a programmatic dependent of it.
+//   * eq(., point) is never written out for these: the terms are taken in chunks of at most 2^11 with one factor in common,
+//     eq = A[low 11 bits] B[the rest], so a pass reads a table of 32 KB and multiplies by B once per chunk.
+// Measured (one instance): a round in the chain kernel 12.3 -> 4.4 us, 2^10 fractions 906 -> 318 us, 2^24 fractions 7.95 -> 3.84 ms.
+#include <algorithm>
 #include <vector>
 
-#include "blake2s.cuh"
+#include "channel.cuh"
 #include "common.cuh"
-#include "gkr_internal.cuh"
 #include "gkr_resident.hpp"
 #include "host/b200_backend.hpp"
 
@@ -20,727 +31,1247 @@ namespace zk {
 
 constexpr int RES_MAX_INST = 16;
 constexpr int RES_MAX_VARS = 32;
-constexpr int RES_MAX_ROUNDS = RES_MAX_VARS * (RES_MAX_VARS + 1) / 2;
+constexpr int RES_THREADS = 512;          // the chain kernel's CTA
+constexpr int RES_WARPS = RES_THREADS / 32;
+// The chain kernel takes a layer over once its pass reads at most this many entries (log2): 2^13 entries folded to 2^12 of two
+// columns are 128 KB of its shared memory, and the pass itself takes one SM about 5 us, what a launch of its own costs.
+constexpr int CHAIN_LOG = 13;
+constexpr int CHAIN_EQ_LOG = CHAIN_LOG - 2;                        // the most terms (log2) a pass of the chain kernel has
+constexpr size_t CHAIN_EQ_BYTES = (size_t)16 << CHAIN_EQ_LOG;
+constexpr size_t CHAIN_WORK_BYTES = (size_t)32 << (CHAIN_LOG - 1);
+constexpr size_t CHAIN_SMEM = CHAIN_EQ_BYTES + CHAIN_WORK_BYTES;
+constexpr int EQ_LOW = 11;                                         // low table of the launched rounds
+constexpr int EQ_HIGH_MAX = 12;
+constexpr int BASIS_Q = 16;                                        // (L0 - L1)[4], L1[4], L2[4], e0a, e2a, y, 1 - y
+constexpr int POLY_WORDS = 20, MASK_WORDS = 16;
+constexpr int STEP_LEVELS = 5;
 
-struct Poly4 { qm31 c[4]; int n; };
-
-struct ResState {
-    uint32_t digest[8];
-    uint32_t n_draws, error, ood_len, pad;
-    qm31 alpha, lambda, challenge, eq_v;
-    qm31 ood[RES_MAX_VARS + 1];
-    qm31 ood_prefix[RES_MAX_VARS + 2];  // ood_prefix[j] = prod_{i < j} (1 - ood[i])
-    qm31 assignment[RES_MAX_VARS + 1];
-    qm31 claims[RES_MAX_INST][2];
-    uint32_t n_claims[RES_MAX_INST];
-    qm31 sc_claim[RES_MAX_INST];
-    qm31 eq_corr[RES_MAX_INST];
-    uint32_t sums[RES_MAX_INST][8];
-    // proof pieces
-    qm31 output_claims[RES_MAX_INST][2];
-    uint32_t n_output_claims[RES_MAX_INST];
-    Poly4 round_polys[RES_MAX_ROUNDS];
-    qm31 masks[RES_MAX_VARS][RES_MAX_INST][4];  // [layer][oracle][column 0: (v0, v1), column 1: (v0, v1)]
-};
-
-// ---- channel (core/channel/blake2s.rs:58-120 with the M31 reduction of every digest word)
-// The transcript steps are executed by one whole warp. Scalar work is done redundantly by every lane (free
-// under SIMT); the Blake2s compression is spread over four lanes, one column / diagonal G function each
-// (RFC 7693 section 3.2), which shortens its dependency chain fourfold. The message block sits in shared
-// memory so that a lane can pick the two words its G function needs in a round.
-__constant__ uint8_t c_sigma[10][16] = {
-    {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15}, {14, 10, 4, 8, 9, 15, 13, 6, 1, 12, 0, 2, 11, 7, 5, 3},
-    {11, 8, 12, 0, 5, 2, 15, 13, 10, 14, 3, 6, 7, 1, 9, 4}, {7, 9, 3, 1, 13, 12, 11, 14, 2, 6, 5, 10, 4, 0, 15, 8},
-    {9, 0, 5, 7, 2, 4, 10, 15, 14, 1, 11, 12, 6, 8, 3, 13}, {2, 12, 6, 10, 0, 11, 8, 3, 4, 13, 7, 5, 15, 14, 1, 9},
-    {12, 5, 1, 15, 14, 13, 4, 10, 0, 7, 6, 3, 9, 2, 8, 11}, {13, 11, 7, 14, 12, 1, 3, 9, 5, 0, 15, 4, 8, 6, 2, 10},
-    {6, 15, 14, 9, 11, 3, 0, 8, 12, 2, 13, 7, 1, 4, 10, 5}, {10, 2, 8, 4, 7, 6, 1, 5, 15, 11, 9, 14, 3, 12, 13, 0}};
-
-struct Chan { uint32_t digest[8]; uint32_t n_draws; };
-
-// Warp-collective. h: chaining value (same in every lane); m: 16 message words in shared memory.
-__device__ void b2s_compress_warp(uint32_t h[8], const uint32_t* m, uint32_t t, bool last) {
-    const int l = threadIdx.x & 3;
-    const uint32_t iv[8] = {B2S_IV0, B2S_IV1, B2S_IV2, B2S_IV3, B2S_IV4, B2S_IV5, B2S_IV6, B2S_IV7};
-    uint32_t a = h[l], b = h[4 + l], c = iv[l], d = iv[4 + l];
-    if (l == 0) d ^= t;
-    if (l == 2 && last) d = ~d;
-    for (int r = 0; r < 10; r++) {
-        uint32_t x = m[c_sigma[r][2 * l]], y = m[c_sigma[r][2 * l + 1]];
-        B2S_G(a, b, c, d, x, y);
-        b = __shfl_sync(0xffffffffu, b, (l + 1) & 3, 4);
-        c = __shfl_sync(0xffffffffu, c, (l + 2) & 3, 4);
-        d = __shfl_sync(0xffffffffu, d, (l + 3) & 3, 4);
-        x = m[c_sigma[r][8 + 2 * l]];
-        y = m[c_sigma[r][8 + 2 * l + 1]];
-        B2S_G(a, b, c, d, x, y);
-        b = __shfl_sync(0xffffffffu, b, (l + 3) & 3, 4);
-        c = __shfl_sync(0xffffffffu, c, (l + 2) & 3, 4);
-        d = __shfl_sync(0xffffffffu, d, (l + 1) & 3, 4);
-    }
-    const uint32_t lo = a ^ c, hi = b ^ d;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        h[i] ^= __shfl_sync(0xffffffffu, lo, i, 4);
-        h[4 + i] ^= __shfl_sync(0xffffffffu, hi, i, 4);
-    }
+__device__ __forceinline__ qm31 ldq_r(const void* p, size_t i) {
+    uint4 v = reinterpret_cast<const uint4*>(p)[i];
+    return {{v.x, v.y, v.z, v.w}};
 }
-
-__shared__ uint32_t s_block[16];  // the message block of the compression in flight (one transcript warp per CTA)
-
-// Warp-collective: digest <- H(digest || w[0..n)), every word reduced mod p.
-__device__ void chan_mix_words(Chan& ch, const uint32_t* w, int n) {
-    const int lane = threadIdx.x & 31;
-    uint32_t h[8];
-    blake2s_init(h);
-    const int total = 8 + n;
-    uint32_t t = 0;
-    int pos = 0;
-    for (;;) {
-        const int rem = total - pos;
-        const bool last = rem <= 16;
-        __syncwarp();
-        if (lane < 16) {
-            const int i = pos + lane;
-            s_block[lane] = lane < rem ? (i < 8 ? ch.digest[i & 7] : w[i - 8]) : 0u;
-        }
-        __syncwarp();
-        t += last ? 4u * (uint32_t)rem : 64u;
-        b2s_compress_warp(h, s_block, t, last);
-        if (last) break;
-        pos += 16;
-    }
-    for (int k = 0; k < 8; k++) ch.digest[k] = reduce_word_m31(h[k]);
-    ch.n_draws = 0;
+__device__ __forceinline__ void stq_r(void* p, size_t i, qm31 v) {
+    reinterpret_cast<uint4*>(p)[i] = make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]);
 }
-__device__ void chan_mix_felts(Chan& ch, const qm31* f, int n) { chan_mix_words(ch, (const uint32_t*)f, 4 * n); }
-__device__ qm31 chan_draw_felt(Chan& ch) {
-    const int lane = threadIdx.x & 31;
-    uint32_t u[8];
-    for (int attempt = 0; attempt < 64; attempt++) {
-        uint32_t h[8];
-        blake2s_init(h);
-        __syncwarp();
-        if (lane < 16) s_block[lane] = lane < 8 ? ch.digest[lane] : (lane == 8 ? ch.n_draws : 0u);
-        __syncwarp();
-        b2s_compress_warp(h, s_block, 37u, true);
-        ch.n_draws++;
-        bool ok = true;
-        for (int k = 0; k < 8; k++) { u[k] = reduce_word_m31(h[k]); ok = ok && u[k] < 2u * P; }
-        if (ok) break;
-    }
-    qm31 r;
-    for (int k = 0; k < 4; k++) r.c[k] = u[k] >= P ? u[k] - P : u[k];
-    return r;
-}
-__device__ Chan chan_load(const ResState* st) {
-    Chan ch;
-    for (int k = 0; k < 8; k++) ch.digest[k] = st->digest[k];
-    ch.n_draws = st->n_draws;
-    return ch;
-}
-__device__ void chan_store(ResState* st, const Chan& ch) {
-    for (int k = 0; k < 8; k++) st->digest[k] = ch.digest[k];
-    st->n_draws = ch.n_draws;
-}
-
-// ---- univariate polynomials of degree <= 3 (lookups/utils.rs:26-54, 165-170)
-__device__ void p_trim(Poly4& p) { while (p.n > 0 && qm31_is_zero(p.c[p.n - 1])) p.n--; }
-__device__ qm31 p_eval(const Poly4& p, qm31 x) {
-    qm31 acc = qm31_zero();
-    for (int i = p.n; i-- > 0;) acc = qm31_add(qm31_mul(acc, x), p.c[i]);
-    return acc;
-}
-__device__ Poly4 p_add(const Poly4& a, const Poly4& b) {
-    Poly4 r;
-    r.n = a.n > b.n ? a.n : b.n;
-    for (int i = 0; i < 4; i++) r.c[i] = qm31_add(i < a.n ? a.c[i] : qm31_zero(), i < b.n ? b.c[i] : qm31_zero());
-    return r;
-}
-__device__ qm31 eq1(qm31 x, qm31 y) {
-    return qm31_add(qm31_mul(x, y), qm31_mul(qm31_sub(qm31_one(), x), qm31_sub(qm31_one(), y)));
-}
-// gkr_prover.rs:884-923: the degree-3 polynomial through (0, r0), (1, r1), (2, r2), (b, 0) with
-// b = (1 - y) / (1 - 2y), by Lagrange interpolation (lookups/utils.rs:26-54). Field inverses are unique, so
-// the five inversions the formula needs (of prod_i eq(0, y_i), 1 - 2y, and of b, 1 - b, 2 - b, which are
-// (1 - y), -y, (1 - 3y) over (1 - 2y)) are taken with ONE inversion of their product (Montgomery's trick);
-// the fourth Lagrange term has value 0 and vanishes, exactly as its trimmed polynomial does on the host.
-// Warp-collective helpers: lane l computes its own product (or inverse), then every lane reads the results it
-// needs. The independent multiplications of a level run side by side instead of one after the other.
-__device__ __forceinline__ qm31 bcast(qm31 v, int src) {
+__device__ __forceinline__ qm31 shfl_q(qm31 v, int src) {
     qm31 r;
 #pragma unroll
     for (int c = 0; c < 4; c++) r.c[c] = __shfl_sync(0xffffffffu, v.c[c], src);
     return r;
 }
-template <int N>
-__device__ __forceinline__ void par_mul(const qm31 (&x)[N], const qm31 (&y)[N], qm31 (&out)[N]) {
-    const int lane = threadIdx.x & 31;
-    qm31 mx = x[0], my = y[0];
+__device__ __forceinline__ qm31 warp_sum_q(qm31 v) {
+    qm31 r;
 #pragma unroll
-    for (int i = 1; i < N; i++)
-        if (lane == i) { mx = x[i]; my = y[i]; }
-    const qm31 p = qm31_mul(mx, my);
-#pragma unroll
-    for (int i = 0; i < N; i++) out[i] = bcast(p, i);
+    for (int c = 0; c < 4; c++) r.c[c] = warp_sum_m31(v.c[c]);
+    return r;
 }
-__device__ Poly4 correct_sum(qm31 f0, qm31 f2, qm31 claim, const qm31* y, const qm31* one_minus_y_prefix, int n, int k) {
-    const int lane = threadIdx.x & 31;
-    // a = prod_{i < n-k+1} eq(0, y_i) = prod (1 - y_i): kept as prefix products by layer_end
-    const qm31 a = one_minus_y_prefix[n - k + 1];
-    const qm31 one = qm31_one(), yk = y[n - k];
-    const qm31 d = qm31_sub(one, qm31_dbl(yk));                       // 1 - 2y
-    const qm31 omy = qm31_sub(one, yk);                                // 1 - y = eq(0, y)
-    const qm31 m3y = qm31_sub(omy, qm31_dbl(yk));                      // 1 - 3y = -eq(2, y)
-    // level 1: the five inversions (of a, 1-2y, 1-y, y, 1-3y), one per lane
-    qm31 mine = a;
-    if (lane == 1) mine = d;
-    if (lane == 2) mine = omy;
-    if (lane == 3) mine = yk;
-    if (lane == 4) mine = m3y;
-    const qm31 minv = qm31_inv(mine);
-    const qm31 a_inv = bcast(minv, 0), d_inv = bcast(minv, 1), omy_inv = bcast(minv, 2), y_inv = bcast(minv, 3), m3y_inv = bcast(minv, 4);
-    // level 2
-    qm31 l2[6];
-    {
-        const qm31 x[6] = {omy, d, d, d, f0, f2}, z[6] = {d_inv, omy_inv, y_inv, m3y_inv, omy, qm31_neg(m3y)};
-        par_mul<6>(x, z, l2);
-    }
-    const qm31 b = l2[0], inv_b = l2[1], inv_1mb = qm31_neg(l2[2]), inv_2mb = l2[3];   // b, 1/b, 1/(1-b), 1/(2-b)
-    // level 3: r0 = f0 eq(0, y) / a, r2 = f2 eq(2, y) / a
-    qm31 l3[2];
-    {
-        const qm31 x[2] = {l2[4], l2[5]}, z[2] = {a_inv, a_inv};
-        par_mul<2>(x, z, l3);
-    }
-    const qm31 r0 = l3[0], r2 = l3[1], r1 = qm31_sub(claim, r0);
-    // level 4: Lagrange weights p_i = ys[i] * prod_{j != i} 1 / (xs[i] - xs[j]) over xs = {0, 1, 2, b}; ys[3] = 0
-    const uint32_t half = 1u << 30;  // 1 / 2
-    qm31 l4[3];
-    {
-        const qm31 x[3] = {qm31_mul_m31(r0, half), r1, qm31_mul_m31(r2, half)}, z[3] = {inv_b, inv_1mb, inv_2mb};
-        par_mul<3>(x, z, l4);
-    }
-    const qm31 p0 = qm31_neg(l4[0]), p1 = qm31_neg(l4[1]), p2 = l4[2];
-    // level 5: sum_i p_i prod_{j != i} (t - xs[j]), expanded:
-    //   (t-1)(t-2)(t-b) = t^3 - (3+b) t^2 + (2+3b) t - 2b;  t(t-2)(t-b) = t^3 - (2+b) t^2 + 2b t;  t(t-1)(t-b) = t^3 - (1+b) t^2 + b t
-    const qm31 b2 = qm31_dbl(b), b3 = qm31_add(b2, b);
-    qm31 l5[7];
-    {
-        const qm31 x[7] = {qm31_add(qm31_from_m31(3), b), qm31_add(qm31_from_m31(2), b), qm31_add(one, b), qm31_add(qm31_from_m31(2), b3), b2, b, b2};
-        const qm31 z[7] = {p0, p1, p2, p0, p1, p2, p0};
-        par_mul<7>(x, z, l5);
-    }
-    Poly4 c;
-    c.n = 4;
-    c.c[3] = qm31_add(qm31_add(p0, p1), p2);
-    c.c[2] = qm31_neg(qm31_add(qm31_add(l5[0], l5[1]), l5[2]));
-    c.c[1] = qm31_add(qm31_add(l5[3], l5[4]), l5[5]);
-    c.c[0] = qm31_neg(l5[6]);
-    p_trim(c);
-    return c;
-}
+// The steps of a transcript are run once a round by one warp, and what such code costs is as much the fetching of its instructions
+// as the arithmetic: a taken branch to code that has left the instruction cache of the SM's quarter stalls some 70 cycles. (With
+// every product inlined behind its own operand selection, or called, an update of three products in a row took 2,900-3,500 cycles
+// and an empty loop over the oracles 550.) So there is one copy of the hash, one product for everything that is not on a round's
+// path, and the products that are on it run from a table (step_level).
+__device__ __noinline__ qm31 qmul(qm31 a, qm31 b) { return qm31_mul(a, b); }
+__device__ __noinline__ void chan_step_shared(ChanSm& s, int n, int draws, qm31* felts) { chan_step(s, n, draws, reinterpret_cast<uint32_t*>(felts)); }
+__device__ __forceinline__ qm31 one_minus(qm31 v) { return qm31_sub(qm31_one(), v); }
 
-// ---- the three transcript steps
-struct BeginArgs {
-    int n_inst, n_oracles, nv;
-    int activate[RES_MAX_INST], active[RES_MAX_INST], kind[RES_MAX_INST];
-    const uint32_t* out_num[RES_MAX_INST];  // output layer (one entry per column)
-    const uint32_t* out_den[RES_MAX_INST];
-    int oracle_inst[RES_MAX_INST], oracle_nvars[RES_MAX_INST];
+// ---- the transcript's state between launches, and its copy in shared memory while a kernel works on it
+struct alignas(16) ResState {
+    uint32_t digest[8];
+    uint32_t n_draws, pad[3];
+    qm31 alpha, lambda, challenge;       // (alpha and lambda are drawn together)
+    qm31 ood[RES_MAX_VARS + 1];
+    qm31 prefix[RES_MAX_VARS + 2];       // prefix[j] = prod_{i < j} (1 - ood[i])
+    qm31 assign[RES_MAX_VARS + 1];       // the layer's challenges so far
+    qm31 prefix_next[RES_MAX_VARS + 2];  // the same products over them: the next layer's prefix
+    qm31 claims[RES_MAX_INST][2];
+    qm31 out_claims[RES_MAX_INST][2];
+    uint32_t n_claims[RES_MAX_INST], n_out_claims[RES_MAX_INST];
+    qm31 sc[RES_MAX_INST];               // claims of the layer's oracles
+    qm31 corr[RES_MAX_INST];             // eq(assignment, point) over the variables fixed so far
+    qm31 apow[RES_MAX_INST];             // alpha^k
+    uint32_t sums[RES_MAX_INST][8];
+    uint4 steps[STEP_LEVELS][32];        // the products of a transcript step (step_level)
 };
-// Every lane of the warp runs the step and writes the same values; see the channel above.
-__global__ void res_layer_begin_kernel(ResState* st, BeginArgs a) {
-    if (threadIdx.x >= 32 || blockIdx.x != 0) return;
-    Chan ch = chan_load(st);
-    for (int i = 0; i < a.n_inst; i++)
-        if (a.activate[i]) {
-            const uint32_t* d = a.out_den[i];
-            qm31 den0{{d[0], d[1], d[2], d[3]}};
-            int n = 2;
-            if (a.kind[i] == ZKB_GKR_GRAND_PRODUCT) { st->claims[i][0] = den0; n = 1; }
-            else if (a.kind[i] == ZKB_GKR_LOGUP_GENERIC) { const uint32_t* q = a.out_num[i]; st->claims[i][0] = qm31{{q[0], q[1], q[2], q[3]}}; st->claims[i][1] = den0; }
-            else if (a.kind[i] == ZKB_GKR_LOGUP_MULTIPLICITIES) { st->claims[i][0] = qm31_from_m31(a.out_num[i][0]); st->claims[i][1] = den0; }
-            else { st->claims[i][0] = qm31_one(); st->claims[i][1] = den0; }
-            st->n_claims[i] = n;
-            for (int k = 0; k < n; k++) st->output_claims[i][k] = st->claims[i][k];
-            st->n_output_claims[i] = n;
-        }
+static_assert(sizeof(ResState) % 16 == 0, "ResState is copied in 16-byte pieces");
+
+struct alignas(16) TrSm {
+    ResState s;
+    ChanSm ch;
+    qm31 H0[RES_MAX_INST], H2[RES_MAX_INST];  // several oracles: corr e0a, corr e2a (r0 = sum0 H0, r2 = sum2 H2),
+    qm31 G0[RES_MAX_INST], G2[RES_MAX_INST];  // and the same times alpha^k
+    qm31 base[4];                             // the combined polynomial's share that does not depend on the sums
+    qm31 coef[4];                             // the round's polynomial
+    // one oracle: what a coefficient takes of the two sums (H0 (L0 - L1) and H2 L2), the round's H0 and H2, corr e0a and corr e2a of
+    // the round after before its correction, the challenge and one minus it, the prefix product, intermediate values, zero
+    qm31 A[8], H[2], next_h[2], r, omr, pcur, tmp[5], zero, sink[32];
+    uint32_t n_vars[RES_MAX_INST];            // variables of the layer's oracles
+};
+
+// Any set of threads; a barrier must follow (and precede tr_store's readers).
+__device__ __forceinline__ void tr_load(TrSm& t, const ResState* st, int thread, int n_threads) {
+    for (int i = thread; i < (int)(sizeof(ResState) / 16); i += n_threads) reinterpret_cast<uint4*>(&t.s)[i] = __ldcg(reinterpret_cast<const uint4*>(st) + i);
+    chan_make_schedule(t.ch, thread, n_threads);
+}
+__device__ __forceinline__ void tr_open_channel(TrSm& t, int lane) {  // one warp, after tr_load's barrier
+    t.ch.msg[lane] = lane < 8 ? t.s.digest[lane] : 0u;
+    if (lane == 0) t.ch.n_draws = t.s.n_draws;
     __syncwarp();
-    for (int i = 0; i < a.n_inst; i++)
-        if (a.active[i]) chan_mix_felts(ch, st->claims[i], (int)st->n_claims[i]);
-    st->eq_v = st->ood_len == 0 ? qm31_one() : eq1(qm31_zero(), st->ood[0]);
-    const qm31 alpha = chan_draw_felt(ch), lambda = chan_draw_felt(ch);
-    st->alpha = alpha;
-    st->lambda = lambda;
-    chan_store(st, ch);
-    for (int k = 0; k < a.n_oracles; k++) {
-        int i = a.oracle_inst[k];
-        qm31 acc = qm31_zero();
-        for (int j = (int)st->n_claims[i]; j-- > 0;) acc = qm31_add(qm31_mul(acc, lambda), st->claims[i][j]);
-        st->sc_claim[k] = qm31_mul_m31(acc, 1u << (a.nv - a.oracle_nvars[k]));
-        st->eq_corr[k] = qm31_one();
+}
+__device__ __forceinline__ void tr_close_channel(TrSm& t, int lane) {
+    __syncwarp();
+    if (lane < 8) t.s.digest[lane] = t.ch.msg[lane];
+    if (lane == 0) t.s.n_draws = t.ch.n_draws;
+    __syncwarp();
+}
+__device__ __forceinline__ void tr_store(const TrSm& t, ResState* st, int thread, int n_threads) {
+    for (int i = thread; i < (int)(sizeof(ResState) / 16); i += n_threads) reinterpret_cast<uint4*>(st)[i] = reinterpret_cast<const uint4*>(&t.s)[i];
+}
+
+// Basis of the rounds of a layer (correct_sum_as_poly_in_first_variable, gkr_prover.rs:884-923). With y = ood[n - k] the
+// variable a round with k variables left fixes, an oracle's round polynomial goes through (0, r0), (1, r1), (2, r2), (b, 0) with
+// b = (1 - y) / (1 - 2y), i.e. it is r0 L0 + r1 L1 + r2 L2; r0 = sum0 corr e0a, r2 = sum2 corr e2a with e0a = eq(0, y) / a and
+// e2a = eq(2, y) / a, a = prod_{i <= n - k} eq(0, y_i). The inversions (of a, 1 - 2y, 1 - y, y, 1 - 3y; those of b, 1 - b and 2 - b
+// follow) are one per thread.
+__device__ __forceinline__ void basis_inverses(const TrSm& t, qm31* inv, int nv, int thread, int n_threads) {
+    for (int i = thread; i < 5 * nv; i += n_threads) {
+        const int j = i / 5, w = i % 5;  // round j: nv - j variables left; ood has nv entries
+        const qm31 y = t.s.ood[j], omy = one_minus(y);
+        qm31 v = t.s.prefix[j + 1];
+        if (w == 1) v = one_minus(qm31_dbl(y));
+        if (w == 2) v = omy;
+        if (w == 3) v = y;
+        if (w == 4) v = qm31_sub(omy, qm31_dbl(y));
+        inv[i] = qm31_inv(v);
+    }
+}
+__device__ __forceinline__ void basis_rounds(const TrSm& t, const qm31* inv, qm31* basis, int nv, int thread, int n_threads) {
+    for (int i = thread; i < BASIS_Q * nv; i += n_threads) {
+        const int j = i / BASIS_Q, w = i % BASIS_Q;
+        const qm31* iv = inv + 5 * j;
+        const qm31 y = t.s.ood[j], omy = one_minus(y), d = one_minus(qm31_dbl(y));
+        qm31 v = w == 14 ? y : omy;
+        if (w < 12) {
+            const int c = w & 3;
+            const qm31 b = qmul(omy, iv[1]), b2 = qm31_dbl(b);
+            auto small = [](uint32_t m) { return qm31_from_m31(m); };
+            // L1 = -t(t-2)(t-b) / (1-b), L2 = t(t-1)(t-b) / 2(2-b), L0 = -(t-1)(t-2)(t-b) / 2b, low coefficients first;
+            // 1/b = d / (1-y), -1/(1-b) = d / y, 1/(2-b) = d / (1-3y)
+            const qm31 p1 = c == 0 ? qm31_zero() : c == 1 ? b2 : c == 2 ? qm31_neg(qm31_add(small(2), b)) : qm31_one();
+            if (w >= 8) {
+                const qm31 p2 = c == 0 ? qm31_zero() : c == 1 ? b : c == 2 ? qm31_neg(qm31_add(qm31_one(), b)) : qm31_one();
+                v = qm31_mul_m31(qmul(p2, qmul(d, iv[4])), 1u << 30);
+            } else {
+                v = qmul(p1, qmul(d, iv[3]));
+                if (w < 4) {
+                    const qm31 p0 = c == 0 ? b2 : c == 1 ? qm31_neg(qm31_add(small(2), qm31_add(b2, b))) : c == 2 ? qm31_add(small(3), b) : qm31_neg(qm31_one());
+                    v = qm31_sub(qm31_mul_m31(qmul(p0, qmul(d, iv[2])), 1u << 30), v);
+                }
+            }
+        } else if (w == 12) {
+            v = qmul(omy, iv[0]);
+        } else if (w == 13) {
+            v = qmul(qm31_neg(qm31_sub(omy, qm31_dbl(y))), iv[0]);  // eq(2, y) = 3y - 1
+        }
+        basis[i] = v;
     }
 }
 
-struct RoundArgs {
-    int n_oracles, n_rem, round, poly_slot;
-    int nvars[RES_MAX_INST];
-};
-// Warp-collective.
-__device__ void round_step(ResState* st, const RoundArgs& a) {
-    Chan ch = chan_load(st);
-    const qm31 alpha = st->alpha;
-    Poly4 rp[RES_MAX_INST];
-    const uint32_t half = m31_inv(2);
-    for (int k = 0; k < a.n_oracles; k++) {
-        if (a.n_rem == a.nvars[k]) {
-            const uint32_t* s = st->sums[k];
-            qm31 s0 = qm31_mul(qm31{{s[0], s[1], s[2], s[3]}}, st->eq_corr[k]);
-            qm31 s2 = qm31_mul(qm31{{s[4], s[5], s[6], s[7]}}, st->eq_corr[k]);
-            rp[k] = correct_sum(s0, s2, st->sc_claim[k], st->ood, st->ood_prefix, (int)st->ood_len, a.nvars[k]);
-        } else {
-            rp[k].n = 1;
-            rp[k].c[0] = qm31_mul_m31(st->sc_claim[k], half);
-            for (int j = 1; j < 4; j++) rp[k].c[j] = qm31_zero();
-            p_trim(rp[k]);
-        }
-        qm31 e = rp[k].n ? rp[k].c[0] : qm31_zero();  // r(0) + r(1) = c0 + (c0 + c1 + c2 + c3)
-        for (int j = 0; j < rp[k].n; j++) e = qm31_add(e, rp[k].c[j]);
-        if (!qm31_eq(e, st->sc_claim[k])) st->error = 1u;  // the round polynomial does not match the claim
-    }
-    Poly4 combined;
-    combined.n = 0;
-    for (int j = 0; j < 4; j++) combined.c[j] = qm31_zero();
-    for (int k = a.n_oracles; k-- > 0;) {
-        for (int j = 0; j < combined.n; j++) combined.c[j] = qm31_mul(combined.c[j], alpha);
-        combined = p_add(combined, rp[k]);
-    }
-    chan_mix_felts(ch, combined.c, combined.n);
-    qm31 challenge = chan_draw_felt(ch);
-    chan_store(st, ch);
-    for (int k = 0; k < a.n_oracles; k++) st->sc_claim[k] = p_eval(rp[k], challenge);
-    for (int k = 0; k < a.n_oracles; k++)
-        if (a.n_rem == a.nvars[k] && a.nvars[k] != 0) {
-            const qm31 z0 = st->ood[st->ood_len - a.nvars[k]], old = st->eq_corr[k];
-            const qm31 upd = qm31_mul(old, eq1(challenge, z0));
-            __syncwarp();  // every lane has read the old value before any lane replaces it
-            st->eq_corr[k] = upd;
-        }
-    st->round_polys[a.poly_slot] = combined;
-    st->assignment[a.round] = challenge;
-    st->challenge = challenge;
+// The steps below are chains of a few dependent secure products on one warp. Each level of a chain is ONE product whose operands
+// the lanes choose for themselves (a branch per product would run them one after the other).
+
+// ---- one oracle. Its round polynomial is the batch's, so its next claim is that polynomial at the challenge, and everything a
+// round needs beside its sums follows in three levels of products: the coefficients are sum0 A[c] + sum2 A[4 + c] + base[c].
+//
+// A level: every lane takes x (z + z') + a of four values in TrSm (and the basis behind it) and stores it; the byte offsets are in
+// the level's table, so a level is the same thirty instructions and one product for all lanes whatever they compute, and the
+// levels are one loop. z may move with the round (its offset in the basis).
+__device__ __forceinline__ qm31 step_level(TrSm& t, const uint4 e, uint32_t basis_off) {
+    char* const base = reinterpret_cast<char*>(&t);
+    const qm31 x = ldq_r(base + e.x, 0);
+    const qm31 z = qm31_add(ldq_r(base + (e.y & 0xffffu) + e.w * basis_off, 0), ldq_r(base + (e.y >> 16), 0));
+    const qm31 m = qm31_add(qm31_mul(x, z), ldq_r(base + (e.z & 0xffffu), 0));
+    stq_r(base + (e.z >> 16), 0, m);
+    __syncwarp();
+    return m;
 }
-__global__ void res_round_kernel(ResState* st, RoundArgs a) {
-    if (threadIdx.x >= 32 || blockIdx.x != 0) return;
-    round_step(st, a);
+// basis_at: byte offset of the basis of round 0 from TrSm.
+__device__ __forceinline__ void step_tables(TrSm& t, uint32_t basis_at, int thread, int n_threads) {
+    for (int i = thread; i < STEP_LEVELS * 32; i += n_threads) {
+        const int level = i >> 5, l = i & 31;
+        auto off = [&](const void* p) { return (uint32_t)(reinterpret_cast<const char*>(p) - reinterpret_cast<const char*>(&t)); };
+        const uint32_t zero = off(&t.zero);
+        uint32_t x = zero, z = zero, z2 = zero, a = zero, out = off(&t.sink[l]), moving = 0;
+        auto B = [&](int ahead, int q) { moving = 1; return basis_at + 16u * (uint32_t)(BASIS_Q * ahead + q); };
+        if (level == 0) {         // prepare a layer's first round: claim L1, corr e0a, corr e2a, and those of the round after
+            if (l < 4) { x = off(&t.s.sc[0]); z = B(0, 4 + l); out = off(&t.base[l]); }
+            else if (l < 6) { x = off(&t.s.corr[0]); z = B(0, 8 + l); out = off(&t.H[l - 4]); }
+            else if (l < 8) { x = off(&t.s.corr[0]); z = B(1, 6 + l); out = off(&t.next_h[l - 6]); }
+        } else if (level == 1) {
+            if (l < 8) { x = off(&t.H[l >> 2]); z = B(0, l < 4 ? l : 4 + l); out = off(&t.A[l]); }
+        } else if (level == 2) {  // after a challenge: (c3 r + c2), (c1 r + c0), r^2, the two parts of eq(r, y), the prefix product
+            if (l < 2) { x = off(&t.coef[3 - 2 * l]); z = off(&t.r); a = off(&t.coef[2 - 2 * l]); out = off(&t.tmp[l]); }
+            else if (l == 2) { x = off(&t.r); z = off(&t.r); out = off(&t.tmp[2]); }
+            else if (l == 3) { x = off(&t.r); z = B(0, 14); out = off(&t.tmp[3]); }
+            else if (l == 4) { x = off(&t.omr); z = B(0, 15); out = off(&t.tmp[4]); }
+            else if (l == 5) { x = off(&t.pcur); z = off(&t.omr); out = off(&t.pcur); }
+        } else if (level == 3) {  // the claim; the next round's H, the correction
+            if (l == 0) { x = off(&t.tmp[0]); z = off(&t.tmp[2]); a = off(&t.tmp[1]); out = off(&t.s.sc[0]); }
+            else if (l < 4) { x = l < 3 ? off(&t.next_h[l - 1]) : off(&t.s.corr[0]); z = off(&t.tmp[3]); z2 = off(&t.tmp[4]); out = l < 3 ? off(&t.H[l - 1]) : x; }
+        } else {                  // prepare the next round, and the H of the round after it
+            if (l < 8) { x = off(&t.H[l >> 2]); z = B(1, l < 4 ? l : 4 + l); out = off(&t.A[l]); }
+            else if (l < 12) { x = off(&t.s.sc[0]); z = B(1, 4 + l - 8); out = off(&t.base[l - 8]); }
+            else if (l < 14) { x = off(&t.s.corr[0]); z = B(2, l); out = off(&t.next_h[l - 12]); }
+        }
+        t.s.steps[level][l] = make_uint4(x, z | z2 << 16, a | out << 16, moving);
+    }
 }
 
-// The last rounds of a layer's sum-check in ONE launch: once every live oracle has at most 2^14 entries, a
-// single CTA runs round after round (sums over the layer, the transcript step on thread 0, fix_first_variable),
-// so a round costs its own latency and no launch. The first fold goes from the oracle's layer into work buffers
-// (the layer may be the caller's input, which is never modified), later folds are in place there.
-constexpr int TAIL_MAX_LOG = 14;
-constexpr int TAIL_THREADS = 512;
-struct TailArgs {
-    int n_oracles, nv, round_start, first_poly_slot;
-    int kind[RES_MAX_INST], nvars[RES_MAX_INST];
-    const uint32_t* num[RES_MAX_INST];
-    const uint32_t* den[RES_MAX_INST];
-    uint32_t* num_w[RES_MAX_INST];  // n/2 QM31 each (unused for kinds without numerators)
-    uint32_t* den_w[RES_MAX_INST];
-    const uint32_t* eq_evals;
-};
-__device__ __forceinline__ qm31 ldq_r(const uint32_t* p, size_t i) {
-    uint4 v = reinterpret_cast<const uint4*>(p)[i];
-    return {{v.x, v.y, v.z, v.w}};
+// ---- several oracles, taken eight at a time: lane = 8 q + k, q saying which of up to four products of oracle k the lane has
+__device__ __noinline__ void many_prepare(TrSm& t, const qm31* B, int K, uint32_t n_rem) {
+    const int lane = threadIdx.x & 31, q = lane >> 3;
+    qm31 ac_sum = qm31_zero(), cw_sum = qm31_zero();
+    for (int kb = 0; kb < K; kb += 8) {
+        const int k = kb + (lane & 7);
+        const bool live = k < K, act = live && n_rem <= t.n_vars[k];
+        const qm31 a = live ? t.s.apow[k] : qm31_zero(), sc = live ? t.s.sc[k] : qm31_zero(), corr = live ? t.s.corr[k] : qm31_zero();
+        // a * claim (half of it when the oracle waits: it contributes the constant claim / 2), corr * e0a, corr * e2a
+        const qm31 m = qmul(q == 0 ? a : corr, q == 0 ? (act ? sc : qm31_mul_m31(sc, 1u << 30)) : q == 1 ? B[12] : B[13]);
+        const qm31 g = qmul(a, m);
+        if (act && q == 1) { t.H0[k] = m; t.G0[k] = g; }
+        if (act && q == 2) { t.H2[k] = m; t.G2[k] = g; }
+        ac_sum = qm31_add(ac_sum, warp_sum_q(q == 0 && act ? m : qm31_zero()));
+        cw_sum = qm31_add(cw_sum, warp_sum_q(q == 0 && live && !act ? m : qm31_zero()));
+    }
+    qm31 v = qmul(ac_sum, B[4 + (lane & 3)]);
+    if (lane == 0) v = qm31_add(v, cw_sum);
+    if (lane < 4) t.base[lane] = v;
+    __syncwarp();
 }
-__device__ __forceinline__ void stq_r(uint32_t* p, size_t i, qm31 v) {
-    reinterpret_cast<uint4*>(p)[i] = make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]);
+// The length of the combination when its leading coefficient vanishes: it keeps the length of its longest term (every term trimmed,
+// their sum not), so the terms' own lengths decide.
+__device__ __noinline__ int many_length(const TrSm& t, const qm31* B, int K, uint32_t n_rem) {
+    const int lane = threadIdx.x & 31;
+    int len = 0;
+    if (lane < K) {
+        if (n_rem <= t.n_vars[lane]) {
+            const qm31 r0 = qmul(ldq_r(t.s.sums[lane], 0), t.H0[lane]), r2 = qmul(ldq_r(t.s.sums[lane], 1), t.H2[lane]);
+            for (int c = 0; c < 4; c++)  // r0 L0 + (claim - r0) L1 + r2 L2
+                if (!qm31_is_zero(qm31_add(qm31_add(qmul(r0, B[c]), qmul(t.s.sc[lane], B[4 + c])), qmul(r2, B[8 + c])))) len = c + 1;
+        } else if (!qm31_is_zero(t.s.sc[lane])) {
+            len = 1;
+        }
+    }
+    return __reduce_max_sync(0xffffffffu, len);
 }
-// The summand of sum_as_poly_in_first_variable at t = 0 and t = 2 for term i (cpu/lookups/gkr.rs:39-211).
-__device__ void sum_term(int kind, const uint32_t* num, const uint32_t* den, size_t nt, size_t i, qm31 lambda, qm31& t0, qm31& t2) {
-    qm31 d00 = ldq_r(den, 2 * i), d01 = ldq_r(den, 2 * i + 1), d10 = ldq_r(den, 2 * (nt + i)), d11 = ldq_r(den, 2 * (nt + i) + 1);
-    qm31 d20 = qm31_sub(qm31_dbl(d10), d00), d21 = qm31_sub(qm31_dbl(d11), d01);
-    if (kind == ZKB_GKR_GRAND_PRODUCT) {
-        t0 = qm31_mul(d00, d01);
-        t2 = qm31_mul(d20, d21);
+// Coefficient (lane & 3) of the batch's polynomial: r1 = claim - r0, so the sums enter as S0 (L0 - L1) + S2 L2.
+__device__ __noinline__ qm31 many_coefficients(const TrSm& t, const qm31* B, int K, uint32_t n_rem) {
+    const int lane = threadIdx.x & 31, k = lane >> 1;
+    const bool act = k < K && n_rem <= t.n_vars[k];
+    const qm31 part = qmul(act ? ldq_r(t.s.sums[k], lane & 1) : qm31_zero(), act ? ((lane & 1) ? t.G2[k] : t.G0[k]) : qm31_zero());
+    const qm31 S0 = warp_sum_q((lane & 1) ? qm31_zero() : part), S2 = warp_sum_q((lane & 1) ? part : qm31_zero());
+    return qmul((lane & 4) ? S2 : S0, B[(lane & 3) + ((lane & 4) ? 8 : 0)]);
+}
+// Claims and corrections at the round's challenge (sumcheck.rs:150-171), and the next layer's prefix product.
+__device__ __noinline__ void many_update(TrSm& t, const qm31* B, int K, uint32_t n_rem, int round) {
+    const int lane = threadIdx.x & 31, q = lane >> 3;
+    const qm31 r = t.s.challenge, y = B[14];
+    // the basis at r, (L3 r + L2) r^2 + (L1 r + L0) (lanes 0-2 and 4-6), r^2 (8), eq(r, y) (9, 10), the prefix product (11)
+    const int w = lane & 3;
+    auto L = [&](int c) { return w == 0 ? qm31_add(B[c], B[4 + c]) : B[4 * w + c]; };
+    qm31 x = r, z = r;
+    if (lane < 8 && w < 3) x = L(lane < 4 ? 3 : 1);
+    if (lane == 9) x = y;
+    if (lane == 10) { x = one_minus(y); z = one_minus(r); }
+    if (lane == 11) { x = t.s.prefix_next[round]; z = one_minus(r); }
+    qm31 m = qmul(x, z);
+    if (lane == 11) t.s.prefix_next[round + 1] = m;
+    const qm31 step = qm31_add(shfl_q(m, 9), shfl_q(m, 10)), r2v = shfl_q(m, 8);
+    if (lane < 8 && w < 3) m = qm31_add(m, L(lane < 4 ? 2 : 0));
+    const qm31 at = qm31_add(qmul(m, r2v), shfl_q(m, (lane + 4) & 31));
+    const qm31 l0 = shfl_q(at, 0), l1 = shfl_q(at, 1), l2 = shfl_q(at, 2);
+    for (int kb = 0; kb < K; kb += 8) {
+        const int k = kb + (lane & 7);
+        const bool live = k < K, act = live && n_rem <= t.n_vars[k];
+        const qm31 sc = live ? t.s.sc[k] : qm31_zero();
+        // round values: r0 (q = 0), r2 (q = 2), r1 = claim - r0 (q = 1)
+        const qm31 rv = qmul(act && !(q & 1) ? ldq_r(t.s.sums[k], q >> 1) : qm31_zero(), act ? (q == 0 ? t.H0[k] : t.H2[k]) : qm31_zero());
+        const qm31 r0 = shfl_q(rv, lane & 7);
+        const qm31 v = qmul(q == 0 ? r0 : q == 1 ? qm31_sub(sc, r0) : q == 2 ? rv : live ? t.s.corr[k] : qm31_zero(), q == 0 ? l0 : q == 1 ? l1 : q == 2 ? l2 : step);
+        const qm31 sum = qm31_add(qm31_add(v, shfl_q(v, (lane + 8) & 31)), shfl_q(v, (lane + 16) & 31));
+        if (act && q == 0) t.s.sc[k] = sum;
+        if (act && q == 3) t.s.corr[k] = v;
+        if (live && !act && q == 0) t.s.sc[k] = qm31_mul_m31(sc, 1u << 30);
+    }
+    __syncwarp();
+}
+
+// ---- the three parts of a round's transcript, each by one warp
+// B: the round's basis, basis_off its byte offset from the first round's.
+__device__ __forceinline__ void tr_prepare(TrSm& t, const qm31* B, uint32_t basis_off, int K, uint32_t n_rem) {
+    if (K > 1) { many_prepare(t, B, K, n_rem); return; }
+    const int lane = threadIdx.x & 31;
+    uint4 e = t.s.steps[0][lane];
+#pragma unroll 1
+    for (int level = 0; level < 2; level++) {
+        const uint4 next = t.s.steps[1][lane];
+        step_level(t, e, basis_off);
+        e = next;
+    }
+}
+// The round polynomial of the batch from the oracles' sums (sumcheck.rs:139-149), mixed into the channel, and the round's
+// challenge. poly: POLY_WORDS words of the proof. parts: the one oracle's sums as two addends per node, or NULL.
+__device__ __forceinline__ void tr_round(TrSm& t, const qm31* B, int K, uint32_t n_rem, int round, uint32_t* poly, const qm31* parts) {
+    const int lane = threadIdx.x & 31, node = (lane >> 2) & 1;
+    qm31 p;
+    if (K == 1) p = qm31_mul(parts ? qm31_add(parts[node], parts[2 + node]) : ldq_r(t.s.sums[0], node), t.A[lane & 7]);
+    else p = many_coefficients(t, B, K, n_rem);
+    const qm31 c = qm31_add(qm31_add(p, shfl_q(p, (lane + 4) & 31)), t.base[lane & 3]);
+    if (lane < 4) {
+        stq_r(t.ch.msg + 8, lane, c);
+        stq_r(poly, lane, c);
+        t.coef[lane] = c;
+    }
+    const unsigned nonzero = __ballot_sync(0xffffffffu, lane < 4 && !qm31_is_zero(c));
+    int len = 32 - __clz(nonzero);
+    if (K > 1 && len < 4) len = many_length(t, B, K, n_rem);
+    if (lane == 0) poly[16] = (uint32_t)len;
+    chan_step_shared(t.ch, 4 * len, 1, &t.r);
+    if (lane == 0) { const qm31 r = t.r; t.s.challenge = r; t.omr = one_minus(r); t.s.assign[round] = r; }
+    __syncwarp();
+}
+// Reads up to two bases after B (the rounds' whose H it prepares), whatever is there after the last one.
+__device__ __forceinline__ void tr_update(TrSm& t, const qm31* B, uint32_t basis_off, int K, uint32_t n_rem, int round, bool prepare_next) {
+    if (K > 1) {
+        many_update(t, B, K, n_rem, round);
+        if (prepare_next && n_rem > 1) many_prepare(t, B + BASIS_Q, K, n_rem - 1);
         return;
     }
-    qm31 n0, n2;
-    if (kind == ZKB_GKR_LOGUP_SINGLES) {
-        n0 = qm31_add(d00, d01);
-        n2 = qm31_add(d20, d21);
-    } else if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) {
-        uint32_t a0 = num[2 * i], a1 = num[2 * i + 1], b0 = num[2 * (nt + i)], b1 = num[2 * (nt + i) + 1];
-        uint32_t n20 = m31_sub(m31_dbl(b0), a0), n21 = m31_sub(m31_dbl(b1), a1);
-        n0 = qm31_add(qm31_mul_m31(d01, a0), qm31_mul_m31(d00, a1));
-        n2 = qm31_add(qm31_mul_m31(d21, n20), qm31_mul_m31(d20, n21));
-    } else {
-        qm31 n00 = ldq_r(num, 2 * i), n01 = ldq_r(num, 2 * i + 1), n10 = ldq_r(num, 2 * (nt + i)), n11 = ldq_r(num, 2 * (nt + i) + 1);
-        qm31 n20 = qm31_sub(qm31_dbl(n10), n00), n21 = qm31_sub(qm31_dbl(n11), n01);
-        n0 = qm31_add(qm31_mul(d01, n00), qm31_mul(d00, n01));
-        n2 = qm31_add(qm31_mul(d21, n20), qm31_mul(d20, n21));
+    const int lane = threadIdx.x & 31;
+    uint4 e = t.s.steps[2][lane];
+#pragma unroll 1
+    for (int level = 2; level < (prepare_next ? 5 : 4); level++) {
+        const uint4 next = t.s.steps[level < 4 ? level + 1 : 4][lane];
+        const qm31 m = step_level(t, e, basis_off);
+        if (level == 2 && lane == 5) t.s.prefix_next[round + 1] = m;
+        e = next;
     }
-    t0 = qm31_add(n0, qm31_mul(lambda, qm31_mul(d00, d01)));
-    t2 = qm31_add(n2, qm31_mul(lambda, qm31_mul(d20, d21)));
+    __syncwarp();
 }
-__global__ void __launch_bounds__(TAIL_THREADS) res_tail_kernel(ResState* st, TailArgs a) {
-    __shared__ uint32_t red[TAIL_THREADS / 32][8];
-    __shared__ qm31 sh_challenge;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // every thread tracks the oracles' current layers identically
-    int kind[RES_MAX_INST], nvars[RES_MAX_INST];
-    const uint32_t* num[RES_MAX_INST];
-    const uint32_t* den[RES_MAX_INST];
-    bool folded[RES_MAX_INST];
-    for (int k = 0; k < a.n_oracles; k++) { kind[k] = a.kind[k]; nvars[k] = a.nvars[k]; num[k] = a.num[k]; den[k] = a.den[k]; folded[k] = false; }
-    const qm31 lambda = st->lambda;
-    for (int round = a.round_start; round < a.nv; round++) {
-        const int n_rem = a.nv - round;
-        for (int k = 0; k < a.n_oracles; k++) {
-            if (n_rem != nvars[k]) continue;
-            const size_t nt = ((size_t)2 << nvars[k]) / 4;  // the layer has 2^(nvars + 1) entries
-            qm31 s0 = qm31_zero(), s2 = qm31_zero();
-            for (size_t i = tid; i < nt; i += TAIL_THREADS) {
-                qm31 t0, t2;
-                sum_term(kind[k], num[k], den[k], nt, i, lambda, t0, t2);
-                qm31 e = ldq_r(a.eq_evals, i);
-                s0 = qm31_add(s0, qm31_mul(e, t0));
-                s2 = qm31_add(s2, qm31_mul(e, t2));
-            }
+
+// ---- one term of the round sums: t0 and t2 of sum_as_poly_in_first_variable (cpu/lookups/gkr.rs:39-211) from the denominators
+// (and numerators) at (0, i, {0, 1}) and (1, i, {0, 1}); n0 d1 + n1 d0 + lambda d0 d1 taken as (n0 + lambda d0) d1 + n1 d0
+template <int KIND>
+__device__ __forceinline__ qm31 term_at(qm31 d0, qm31 d1, qm31 n0, qm31 n1, qm31 lambda) {
+    if (KIND == ZKB_GKR_GRAND_PRODUCT) return qm31_mul(d0, d1);
+    if (KIND == ZKB_GKR_LOGUP_SINGLES) return qm31_add(qm31_add(d0, d1), qm31_mul(lambda, qm31_mul(d0, d1)));
+    return qm31_add(qm31_mul(qm31_add(n0, qm31_mul(lambda, d0)), d1), qm31_mul(n1, d0));
+}
+__device__ __forceinline__ qm31 at_two(qm31 v0, qm31 v1) { return qm31_sub(qm31_dbl(v1), v0); }
+__device__ __forceinline__ qm31 fold_q(qm31 r, qm31 a, qm31 b) { return qm31_add(qm31_mul(r, qm31_sub(b, a)), a); }
+__device__ __forceinline__ qm31 fold_m(qm31 r, uint32_t a, uint32_t b) {
+    qm31 v = qm31_mul_m31(r, m31_sub(b, a));
+    v.c[0] = m31_add(v.c[0], a);
+    return v;
+}
+
+// Term i of a layer's pass. FOLD: the layer (n entries) is first fixed at r, entries o and o + n/2 of every column giving entry o
+// of the outputs; a thread reads and writes only the entries of its own terms, so the outputs may be the inputs' first half.
+// nt: terms of the pass.
+template <int KIND, bool FOLD>
+__device__ __forceinline__ void pass_term(const void* num, const void* den, void* num_out, void* den_out, size_t nt, size_t i, qm31 r, qm31 lambda,
+                                          qm31& t0, qm31& t2) {
+    const size_t o[4] = {2 * i, 2 * i + 1, 2 * (nt + i), 2 * (nt + i) + 1};
+    const size_t half = 4 * nt;  // entries after the fold
+    qm31 d[4], u[4];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    s0.c[c] = m31_add(s0.c[c], __shfl_down_sync(0xffffffffu, s0.c[c], off));
-                    s2.c[c] = m31_add(s2.c[c], __shfl_down_sync(0xffffffffu, s2.c[c], off));
-                }
-            if (lane == 0)
-                for (int c = 0; c < 4; c++) { red[warp][c] = s0.c[c]; red[warp][4 + c] = s2.c[c]; }
-            __syncthreads();
-            if (tid < 8) {
-                uint32_t acc = 0;
-                for (int w = 0; w < TAIL_THREADS / 32; w++) acc = m31_add(acc, red[w][tid]);
-                st->sums[k][tid] = acc;
+    for (int q = 0; q < 4; q++) {
+        u[q] = qm31_zero();
+        if (FOLD) {
+            d[q] = fold_q(r, ldq_r(den, o[q]), ldq_r(den, o[q] + half));
+            stq_r(den_out, o[q], d[q]);
+            if (KIND == ZKB_GKR_LOGUP_GENERIC) u[q] = fold_q(r, ldq_r(num, o[q]), ldq_r(num, o[q] + half));
+            if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) {
+                const uint32_t* m = static_cast<const uint32_t*>(num);
+                u[q] = fold_m(r, m[o[q]], m[o[q] + half]);
             }
-            __syncthreads();
+            if (KIND == ZKB_GKR_LOGUP_GENERIC || KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) stq_r(num_out, o[q], u[q]);
+        } else {
+            d[q] = ldq_r(den, o[q]);
+            if (KIND == ZKB_GKR_LOGUP_GENERIC) u[q] = ldq_r(num, o[q]);
+            if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) u[q] = qm31_from_m31(static_cast<const uint32_t*>(num)[o[q]]);
         }
-        if (warp == 0) {
-            RoundArgs ra;
-            ra.n_oracles = a.n_oracles;
-            ra.n_rem = n_rem;
-            ra.round = round;
-            ra.poly_slot = a.first_poly_slot + (round - a.round_start);
-            for (int k = 0; k < a.n_oracles; k++) ra.nvars[k] = nvars[k];
-            round_step(st, ra);
-            __syncwarp();
-            if (lane == 0) sh_challenge = st->challenge;
-        }
+    }
+    t0 = term_at<KIND>(d[0], d[1], u[0], u[1], lambda);
+    t2 = term_at<KIND>(at_two(d[0], d[2]), at_two(d[1], d[3]), at_two(u[0], u[2]), at_two(u[1], u[3]), lambda);
+}
+
+// ---- towers: up to ten levels of a layer's halvings per launch (gen_layers, gkr_prover.rs:847-852). A level's entries come from
+// adjacent pairs, so a CTA that takes 2^10 consecutive entries builds its share of every level above them; the levels stay in
+// shared memory for the next one and every one is written. One launch per level read each level back from memory and cost a
+// launch for the many short ones (a 2^24 tower: 24 launches, 290 us; now three, 218 us).
+constexpr int TOWER_LEVELS = 10, TOWER_THREADS = 256;
+struct TowerArgs {
+    const uint32_t *num, *den;  // 2^log entries
+    uint32_t *num_out[TOWER_LEVELS], *den_out[TOWER_LEVELS];
+    int levels, cta_log;        // a CTA takes 2^cta_log entries, levels <= cta_log
+};
+template <int KIND>
+__device__ __forceinline__ void tower_pair(qm31 n0, qm31 n1, qm31 d0, qm31 d1, qm31& n, qm31& d) {
+    d = qm31_mul(d0, d1);
+    if (KIND == ZKB_GKR_LOGUP_SINGLES) n = qm31_add(d0, d1);
+    else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) n = qm31_add(qm31_mul_m31(d1, n0.c[0]), qm31_mul_m31(d0, n1.c[0]));
+    else if (KIND == ZKB_GKR_LOGUP_GENERIC) n = qm31_add(qm31_mul(d1, n0), qm31_mul(d0, n1));
+    else n = qm31_zero();
+}
+template <int KIND>
+__global__ void __launch_bounds__(TOWER_THREADS) tower_kernel(TowerArgs a) {
+    constexpr bool HAS_NUM_OUT = KIND != ZKB_GKR_GRAND_PRODUCT;
+    constexpr int KIND2 = HAS_NUM_OUT ? ZKB_GKR_LOGUP_GENERIC : ZKB_GKR_GRAND_PRODUCT;
+    __shared__ uint4 sd[512], sn[HAS_NUM_OUT ? 512 : 1];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t half = 1u << (a.cta_log - 1);
+    const size_t first = (size_t)blockIdx.x * half;
+    for (uint32_t i = threadIdx.x; i < half; i += TOWER_THREADS) {
+        const size_t o = first + i;
+        qm31 n0 = qm31_zero(), n1 = qm31_zero(), n, d;
+        if (KIND == ZKB_GKR_LOGUP_GENERIC) { n0 = ldq_r(a.num, 2 * o); n1 = ldq_r(a.num, 2 * o + 1); }
+        if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) { n0.c[0] = a.num[2 * o]; n1.c[0] = a.num[2 * o + 1]; }
+        tower_pair<KIND>(n0, n1, ldq_r(a.den, 2 * o), ldq_r(a.den, 2 * o + 1), n, d);
+        stq_r(a.den_out[0], o, d);
+        stq_r(sd, i, d);
+        if (HAS_NUM_OUT) { stq_r(a.num_out[0], o, n); stq_r(sn, i, n); }
+    }
+    for (int l = 1; l < a.levels; l++) {
+        const uint32_t m = half >> l;
         __syncthreads();
-        const qm31 r = sh_challenge;
-        for (int k = 0; k < a.n_oracles; k++) {
-            if (n_rem != nvars[k] || nvars[k] == 0) continue;
-            const size_t half = (size_t)1 << nvars[k];  // entries after the fold
-            const bool has_num = kind[k] == ZKB_GKR_LOGUP_GENERIC || kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES;
-            for (size_t i = tid; i < half; i += TAIL_THREADS) {
-                qm31 x = ldq_r(den[k], i), y = ldq_r(den[k], i + half);
-                stq_r(a.den_w[k], i, qm31_add(qm31_mul(r, qm31_sub(y, x)), x));
-                if (kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES) {
-                    uint32_t p = num[k][i], q = num[k][i + half];
-                    qm31 v = qm31_mul_m31(r, m31_sub(q, p));
-                    v.c[0] = m31_add(v.c[0], p);
-                    stq_r(a.num_w[k], i, v);
-                } else if (has_num) {
-                    qm31 p = ldq_r(num[k], i), q = ldq_r(num[k], i + half);
-                    stq_r(a.num_w[k], i, qm31_add(qm31_mul(r, qm31_sub(q, p)), p));
-                }
-            }
-            den[k] = a.den_w[k];
-            if (has_num) { num[k] = a.num_w[k]; kind[k] = ZKB_GKR_LOGUP_GENERIC; }
-            folded[k] = true;
-            nvars[k]--;
+        qm31 n, d;
+        const uint32_t i = threadIdx.x;  // at most 256 from the second level on
+        if (i < m) tower_pair<KIND2>(HAS_NUM_OUT ? ldq_r(sn, 2 * i) : qm31_zero(), HAS_NUM_OUT ? ldq_r(sn, 2 * i + 1) : qm31_zero(), ldq_r(sd, 2 * i), ldq_r(sd, 2 * i + 1), n, d);
+        __syncthreads();
+        if (i < m) {
+            const size_t o = (size_t)blockIdx.x * m + i;
+            stq_r(a.den_out[l], o, d);
+            stq_r(sd, i, d);
+            if (HAS_NUM_OUT) { stq_r(a.num_out[l], o, n); stq_r(sn, i, n); }
         }
-        __syncthreads();  // the folded layers are complete (and visible) before the next round reads them
     }
 }
 
-struct EndArgs {
-    int n_oracles, nv, layer;
-    int kind[RES_MAX_INST], inst[RES_MAX_INST];
-    const uint32_t* num[RES_MAX_INST];  // the constant oracle's columns: two entries each
-    const uint32_t* den[RES_MAX_INST];
+// ---- rounds on large layers, one launch each
+struct RoundArgs {
+    const uint32_t *num, *den;
+    uint32_t *num_out, *den_out;
+    const uint32_t *eq_low, *eq_high;  // eq = low[i mod 2^EQ_LOW] high[i >> EQ_LOW]
+    size_t nt;                          // terms of the pass
+    uint32_t chunk_log;                 // terms a CTA takes at a time: 2^chunk_log <= 2^EQ_LOW
+    uint32_t* partials;
+    unsigned int* ticket;
+    ResState* st;
+    const qm31* basis;                  // of the round whose sums these are; the next round's follows
+    uint32_t* poly;
+    int oracle;                         // whose sums these are
+    int n_oracles, n_rem, round, transcript;  // transcript: this launch completes the round's sums and runs its step
+    uint32_t n_vars[RES_MAX_INST];
 };
-__global__ void res_layer_end_kernel(ResState* st, EndArgs a) {
-    if (threadIdx.x >= 32 || blockIdx.x != 0) return;
-    Chan ch = chan_load(st);
-    int ncols[RES_MAX_INST];
-    for (int k = 0; k < a.n_oracles; k++) {  // try_into_mask, gkr_prover.rs:572-597
-        qm31* m = st->masks[a.layer][k];
-        const uint32_t* d = a.den[k];
-        qm31 d0{{d[0], d[1], d[2], d[3]}}, d1{{d[4], d[5], d[6], d[7]}};
-        if (a.kind[k] == ZKB_GKR_GRAND_PRODUCT) { m[0] = d0; m[1] = d1; ncols[k] = 1; }
-        else if (a.kind[k] == ZKB_GKR_LOGUP_GENERIC) {
-            const uint32_t* q = a.num[k];
-            m[0] = qm31{{q[0], q[1], q[2], q[3]}}; m[1] = qm31{{q[4], q[5], q[6], q[7]}}; m[2] = d0; m[3] = d1; ncols[k] = 2;
-        } else { m[0] = qm31_one(); m[1] = qm31_one(); m[2] = d0; m[3] = d1; ncols[k] = 2; }
+constexpr int ROUND_THREADS = 256;
+constexpr int ROUND_MAX_CTAS = 148 * 4;
+template <int KIND, bool FOLD>
+__global__ void __launch_bounds__(ROUND_THREADS, 2) res_round_kernel(const __grid_constant__ RoundArgs a) {
+    __shared__ struct alignas(16) { TrSm tr; qm31 basis[3 * BASIS_Q]; } sm;
+    TrSm& tr = sm.tr;
+    __shared__ uint32_t red[ROUND_THREADS / 32][8];
+    __shared__ bool is_last;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const qm31 lambda = ldq_r(&a.st->lambda, 0);
+    const qm31 r = FOLD ? ldq_r(&a.st->challenge, 0) : qm31_zero();
+    qm31 s0 = qm31_zero(), s2 = qm31_zero();
+    const size_t n_chunks = a.nt >> a.chunk_log;
+    for (size_t ck = blockIdx.x; ck < n_chunks; ck += gridDim.x) {
+        const size_t begin = ck << a.chunk_log;
+        qm31 c0 = qm31_zero(), c2 = qm31_zero();
+        for (size_t i = begin + tid; i < begin + ((size_t)1 << a.chunk_log); i += ROUND_THREADS) {
+            qm31 t0, t2;
+            pass_term<KIND, FOLD>(a.num, a.den, a.num_out, a.den_out, a.nt, i, r, lambda, t0, t2);
+            const qm31 e = ldq_r(a.eq_low, i & ((1u << EQ_LOW) - 1));
+            c0 = qm31_add(c0, qm31_mul(e, t0));
+            c2 = qm31_add(c2, qm31_mul(e, t2));
+        }
+        const qm31 eh = ldq_r(a.eq_high, begin >> EQ_LOW);
+        s0 = qm31_add(s0, qm31_mul(eh, c0));
+        s2 = qm31_add(s2, qm31_mul(eh, c2));
+    }
+    s0 = warp_sum_q(s0);
+    s2 = warp_sum_q(s2);
+    if (lane == 0) { stq_r(red[warp], 0, s0); stq_r(red[warp], 1, s2); }
+    __syncthreads();
+    if (tid < 8) {
+        uint32_t acc = 0;
+#pragma unroll
+        for (int w = 0; w < ROUND_THREADS / 32; w++) acc = m31_add(acc, red[w][tid]);
+        a.partials[8 * blockIdx.x + tid] = acc;
+        __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) is_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    // every other CTA has ended or is about to: the next launch may be scheduled and run up to its wait
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __threadfence();
+    if (tid == 0) *a.ticket = 0u;
+    // the partial sums: word tid & 7 of every 32nd CTA per thread, then over the threads (eight threads that walk the CTAs one
+    // after the other take 20 us for 592 of them)
+    {
+        uint32_t acc = 0;
+        for (unsigned b = tid >> 3; b < gridDim.x; b += ROUND_THREADS / 8) acc = m31_add(acc, __ldcg(&a.partials[8 * b + (tid & 7)]));
+        acc = m31_add(acc, __shfl_xor_sync(0xffffffffu, acc, 8));
+        acc = m31_add(acc, __shfl_xor_sync(0xffffffffu, acc, 16));
+        __syncthreads();
+        if (lane < 8) red[warp][lane] = acc;
+    }
+    if (a.transcript) {
+        tr_load(tr, a.st, tid, ROUND_THREADS);
+        if (tid == 32) tr.zero = qm31_zero();
+        if (tid < RES_MAX_INST) tr.n_vars[tid] = a.n_vars[tid];
+        if (tid >= 64 && tid < 64 + 2 * BASIS_Q) sm.basis[tid - 64] = ldq_r(a.basis, tid - 64);  // this round's and the next one's
+    }
+    __syncthreads();
+    uint32_t mine = 0;
+    if (tid < 8) {
+#pragma unroll
+        for (int w = 0; w < ROUND_THREADS / 32; w++) mine = m31_add(mine, red[w][tid]);
+        if (a.transcript) tr.s.sums[a.oracle][tid] = mine;
+        else a.st->sums[a.oracle][tid] = mine;
+    }
+    if (!a.transcript) return;
+    __syncthreads();
+    if (warp == 0) {
+        tr_open_channel(tr, lane);
+        if (lane == 0) tr.pcur = tr.s.prefix_next[a.round];
+        tr_prepare(tr, sm.basis, 0u, a.n_oracles, (uint32_t)a.n_rem);
+        tr_round(tr, sm.basis, a.n_oracles, (uint32_t)a.n_rem, a.round, a.poly, nullptr);
+        tr_close_channel(tr, lane);
+        tr_update(tr, sm.basis, 0u, a.n_oracles, (uint32_t)a.n_rem, a.round, false);
+    }
+    __syncthreads();
+    tr_store(tr, a.st, tid, ROUND_THREADS);
+}
+
+// ---- whole layers in one CTA
+enum : uint32_t { CHAIN_BEGIN = 1, CHAIN_ROUNDS = 2, CHAIN_END = 4 };
+struct alignas(16) ChainLayer {
+    uint32_t flags;
+    int nv, round_start;               // rounds of the layer; the first the chain kernel runs
+    int n_inst, n_oracles, last_active;
+    int table_bits;                    // CHAIN_BEGIN without CHAIN_ROUNDS: bits of the high table (the low one has EQ_LOW)
+    uint32_t *eq_low, *eq_high;        // where the two tables go
+    qm31* basis;                       // the layer's basis in device memory (written with the tables, read when the rounds resume)
+    uint32_t* polys;                   // POLY_WORDS per round of this layer
+    uint32_t* masks;                   // MASK_WORDS per oracle
+    // instances: the kind of the output layer of those that start here, -1 otherwise; its entry; whether the instance is active
+    int start_kind[RES_MAX_INST], active[RES_MAX_INST];
+    const uint32_t *out_num[RES_MAX_INST], *out_den[RES_MAX_INST];
+    // oracles: instance, variables, the arrays the first pass of the launch reads and their kind, where folded layers go (a byte
+    // offset into the CTA's work area, or, with work_global, an address)
+    int inst[RES_MAX_INST], kind[RES_MAX_INST];
+    uint32_t n_vars[RES_MAX_INST];
+    const uint32_t *num[RES_MAX_INST], *den[RES_MAX_INST];
+    uint64_t num_work[RES_MAX_INST], den_work[RES_MAX_INST];
+    uint64_t work_global;
+};
+static_assert(sizeof(ChainLayer) % 16 == 0, "ChainLayer is copied in 16-byte pieces");
+
+// While the first warp hashes at the start of a layer, the warps after it form the basis of its rounds and the rest eq(., point).
+constexpr int BASIS_THREADS = 160, EQ_THREADS = RES_THREADS - 32 - BASIS_THREADS;
+__device__ __forceinline__ void basis_bar() { asm volatile("bar.sync 1, %0;" ::"n"(BASIS_THREADS) : "memory"); }
+__device__ __forceinline__ void eq_bar() { asm volatile("bar.sync 2, %0;" ::"n"(EQ_THREADS) : "memory"); }
+
+// table[x] = v prod_{k < bits} (bit k of x ? y_k : 1 - y_k), y_k = ood[ny - first_bit - k] (gen_eq_evals: index bit k pairs with the
+// k-th variable from the end). By the EQ_THREADS last threads.
+__device__ __forceinline__ void eq_build(void* table, const qm31* ood, int ny, int first_bit, int bits, qm31 v) {
+    const int th = threadIdx.x - (RES_THREADS - EQ_THREADS);
+    if (th == 0) stq_r(table, 0, v);
+    eq_bar();
+    for (int k = 0; k < bits; k++) {
+        const uint32_t len = 1u << k;
+        const qm31 y = ood[ny - first_bit - k];
+        for (uint32_t j = th; j < len; j += EQ_THREADS) {
+            const qm31 e = ldq_r(table, j), hi = qmul(e, y);
+            stq_r(table, j, qm31_sub(e, hi));
+            stq_r(table, j + len, hi);
+        }
+        eq_bar();
+    }
+}
+
+// The claims of the instances that start here, every active instance's claims into the channel, alpha and lambda, the oracles'
+// claims (gkr_prover.rs:669-735). Warp-collective.
+__device__ __forceinline__ void tr_begin(TrSm& t, const ChainLayer& L) {
+    const int lane = threadIdx.x & 31;
+    if (lane < L.n_inst && L.start_kind[lane] >= 0) {
+        const int kind = L.start_kind[lane];
+        const qm31 den0 = ldq_r(L.out_den[lane], 0);
+        int n = 2;
+        qm31 first = qm31_one();
+        if (kind == ZKB_GKR_GRAND_PRODUCT) { first = den0; n = 1; }
+        else if (kind == ZKB_GKR_LOGUP_GENERIC) first = ldq_r(L.out_num[lane], 0);
+        else if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) first = qm31_from_m31(L.out_num[lane][0]);
+        t.s.claims[lane][0] = first;
+        t.s.claims[lane][1] = den0;
+        t.s.n_claims[lane] = n;
+        t.s.out_claims[lane][0] = first;
+        t.s.out_claims[lane][1] = den0;
+        t.s.n_out_claims[lane] = n;
     }
     __syncwarp();
-    for (int k = 0; k < a.n_oracles; k++) chan_mix_felts(ch, st->masks[a.layer][k], 2 * ncols[k]);
-    qm31 challenge = chan_draw_felt(ch);
-    chan_store(st, ch);
-    for (int j = 0; j < a.nv; j++) st->ood[j] = st->assignment[j];
-    st->ood[a.nv] = challenge;
-    st->ood_len = (uint32_t)a.nv + 1u;
-    st->ood_prefix[0] = qm31_one();
-    for (int j = 0; j <= a.nv; j++) st->ood_prefix[j + 1] = qm31_mul(st->ood_prefix[j], qm31_sub(qm31_one(), st->ood[j]));
-    for (int k = 0; k < a.n_oracles; k++) {
-        const qm31* m = st->masks[a.layer][k];
-        int i = a.inst[k];
-        for (int c = 0; c < ncols[k]; c++)
-            st->claims[i][c] = qm31_add(qm31_mul(challenge, qm31_sub(m[2 * c + 1], m[2 * c])), m[2 * c]);
-        st->n_claims[i] = (uint32_t)ncols[k];
+    for (int i = 0; i < L.n_inst; i++)
+        if (L.active[i]) {
+            const int n = 4 * (int)t.s.n_claims[i];
+            if (lane < n) t.ch.msg[8 + lane] = reinterpret_cast<const uint32_t*>(t.s.claims[i])[lane];
+            chan_step_shared(t.ch, n, i == L.last_active ? 2 : 0, &t.s.alpha);
+        }
+    const qm31 alpha = t.s.alpha, lambda = t.s.lambda;
+    if (lane == 0) { t.s.prefix_next[0] = qm31_one(); t.pcur = qm31_one(); }
+    const int K = L.n_oracles, k = lane & 15;
+    qm31 pw = qm31_one();
+    if (K > 1) {  // alpha^k by the bits of k
+        qm31 sq = alpha;
+        for (int b = 0; (1 << b) < K; b++) {
+            const qm31 m = qmul(pw, sq);
+            if ((k >> b) & 1) pw = m;
+            sq = qmul(sq, sq);
+        }
     }
+    const int i = k < K ? L.inst[k] : 0;
+    const bool two = t.s.n_claims[i] == 2;
+    const qm31 h = qmul(lambda, t.s.claims[i][1]);
+    if (lane < K) {
+        t.s.apow[k] = pw;
+        t.s.corr[k] = qm31_one();
+        t.s.sc[k] = qm31_mul_m31(two ? qm31_add(h, t.s.claims[i][0]) : t.s.claims[i][0], 1u << (L.nv - (int)L.n_vars[k]));
+    }
+    __syncwarp();
+}
+
+// The masks into the channel, the next layer's point and claims (gkr_prover.rs:745-800). Warp-collective. Oracle k's two entries
+// per column are at num(k) / den(k), of kind kind(k): what the folds have made of the layer.
+template <class Kind, class Num, class Den>
+__device__ __forceinline__ void tr_end(TrSm& t, const ChainLayer& L, Kind kind, Num num, Den den) {
+    const int lane = threadIdx.x & 31, K = L.n_oracles, nv = L.nv;
+    for (int k = 0; k < K; k++) {
+        uint32_t* out = L.masks + (size_t)MASK_WORDS * k;
+        const bool one_col = kind(k) == ZKB_GKR_GRAND_PRODUCT;
+        if (lane < 16) {
+            uint32_t v = 0u;
+            const uint32_t* d = static_cast<const uint32_t*>(den(k));
+            if (one_col) v = lane < 8 ? d[lane] : 0u;
+            else if (lane >= 8) v = d[lane - 8];
+            else if (kind(k) == ZKB_GKR_LOGUP_GENERIC) v = static_cast<const uint32_t*>(num(k))[lane];
+            else v = (lane & 3) == 0 ? 1u : 0u;
+            t.ch.msg[8 + lane] = v;
+            out[lane] = v;
+        }
+        chan_step_shared(t.ch, one_col ? 8 : 16, k == K - 1 ? 1 : 0, &t.s.challenge);
+    }
+    const qm31 c = t.s.challenge;
+    if (lane <= nv) {
+        if (lane < nv) t.s.ood[lane] = t.s.assign[lane];
+        t.s.prefix[lane] = t.s.prefix_next[lane];
+    }
+    const qm31 last = qmul(t.s.prefix_next[nv], one_minus(c));
+    if (lane == 0) { t.s.ood[nv] = c; t.s.prefix[nv + 1] = last; }
+    // claims: two columns of up to sixteen oracles
+    const int k = lane & 15, col = lane >> 4;
+    const bool live = k < K && !(col == 1 && kind(k) == ZKB_GKR_GRAND_PRODUCT);
+    qm31 a = qm31_zero(), b = qm31_zero();
+    if (live) {
+        const bool one_col = kind(k) == ZKB_GKR_GRAND_PRODUCT;
+        if (col == 1 || one_col) { a = ldq_r(den(k), 0); b = ldq_r(den(k), 1); }
+        else if (kind(k) == ZKB_GKR_LOGUP_GENERIC) { a = ldq_r(num(k), 0); b = ldq_r(num(k), 1); }
+        else a = b = qm31_one();
+    }
+    const qm31 v = qm31_add(qmul(c, qm31_sub(b, a)), a);
+    if (live) {
+        t.s.claims[L.inst[k]][col] = v;
+        t.s.n_claims[L.inst[k]] = kind(k) == ZKB_GKR_GRAND_PRODUCT ? 1u : 2u;
+    }
+    __syncwarp();
+}
+
+// Sum over a pass's terms by every thread of the CTA, each thread's share in s0 / s2.
+template <int KIND, bool FOLD>
+__device__ __forceinline__ void chain_pass(const void* num, const void* den, void* num_out, void* den_out, uint32_t nt, qm31 r, qm31 lambda, const void* eq,
+                                           qm31& s0, qm31& s2) {
+    for (uint32_t i = (threadIdx.x - 64u) & (RES_THREADS - 1); i < nt; i += RES_THREADS) {
+        qm31 t0, t2;
+        pass_term<KIND, FOLD>(num, den, num_out, den_out, nt, i, r, lambda, t0, t2);
+        const qm31 e = ldq_r(eq, i);
+        s0 = qm31_add(s0, qm31_mul(e, t0));
+        s2 = qm31_add(s2, qm31_mul(e, t2));
+    }
+}
+
+// A pass of few terms is the latency of one thread's 16 multiplications: it is taken in two steps instead, one multiplication per
+// thread for the fold (an entry each), then a unit of work per warp: 32 terms at one node (t = 0 or t = 2), and of a term one of
+// the two products it is the sum of, (n0 + lambda d0) d1 or n1 d0, times eq.
+constexpr uint32_t CHAIN_SMALL = 256;
+__device__ __forceinline__ qm31 small_unit(int kind, const void* num, const void* den, uint32_t nt, uint32_t i, int node, int part, qm31 lambda, const void* eq) {
+    qm31 s = qm31_zero();
+    if (i < nt) {
+        auto at = [&](const void* p, uint32_t b) {
+            const qm31 v0 = ldq_r(p, 2 * i + b);
+            return node ? at_two(v0, ldq_r(p, 2 * (nt + i) + b)) : v0;
+        };
+        qm31 n = kind == ZKB_GKR_GRAND_PRODUCT ? qm31_zero() : qm31_one();  // numerator `part`; LogUpSingles has ones
+        if (kind == ZKB_GKR_LOGUP_GENERIC) {
+            n = at(num, part);
+        } else if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) {
+            const uint32_t* m = static_cast<const uint32_t*>(num);
+            const uint32_t v0 = m[2 * i + part];
+            n = qm31_from_m31(node ? m31_sub(m31_dbl(m[2 * (nt + i) + part]), v0) : v0);
+        }
+        const qm31 d0 = at(den, 0);
+        if (part == 0) s = qm31_mul(qm31_add(n, kind == ZKB_GKR_GRAND_PRODUCT ? d0 : qm31_mul(lambda, d0)), at(den, 1));
+        else s = qm31_mul(n, d0);
+        s = qm31_mul(ldq_r(eq, i), s);
+    }
+    return warp_sum_q(s);
+}
+// The same once numerators have been changed for m = n + (lambda / 2) d: products m0 d1 and m1 d0 (a grand product: d0 d1).
+__device__ __forceinline__ qm31 small_unit_m(bool product, const void* m, const void* den, uint32_t nt, uint32_t i, int node, int part, const void* eq) {
+    qm31 s = qm31_zero();
+    if (i < nt && !(product && part)) {
+        auto at = [&](const void* p, uint32_t b) {
+            const qm31 v0 = ldq_r(p, 2 * i + b);
+            return node ? at_two(v0, ldq_r(p, 2 * (nt + i) + b)) : v0;
+        };
+        s = qm31_mul(ldq_r(eq, i), qm31_mul(at(product ? den : m, part), at(den, 1 - part)));
+    }
+    if (nt >= 16) return warp_sum_q(s);
+    for (uint32_t off = nt >> 1; off; off >>= 1) s = qm31_add(s, shfl_q(s, (threadIdx.x & 31) + off));  // lane 0 has the sum
+    return s;
+}
+
+struct ResInit { uint32_t digest[8], n_draws; int use; };  // use: the proof's first launch starts from this channel, not from *st
+__global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st, const ChainLayer* __restrict__ layers, int n_layers, ResInit init) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ struct alignas(16) { TrSm tr; qm31 basis[(RES_MAX_VARS + 2) * BASIS_Q]; } sm;
+    TrSm& tr = sm.tr;
+    qm31* const basis = sm.basis;
+    __shared__ ChainLayer layer_buf[2];  // the layer at hand and the next one
+    __shared__ qm31 inv[RES_MAX_VARS * 5];
+    __shared__ qm31 red[RES_MAX_INST][32];  // per oracle: a warp's two sums (warps x 2), or the units of a small pass
+    void* const eq = dyn;
+    unsigned char* const work = dyn + CHAIN_EQ_BYTES;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (init.use) {
+        for (int i = tid; i < (int)(sizeof(ResState) / 4); i += RES_THREADS) {
+            uint32_t v = i == 8 ? init.n_draws : 0u;
+#pragma unroll
+            for (int k = 0; k < 8; k++) v = i == k ? init.digest[k] : v;
+            reinterpret_cast<uint32_t*>(&tr.s)[i] = v;
+        }
+        chan_make_schedule(tr.ch, tid, RES_THREADS);
+        __syncthreads();
+        // the round kernels keep their bases behind TrSm too: the table travels with the state
+        step_tables(tr, (uint32_t)((const char*)basis - (const char*)&tr), tid, RES_THREADS);
+    } else {
+        tr_load(tr, st, tid, RES_THREADS);
+    }
+    if (tid == 32) tr.zero = qm31_zero();
+    __syncthreads();
+    if (warp == 0) tr_open_channel(tr, lane);
+    for (int d = 0; d < n_layers; d++) {
+        ChainLayer& L = layer_buf[d & 1];
+        if (d == 0)
+            for (int i = tid; i < (int)(sizeof(ChainLayer) / 16); i += RES_THREADS) reinterpret_cast<uint4*>(&L)[i] = __ldg(reinterpret_cast<const uint4*>(layers) + i);
+        __syncthreads();
+        const int K = L.n_oracles, nv = L.nv, ny = nv - 1;
+        if (tid == 0 && L.round_start) tr.pcur = tr.s.prefix_next[L.round_start];
+        if (tid < K) tr.n_vars[tid] = L.n_vars[tid];
+        if (warp == 0) {
+            if (L.flags & CHAIN_BEGIN) tr_begin(tr, L);
+        } else if (tid < 32 + BASIS_THREADS) {
+            const int th = tid - 32;
+            if (L.flags & CHAIN_BEGIN) {
+                basis_inverses(tr, inv, nv, th, BASIS_THREADS);
+                basis_bar();
+                basis_rounds(tr, inv, basis, nv, th, BASIS_THREADS);
+                basis_bar();
+                if (!(L.flags & CHAIN_ROUNDS))  // the rounds on launches of their own come next and read it from memory
+                    for (int i = th; i < BASIS_Q * nv; i += BASIS_THREADS) L.basis[i] = basis[i];
+            } else if (L.flags & CHAIN_ROUNDS) {
+                for (int i = th; i < BASIS_Q * nv; i += BASIS_THREADS) basis[i] = L.basis[i];
+            }
+        } else if ((L.flags & CHAIN_ROUNDS) && nv > 0) {
+            // the passes have at most 2^bits terms: index bits above are zero, a factor 1 - y each
+            const int bits = nv - L.round_start - 1;
+            if (bits >= 0) eq_build(eq, tr.s.ood, ny, 0, bits, tr.s.prefix[ny - bits + 1]);
+        } else if ((L.flags & CHAIN_BEGIN) && !(L.flags & CHAIN_ROUNDS)) {
+            const int th = tid - (RES_THREADS - EQ_THREADS);
+            eq_build(eq, tr.s.ood, ny, 0, EQ_LOW, qm31_one());
+            for (uint32_t i = th; i < (1u << EQ_LOW); i += EQ_THREADS) stq_r(L.eq_low, i, ldq_r(eq, i));
+            eq_build(work, tr.s.ood, ny, EQ_LOW, L.table_bits, tr.s.prefix[1]);
+            for (uint32_t i = th; i < (1u << L.table_bits); i += EQ_THREADS) stq_r(L.eq_high, i, ldq_r(work, i));
+        }
+        __syncthreads();
+        if (warp == RES_WARPS - 1 && d + 1 < n_layers)  // under the rounds
+            for (int i = lane; i < (int)(sizeof(ChainLayer) / 16); i += 32) reinterpret_cast<uint4*>(&layer_buf[(d + 1) & 1])[i] = __ldg(reinterpret_cast<const uint4*>(layers + d + 1) + i);
+        // oracle k's arrays: the caller's until the first fold of this launch, then the work area's
+        auto den_work = [&](int k) { return L.work_global ? reinterpret_cast<void*>(L.den_work[k]) : static_cast<void*>(work + L.den_work[k]); };
+        auto num_work = [&](int k) { return L.work_global ? reinterpret_cast<void*>(L.num_work[k]) : static_cast<void*>(work + L.num_work[k]); };
+        if (L.flags & CHAIN_ROUNDS) {
+            // one oracle: where its layer is, and whether small folds (below) have begun
+            struct { const void *num, *den; int kind; bool folds; } one = {L.num[0], L.den[0], L.kind[0], false};
+            const bool one_product = L.kind[0] == ZKB_GKR_GRAND_PRODUCT;
+            const qm31 half_lambda = qm31_mul_m31(tr.s.lambda, 1u << 30);
+            for (int round = L.round_start; round <= nv; round++) {
+                // Pass of this round: the oracles that were active before are fixed at the last challenge; those and the ones that
+                // enter now give their sums (none after the last round). The second warp brings claims and corrections up to date
+                // and prepares this round meanwhile.
+                const uint32_t n_rem = (uint32_t)(nv - round);
+                const qm31 r = tr.s.challenge, lambda = tr.s.lambda;
+                const bool sums = round < nv;
+                const uint32_t nt = sums ? 1u << (n_rem - 1) : 0u;
+                const bool small = nt <= CHAIN_SMALL;
+                if (warp == 1) {
+                    if (round > L.round_start) tr_update(tr, basis + BASIS_Q * (round - 1), 16u * BASIS_Q * (round - 1), K, n_rem + 1, round - 1, true);
+                    else if (sums) tr_prepare(tr, basis + BASIS_Q * round, 16u * BASIS_Q * round, K, n_rem);
+                }
+                if (K == 1 && small) {
+                    if (warp < 2) {
+                    } else if (one.folds && n_rem) {  // later folds: an entry of either column per thread
+                        const uint32_t e_out = 2u << n_rem, log_e = n_rem + 1;
+                        for (uint32_t i = tid - 64u; i < (one_product ? 1u : 2u) * e_out; i += RES_THREADS - 64u) {
+                            unsigned char* const p = work + (i >> log_e ? L.num_work[0] : 0u);
+                            const uint32_t e = i & (e_out - 1);
+                            stq_r(p, e, fold_q(r, ldq_r(p, e), ldq_r(p, e + e_out)));
+                        }
+                    } else if (tr.n_vars[0] > n_rem) {
+                        // the first small fold, which changes n for m = n + (lambda / 2) d (a term is then m0 d1 + m1 d0), and the
+                        // last one, which leaves the mask: n again
+                        const uint32_t e_out = 2u << n_rem;
+                        for (uint32_t e = tid - 64u; e < e_out; e += RES_THREADS - 64u) {
+                            const qm31 d = fold_q(r, ldq_r(one.den, e), ldq_r(one.den, e + e_out));
+                            qm31 n = qm31_one();
+                            if (one.kind == ZKB_GKR_LOGUP_MULTIPLICITIES && !one.folds) {
+                                const uint32_t* m = static_cast<const uint32_t*>(one.num);
+                                n = fold_m(r, m[e], m[e + e_out]);
+                            } else if (one.kind == ZKB_GKR_LOGUP_GENERIC || one.folds) {
+                                if (!one_product) n = fold_q(r, ldq_r(one.num, e), ldq_r(one.num, e + e_out));
+                            }
+                            stq_r(work, e, d);
+                            if (!one_product) {
+                                const qm31 hd = qm31_mul(half_lambda, d);
+                                stq_r(work + L.num_work[0], e, !n_rem ? (one.folds ? qm31_sub(n, hd) : n) : qm31_add(n, hd));
+                            }
+                        }
+                    }
+                    if (tr.n_vars[0] > n_rem) { one.den = work; one.num = work + L.num_work[0]; one.folds = true; }
+                }
+                for (int k = small && (warp < 2 || K == 1) ? K : 0; k < K; k++) {
+                    const uint32_t vars = tr.n_vars[k];
+                    const bool fold = vars > n_rem, fresh = round == L.round_start || vars == n_rem + 1;  // fresh: nothing folded here yet
+                    if (!fold && (vars < n_rem || small)) continue;
+                    const int kind = fresh || L.kind[k] != ZKB_GKR_LOGUP_MULTIPLICITIES ? L.kind[k] : (int)ZKB_GKR_LOGUP_GENERIC;
+                    const void* den = fresh || !fold ? static_cast<const void*>(L.den[k]) : den_work(k);
+                    const void* num = fresh || !fold ? static_cast<const void*>(L.num[k]) : num_work(k);
+                    void *den_w = den_work(k), *num_w = num_work(k);
+                    if (small) {
+                        const uint32_t e_out = 2u << n_rem;  // entries of the fixed layer
+                        const bool has_num = kind == ZKB_GKR_LOGUP_GENERIC || kind == ZKB_GKR_LOGUP_MULTIPLICITIES;
+                        for (uint32_t i = tid - 64u; i < (has_num ? 2 : 1) * e_out; i += RES_THREADS - 64u) {  // not by the first two warps
+                            const uint32_t e = i & (e_out - 1);
+                            if (i >= e_out && kind == ZKB_GKR_LOGUP_MULTIPLICITIES) {
+                                const uint32_t* m = static_cast<const uint32_t*>(num);
+                                stq_r(num_w, e, fold_m(r, m[e], m[e + e_out]));
+                            } else {
+                                const void* p = i < e_out ? den : num;
+                                stq_r(i < e_out ? den_w : num_w, e, fold_q(r, ldq_r(p, e), ldq_r(p, e + e_out)));
+                            }
+                        }
+                        continue;
+                    }
+                    qm31 s0 = qm31_zero(), s2 = qm31_zero();
+                    switch (kind + (fold ? 4 : 0)) {
+                        case 0: chain_pass<0, false>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 1: chain_pass<1, false>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 2: chain_pass<2, false>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 3: chain_pass<3, false>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 4: chain_pass<0, true>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 5: chain_pass<1, true>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        case 6: chain_pass<2, true>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                        default: chain_pass<3, true>(num, den, num_w, den_w, nt, r, lambda, eq, s0, s2); break;
+                    }
+                    s0 = warp_sum_q(s0);
+                    s2 = warp_sum_q(s2);
+                    if (lane == 0) { red[k][2 * warp] = s0; red[k][2 * warp + 1] = s2; }
+                    if (K == 1 && fold) {
+                        one.den = den_w;
+                        one.num = num_w;
+                        if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) one.kind = ZKB_GKR_LOGUP_GENERIC;
+                    }
+                }
+                __syncthreads();
+                if (!sums) break;
+                uint32_t units = 2 * RES_WARPS;
+                if (small) {
+                    // by the warps after the first two, whose instruction caches hold the transcript
+                    units = 4 * ((nt + 31) / 32);
+                    if (K == 1) {
+                        for (uint32_t w = (warp + RES_WARPS - 2) & (RES_WARPS - 1); w < units; w += RES_WARPS) {
+                            const uint32_t i = 32 * (w >> 2) + lane;
+                            const qm31 v = one.folds ? small_unit_m(one_product, one.num, one.den, nt, i, w & 1, (w >> 1) & 1, eq)
+                                                     : small_unit(one.kind, one.num, one.den, nt, i, w & 1, (w >> 1) & 1, lambda, eq);
+                            if (lane == 0) red[0][w] = v;
+                        }
+                    } else {
+                        for (uint32_t u = (warp + RES_WARPS - 2) & (RES_WARPS - 1); u < units * K; u += RES_WARPS) {
+                            const int k = u / units, w = u % units;
+                            if (tr.n_vars[k] < n_rem) continue;
+                            const bool folded = tr.n_vars[k] > n_rem;
+                            const void* den = folded ? den_work(k) : static_cast<const void*>(L.den[k]);
+                            const void* num = folded ? num_work(k) : static_cast<const void*>(L.num[k]);
+                            const int kind = folded && L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES ? (int)ZKB_GKR_LOGUP_GENERIC : L.kind[k];
+                            const qm31 v = small_unit(kind, num, den, nt, 32 * (w >> 2) + lane, w & 1, (w >> 1) & 1, lambda, eq);
+                            if (lane == 0) red[k][w] = v;
+                        }
+                    }
+                    __syncthreads();
+                }
+                if (warp == 0 && (K > 1 || units > 4)) {  // one oracle with four units: tr_round adds them itself
+                    for (int k = 0; k < K; k++) {
+                        if (tr.n_vars[k] < n_rem) continue;
+                        const qm31 v = (uint32_t)lane < units ? red[k][lane] : qm31_zero();
+                        const qm31 s0 = warp_sum_q((lane & 1) ? qm31_zero() : v), s2 = warp_sum_q((lane & 1) ? v : qm31_zero());
+                        if (lane == 0) { stq_r(tr.s.sums[k], 0, s0); stq_r(tr.s.sums[k], 1, s2); }
+                    }
+                    __syncwarp();
+                }
+                if (warp == 0) tr_round(tr, basis + BASIS_Q * round, K, n_rem, round, L.polys + (size_t)POLY_WORDS * round, K == 1 && units == 4 ? red[0] : nullptr);
+                __syncthreads();
+            }
+        }
+        if ((L.flags & CHAIN_END) && warp == 0) {
+            tr_end(tr, L, [&](int k) { return L.n_vars[k] && L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES ? (int)ZKB_GKR_LOGUP_GENERIC : L.kind[k]; },
+                   [&](int k) { return L.n_vars[k] ? num_work(k) : static_cast<const void*>(L.num[k]); },
+                   [&](int k) { return L.n_vars[k] ? den_work(k) : static_cast<const void*>(L.den[k]); });
+        }
+    }
+    __syncthreads();
+    if (warp == 0) tr_close_channel(tr, lane);
+    __syncthreads();
+    tr_store(tr, st, tid, RES_THREADS);
 }
 
 }  // namespace zk
 
 using namespace zk;
-using b200::B200Backend;
 using b200::BaseColumn;
 using b200::Device;
 using b200::Layer;
-using b200::SecureMle;
 
 namespace b200 {
 
 bool gkr_resident_supported(int n_inst, const uint64_t* ns) {
     if (n_inst < 1 || n_inst > RES_MAX_INST) return false;
     for (int i = 0; i < n_inst; i++)
-        if (ns[i] < 2 || ns[i] > ((uint64_t)1 << 30)) return false;
+        if (ns[i] < 2 || ns[i] > ((uint64_t)1 << (EQ_LOW + EQ_HIGH_MAX + 2))) return false;
     return true;
 }
+
+namespace {
+
+// One instance's layers: level 0 is the caller's input, level j has 2^(log - j) entries.
+struct Tower {
+    int kind, log;
+    const uint32_t *num, *den;
+    std::vector<uint32_t*> num_l, den_l;  // levels 1 ... log at [level]
+    int kind_at(int level) const { return level == 0 || kind == ZKB_GKR_GRAND_PRODUCT ? kind : (int)ZKB_GKR_LOGUP_GENERIC; }
+    const uint32_t* num_at(int level) const { return level == 0 ? num : num_l[level]; }
+    const uint32_t* den_at(int level) const { return level == 0 ? den : den_l[level]; }
+};
+
+// Launches of one proof: all but the first are programmatic dependents of the one before (every kernel here waits for its
+// predecessor before it reads anything), except under the per-kernel timeline, whose events sit between the launches.
+struct Launcher {
+    zkb_ctx* ctx;
+    bool chained = false;
+    cudaError_t err = cudaSuccess;
+    template <class... P, class... A>
+    void run(const char* name, void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, A... args) {
+        if (err != cudaSuccess) return;
+        ProfScope prof(ctx, name);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = chained && !ctx->prof_on ? 1 : 0;
+        err = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+        chained = true;
+    }
+};
+
+}  // namespace
 
 int gkr_prove_resident(zkb_ctx* ctx, std::vector<Layer> input_layers, uint32_t digest[8], uint32_t* n_draws,
                        std::vector<uint32_t>& o) {
     Device d(ctx);
-    const size_t n_inst = input_layers.size();
-    std::vector<size_t> n_layers_by_inst;
-    for (auto& l : input_layers) n_layers_by_inst.push_back(l.n_variables());
-    size_t n_layers = 0;
-    for (auto v : n_layers_by_inst) n_layers = std::max(n_layers, v);
-    std::vector<std::vector<Layer>> towers(n_inst);  // gen_layers, gkr_prover.rs:847-852
-    for (size_t i = 0; i < n_inst; i++) {
-        towers[i].push_back(std::move(input_layers[i]));
-        while (towers[i].back().n_variables() > 0) towers[i].push_back(B200Backend::next_layer(d, towers[i].back()));
-    }
-    BaseColumn state_buf(d, (sizeof(ResState) + 3) / 4, true);
-    ResState* st = reinterpret_cast<ResState*>(state_buf.ptr());
-    {
-        uint32_t head[12] = {0};
-        for (int k = 0; k < 8; k++) head[k] = digest[k];
-        head[8] = *n_draws;
-        d.check(zkb_h2d(ctx, st, head, sizeof(head)));
-    }
-    cudaStream_t stream = ctx->stream;
     DeviceGuard guard(ctx);
-    std::vector<bool> active(n_inst, false);
-    std::vector<std::vector<int>> layer_oracle_inst(n_layers);   // per layer: instance of each oracle
-    std::vector<std::vector<int>> layer_oracle_cols(n_layers);   // per layer: columns of each oracle's mask
-    std::vector<int> layer_first_poly(n_layers), layer_nv(n_layers);
-    int poly_slot = 0;
-    auto take = [&](size_t i) { Layer l = std::move(towers[i].back()); towers[i].pop_back(); return l; };
-    size_t ood_len = 0;
-    for (size_t layer = 0; layer < n_layers; layer++) {
-        const size_t n_remaining = n_layers - layer;
-        BeginArgs ba;
-        memset(&ba, 0, sizeof(ba));
-        ba.n_inst = (int)n_inst;
-        std::vector<Layer> out_layers;  // kept alive until the kernel has read them (stream-ordered frees)
-        for (size_t i = 0; i < n_inst; i++)
-            if (n_layers_by_inst[i] == n_remaining) {
-                out_layers.push_back(take(i));
-                const Layer& out = out_layers.back();
-                ba.activate[i] = 1;
-                ba.kind[i] = out.kind;
-                ba.out_den[i] = out.den.words.ptr();
-                ba.out_num[i] = out.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? out.num_base.ptr() : out.num_ptr();
-                active[i] = true;
-            }
-        std::vector<Layer> oracle_layers;
-        std::vector<int> nvars;
-        for (size_t i = 0; i < n_inst; i++) {
-            ba.active[i] = active[i] ? 1 : 0;
-            if (active[i]) {
-                ba.oracle_inst[oracle_layers.size()] = (int)i;
-                oracle_layers.push_back(take(i));
-                nvars.push_back((int)oracle_layers.back().n_variables() - 1);
-            }
+    const int n_inst = (int)input_layers.size();
+    std::vector<Tower> towers(n_inst);
+    int n_layers = 0;
+    for (int i = 0; i < n_inst; i++) {
+        const Layer& l = input_layers[i];
+        towers[i].kind = l.kind;
+        towers[i].log = (int)l.n_variables();
+        towers[i].num = l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? l.num_base.ptr() : l.num_ptr();
+        towers[i].den = l.den.words.ptr();
+        n_layers = std::max(n_layers, towers[i].log);
+    }
+    // ---- one allocation: the proof (state, round polynomials, masks: what the copy at the end brings back), the towers, the
+    // folded copies of the input layers, the basis and eq tables of the layers whose rounds are launches
+    const size_t n_polys = (size_t)n_layers * (n_layers - 1) / 2;
+    size_t words = 0;
+    auto reserve = [&](size_t n) { size_t at = words; words += (n + 63) & ~(size_t)63; return at; };
+    const size_t at_state = reserve(sizeof(ResState) / 4), at_polys = reserve(n_polys * POLY_WORDS);
+    std::vector<size_t> at_masks(n_layers);
+    std::vector<std::vector<int>> oracle_inst(n_layers);
+    for (int layer = 0; layer < n_layers; layer++) {
+        for (int i = 0; i < n_inst; i++)
+            if (towers[i].log >= n_layers - layer) oracle_inst[layer].push_back(i);
+        at_masks[layer] = reserve(MASK_WORDS * oracle_inst[layer].size());
+    }
+    const size_t copy_words = words;
+    std::vector<std::vector<std::pair<size_t, size_t>>> at_tower(n_inst);
+    std::vector<std::pair<size_t, size_t>> at_fold(n_inst);
+    for (int i = 0; i < n_inst; i++) {
+        at_tower[i].resize(towers[i].log + 1);
+        const bool nums = towers[i].kind != ZKB_GKR_GRAND_PRODUCT;
+        for (int lv = 1; lv <= towers[i].log; lv++) {
+            at_tower[i][lv].second = reserve((size_t)4 << (towers[i].log - lv));
+            at_tower[i][lv].first = nums ? reserve((size_t)4 << (towers[i].log - lv)) : 0;
         }
-        const int n_or = (int)oracle_layers.size();
-        int nv = 0;
-        for (int v : nvars) nv = std::max(nv, v);
-        for (int k = 0; k < n_or; k++) ba.oracle_nvars[k] = nvars[k];
-        ba.n_oracles = n_or;
-        ba.nv = nv;
-        { ProfScope prof(ctx, "res_layer_begin_kernel"); res_layer_begin_kernel<<<1, 32, 0, stream>>>(st, ba); }
-        ZKB_LAUNCH_CHECK(ctx);
-        out_layers.clear();
-        // EqEvals::generate (gkr_prover.rs:235-247): eq(., ood[1..]) scaled by eq(0, ood[0]); nv - ... entries
-        const int ny = ood_len == 0 ? 0 : (int)ood_len - 1;
-        SecureMle eq_evals(d, (size_t)1 << ny);
-        {
-            const uint32_t* d_y = ood_len == 0 ? nullptr : reinterpret_cast<const uint32_t*>(&st->ood[1]);
-            int rc = gkr_eq_evals_launch(ctx, d_y, ny, reinterpret_cast<const uint32_t*>(&st->eq_v), eq_evals.words.ptr());
-            if (rc) return rc;
+        const bool fold_nums = towers[i].kind == ZKB_GKR_LOGUP_GENERIC || towers[i].kind == ZKB_GKR_LOGUP_MULTIPLICITIES;
+        at_fold[i].second = reserve((size_t)2 << towers[i].log);
+        at_fold[i].first = fold_nums ? reserve((size_t)2 << towers[i].log) : 0;
+    }
+    const size_t at_basis = reserve(4 * BASIS_Q * RES_MAX_VARS), at_low = reserve((size_t)4 << EQ_LOW), at_high = reserve((size_t)4 << EQ_HIGH_MAX);
+    BaseColumn buf(d, words);
+    uint32_t* const base = buf.ptr();
+    ResState* const st = reinterpret_cast<ResState*>(base + at_state);
+    for (int i = 0; i < n_inst; i++) {
+        towers[i].num_l.assign(towers[i].log + 1, nullptr);
+        towers[i].den_l.assign(towers[i].log + 1, nullptr);
+        for (int lv = 1; lv <= towers[i].log; lv++) {
+            towers[i].den_l[lv] = base + at_tower[i][lv].second;
+            if (towers[i].kind != ZKB_GKR_GRAND_PRODUCT) towers[i].num_l[lv] = base + at_tower[i][lv].first;
         }
-        const uint32_t* d_lambda = reinterpret_cast<const uint32_t*>(&st->lambda);
-        const uint32_t* d_r = reinterpret_cast<const uint32_t*>(&st->challenge);
-        std::vector<bool> have_sums(n_or, false);
-        layer_first_poly[layer] = poly_slot;
-        layer_nv[layer] = nv;
-        // rounds in which some layer still has more than 2^TAIL_MAX_LOG entries run as separate launches
-        const int round_start = nv > TAIL_MAX_LOG - 1 ? nv - (TAIL_MAX_LOG - 1) : 0;
-        for (int round = 0; round < round_start; round++) {
-            const int n_rem = nv - round;
-            for (int k = 0; k < n_or; k++)
-                if (n_rem == nvars[k] && !have_sums[k]) {
-                    const Layer& l = oracle_layers[k];
-                    const uint32_t* num = l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? l.num_base.ptr() : l.num_ptr();
-                    int rc = gkr_sum_launch(ctx, l.kind, num, l.den.words.ptr(), l.len(), eq_evals.words.ptr(), d_lambda, st->sums[k]);
-                    if (rc) return rc;
-                }
-            RoundArgs ra;
-            memset(&ra, 0, sizeof(ra));
-            ra.n_oracles = n_or;
-            ra.n_rem = n_rem;
-            ra.round = round;
-            ra.poly_slot = poly_slot++;
-            for (int k = 0; k < n_or; k++) ra.nvars[k] = nvars[k];
-            { ProfScope prof(ctx, "res_round_kernel"); res_round_kernel<<<1, 32, 0, stream>>>(st, ra); }
-            ZKB_LAUNCH_CHECK(ctx);
-            for (int k = 0; k < n_or; k++)
-                if (n_rem == nvars[k] && nvars[k] != 0) {
-                    Layer& l = oracle_layers[k];
-                    const size_t n = l.len();
-                    Layer out;
-                    out.kind = l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? ZKB_GKR_LOGUP_GENERIC : l.kind;
-                    out.den = SecureMle(d, n / 2);
-                    if (out.kind == ZKB_GKR_LOGUP_GENERIC) out.num = SecureMle(d, n / 2);
-                    const uint32_t* num = l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? l.num_base.ptr() : l.num_ptr();
-                    int rc;
-                    if (n >= 8) {
-                        rc = gkr_fold_sum_launch(ctx, l.kind, num, l.den.words.ptr(), n, d_r, eq_evals.words.ptr(), d_lambda,
-                                                 out.kind == ZKB_GKR_LOGUP_GENERIC ? out.num.words.ptr() : nullptr, out.den.words.ptr(),
-                                                 st->sums[k]);
-                        have_sums[k] = true;
-                    } else {
-                        rc = gkr_mle_fix_launch(ctx, false, l.den.words.ptr(), n, d_r, out.den.words.ptr());
-                        if (!rc && l.kind == ZKB_GKR_LOGUP_GENERIC) rc = gkr_mle_fix_launch(ctx, false, l.num.words.ptr(), n, d_r, out.num.words.ptr());
-                        if (!rc && l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) rc = gkr_mle_fix_launch(ctx, true, l.num_base.ptr(), n, d_r, out.num.words.ptr());
-                        have_sums[k] = false;
+    }
+    // ---- the plan: chain layers, and the launched rounds that go between two of them
+    struct Step { int chain_first, chain_count; std::vector<std::pair<int, RoundArgs>> rounds; };  // (kind + 4 if it folds, arguments)
+    std::vector<ChainLayer> chain;
+    std::vector<Step> steps(1, Step{0, 0, {}});
+    int poly_base = 0;
+    for (int layer = 0; layer < n_layers; layer++) {
+        const int nv = layer, K = (int)oracle_inst[layer].size();
+        ChainLayer L;
+        memset(&L, 0, sizeof(L));
+        L.nv = nv;
+        L.n_inst = n_inst;
+        L.n_oracles = K;
+        L.polys = base + at_polys + (size_t)POLY_WORDS * poly_base;
+        L.masks = base + at_masks[layer];
+        L.basis = reinterpret_cast<qm31*>(base + at_basis);
+        L.eq_low = base + at_low;
+        L.eq_high = base + at_high;
+        for (int i = 0; i < n_inst; i++) {
+            const Tower& t = towers[i];
+            L.start_kind[i] = -1;
+            L.active[i] = t.log >= n_layers - layer;
+            if (L.active[i]) L.last_active = i;
+            if (t.log == n_layers - layer) { L.start_kind[i] = t.kind_at(t.log); L.out_num[i] = t.num_at(t.log); L.out_den[i] = t.den_at(t.log); }
+        }
+        std::vector<int> level(K);
+        size_t smem = 0;
+        for (int k = 0; k < K; k++) {
+            const int i = oracle_inst[layer][k];
+            const Tower& t = towers[i];
+            const int log_entries = 1 + layer - (n_layers - t.log);
+            level[k] = t.log - log_entries;
+            L.inst[k] = i;
+            L.n_vars[k] = (uint32_t)(log_entries - 1);
+            L.kind[k] = t.kind_at(level[k]);
+            L.num[k] = t.num_at(level[k]);
+            L.den[k] = t.den_at(level[k]);
+            if (L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES && L.n_vars[k] == 0)
+                return set_error(ctx, ZKB_EINVAL, "gkr: a multiplicities layer cannot be a mask");
+            const size_t bytes = (size_t)16 << std::min<uint32_t>(L.n_vars[k], CHAIN_LOG - 1);
+            L.den_work[k] = smem; smem += bytes;
+            if (L.kind[k] != ZKB_GKR_GRAND_PRODUCT) { L.num_work[k] = smem; smem += bytes; }
+        }
+        L.work_global = smem > CHAIN_WORK_BYTES ? 1 : 0;
+        if (L.work_global)  // several tall oracles at once: in place for the towers' layers, the folded copies for the inputs
+            for (int k = 0; k < K; k++) {
+                const Tower& t = towers[L.inst[k]];
+                L.den_work[k] = (uint64_t)(level[k] ? t.den_l[level[k]] : base + at_fold[L.inst[k]].second);
+                L.num_work[k] = (uint64_t)(level[k] ? t.num_l[level[k]] : base + at_fold[L.inst[k]].first);
+            }
+        // Rounds whose pass reads more than 2^CHAIN_LOG entries are launches of their own (the first pass of a layer reads
+        // 2^(nv + 1), a fold with k variables left after it 2^(k + 2)).
+        const int round_start = nv + 1 > CHAIN_LOG ? nv - (CHAIN_LOG - 2) : 0;
+        if (round_start > 0) {
+            ChainLayer B = L;
+            B.flags = CHAIN_BEGIN;
+            B.table_bits = nv - 1 - EQ_LOW;
+            chain.push_back(B);
+            steps.back().chain_count++;
+            std::vector<int> kind(L.kind, L.kind + K);
+            for (int round = 0; round < round_start; round++) {
+                const uint32_t n_rem = (uint32_t)(nv - round);
+                size_t last = 0;
+                for (int k = 0; k < K; k++) {
+                    if (L.n_vars[k] < n_rem) continue;
+                    RoundArgs a;
+                    memset(&a, 0, sizeof(a));
+                    const bool fold = L.n_vars[k] > n_rem;
+                    const Tower& t = towers[L.inst[k]];
+                    a.num = L.num[k];
+                    a.den = L.den[k];
+                    const int in_kind = kind[k];
+                    if (fold) {
+                        a.den_out = level[k] ? t.den_l[level[k]] : base + at_fold[L.inst[k]].second;
+                        a.num_out = level[k] ? t.num_l[level[k]] : base + at_fold[L.inst[k]].first;
+                        L.den[k] = a.den_out;
+                        if (in_kind == ZKB_GKR_LOGUP_GENERIC || in_kind == ZKB_GKR_LOGUP_MULTIPLICITIES) { L.num[k] = a.num_out; kind[k] = ZKB_GKR_LOGUP_GENERIC; }
                     }
-                    if (rc) return rc;
-                    l = std::move(out);
-                    nvars[k]--;  // the oracle's n_variables() follows its layer
+                    a.eq_low = L.eq_low;
+                    a.eq_high = L.eq_high;
+                    a.nt = (size_t)1 << (n_rem - 1);
+                    // chunks: as long as possible (a factor of the high table is taken once per chunk) while there are enough for every SM
+                    a.chunk_log = EQ_LOW;
+                    while (a.chunk_log > 8 && (a.nt >> a.chunk_log) < 148 * 2) a.chunk_log--;
+                    a.partials = ctx->scratch;
+                    a.ticket = ctx->ticket;
+                    a.st = st;
+                    a.basis = L.basis + BASIS_Q * round;
+                    a.poly = L.polys + (size_t)POLY_WORDS * round;
+                    a.oracle = k;
+                    a.n_oracles = K;
+                    a.n_rem = (int)n_rem;
+                    a.round = round;
+                    for (int q = 0; q < K; q++) a.n_vars[q] = L.n_vars[q];
+                    steps.back().rounds.push_back({in_kind + (fold ? 4 : 0), a});
+                    last = steps.back().rounds.size() - 1;
                 }
+                steps.back().rounds[last].second.transcript = 1;
+            }
+            for (int k = 0; k < K; k++) L.kind[k] = kind[k];
+            L.flags = CHAIN_ROUNDS | CHAIN_END;
+            L.round_start = round_start;
+            steps.push_back(Step{(int)chain.size(), 0, {}});
+        } else {
+            L.flags = CHAIN_BEGIN | CHAIN_ROUNDS | CHAIN_END;
         }
-        // the remaining rounds: one launch
-        std::vector<SecureMle> work;  // alive until layer_end has been enqueued (stream-ordered frees)
-        std::vector<int> fin_kind(n_or);
-        std::vector<const uint32_t*> fin_num(n_or), fin_den(n_or);
-        TailArgs ta;
-        memset(&ta, 0, sizeof(ta));
-        ta.n_oracles = n_or;
-        ta.nv = nv;
-        ta.round_start = round_start;
-        ta.first_poly_slot = poly_slot;
-        ta.eq_evals = eq_evals.words.ptr();
-        for (int k = 0; k < n_or; k++) {
-            const Layer& l = oracle_layers[k];
-            ta.kind[k] = l.kind;
-            ta.nvars[k] = nvars[k];
-            ta.num[k] = l.num_ptr();
-            ta.den[k] = l.den.words.ptr();
-            fin_kind[k] = l.kind;
-            fin_num[k] = l.num_ptr();
-            fin_den[k] = l.den.words.ptr();
-            if (l.len() > ((size_t)1 << TAIL_MAX_LOG) && round_start < nv) return set_error(ctx, ZKB_EINVAL, "gkr: tail layer too large");
-            if (nvars[k] >= 1 && round_start < nv) {  // folded at least once by the tail kernel
-                const bool has_num = l.kind == ZKB_GKR_LOGUP_GENERIC || l.kind == ZKB_GKR_LOGUP_MULTIPLICITIES;
-                work.emplace_back(d, l.len() / 2);
-                ta.den_w[k] = work.back().words.ptr();
-                fin_den[k] = ta.den_w[k];
-                if (has_num) {
-                    work.emplace_back(d, l.len() / 2);
-                    ta.num_w[k] = work.back().words.ptr();
-                    fin_num[k] = ta.num_w[k];
-                    fin_kind[k] = ZKB_GKR_LOGUP_GENERIC;
-                }
-            } else if (l.len() != 2) {
-                return set_error(ctx, ZKB_EINVAL, "gkr: oracle is not constant after sumcheck");
+        chain.push_back(L);
+        steps.back().chain_count++;
+        poly_base += nv;
+    }
+    // ---- enqueue
+    void* d_chain = nullptr;
+    if (int rc = stage_blob(ctx, chain.data(), chain.size() * sizeof(ChainLayer), &d_chain)) return rc;
+    if (!ctx->res_ready) {
+        ZKB_CUDA(ctx, cudaFuncSetAttribute(res_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHAIN_SMEM));
+        ctx->res_ready = true;
+    }
+    Launcher launch{ctx};
+    for (int i = 0; i < n_inst; i++) {
+        const Tower& t = towers[i];
+        for (int level = 0; level < t.log;) {
+            TowerArgs a;
+            memset(&a, 0, sizeof(a));
+            a.num = t.num_at(level);
+            a.den = t.den_at(level);
+            a.cta_log = std::min(TOWER_LEVELS, t.log - level);
+            a.levels = a.cta_log;
+            for (int l = 0; l < a.levels; l++) { a.num_out[l] = t.num_l[level + 1 + l]; a.den_out[l] = t.den_l[level + 1 + l]; }
+            const unsigned grid = 1u << (t.log - level - a.cta_log);
+            switch (t.kind_at(level)) {
+                case ZKB_GKR_GRAND_PRODUCT: launch.run("tower_kernel", tower_kernel<0>, grid, TOWER_THREADS, 0, a); break;
+                case ZKB_GKR_LOGUP_GENERIC: launch.run("tower_kernel", tower_kernel<1>, grid, TOWER_THREADS, 0, a); break;
+                case ZKB_GKR_LOGUP_MULTIPLICITIES: launch.run("tower_kernel", tower_kernel<2>, grid, TOWER_THREADS, 0, a); break;
+                default: launch.run("tower_kernel", tower_kernel<3>, grid, TOWER_THREADS, 0, a); break;
+            }
+            level += a.levels;
+        }
+    }
+    ResInit init;
+    memcpy(init.digest, digest, 32);
+    init.n_draws = *n_draws;
+    init.use = 1;
+    for (auto& s : steps) {
+        launch.run("res_chain_kernel", res_chain_kernel, 1u, RES_THREADS, CHAIN_SMEM, st, (const ChainLayer*)d_chain + s.chain_first, s.chain_count, init);
+        init.use = 0;
+        for (auto& r : s.rounds) {
+            const unsigned grid = (unsigned)std::min<size_t>(r.second.nt >> r.second.chunk_log, ROUND_MAX_CTAS);
+            switch (r.first) {
+                case 0: launch.run("res_round_kernel(sums)", res_round_kernel<0, false>, grid, ROUND_THREADS, 0, r.second); break;
+                case 1: launch.run("res_round_kernel(sums)", res_round_kernel<1, false>, grid, ROUND_THREADS, 0, r.second); break;
+                case 2: launch.run("res_round_kernel(sums)", res_round_kernel<2, false>, grid, ROUND_THREADS, 0, r.second); break;
+                case 3: launch.run("res_round_kernel(sums)", res_round_kernel<3, false>, grid, ROUND_THREADS, 0, r.second); break;
+                case 4: launch.run("res_round_kernel(fold)", res_round_kernel<0, true>, grid, ROUND_THREADS, 0, r.second); break;
+                case 5: launch.run("res_round_kernel(fold)", res_round_kernel<1, true>, grid, ROUND_THREADS, 0, r.second); break;
+                case 6: launch.run("res_round_kernel(fold)", res_round_kernel<2, true>, grid, ROUND_THREADS, 0, r.second); break;
+                default: launch.run("res_round_kernel(fold)", res_round_kernel<3, true>, grid, ROUND_THREADS, 0, r.second); break;
             }
         }
-        if (round_start < nv) {
-            ProfScope prof(ctx, "res_tail_kernel");
-            res_tail_kernel<<<1, TAIL_THREADS, 0, stream>>>(st, ta);
-            ZKB_LAUNCH_CHECK(ctx);
-            poly_slot += nv - round_start;
-        }
-        EndArgs ea;
-        memset(&ea, 0, sizeof(ea));
-        ea.n_oracles = n_or;
-        ea.nv = nv;
-        ea.layer = (int)layer;
-        for (int k = 0; k < n_or; k++) {
-            if (fin_kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES) return set_error(ctx, ZKB_EINVAL, "gkr: a multiplicities layer cannot be a mask");
-            ea.kind[k] = fin_kind[k];
-            ea.inst[k] = ba.oracle_inst[k];
-            ea.den[k] = fin_den[k];
-            ea.num[k] = fin_num[k];
-            layer_oracle_inst[layer].push_back(ba.oracle_inst[k]);
-            layer_oracle_cols[layer].push_back(fin_kind[k] == ZKB_GKR_GRAND_PRODUCT ? 1 : 2);
-        }
-        { ProfScope prof(ctx, "res_layer_end_kernel"); res_layer_end_kernel<<<1, 32, 0, stream>>>(st, ea); }
-        ZKB_LAUNCH_CHECK(ctx);
-        ood_len = (size_t)nv + 1;
     }
-    // one copy, one synchronisation
-    std::vector<uint32_t> raw = state_buf.to_cpu();
-    const ResState* h = reinterpret_cast<const ResState*>(raw.data());
-    if (h->error) return set_error(ctx, ZKB_EINVAL, "sumcheck: round polynomial does not match the claim");
-    for (int k = 0; k < 8; k++) digest[k] = h->digest[k];
-    *n_draws = h->n_draws;
-    auto put = [&](const qm31& q) { o.insert(o.end(), q.c, q.c + 4); };
+    if (launch.err != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr: %s", cudaGetErrorString(launch.err));
+    // ---- one copy, one synchronisation
+    if (copy_words > (size_t)SMALL_WORDS) return set_error(ctx, ZKB_EINVAL, "gkr: the proof exceeds the landing buffer");
+    ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, base, copy_words * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const uint32_t* h = ctx->h_small;
+    const ResState* hs = reinterpret_cast<const ResState*>(h + at_state);
+    memcpy(digest, hs->digest, 32);
+    *n_draws = hs->n_draws;
+    auto put = [&](const uint32_t* q) { o.insert(o.end(), q, q + 4); };
+    o.reserve(o.size() + copy_words);
     o.push_back((uint32_t)n_layers);
-    for (size_t layer = 0; layer < n_layers; layer++) {
-        o.push_back((uint32_t)layer_nv[layer]);
-        for (int r = 0; r < layer_nv[layer]; r++) {
-            const Poly4& p = h->round_polys[layer_first_poly[layer] + r];
-            o.push_back((uint32_t)p.n);
-            for (int j = 0; j < p.n; j++) put(p.c[j]);
+    const uint32_t* poly = h + at_polys;
+    for (int layer = 0; layer < n_layers; layer++) {
+        o.push_back((uint32_t)layer);
+        for (int r = 0; r < layer; r++, poly += POLY_WORDS) {
+            o.push_back(poly[16]);
+            for (uint32_t j = 0; j < poly[16]; j++) put(poly + 4 * j);
         }
     }
-    for (size_t i = 0; i < n_inst; i++) {
-        std::vector<std::pair<size_t, int>> where;  // (layer, oracle index) of every mask of this instance
-        for (size_t layer = 0; layer < n_layers; layer++)
-            for (size_t k = 0; k < layer_oracle_inst[layer].size(); k++)
-                if (layer_oracle_inst[layer][k] == (int)i) where.push_back({layer, (int)k});
-        o.push_back((uint32_t)where.size());
-        for (auto& w : where) {
-            int cols = layer_oracle_cols[w.first][w.second];
-            o.push_back((uint32_t)cols);
-            for (int c = 0; c < 2 * cols; c++) put(h->masks[w.first][w.second][c]);
+    for (int i = 0; i < n_inst; i++) {
+        o.push_back((uint32_t)towers[i].log);  // one mask per layer the instance is in
+        for (int layer = n_layers - towers[i].log; layer < n_layers; layer++) {
+            const size_t k = std::find(oracle_inst[layer].begin(), oracle_inst[layer].end(), i) - oracle_inst[layer].begin();
+            const uint32_t* m = h + at_masks[layer] + MASK_WORDS * k;
+            const uint32_t cols = towers[i].kind == ZKB_GKR_GRAND_PRODUCT ? 1u : 2u;
+            o.push_back(cols);
+            for (uint32_t c = 0; c < 2 * cols; c++) put(m + 4 * c);
         }
     }
-    for (size_t i = 0; i < n_inst; i++) {
-        o.push_back(h->n_output_claims[i]);
-        for (uint32_t c = 0; c < h->n_output_claims[i]; c++) put(h->output_claims[i][c]);
+    for (int i = 0; i < n_inst; i++) {
+        o.push_back(hs->n_out_claims[i]);
+        for (uint32_t c = 0; c < hs->n_out_claims[i]; c++) put(hs->out_claims[i][c].c);
     }
-    o.push_back(h->ood_len);
-    for (uint32_t j = 0; j < h->ood_len; j++) put(h->ood[j]);
-    for (size_t i = 0; i < n_inst; i++) {
-        o.push_back(h->n_claims[i]);
-        for (uint32_t c = 0; c < h->n_claims[i]; c++) put(h->claims[i][c]);
+    o.push_back((uint32_t)n_layers);
+    for (int j = 0; j < n_layers; j++) put(hs->ood[j].c);
+    for (int i = 0; i < n_inst; i++) {
+        o.push_back(hs->n_claims[i]);
+        for (uint32_t c = 0; c < hs->n_claims[i]; c++) put(hs->claims[i][c].c);
     }
     return ZKB_OK;
 }
