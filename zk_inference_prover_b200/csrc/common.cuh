@@ -8,6 +8,8 @@
 #include "../../include/zkb200.h"
 #include "m31.cuh"
 
+namespace zk { struct BlockCache; }
+
 struct zkb_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -26,6 +28,12 @@ struct zkb_ctx {
     void** h_ring = nullptr;
     void** d_ring = nullptr;
     size_t ring_cap = 0, ring_pos = 0;
+    // The tables staged last, still intact in the ring: a table of the same pointers is not copied again (stage_ptrs).
+    struct StagedTable { size_t pos, n; };
+    static constexpr int STAGED_TABLES = 32;
+    StagedTable staged[STAGED_TABLES] = {};
+    int staged_next = 0;
+    zk::BlockCache* blocks = nullptr;  // small device allocations given back (zkb_malloc)
     // Scratch for per-block partial results (round sums, point evaluations) and a ticket counter.
     uint32_t* scratch = nullptr;
     size_t scratch_words = 0;
@@ -53,7 +61,7 @@ struct zkb_ctx {
 
 namespace zk {
 
-constexpr int RING_SLOTS = 1 << 18;        // pointer-table staging capacity (2 MiB of pointers)
+constexpr int RING_SLOTS = 1 << 20;        // pointer-table staging capacity (8 MiB of pointers)
 constexpr size_t SCRATCH_WORDS = 1 << 22;  // 16 MiB of scratch words
 constexpr int SMALL_WORDS = 1 << 15;
 
@@ -76,14 +84,14 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...);
 
 // RAII guard making the context's device current for the duration of a call.
 struct DeviceGuard {
-    int prev = -1;
+    int prev = -1, dev;
     bool ok = true;
-    explicit DeviceGuard(const zkb_ctx* ctx) {
+    explicit DeviceGuard(const zkb_ctx* ctx) : dev(ctx->device) {
         if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
         if (prev != ctx->device) ok = cudaSetDevice(ctx->device) == cudaSuccess;
     }
     ~DeviceGuard() {
-        if (prev >= 0) cudaSetDevice(prev);
+        if (prev >= 0 && prev != dev) cudaSetDevice(prev);
     }
 };
 

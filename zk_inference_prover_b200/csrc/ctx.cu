@@ -1,5 +1,6 @@
 // Context lifetime, device memory helpers, the twiddle tower and small utilities.
 #include <cstdarg>
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -17,18 +18,62 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...) {
     return code;
 }
 
+// The ring is used from its start again: earlier slots may still be in flight, so drain the stream, and forget what they held.
+static int stage_wrap(zkb_ctx* ctx) {
+    ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->ring_pos = 0;
+    for (auto& t : ctx->staged) t.n = 0;
+    return ZKB_OK;
+}
+
+// Device memory of a proof's small arrays (tree layers, FRI layers, coordinate columns): a proof allocates hundreds of them, and
+// the stream-ordered allocator takes 0.6-0.8 us of host time for each allocation and each release (716 us of a ten-column proof
+// were 230 of them). Blocks of up to 2^BLOCK_MAX_LOG bytes are rounded up to a power of two and kept per size when they are freed,
+// up to KEPT_BYTES in all; they go back to the pool beyond that, when an allocation fails and with the context. A context's work is
+// ordered on one stream, so a kept block is as reusable as one the pool would hand out on that stream.
+struct BlockCache {
+    static constexpr int MIN_LOG = 8, MAX_LOG = 24;
+    static constexpr size_t KEPT_BYTES = (size_t)256 << 20;
+    std::unordered_map<void*, int> live;  // block -> log2 of its size
+    std::vector<void*> kept[MAX_LOG + 1];
+    size_t kept_bytes = 0;
+    static int log_of(size_t bytes) {
+        int l = MIN_LOG;
+        while (((size_t)1 << l) < bytes) l++;
+        return l;
+    }
+    void release(cudaStream_t stream) {
+        for (auto& k : kept) {
+            for (void* p : k) cudaFreeAsync(p, stream);
+            k.clear();
+        }
+        kept_bytes = 0;
+    }
+};
+
+// Copies the table into the ring, unless the same table is still there from an earlier call: a tree's columns are named by the
+// interpolation, the extension, the hashing, the sampling, the numerators and the decommitment in turn, and a copy of a table in
+// between two kernels costs 2-3 us of the stream.
 int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out) {
     if (n < 0 || (size_t)n > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_ptrs: %d pointers exceed the staging ring", n);
     if (n == 0) { *out = ctx->d_ring; return ZKB_OK; }
+    // Near the ring's end a table from its first half is not reused: a later table of the same operator (operators stage less than a
+    // quarter of the ring) might start the ring again and be written over it.
+    const size_t from = ctx->ring_pos > ctx->ring_cap / 4 * 3 ? ctx->ring_cap / 2 : 0;
+    for (const auto& t : ctx->staged) {
+        if (t.n != (size_t)n || t.pos < from || ctx->h_ring[t.pos] != h_ptrs[0] || memcmp(ctx->h_ring + t.pos, h_ptrs, (size_t)n * sizeof(void*))) continue;
+        *out = ctx->d_ring + t.pos;
+        return ZKB_OK;
+    }
     if (ctx->ring_pos + (size_t)n > ctx->ring_cap) {
-        // Wrap: earlier slots may still be in flight, so drain the stream first.
-        ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        ctx->ring_pos = 0;
+        if (int rc = stage_wrap(ctx)) return rc;
     }
     void** h = ctx->h_ring + ctx->ring_pos;
     void** d = ctx->d_ring + ctx->ring_pos;
     memcpy(h, h_ptrs, (size_t)n * sizeof(void*));
     ZKB_CUDA(ctx, cudaMemcpyAsync(d, h, (size_t)n * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->staged[ctx->staged_next] = {ctx->ring_pos, (size_t)n};
+    ctx->staged_next = (ctx->staged_next + 1) % zkb_ctx::STAGED_TABLES;
     ctx->ring_pos += (size_t)n;
     *out = d;
     return ZKB_OK;
@@ -39,7 +84,7 @@ int stage_blob(zkb_ctx* ctx, const void* h_data, size_t bytes, void** out) {
     if (slots + 1 > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_blob: %zu bytes exceed the staging ring", bytes);
     size_t pos = (ctx->ring_pos + 1) & ~(size_t)1;  // slots are 8 bytes and the ring's base is aligned: even slots are 16-byte aligned
     if (pos + slots > ctx->ring_cap) {
-        ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // earlier slots may still be in flight
+        if (int rc = stage_wrap(ctx)) return rc;
         pos = 0;
     }
     memcpy(ctx->h_ring + pos, h_data, bytes);
@@ -101,6 +146,32 @@ __global__ void gather_words_kernel(const uint32_t* const* __restrict__ addrs, s
     if (t < n) out[t] = *addrs[t];
 }
 
+// Everything a read plan asks for (gather_plan). Thread t < n_cells: cell t of the blocks (their out_off ascending, found by
+// bisection); then a word per word address; then eight words per hash address.
+struct PlanBlock { const uint32_t* const* cols; uint32_t ncols, idx, out_off, pad; };  // idx: where its row indices start
+__global__ void __launch_bounds__(256) gather_plan_kernel(const PlanBlock* __restrict__ blocks, int n_blocks, const uint32_t* __restrict__ idx, uint32_t n_cells,
+                                                          const uint32_t* const* __restrict__ words, uint32_t n_words,
+                                                          const uint32_t* const* __restrict__ hashes, uint32_t n_hashes, uint32_t* __restrict__ out) {
+    uint32_t t = blockIdx.x * 256u + threadIdx.x;
+    if (t < n_cells) {
+        int lo = 0, hi = n_blocks - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (blocks[mid].out_off <= t) lo = mid; else hi = mid - 1;
+        }
+        const PlanBlock b = blocks[lo];
+        const uint32_t e = t - b.out_off;
+        out[t] = b.cols[e % b.ncols][idx[b.idx + e / b.ncols]];
+        return;
+    }
+    if (t < n_cells + n_words) {
+        out[t] = *words[t - n_cells];
+        return;
+    }
+    const uint32_t h = t - n_cells - n_words;
+    if (h < 8 * n_hashes) out[t] = hashes[h >> 3][h & 7];
+}
+
 }  // namespace zk
 
 using namespace zk;
@@ -117,8 +188,10 @@ int zkb_init(int device, int max_log_size, zkb_ctx** out) {
     if (!ctx) return ZKB_ENOMEM;
     ctx->device = device;
     ctx->max_log = max_log_size;
+    ctx->blocks = new (std::nothrow) BlockCache();
+    if (!ctx->blocks) { delete ctx; return ZKB_ENOMEM; }
     cudaError_t e = cudaSetDevice(device);
-    if (e != cudaSuccess) { delete ctx; return ZKB_ECUDA; }
+    if (e != cudaSuccess) { delete ctx->blocks; delete ctx; return ZKB_ECUDA; }
     auto fail = [&](int code) { zkb_destroy(ctx); return code; };
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(ZKB_ECUDA);
     ctx->tw_len = (size_t)1 << (max_log_size - 1);
@@ -161,7 +234,11 @@ int zkb_init(int device, int max_log_size, zkb_ctx** out) {
 int zkb_destroy(zkb_ctx* ctx) {
     if (!ctx) return ZKB_EINVAL;
     cudaSetDevice(ctx->device);
-    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->stream) {
+        ctx->blocks->release(ctx->stream);
+        cudaStreamSynchronize(ctx->stream);
+    }
+    delete ctx->blocks;
     if (ctx->tw) cudaFree(ctx->tw);
     if (ctx->itw) cudaFree(ctx->itw);
     if (ctx->tw2) cudaFree(ctx->tw2);
@@ -278,7 +355,25 @@ int zkb_malloc(zkb_ctx* ctx, size_t bytes, void** dptr) {
     if (bytes == 0) return ZKB_OK;
     // Stream-ordered allocation from the device's default pool (kept warm: the release threshold
     // is raised in zkb_init), so neither allocation nor release synchronises the device.
-    ZKB_CUDA(ctx, cudaMallocAsync(dptr, bytes, ctx->stream));
+    BlockCache& bc = *ctx->blocks;
+    const bool small = bytes <= ((size_t)1 << BlockCache::MAX_LOG);
+    const int log = small ? BlockCache::log_of(bytes) : 0;
+    if (small && !bc.kept[log].empty()) {
+        *dptr = bc.kept[log].back();
+        bc.kept[log].pop_back();
+        bc.kept_bytes -= (size_t)1 << log;
+        bc.live[*dptr] = log;
+        return ZKB_OK;
+    }
+    const size_t want = small ? (size_t)1 << log : bytes;
+    cudaError_t e = cudaMallocAsync(dptr, want, ctx->stream);
+    if (e == cudaErrorMemoryAllocation && bc.kept_bytes) {
+        (void)cudaGetLastError();
+        bc.release(ctx->stream);
+        e = cudaMallocAsync(dptr, want, ctx->stream);
+    }
+    ZKB_CUDA(ctx, e);
+    if (small) bc.live[*dptr] = log;
     return ZKB_OK;
 }
 
@@ -286,6 +381,17 @@ int zkb_free(zkb_ctx* ctx, void* dptr) {
     if (!ctx) return ZKB_EINVAL;
     if (!dptr) return ZKB_OK;
     DeviceGuard g(ctx);
+    BlockCache& bc = *ctx->blocks;
+    auto it = bc.live.find(dptr);
+    if (it != bc.live.end()) {
+        const int log = it->second;
+        bc.live.erase(it);
+        if (bc.kept_bytes + ((size_t)1 << log) <= BlockCache::KEPT_BYTES) {
+            bc.kept[log].push_back(dptr);
+            bc.kept_bytes += (size_t)1 << log;
+            return ZKB_OK;
+        }
+    }
     ZKB_CUDA(ctx, cudaFreeAsync(dptr, ctx->stream));
     return ZKB_OK;
 }
@@ -548,36 +654,69 @@ int zkb_secure_powers(zkb_ctx* ctx, const uint32_t h_felt[4], size_t n, uint32_t
 
 namespace zk {
 
-int gather_blocks(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t total_words, uint32_t* h_out) {
-    if (n_blocks <= 0 || total_words == 0) return ZKB_OK;
+int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t total_words, const uint32_t* const* word_addrs, size_t n_words,
+                const uint32_t* const* hash_addrs, size_t n_hashes, uint32_t* h_out) {
+    const size_t results = total_words + n_words + 8 * n_hashes;
+    if (results == 0) return ZKB_OK;
     DeviceGuard g(ctx);
-    std::vector<uint32_t> idx;
-    for (int b = 0; b < n_blocks; b++) idx.insert(idx.end(), blocks[b].idx, blocks[b].idx + blocks[b].nidx);
-    uint32_t* d_buf = nullptr;  // [indices | results]
-    ZKB_CUDA(ctx, cudaMallocAsync((void**)&d_buf, (idx.size() + total_words) * 4, ctx->stream));
-    cudaError_t e = cudaMemcpyAsync(d_buf, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, ctx->stream);
-    uint32_t* d_out = d_buf + idx.size();
-    size_t ioff = 0;
+    size_t n_idx = 0;
+    for (int b = 0; b < n_blocks; b++) n_idx += (size_t)blocks[b].nidx;
+    // [word addresses | hash addresses | block descriptors | row indices]
+    const size_t at_hash = 8 * n_words, at_blocks = at_hash + 8 * n_hashes, at_idx = at_blocks + sizeof(PlanBlock) * (size_t)n_blocks;
+    std::vector<unsigned char> blob(at_idx + 4 * n_idx);
+    if (n_words) memcpy(blob.data(), word_addrs, 8 * n_words);
+    if (n_hashes) memcpy(blob.data() + at_hash, hash_addrs, 8 * n_hashes);
+    PlanBlock* pb = reinterpret_cast<PlanBlock*>(blob.data() + at_blocks);
+    uint32_t* pi = reinterpret_cast<uint32_t*>(blob.data() + at_idx);
+    size_t first_idx = 0;
+    for (int b = 0; b < n_blocks; b++) {
+        void** cols;
+        if (int rc = stage_ptrs(ctx, (const void* const*)blocks[b].cols, blocks[b].ncols, &cols)) return rc;
+        if (blocks[b].nidx) memcpy(pi + first_idx, blocks[b].idx, 4 * (size_t)blocks[b].nidx);
+        pb[b] = {(const uint32_t* const*)cols, (uint32_t)blocks[b].ncols, (uint32_t)first_idx, (uint32_t)blocks[b].out_off, 0u};
+        first_idx += (size_t)blocks[b].nidx;
+    }
+    // a plan too long for the staging ring brings its own memory
+    unsigned char *d_blob = nullptr, *d_own = nullptr;
+    uint32_t* d_out = nullptr;
+    cudaError_t e = cudaSuccess;
     int rc = ZKB_OK;
-    for (int b = 0; b < n_blocks && e == cudaSuccess && rc == ZKB_OK; b++) {
-        const GatherBlock& blk = blocks[b];
-        size_t total = (size_t)blk.ncols * blk.nidx;
-        if (total) {
-            void** d_cols;
-            rc = stage_ptrs(ctx, (const void* const*)blk.cols, blk.ncols, &d_cols);
-            if (rc == ZKB_OK) {
-                gather_multi_kernel<<<(unsigned)((total + 255) / 256), 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, blk.ncols,
-                                                                                              d_buf + ioff, blk.nidx, d_out + blk.out_off);
-                e = cudaGetLastError();
+    if (blob.size() <= sizeof(void*) * (ctx->ring_cap / 8)) {
+        rc = stage_blob(ctx, blob.data(), blob.size(), (void**)&d_blob);
+    } else {
+        rc = zkb_malloc(ctx, blob.size(), (void**)&d_own);
+        d_blob = d_own;
+        if (rc == ZKB_OK) e = cudaMemcpyAsync(d_blob, blob.data(), blob.size(), cudaMemcpyHostToDevice, ctx->stream);
+    }
+    if (rc == ZKB_OK) rc = zkb_malloc(ctx, results * 4, (void**)&d_out);
+    if (rc == ZKB_OK && e == cudaSuccess) {
+        const uint32_t* const* d_words = reinterpret_cast<const uint32_t* const*>(d_blob);
+        const uint32_t* const* d_hashes = reinterpret_cast<const uint32_t* const*>(d_blob + at_hash);
+        const PlanBlock* d_blocks = reinterpret_cast<const PlanBlock*>(d_blob + at_blocks);
+        const uint32_t* d_idx = reinterpret_cast<const uint32_t*>(d_blob + at_idx);
+        // Up to 2^20 cells one launch reads everything; beyond, a launch per block, whose threads need no bisection.
+        const bool one = total_words <= ((size_t)1 << 20);
+        if (!one) {
+            for (int b = 0; b < n_blocks; b++) {
+                const size_t cells = (size_t)blocks[b].ncols * blocks[b].nidx;
+                if (cells)
+                    gather_multi_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, ctx->stream>>>(pb[b].cols, blocks[b].ncols, d_idx + pb[b].idx, blocks[b].nidx,
+                                                                                                  d_out + blocks[b].out_off);
             }
         }
-        ioff += blk.nidx;
+        const uint32_t cells = one ? (uint32_t)total_words : 0u;
+        const size_t threads = cells + n_words + 8 * n_hashes;
+        if (threads)
+            gather_plan_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(d_blocks, n_blocks, d_idx, cells, d_words, (uint32_t)n_words, d_hashes,
+                                                                                           (uint32_t)n_hashes, d_out + (one ? 0 : total_words));
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, d_out, results * 4, cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     }
-    if (e == cudaSuccess && rc == ZKB_OK) e = cudaMemcpyAsync(h_out, d_out, total_words * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess && rc == ZKB_OK) e = cudaStreamSynchronize(ctx->stream);
-    cudaFreeAsync(d_buf, ctx->stream);
+    zkb_free(ctx, d_out);
+    zkb_free(ctx, d_own);
     if (rc != ZKB_OK) return rc;
-    if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gather_blocks: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gather_plan: %s", cudaGetErrorString(e));
     return ZKB_OK;
 }
 

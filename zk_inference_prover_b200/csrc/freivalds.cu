@@ -355,15 +355,11 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     cur = qm31_one();
     for (uint32_t p = 0; p < pk; p++) { pows.push_back(cur); cur = qm31_mul(cur, rv); }
     qm31 rv_step = cur;
-    // the powers go up through the pinned staging ring (two 8-byte slots each): no synchronisation with the work before
-    void **d_base, **d_pre, **d_out, **d_pw;
-    int rc = ZKB_OK;
-    if (ctx->ring_pos & 1) {  // the ring hands out 8-byte slots; the kernels read the powers as 16-byte words
-        const void* pad = nullptr;
-        if ((rc = stage_ptrs(ctx, &pad, 1, &d_pw))) return rc;
-    }
-    if ((rc = stage_ptrs(ctx, reinterpret_cast<const void* const*>(pows.data()), (int)(pows.size() * 2), &d_pw))) return rc;
-    if ((uintptr_t)d_pw & 15) return set_error(ctx, ZKB_ECUDA, "zkb_freivalds_acc: staging ring misaligned");
+    // the powers go up through the pinned staging ring: no synchronisation with the work before
+    void **d_base, **d_pre, **d_out;
+    void* d_pw;
+    int rc = stage_blob(ctx, pows.data(), pows.size() * sizeof(qm31), &d_pw);
+    if (rc) return rc;
     uint4* d_pows = reinterpret_cast<uint4*>(d_pw);
     rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)pq, &d_base);
     if (rc) return rc;

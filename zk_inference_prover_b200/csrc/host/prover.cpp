@@ -74,10 +74,11 @@ static std::vector<size_t> fold_queries(const std::vector<size_t>& q, uint32_t n
 // Every address a decommitment will read is known once the query positions are: collect them all,
 // read them in one device round trip, then assemble the proof parts from the results.
 struct GatherPlan {
-    std::vector<const uint32_t*> addrs;
-    std::vector<uint32_t> words;
+    std::vector<const uint32_t*> addrs;        // single words
+    std::vector<const uint32_t*> hash_addrs;   // eight words each
+    std::vector<uint32_t> words, hash_words;
     size_t add(const uint32_t* p) { addrs.push_back(p); return addrs.size() - 1; }
-    size_t add_hash(const uint32_t* p) { size_t s = addrs.size(); for (int k = 0; k < 8; k++) addrs.push_back(p + k); return s; }
+    size_t add_hash(const uint32_t* p) { hash_addrs.push_back(p); return hash_addrs.size() - 1; }
     // Rows of many columns at once (the queried and witness values of one tree layer): row-major [row][column] in
     // block_words from the returned offset. One pointer per column and one index per row travel, not one address per word.
     struct Block { std::vector<const uint32_t*> cols; std::vector<uint32_t> idx; size_t out_off; };
@@ -86,9 +87,8 @@ struct GatherPlan {
     // that size comes from mmap, and its first-touch page faults cost as much as the gather itself.
     uint32_t* block_words = nullptr;
     size_t block_total = 0;
-    // Page-locked once it is large (from 4 MiB): the device-to-host copy of a wide tree's values then runs at the link's
-    // speed instead of through the driver's bounce buffers (50 MB: 4 ms pageable). Small buffers stay ordinary memory:
-    // pinning costs more than it saves there.
+    // Page-locked: the device-to-host copy of a wide tree's values then runs at the link's speed instead of through the
+    // driver's bounce buffers (50 MB: 4 ms pageable), and a short one does not wait for them.
     struct Arena {
         uint32_t* p = nullptr;
         size_t words = 0;
@@ -104,9 +104,9 @@ struct GatherPlan {
         thread_local Arena a;
         if (a.words < words) {
             a.release();
-            size_t want = words + words / 4;
+            size_t want = std::max<size_t>(words + words / 4, (size_t)1 << 18);
             void* q = nullptr;
-            if (want * 4 >= ((size_t)4 << 20) && cudaMallocHost(&q, want * 4) == cudaSuccess && q) a.pinned = true;
+            if (cudaMallocHost(&q, want * 4) == cudaSuccess && q) a.pinned = true;
             else { (void)cudaGetLastError(); q = malloc(want * 4); a.pinned = false; }
             if (!q) throw Error(ZKB_ENOMEM, "gather buffer");
             a.p = (uint32_t*)q;
@@ -124,16 +124,17 @@ struct GatherPlan {
         return blocks.back().out_off;
     }
     void execute(const Device& d) {
-        words.resize(addrs.size());
-        d.check(zkb_gather_words(d.ctx(), addrs.data(), addrs.size(), words.data()));
-        if (block_total) {
-            block_words = arena(block_total);
-            std::vector<zk::GatherBlock> gb;
-            for (auto& b : blocks) gb.push_back({b.cols.data(), (int)b.cols.size(), b.idx.data(), (int)b.idx.size(), b.out_off});
-            d.check(zk::gather_blocks(d.ctx(), gb.data(), (int)gb.size(), block_total, block_words));
-        }
+        const size_t n = addrs.size(), nh = hash_addrs.size();
+        uint32_t* out = arena(block_total + n + 8 * nh);
+        std::vector<zk::GatherBlock> gb;
+        gb.reserve(blocks.size());
+        for (auto& b : blocks) gb.push_back({b.cols.data(), (int)b.cols.size(), b.idx.data(), (int)b.idx.size(), b.out_off});
+        d.check(zk::gather_plan(d.ctx(), gb.data(), (int)gb.size(), block_total, addrs.data(), n, hash_addrs.data(), nh, out));
+        block_words = out;
+        words.assign(out + block_total, out + block_total + n);
+        hash_words.assign(out + block_total + n, out + block_total + n + 8 * nh);
     }
-    Hash hash_at(size_t slot) const { Hash h; for (int k = 0; k < 8; k++) h[k] = words[slot + k]; return h; }
+    Hash hash_at(size_t slot) const { Hash h; for (int k = 0; k < 8; k++) h[k] = hash_words[8 * slot + k]; return h; }
 };
 
 // ------------------------------------------------------------------ MerkleProver (STWO/prover/vcs/prover.rs:17-217)
