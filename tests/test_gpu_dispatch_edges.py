@@ -1,0 +1,38 @@
+"""Proofs at the sizes where the library changes how it runs them, word for word against the oracle: FRI layers that fit the
+one-launch tail (2^10 values) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
+the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit."""
+import pytest
+
+from util import m31_column, qm31_array
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("log_n", [1, 2, 3, 8, 9, 10, 11])
+@pytest.mark.parametrize("kw", [
+    dict(pow_bits=4, log_blowup=1, log_last_layer=0, n_queries=3),
+    dict(pow_bits=0, log_blowup=2, log_last_layer=2, n_queries=5),
+    dict(pow_bits=6, log_blowup=1, log_last_layer=3, n_queries=2),
+    dict(pow_bits=1, log_blowup=4, log_last_layer=2, n_queries=4),
+])
+def test_pcs_proof_around_the_fri_tail(ctx, oracle, log_n, kw):
+    if log_n < kw["log_last_layer"] + 1:
+        pytest.skip("the last layer would be larger than the first fold")
+    trees = [[m31_column(6000 + 10 * log_n + c, 1 << log_n) for c in range(3)]]
+    want = oracle.pcs_prove(trees, **kw)
+    got = ctx.pcs_prove_host(trees, **kw)
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+@pytest.mark.parametrize("log_n", [1, 2, 3, 6, 7, 8, 9, 10, 12, 13, 14, 15])
+def test_gkr_single_instance_around_the_chain(ctx, oracle, kind, log_n):
+    if kind == 2 and log_n == 1:
+        pytest.skip("a multiplicities layer of two entries is not an input the protocol has")
+    n = 1 << log_n
+    den = qm31_array(7000 + log_n, n, nonzero=True)
+    num = qm31_array(7100 + log_n, n) if kind == 1 else m31_column(7200 + log_n, n) if kind == 2 else None
+    want = oracle.gkr_prove([(kind, num, den)], 0x5EED0004, verify=True)
+    nb, db = ctx.upload(num) if num is not None else None, ctx.upload(den)
+    got = ctx.gkr_prove_device([(kind, nb.ptr if nb else 0, db.ptr, n)], 0x5EED0004)
+    assert len(got) == len(want) and (got == want).all()

@@ -418,22 +418,30 @@ int zkb_grind(zkb_ctx* ctx, const uint32_t h_prefixed_digest[8], int pow_bits, i
     DeviceGuard g(ctx);
     const uint32_t* d = h_prefixed_digest;
     const unsigned LOW = 1u << 20;
+    if (pow_bits == 0) {  // every nonce passes
+        *h_nonce = 0;
+        return ZKB_OK;
+    }
+    // Half of the first 2^20 nonces already pass a few bits: a first launch over 2^(pow_bits + 4) of them finds the smallest in all
+    // but one case in nine million; the whole search follows otherwise.
+    unsigned first = pow_bits + 4 < 12 ? 1u << 12 : pow_bits + 4 < 20 ? 1u << (pow_bits + 4) : LOW;
     // Bounded search: hi values are tried in order; a miss over 2^20 nonces has probability
     // (1 - 2^-pow_bits)^(2^20), so the bound of 2^12 rounds is never reached for pow_bits <= 32
     // in practice and keeps the loop finite.
-    for (uint32_t hi = 0; hi < (1u << 12); hi++) {
-        unsigned int init = 0xffffffffu;
-        ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->ticket + 8, &init, 4, cudaMemcpyHostToDevice, ctx->stream));
-        grind_kernel<<<LOW / 256, 256, 0, ctx->stream>>>(d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], hi, pow_bits,
+    for (uint32_t hi = 0; hi < (1u << 12);) {
+        ZKB_CUDA(ctx, cudaMemsetAsync(ctx->ticket + 8, 0xff, 4, ctx->stream));
+        grind_kernel<<<first / 256, 256, 0, ctx->stream>>>(d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], hi, pow_bits,
                                                          m31_out, ctx->ticket + 8);
         ZKB_LAUNCH_CHECK(ctx);
-        unsigned int best = 0;
-        ZKB_CUDA(ctx, cudaMemcpyAsync(&best, ctx->ticket + 8, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, ctx->ticket + 8, 4, cudaMemcpyDeviceToHost, ctx->stream));
         ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        const unsigned int best = ctx->h_small[0];
         if (best != 0xffffffffu) {
             *h_nonce = ((uint64_t)hi << 32) | best;
             return ZKB_OK;
         }
+        if (first == LOW) hi++;
+        first = LOW;
     }
     return set_error(ctx, ZKB_ETIMEOUT, "zkb_grind: no nonce found in 2^32 attempts");
 }

@@ -43,6 +43,7 @@ struct zkb_ctx {
     // and a pinned landing buffer for the per-item results; both allocated on first use.
     unsigned int* batch_tickets = nullptr;
     uint32_t* h_batch = nullptr;
+    bool fri_tail_ready = false;   // fri_tail.cu: the same
     bool res_ready = false;        // gkr_resident.cu: its kernels' attributes are set on this device
     unsigned int batch_round = 0;  // sequence number of the last batched round launched
     cudaEvent_t events[64] = {nullptr};

@@ -1,0 +1,202 @@
+// The last layers of a FRI commitment (FriProver::commit, nitroo/crates/stwo/src/prover/fri.rs:109-221), from a layer of at most
+// 2^10 values down to the last one, in ONE launch of one CTA: per layer the leaf hashes, the tree, the channel step on its root
+// (mix, draw the folding challenge) and the fold.
+//
+// What bounds it: dependency depth. A layer of 2^l values is a chain of l + 1 tree levels and two channel compressions, each some
+// 0.9 us; at 2^10 values the leaves and the level above them are another 9 us of one SM's hashing. As launches (fold and leaves, tree
+// top with channel step) a layer also paid two launches, the gaps around them and a dozen allocations for its arrays: a ten-column
+// proof of 2^8 rows spent 190 us of device time in them and as much on the host. Layers stay in shared memory; what the decommitment
+// reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs.
+#include "channel.cuh"
+#include "common.cuh"
+#include "fri_tail.hpp"
+
+namespace zk {
+
+constexpr int TAIL_THREADS = 512;
+constexpr size_t TAIL_N = (size_t)1 << FRI_TAIL_LOG;
+
+__device__ __forceinline__ uint32_t bitrev_bits(uint32_t i, int bits) { return bits ? __brev(i) >> (32 - bits) : 0u; }
+
+// Dynamic shared memory: two layers of values and two of hashes, word by word ([word][node]: a node's two children then lie next to
+// each other in every word's row, two-way bank conflicts instead of sixteen).
+constexpr size_t TAIL_SMEM = (2 * 4 + 2 * 8) * TAIL_N * 4;
+
+__global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_constant__ FriTailArgs a, const uint32_t* __restrict__ itw) {
+    extern __shared__ uint32_t dyn[];
+    __shared__ ChanSm ch;
+    __shared__ uint32_t alpha_w[4];
+    uint32_t *ev = dyn, *ev_next = ev + 4 * TAIL_N, *const ha = ev_next + 4 * TAIL_N, *const hb = ha + 8 * TAIL_N;
+    const int tid = threadIdx.x, lane = tid & 31;
+    chan_make_schedule(ch, tid, TAIL_THREADS);
+    if (tid < 32) ch.msg[tid] = tid < 8 ? (a.chan ? a.chan[tid] : a.digest[tid]) : 0u;
+    if (tid == 0) ch.n_draws = a.chan ? a.chan[8] : a.n_draws;
+    for (int i = tid; i < 4 << a.first_log; i += TAIL_THREADS) {
+        const int c = i >> a.first_log, r = i & ((1 << a.first_log) - 1);
+        ev[c * TAIL_N + r] = a.src[c][r];
+    }
+    __syncthreads();
+    for (int k = 0; k < a.n_layers; k++) {
+        const int log = a.first_log - k;
+        uint32_t *cur = ha, *below = hb;
+        // leaves (level log) and nodes: one loop, so that the code of the hash is there once
+#pragma unroll 1
+        for (int lv = log; lv >= 0; lv--) {
+            uint32_t* const out = a.tree[k] + ((size_t)8 << lv);
+            const bool leaf = lv == log;
+            for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
+                uint32_t h[8], m[16];
+                blake2s_init(h);
+#pragma unroll
+                for (int w = 0; w < 16; w++)
+                    m[w] = leaf ? (w < 4 ? ev[w * TAIL_N + i] : 0u) : below[(w & 7) * TAIL_N + 2 * i + (w >> 3)];
+                blake2s_compress(h, m, leaf ? 16u : 64u, true);
+#pragma unroll
+                for (int w = 0; w < 8; w++) {
+                    h[w] = reduce_word_m31(h[w]);
+                    cur[w * TAIL_N + i] = h[w];
+                }
+                uint4* const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
+                o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+                o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            }
+            uint32_t* const t = cur;
+            cur = below;
+            below = t;
+            __syncthreads();
+        }
+        // the root is in below[.][0]: mix it in, draw the challenge
+        if (tid < 32) {
+            if (lane < 8) {
+                const uint32_t w = below[lane * TAIL_N];
+                ch.msg[8 + lane] = w;
+                a.out[FRI_TAIL_ROOTS + 8 * k + lane] = w;
+            }
+            chan_step(ch, 8, 1, alpha_w);
+        }
+        __syncthreads();
+        const qm31 alpha{{alpha_w[0], alpha_w[1], alpha_w[2], alpha_w[3]}};
+        const uint32_t half = 1u << (log - 1);
+        const size_t stride = log - 1 < 2 ? 4 : half;
+        for (uint32_t i = tid; i < half; i += TAIL_THREADS) {
+            uint32_t t, ix;
+            if (a.circle && k == 0) half_coset_point(itw, log, i, ix, t);
+            else t = itw[half + i];  // T_log^-1 starts at 2^(log - 1)
+            qm31 x, y;
+#pragma unroll
+            for (int c = 0; c < 4; c++) { x.c[c] = ev[c * TAIL_N + 2 * i]; y.c[c] = ev[c * TAIL_N + 2 * i + 1]; }
+            const qm31 r = qm31_add(qm31_add(x, y), qm31_mul(alpha, qm31_mul_m31(qm31_sub(x, y), t)));
+#pragma unroll
+            for (int c = 0; c < 4; c++) { ev_next[c * TAIL_N + i] = r.c[c]; a.evals[k][c * stride + i] = r.c[c]; }
+        }
+        uint32_t* const t = ev;
+        ev = ev_next;
+        ev_next = t;
+        __syncthreads();
+    }
+    if (tid >= 32) return;
+    uint32_t too_high = 0u;
+    if (a.last_bound >= 0) {
+        // commit_last_layer (fri.rs:193-221): interpolate on the line domain of last_log, value `lane` of the natural order per lane
+        const int log = a.last_log, lb = a.last_bound;
+        const uint32_t n = 1u << log, pos = bitrev_bits((uint32_t)lane & (n - 1), log);
+        qm31 v;
+#pragma unroll
+        for (int c = 0; c < 4; c++) v.c[c] = ev[c * TAIL_N + pos];
+        for (int k = log; k > 0; k--) {
+            const uint32_t half = 1u << (k - 1), p = (uint32_t)lane & (2 * half - 1);
+            const bool low = p < half;
+            qm31 o;
+#pragma unroll
+            for (int c = 0; c < 4; c++) o.c[c] = __shfl_xor_sync(0xffffffffu, v.c[c], half);
+            const uint32_t xinv = itw[half + bitrev_bits(p & (half - 1), k - 1)];
+            v = low ? qm31_add(v, o) : qm31_mul_m31(qm31_sub(o, v), xinv);
+        }
+        v = qm31_mul_m31(v, m31_inv(n));
+        // lane l holds the coefficient at bitrev(l) of the bit-reversed order, of which only the first 2^lb may be non-zero
+        const uint32_t j = pos;
+        too_high = __any_sync(0xffffffffu, (uint32_t)lane < n && j >= (1u << lb) && !qm31_is_zero(v)) ? 1u : 0u;
+        const uint32_t slot = bitrev_bits(j & ((1u << lb) - 1), lb);
+        if ((uint32_t)lane < n && j < (1u << lb)) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                ch.msg[8 + 4 * slot + c] = v.c[c];
+                a.out[32 + 4 * slot + c] = v.c[c];
+            }
+        }
+        chan_step(ch, 4 << lb, 0, alpha_w);
+        // the digest a proof of work is searched for: H(prefix, 12 zero bytes, digest, pow_bits), channel/blake2s.rs:124-133
+        const uint32_t d = lane < 8 ? ch.msg[lane] : 0u;
+        const uint32_t shifted = __shfl_sync(0xffffffffu, d, (lane - 4) & 31);
+        uint32_t* const block = ch.msg + 16;
+        if (lane < 16) block[lane] = lane == 0 ? 0x12345678u : lane < 4 ? 0u : lane < 12 ? shifted : lane == 12 ? a.pow_bits : 0u;
+        __syncwarp();
+        const QuadConst q;
+        const uint2 h = b2s_compress_quad(make_uint2(q.h0, q.h1), block, ch.sched, q, 52u, 0xffffffffu);
+        if (lane < 4) { a.out[16 + lane] = reduce_word_m31(h.x); a.out[20 + lane] = reduce_word_m31(h.y); }
+    }
+    if (lane < 8) a.out[lane] = ch.msg[lane];
+    if (lane == 8) a.out[8] = ch.n_draws;
+    if (lane == 9) a.out[9] = too_high;
+    if (lane == 10) a.out[10] = 0xffffffffu;
+}
+
+__global__ void __launch_bounds__(256) grind_first_kernel(const uint32_t* __restrict__ prefixed, int pow_bits, unsigned int* __restrict__ best) {
+    const uint32_t lo = blockIdx.x * 256u + threadIdx.x;
+    uint32_t h[8], m[16];
+#pragma unroll
+    for (int w = 0; w < 16; w++) m[w] = w < 8 ? prefixed[w] : 0u;
+    m[8] = lo;
+    blake2s_init(h);
+    blake2s_compress(h, m, 40u, true);
+    const uint32_t w = reduce_word_m31(h[0]);
+    const int tz = w ? __ffs(w) - 1 : 32;
+    if (tz >= pow_bits) atomicMin(best, lo);
+}
+
+int fri_tail(zkb_ctx* ctx, const FriTailArgs& args) {
+    ZKB_CHECK_ARG(ctx, args.n_layers >= 1 && args.first_log <= FRI_TAIL_LOG && args.first_log - args.n_layers >= 0);
+    ZKB_CHECK_ARG(ctx, args.first_log <= ctx->max_log - (args.circle ? 0 : 1));
+    ZKB_CHECK_ARG(ctx, !args.circle || args.first_log >= 3);
+    ZKB_CHECK_ARG(ctx, args.last_bound < 0 || (args.last_log == args.first_log - args.n_layers && args.last_log <= FRI_TAIL_MAX_LAST &&
+                                              args.last_bound <= FRI_TAIL_MAX_BOUND && args.last_bound <= args.last_log));
+    DeviceGuard g(ctx);
+    if (!ctx->fri_tail_ready) {
+        ZKB_CUDA(ctx, cudaFuncSetAttribute(fri_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM));
+        ctx->fri_tail_ready = true;
+    }
+    ProfScope prof(ctx, "fri_tail_kernel");
+    fri_tail_kernel<<<1, TAIL_THREADS, TAIL_SMEM, ctx->stream>>>(args, ctx->itw);
+    ZKB_LAUNCH_CHECK(ctx);
+    return ZKB_OK;
+}
+
+int grind_first(zkb_ctx* ctx, const uint32_t* prefixed, int pow_bits, uint32_t* best) {
+    // 2^(pow_bits + 4) nonces all fail with probability e^-16; zkb_grind then searches from the start
+    const int log = pow_bits + 4 < 12 ? 12 : pow_bits + 4 > 20 ? 20 : pow_bits + 4;
+    DeviceGuard g(ctx);
+    ProfScope prof(ctx, "grind_kernel");
+    grind_first_kernel<<<1u << (log - 8), 256, 0, ctx->stream>>>(prefixed, pow_bits, best);
+    ZKB_LAUNCH_CHECK(ctx);
+    return ZKB_OK;
+}
+
+// (the ring's slots are 8 bytes; the copy is ordered on the stream like every use of dst)
+int upload_small(zkb_ctx* ctx, uint32_t* dst, const uint32_t* h, size_t words) {
+    DeviceGuard g(ctx);
+    void* staged = nullptr;
+    if (int rc = stage_blob(ctx, h, words * 4, &staged)) return rc;
+    ZKB_CUDA(ctx, cudaMemcpyAsync(dst, staged, words * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    return ZKB_OK;
+}
+
+int read_small(zkb_ctx* ctx, const uint32_t* d, size_t words, const uint32_t** h) {
+    ZKB_CHECK_ARG(ctx, words <= (size_t)SMALL_WORDS);
+    DeviceGuard g(ctx);
+    ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, d, words * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *h = ctx->h_small;
+    return ZKB_OK;
+}
+
+}  // namespace zk

@@ -1,0 +1,44 @@
+// The last layers of a FRI commitment in one launch (fri_tail.cu); internal to the library.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+
+struct zkb_ctx;
+
+namespace zk {
+
+constexpr int FRI_TAIL_LOG = 10;         // largest layer (log2) the launch takes
+constexpr int FRI_TAIL_MAX_LAST = 5;     // largest last layer (log2) it interpolates
+constexpr int FRI_TAIL_MAX_BOUND = 2;    // largest log2 of the last layer's coefficients it mixes into the channel
+
+struct FriTailArgs {
+    const uint32_t* src[4];              // the first layer's coordinate columns
+    int first_log, n_layers;             // its size; committed layers (each half the one before), at least one
+    int circle;                          // the first layer lies on the circle domain (first_log >= 3); line domains otherwise
+    // Layer k's tree: level j (2^j hashes) at tree[k] + 8 * 2^j. Folded layer k (what layer k becomes): coordinate c at
+    // evals[k] + c * fri_tail_stride(log).
+    uint32_t* tree[FRI_TAIL_LOG + 1];
+    uint32_t* evals[FRI_TAIL_LOG + 1];
+    const uint32_t* chan;                // channel state on the device (digest, n_draws), or NULL: the one below
+    uint32_t digest[8], n_draws;
+    uint32_t* out;                       // fri_tail_out_words(n_layers) words, see below
+    // last_bound >= 0: also interpolate the last layer (2^last_log values), mix its 2^last_bound coefficients into the channel and
+    // leave the digest a proof of work of pow_bits is searched for, with the search's result slot set to "none found".
+    int last_log, last_bound;
+    uint32_t pow_bits;
+};
+// out: [0,8) digest, [8] draws, [9] not zero if the last layer has a higher degree, [10] smallest nonce found (all ones: none),
+// [16,24) the digest to search with, [32, 32 + 16) the last layer's coefficients, then a root per layer.
+constexpr size_t FRI_TAIL_ROOTS = 48;
+inline size_t fri_tail_out_words(int n_layers) { return FRI_TAIL_ROOTS + 8 * (size_t)n_layers; }
+inline size_t fri_tail_stride(int log) { return log < 2 ? 4 : (size_t)1 << log; }
+
+int fri_tail(zkb_ctx* ctx, const FriTailArgs& args);
+// The first nonces (several times 2^pow_bits of them) tested against the digest at prefixed; the smallest that passes goes to *best.
+int grind_first(zkb_ctx* ctx, const uint32_t* prefixed, int pow_bits, uint32_t* best);
+// A few words to device memory through the staging ring: no synchronisation.
+int upload_small(zkb_ctx* ctx, uint32_t* dst, const uint32_t* h, size_t words);
+// `words` of device memory to the context's page-locked buffer and a synchronisation; *h is valid until the next such read.
+int read_small(zkb_ctx* ctx, const uint32_t* d, size_t words, const uint32_t** h);
+
+}  // namespace zk

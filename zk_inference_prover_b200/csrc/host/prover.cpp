@@ -23,6 +23,7 @@
 #include "../fft_internal.hpp"
 #include "../gkr_resident.hpp"
 #include "../gkr_batch.hpp"
+#include "../fri_tail.hpp"
 #include "../gather_blocks.hpp"
 #include "channel.hpp"
 
@@ -387,57 +388,142 @@ struct FriProver {
     MerkleProver first_tree;
     struct Inner { SecureColumnByCoords eval; MerkleProver tree; uint32_t fold_step; };
     std::vector<Inner> inner;
+    BaseColumn tail_slab;  // trees and layers of the launch that runs the last layers, which `inner` holds views of
     std::vector<qm31> last_layer_poly;
 
-    // fri.rs:109-221
-    static FriProver commit(const Device& d, Channel& ch, FriConfig config, const SecureColumnByCoords& column) {
+    bool have_nonce = false;  // the proof of work was searched for along with the commitment (grind_bits)
+    uint64_t nonce = 0;
+
+    // A tree in memory laid out as the tail's launch writes it (FriTailArgs::tree).
+    static MerkleProver tree_view(const Device& d, uint32_t* tree, uint32_t log, const SecureColumnByCoords& eval) {
+        MerkleProver mp;
+        for (uint32_t j = 0; j <= log; j++) mp.layers.push_back(HashColumn::view(d, tree + ((size_t)8 << j), (size_t)8 << j));
+        mp.layer_col_ptrs.resize(log + 1);
+        for (auto p : eval.cptrs()) mp.layer_col_ptrs[log].push_back(p);
+        mp.n_columns = 4;
+        return mp;
+    }
+
+    // fri.rs:109-221. grind_bits >= 0: the proof of work of that many bits follows the commitment in the transcript, and its first
+    // nonces may be tested in the same round trip (have_nonce says whether one was found).
+    static FriProver commit(const Device& d, Channel& ch, FriConfig config, const SecureColumnByCoords& column, int grind_bits = -1) {
         FriProver fp;
         fp.config = config;
         fp.first_column = &column;
         uint32_t first_log = column.columns[0].log_size(), inner_log = first_log - 1;
         uint32_t last_log = ilog2(config.last_layer_domain_size());
-        SecureColumnByCoords layer(d, (size_t)1 << inner_log, true);
+        SecureColumnByCoords layer;
+        bool last_done = false;
         if (config.line_fold_step == 1) {
             // Device-resident commit phase: every layer's tree, the channel step (mix the root, draw the
             // folding challenge) and the fold are enqueued back to back; the host reads all roots and the
-            // channel state once, after the last fold.
-            size_t n_layers = 1 + (inner_log > last_log ? inner_log - last_log : 0);
-            BaseColumn fs(d, 16 + 12 * n_layers);  // [channel 16 | challenges 4 each (16-byte aligned) | roots 8 each]
+            // channel state once, after the last fold. Layers of at most 2^FRI_TAIL_LOG values run in one launch.
+            const size_t n_layers = 1 + (inner_log > last_log ? inner_log - last_log : 0);
+            const size_t tail = first_log > (uint32_t)zk::FRI_TAIL_LOG ? std::min<size_t>(n_layers, first_log - zk::FRI_TAIL_LOG)
+                                : first_log >= 3 && inner_log >= last_log ? 0 : n_layers;  // the first layer of that launch
+            const bool last_in_tail = tail < n_layers && last_log <= (uint32_t)zk::FRI_TAIL_MAX_LAST &&
+                                      config.log_last_layer_degree_bound <= (uint32_t)zk::FRI_TAIL_MAX_BOUND;
+            // [channel 16 | challenges 4 each (16-byte aligned) | roots 8 each | the tail's results]
+            const size_t tail_at = 16 + 12 * tail, tail_layers = n_layers - tail;
+            BaseColumn fs(d, tail_at + zk::fri_tail_out_words((int)tail_layers));
             uint32_t* chan = fs.ptr();
             uint32_t* alphas = fs.ptr() + 16;
-            uint32_t* roots = fs.ptr() + 16 + 4 * n_layers;
-            uint32_t st[16] = {0};
-            for (int k = 0; k < 8; k++) st[k] = ch.digest()[k];
-            st[8] = ch.n_draws();
-            d.check(zkb_h2d(d.ctx(), chan, st, sizeof(st)));
-            bool stepped = false;
-            MerkleProver::ChanStep step0{chan, alphas, roots};
-            fp.first_tree = MerkleProver::commit(d, column.refs(), nullptr, &step0, &stepped);
-            if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, fp.first_tree.layers[0].ptr(), alphas, roots));
-            // every fold but the last also hashes the leaves of the layer it produces: that layer is committed next
-            HashColumn leaves;
-            bool have_leaves = n_layers > 1 && first_log >= 3;
-            B200Backend::fold_circle_into_line(d, layer, column, alphas, have_leaves ? &leaves : nullptr);
-            for (size_t k = 1; k < n_layers; k++) {
-                Inner in{std::move(layer), {}, 1};
-                std::vector<const BaseColumn*> refs = in.eval.refs();
-                MerkleProver::ChanStep step{chan, alphas + 4 * k, roots + 8 * k};
-                in.tree = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr, &step, &stepped);
-                if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, in.tree.layers[0].ptr(), alphas + 4 * k, roots + 8 * k));
-                have_leaves = k + 1 < n_layers;
-                if (have_leaves) layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k, leaves);
-                else layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k);
-                fp.inner.push_back(std::move(in));
+            uint32_t* roots = fs.ptr() + 16 + 4 * tail;
+            if (tail > 0) {
+                uint32_t st[16] = {0};
+                for (int k = 0; k < 8; k++) st[k] = ch.digest()[k];
+                st[8] = ch.n_draws();
+                d.check(zk::upload_small(d.ctx(), chan, st, 16));
+                layer = SecureColumnByCoords(d, (size_t)1 << inner_log, true);
+                bool stepped = false;
+                MerkleProver::ChanStep step0{chan, alphas, roots};
+                fp.first_tree = MerkleProver::commit(d, column.refs(), nullptr, &step0, &stepped);
+                if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, fp.first_tree.layers[0].ptr(), alphas, roots));
+                // every fold but the last also hashes the leaves of the layer it produces: that layer is committed next
+                HashColumn leaves;
+                bool have_leaves = tail > 1 && first_log >= 3;
+                B200Backend::fold_circle_into_line(d, layer, column, alphas, have_leaves ? &leaves : nullptr);
+                for (size_t k = 1; k < tail; k++) {
+                    Inner in{std::move(layer), {}, 1};
+                    std::vector<const BaseColumn*> refs = in.eval.refs();
+                    MerkleProver::ChanStep step{chan, alphas + 4 * k, roots + 8 * k};
+                    in.tree = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr, &step, &stepped);
+                    if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, in.tree.layers[0].ptr(), alphas + 4 * k, roots + 8 * k));
+                    have_leaves = k + 1 < tail;
+                    if (have_leaves) layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k, leaves);
+                    else layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k);
+                    fp.inner.push_back(std::move(in));
+                }
             }
-            std::vector<uint32_t> h = fs.to_cpu();  // one copy, one synchronisation
+            if (tail_layers > 0) {
+                zk::FriTailArgs ta;
+                memset(&ta, 0, sizeof(ta));
+                const uint32_t log0 = first_log - (uint32_t)tail;
+                size_t words = 0;
+                for (uint32_t k = 0; k < tail_layers; k++) words += ((size_t)16 << (log0 - k)) + 4 * zk::fri_tail_stride((int)(log0 - k) - 1);
+                fp.tail_slab = BaseColumn(d, words);
+                uint32_t* at = fp.tail_slab.ptr();
+                for (uint32_t k = 0; k < tail_layers; k++) {
+                    ta.tree[k] = at; at += (size_t)16 << (log0 - k);
+                    ta.evals[k] = at; at += 4 * zk::fri_tail_stride((int)(log0 - k) - 1);
+                }
+                const auto src = tail ? layer.cptrs() : column.cptrs();
+                for (int c = 0; c < 4; c++) ta.src[c] = src[c];
+                ta.first_log = (int)log0;
+                ta.n_layers = (int)tail_layers;
+                ta.circle = tail == 0;
+                if (tail) ta.chan = chan;
+                for (int k = 0; k < 8; k++) ta.digest[k] = ch.digest()[k];
+                ta.n_draws = ch.n_draws();
+                ta.out = fs.ptr() + tail_at;
+                ta.last_log = (int)last_log;
+                ta.last_bound = last_in_tail ? (int)config.log_last_layer_degree_bound : -1;
+                ta.pow_bits = grind_bits > 0 ? (uint32_t)grind_bits : 0u;
+                d.check(zk::fri_tail(d.ctx(), ta));
+                if (last_in_tail && grind_bits > 0) d.check(zk::grind_first(d.ctx(), ta.out + 16, grind_bits, ta.out + 10));
+                for (uint32_t k = 0; k < tail_layers; k++) {
+                    const uint32_t log = log0 - k;
+                    if (k > 0) {
+                        layer = SecureColumnByCoords();
+                        for (int c = 0; c < 4; c++)
+                            layer.columns[c] = BaseColumn::view(d, ta.evals[k - 1] + c * zk::fri_tail_stride((int)log), (size_t)1 << log);
+                    }
+                    if (tail + k == 0) fp.first_tree = tree_view(d, ta.tree[0], log, column);
+                    else {
+                        Inner in{std::move(layer), {}, 1};
+                        in.tree = tree_view(d, ta.tree[k], log, in.eval);
+                        fp.inner.push_back(std::move(in));
+                    }
+                }
+                layer = SecureColumnByCoords();
+                for (int c = 0; c < 4; c++)
+                    layer.columns[c] = BaseColumn::view(d, ta.evals[tail_layers - 1] + c * zk::fri_tail_stride((int)last_log), (size_t)1 << last_log);
+            }
+            const uint32_t* h = nullptr;  // one copy, one synchronisation
+            d.check(zk::read_small(d.ctx(), fs.ptr(), fs.len(), &h));
+            const uint32_t* const state = tail_layers ? h + tail_at : h;
             HashWords dg;
-            for (int k = 0; k < 8; k++) dg[k] = h[k];
-            ch.set_state(dg, h[8]);
-            auto root_at = [&](size_t k) { Hash r; for (int w = 0; w < 8; w++) r[w] = h[16 + 4 * n_layers + 8 * k + w]; return r; };
+            for (int k = 0; k < 8; k++) dg[k] = state[k];
+            ch.set_state(dg, state[8]);
+            auto root_at = [&](size_t k) {
+                const uint32_t* w = k < tail ? h + 16 + 4 * tail + 8 * k : h + tail_at + zk::FRI_TAIL_ROOTS + 8 * (k - tail);
+                Hash r;
+                for (int i = 0; i < 8; i++) r[i] = w[i];
+                return r;
+            };
             fp.first_tree.root_cache = root_at(0);
             fp.first_tree.have_root = true;
             for (size_t k = 1; k < n_layers; k++) { fp.inner[k - 1].tree.root_cache = root_at(k); fp.inner[k - 1].tree.have_root = true; }
+            if (last_in_tail) {
+                if (state[9]) throw Error(ZKB_EINVAL, "FRI: invalid degree");
+                for (size_t i = 0; i < (size_t)1 << config.log_last_layer_degree_bound; i++)
+                    fp.last_layer_poly.push_back(qm31{{state[32 + 4 * i], state[33 + 4 * i], state[34 + 4 * i], state[35 + 4 * i]}});
+                fp.have_nonce = grind_bits == 0 || (grind_bits > 0 && state[10] != 0xffffffffu);
+                fp.nonce = grind_bits > 0 ? state[10] : 0;
+                last_done = true;
+            }
         } else {
+            layer = SecureColumnByCoords(d, (size_t)1 << inner_log, true);
             fp.first_tree = MerkleProver::commit(d, column.refs());
             ch.mix_root(fp.first_tree.root(d));
             qm31 alpha = ch.draw_secure_felt();
@@ -461,6 +547,7 @@ struct FriProver {
                 }
             }
         }
+        if (last_done) return fp;
         // commit_last_layer, fri.rs:193-221
         if (layer.len() != config.last_layer_domain_size()) throw Error(ZKB_EINVAL, "FRI: unexpected last layer size");
         std::vector<size_t> all(layer.len());
@@ -898,9 +985,9 @@ struct CommitmentSchemeProver {
         SecureColumnByCoords quotients = compute_fri_quotients(samples, random_coeff, lifting_log);
         hc.reset();
         mark(4);
-        FriProver fri = FriProver::commit(d, ch, config.fri, quotients);
+        FriProver fri = FriProver::commit(d, ch, config.fri, quotients, (int)config.pow_bits);
         mark(5);
-        proof.proof_of_work = B200Backend::grind(d, ch.pow_prefixed_digest(config.pow_bits), config.pow_bits);
+        proof.proof_of_work = fri.have_nonce ? fri.nonce : B200Backend::grind(d, ch.pow_prefixed_digest(config.pow_bits), config.pow_bits);
         ch.mix_u64(proof.proof_of_work);
         mark(6);
         hc.reset(new HostClock("pcs.decommit.plan"));
