@@ -61,15 +61,16 @@ struct GkrLayerRound {
     int n_fix;
 };
 
-constexpr int GKR_LAYER_MAX_ROUNDS = 60;
+constexpr int GKR_LAYER_MAX_ROUNDS = 31;
+constexpr size_t GKR_LAYER_MASK_WORDS = 16;  // per oracle: the two fixed denominators, the two fixed numerators
 constexpr size_t GKR_LAYER_OUT_WORDS = 24;  // per round: [0,16) coefficients, [16] length, [20,24) challenge
 
 // n_vars[k]: variables of oracle k's sum-check (it is active in the rounds with n_rem <= n_vars[k]); alpha_pow[k] = alpha^k;
 // claims[k]: its claim before the first round (4 words each). chan: digest (8 words) and n_draws, in and out.
-// h_out: n_rounds x GKR_LAYER_OUT_WORDS; h_res: n_oracles x GKR_BATCH_RESULT_WORDS (the last sums and, for every oracle that
-// had a round, its mask).
+// h_out: n_rounds x GKR_LAYER_OUT_WORDS; h_masks: n_oracles x GKR_LAYER_MASK_WORDS (of every oracle that had a round). degenerate:
+// a round polynomial's leading coefficient vanished; the results do not follow the transcript then and must be thrown away.
 int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const uint32_t* alpha_pow, const uint32_t* claims,
                     GkrLayerRound* rounds, int n_rounds, const uint32_t* eq_evals, const uint32_t h_lambda[4], uint32_t chan[9],
-                    uint32_t* h_out, uint32_t* h_res);
+                    uint32_t* h_out, uint32_t* h_masks, bool* degenerate);
 
 }  // namespace zk

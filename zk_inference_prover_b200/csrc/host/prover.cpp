@@ -1152,8 +1152,9 @@ static Layer layer_view(const Device& d, int kind, const uint32_t* num, const ui
     return l;
 }
 
-// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream.
-static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::vector<Layer> input_layers) {
+// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream. host_rounds: the transcript of the rounds stays on
+// the host; otherwise *degenerate may be set, and the caller proves again that way (see gkr_batch.hpp).
+static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::vector<Layer> input_layers, bool host_rounds_only, bool* degenerate) {
     size_t n_inst = input_layers.size();
     std::vector<size_t> n_layers_by_inst;
     for (auto& l : input_layers) n_layers_by_inst.push_back(l.n_variables());
@@ -1269,14 +1270,14 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::
         // device (gkr_batch_layer); ZKB_GKR_ROUNDS=host keeps the channel on the host and returns to it every round, and
         // ZKB_GKR_ROUNDS=launches keeps a launch per round also for the small rounds (both for comparison and tests).
         const char* rounds_env = getenv("ZKB_GKR_ROUNDS");
-        bool host_rounds = rounds_env && !strcmp(rounds_env, "host");
+        bool host_rounds = host_rounds_only || (rounds_env && !strcmp(rounds_env, "host"));
         {
             // The layer's description is staged as one block (an item per oracle and active round, 64 bytes each, and some
-            // 52 bytes per oracle): a batch of thousands of tall instances would not fit the staging ring (2 MiB) and takes
+            // 52 bytes per oracle): a batch of thousands of tall instances would not fit the staging ring and takes
             // the round-by-round path, which stages one round's items at a time.
             size_t items = 0;
             for (auto& o : oracles) items += o.n_variables() + 1;
-            if (64 * items + 64 * oracles.size() + 256 * nv + 4096 > ((size_t)1 << 20)) host_rounds = true;
+            if (64 * items + 64 * oracles.size() + 256 * nv + 8192 > ((size_t)2 << 20) || nv > (size_t)zk::GKR_LAYER_MAX_ROUNDS) host_rounds = true;
         }
         if (nv > 0 && !host_rounds) {
             std::unique_ptr<HostClock> hc(new HostClock("gkr.layer.plan"));
@@ -1347,10 +1348,11 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::
             uint32_t chan[9];
             memcpy(chan, ch.digest().data(), 32);
             chan[8] = ch.n_draws();
-            std::vector<uint32_t> out_words(zk::GKR_LAYER_OUT_WORDS * nv), res(zk::GKR_BATCH_RESULT_WORDS * K);
+            std::vector<uint32_t> out_words(zk::GKR_LAYER_OUT_WORDS * nv), res(zk::GKR_LAYER_MASK_WORDS * K);
             d.check(zk::gkr_batch_layer(d.ctx(), (int)K, n_vars.data(), alpha_pow[0].c, sc_claims[0].c, plan.data(), (int)nv, eq_evals.words.ptr(),
-                                        lambda.c, chan, out_words.data(), res.data()));
+                                        lambda.c, chan, out_words.data(), res.data(), degenerate));
             retired.clear();
+            if (*degenerate) return {};
             HashWords digest;
             memcpy(digest.data(), chan, 32);
             ch.set_state(digest, chan[8]);
@@ -1364,10 +1366,10 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::
             for (size_t k = 0; k < K; k++) {
                 if (n_vars[k] == 0) continue;  // no round, no mask from a launch: read with the others below
                 GkrOracle& o = oracles[k];
-                const uint32_t* w = res.data() + zk::GKR_BATCH_RESULT_WORDS * k;
+                const uint32_t* w = res.data() + zk::GKR_LAYER_MASK_WORDS * k;
                 for (int e = 0; e < 2; e++) {
-                    o.mask_den[e] = qm31{{w[8 + 4 * e], w[9 + 4 * e], w[10 + 4 * e], w[11 + 4 * e]}};
-                    o.mask_num[e] = qm31{{w[16 + 4 * e], w[17 + 4 * e], w[18 + 4 * e], w[19 + 4 * e]}};
+                    o.mask_den[e] = qm31{{w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]}};
+                    o.mask_num[e] = qm31{{w[8 + 4 * e], w[9 + 4 * e], w[10 + 4 * e], w[11 + 4 * e]}};
                 }
                 o.have_mask = true;
             }
@@ -2293,18 +2295,21 @@ int zkb_gkr_prove_device(zkb_ctx* ctx, int n_inst, const int* kinds, const uint3
     if (n_inst <= 0 || !kinds || !d_nums || !d_dens || !ns || !h_out || !n_words) return ZKB_EINVAL;
     try {
         Device dev(ctx);
-        std::vector<Layer> layers;
-        for (int i = 0; i < n_inst; i++) {
+        for (int i = 0; i < n_inst; i++)
             if (kinds[i] < 0 || kinds[i] > 3 || ns[i] < 1 || (ns[i] & (ns[i] - 1))) return ZKB_EINVAL;
-            layers.push_back(layer_view(dev, kinds[i], d_nums[i], d_dens[i], ns[i]));
-        }
+        auto layers = [&] {
+            std::vector<Layer> v;
+            for (int i = 0; i < n_inst; i++) v.push_back(layer_view(dev, kinds[i], d_nums[i], d_dens[i], ns[i]));
+            return v;
+        };
         Channel ch;
         ch.mix_u64(seed);
         std::vector<uint32_t> w;
-        // Two drivers give the same proof. With the transcript on the device a round costs no host round trip but runs its
-        // Fiat-Shamir step on one warp, which pays for ONE large instance; a batch of several instances is cheaper with one
-        // launch and one read-back per round for all of them. ZKB_GKR_DRIVER=resident|batch overrides the choice.
-        bool resident = gkr_resident_supported(n_inst, ns) && n_inst <= 2;
+        // Two drivers give the same proof. With everything on the device a layer costs no host round trip, but its masks and claims are
+        // hashed there, some 2.3 us an instance, and an instance's passes are launches of their own: measured against the batch driver
+        // (one launch a round for all instances, masks hashed on the host), 0.45-0.75 of its time for two to four instances of 2^8 to
+        // 2^16 entries, equal at six, twice at sixteen. ZKB_GKR_DRIVER=resident|batch overrides the choice.
+        bool resident = gkr_resident_supported(n_inst, ns) && n_inst <= 4;
         if (const char* pick = getenv("ZKB_GKR_DRIVER")) {
             if (!strcmp(pick, "resident")) resident = gkr_resident_supported(n_inst, ns);
             else if (!strcmp(pick, "batch")) resident = false;
@@ -2313,13 +2318,19 @@ int zkb_gkr_prove_device(zkb_ctx* ctx, int n_inst, const int* kinds, const uint3
             // the transcript stays on the device: no host round trip per sum-check round
             uint32_t dg[8], nd = ch.n_draws();
             for (int k = 0; k < 8; k++) dg[k] = ch.digest()[k];
-            int rc = gkr_prove_resident(ctx, std::move(layers), dg, &nd, w);
+            int rc = gkr_prove_resident(ctx, layers(), dg, &nd, w);
             if (rc) return rc;
             HashWords hw;
             for (int k = 0; k < 8; k++) hw[k] = dg[k];
             ch.set_state(hw, nd);
         } else {
-            w = gkr_prove_batch(dev, ch, std::move(layers));
+            bool degenerate = false;
+            const Channel before = ch;
+            w = gkr_prove_batch(dev, ch, layers(), false, &degenerate);
+            if (degenerate) {
+                ch = before;
+                w = gkr_prove_batch(dev, ch, layers(), true, &degenerate);
+            }
         }
         w.insert(w.end(), ch.digest().begin(), ch.digest().end());
         *n_words = w.size();
