@@ -14,10 +14,10 @@
 //   mode 0  sum_as_poly_in_first_variable sums of the item's layer (first round of a layer's sum-check)
 //   mode 1  fix_first_variable with the round's challenge on every column, and the sums of the fixed layer
 //   mode 2  fix_first_variable of a 4-entry layer; the 2 fixed entries are also copied to the results (the mask)
-//   mode 3  next_layer (generation of the towers)
 //
 // Arithmetic as in gkr.cu / gkr_fused.cu (cpu/lookups/gkr.rs:17-263, cpu/lookups/mle.rs:13-46).
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
@@ -26,6 +26,7 @@
 #include "channel.cuh"
 #include "common.cuh"
 #include "gkr_batch.hpp"
+#include "gkr_tower.cuh"
 
 namespace zk {
 
@@ -222,13 +223,23 @@ __device__ __forceinline__ void batch_step_open(GkrStepSm& sm, const GkrStepStat
     if (lane == 0) sm.ch.n_draws = st.n_draws;
     __syncwarp();
 }
-// The channel's state to where the next launch and, at the end, the host find it.
-__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, GkrStepState* st, uint32_t degenerate, uint32_t* final_words, int lane) {
+// The channel's state to where the next launch finds it.
+__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, GkrStepState* st, uint32_t degenerate, int lane) {
     const uint32_t w = lane < 8 ? sm.ch.msg[lane] : lane == 8 ? sm.ch.n_draws : lane == 9 ? degenerate : 0u;
-    if (lane < 12) {
-        reinterpret_cast<uint32_t*>(st)[lane] = w;
-        final_words[lane] = w;
-    }
+    if (lane < 12) reinterpret_cast<uint32_t*>(st)[lane] = w;
+}
+
+// What a layer brings back is written by its last launch into page-locked host memory (the masks by the threads that fix them; the
+// rounds' records and the channel, which the launches before keep on the device, by `threads` threads at the end), then the layer's
+// number: the host has it a PCIe write after the last round, without a copy and a stream synchronisation of its own.
+struct GkrLayerOut {
+    uint32_t *records, *channel, *masks;  // host
+    volatile unsigned int* flag;
+    unsigned int id;
+};
+__device__ __forceinline__ void layer_out_words(const GkrLayerOut& o, const uint32_t* records, int n_rounds, const GkrStepState* st, int i, int threads) {
+    for (int k = i; k < 6 * n_rounds; k += threads) reinterpret_cast<uint4*>(o.records)[k] = __ldcg(reinterpret_cast<const uint4*>(records) + k);
+    if (i < 3) reinterpret_cast<uint4*>(o.channel)[i] = __ldcg(reinterpret_cast<const uint4*>(st) + i);
 }
 __device__ __forceinline__ qm31 acc_value(const unsigned long long* a) { return {{m31_reduce64(a[0]), m31_reduce64(a[1]), m31_reduce64(a[2]), m31_reduce64(a[3])}}; }
 
@@ -253,11 +264,10 @@ __device__ __forceinline__ void item_sums_of(const GkrBatchItem& it, size_t firs
 }
 
 // One launch of a layer enqueued at once: the items' passes, each CTA's sums to its group's accumulator; the CTA that finishes last
-// goes on with the transcript step of round `step` (-1: none, the masks). parity: which half of the accumulators this round uses.
+// goes on with the transcript step of round `step` (-1: none, the masks and the way to the host).
 __global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items, int n_items, const uint32_t* __restrict__ eq, qm31 lambda,
                                                               const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
-                                                              uint32_t* __restrict__ out, uint32_t* __restrict__ final_words, uint32_t* __restrict__ masks,
-                                                              unsigned int* __restrict__ done, int step) {
+                                                              uint32_t* __restrict__ records, unsigned int* __restrict__ done, int step, int n_rounds, GkrLayerOut host) {
     __shared__ uint32_t sh[8][8];
     __shared__ GkrStepSm sm;
     __shared__ GkrStepConst consts;
@@ -270,7 +280,7 @@ __global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem
     const qm31 r = ldqb(reinterpret_cast<const uint32_t*>(&st->challenge), 0);
     const uint32_t oracle = (uint32_t)it.slot, group = (uint32_t)(it.slot >> 32);
     if (it.mode == 2) {
-        if (threadIdx.x < 2) fix_mask(it, threadIdx.x, r, masks + 16 * (size_t)oracle);
+        if (threadIdx.x < 2) fix_mask(it, threadIdx.x, r, host.masks + 16 * (size_t)oracle);
     } else {
         qm31 s0 = qm31_zero(), s2 = qm31_zero();
         item_sums_of(it, (size_t)bx * blockDim.x + threadIdx.x, (size_t)it.blocks * blockDim.x, r, eq, lambda, s0, s2);
@@ -294,7 +304,7 @@ __global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem
     }
     if (warp != 0) return;
     // Masks are written by two lanes of this warp too: one fence orders either before the count.
-    __threadfence();
+    if (step < 0) __threadfence_system(); else __threadfence();
     __syncwarp();
     unsigned int n = 0;
     if (lane == 0) n = atomicAdd(done, 1u);
@@ -302,7 +312,13 @@ __global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __threadfence();
     if (lane == 0) *done = 0u;
-    if (step < 0) return;
+    if (step < 0) {
+        layer_out_words(host, records, n_rounds, st, lane, 32);
+        __threadfence_system();
+        __syncwarp();
+        if (lane == 0) *host.flag = host.id;
+        return;
+    }
     if (lane < 16) reinterpret_cast<uint4*>(&consts)[lane] = reinterpret_cast<const uint4*>(rc + step)[lane];
     batch_step_open(sm, *st, lane);
     unsigned long long a[8];
@@ -311,8 +327,8 @@ __global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem
         a[c] = __ldcg(&st->acc[step & 1][lane][c]);
         st->acc[step & 1][lane][c] = 0ull;  // for the round after the next
     }
-    batch_step(sm, *st, consts, acc_value(a), acc_value(a + 4), out + GKR_LAYER_OUT_WORDS * (size_t)step);
-    batch_step_close(sm, st, st->degenerate, final_words, lane);
+    batch_step(sm, *st, consts, acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)step);
+    batch_step_close(sm, st, st->degenerate, lane);
 }
 
 // ---- a single round with its results to the host
@@ -392,7 +408,7 @@ __global__ void __launch_bounds__(256) gkr_batch_round_kernel(const GkrBatchItem
 __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const GkrBatchItem* __restrict__ items_base, const uint4* __restrict__ tables,
                                                                           int n_tables, const uint32_t* __restrict__ eq, qm31 lambda,
                                                                           const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
-                                                                          uint32_t* __restrict__ out, uint32_t* __restrict__ final_words, uint32_t* __restrict__ masks) {
+                                                                          uint32_t* __restrict__ records, int n_rounds, GkrLayerOut host) {
     __shared__ GkrStepSm sm;
     __shared__ struct alignas(16) { uint32_t digest[8], n_draws, degenerate, pad[2]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
     GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
@@ -420,7 +436,7 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
             if (live) {
                 it = items[idx];
                 if (it.mode == 2) {
-                    if (sub < 2) fix_mask(it, sub, r, masks + 16 * (size_t)(uint32_t)it.slot);
+                    if (sub < 2) fix_mask(it, sub, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
                 } else {
                     item_sums_of(it, sub, g, r, eq, lambda, s0, s2);
                 }
@@ -460,7 +476,7 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
 #pragma unroll
                     for (int c = 0; c < 4; c++)
                         v[z].c[c] = m31_reduce64(acc[round & 1][lane][8 * z + 2 * c] + ((uint64_t)acc[round & 1][lane][8 * z + 2 * c + 1] << 16));
-                batch_step(sm, s, consts, v[0], v[1], out + GKR_LAYER_OUT_WORDS * (size_t)round);
+                batch_step(sm, s, consts, v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)round);
             } else if (warp == 1) {
 #pragma unroll
                 for (int c = 0; c < 16; c++) acc[(round + 1) & 1][lane][c] = 0u;
@@ -468,49 +484,50 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
             __syncthreads();
         }
     }
-    if (warp == 0) {
-        batch_step_close(sm, st, s.degenerate, final_words, lane);
-    }
+    if (warp == 0) batch_step_close(sm, st, s.degenerate, lane);
+    __threadfence();
+    __syncthreads();
+    layer_out_words(host, records, n_rounds, st, tid, GKR_TAIL_THREADS);
+    __threadfence_system();
+    __syncthreads();
+    if (tid == 0) *host.flag = host.id;
 }
 
-template <int KIND>
-__device__ __forceinline__ void item_next_layer(const GkrBatchItem& it, uint32_t bx) {
-    const size_t half = it.n / 2, stride = (size_t)it.blocks * blockDim.x;
-    for (size_t i = (size_t)bx * blockDim.x + threadIdx.x; i < half; i += stride) {
-        qm31 d0 = ldqb(it.den, 2 * i), d1 = ldqb(it.den, 2 * i + 1);
-        if (KIND != ZKB_GKR_GRAND_PRODUCT) {
-            qm31 n;
-            if (KIND == ZKB_GKR_LOGUP_SINGLES) n = qm31_add(d0, d1);
-            else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) n = qm31_add(qm31_mul_m31(d1, it.num[2 * i]), qm31_mul_m31(d0, it.num[2 * i + 1]));
-            else n = qm31_add(qm31_mul(d1, ldqb(it.num, 2 * i)), qm31_mul(d0, ldqb(it.num, 2 * i + 1)));
-            stqb(it.num_out, i, n);
-        }
-        stqb(it.den_out, i, qm31_mul(d0, d1));
-    }
-}
-
-__global__ void __launch_bounds__(256) gkr_batch_next_layer_kernel(const GkrBatchItem* __restrict__ items, int n_items) {
-    const int idx = find_item(items, n_items, blockIdx.x);
-    const GkrBatchItem it = items[idx];
+// The towers of all instances, ten levels a launch (gkr_tower.cuh); an item's layers lie one after the other from num_out / den_out
+// on. A launch per level and its table cost some 15 us of host time each, for levels of a microsecond or two: 582 instances of up
+// to 2^19 entries took 19 launches, now two.
+__global__ void __launch_bounds__(TOWER_THREADS) gkr_batch_tower_kernel(const GkrBatchItem* __restrict__ items, int n_items, int level0, uint32_t* __restrict__ tops) {
+    __shared__ uint4 sd[512], sn[512];
+    const GkrBatchItem it = items[find_item(items, n_items, blockIdx.x)];
+    const int log = 63 - __clzll(it.n), left = log - level0, cta_log = left < TOWER_LEVELS ? left : TOWER_LEVELS;
+    auto words_before = [&](int level) { return 4 * (it.n - (it.n >> (level - 1))); };
+    auto outs = [&](int l, uint32_t*& num, uint32_t*& den) {
+        const size_t at = words_before(level0 + l + 1);
+        num = it.num_out + at;
+        den = it.den_out + at;
+    };
+    uint32_t* const top = left == cta_log ? tops + GKR_TOP_WORDS * it.slot : nullptr;
     const uint32_t bx = blockIdx.x - it.first_block;
-    switch (it.kind) {
-        case ZKB_GKR_GRAND_PRODUCT: item_next_layer<ZKB_GKR_GRAND_PRODUCT>(it, bx); break;
-        case ZKB_GKR_LOGUP_GENERIC: item_next_layer<ZKB_GKR_LOGUP_GENERIC>(it, bx); break;
-        case ZKB_GKR_LOGUP_MULTIPLICITIES: item_next_layer<ZKB_GKR_LOGUP_MULTIPLICITIES>(it, bx); break;
-        default: item_next_layer<ZKB_GKR_LOGUP_SINGLES>(it, bx); break;
+    const uint32_t *num = it.num, *den = it.den;
+    if (level0) {
+        num = it.num_out + words_before(level0);
+        den = it.den_out + words_before(level0);
+    }
+    switch (level0 == 0 || it.kind == ZKB_GKR_GRAND_PRODUCT ? it.kind : ZKB_GKR_LOGUP_GENERIC) {
+        case ZKB_GKR_GRAND_PRODUCT: tower_cta<ZKB_GKR_GRAND_PRODUCT>(num, den, bx, cta_log, cta_log, sd, sn, outs, top); break;
+        case ZKB_GKR_LOGUP_GENERIC: tower_cta<ZKB_GKR_LOGUP_GENERIC>(num, den, bx, cta_log, cta_log, sd, sn, outs, top); break;
+        case ZKB_GKR_LOGUP_MULTIPLICITIES: tower_cta<ZKB_GKR_LOGUP_MULTIPLICITIES>(num, den, bx, cta_log, cta_log, sd, sn, outs, top); break;
+        default: tower_cta<ZKB_GKR_LOGUP_SINGLES>(num, den, bx, cta_log, cta_log, sd, sn, outs, top); break;
     }
 }
 
 // Splits the flat grid over the items (first_block, blocks) by the work each has; returns the number of CTAs.
-uint32_t plan_blocks(GkrBatchItem* items, int n_items, uint32_t threads_per_unit_shift) {
+uint32_t plan_blocks(GkrBatchItem* items, int n_items) {
     uint32_t total = 0;
     for (int k = 0; k < n_items; k++) {
         GkrBatchItem& it = items[k];
-        size_t units = it.mode == 3 ? it.n / 2 : it.mode == 0 ? it.n / 4 : it.mode == 1 ? it.n / 8 : 1;
-        size_t blocks = (units + 255) / 256;
-        blocks = (blocks + threads_per_unit_shift) >> threads_per_unit_shift;  // a few units per thread on large items
-        if (blocks < 1) blocks = 1;
-        if (blocks > 148u * 4u) blocks = 148u * 4u;
+        const size_t units = it.mode == 0 ? it.n / 4 : it.mode == 1 ? it.n / 8 : 1;
+        const size_t blocks = std::min<size_t>(std::max<size_t>((units + 255) / 256, 1), 148u * 4u);
         it.first_block = total;
         it.blocks = (uint32_t)blocks;
         total += it.blocks;
@@ -528,21 +545,6 @@ int stage_items(zkb_ctx* ctx, const GkrBatchItem* items, int n_items, const GkrB
 }
 
 }  // namespace
-
-int gkr_batch_next_layer(zkb_ctx* ctx, GkrBatchItem* items, int n_items) {
-    if (n_items <= 0) return ZKB_OK;
-    if ((size_t)n_items > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
-    DeviceGuard g(ctx);
-    for (int k = 0; k < n_items; k++) items[k].mode = 3;
-    uint32_t total = plan_blocks(items, n_items, 1);
-    const GkrBatchItem* d_items;
-    int rc = stage_items(ctx, items, n_items, &d_items);
-    if (rc) return rc;
-    ProfScope prof(ctx, "gkr_batch_next_layer_kernel");
-    gkr_batch_next_layer_kernel<<<total, 256, 0, ctx->stream>>>(d_items, n_items);
-    ZKB_LAUNCH_CHECK(ctx);
-    return ZKB_OK;
-}
 
 // Page-locked words: the per-item results of a round, then the sequence number of the last completed round. (A layer enqueued at once
 // lands its records there: never more words, with at most a mask per oracle and 24 words a round.)
@@ -566,12 +568,66 @@ static int batch_buffers(zkb_ctx* ctx) {
     return ZKB_OK;
 }
 
+// Waits for a launch to report `id`: a bounded spin on the host (about 20 ms), then the stream.
+static cudaError_t batch_wait(zkb_ctx* ctx, unsigned int id) {
+    volatile unsigned int* flag = reinterpret_cast<volatile unsigned int*>(ctx->h_batch + H_BATCH_FLAG);
+    if (!ctx->prof_on)
+        for (long spin = 0; spin < 20000000L && *flag != id; spin++) {
+#if defined(__x86_64__)
+            __builtin_ia32_pause();
+#endif
+        }
+    cudaError_t e = cudaSuccess;
+    if (*flag != id) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess && *flag != id) e = cudaErrorUnknown;  // the launch ended without completing every item
+    std::atomic_thread_fence(std::memory_order_acquire);
+    return e;
+}
+
+int gkr_batch_towers(zkb_ctx* ctx, GkrBatchItem* items, int n_items, uint32_t* h_tops) {
+    if (n_items <= 0) return ZKB_OK;
+    if ((size_t)n_items > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
+    DeviceGuard g(ctx);
+    if (int rc = batch_buffers(ctx)) return rc;
+    uint32_t* d_tops = nullptr;
+    if (int rc = zkb_malloc(ctx, GKR_TOP_WORDS * 4 * (size_t)n_items, (void**)&d_tops)) return rc;
+    for (int k = 0; k < n_items; k++) items[k].slot = (unsigned long long)k;
+    cudaError_t e = cudaSuccess;
+    int rc = ZKB_OK;
+    std::vector<GkrBatchItem> live;
+    for (int level0 = 0; rc == ZKB_OK && e == cudaSuccess; level0 += TOWER_LEVELS) {
+        live.clear();
+        uint32_t total = 0;
+        for (int k = 0; k < n_items; k++) {
+            if ((items[k].n >> level0) < 2) continue;
+            live.push_back(items[k]);
+            live.back().first_block = total;
+            total += (uint32_t)std::max<unsigned long long>(items[k].n >> (level0 + TOWER_LEVELS), 1);
+        }
+        if (live.empty()) break;
+        const GkrBatchItem* d_items;
+        rc = stage_items(ctx, live.data(), (int)live.size(), &d_items);
+        if (rc) break;
+        ProfScope prof(ctx, "gkr_batch_tower_kernel");
+        gkr_batch_tower_kernel<<<total, TOWER_THREADS, 0, ctx->stream>>>(d_items, (int)live.size(), level0, d_tops);
+        e = cudaGetLastError();
+    }
+    const size_t bytes = GKR_TOP_WORDS * 4 * (size_t)n_items;
+    if (rc == ZKB_OK && e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_batch, d_tops, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    if (rc == ZKB_OK && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    zkb_free(ctx, d_tops);
+    if (rc) return rc;
+    if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr batch towers: %s", cudaGetErrorString(e));
+    memcpy(h_tops, ctx->h_batch, bytes);
+    return ZKB_OK;
+}
+
 int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32_t h_r[4], const uint32_t* eq_evals, const uint32_t h_lambda[4],
                     uint32_t* h_results) {
     if (n_items <= 0) return ZKB_OK;
     if ((size_t)n_items > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
     DeviceGuard g(ctx);
-    uint32_t total = plan_blocks(items, n_items, 0);
+    uint32_t total = plan_blocks(items, n_items);
     if (int rc = batch_buffers(ctx)) return rc;
     // The device writes the results straight into the page-locked host buffer (unified addressing: the host pointer is valid
     // on the device). scratch: [(unused) | partials]
@@ -593,16 +649,7 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
     }
     const size_t bytes = (size_t)n_items * GKR_BATCH_RESULT_WORDS * 4;
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess && !ctx->prof_on) {
-        // wait on the host for the round's sequence number: a bounded spin (about 20 ms), then the stream
-        for (long spin = 0; spin < 20000000L && *flag != round_id; spin++) {
-#if defined(__x86_64__)
-            __builtin_ia32_pause();
-#endif
-        }
-    }
-    if (e == cudaSuccess && *flag != round_id) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess && *flag != round_id) e = cudaErrorUnknown;  // the launch ended without completing every item
+    if (e == cudaSuccess) e = batch_wait(ctx, round_id);
     if (e != cudaSuccess) {
         // a launch that did not run to its end may have left tickets counted up
         cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream);
@@ -612,73 +659,62 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
     return ZKB_OK;
 }
 
-int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const uint32_t* alpha_pow, const uint32_t* claims,
-                    GkrLayerRound* rounds, int n_rounds, const uint32_t* eq_evals, const uint32_t h_lambda[4], uint32_t chan[9],
-                    uint32_t* h_out, uint32_t* h_masks, bool* degenerate) {
-    *degenerate = false;
-    if (n_oracles <= 0 || n_rounds <= 0) return ZKB_OK;
-    if ((size_t)n_oracles > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
+int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
+    const int n_rounds = plan.n_rounds;
+    if (plan.n_vars.size() > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
     if (n_rounds > GKR_LAYER_MAX_ROUNDS) return set_error(ctx, ZKB_EINVAL, "gkr batch: %d rounds in a layer", n_rounds);
     DeviceGuard g(ctx);
-    if (int rc = batch_buffers(ctx)) return rc;
-    const size_t K = (size_t)n_oracles;
-    // The staged block: the transcript's state, the powers of alpha, the rounds' constants, the rounds' item tables (every part a
-    // multiple of four words).
-    const size_t o_state = 0, o_alpha = sizeof(GkrStepState) / 4, o_rounds = o_alpha + 4 * K, o_items = o_rounds + (sizeof(GkrStepConst) / 4) * (size_t)n_rounds;
-    // Launch j (0 <= j <= n_rounds) carries the fixes of round j - 1 (challenge of that round) and the first sums of the oracles
-    // that enter in round j, and its completing CTA runs the transcript step of round j: one launch per round and one more.
-    size_t n_items = 0;
-    for (int j = 0; j < n_rounds; j++) n_items += (size_t)rounds[j].n_fix + rounds[j].n_first;
-    std::vector<size_t> table_at((size_t)n_rounds + 2);
-    const size_t o_tables = o_items + (sizeof(GkrBatchItem) / 4) * n_items;
-    std::vector<uint32_t>& blob = ctx_blob();
-    blob.assign(o_tables + 4 * ((size_t)n_rounds + 1), 0u);
-    GkrBatchItem* const items = reinterpret_cast<GkrBatchItem*>(&blob[o_items]);
-    std::vector<uint32_t> totals((size_t)n_rounds + 1, 0u);
-    std::vector<uint32_t> group((size_t)n_rounds + 1, 2u);
     // The small rounds at the end of the layer go to one single-CTA launch: from the first table on after which every table
     // is at most GKR_TAIL_MAX_UNITS units of work (a unit = what one thread does in a pass: eight entries of a fix): one unit
     // per thread of the CTA.
     constexpr size_t GKR_TAIL_MAX_UNITS = 512;
-    std::vector<char> small((size_t)n_rounds + 1, 0);
-    size_t at = 0;
-    for (int j = 0; j <= n_rounds; j++) {
-        table_at[j] = at;
-        GkrBatchItem* const t = items + at;
-        if (j > 0 && rounds[j - 1].n_fix) memcpy(items + at, rounds[j - 1].fix, sizeof(GkrBatchItem) * (size_t)rounds[j - 1].n_fix), at += (size_t)rounds[j - 1].n_fix;
-        if (j < n_rounds && rounds[j].n_first) memcpy(items + at, rounds[j].first, sizeof(GkrBatchItem) * (size_t)rounds[j].n_first), at += (size_t)rounds[j].n_first;
-        const int nt = (int)(at - table_at[j]);
-        if (!nt) {
-            if (j < n_rounds) return set_error(ctx, ZKB_EINVAL, "gkr batch: round %d of the layer has no work", j);
-            small[j] = 1;
-            continue;
-        }
-        totals[j] = plan_blocks(t, nt, 0);
+    plan.ctas.assign((size_t)n_rounds + 1, 0u);
+    plan.lanes.assign((size_t)n_rounds + 1, 2u);
+    plan.tail_from = n_rounds + 1;
+    bool tail = true;
+    if (const char* e = getenv("ZKB_GKR_ROUNDS")) tail = strcmp(e, "launches") != 0;
+    for (int j = n_rounds; j >= 0; j--) {
+        GkrBatchItem* const t = plan.items.data() + plan.table_at[j];
+        const int nt = (int)(plan.table_at[j + 1] - plan.table_at[j]);
+        if (!nt) return set_error(ctx, ZKB_EINVAL, "gkr batch: round %d of the layer has no work", j);
+        plan.ctas[j] = plan_blocks(t, nt);
         size_t units = 0, widest = 1;
         for (int q = 0; q < nt; q++) {
-            t[q].slot = (t[q].slot & 0xffffffffull) | (unsigned long long)(n_rounds - (int)n_vars[t[q].slot & 0xffffffffull]) << 32;
+            t[q].slot = (t[q].slot & 0xffffffffull) | (unsigned long long)(n_rounds - (int)plan.n_vars[t[q].slot & 0xffffffffull]) << 32;
             const size_t u = t[q].mode == 0 ? t[q].n / 4 : t[q].mode == 1 ? t[q].n / 8 : 2;
             units += u;
             widest = std::max(widest, u);
         }
-        uint32_t gsz = 2;
-        while (gsz < 32 && gsz < widest) gsz *= 2;
-        group[j] = gsz;
-        small[j] = units <= GKR_TAIL_MAX_UNITS;
+        while (plan.lanes[j] < 32 && plan.lanes[j] < widest) plan.lanes[j] *= 2;
+        tail = tail && units <= GKR_TAIL_MAX_UNITS;
+        if (tail) plan.tail_from = j;
     }
-    table_at[n_rounds + 1] = at;
-    int j_tail = n_rounds + 1;
-    while (j_tail > 0 && small[j_tail - 1]) j_tail--;
-    if (const char* e = getenv("ZKB_GKR_ROUNDS"))
-        if (!strcmp(e, "launches")) j_tail = n_rounds + 1;
-    const size_t n_tail_tables = (size_t)(n_rounds + 1 - j_tail);
+    void* d = nullptr;
+    if (int rc = stage_blob(ctx, plan.items.data(), plan.items.size() * sizeof(GkrBatchItem), &d)) return rc;
+    plan.d_items = static_cast<const GkrBatchItem*>(d);
+    return ZKB_OK;
+}
+
+int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
+                          const uint32_t* eq_evals, const uint32_t h_lambda[4], const uint32_t chan[9]) {
+    DeviceGuard g(ctx);
+    if (int rc = batch_buffers(ctx)) return rc;
+    const size_t K = plan.n_vars.size();
+    const int n_rounds = plan.n_rounds, n_tail_tables = n_rounds + 1 - plan.tail_from;
+    // The staged block: the transcript's state, the powers of alpha, the rounds' constants, the tail's tables, room for the rounds'
+    // records (every part a multiple of four words).
+    const size_t o_state = 0, o_alpha = sizeof(GkrStepState) / 4, o_rounds = o_alpha + 4 * K, o_tables = o_rounds + (sizeof(GkrStepConst) / 4) * (size_t)n_rounds;
+    const size_t o_records = o_tables + 4 * ((size_t)n_rounds + 1);
+    std::vector<uint32_t>& blob = ctx_blob();
+    blob.assign(o_records + GKR_LAYER_OUT_WORDS * (size_t)n_rounds, 0u);
     auto q4 = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
     // The oracles' claims by the round they enter in (group; those without variables never do), each times alpha^k. The claims come
     // scaled by 2^(rounds they wait), and a waiting oracle's claim halves every round (sumcheck.rs:115-125).
-    std::vector<qm31> entering((size_t)n_rounds + 1, qm31_zero());
+    qm31 entering[GKR_LAYER_MAX_ROUNDS + 1];
+    for (auto& v : entering) v = qm31_zero();
     for (size_t k = 0; k < K; k++) {
-        qm31& e = entering[(size_t)n_rounds - n_vars[k]];
-        e = qm31_add(e, qm31_mul(q4(alpha_pow + 4 * k), q4(claims + 4 * k)));
+        qm31& v = entering[n_rounds - (int)plan.n_vars[k]];
+        v = qm31_add(v, qm31_mul(q4(alpha_pow + 4 * k), q4(claims + 4 * k)));
     }
     GkrStepState& st = *reinterpret_cast<GkrStepState*>(&blob[o_state]);
     memcpy(st.digest, chan, 32);
@@ -691,7 +727,7 @@ int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const u
     for (int j = n_rounds; j-- > 0;) {
         waiting = qm31_add(waiting, entering[j + 1]);  // all that enter after round j
         GkrStepConst& c = consts[j];
-        const GkrRoundConst& rc = rounds[j].rc;
+        const GkrRoundConst& rc = rounds[j];
         const uint32_t half_pow = m31_inv(1u << (j + 1 < 31 ? j + 1 : 0));  // 2^-(j + 1)
         for (int t = 0; t < 4; t++) {
             c.A[t] = qm31_mul(q4(rc.e0a), qm31_sub(q4(rc.L[0][t]), q4(rc.L[1][t])));
@@ -703,24 +739,25 @@ int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const u
         c.entering = j + 1 < n_rounds ? qm31_mul_m31(entering[j + 1], half_pow) : qm31_zero();
         c.round = (uint32_t)j;
     }
-    for (int j = j_tail; j <= n_rounds; j++) {
-        uint32_t* tb = &blob[o_tables + 4 * (size_t)(j - j_tail)];
-        tb[0] = (uint32_t)table_at[j];
-        tb[1] = (uint32_t)(table_at[j + 1] - table_at[j]);
-        tb[2] = group[j];
+    for (int j = plan.tail_from; j <= n_rounds; j++) {
+        uint32_t* tb = &blob[o_tables + 4 * (size_t)(j - plan.tail_from)];
+        tb[0] = (uint32_t)plan.table_at[j];
+        tb[1] = (uint32_t)(plan.table_at[j + 1] - plan.table_at[j]);
+        tb[2] = plan.lanes[j];
         tb[3] = j < n_rounds ? (uint32_t)j + 1u : 0u;
     }
     void* d_blob_v = nullptr;
     if (int rc = stage_blob(ctx, blob.data(), blob.size() * 4, &d_blob_v)) return rc;
     uint32_t* d_blob = static_cast<uint32_t*>(d_blob_v);
-    // what comes back in one copy: the rounds' records, the channel, the masks
-    const size_t o_chan = GKR_LAYER_OUT_WORDS * (size_t)n_rounds, o_masks = o_chan + 12, out_words = o_masks + GKR_LAYER_MASK_WORDS * K;
-    uint32_t* d_out = nullptr;
-    if (int rc = zkb_malloc(ctx, out_words * 4, (void**)&d_out)) return rc;
     GkrStepState* d_state = reinterpret_cast<GkrStepState*>(d_blob + o_state);
     const GkrStepConst* d_consts = reinterpret_cast<const GkrStepConst*>(d_blob + o_rounds);
-    const GkrBatchItem* d_items = reinterpret_cast<const GkrBatchItem*>(d_blob + o_items);
     const qm31 lam = q4(h_lambda);
+    GkrLayerOut host;
+    host.records = ctx->h_batch;
+    host.channel = host.records + GKR_LAYER_OUT_WORDS * (size_t)n_rounds;
+    host.masks = host.channel + 12;
+    host.flag = reinterpret_cast<volatile unsigned int*>(ctx->h_batch + H_BATCH_FLAG);
+    host.id = ++ctx->batch_round;
     cudaError_t e = cudaSuccess;
     // Each launch but the first is a programmatic dependent of the one before it (ZKB_GKR_PDL=0: plain stream order).
     const char* pdl_env = getenv("ZKB_GKR_PDL");
@@ -733,16 +770,16 @@ int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const u
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
     bool launched = false;
-    for (int j = 0; j < j_tail && j <= n_rounds && e == cudaSuccess; j++) {
-        const int nt = (int)(table_at[j + 1] - table_at[j]);
-        if (!nt) continue;
-        ProfScope prof(ctx, totals[j] <= 8 ? "gkr_batch_layer_kernel(<=8 CTAs)" : totals[j] <= 128 ? "gkr_batch_layer_kernel(<=128 CTAs)"
-                                 : totals[j] <= 2048 ? "gkr_batch_layer_kernel(<=2048 CTAs)" : "gkr_batch_layer_kernel(>2048 CTAs)");
-        cfg.gridDim = dim3(totals[j]);
+    for (int j = 0; j < plan.tail_from && e == cudaSuccess; j++) {
+        const uint32_t ctas = plan.ctas[j];
+        ProfScope prof(ctx, ctas <= 8 ? "gkr_batch_layer_kernel(<=8 CTAs)" : ctas <= 128 ? "gkr_batch_layer_kernel(<=128 CTAs)"
+                                 : ctas <= 2048 ? "gkr_batch_layer_kernel(<=2048 CTAs)" : "gkr_batch_layer_kernel(>2048 CTAs)");
+        cfg.gridDim = dim3(ctas);
         cfg.blockDim = dim3(256);
         cfg.numAttrs = pdl && launched ? 1 : 0;  // the first launch follows a copy, not a kernel of this chain
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, d_items + table_at[j], nt, eq_evals, lam, (const uint32_t*)(d_blob + o_alpha), d_state, d_consts,
-                               d_out, d_out + o_chan, d_out + o_masks, ctx->batch_tickets + GKR_BATCH_MAX_ITEMS, j < n_rounds ? j : -1);
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items + plan.table_at[j], (int)(plan.table_at[j + 1] - plan.table_at[j]), eq_evals, lam,
+                               (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_blob + o_records, ctx->batch_tickets + GKR_BATCH_MAX_ITEMS,
+                               j < n_rounds ? j : -1, n_rounds, host);
         launched = true;
     }
     if (n_tail_tables && e == cudaSuccess) {
@@ -750,21 +787,27 @@ int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const u
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(GKR_TAIL_THREADS);
         cfg.numAttrs = pdl && launched ? 1 : 0;
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_tail_kernel, d_items, reinterpret_cast<const uint4*>(d_blob + o_tables), (int)n_tail_tables, eq_evals, lam,
-                               (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_out, d_out + o_chan, d_out + o_masks);
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_tail_kernel, plan.d_items, reinterpret_cast<const uint4*>(d_blob + o_tables), n_tail_tables, eq_evals, lam,
+                               (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_blob + o_records, n_rounds, host);
     }
-    uint32_t* h = ctx->h_batch;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_out, out_words * 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    zkb_free(ctx, d_out);
     if (e != cudaSuccess) {
         cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream);
         return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
     }
-    memcpy(h_out, h, o_chan * 4);
-    memcpy(chan, h + o_chan, 9 * 4);
-    *degenerate = h[o_chan + 9] != 0u;
-    memcpy(h_masks, h + o_masks, GKR_LAYER_MASK_WORDS * K * 4);
+    return ZKB_OK;
+}
+
+int gkr_batch_layer_end(zkb_ctx* ctx, const GkrLayerPlan& plan, GkrLayerResult& res) {
+    DeviceGuard g(ctx);
+    const cudaError_t e = batch_wait(ctx, ctx->batch_round);
+    if (e != cudaSuccess) {
+        cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream);
+        return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
+    }
+    res.records = ctx->h_batch;
+    res.channel = res.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
+    res.masks = res.channel + 12;
+    res.degenerate = res.channel[9] != 0u;
     return ZKB_OK;
 }
 

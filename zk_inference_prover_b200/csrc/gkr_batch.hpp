@@ -2,6 +2,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 struct zkb_ctx;
 
@@ -9,7 +10,7 @@ namespace zk {
 
 // What to do for one instance in a batched launch. kind: ZKB_GKR_* of the INPUT arrays; n: entries of the input layer.
 // mode 0: round sums of the layer; 1: fix the first variable into num_out/den_out (n >= 8) and round sums of the result;
-// 2: fix the first variable of a 4-entry layer, the result also copied to the result words; 3: next_layer.
+// 2: fix the first variable of a 4-entry layer, the result also copied to the result words.
 // first_block / blocks are filled by the launcher.
 struct GkrBatchItem {
     const uint32_t* num;
@@ -26,8 +27,11 @@ constexpr size_t GKR_BATCH_MAX_ITEMS = 8192;
 // Per item: [0,8) the two sums (t = 0, t = 2); mode 2 only: [8,16) the two fixed denominators, [16,24) the two fixed numerators.
 constexpr size_t GKR_BATCH_RESULT_WORDS = 24;
 
-// next_layer of every item, one launch, stream-ordered.
-int gkr_batch_next_layer(zkb_ctx* ctx, GkrBatchItem* items, int n_items);
+// The layers above every item's input (num, den, n >= 2 entries, kind), one after the other from den_out and (but for a grand
+// product) num_out on, n - 1 entries each: level 1 first. h_tops: per item the output's denominator and numerator, then the two
+// denominators and the two numerators of the layer below it (numerators of an input without its own: undefined).
+constexpr size_t GKR_TOP_WORDS = 24;
+int gkr_batch_towers(zkb_ctx* ctx, GkrBatchItem* items, int n_items, uint32_t* h_tops);
 // One round for every item with the transcript on the host: one launch that writes n_items * GKR_BATCH_RESULT_WORDS words and
 // a completion word into page-locked host memory; returns when the host has seen the completion word (h_results filled).
 int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32_t h_r[4], const uint32_t* eq_evals, const uint32_t h_lambda[4],
@@ -53,24 +57,34 @@ struct GkrRoundConst {
 };
 static_assert(sizeof(GkrRoundConst) == 256, "GkrRoundConst layout");
 
-struct GkrLayerRound {
-    GkrRoundConst rc;
-    GkrBatchItem* first;  // mode 0 items of the oracles that enter in this round (slot = oracle)
-    int n_first;
-    GkrBatchItem* fix;    // mode 1 / 2 items of every active oracle (slot = oracle)
-    int n_fix;
-};
-
 constexpr int GKR_LAYER_MAX_ROUNDS = 31;
 constexpr size_t GKR_LAYER_MASK_WORDS = 16;  // per oracle: the two fixed denominators, the two fixed numerators
 constexpr size_t GKR_LAYER_OUT_WORDS = 24;  // per round: [0,16) coefficients, [16] length, [20,24) challenge
 
-// n_vars[k]: variables of oracle k's sum-check (it is active in the rounds with n_rem <= n_vars[k]); alpha_pow[k] = alpha^k;
-// claims[k]: its claim before the first round (4 words each). chan: digest (8 words) and n_draws, in and out.
-// h_out: n_rounds x GKR_LAYER_OUT_WORDS; h_masks: n_oracles x GKR_LAYER_MASK_WORDS (of every oracle that had a round). degenerate:
-// a round polynomial's leading coefficient vanished; the results do not follow the transcript then and must be thrown away.
-int gkr_batch_layer(zkb_ctx* ctx, int n_oracles, const uint32_t* n_vars, const uint32_t* alpha_pow, const uint32_t* claims,
-                    GkrLayerRound* rounds, int n_rounds, const uint32_t* eq_evals, const uint32_t h_lambda[4], uint32_t chan[9],
-                    uint32_t* h_out, uint32_t* h_masks, bool* degenerate);
+// What depends on the oracles' sizes and addresses only: a caller makes and stages it while the layer before runs.
+struct GkrLayerPlan {
+    int n_rounds = 0;                // the variables of the largest oracle
+    std::vector<uint32_t> n_vars;    // per oracle: it is active in the rounds with at most so many variables left
+    std::vector<GkrBatchItem> items; // table after table; table j: the fixes of round j - 1, the first sums of those entering in round j (slot = oracle)
+    std::vector<size_t> table_at;    // n_rounds + 2
+    std::vector<uint32_t> ctas, lanes;  // from here on filled by gkr_batch_plan
+    int tail_from = 0;
+    const GkrBatchItem* d_items = nullptr;
+};
+int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
+
+// alpha_pow[k] = alpha^k; claims[k]: oracle k's claim before the first round (4 words each). chan: digest (8 words) and n_draws.
+// Enqueues the layer; gkr_batch_layer_end waits for it. Only gkr_batch_plan may come between the two.
+int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
+                          const uint32_t* eq_evals, const uint32_t h_lambda[4], const uint32_t chan[9]);
+
+// In the context's memory, until the next call: n_rounds x GKR_LAYER_OUT_WORDS, the channel as above, n_oracles x GKR_LAYER_MASK_WORDS
+// (of every oracle that had a round). degenerate: a round polynomial's leading coefficient vanished; the results do not follow
+// the transcript then and must be thrown away.
+struct GkrLayerResult {
+    const uint32_t *records, *channel, *masks;
+    bool degenerate;
+};
+int gkr_batch_layer_end(zkb_ctx* ctx, const GkrLayerPlan& plan, GkrLayerResult& res);
 
 }  // namespace zk

@@ -24,6 +24,7 @@
 
 #include "channel.cuh"
 #include "common.cuh"
+#include "gkr_tower.cuh"
 #include "gkr_resident.hpp"
 #include "host/b200_backend.hpp"
 
@@ -405,56 +406,17 @@ __device__ __forceinline__ void pass_term(const void* num, const void* den, void
     t2 = term_at<KIND>(at_two(d[0], d[2]), at_two(d[1], d[3]), at_two(u[0], u[2]), at_two(u[1], u[3]), lambda);
 }
 
-// ---- towers: up to ten levels of a layer's halvings per launch (gen_layers, gkr_prover.rs:847-852). A level's entries come from
-// adjacent pairs, so a CTA that takes 2^10 consecutive entries builds its share of every level above them; the levels stay in
-// shared memory for the next one and every one is written. One launch per level read each level back from memory and cost a
-// launch for the many short ones (a 2^24 tower: 24 launches, 290 us; now three, 218 us).
-constexpr int TOWER_LEVELS = 10, TOWER_THREADS = 256;
+// ---- towers: gkr_tower.cuh's levels, the launches a chain of programmatic dependents
 struct TowerArgs {
     const uint32_t *num, *den;  // 2^log entries
     uint32_t *num_out[TOWER_LEVELS], *den_out[TOWER_LEVELS];
     int levels, cta_log;        // a CTA takes 2^cta_log entries, levels <= cta_log
 };
 template <int KIND>
-__device__ __forceinline__ void tower_pair(qm31 n0, qm31 n1, qm31 d0, qm31 d1, qm31& n, qm31& d) {
-    d = qm31_mul(d0, d1);
-    if (KIND == ZKB_GKR_LOGUP_SINGLES) n = qm31_add(d0, d1);
-    else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) n = qm31_add(qm31_mul_m31(d1, n0.c[0]), qm31_mul_m31(d0, n1.c[0]));
-    else if (KIND == ZKB_GKR_LOGUP_GENERIC) n = qm31_add(qm31_mul(d1, n0), qm31_mul(d0, n1));
-    else n = qm31_zero();
-}
-template <int KIND>
 __global__ void __launch_bounds__(TOWER_THREADS) tower_kernel(TowerArgs a) {
-    constexpr bool HAS_NUM_OUT = KIND != ZKB_GKR_GRAND_PRODUCT;
-    constexpr int KIND2 = HAS_NUM_OUT ? ZKB_GKR_LOGUP_GENERIC : ZKB_GKR_GRAND_PRODUCT;
-    __shared__ uint4 sd[512], sn[HAS_NUM_OUT ? 512 : 1];
+    __shared__ uint4 sd[512], sn[KIND != ZKB_GKR_GRAND_PRODUCT ? 512 : 1];
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t half = 1u << (a.cta_log - 1);
-    const size_t first = (size_t)blockIdx.x * half;
-    for (uint32_t i = threadIdx.x; i < half; i += TOWER_THREADS) {
-        const size_t o = first + i;
-        qm31 n0 = qm31_zero(), n1 = qm31_zero(), n, d;
-        if (KIND == ZKB_GKR_LOGUP_GENERIC) { n0 = ldq_r(a.num, 2 * o); n1 = ldq_r(a.num, 2 * o + 1); }
-        if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) { n0.c[0] = a.num[2 * o]; n1.c[0] = a.num[2 * o + 1]; }
-        tower_pair<KIND>(n0, n1, ldq_r(a.den, 2 * o), ldq_r(a.den, 2 * o + 1), n, d);
-        stq_r(a.den_out[0], o, d);
-        stq_r(sd, i, d);
-        if (HAS_NUM_OUT) { stq_r(a.num_out[0], o, n); stq_r(sn, i, n); }
-    }
-    for (int l = 1; l < a.levels; l++) {
-        const uint32_t m = half >> l;
-        __syncthreads();
-        qm31 n, d;
-        const uint32_t i = threadIdx.x;  // at most 256 from the second level on
-        if (i < m) tower_pair<KIND2>(HAS_NUM_OUT ? ldq_r(sn, 2 * i) : qm31_zero(), HAS_NUM_OUT ? ldq_r(sn, 2 * i + 1) : qm31_zero(), ldq_r(sd, 2 * i), ldq_r(sd, 2 * i + 1), n, d);
-        __syncthreads();
-        if (i < m) {
-            const size_t o = (size_t)blockIdx.x * m + i;
-            stq_r(a.den_out[l], o, d);
-            stq_r(sd, i, d);
-            if (HAS_NUM_OUT) { stq_r(a.num_out[l], o, n); stq_r(sn, i, n); }
-        }
-    }
+    tower_cta<KIND>(a.num, a.den, blockIdx.x, a.cta_log, a.levels, sd, sn, [&](int l, uint32_t*& num, uint32_t*& den) { num = a.num_out[l]; den = a.den_out[l]; }, nullptr);
 }
 
 // ---- rounds on large layers, one launch each

@@ -140,7 +140,6 @@ struct Layer {
     SecureMle num;      // LOGUP_GENERIC numerators
     BaseColumn num_base;  // LOGUP_MULTIPLICITIES numerators
     SecureMle den;      // denominators, or the grand-product column
-    bool writable = false;  // the arrays are the prover's own scratch (a tower layer, a fixed layer): they may be overwritten
     size_t len() const { return den.len(); }
     size_t n_variables() const { size_t l = 0; while (((size_t)1 << (l + 1)) <= len()) l++; return l; }
     const uint32_t* num_ptr() const {

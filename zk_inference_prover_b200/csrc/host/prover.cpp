@@ -1078,11 +1078,6 @@ struct UniPoly {
 };
 
 static qm31 eq1(qm31 x, qm31 y) { return x * y + (qm31_one() - x) * (qm31_one() - y); }  // utils.rs:165-170
-static qm31 horner(const std::vector<qm31>& v, qm31 x) {
-    qm31 acc = qm31_zero();
-    for (size_t i = v.size(); i-- > 0;) acc = acc * x + v[i];
-    return acc;
-}
 
 // correct_sum_as_poly_in_first_variable (gkr_prover.rs:884-923), split in two.
 // The part that depends only on the out-of-domain point y and on the number of
@@ -1126,23 +1121,6 @@ struct RoundBasis {
     }
 };
 
-struct GkrOracle {  // GkrMultivariatePolyOracle, gkr_prover.rs:473-556
-    Layer input_layer;
-    qm31 eq_fixed_var_correction;
-    bool have_sums = false;  // the next round's sums, produced together with the last fix
-    std::pair<qm31, qm31> sums;
-    bool have_mask = false;  // the two entries of every column after the last fix, read back with that round's results
-    qm31 mask_den[2], mask_num[2];
-    size_t n_variables() const { return input_layer.n_variables() - 1; }
-};
-
-static std::vector<qm31> mle_to_cpu(const Device& d, const SecureMle& m) {
-    auto w = m.words.to_cpu();
-    std::vector<qm31> out(m.len());
-    for (size_t i = 0; i < out.size(); i++) out[i] = {{w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]}};
-    return out;
-}
-
 static Layer layer_view(const Device& d, int kind, const uint32_t* num, const uint32_t* den, size_t n) {
     Layer l;
     l.kind = kind;
@@ -1152,149 +1130,262 @@ static Layer layer_view(const Device& d, int kind, const uint32_t* num, const ui
     return l;
 }
 
-// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream. host_rounds: the transcript of the rounds stays on
-// the host; otherwise *degenerate may be set, and the caller proves again that way (see gkr_batch.hpp).
-static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::vector<Layer> input_layers, bool host_rounds_only, bool* degenerate) {
-    size_t n_inst = input_layers.size();
-    std::vector<size_t> n_layers_by_inst;
-    for (auto& l : input_layers) n_layers_by_inst.push_back(l.n_variables());
-    size_t n_layers = *std::max_element(n_layers_by_inst.begin(), n_layers_by_inst.end());
-    std::vector<std::vector<Layer>> towers(n_inst);  // gen_layers, :847-852; one launch per level for the whole batch
-    for (size_t i = 0; i < n_inst; i++) towers[i].push_back(std::move(input_layers[i]));
-    std::vector<zk::GkrBatchItem> items;
-    auto item_of = [](const Layer& in, Layer& out, uint32_t mode) {
-        zk::GkrBatchItem it{};
-        it.num = in.num_ptr();
-        it.den = in.den.words.ptr();
-        it.num_out = out.kind == ZKB_GKR_LOGUP_GENERIC ? out.num.words.ptr() : nullptr;
-        it.den_out = out.den.words.ptr();
-        it.n = in.len();
-        it.kind = (uint32_t)in.kind;
-        it.mode = mode;
-        return it;
-    };
-    std::vector<BaseColumn> slabs;  // one allocation per tower level; the layers of that level are views of it
-    std::unique_ptr<HostClock> hc_towers(new HostClock("gkr.towers"));
-    for (;;) {
-        items.clear();
-        size_t words = 0;
-        for (size_t i = 0; i < n_inst; i++) {
-            const Layer& in = towers[i].back();
-            if (in.n_variables() == 0) continue;
-            words += (in.kind == ZKB_GKR_GRAND_PRODUCT ? 1 : 2) * 4 * (in.len() / 2);
-        }
-        if (!words) break;
-        slabs.emplace_back(d, words);
-        uint32_t* cur = slabs.back().ptr();
-        for (size_t i = 0; i < n_inst; i++) {
-            const Layer& in = towers[i].back();
-            if (in.n_variables() == 0) continue;
-            const size_t half_words = 4 * (in.len() / 2);
-            Layer out;
-            out.writable = true;
-            out.kind = in.kind == ZKB_GKR_GRAND_PRODUCT ? ZKB_GKR_GRAND_PRODUCT : ZKB_GKR_LOGUP_GENERIC;
-            out.den.words = BaseColumn::view(d, cur, half_words);
-            cur += half_words;
-            if (out.kind == ZKB_GKR_LOGUP_GENERIC) { out.num.words = BaseColumn::view(d, cur, half_words); cur += half_words; }
-            items.push_back(item_of(in, out, 3));
-            towers[i].push_back(std::move(out));
-        }
-        d.check(zk::gkr_batch_next_layer(d.ctx(), items.data(), (int)items.size()));
-    }
-    hc_towers.reset();
+// The sum-check of a layer with the transcript on the host, a launch a round: table j of the plan gives the sums of round j (of the layers
+// fixed with the challenge before, and of the oracles that enter), the last table the masks (GKR_LAYER_MASK_WORDS per oracle).
+static void host_rounds(const Device& d, Channel& ch, zk::GkrLayerPlan& plan, qm31 alpha, qm31 lambda, const std::vector<qm31>& ood_point, const SecureMle& eq_evals,
+                        std::vector<qm31>& sc_claims, std::vector<UniPoly>& round_polys, std::vector<qm31>& assignment, std::vector<uint32_t>& mask_words) {
+    const size_t K = plan.n_vars.size();
+    const int nv = plan.n_rounds;
+    const uint32_t half = m31_inv(2);
     std::vector<uint32_t> results;
-    // the output layers (one entry per column) of all instances, read in one gather
-    GatherPlan top_plan;
-    std::vector<size_t> top_slot(n_inst, SIZE_MAX);
-    for (size_t i = 0; i < n_inst; i++) {
-        const Layer& t = towers[i].back();
-        if (t.len() != 1 || (t.kind != ZKB_GKR_GRAND_PRODUCT && t.kind != ZKB_GKR_LOGUP_GENERIC)) continue;
-        top_slot[i] = top_plan.addrs.size();
-        for (int w = 0; w < 4; w++) top_plan.add(t.den.words.ptr() + w);
-        if (t.kind == ZKB_GKR_LOGUP_GENERIC)
-            for (int w = 0; w < 4; w++) top_plan.add(t.num.words.ptr() + w);
+    std::vector<qm31> rv(3 * K), corr(K, qm31_one());
+    std::vector<std::pair<qm31, qm31>> sums(K);
+    mask_words.assign(zk::GKR_LAYER_MASK_WORDS * K, 0u);
+    auto q_at = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
+    qm31 challenge = qm31_zero();
+    for (int round = 0; round <= nv; round++) {
+        zk::GkrBatchItem* items = plan.items.data() + plan.table_at[round];
+        const size_t n_items = plan.table_at[round + 1] - plan.table_at[round];
+        {
+            HostClock hc("gkr.round.launch_wait");
+            results.resize(n_items * zk::GKR_BATCH_RESULT_WORDS);
+            d.check(zk::gkr_batch_round(d.ctx(), items, (int)n_items, challenge.c, eq_evals.words.ptr(), lambda.c, results.data()));
+        }
+        for (size_t j = 0; j < n_items; j++) {
+            const uint32_t* w = results.data() + j * zk::GKR_BATCH_RESULT_WORDS;
+            const size_t k = (size_t)items[j].slot;
+            if (items[j].mode == 2) memcpy(&mask_words[zk::GKR_LAYER_MASK_WORDS * k], w + 8, 64);
+            else sums[k] = {q_at(w), q_at(w + 4)};
+        }
+        if (round == nv) break;
+        // Every active oracle has n_rem variables left, so all their round polynomials are r0 L0 + r1 L1 + r2 L2 over the
+        // same basis, and the random linear combination over the batch (sumcheck.rs:139-149, Horner in alpha from the
+        // last oracle down) is (sum alpha^k r0_k) L0 + (sum alpha^k r1_k) L1 + (sum alpha^k r2_k) L2 plus the constants of
+        // the oracles that wait: eleven multiplications per oracle and round instead of a Lagrange interpolation each.
+        // r0 + r1 is the claim by construction, which is the check sumcheck.rs:128-130 makes.
+        HostClock hc("gkr.round.algebra");
+        const size_t n_rem = (size_t)(nv - round);
+        const RoundBasis basis(ood_point, n_rem);
+        auto act = [&](size_t k) { return n_rem <= plan.n_vars[k]; };
+        qm31 S[3] = {qm31_zero(), qm31_zero(), qm31_zero()}, Sc = qm31_zero();
+        for (size_t k = K; k-- > 0;) {
+            for (int t = 0; t < 3; t++) S[t] = S[t] * alpha;
+            Sc = Sc * alpha;
+            if (act(k)) {
+                rv[3 * k] = sums[k].first * corr[k] * basis.e0a;
+                rv[3 * k + 1] = sc_claims[k] - rv[3 * k];
+                rv[3 * k + 2] = sums[k].second * corr[k] * basis.e2a;
+                for (int t = 0; t < 3; t++) S[t] = S[t] + rv[3 * k + t];
+            } else {
+                rv[3 * k] = qm31_mul_m31(sc_claims[k], half);
+                Sc = Sc + rv[3 * k];
+            }
+        }
+        UniPoly combined;
+        combined.c.resize(4);
+        for (int t = 0; t < 4; t++) combined.c[t] = S[0] * basis.L[0][t] + S[1] * basis.L[1][t] + S[2] * basis.L[2][t];
+        combined.c[0] = combined.c[0] + Sc;
+        if (qm31_is_zero(combined.c[3])) {
+            // The combination keeps the length of its longest term. A vanishing leading coefficient does not say which
+            // case this is (every term short, or a cancellation), so this round goes term by term.
+            combined = UniPoly();
+            for (size_t k = K; k-- > 0;) {
+                UniPoly rp;
+                if (act(k)) rp = basis.round_poly(rv[3 * k], rv[3 * k + 1], rv[3 * k + 2]);
+                else { rp.c = {rv[3 * k]}; rp.trim(); }
+                for (auto& c : combined.c) c = c * alpha;
+                combined = UniPoly::add(combined, rp);
+            }
+        }
+        ch.mix_felts(combined.c);
+        challenge = ch.draw_secure_felt();
+        qm31 Lc[3];
+        for (int t = 0; t < 3; t++) Lc[t] = ((basis.L[t][3] * challenge + basis.L[t][2]) * challenge + basis.L[t][1]) * challenge + basis.L[t][0];
+        const qm31 eq_step = eq1(challenge, ood_point[ood_point.size() - n_rem]);  // the same for every active oracle
+        for (size_t k = 0; k < K; k++) {
+            if (act(k)) {
+                sc_claims[k] = rv[3 * k] * Lc[0] + rv[3 * k + 1] * Lc[1] + rv[3 * k + 2] * Lc[2];
+                corr[k] = corr[k] * eq_step;
+            } else sc_claims[k] = rv[3 * k];
+        }
+        round_polys.push_back(std::move(combined));
+        assignment.push_back(challenge);
     }
-    if (!top_plan.addrs.empty()) top_plan.execute(d);
-    auto top_q = [&](size_t slot) { return qm31{{top_plan.words[slot], top_plan.words[slot + 1], top_plan.words[slot + 2], top_plan.words[slot + 3]}}; };
+}
+
+// An instance of a batch: the input and the layers above it. Level 0 is the input, level l has 2^(log - l) entries; the levels from
+// 1 on lie one after the other. A round fixes a level in place (a thread of the fixing kernel reads entries i and i + n/2 and
+// writes entry i, and no other thread touches either), but the input, which is the caller's, into the fold arrays.
+struct BatchTower {
+    int kind, log;
+    const uint32_t *num, *den;
+    uint32_t *num_levels, *den_levels, *num_fold, *den_fold;  // numerators: null where the kind has none
+    int kind_at(int level) const { return level == 0 || kind == ZKB_GKR_GRAND_PRODUCT ? kind : ZKB_GKR_LOGUP_GENERIC; }
+    size_t offset(int level) const { return 4 * (((size_t)1 << log) - ((size_t)1 << (log - level + 1))); }
+};
+
+// The tables of one layer's sum-check (gkr_batch.hpp). Every oracle is level `level` of its instance's tower: those of at least
+// level + 1 levels take part, inst[k] is oracle k's.
+static void plan_layer(const std::vector<BatchTower>& towers, int level, int n_rounds, zk::GkrLayerPlan& plan, std::vector<size_t>& inst) {
+    inst.clear();
+    plan.n_rounds = n_rounds;
+    plan.n_vars.clear();
+    plan.items.clear();
+    plan.table_at.clear();
+    for (size_t i = 0; i < towers.size(); i++)
+        if (towers[i].log > level) {
+            inst.push_back(i);
+            plan.n_vars.push_back((uint32_t)(towers[i].log - level - 1));
+        }
+    if (!n_rounds) return;
+    // round q fixes a layer of 2^(n_rounds - q + 1) entries
+    for (int j = 0; j <= n_rounds; j++) {
+        plan.table_at.push_back(plan.items.size());
+        for (int fix = 1; fix >= 0; fix--) {
+            const int round = fix ? j - 1 : j;
+            if (round < 0 || round == n_rounds) continue;
+            const uint32_t n_rem = (uint32_t)(n_rounds - round);
+            for (size_t k = 0; k < inst.size(); k++) {
+                const bool enters = plan.n_vars[k] == n_rem;
+                if (fix ? plan.n_vars[k] < n_rem : !enters) continue;
+                const BatchTower& t = towers[inst[k]];
+                zk::GkrBatchItem it{};
+                it.n = (unsigned long long)2 << n_rem;
+                it.kind = (uint32_t)t.kind_at(level);
+                it.mode = !fix ? 0u : it.n >= 8 ? 1u : 2u;
+                it.slot = k;
+                const bool num = it.kind == ZKB_GKR_LOGUP_GENERIC || it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES;
+                if (level) {
+                    it.den = it.den_out = t.den_levels + t.offset(level);
+                    if (num) it.num = it.num_out = t.num_levels + t.offset(level);
+                } else {
+                    it.den_out = t.den_fold;
+                    it.den = enters ? t.den : t.den_fold;
+                    if (num) { it.num_out = t.num_fold; it.num = enters ? t.num : t.num_fold; }
+                    if (it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES && !enters) it.kind = ZKB_GKR_LOGUP_GENERIC;
+                }
+                plan.items.push_back(it);
+            }
+        }
+    }
+    plan.table_at.push_back(plan.items.size());
+}
+
+// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream. host_rounds_only: the transcript of the rounds stays on
+// the host; otherwise *degenerate may be set, and the caller proves again that way (see gkr_batch.hpp).
+static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const std::vector<Layer>& input_layers, bool host_rounds_only, bool* degenerate) {
+    const size_t n_inst = input_layers.size();
+    std::unique_ptr<HostClock> hc(new HostClock("gkr.towers"));
+    std::vector<BatchTower> towers(n_inst);  // gen_layers, :847-852
+    int n_layers = 0;
+    BaseColumn slab;
+    for (int pass = 0; pass < 2; pass++) {  // one allocation for all towers and fold arrays: its size, then the places
+        size_t words = 0;
+        auto take = [&](size_t n) { uint32_t* p = pass ? slab.ptr() + words : nullptr; words += n; return p; };
+        for (size_t i = 0; i < n_inst; i++) {
+            const Layer& in = input_layers[i];
+            BatchTower& t = towers[i];
+            t = {in.kind, (int)in.n_variables(), in.num_ptr(), in.den.words.ptr(), nullptr, nullptr, nullptr, nullptr};
+            n_layers = std::max(n_layers, t.log);
+            if (!t.log) continue;
+            const size_t n = in.len();
+            t.den_levels = take(4 * (n - 1));
+            t.den_fold = take(2 * n);
+            if (t.kind != ZKB_GKR_GRAND_PRODUCT) t.num_levels = take(4 * (n - 1));
+            if (t.num) t.num_fold = take(2 * n);
+        }
+        if (!pass && words) slab = BaseColumn(d, words);
+    }
+    std::vector<zk::GkrBatchItem> items;
+    std::vector<size_t> top_of(n_inst, 0);
+    for (size_t i = 0; i < n_inst; i++) {
+        const BatchTower& t = towers[i];
+        if (!t.log) continue;
+        top_of[i] = zk::GKR_TOP_WORDS * items.size();
+        zk::GkrBatchItem it{};
+        it.num = t.num;
+        it.den = t.den;
+        it.num_out = t.num_levels;
+        it.den_out = t.den_levels;
+        it.n = (unsigned long long)1 << t.log;
+        it.kind = (uint32_t)t.kind;
+        items.push_back(it);
+    }
+    std::vector<uint32_t> tops(zk::GKR_TOP_WORDS * items.size()), results;
+    if (!items.empty()) d.check(zk::gkr_batch_towers(d.ctx(), items.data(), (int)items.size(), tops.data()));
+    hc.reset();
+    auto q_at = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
+
+    // claims and masks: num, den of a fraction (2 columns), or the product (1); column c of a mask is (v[2c], v[2c+1])
+    struct Claim { uint32_t n_cols = 0; qm31 v[2]; };
+    struct MaskRec { uint32_t n_cols; qm31 v[4]; };
     std::vector<std::vector<UniPoly>> sumcheck_round_polys;
-    struct MaskRec { uint32_t n_cols; qm31 v[4]; };  // column c is (v[2c], v[2c+1])
     std::vector<std::vector<MaskRec>> masks_by_inst(n_inst);
-    for (size_t i = 0; i < n_inst; i++) masks_by_inst[i].reserve(n_layers_by_inst[i]);
-    std::vector<std::vector<qm31>> output_claims(n_inst), claims(n_inst);
-    std::vector<bool> active(n_inst, false);
+    for (size_t i = 0; i < n_inst; i++) masks_by_inst[i].reserve((size_t)towers[i].log);
+    std::vector<Claim> output_claims(n_inst), claims(n_inst);
     std::vector<qm31> ood_point;
 
-    auto take = [&](size_t i) { Layer l = std::move(towers[i].back()); towers[i].pop_back(); return l; };
-    for (size_t layer = 0; layer < n_layers; layer++) {
-        size_t n_remaining = n_layers - layer;
-        for (size_t i = 0; i < n_inst; i++)
-            if (n_layers_by_inst[i] == n_remaining) {
-                Layer out = take(i);  // output layer: one entry per column
-                std::vector<qm31> vals;
-                const bool planned = top_slot[i] != SIZE_MAX;
-                qm31 den0 = planned ? top_q(top_slot[i]) : mle_to_cpu(d, out.den)[0];
-                if (out.kind == ZKB_GKR_GRAND_PRODUCT) vals = {den0};
-                else if (out.kind == ZKB_GKR_LOGUP_GENERIC) vals = {planned ? top_q(top_slot[i] + 4) : mle_to_cpu(d, out.num)[0], den0};
-                else if (out.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) vals = {qm31_from_m31(out.num_base.to_cpu()[0]), den0};
-                else vals = {qm31_one(), den0};
-                claims[i] = vals;
-                output_claims[i] = vals;
-                active[i] = true;
-            }
-        for (size_t i = 0; i < n_inst; i++)
-            if (active[i]) ch.mix_felts(claims[i]);
+    // Whether the transcript of a layer's rounds stays on the device (gkr_batch_layer_begin; ZKB_GKR_ROUNDS=host: never). The layer's
+    // description is staged as one block (an item per oracle and active round, 64 bytes each, and some 52 bytes per oracle): a batch of
+    // thousands of tall instances would not fit the staging ring and takes the round-by-round path, which stages one round's items at a time.
+    const char* rounds_env = getenv("ZKB_GKR_ROUNDS");
+    const bool never = host_rounds_only || (rounds_env && !strcmp(rounds_env, "host"));
+    auto on_device = [&](const zk::GkrLayerPlan& p) {
+        return !never && p.n_rounds > 0 && p.n_rounds <= zk::GKR_LAYER_MAX_ROUNDS &&
+               64 * p.items.size() + 64 * p.n_vars.size() + 256 * (size_t)p.n_rounds + 8192 <= ((size_t)2 << 20);
+    };
+    // A layer's tables depend on the towers' sizes only: they are made and staged while the layer before runs.
+    zk::GkrLayerPlan plan, next_plan;
+    std::vector<size_t> inst, next_inst;
+    auto make_next = [&](int layer) {
+        HostClock hc_plan("gkr.layer.plan");
+        plan_layer(towers, n_layers - layer - 1, layer, next_plan, next_inst);
+        if (on_device(next_plan)) d.check(zk::gkr_batch_plan(d.ctx(), next_plan));
+    };
+    if (n_layers) make_next(0);
+    std::vector<qm31> alpha_pow, sc_claims;
+    std::vector<zk::GkrRoundConst> consts;
+    std::vector<uint32_t> mask_words;
+    for (int layer = 0; layer < n_layers; layer++) {
+        std::swap(plan, next_plan);
+        std::swap(inst, next_inst);
+        const int n_remaining = n_layers - layer, level = n_remaining - 1, nv = layer;
+        const size_t K = inst.size();
         // EqEvals::generate, :235-247
-        std::unique_ptr<HostClock> hc_eq(new HostClock("gkr.layer.eq_evals"));
+        hc.reset(new HostClock("gkr.layer.eq_evals"));
         SecureMle eq_evals;
         if (ood_point.empty()) eq_evals = B200Backend::gen_eq_evals(d, {}, qm31_one());
         else eq_evals = B200Backend::gen_eq_evals(d, std::vector<qm31>(ood_point.begin() + 1, ood_point.end()), eq1(qm31_zero(), ood_point[0]));
-        hc_eq.reset();
-        qm31 sumcheck_alpha = ch.draw_secure_felt();
-        qm31 lambda = ch.draw_secure_felt();
-        std::vector<GkrOracle> oracles;
-        std::vector<qm31> sc_claims;
-        std::vector<size_t> sc_inst;
-        for (size_t i = 0; i < n_inst; i++)
-            if (active[i]) {
-                oracles.push_back({take(i), qm31_one(), false, {}});
-                sc_claims.push_back(horner(claims[i], lambda));
-                sc_inst.push_back(i);
+        hc.reset(new HostClock("gkr.layer.claims"));
+        for (size_t i : inst) {
+            if (towers[i].log == n_remaining) {  // its output layer: one entry per column
+                const uint32_t* w = tops.data() + top_of[i];
+                Claim& c = claims[i];
+                if (towers[i].kind == ZKB_GKR_GRAND_PRODUCT) { c.n_cols = 1; c.v[0] = q_at(w); }
+                else { c.n_cols = 2; c.v[0] = q_at(w + 4); c.v[1] = q_at(w); }
+                output_claims[i] = c;
             }
-        size_t nv = 0;
-        for (auto& o : oracles) nv = std::max(nv, o.n_variables());
-        for (size_t k = 0; k < oracles.size(); k++) sc_claims[k] = qm31_mul_m31(sc_claims[k], 1u << (nv - oracles[k].n_variables()));
+            ch.mix_felts(claims[i].v, claims[i].n_cols);
+        }
+        const qm31 sumcheck_alpha = ch.draw_secure_felt();
+        const qm31 lambda = ch.draw_secure_felt();
+        alpha_pow.resize(K);
+        sc_claims.resize(K);
+        for (size_t k = 0; k < K; k++) {
+            const Claim& c = claims[inst[k]];
+            alpha_pow[k] = k ? alpha_pow[k - 1] * sumcheck_alpha : qm31_one();
+            sc_claims[k] = qm31_mul_m31(c.n_cols == 1 ? c.v[0] : c.v[0] + lambda * c.v[1], 1u << (nv - (int)plan.n_vars[k]));
+        }
         std::vector<UniPoly> round_polys;
         std::vector<qm31> assignment;
-        const uint32_t half = m31_inv(2);
-        // By default the whole sum-check of the layer is enqueued at once and the transcript of its rounds stays on the
-        // device (gkr_batch_layer); ZKB_GKR_ROUNDS=host keeps the channel on the host and returns to it every round, and
-        // ZKB_GKR_ROUNDS=launches keeps a launch per round also for the small rounds (both for comparison and tests).
-        const char* rounds_env = getenv("ZKB_GKR_ROUNDS");
-        bool host_rounds = host_rounds_only || (rounds_env && !strcmp(rounds_env, "host"));
-        {
-            // The layer's description is staged as one block (an item per oracle and active round, 64 bytes each, and some
-            // 52 bytes per oracle): a batch of thousands of tall instances would not fit the staging ring and takes
-            // the round-by-round path, which stages one round's items at a time.
-            size_t items = 0;
-            for (auto& o : oracles) items += o.n_variables() + 1;
-            if (64 * items + 64 * oracles.size() + 256 * nv + 8192 > ((size_t)2 << 20) || nv > (size_t)zk::GKR_LAYER_MAX_ROUNDS) host_rounds = true;
-        }
-        if (nv > 0 && !host_rounds) {
-            std::unique_ptr<HostClock> hc(new HostClock("gkr.layer.plan"));
-            const size_t K = oracles.size();
-            std::vector<uint32_t> n_vars(K);
-            std::vector<qm31> alpha_pow(K);
-            for (size_t k = 0; k < K; k++) {
-                n_vars[k] = (uint32_t)oracles[k].n_variables();
-                alpha_pow[k] = k ? alpha_pow[k - 1] * sumcheck_alpha : qm31_one();
-            }
-            std::vector<std::vector<zk::GkrBatchItem>> first(nv), fix(nv);
-            std::vector<zk::GkrLayerRound> plan(nv);
-            std::vector<Layer> retired;  // layers replaced by their fixed copies: alive until the enqueued launches have read them
-            for (size_t round = 0; round < nv; round++) {
-                const size_t n_rem = nv - round;
+        const uint32_t* masks_at = nullptr;  // GKR_LAYER_MASK_WORDS per oracle that had a round
+        if (on_device(plan)) {
+            hc.reset(new HostClock("gkr.layer.begin"));
+            consts.resize((size_t)nv);
+            for (int round = 0; round < nv; round++) {
+                const size_t n_rem = (size_t)(nv - round);
                 const RoundBasis basis(ood_point, n_rem);
-                zk::GkrRoundConst& rc = plan[round].rc;
+                zk::GkrRoundConst& rc = consts[round];
                 memset(&rc, 0, sizeof(rc));
                 memcpy(rc.e0a, basis.e0a.c, 16);
                 memcpy(rc.e2a, basis.e2a.c, 16);
@@ -1302,276 +1393,83 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, std::
                     for (int t = 0; t < 4; t++) memcpy(rc.L[i][t], basis.L[i][t].c, 16);
                 memcpy(rc.y, ood_point[ood_point.size() - n_rem].c, 16);
                 rc.n_rem = (uint32_t)n_rem;
-                for (size_t k = 0; k < K; k++) {
-                    GkrOracle& o = oracles[k];
-                    if (n_rem != o.n_variables() || o.n_variables() == 0) continue;
-                    Layer& in = o.input_layer;
-                    if (n_vars[k] == n_rem) {  // enters in this round: its first sums
-                        zk::GkrBatchItem it{};
-                        it.num = in.num_ptr();
-                        it.den = in.den.words.ptr();
-                        it.n = in.len();
-                        it.kind = (uint32_t)in.kind;
-                        it.mode = 0;
-                        it.slot = k;
-                        first[round].push_back(it);
-                    }
-                    Layer out;  // Layer::fix_first_variable, gkr_prover.rs:354-381
-                    out.writable = true;
-                    out.kind = in.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? ZKB_GKR_LOGUP_GENERIC : in.kind;
-                    const uint32_t mode = in.len() >= 8 ? 1 : 2;
-                    if (in.writable && in.kind != ZKB_GKR_LOGUP_MULTIPLICITIES) {
-                        // in place: the result is the first half of the layer (see the host-round path below)
-                        out.den.words = BaseColumn::view(d, in.den.words.ptr(), in.den.words.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) out.num.words = BaseColumn::view(d, in.num.words.ptr(), in.num.words.len() / 2);
-                        zk::GkrBatchItem it = item_of(in, out, mode);
-                        it.slot = k;
-                        fix[round].push_back(it);
-                        in.den.words.shrink(in.den.words.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) in.num.words.shrink(in.num.words.len() / 2);
-                    } else {
-                        out.den = SecureMle(d, in.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) out.num = SecureMle(d, in.len() / 2);
-                        zk::GkrBatchItem it = item_of(in, out, mode);
-                        it.slot = k;
-                        fix[round].push_back(it);
-                        retired.push_back(std::move(in));
-                        in = std::move(out);
-                    }
-                }
-                plan[round].first = first[round].data();
-                plan[round].n_first = (int)first[round].size();
-                plan[round].fix = fix[round].data();
-                plan[round].n_fix = (int)fix[round].size();
             }
-            hc.reset(new HostClock("gkr.layer.rounds"));
             uint32_t chan[9];
             memcpy(chan, ch.digest().data(), 32);
             chan[8] = ch.n_draws();
-            std::vector<uint32_t> out_words(zk::GKR_LAYER_OUT_WORDS * nv), res(zk::GKR_LAYER_MASK_WORDS * K);
-            d.check(zk::gkr_batch_layer(d.ctx(), (int)K, n_vars.data(), alpha_pow[0].c, sc_claims[0].c, plan.data(), (int)nv, eq_evals.words.ptr(),
-                                        lambda.c, chan, out_words.data(), res.data(), degenerate));
-            retired.clear();
-            if (*degenerate) return {};
-            HashWords digest;
-            memcpy(digest.data(), chan, 32);
-            ch.set_state(digest, chan[8]);
-            for (size_t round = 0; round < nv; round++) {
-                const uint32_t* w = out_words.data() + zk::GKR_LAYER_OUT_WORDS * round;
-                UniPoly rp;
-                for (uint32_t t = 0; t < w[16] && t < 4; t++) rp.c.push_back(qm31{{w[4 * t], w[4 * t + 1], w[4 * t + 2], w[4 * t + 3]}});
-                round_polys.push_back(std::move(rp));
-                assignment.push_back(qm31{{w[20], w[21], w[22], w[23]}});
-            }
-            for (size_t k = 0; k < K; k++) {
-                if (n_vars[k] == 0) continue;  // no round, no mask from a launch: read with the others below
-                GkrOracle& o = oracles[k];
-                const uint32_t* w = res.data() + zk::GKR_LAYER_MASK_WORDS * k;
-                for (int e = 0; e < 2; e++) {
-                    o.mask_den[e] = qm31{{w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]}};
-                    o.mask_num[e] = qm31{{w[8 + 4 * e], w[9 + 4 * e], w[10 + 4 * e], w[11 + 4 * e]}};
-                }
-                o.have_mask = true;
-            }
-        }
-        for (size_t round = 0; host_rounds && round < nv; round++) {
-            size_t n_rem = nv - round;
-            // the oracles that enter the sum-check in this round have no sums yet: one launch for all of them
-            std::unique_ptr<HostClock> hc(new HostClock("gkr.round.first_sums"));
-            items.clear();
-            std::vector<size_t> who;
-            for (size_t k = 0; k < oracles.size(); k++)
-                if (n_rem == oracles[k].n_variables() && !oracles[k].have_sums) {
-                    zk::GkrBatchItem it{};
-                    it.num = oracles[k].input_layer.num_ptr();
-                    it.den = oracles[k].input_layer.den.words.ptr();
-                    it.n = oracles[k].input_layer.len();
-                    it.kind = (uint32_t)oracles[k].input_layer.kind;
-                    it.mode = 0;
-                    items.push_back(it);
-                    who.push_back(k);
-                }
-            if (!items.empty()) {
-                results.resize(items.size() * zk::GKR_BATCH_RESULT_WORDS);
-                qm31 zero = qm31_zero();
-                d.check(zk::gkr_batch_round(d.ctx(), items.data(), (int)items.size(), zero.c, eq_evals.words.ptr(), lambda.c, results.data()));
-                for (size_t j = 0; j < who.size(); j++) {
-                    const uint32_t* w = results.data() + j * zk::GKR_BATCH_RESULT_WORDS;
-                    oracles[who[j]].sums = {qm31{{w[0], w[1], w[2], w[3]}}, qm31{{w[4], w[5], w[6], w[7]}}};
-                    oracles[who[j]].have_sums = true;
-                }
-            }
-            // Every active oracle has n_rem variables left, so all their round polynomials are r0 L0 + r1 L1 + r2 L2 over the
-            // same basis, and the random linear combination over the batch (sumcheck.rs:139-149, Horner in alpha from the
-            // last oracle down) is (sum alpha^k r0_k) L0 + (sum alpha^k r1_k) L1 + (sum alpha^k r2_k) L2 plus the constants of
-            // the oracles that wait: eleven multiplications per oracle and round instead of a Lagrange interpolation each.
-            // r0 + r1 is the claim by construction, which is the check sumcheck.rs:128-130 makes.
-            hc.reset(new HostClock("gkr.round.algebra"));
-            const RoundBasis basis(ood_point, n_rem);
-            const size_t K = oracles.size();
-            std::vector<qm31> rv(3 * K);
-            std::vector<char> act(K);
-            qm31 S[3] = {qm31_zero(), qm31_zero(), qm31_zero()}, Sc = qm31_zero();
-            for (size_t k = K; k-- > 0;) {
-                for (int t = 0; t < 3; t++) S[t] = S[t] * sumcheck_alpha;
-                Sc = Sc * sumcheck_alpha;
-                act[k] = n_rem == oracles[k].n_variables();
-                if (act[k]) {
-                    const qm31 corr = oracles[k].eq_fixed_var_correction;
-                    rv[3 * k] = oracles[k].sums.first * corr * basis.e0a;
-                    rv[3 * k + 1] = sc_claims[k] - rv[3 * k];
-                    rv[3 * k + 2] = oracles[k].sums.second * corr * basis.e2a;
-                    oracles[k].have_sums = false;
-                    for (int t = 0; t < 3; t++) S[t] = S[t] + rv[3 * k + t];
-                } else {
-                    rv[3 * k] = qm31_mul_m31(sc_claims[k], half);
-                    Sc = Sc + rv[3 * k];
-                }
-            }
-            UniPoly combined;
-            combined.c.resize(4);
-            for (int t = 0; t < 4; t++) combined.c[t] = S[0] * basis.L[0][t] + S[1] * basis.L[1][t] + S[2] * basis.L[2][t];
-            combined.c[0] = combined.c[0] + Sc;
-            if (qm31_is_zero(combined.c[3])) {
-                // The combination keeps the length of its longest term. A vanishing leading coefficient does not say which
-                // case this is (every term short, or a cancellation), so this round goes term by term.
-                combined = UniPoly();
-                for (size_t k = K; k-- > 0;) {
-                    UniPoly rp;
-                    if (act[k]) rp = basis.round_poly(rv[3 * k], rv[3 * k + 1], rv[3 * k + 2]);
-                    else { rp.c = {rv[3 * k]}; rp.trim(); }
-                    for (auto& c : combined.c) c = c * sumcheck_alpha;
-                    combined = UniPoly::add(combined, rp);
-                }
-            }
-            hc.reset(new HostClock("gkr.round.channel"));
-            ch.mix_felts(combined.c);
-            qm31 challenge = ch.draw_secure_felt();
-            hc.reset(new HostClock("gkr.round.claims"));
-            qm31 Lc[3];
-            for (int t = 0; t < 3; t++) Lc[t] = ((basis.L[t][3] * challenge + basis.L[t][2]) * challenge + basis.L[t][1]) * challenge + basis.L[t][0];
-            for (size_t k = 0; k < K; k++)
-                sc_claims[k] = act[k] ? rv[3 * k] * Lc[0] + rv[3 * k + 1] * Lc[1] + rv[3 * k + 2] * Lc[2] : rv[3 * k];
-            const qm31 eq_step = eq1(challenge, ood_point[ood_point.size() - n_rem]);  // the same for every active oracle
-            // fix the first variable of every active oracle (and take the next round's sums in the same pass): one launch
-            hc.reset(new HostClock("gkr.round.fix_prepare"));
-            items.clear();
-            who.clear();
-            std::vector<Layer> fixed;
-            for (size_t k = 0; k < oracles.size(); k++)
-                if (n_rem == oracles[k].n_variables() && oracles[k].n_variables() != 0) {
-                    oracles[k].eq_fixed_var_correction = oracles[k].eq_fixed_var_correction * eq_step;
-                    Layer& in = oracles[k].input_layer;
-                    Layer out;  // Layer::fix_first_variable, gkr_prover.rs:354-381
-                    out.writable = true;
-                    out.kind = in.kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? ZKB_GKR_LOGUP_GENERIC : in.kind;
-                    if (in.writable && in.kind != ZKB_GKR_LOGUP_MULTIPLICITIES) {
-                        // A thread of the fixing kernel reads entries i and i + n/2 and writes entry i, and no other thread
-                        // touches either: the prover's own layers are fixed in place, the result being their first half.
-                        out.den.words = BaseColumn::view(d, in.den.words.ptr(), in.den.words.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) out.num.words = BaseColumn::view(d, in.num.words.ptr(), in.num.words.len() / 2);
-                        items.push_back(item_of(in, out, in.len() >= 8 ? 1 : 2));
-                        // keep the allocation alive under its new, shorter shape
-                        in.den.words.shrink(in.den.words.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) in.num.words.shrink(in.num.words.len() / 2);
-                        out = std::move(in);
-                        out.writable = true;
-                    } else {
-                        out.den = SecureMle(d, in.len() / 2);
-                        if (out.kind == ZKB_GKR_LOGUP_GENERIC) out.num = SecureMle(d, in.len() / 2);
-                        items.push_back(item_of(in, out, in.len() >= 8 ? 1 : 2));
-                    }
-                    fixed.push_back(std::move(out));
-                    who.push_back(k);
-                }
-            if (!items.empty()) {
-                hc.reset(new HostClock("gkr.round.fix_launch_wait"));
-                results.resize(items.size() * zk::GKR_BATCH_RESULT_WORDS);
-                d.check(zk::gkr_batch_round(d.ctx(), items.data(), (int)items.size(), challenge.c, eq_evals.words.ptr(), lambda.c, results.data()));
-                hc.reset(new HostClock("gkr.round.fix_results"));
-                for (size_t j = 0; j < who.size(); j++) {
-                    GkrOracle& o = oracles[who[j]];
-                    const uint32_t* w = results.data() + j * zk::GKR_BATCH_RESULT_WORDS;
-                    if (items[j].mode == 1) {
-                        o.sums = {qm31{{w[0], w[1], w[2], w[3]}}, qm31{{w[4], w[5], w[6], w[7]}}};
-                        o.have_sums = true;
-                    } else {
-                        for (int e = 0; e < 2; e++) {
-                            o.mask_den[e] = qm31{{w[8 + 4 * e], w[9 + 4 * e], w[10 + 4 * e], w[11 + 4 * e]}};
-                            o.mask_num[e] = qm31{{w[16 + 4 * e], w[17 + 4 * e], w[18 + 4 * e], w[19 + 4 * e]}};
-                        }
-                        o.have_mask = true;
-                    }
-                    o.input_layer = std::move(fixed[j]);
-                }
-            }
+            d.check(zk::gkr_batch_layer_begin(d.ctx(), plan, alpha_pow[0].c, sc_claims[0].c, consts.data(), eq_evals.words.ptr(), lambda.c, chan));
             hc.reset();
-            round_polys.push_back(combined);
-            assignment.push_back(challenge);
+            if (layer + 1 < n_layers) make_next(layer + 1);
+            hc.reset(new HostClock("gkr.layer.wait"));
+            zk::GkrLayerResult res;
+            d.check(zk::gkr_batch_layer_end(d.ctx(), plan, res));
+            if (res.degenerate) { *degenerate = true; return {}; }
+            HashWords digest;
+            memcpy(digest.data(), res.channel, 32);
+            ch.set_state(digest, res.channel[8]);
+            for (int round = 0; round < nv; round++) {
+                const uint32_t* w = res.records + zk::GKR_LAYER_OUT_WORDS * (size_t)round;
+                UniPoly rp;
+                for (uint32_t t = 0; t < w[16] && t < 4; t++) rp.c.push_back(q_at(w + 4 * t));
+                round_polys.push_back(std::move(rp));
+                assignment.push_back(q_at(w + 20));
+            }
+            masks_at = res.masks;
+        } else {
+            if (nv > 0) host_rounds(d, ch, plan, sumcheck_alpha, lambda, ood_point, eq_evals, sc_claims, round_polys, assignment, mask_words);
+            masks_at = mask_words.data();
+            if (layer + 1 < n_layers) make_next(layer + 1);
         }
-        HostClock hc_masks("gkr.layer.masks");
-        sumcheck_round_polys.push_back(round_polys);
-        // try_into_mask, :572-597. A mask is one column pair (grand product) or two (numerators, denominators): kept as flat
-        // records; a batch has hundreds of oracles per layer, and a vector of vectors per oracle cost more than the hashing.
-        std::vector<MaskRec> masks(oracles.size());
-        // An oracle that entered this layer with two entries had no sum-check round, so no launch has returned its mask:
-        // those (every instance once, in the layer above its output) are read in one gather, not one copy per column.
-        GatherPlan mask_plan;
-        std::vector<size_t> mask_slot(oracles.size(), SIZE_MAX);
-        for (size_t k = 0; k < oracles.size(); k++) {
-            const GkrOracle& o = oracles[k];
-            if (o.have_mask || o.input_layer.len() != 2) continue;
-            mask_slot[k] = mask_plan.addrs.size();
-            for (int w = 0; w < 8; w++) mask_plan.add(o.input_layer.den.words.ptr() + w);
-            if (o.input_layer.kind == ZKB_GKR_LOGUP_GENERIC)
-                for (int w = 0; w < 8; w++) mask_plan.add(o.input_layer.num.words.ptr() + w);
+        hc.reset(new HostClock("gkr.layer.masks"));
+        sumcheck_round_polys.push_back(std::move(round_polys));
+        // try_into_mask, :572-597. An oracle that entered with two entries had no sum-check round: its mask came with the towers.
+        for (size_t k = 0; k < K; k++) {
+            const size_t i = inst[k];
+            const bool had_round = plan.n_vars[k] > 0;
+            const uint32_t* w = had_round ? masks_at + zk::GKR_LAYER_MASK_WORDS * k : tops.data() + top_of[i] + 8;
+            const int kind = towers[i].kind_at(level);
+            MaskRec m;
+            if (kind == ZKB_GKR_GRAND_PRODUCT) { m.n_cols = 1; m.v[0] = q_at(w); m.v[1] = q_at(w + 4); }
+            else {
+                if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES && !had_round) throw Error(ZKB_EINVAL, "gkr: a multiplicities layer cannot be a mask");
+                m.n_cols = 2;
+                m.v[0] = kind == ZKB_GKR_LOGUP_SINGLES ? qm31_one() : q_at(w + 8);
+                m.v[1] = kind == ZKB_GKR_LOGUP_SINGLES ? qm31_one() : q_at(w + 12);
+                m.v[2] = q_at(w);
+                m.v[3] = q_at(w + 4);
+            }
+            ch.mix_felts(m.v, 2 * m.n_cols);
+            masks_by_inst[i].push_back(m);
         }
-        if (!mask_plan.addrs.empty()) mask_plan.execute(d);
-        auto gathered = [&](size_t slot) { return qm31{{mask_plan.words[slot], mask_plan.words[slot + 1], mask_plan.words[slot + 2], mask_plan.words[slot + 3]}}; };
-        for (size_t k = 0; k < oracles.size(); k++) {
-            const GkrOracle& o = oracles[k];
-            const Layer& l = o.input_layer;
-            if (l.len() != 2) throw Error(ZKB_EINVAL, "gkr: oracle is not constant after sumcheck");
-            MaskRec& m = masks[k];
-            qm31 den[2], num[2];
-            if (o.have_mask) { den[0] = o.mask_den[0]; den[1] = o.mask_den[1]; }
-            else { den[0] = gathered(mask_slot[k]); den[1] = gathered(mask_slot[k] + 4); }
-            if (l.kind == ZKB_GKR_GRAND_PRODUCT) { m.n_cols = 1; m.v[0] = den[0]; m.v[1] = den[1]; continue; }
-            if (l.kind == ZKB_GKR_LOGUP_GENERIC) {
-                if (o.have_mask) { num[0] = o.mask_num[0]; num[1] = o.mask_num[1]; }
-                else { num[0] = gathered(mask_slot[k] + 8); num[1] = gathered(mask_slot[k] + 12); }
-            } else if (l.kind == ZKB_GKR_LOGUP_SINGLES) num[0] = num[1] = qm31_one();
-            else throw Error(ZKB_EINVAL, "gkr: a multiplicities layer cannot be a mask");
-            m.n_cols = 2; m.v[0] = num[0]; m.v[1] = num[1]; m.v[2] = den[0]; m.v[3] = den[1];
-        }
-        for (size_t k = 0; k < oracles.size(); k++) {
-            ch.mix_felts(masks[k].v, 2 * masks[k].n_cols);
-            masks_by_inst[sc_inst[k]].push_back(masks[k]);
-        }
-        qm31 challenge = ch.draw_secure_felt();
-        ood_point = assignment;
+        const qm31 challenge = ch.draw_secure_felt();
+        ood_point = std::move(assignment);
         ood_point.push_back(challenge);
-        for (size_t k = 0; k < oracles.size(); k++) {
-            std::vector<qm31>& next = claims[sc_inst[k]];
-            next.resize(masks[k].n_cols);
-            for (uint32_t c = 0; c < masks[k].n_cols; c++) next[c] = challenge * (masks[k].v[2 * c + 1] - masks[k].v[2 * c]) + masks[k].v[2 * c];
+        for (size_t i : inst) {
+            const MaskRec& m = masks_by_inst[i].back();
+            claims[i].n_cols = m.n_cols;
+            for (uint32_t c = 0; c < m.n_cols; c++) claims[i].v[c] = challenge * (m.v[2 * c + 1] - m.v[2 * c]) + m.v[2 * c];
         }
+        hc.reset();
     }
     std::vector<uint32_t> o;
-    auto put = [&](qm31 q) { o.insert(o.end(), q.c, q.c + 4); };
+    size_t room = 16 + 4 * (ood_point.size() + 1) + 32 * n_inst;
+    for (auto& l : sumcheck_round_polys) room += 1 + 17 * l.size();
+    for (auto& m : masks_by_inst) room += 17 * m.size();
+    o.reserve(room);
+    auto put = [&](const qm31* q, size_t n) { for (size_t k = 0; k < n; k++) o.insert(o.end(), q[k].c, q[k].c + 4); };
     o.push_back((uint32_t)sumcheck_round_polys.size());
     for (auto& l : sumcheck_round_polys) {
         o.push_back((uint32_t)l.size());
-        for (auto& p : l) { o.push_back((uint32_t)p.c.size()); for (auto q : p.c) put(q); }
+        for (auto& p : l) { o.push_back((uint32_t)p.c.size()); put(p.c.data(), p.c.size()); }
     }
-    for (auto& inst : masks_by_inst) {
-        o.push_back((uint32_t)inst.size());
-        for (auto& m : inst) { o.push_back(m.n_cols); for (uint32_t c = 0; c < 2 * m.n_cols; c++) put(m.v[c]); }
+    for (auto& of : masks_by_inst) {
+        o.push_back((uint32_t)of.size());
+        for (auto& m : of) { o.push_back(m.n_cols); put(m.v, 2 * m.n_cols); }
     }
-    for (auto& c : output_claims) { o.push_back((uint32_t)c.size()); for (auto q : c) put(q); }
+    for (auto& c : output_claims) { o.push_back(c.n_cols); put(c.v, c.n_cols); }
     o.push_back((uint32_t)ood_point.size());
-    for (auto q : ood_point) put(q);
-    for (auto& c : claims) { o.push_back((uint32_t)c.size()); for (auto q : c) put(q); }
+    put(ood_point.data(), ood_point.size());
+    for (auto& c : claims) { o.push_back(c.n_cols); put(c.v, c.n_cols); }
     return o;
 }
 
