@@ -1,6 +1,8 @@
 """Proofs at the sizes where the library changes how it runs them, word for word against the oracle: FRI layers that fit the
 one-launch tail (2^10 values) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
-the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit."""
+the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit;
+batches whose towers take one launch (2^10 entries) and two; samples whose quotient lines are worked out on the host and on the
+device (from 512 on, in pieces of 1,024)."""
 import pytest
 
 from util import m31_column, qm31_array
@@ -35,4 +37,29 @@ def test_gkr_single_instance_around_the_chain(ctx, oracle, kind, log_n):
     want = oracle.gkr_prove([(kind, num, den)], 0x5EED0004, verify=True)
     nb, db = ctx.upload(num) if num is not None else None, ctx.upload(den)
     got = ctx.gkr_prove_device([(kind, nb.ptr if nb else 0, db.ptr, n)], 0x5EED0004)
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("log_n", [2, 9, 10, 11, 12])
+def test_gkr_batch_around_the_tower_launches(ctx, oracle, log_n):
+    inst, dev, keep = [], [], []
+    for k, kind in enumerate([0, 3, 1, 2, 0, 3, 1]):  # more than the driver of a few instances takes
+        n = 1 << max(1 + (kind == 2), log_n - k // 4 * (log_n - 1))
+        den = qm31_array(7300 + 10 * log_n + k, n, nonzero=True)
+        num = qm31_array(7400 + 10 * log_n + k, n) if kind == 1 else m31_column(7500 + 10 * log_n + k, n) if kind == 2 else None
+        inst.append((kind, num, den))
+        keep.append((ctx.upload(num) if num is not None else None, ctx.upload(den)))
+        dev.append((kind, keep[-1][0].ptr if keep[-1][0] else 0, keep[-1][1].ptr, n))
+    want = oracle.gkr_prove(inst, 0x5EED0005, verify=True)
+    got = ctx.gkr_prove_device(dev, 0x5EED0005)
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("n_cols", [382, 383, 2200])
+def test_pcs_proof_around_the_line_kernel(ctx, oracle, n_cols):
+    # 511, 512 entries (a column with two samples has three); more than 1,024 of a size; the last tree holds the tallest column
+    trees = [[m31_column(6500 + c, 1 << (3 if c % 2 else 4)) for c in range(n_cols)], [m31_column(6400, 1 << 5)]]
+    kw = dict(pow_bits=0, log_blowup=1, log_last_layer=0, n_queries=3, two_sample_every=6)
+    want = oracle.pcs_prove(trees, **kw)
+    got = ctx.pcs_prove_host(trees, **kw)
     assert len(got) == len(want) and (got == want).all()

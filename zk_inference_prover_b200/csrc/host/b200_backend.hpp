@@ -67,6 +67,12 @@ class BaseColumn {
         c.dev_ = &d; c.ptr_ = ptr; c.len_ = len; c.owned_ = false;
         return c;
     }
+    // A block of the context's memory that an operator allocated: freed with the object.
+    static BaseColumn adopt(const Device& d, uint32_t* ptr) {
+        BaseColumn c = view(d, ptr, 0);
+        c.owned_ = true;
+        return c;
+    }
     BaseColumn(BaseColumn&& o) noexcept { *this = std::move(o); }
     BaseColumn& operator=(BaseColumn&& o) noexcept {
         if (this != &o) {

@@ -26,6 +26,7 @@
 #include "../fri_tail.hpp"
 #include "../gather_blocks.hpp"
 #include "channel.hpp"
+#include "../quot_lines.hpp"
 
 // Records a message on the context (defined with the context, ctx.cu).
 extern "C" int zk_set_error_public(zkb_ctx* ctx, int code, const char* msg);
@@ -82,7 +83,7 @@ struct GatherPlan {
     size_t add_hash(const uint32_t* p) { hash_addrs.push_back(p); return hash_addrs.size() - 1; }
     // Rows of many columns at once (the queried and witness values of one tree layer): row-major [row][column] in
     // block_words from the returned offset. One pointer per column and one index per row travel, not one address per word.
-    struct Block { std::vector<const uint32_t*> cols; std::vector<uint32_t> idx; size_t out_off; };
+    struct Block { const std::vector<const uint32_t*>* cols; std::vector<uint32_t> idx; size_t out_off; };  // cols: its owner outlives the plan
     std::vector<Block> blocks;
     // Tens of megabytes for trees of many columns. The buffer is kept per thread between proofs: a fresh allocation of
     // that size comes from mmap, and its first-touch page faults cost as much as the gather itself.
@@ -117,7 +118,8 @@ struct GatherPlan {
     }
     size_t add_block(const std::vector<const uint32_t*>& cols, const std::vector<size_t>& rows) {
         Block b;
-        b.cols = cols;
+        b.cols = &cols;
+        b.idx.reserve(rows.size());
         for (auto r : rows) b.idx.push_back((uint32_t)r);
         b.out_off = block_total;
         block_total += cols.size() * rows.size();
@@ -129,7 +131,7 @@ struct GatherPlan {
         uint32_t* out = arena(block_total + n + 8 * nh);
         std::vector<zk::GatherBlock> gb;
         gb.reserve(blocks.size());
-        for (auto& b : blocks) gb.push_back({b.cols.data(), (int)b.cols.size(), b.idx.data(), (int)b.idx.size(), b.out_off});
+        for (auto& b : blocks) gb.push_back({b.cols->data(), (int)b.cols->size(), b.idx.data(), (int)b.idx.size(), b.out_off});
         d.check(zk::gather_plan(d.ctx(), gb.data(), (int)gb.size(), block_total, addrs.data(), n, hash_addrs.data(), nh, out));
         block_words = out;
         words.assign(out + block_total, out + block_total + n);
@@ -165,12 +167,18 @@ struct PendingMerkle {  // slots of a planned decommitment
     }
 };
 
+// Queries of one layer only.
+struct QueriesOf {
+    uint32_t log;
+    const std::vector<size_t>& positions;
+    const std::vector<size_t>& operator()(uint32_t l) const { static const std::vector<size_t> none; return l == log ? positions : none; }
+};
+
 struct MerkleProver {
     std::vector<HashColumn> layers;  // layers[log_size]; layers[0] holds the root
     // the committed columns of each layer (device addresses, in commitment order), kept for the decommitment: sorting tens
     // of thousands of columns by size a second time costs milliseconds
     std::vector<std::vector<const uint32_t*>> layer_col_ptrs;
-    size_t n_columns = 0;
 
     // `leaves`, when given, is the already hashed largest layer (see zkb_merkle_leaves_partial).
     // `chan_step`, when given, is a FRI layer's channel step (channel state, challenge slot, root copy; device addresses) to run
@@ -195,7 +203,6 @@ struct MerkleProver {
         uint32_t max_log = sorted[0]->log_size();
         mp.layers.resize(max_log + 1);
         mp.layer_col_ptrs.resize(max_log + 1);
-        mp.n_columns = sorted.size();
         size_t pos = 0;
         for (uint32_t log = max_log + 1; log-- > 0;) {
             std::vector<const BaseColumn*> layer_cols;
@@ -237,62 +244,46 @@ struct MerkleProver {
     mutable bool have_root = false;
 
     // :84-217 — the reference plans the indices of all layers on the host first (its phase 1) and then
-    // reads layer by layer; here the reads of all layers join one GatherPlan.
+    // reads layer by layer; here the reads of all layers join one GatherPlan, over the layers' columns as commit() recorded them.
+    // queries(log): the ascending distinct nodes queried of the layer of 2^log (rows of its columns).
     // `hashes_per_layer`, when given, receives the number of witness hashes each layer contributed (largest layer first).
-    PendingMerkle plan_decommit(GatherPlan& plan, const std::map<uint32_t, std::vector<size_t>>& queries_per_log_size,
-                                const std::vector<const BaseColumn*>& columns, std::vector<size_t>* hashes_per_layer = nullptr) const {
+    template <class Queries>
+    PendingMerkle plan_decommit(GatherPlan& plan, Queries queries, std::vector<size_t>* hashes_per_layer = nullptr) const {
         PendingMerkle pm;
-        // the layers' column lists as recorded by commit(); sorted again only for a tree that was not built there
-        const bool recorded = layer_col_ptrs.size() == layers.size() && n_columns == columns.size();
-        std::vector<const BaseColumn*> sorted;
-        if (!recorded) {
-            sorted = columns;
-            std::stable_sort(sorted.begin(), sorted.end(), [](const BaseColumn* a, const BaseColumn* b) { return a->len() > b->len(); });
-        }
-        size_t pos = 0;
-        std::vector<size_t> last;
+        static const std::vector<const uint32_t*> no_columns;
+        // Sorted vectors walked in step: `last` (the nodes of the layer below) is ascending, so are its halves and the layer's
+        // own queries; a FRI proof plans some twenty trees of some twenty layers each.
+        std::vector<size_t> last, nodes, order, witness_nodes;
         for (uint32_t log = (uint32_t)layers.size(); log-- > 0;) {
-            bool has_prev = (size_t)log + 1 < layers.size();
-            // Sorted vectors, not sets: `last` (the nodes of the layer below) is ascending, so are its halves and the layer's
-            // own queries; a FRI proof plans some twenty trees of some twenty layers each.
-            const std::vector<size_t>& prev_nodes = last;
-            std::vector<size_t> parents, col_queries, merged_nodes;
-            parents.reserve(last.size());
-            for (auto q : last)
-                if (parents.empty() || parents.back() != q / 2) parents.push_back(q / 2);
-            auto it = queries_per_log_size.find(log);
-            if (it != queries_per_log_size.end()) {
-                col_queries = it->second;
-                if (!std::is_sorted(col_queries.begin(), col_queries.end())) std::sort(col_queries.begin(), col_queries.end());
-                col_queries.erase(std::unique(col_queries.begin(), col_queries.end()), col_queries.end());
+            const bool has_prev = (size_t)log + 1 < layers.size();
+            const std::vector<const uint32_t*>& ptrs = log < layer_col_ptrs.size() ? layer_col_ptrs[log] : no_columns;
+            const std::vector<size_t>& col_queries = queries(log);
+            nodes.clear();
+            order.clear();
+            witness_nodes.clear();
+            size_t p = 0, q = 0, hashes = 0;
+            while (p < last.size() || q < col_queries.size()) {
+                const size_t node = p == last.size() ? col_queries[q] : q == col_queries.size() ? last[p] / 2 : std::min(last[p] / 2, col_queries[q]);
+                bool child[2] = {false, false};
+                for (; p < last.size() && last[p] / 2 == node; p++) child[last[p] & 1] = true;
+                const bool queried = q < col_queries.size() && col_queries[q] == node;
+                if (queried) q++;
+                if (has_prev)
+                    for (size_t k = 0; k < 2; k++)
+                        if (!child[k]) { pm.hash_slots.push_back(plan.add_hash(layers[log + 1].ptr() + 8 * (2 * node + k))); hashes++; }
+                nodes.push_back(node);
+                (queried ? order : witness_nodes).push_back(node);
             }
-            merged_nodes.reserve(parents.size() + col_queries.size());
-            std::set_union(parents.begin(), parents.end(), col_queries.begin(), col_queries.end(), std::back_inserter(merged_nodes));
-            auto in_prev = [&](size_t node) { return std::binary_search(prev_nodes.begin(), prev_nodes.end(), node); };
-            auto is_query = [&](size_t node) { return std::binary_search(col_queries.begin(), col_queries.end(), node); };
-            std::vector<const uint32_t*> layer_ptrs_own;
-            if (!recorded)
-                while (pos < sorted.size() && sorted[pos]->log_size() == log) layer_ptrs_own.push_back(sorted[pos++]->ptr());
-            const std::vector<const uint32_t*>& ptrs = recorded ? layer_col_ptrs[log] : layer_ptrs_own;
-            std::vector<size_t> witness_children, queried_nodes, witness_nodes;
-            for (size_t node : merged_nodes) {
-                if (has_prev) {
-                    if (!in_prev(2 * node)) witness_children.push_back(2 * node);
-                    if (!in_prev(2 * node + 1)) witness_children.push_back(2 * node + 1);
-                }
-                (is_query(node) ? queried_nodes : witness_nodes).push_back(node);
-            }
-            for (size_t child : witness_children) pm.hash_slots.push_back(plan.add_hash(layers[log + 1].ptr() + 8 * child));
-            if (hashes_per_layer) hashes_per_layer->push_back(witness_children.size());
-            if (!ptrs.empty() && !merged_nodes.empty()) {
+            if (hashes_per_layer) hashes_per_layer->push_back(hashes);
+            if (!ptrs.empty() && !nodes.empty()) {
                 // every node of the layer is read once; the proof lists the queried nodes' values first, then the witnesses'
-                std::vector<size_t> order(queried_nodes);
+                const size_t n_queried = order.size();
                 order.insert(order.end(), witness_nodes.begin(), witness_nodes.end());
-                size_t off = plan.add_block(ptrs, order);
-                if (!queried_nodes.empty()) pm.runs.push_back({off, queried_nodes.size() * ptrs.size(), true});
-                if (!witness_nodes.empty()) pm.runs.push_back({off + queried_nodes.size() * ptrs.size(), witness_nodes.size() * ptrs.size(), false});
+                const size_t off = plan.add_block(ptrs, order);
+                if (n_queried) pm.runs.push_back({off, n_queried * ptrs.size(), true});
+                if (!witness_nodes.empty()) pm.runs.push_back({off + n_queried * ptrs.size(), witness_nodes.size() * ptrs.size(), false});
             }
-            last = merged_nodes;
+            std::swap(last, nodes);
         }
         return pm;
     }
@@ -376,8 +367,7 @@ static PendingFriLayer plan_fri_layer(GatherPlan& plan, const Device& d, const S
     }
     for (size_t p : positions)
         for (int k = 0; k < 4; k++) pl.eval_slots.push_back(plan.add(column.columns[k].ptr() + p));
-    std::map<uint32_t, std::vector<size_t>> q{{column.columns[0].log_size(), positions}};
-    pl.merkle = tree.plan_decommit(plan, q, column.refs());
+    pl.merkle = tree.plan_decommit(plan, QueriesOf{column.columns[0].log_size(), positions});
     pl.commitment = tree.root(d);
     return pl;
 }
@@ -400,7 +390,6 @@ struct FriProver {
         for (uint32_t j = 0; j <= log; j++) mp.layers.push_back(HashColumn::view(d, tree + ((size_t)8 << j), (size_t)8 << j));
         mp.layer_col_ptrs.resize(log + 1);
         for (auto p : eval.cptrs()) mp.layer_col_ptrs[log].push_back(p);
-        mp.n_columns = 4;
         return mp;
     }
 
@@ -638,9 +627,30 @@ static bool point_less(const CirclePointQ& a, const CirclePointQ& b) {
     return false;
 }
 
+// The out-of-domain sample points of all columns, flat (a segment has tens of thousands of columns, most of them with one sample at
+// one of a handful of points: a vector a column is an allocation a column). Columns are numbered through the trees; column i has the
+// samples first[i] ... first[i + 1] - 1, sample s is at points[point_of[s]].
+struct SamplePoints {
+    std::vector<CirclePointQ> points;
+    std::vector<uint32_t> point_of;
+    std::vector<size_t> first{0};
+    uint32_t intern(const CirclePointQ& p) {
+        for (size_t k = 0; k < points.size(); k++) if (points[k] == p) return (uint32_t)k;
+        points.push_back(p);
+        return (uint32_t)(points.size() - 1);
+    }
+    void end_column() { first.push_back(point_of.size()); }
+};
+struct SampledValues {
+    std::vector<size_t> tree_first{0};  // the trees' first columns
+    std::vector<size_t> first{0};       // the columns' first values
+    std::vector<qm31> values;
+    const qm31* at(size_t tree, size_t column) const { return values.data() + first[tree_first[tree] + column]; }
+};
+
 struct PcsProof {
     std::vector<Hash> commitments;
-    std::vector<std::vector<std::vector<qm31>>> sampled_values;
+    SampledValues sampled_values;
     std::vector<MerkleDecommitment> decommitments;
     std::vector<Words> queried_values;
     uint64_t proof_of_work = 0;
@@ -694,15 +704,20 @@ struct PcsProof {
     }
     template <class O> void write(O& o) const {
         size_t expect = 1 << 16;
-        for (auto& t : sampled_values) expect += 6 * t.size();
+        expect += 4 * sampled_values.values.size() + 2 * sampled_values.first.size();
         for (auto& d : decommitments) expect += 8 * d.hash_witness.size() + d.column_witness.size();
         for (auto& t : queried_values) expect += t.size();
         o.reserve(expect);
         o.push_back((uint32_t)commitments.size());
         for (auto& h : commitments) put_hash(o, h);
-        for (auto& t : sampled_values) {
-            o.push_back((uint32_t)t.size());
-            for (auto& c : t) { o.push_back((uint32_t)c.size()); for (auto q : c) put_q(o, q); }
+        const SampledValues& sv = sampled_values;
+        for (size_t t = 0; t + 1 < sv.tree_first.size(); t++) {
+            o.push_back((uint32_t)(sv.tree_first[t + 1] - sv.tree_first[t]));
+            for (size_t c = sv.tree_first[t]; c < sv.tree_first[t + 1]; c++) {
+                const size_t n = sv.first[c + 1] - sv.first[c];
+                o.push_back((uint32_t)n);
+                if (n) o.insert(o.end(), sv.values[sv.first[c]].c, sv.values[sv.first[c]].c + 4 * n);
+            }
         }
         for (auto& d : decommitments) put_dec(o, d);
         for (auto& t : queried_values) { o.push_back((uint32_t)t.size()); t.append_to(o); }
@@ -813,94 +828,118 @@ struct CommitmentSchemeProver {
         trees.push_back(std::move(t));
     }
 
-    // pcs/quotient_ops.rs:73-194 with STWO/core/pcs/quotients.rs:306-345 and :75-104
-    SecureColumnByCoords compute_fri_quotients(const std::vector<std::vector<std::vector<PointSample>>>& samples, qm31 random_coeff,
-                                               uint32_t lifting_log) {
-        std::unique_ptr<HostClock> hc(new HostClock("pcs.quot.flatten"));
-        std::vector<const BaseColumn*> flat_cols;
-        std::vector<uint32_t> flat_logs;
-        size_t n_flat = 0;
-        for (auto& t : trees) n_flat += t.evals.size();
-        flat_cols.reserve(n_flat); flat_logs.reserve(n_flat);
-        // step of CanonicCoset(lifting_log): the point of index 2^(31 - lifting_log)
-        cpoint gen = host_circle_point(1u << (31 - lifting_log));
-        // Sample j of the flattened list takes random_coeff^j (quotients.rs:306-345 multiplies as it goes): the powers are
-        // filled in chunks on several threads, each starting from its own power.
-        std::vector<size_t> first_pow;
-        first_pow.reserve(n_flat + 1);
-        size_t n_pows = 0;
-        for (size_t t = 0; t < trees.size(); t++)
-            for (size_t c = 0; c < trees[t].evals.size(); c++) {
-                first_pow.push_back(n_pows);
-                const size_t ns = samples[t][c].size();
-                n_pows += ns + (ns == 2 ? 1 : 0);
+    // pcs/quotient_ops.rs:73-194 with STWO/core/pcs/quotients.rs:306-345 and :75-104: what is accumulated for which columns. It depends on
+    // the columns' sizes and the sample points only, so it is made and uploaded while the samples are evaluated and hashed.
+    struct Numerators {
+        struct Group { uint32_t log; size_t first_col, n_cols, first_batch, n_batches; };
+        std::vector<const uint32_t*> cols;  // by ascending size, in their own order within a size
+        std::vector<Group> groups;
+        zk::NumeratorEntries entries;       // batch after batch
+        std::vector<zk::NumeratorBatch> batches;
+        std::vector<uint32_t> batch_point;  // of the points below
+        std::vector<CirclePointQ> points;   // the sample points, then the shifted ones
+        zk::NumeratorLines lines;
+    };
+    // place_of[s]: where sample s's value lies in the value array.
+    Numerators plan_numerators(const SamplePoints& sp, const std::vector<uint32_t>& place_of, uint32_t lifting_log) const {
+        Numerators nu;
+        nu.points = sp.points;
+        const size_t n_cols = sp.first.size() - 1;
+        std::vector<const BaseColumn*> flat;
+        std::vector<uint8_t> logs;
+        flat.reserve(n_cols);
+        logs.reserve(n_cols);
+        size_t first_of[34] = {0};
+        for (auto& t : trees)
+            for (auto& e : t.evals) {
+                flat.push_back(&e);
+                logs.push_back((uint8_t)std::min<uint32_t>(e.log_size(), 32));
+                first_of[logs.back() + 1]++;
             }
-        first_pow.push_back(n_pows);
-        // column i's samples with their powers: flat_samples[first_pow[i] .. first_pow[i + 1]) (one array: a vector per column
-        // is an allocation per column)
-        std::vector<std::pair<PointSample, qm31>> flat_samples(n_pows);
-        parallel_chunks(n_pows, 8192, [&](size_t lo, size_t hi, size_t) {
-            qm31 p = qm31_one(), sq = random_coeff;
-            for (size_t e = lo; e; e >>= 1) { if (e & 1) p = p * sq; sq = sq * sq; }
-            for (size_t i = lo; i < hi; i++) { flat_samples[i].second = p; p = p * random_coeff; }
-        });
-        // the periodicity sample's point depends on the column's height and the sampled point only: a handful of distinct ones
-        struct Shifted { uint32_t log_size; CirclePointQ from, to; };
+        // Entry j of the flattened list takes random_coeff^j (quotients.rs:306-345 multiplies as it goes): a column with two samples
+        // has a third entry before them, its second sample at that point shifted by the column's period.
+        std::vector<uint32_t> first_pow(n_cols);
+        uint32_t n_pows = 0;
+        for (size_t c = 0; c < n_cols; c++) {
+            const size_t ns = sp.first[c + 1] - sp.first[c];
+            first_pow[c] = n_pows;
+            n_pows += (uint32_t)(ns + (ns == 2 ? 1 : 0));
+        }
+        for (int k = 1; k < 34; k++) first_of[k] += first_of[k - 1];
+        std::vector<uint32_t> order(n_cols);
+        for (size_t c = 0; c < n_cols; c++) order[first_of[logs[c]]++] = (uint32_t)c;
+        // the shifted points: a handful of distinct (size, point) pairs
+        struct Shifted { uint32_t log, from, to; };
         std::vector<Shifted> shifted;
-        for (size_t t = 0; t < trees.size(); t++)
-            for (size_t c = 0; c < trees[t].evals.size(); c++) {
-                uint32_t log_size = trees[t].evals[c].log_size();
-                flat_cols.push_back(&trees[t].evals[c]);
-                flat_logs.push_back(log_size);
-                const auto& sc = samples[t][c];
-                std::pair<PointSample, qm31>* v = flat_samples.data() + first_pow[flat_cols.size() - 1];
-                if (!sc.empty()) {
-                    if (sc.size() == 2) {
-                        const Shifted* hit = nullptr;
-                        for (auto& sh : shifted) if (sh.log_size == log_size && sh.from == sc[1].point) { hit = &sh; break; }
-                        if (!hit) {
-                            cpoint per = gen;
-                            for (uint32_t k = 0; k < log_size; k++) per = cpoint_add(per, per);
-                            CirclePointQ pq{qm31_from_m31(per.x), qm31_from_m31(per.y)};
-                            shifted.push_back({log_size, sc[1].point, point_add(sc[1].point, pq)});
-                            hit = &shifted.back();
-                        }
-                        (v++)->first = PointSample{hit->to, sc[1].value};
+        auto shift_of = [&](uint32_t log, uint32_t from) {
+            for (auto& s : shifted) if (s.log == log && s.from == from) return s.to;
+            cpoint per = host_circle_point(1u << (31 - lifting_log));  // step of CanonicCoset(lifting_log)
+            for (uint32_t k = 0; k < log; k++) per = cpoint_add(per, per);
+            const CirclePointQ p = point_add(nu.points[from], {qm31_from_m31(per.x), qm31_from_m31(per.y)});
+            uint32_t to = 0;
+            while (to < nu.points.size() && !(nu.points[to] == p)) to++;
+            if (to == nu.points.size()) nu.points.push_back(p);
+            shifted.push_back({log, from, to});
+            return to;
+        };
+        // every entry's batch (a size's points in the order they come up), then the batches' entries in place
+        struct Raw { uint32_t batch, col, val, pow; };
+        std::vector<Raw> raw;
+        raw.reserve(n_pows);
+        nu.cols.reserve(n_cols);
+        std::vector<uint32_t> batch_of;  // per point, within the size at hand; ~0: none yet
+        for (size_t i = 0; i < n_cols;) {
+            const uint32_t log = logs[order[i]];
+            const size_t first_col = nu.cols.size(), first_batch = nu.batches.size();
+            std::fill(batch_of.begin(), batch_of.end(), ~0u);
+            for (; i < n_cols && logs[order[i]] == log; i++) {
+                const uint32_t c = order[i];
+                const uint32_t col = (uint32_t)(nu.cols.size() - first_col);
+                nu.cols.push_back(flat[c]->ptr());
+                uint32_t pow = first_pow[c];
+                auto entry = [&](uint32_t point, size_t sample) {
+                    if (point >= batch_of.size()) batch_of.resize(point + 1, ~0u);
+                    if (batch_of[point] == ~0u) {
+                        batch_of[point] = (uint32_t)nu.batches.size();
+                        nu.batches.push_back({nu.points[point].y, 0, 0, qm31_zero(), qm31_zero()});
+                        nu.batch_point.push_back(point);
                     }
-                    for (auto& smp : sc) (v++)->first = smp;
-                }
+                    nu.batches[batch_of[point]].count++;
+                    raw.push_back({batch_of[point], col, place_of[sample], pow++});
+                };
+                const size_t s0 = sp.first[c], s1 = sp.first[c + 1];
+                if (s1 - s0 == 2) entry(shift_of(log, sp.point_of[s0 + 1]), s0 + 1);
+                for (size_t s = s0; s < s1; s++) entry(sp.point_of[s], s);
             }
-        hc.reset(new HostClock("pcs.quot.groups"));
-        // the columns by ascending size, in their own order within a size: a counting sort (sizes are below 2^32)
-        std::vector<size_t> order(flat_cols.size());
-        {
-            size_t first_of[34] = {0};
-            for (uint32_t lg : flat_logs) first_of[std::min<uint32_t>(lg, 32) + 1]++;
-            for (int k = 1; k < 34; k++) first_of[k] += first_of[k - 1];
-            for (size_t i = 0; i < flat_logs.size(); i++) order[first_of[std::min<uint32_t>(flat_logs[i], 32)]++] = i;
+            nu.groups.push_back({log, first_col, nu.cols.size() - first_col, first_batch, nu.batches.size() - first_batch});
         }
+        std::vector<size_t> at(nu.batches.size());
+        size_t n = 0;
+        for (size_t b = 0; b < at.size(); b++) { nu.batches[b].first = at[b] = n; n += nu.batches[b].count; }
+        nu.entries.col.resize(n);
+        nu.entries.val.resize(n);
+        nu.entries.pow.resize(n);
+        for (auto& r : raw) {
+            const size_t k = at[r.batch]++;
+            nu.entries.col[k] = r.col;
+            nu.entries.val[k] = r.val;
+            nu.entries.pow[k] = r.pow;
+        }
+        return nu;
+    }
+
+    SecureColumnByCoords compute_fri_quotients(Numerators& nu, qm31 random_coeff, const qm31* h_values, const uint32_t* d_values, uint32_t lifting_log) {
+        std::unique_ptr<HostClock> hc(new HostClock("pcs.quot.lines"));
+        d.check(zk::numerator_lines(d.ctx(), nu.entries, nu.batches, nu.lines, random_coeff, h_values, d_values));
+        hc.reset(new HostClock("pcs.quot.numerators"));
         std::vector<AccumulatedNumerators> accs;
-        for (size_t i = 0; i < order.size();) {
-            size_t j = i;
-            while (j < order.size() && flat_logs[order[j]] == flat_logs[order[i]]) j++;
-            std::vector<const BaseColumn*> group_cols;
-            std::vector<ColumnSampleBatch> batches;
-            for (size_t k = i; k < j; k++) {
-                group_cols.push_back(flat_cols[order[k]]);
-                for (size_t q = first_pow[order[k]]; q < first_pow[order[k] + 1]; q++) {
-                    const std::pair<PointSample, qm31>& sp = flat_samples[q];
-                    ColumnSampleBatch* b = nullptr;
-                    for (auto& x : batches) if (x.point == sp.first.point) { b = &x; break; }
-                    if (!b) { batches.push_back({sp.first.point, {}}); b = &batches.back(); }
-                    b->cols_vals_randpows.push_back({k - i, sp.first.value, sp.second});
-                }
+        for (auto& g : nu.groups)
+            for (size_t b = g.first_batch; b < g.first_batch + g.n_batches; b++) {
+                SecureColumnByCoords acc(d, (size_t)1 << g.log);
+                auto o = acc.ptrs();
+                d.check(zk::numerator_run(d.ctx(), nu.cols.data() + g.first_col, (int)g.n_cols, (int)g.log, nu.lines, nu.batches[b], o.data()));
+                accs.push_back({nu.points[nu.batch_point[b]], std::move(acc), nu.batches[b].first_linear});
             }
-            {
-                HostClock hn("pcs.quot.numerators");
-                B200Backend::accumulate_numerators(d, group_cols, batches, accs);
-            }
-            i = j;
-        }
         hc.reset(new HostClock("pcs.quot.combine"));
         std::stable_sort(accs.begin(), accs.end(),
                          [](const AccumulatedNumerators& a, const AccumulatedNumerators& b) { return point_less(a.sample_point, b.sample_point); });
@@ -922,7 +961,7 @@ struct CommitmentSchemeProver {
     }
 
     // pcs/mod.rs:168-419
-    PcsProof prove_values(const std::vector<std::vector<std::vector<CirclePointQ>>>& sampled_points, Channel& ch) {
+    PcsProof prove_values(SamplePoints sp, Channel& ch) {
         PcsProof proof;
         uint32_t lifting_log = trees.back().max_log();
         // Every column is lifted to the height of the LAST tree (pcs/mod.rs:180: in a proof it is the composition tree, which
@@ -930,59 +969,66 @@ struct CommitmentSchemeProver {
         for (auto& t : trees)
             if (!t.evals.empty() && t.max_log() > lifting_log)
                 throw Error(ZKB_EINVAL, "pcs: the last tree must hold the tallest column (every column is lifted to its height)");
-        // batch out-of-domain evaluation: one call per (coefficient size, transformed point) group (:187-265)
+        // batch out-of-domain evaluation: one call per (coefficient size, transformed point) group (:187-265); the values of a group
+        // lie one after the other in the value array, place_of[s] is sample s's
         std::unique_ptr<HostClock> hc(new HostClock("pcs.sample.group"));
-        std::vector<std::vector<std::vector<PointSample>>> samples(trees.size());
-        struct Group { uint32_t log; CirclePointQ pt; std::vector<std::array<size_t, 3>> where; std::vector<const BaseColumn*> cols; };
+        const size_t n_samples = sp.point_of.size();
+        struct Group { uint32_t log; CirclePointQ pt; size_t first, count; };
         std::vector<Group> groups;
-        struct Doubled { CirclePointQ p; uint32_t shift; CirclePointQ tp; };
-        std::vector<Doubled> doubled;
-        for (size_t t = 0; t < trees.size(); t++) {
-            samples[t].resize(trees[t].coeffs.size());
-            for (size_t c = 0; c < trees[t].coeffs.size(); c++) {
-                uint32_t poly_log = trees[t].evals[c].log_size(), coeff_log = trees[t].coeffs[c].log_size();
-                samples[t][c].reserve(sampled_points[t][c].size());
-                for (size_t k = 0; k < sampled_points[t][c].size(); k++) {
-                    CirclePointQ p = sampled_points[t][c][k];
-                    samples[t][c].push_back({p, qm31_zero()});
-                    // most columns share the point and the shift: double once per distinct (point, shift)
-                    CirclePointQ tp;
-                    bool seen = false;
-                    for (auto& m : doubled) if (m.shift == lifting_log - poly_log && m.p == p) { tp = m.tp; seen = true; break; }
-                    if (!seen) { tp = point_repeated_double(p, lifting_log - poly_log); doubled.push_back({p, lifting_log - poly_log, tp}); }
-                    Group* g = nullptr;
-                    for (auto& x : groups) if (x.log == coeff_log && x.pt == tp) { g = &x; break; }
-                    if (!g) { groups.push_back({coeff_log, tp, {}, {}}); g = &groups.back(); }
-                    g->where.push_back({t, c, k});
-                    g->cols.push_back(&trees[t].coeffs[c]);
+        std::vector<int> group_of(sp.points.size() * 64, -1);  // by (point, doublings)
+        std::vector<uint32_t> sample_group(n_samples), place_of(n_samples);
+        size_t flat = 0;
+        for (auto& t : trees) {
+            proof.sampled_values.tree_first.push_back(flat + t.coeffs.size());
+            for (size_t c = 0; c < t.coeffs.size(); c++, flat++) {
+                const uint32_t coeff_log = t.coeffs[c].log_size(), shift = lifting_log - t.evals[c].log_size();
+                for (size_t s = sp.first[flat]; s < sp.first[flat + 1]; s++) {
+                    int& g = group_of[sp.point_of[s] * 64 + shift];
+                    if (g < 0) {
+                        g = (int)groups.size();
+                        groups.push_back({coeff_log, point_repeated_double(sp.points[sp.point_of[s]], shift), 0, 0});
+                    }
+                    sample_group[s] = (uint32_t)g;
+                    groups[g].count++;
                 }
             }
         }
+        size_t at = 0;
+        for (auto& g : groups) { g.first = at; at += g.count; g.count = 0; }
+        std::vector<const uint32_t*> polys(n_samples);
+        flat = 0;
+        for (auto& t : trees)
+            for (size_t c = 0; c < t.coeffs.size(); c++, flat++)
+                for (size_t s = sp.first[flat]; s < sp.first[flat + 1]; s++) {
+                    Group& g = groups[sample_group[s]];
+                    place_of[s] = (uint32_t)(g.first + g.count);
+                    polys[g.first + g.count++] = t.coeffs[c].ptr();
+                }
         hc.reset(new HostClock("pcs.sample.eval"));
+        BaseColumn d_values(d, 4 * n_samples);
         for (auto& g : groups) {
-            auto vals = B200Backend::batch_eval_at_point(d, g.cols, g.pt);
-            for (size_t i = 0; i < vals.size(); i++) samples[g.where[i][0]][g.where[i][1]][g.where[i][2]].value = vals[i];
+            uint32_t pt[8];
+            memcpy(pt, g.pt.x.c, 16);
+            memcpy(pt + 4, g.pt.y.c, 16);
+            d.check(zk::eval_at_point_device(d.ctx(), polys.data() + g.first, (int)g.count, (int)g.log, pt, d_values.ptr() + 4 * g.first));
         }
-        hc.reset(new HostClock("pcs.sample.flatten"));
-        std::vector<qm31> flat_values;
-        size_t n_values = 0;
-        for (auto& t : samples) for (auto& col : t) n_values += col.size();
-        flat_values.reserve(n_values);
-        for (size_t t = 0; t < trees.size(); t++) {
-            proof.sampled_values.emplace_back();
-            proof.sampled_values[t].resize(samples[t].size());
-            for (size_t c = 0; c < samples[t].size(); c++) {
-                std::vector<qm31>& v = proof.sampled_values[t][c];
-                v.reserve(samples[t][c].size());
-                for (auto& smp : samples[t][c]) { v.push_back(smp.value); flat_values.push_back(smp.value); }
-            }
-        }
+        hc.reset(new HostClock("pcs.quot.plan"));
+        Numerators nu = plan_numerators(sp, place_of, lifting_log);
+        d.check(zk::numerator_stage(d.ctx(), nu.entries, nu.batches, nu.lines));
+        BaseColumn lines_block = BaseColumn::adopt(d, nu.lines.block);
+        hc.reset(new HostClock("pcs.sample.read"));
+        qm31* h_values = reinterpret_cast<qm31*>(GatherPlan::arena(4 * n_samples));
+        if (n_samples) d.check(zkb_d2h(d.ctx(), h_values, d_values.ptr(), 16 * n_samples));
+        std::vector<qm31>& values = proof.sampled_values.values;
+        values.resize(n_samples);
+        for (size_t s = 0; s < n_samples; s++) values[s] = h_values[place_of[s]];
         mark(3);
         hc.reset(new HostClock("pcs.quot.mix"));
-        ch.mix_felts(flat_values);
+        ch.mix_felts(values);
         qm31 random_coeff = ch.draw_secure_felt();
         hc.reset(new HostClock("pcs.quot.compute"));
-        SecureColumnByCoords quotients = compute_fri_quotients(samples, random_coeff, lifting_log);
+        SecureColumnByCoords quotients = compute_fri_quotients(nu, random_coeff, h_values, d_values.ptr(), lifting_log);
+        proof.sampled_values.first = std::move(sp.first);
         hc.reset();
         mark(4);
         FriProver fri = FriProver::commit(d, ch, config.fri, quotients, (int)config.pow_bits);
@@ -998,23 +1044,18 @@ struct CommitmentSchemeProver {
         hc2.reset(new HostClock("pcs.decommit.plan.trees"));
         std::vector<PendingMerkle> tree_pending;
         for (auto& t : trees) {  // STWO/core/pcs/utils.rs:200-218, then pcs/mod.rs:575-630
-            uint32_t tree_max = t.max_log();
-            std::vector<size_t> q;
-            for (auto pos : query_positions) q.push_back(((pos >> (lifting_log - tree_max + 1)) << 1) + (pos & 1));
-            std::map<uint32_t, std::vector<size_t>> per_log;
-            std::vector<const BaseColumn*> refs;
-            refs.reserve(t.evals.size());
-            uint64_t seen_logs = 0;  // a tree has tens of thousands of columns and a handful of heights
-            for (auto& e : t.evals) {
-                refs.push_back(&e);
-                uint32_t log = e.log_size();
-                if ((seen_logs >> log) & 1) continue;
-                seen_logs |= (uint64_t)1 << log;
-                std::vector<size_t> positions;
-                for (auto pos : q) positions.push_back(((pos >> (tree_max - log + 1)) << 1) + (pos & 1));
-                per_log[log] = sorted_dedup(positions);
-            }
-            tree_pending.push_back(t.commitment.plan_decommit(plan, per_log, refs));
+            const uint32_t tree_max = t.max_log();
+            std::vector<size_t> of_log;
+            tree_pending.push_back(t.commitment.plan_decommit(plan, [&](uint32_t log) -> const std::vector<size_t>& {
+                of_log.clear();
+                if (log >= t.commitment.layer_col_ptrs.size() || t.commitment.layer_col_ptrs[log].empty()) return of_log;
+                for (auto pos : query_positions) {
+                    const size_t q = ((pos >> (lifting_log - tree_max + 1)) << 1) + (pos & 1);
+                    of_log.push_back(((q >> (tree_max - log + 1)) << 1) + (q & 1));
+                }
+                of_log = sorted_dedup(std::move(of_log));
+                return of_log;
+            }));
         }
         hc2.reset();
         hc.reset(new HostClock("pcs.decommit.gather"));
@@ -1733,11 +1774,11 @@ int zkb_shard_pcs_fri_and_decommit(zkb_shard_pcs* h, uint32_t* h_part, size_t ca
             if ((q >> s.log_local) == (size_t)s.rank) local.push_back(q - ((size_t)s.rank << s.log_local));
             owners.push_back(q >> s.log_local);
         }
-        std::vector<const BaseColumn*> refs;
-        for (auto& c : s.row_cols) refs.push_back(&c);
-        std::vector<size_t> per_layer, top_per_layer;
-        PendingMerkle pm = s.subtree.plan_decommit(plan, {{s.log_local, sorted_dedup(local)}}, refs, &per_layer);
-        PendingMerkle pt = s.top.plan_decommit(plan, {{(uint32_t)s.log_g, sorted_dedup(owners)}}, {}, &top_per_layer);
+        std::vector<size_t> per_layer;
+        local = sorted_dedup(local);
+        owners = sorted_dedup(owners);
+        PendingMerkle pm = s.subtree.plan_decommit(plan, QueriesOf{s.log_local, local}, &per_layer);
+        PendingMerkle pt = s.top.plan_decommit(plan, QueriesOf{(uint32_t)s.log_g, owners});
         plan.execute(s.dev);
         s.fri_proof = s.fri.finish_decommit(plan, fri_pending);
         s.top_dec = pt.finish(plan).second;
@@ -1764,8 +1805,9 @@ int zkb_shard_pcs_finish(zkb_shard_pcs* h, const uint32_t* const* h_parts, const
     return shard_guard(s.ctx, [&] {
         PcsProof proof;
         proof.commitments.push_back(s.root);
-        proof.sampled_values.emplace_back();
-        for (auto v : s.samples) proof.sampled_values[0].push_back({v});
+        proof.sampled_values.values = s.samples;
+        for (size_t k = 0; k < s.samples.size(); k++) proof.sampled_values.first.push_back(k + 1);
+        proof.sampled_values.tree_first.push_back(s.samples.size());
         MerkleDecommitment dec;
         std::vector<uint32_t> values;
         std::vector<size_t> cursor(s.world, 1);
@@ -1904,21 +1946,27 @@ static int pcs_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, uint
         }
         int flat = 0;
         CirclePointQ oods = get_random_point(ch);
-        std::vector<std::vector<std::vector<CirclePointQ>>> points(n_trees);
-        flat = 0;
-        for (int t = 0; t < n_trees; t++)
-            for (int c = 0; c < tree_ncols[t]; c++, flat++) {
-                std::vector<CirclePointQ> p;
-                if (two_sample_every && flat % two_sample_every == 0) {
+        SamplePoints points;
+        points.point_of.reserve((size_t)total);
+        points.first.reserve((size_t)total + 1);
+        const uint32_t at_oods = points.intern(oods);
+        uint32_t step_back[32];  // per column size, the place of its second point
+        for (auto& k : step_back) k = ~0u;
+        for (flat = 0; flat < total; flat++) {
+            if (two_sample_every && flat % two_sample_every == 0) {
+                uint32_t& k = step_back[col_logs[flat]];
+                if (k == ~0u) {
                     // one trace step back: the conjugate of the step of CanonicCoset(col_log)
                     cpoint st = host_circle_point(1u << (31 - col_logs[flat]));
-                    p.push_back(point_add(oods, {qm31_from_m31(st.x), qm31_from_m31(m31_neg(st.y))}));
+                    k = points.intern(point_add(oods, {qm31_from_m31(st.x), qm31_from_m31(m31_neg(st.y))}));
                 }
-                p.push_back(oods);
-                points[t].push_back(p);
+                points.point_of.push_back(k);
             }
+            points.point_of.push_back(at_oods);
+            points.end_column();
+        }
         std::unique_ptr<HostClock> hc(new HostClock("pcs.prove_values"));
-        PcsProof proof = prover.prove_values(points, ch);
+        PcsProof proof = prover.prove_values(std::move(points), ch);
         prover.finish_timing();
         hc.reset(new HostClock("pcs.write"));
         PcsProof::RawSink w{h_out, cap};  // straight into the caller's buffer: a proof of many columns is tens of megabytes
@@ -2081,7 +2129,13 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
                     }
         }
         points.back().assign(8, {oods});
-        PcsProof proof = prover.prove_values(points, ch);
+        SamplePoints flat_points;
+        for (auto& tree : points)
+            for (auto& column : tree) {
+                for (auto& p : column) flat_points.point_of.push_back(flat_points.intern(p));
+                flat_points.end_column();
+            }
+        PcsProof proof = prover.prove_values(std::move(flat_points), ch);
         prover.finish_timing();
         if (composition_ms) dev.check(zkb_event_elapsed_ms(ctx, 28, 29, composition_ms));
 
@@ -2090,9 +2144,9 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
             const qm31 i{{0, 1, 0, 0}}, u{{0, 0, 1, 0}}, iu{{0, 0, 0, 1}};
             return e0 + e1 * i + e2 * u + e3 * iu;
         };
-        const auto& comp = proof.sampled_values.back();
-        const qm31 left = from_partial_evals(comp[0][0], comp[1][0], comp[2][0], comp[3][0]);
-        const qm31 right = from_partial_evals(comp[4][0], comp[5][0], comp[6][0], comp[7][0]);
+        auto comp = [&](size_t c) { return *proof.sampled_values.at((size_t)n_trees, c); };
+        const qm31 left = from_partial_evals(comp(0), comp(1), comp(2), comp(3));
+        const qm31 right = from_partial_evals(comp(4), comp(5), comp(6), comp(7));
         const qm31 committed = left + point_repeated_double(oods, max_log_degree_bound - 1).x * right;
         // coset_vanishing(CanonicCoset(max_log_degree_bound).coset, oods): the shift -initial + step/2 is zero for a canonic coset
         qm31 vanish = oods.x;
@@ -2113,7 +2167,7 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
                         const uint32_t col = prog->tree_base[o.a] + o.b;
                         const auto& offs = offsets[k][col];
                         const size_t j = std::find(offs.begin(), offs.end(), (int32_t)o.c) - offs.begin();
-                        v[i] = proof.sampled_values[where[col].first][where[col].second][j];
+                        v[i] = proof.sampled_values.at((size_t)where[col].first, where[col].second)[j];
                         break;
                     }
                     case ZKB_AIR_CONST_M31: v[i] = qm31_from_m31(o.a); break;

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "quot_lines.hpp"
 
 namespace zk {
 
@@ -132,18 +133,7 @@ __global__ void __launch_bounds__(256) eval_fold_kernel(const uint32_t* const* _
     }
 }
 
-}  // namespace zk
-
-using namespace zk;
-
-extern "C" {
-
-int zkb_eval_at_point_cols(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols, int log_n, const uint32_t* h_point,
-                           uint32_t* h_out) {
-    if (!ctx) return ZKB_EINVAL;
-    ZKB_CHECK_ARG(ctx, ncols >= 0 && log_n >= 0 && log_n <= 30);
-    if (ncols == 0) return ZKB_OK;
-    ZKB_CHECK_ARG(ctx, coeffs && h_point && h_out);
+int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols, int log_n, const uint32_t h_point[8], uint32_t* d_out) {
     DeviceGuard g(ctx);
     // factors m_0 = y, m_1 = x, m_{k+1} = 2 m_k^2 - 1
     EvalFactors f;
@@ -176,18 +166,19 @@ int zkb_eval_at_point_cols(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncol
         if (rc) return rc;
         uint32_t* bufA = ctx->scratch + weights_words;
         uint32_t* bufB = bufA + half_words;
+        uint32_t* const out = d_out + 4 * (size_t)c0;  // what the last kernel writes to
         int log_cur = log_n, level = 0;
         if (use_dot) {
             size_t items = (partials_per_col + DOT_CHUNKS - 1) / DOT_CHUNKS * (size_t)nc;
             unsigned grid = (unsigned)(items < 2 * 148 ? items : 2 * 148);
             ProfScope prof(ctx, "eval_dot_kernel");
-            eval_dot_kernel<<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, weights, bufA);
+            eval_dot_kernel<<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, weights, log_n == first_chunk ? out : bufA);
             ZKB_LAUNCH_CHECK(ctx);
         } else {
             unsigned threads = first_chunk >= 9 ? 256 : 32;
             dim3 grid((unsigned)partials_per_col, nc);
             eval_fold_kernel<true><<<grid, threads, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nullptr, log_cur,
-                                                                      first_chunk, level, f, bufA);
+                                                                      first_chunk, level, f, log_n == first_chunk ? out : bufA);
             ZKB_LAUNCH_CHECK(ctx);
         }
         log_cur -= first_chunk;
@@ -196,16 +187,38 @@ int zkb_eval_at_point_cols(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncol
             int ch = log_cur < EVAL_CHUNK_LOG ? log_cur : EVAL_CHUNK_LOG;
             unsigned threads = ch >= 9 ? 256 : 32;
             dim3 grid(1u << (log_cur - ch), nc);
-            eval_fold_kernel<false><<<grid, threads, 0, ctx->stream>>>(nullptr, bufA, log_cur, ch, level, f, bufB);
+            eval_fold_kernel<false><<<grid, threads, 0, ctx->stream>>>(nullptr, bufA, log_cur, ch, level, f, log_cur == ch ? out : bufB);
             ZKB_LAUNCH_CHECK(ctx);
             log_cur -= ch;
             level += ch;
             uint32_t* t = bufA; bufA = bufB; bufB = t;
         }
-        ZKB_CUDA(ctx, cudaMemcpyAsync(h_out + 4 * (size_t)c0, bufA, (size_t)nc * 16, cudaMemcpyDeviceToHost, ctx->stream));
-        ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     }
     return ZKB_OK;
+}
+
+}  // namespace zk
+
+using namespace zk;
+
+extern "C" {
+
+int zkb_eval_at_point_cols(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols, int log_n, const uint32_t* h_point,
+                           uint32_t* h_out) {
+    if (!ctx) return ZKB_EINVAL;
+    ZKB_CHECK_ARG(ctx, ncols >= 0 && log_n >= 0 && log_n <= 30);
+    if (ncols == 0) return ZKB_OK;
+    ZKB_CHECK_ARG(ctx, coeffs && h_point && h_out);
+    DeviceGuard g(ctx);
+    uint32_t* d_out = nullptr;
+    if (int rc = zkb_malloc(ctx, (size_t)ncols * 16, (void**)&d_out)) return rc;
+    int rc = eval_at_point_device(ctx, coeffs, ncols, log_n, h_point, d_out);
+    cudaError_t e = cudaSuccess;
+    if (rc == ZKB_OK) e = cudaMemcpyAsync(h_out, d_out, (size_t)ncols * 16, cudaMemcpyDeviceToHost, ctx->stream);
+    if (rc == ZKB_OK && e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    zkb_free(ctx, d_out);
+    if (rc == ZKB_OK && e != cudaSuccess) rc = set_error(ctx, ZKB_ECUDA, "eval at point: %s", cudaGetErrorString(e));
+    return rc;
 }
 
 }  // extern "C"

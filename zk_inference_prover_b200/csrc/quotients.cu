@@ -13,6 +13,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fri_tail.hpp"
+#include "quot_lines.hpp"
 
 namespace zk {
 
@@ -236,6 +238,216 @@ static cpoint host_point_q(uint32_t index) {
     return r;
 }
 
+namespace zk {
+
+// ---- the entries' line coefficients (core/pcs/quotients.rs:58-104, core/constraints.rs:119-134)
+//
+// With v an entry's value, p its power of the random coefficient and y its sample point's ordinate: a = p (conj v - v),
+// c = p (conj y - y), b = v c - a y. Only c is needed entry by entry; of a and b the sums over the batch are, and those follow from
+// the sums of p v and p conj v. A proof over tens of thousands of columns has as many entries: 45 ns each on a host core
+// (65,000: 3 ms, 1.2 ms on four), microseconds here, and what does not depend on the coefficient is uploaded before it is drawn.
+struct LineChunk { uint32_t batch, first, count, pad; };
+constexpr uint32_t LINE_CHUNK = 1024;  // entries a CTA takes: a batch's sums meet in a few atomics per warp
+constexpr uint32_t LINE_POW_LOG = 8;   // alpha^e = low[e mod 2^8] high[e / 2^8]
+
+__device__ __forceinline__ qm31 line_ld(const uint32_t* p, size_t i) {
+    const uint4 v = reinterpret_cast<const uint4*>(p)[i];
+    return {{v.x, v.y, v.z, v.w}};
+}
+__device__ __forceinline__ uint32_t line_warp_sum(uint32_t v) {
+    return m31_reduce64(__reduce_add_sync(0xffffffffu, v & 0xffffu) + ((uint64_t)__reduce_add_sync(0xffffffffu, v >> 16) << 16));
+}
+__global__ void __launch_bounds__(256) quot_lines_kernel(const LineChunk* __restrict__ chunks, const uint32_t* __restrict__ batch_c, const uint32_t* __restrict__ val,
+                                                         const uint32_t* __restrict__ pow, const uint32_t* __restrict__ pow_table, const uint32_t* __restrict__ values,
+                                                         uint32_t* __restrict__ out_c, unsigned long long* __restrict__ sums) {
+    const LineChunk ch = chunks[blockIdx.x];
+    const qm31 c = line_ld(batch_c, ch.batch);
+    qm31 s = qm31_zero(), sc = qm31_zero();
+    for (uint32_t i = threadIdx.x; i < ch.count; i += blockDim.x) {
+        const uint32_t e = pow[ch.first + i];
+        const qm31 p = qm31_mul(line_ld(pow_table, e & ((1u << LINE_POW_LOG) - 1)), line_ld(pow_table, (1u << LINE_POW_LOG) + (e >> LINE_POW_LOG)));
+        const qm31 v = line_ld(values, val[ch.first + i]);
+        const qm31 r = qm31_mul(p, c);
+        reinterpret_cast<uint4*>(out_c)[ch.first + i] = make_uint4(r.c[0], r.c[1], r.c[2], r.c[3]);
+        s = qm31_add(s, qm31_mul(p, v));
+        sc = qm31_add(sc, qm31_mul(p, qm31{{v.c[0], v.c[1], m31_neg(v.c[2]), m31_neg(v.c[3])}}));
+    }
+    unsigned long long* const at = sums + 8 * (size_t)ch.batch;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t a = line_warp_sum(s.c[q]), b = line_warp_sum(sc.c[q]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(at + q, (unsigned long long)a);
+            atomicAdd(at + 4 + q, (unsigned long long)b);
+        }
+    }
+}
+
+// The kernels of one accumulation. d_cols: the columns' staged table; scratch_used: words of the scratch buffer that hold its inputs.
+static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const uint32_t* const* d_cols, const uint32_t* d_idx,
+                             const uint32_t* d_c, int k, qm31 b_sum, Secure4 o, size_t scratch_used) {
+    size_t n = (size_t)1 << log_n;
+    bool wide = n >= 4;
+    for (int q = 0; q < 4; q++) wide = wide && ((uintptr_t)o.c[q] & 15) == 0;
+    for (int c = 0; c < ncols; c++) wide = wide && ((uintptr_t)cols[c] & 15) == 0;
+    ProfScope prof(ctx, "quot_numerators_kernel");
+    // Few rows and many columns: split the columns over the grid's second dimension.
+    const unsigned row_blocks = (unsigned)((n / (wide ? 4 : 2) + 255) / 256);
+    const size_t scratch_free = ctx->scratch_words - scratch_used;
+    if (row_blocks < 148u && k >= 8 * NUM_TILE && 4 * n * 2 <= scratch_free) {
+        int S = (int)((2u * 148u + row_blocks - 1) / row_blocks);            // about two CTAs per SM
+        int chunk = ((k + S - 1) / S + NUM_TILE - 1) / NUM_TILE * NUM_TILE;  // whole tiles of columns
+        S = (k + chunk - 1) / chunk;
+        while ((size_t)S * 4 * n + 4 > scratch_free) { chunk += NUM_TILE; S = (k + chunk - 1) / chunk; }
+        uint32_t* partial = ctx->scratch + scratch_used + ((4 - (scratch_used & 3)) & 3);  // 16-byte aligned
+        dim3 grid(row_blocks, (unsigned)S);
+        if (wide)
+            quot_numerators_kernel<4><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
+                                                                     b_sum, n, o, chunk, partial);
+        else
+            quot_numerators_kernel<2><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
+                                                                     b_sum, n, o, chunk, partial);
+        ZKB_LAUNCH_CHECK(ctx);
+        quot_partial_sum_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, o);
+        ZKB_LAUNCH_CHECK(ctx);
+        return ZKB_OK;
+    }
+    if (wide)
+        quot_numerators_kernel<4><<<(unsigned)((n / 4 + 255) / 256), 256, 0, ctx->stream>>>(
+            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
+    else
+        quot_numerators_kernel<2><<<(unsigned)((n / 2 + 255) / 256), 256, 0, ctx->stream>>>(
+            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
+    ZKB_LAUNCH_CHECK(ctx);
+    return ZKB_OK;
+}
+
+static qm31 conj_q(qm31 v) { return {{v.c[0], v.c[1], m31_neg(v.c[2]), m31_neg(v.c[3])}}; }
+
+// Below so many entries the host is done with the coefficients before a launch and its read-back would be (some 20 us).
+constexpr size_t LINES_ON_DEVICE_MIN = 512;
+static size_t words16(size_t n) { return (n + 3) & ~(size_t)3; }
+
+// Uploads `n` words, through the staging ring where they fit a quarter of it.
+static int upload_words(zkb_ctx* ctx, uint32_t* dst, const std::vector<uint32_t>& h) {
+    if (h.empty()) return ZKB_OK;
+    if (h.size() * 4 <= sizeof(void*) * (ctx->ring_cap / 4)) return upload_small(ctx, dst, h.data(), h.size());
+    ZKB_CUDA(ctx, cudaMemcpyAsync(dst, h.data(), h.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    return ZKB_OK;
+}
+
+// The block: [c: 4 n][col: n][val: n][pow: n][chunks][sums: 16 words a batch]
+int numerator_stage(zkb_ctx* ctx, const NumeratorEntries& e, const std::vector<NumeratorBatch>& batches, NumeratorLines& lines) {
+    DeviceGuard g(ctx);
+    const size_t n = e.col.size();
+    const bool device = n >= LINES_ON_DEVICE_MIN;
+    size_t n_chunks = 0;
+    for (auto& b : batches) n_chunks += (b.count + LINE_CHUNK - 1) / LINE_CHUNK;
+    const size_t o_col = 4 * n, words = o_col + 3 * words16(n) + 4 * n_chunks + 16 * batches.size();
+    if (int rc = zkb_malloc(ctx, words * 4 + 16, (void**)&lines.block)) return rc;
+    lines.d_c = lines.block;
+    lines.d_col = lines.block + o_col;
+    if (!device) return ZKB_OK;
+    std::vector<uint32_t> h(3 * words16(n) + 4 * n_chunks);
+    memcpy(h.data(), e.col.data(), 4 * n);
+    memcpy(h.data() + words16(n), e.val.data(), 4 * n);
+    memcpy(h.data() + 2 * words16(n), e.pow.data(), 4 * n);
+    LineChunk* ch = reinterpret_cast<LineChunk*>(h.data() + 3 * words16(n));
+    for (size_t b = 0; b < batches.size(); b++)
+        for (size_t at = 0; at < batches[b].count; at += LINE_CHUNK)
+            *ch++ = {(uint32_t)b, (uint32_t)(batches[b].first + at), (uint32_t)(batches[b].count - at < LINE_CHUNK ? batches[b].count - at : LINE_CHUNK), 0u};
+    return upload_words(ctx, lines.d_col, h);
+}
+
+int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<NumeratorBatch>& batches, NumeratorLines& lines, qm31 random_coeff,
+                    const qm31* h_values, const uint32_t* d_values) {
+    DeviceGuard g(ctx);
+    const size_t n = e.col.size(), nb = batches.size();
+    if (!n) return ZKB_OK;
+    std::vector<qm31> c(nb);
+    for (size_t b = 0; b < nb; b++) {
+        c[b] = qm31_sub(conj_q(batches[b].point_y), batches[b].point_y);
+        if (batches[b].count && qm31_is_zero(c[b])) return set_error(ctx, ZKB_EINVAL, "sample point lies on the base-field circle");
+    }
+    std::vector<qm31> sums(2 * nb, qm31_zero());  // of p v and p conj v
+    if (n < LINES_ON_DEVICE_MIN) {
+        std::vector<qm31> pows(n);
+        size_t top = 0;
+        for (uint32_t p : e.pow) top = p > top ? p : top;
+        pows.resize(top + 1);
+        for (size_t k = 0; k <= top; k++) pows[k] = k ? qm31_mul(pows[k - 1], random_coeff) : qm31_one();
+        std::vector<uint32_t> h(5 * n);
+        for (size_t b = 0; b < nb; b++)
+            for (size_t j = batches[b].first; j < batches[b].first + batches[b].count; j++) {
+                const qm31 p = pows[e.pow[j]], v = h_values[e.val[j]], r = qm31_mul(p, c[b]);
+                memcpy(&h[4 * j], r.c, 16);
+                sums[2 * b] = qm31_add(sums[2 * b], qm31_mul(p, v));
+                sums[2 * b + 1] = qm31_add(sums[2 * b + 1], qm31_mul(p, conj_q(v)));
+            }
+        memcpy(&h[4 * n], e.col.data(), 4 * n);
+        if (int rc = upload_words(ctx, lines.d_c, h)) return rc;
+    } else {
+        size_t n_chunks = 0;
+        for (auto& b : batches) n_chunks += (b.count + LINE_CHUNK - 1) / LINE_CHUNK;
+        uint32_t *d_val = lines.d_col + words16(n), *d_pow = d_val + words16(n), *d_chunks = d_pow + words16(n), *d_sums = d_chunks + 4 * n_chunks;
+        // [the batches' c][alpha^0 ... alpha^255][alpha^(256 k)]
+        const size_t n_low = (size_t)1 << LINE_POW_LOG;
+        uint32_t top = 0;
+        for (uint32_t p : e.pow) top = p > top ? p : top;
+        const size_t n_high = (top >> LINE_POW_LOG) + 1;
+        std::vector<qm31> h(nb + n_low + n_high);
+        for (size_t b = 0; b < nb; b++) h[b] = c[b];
+        qm31* low = h.data() + nb;
+        for (size_t k = 0; k < n_low; k++) low[k] = k ? qm31_mul(low[k - 1], random_coeff) : qm31_one();
+        const qm31 step = qm31_mul(low[n_low - 1], random_coeff);
+        for (size_t k = 0; k < n_high; k++) low[n_low + k] = k ? qm31_mul(low[n_low + k - 1], step) : qm31_one();
+        uint32_t* d_tab = nullptr;
+        if (int rc = zkb_malloc(ctx, h.size() * 16, (void**)&d_tab)) return rc;
+        std::vector<uint32_t> hw(4 * h.size());
+        memcpy(hw.data(), h.data(), h.size() * 16);
+        int rc = upload_words(ctx, d_tab, hw);
+        cudaError_t err = cudaSuccess;
+        if (rc == ZKB_OK) err = cudaMemsetAsync(d_sums, 0, 64 * nb, ctx->stream);
+        if (rc == ZKB_OK && err == cudaSuccess) {
+            ProfScope prof(ctx, "quot_lines_kernel");
+            quot_lines_kernel<<<(unsigned)n_chunks, 256, 0, ctx->stream>>>(reinterpret_cast<const LineChunk*>(d_chunks), d_tab, d_val, d_pow, d_tab + 4 * nb, d_values,
+                                                                           lines.d_c, reinterpret_cast<unsigned long long*>(d_sums));
+            err = cudaGetLastError();
+        }
+        std::vector<unsigned long long> w(8 * nb);
+        if (rc == ZKB_OK && err == cudaSuccess) err = cudaMemcpyAsync(w.data(), d_sums, 64 * nb, cudaMemcpyDeviceToHost, ctx->stream);
+        if (rc == ZKB_OK && err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
+        zkb_free(ctx, d_tab);
+        if (rc) return rc;
+        if (err != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "quotient lines: %s", cudaGetErrorString(err));
+        for (size_t b = 0; b < nb; b++)
+            for (int q = 0; q < 4; q++) {
+                sums[2 * b].c[q] = (uint32_t)(w[8 * b + q] % P);
+                sums[2 * b + 1].c[q] = (uint32_t)(w[8 * b + 4 + q] % P);
+            }
+    }
+    for (size_t b = 0; b < nb; b++) {
+        batches[b].first_linear = qm31_sub(sums[2 * b + 1], sums[2 * b]);
+        batches[b].b_sum = qm31_sub(qm31_mul(c[b], sums[2 * b]), qm31_mul(batches[b].point_y, batches[b].first_linear));
+    }
+    return ZKB_OK;
+}
+
+int numerator_run(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const NumeratorLines& lines, const NumeratorBatch& batch, uint32_t* const out[4]) {
+    DeviceGuard g(ctx);
+    Secure4 o;
+    for (int q = 0; q < 4; q++) o.c[q] = out[q];
+    for (int c = 0; c < ncols; c++) ZKB_CHECK_ARG(ctx, cols[c] != nullptr && ((uintptr_t)cols[c] & 7) == 0);
+    void** d_cols;
+    if (int rc = stage_ptrs(ctx, (const void* const*)cols, ncols, &d_cols)) return rc;
+    return launch_numerators(ctx, cols, ncols, log_n, (const uint32_t* const*)d_cols, lines.d_col + batch.first, lines.d_c + 4 * batch.first, (int)batch.count,
+                             batch.b_sum, o, 0);
+}
+
+}  // namespace zk
+
+using namespace zk;
+
 extern "C" {
 
 int zkb_quot_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const uint32_t* h_col_idx,
@@ -264,40 +476,7 @@ int zkb_quot_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, in
         ZKB_CUDA(ctx, cudaMemcpyAsync(d_c, h_c, (size_t)k * 16, cudaMemcpyHostToDevice, ctx->stream));
         ZKB_CUDA(ctx, cudaMemcpyAsync(d_idx, h_col_idx, (size_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
     }
-    size_t n = (size_t)1 << log_n;
-    bool wide = n >= 4;
-    for (int q = 0; q < 4; q++) wide = wide && ((uintptr_t)out[q] & 15) == 0;
-    for (int c = 0; c < ncols; c++) wide = wide && ((uintptr_t)cols[c] & 15) == 0;
-    ProfScope prof(ctx, "quot_numerators_kernel");
-    // Few rows and many columns: split the columns over the grid's second dimension.
-    const unsigned row_blocks = (unsigned)((n / (wide ? 4 : 2) + 255) / 256);
-    const size_t scratch_free = ctx->scratch_words - (size_t)5 * k;
-    if (row_blocks < 148u && k >= 8 * NUM_TILE && 4 * n * 2 <= scratch_free) {
-        int S = (int)((2u * 148u + row_blocks - 1) / row_blocks);            // about two CTAs per SM
-        int chunk = ((k + S - 1) / S + NUM_TILE - 1) / NUM_TILE * NUM_TILE;  // whole tiles of columns
-        S = (k + chunk - 1) / chunk;
-        while ((size_t)S * 4 * n + 4 > scratch_free) { chunk += NUM_TILE; S = (k + chunk - 1) / chunk; }
-        uint32_t* partial = ctx->scratch + (size_t)5 * k + ((4 - ((size_t)5 * k & 3)) & 3);  // 16-byte aligned
-        dim3 grid(row_blocks, (unsigned)S);
-        if (wide)
-            quot_numerators_kernel<4><<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, n, o, chunk, partial);
-        else
-            quot_numerators_kernel<2><<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, n, o, chunk, partial);
-        ZKB_LAUNCH_CHECK(ctx);
-        quot_partial_sum_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, o);
-        ZKB_LAUNCH_CHECK(ctx);
-        return ZKB_OK;
-    }
-    if (wide)
-        quot_numerators_kernel<4><<<(unsigned)((n / 4 + 255) / 256), 256, 0, ctx->stream>>>(
-            (const uint32_t* const*)d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
-    else
-        quot_numerators_kernel<2><<<(unsigned)((n / 2 + 255) / 256), 256, 0, ctx->stream>>>(
-            (const uint32_t* const*)d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
-    ZKB_LAUNCH_CHECK(ctx);
-    return ZKB_OK;
+    return launch_numerators(ctx, cols, ncols, log_n, (const uint32_t* const*)d_cols, d_idx, d_c, k, b_sum, o, (size_t)5 * k);
 }
 
 int zkb_quot_combine(zkb_ctx* ctx, int n_acc, const uint32_t* const* acc_cols, const int* h_acc_log,
