@@ -263,52 +263,85 @@ __device__ __forceinline__ void item_sums_of(const GkrBatchItem& it, size_t firs
     }
 }
 
-// One launch of a layer enqueued at once: the items' passes, each CTA's sums to its group's accumulator; the CTA that finishes last
-// goes on with the transcript step of round `step` (-1: none, the masks and the way to the host).
-__global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items, int n_items, const uint32_t* __restrict__ eq, qm31 lambda,
+// The terms of `g` neighbouring lanes (a power of two up to 32) are one item's: they are added up, taken times the item's power of
+// alpha and added to its group's sums in shared memory, as 16-bit halves (32-bit adds, no carries to fold; 2^16 terms fit). By
+// whole warps; adds: the lane belongs to an item.
+__device__ __forceinline__ void add_to_group(uint32_t (*acc)[16], int g, bool adds, uint32_t oracle, uint32_t group, const uint32_t* __restrict__ alpha_pow, qm31 s0, qm31 s2) {
+    const int lane = threadIdx.x & 31, sub = lane & (g - 1);
+    const qm31 a = adds ? ldqb(alpha_pow, oracle) : qm31_zero();
+    for (int off = g >> 1; off > 0; off >>= 1) {
+        s0 = qm31_add(s0, shflb(s0, (lane & ~(g - 1)) | ((sub + off) & (g - 1))));
+        s2 = qm31_add(s2, shflb(s2, (lane & ~(g - 1)) | ((sub + off) & (g - 1))));
+    }
+    adds = adds && sub == 0;
+    const unsigned who = __ballot_sync(0xffffffffu, adds);
+    if (!who) return;
+    const qm31 v0 = qmul(s0, a), v2 = qmul(s2, a);
+    const uint32_t g0 = __shfl_sync(0xffffffffu, group, __ffs(who) - 1);
+    if (__all_sync(0xffffffffu, !adds || group == g0)) {  // one group in the warp: add up before going to memory
+        const qm31 a0 = warp_sum_m(adds ? v0 : qm31_zero()), a2 = warp_sum_m(adds ? v2 : qm31_zero());
+        uint32_t w = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) { w = (lane >> 1) == c ? a0.c[c] : w; w = (lane >> 1) == 4 + c ? a2.c[c] : w; }
+        if (lane < 16) atomicAdd(&acc[g0][lane], (lane & 1) ? w >> 16 : w & 0xffffu);
+    } else if (adds) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            atomicAdd(&acc[group][2 * c], v0.c[c] & 0xffffu);
+            atomicAdd(&acc[group][2 * c + 1], v0.c[c] >> 16);
+            atomicAdd(&acc[group][8 + 2 * c], v2.c[c] & 0xffffu);
+            atomicAdd(&acc[group][8 + 2 * c + 1], v2.c[c] >> 16);
+        }
+    }
+}
+
+// One launch of a layer enqueued at once. All items of a round have the same number of terms, 2^terms_log: from 2^8 on an item is
+// 2^ctas_log whole CTAs, below it 2^terms_log neighbouring threads, so that a late round of hundreds of instances is a few full CTAs and
+// not hundreds with a handful of threads at work (582 instances: 22 us a round, now 12). A CTA's sums go to their groups'
+// accumulators; the CTA that finishes last goes on with the transcript step of round `step` (-1: the masks, two threads an item, and
+// the way to the host).
+__global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items, int n_items, int terms_log, int ctas_log,
+                                                              const uint32_t* __restrict__ eq, qm31 lambda,
                                                               const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
                                                               uint32_t* __restrict__ records, unsigned int* __restrict__ done, int step, int n_rounds, GkrLayerOut host) {
-    __shared__ uint32_t sh[8][8];
+    __shared__ uint32_t acc[GKR_GROUPS][16];
     __shared__ GkrStepSm sm;
     __shared__ GkrStepConst consts;
-    const GkrBatchItem it = items[find_item(items, n_items, blockIdx.x)];
-    const uint32_t bx = blockIdx.x - it.first_block;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ bool last;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool packed = terms_log < 8;
+    const uint32_t flat = blockIdx.x * 256 + tid;
+    const uint32_t idx = packed ? flat >> terms_log : blockIdx.x >> ctas_log;
+    const uint32_t first = packed ? flat & ((1u << terms_log) - 1) : (blockIdx.x & ((1u << ctas_log) - 1)) * 256 + tid;
+    const bool live = idx < (uint32_t)n_items;
+    GkrBatchItem it{};
+    if (live) it = items[idx];
+    (&acc[0][0])[tid] = 0u;
+    (&acc[0][0])[256 + tid] = 0u;
     // The launch may start while the one before it is still in its transcript step (programmatic dependent launch): its CTAs get
     // here, with their items looked up, and wait for that grid to end before they touch anything it writes.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const qm31 r = ldqb(reinterpret_cast<const uint32_t*>(&st->challenge), 0);
     const uint32_t oracle = (uint32_t)it.slot, group = (uint32_t)(it.slot >> 32);
-    if (it.mode == 2) {
-        if (threadIdx.x < 2) fix_mask(it, threadIdx.x, r, host.masks + 16 * (size_t)oracle);
+    if (step < 0) {
+        if (live) fix_mask(it, (int)first, r, host.masks + 16 * (size_t)oracle);
+        __threadfence_system();
     } else {
         qm31 s0 = qm31_zero(), s2 = qm31_zero();
-        item_sums_of(it, (size_t)bx * blockDim.x + threadIdx.x, (size_t)it.blocks * blockDim.x, r, eq, lambda, s0, s2);
-        s0 = warp_sum_m(s0);
-        s2 = warp_sum_m(s2);
-        if (lane == 0) { stqb(sh[warp], 0, s0); stqb(sh[warp], 1, s2); }
+        if (live) item_sums_of(it, first, packed ? (size_t)1 << terms_log : (size_t)256 << ctas_log, r, eq, lambda, s0, s2);
         __syncthreads();
-        if (warp == 0) {
-            qm31 v = qm31_zero();
-            if (lane < 2) {
-#pragma unroll
-                for (int w = 0; w < 8; w++) v = qm31_add(v, ldqb(sh[w], lane));
-            }
-            v = qmul(v, ldqb(alpha_pow, oracle));
-            unsigned long long* const acc = st->acc[step & 1][group] + 4 * lane;
-            if (lane < 2) {
-#pragma unroll
-                for (int c = 0; c < 4; c++) atomicAdd(acc + c, (unsigned long long)v.c[c]);
-            }
-        }
+        add_to_group(acc, terms_log < 5 ? 1 << terms_log : 32, live, oracle, group, alpha_pow, s0, s2);
+        __syncthreads();
+        const uint32_t* const h = &acc[tid >> 3][2 * (tid & 7)];
+        const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
+        if (v) atomicAdd(&st->acc[step & 1][tid >> 3][tid & 7], v);
+        __threadfence();
     }
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
     if (warp != 0) return;
-    // Masks are written by two lanes of this warp too: one fence orders either before the count.
-    if (step < 0) __threadfence_system(); else __threadfence();
     __syncwarp();
-    unsigned int n = 0;
-    if (lane == 0) n = atomicAdd(done, 1u);
-    if (__shfl_sync(0xffffffffu, n, 0) != gridDim.x - 1) return;
+    if (!last) return;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __threadfence();
     if (lane == 0) *done = 0u;
@@ -402,9 +435,9 @@ __global__ void __launch_bounds__(256) gkr_batch_round_kernel(const GkrBatchItem
 // round then costs its launch, its first pass through cold instruction memory and its drain for a microsecond
 // of work. Here one CTA runs table after table (the fixes of a round and the first sums of the oracles that enter the next,
 // then the transcript step, as the launches of gkr_batch_layer do), with the transcript's state in shared memory. An item is worked
-// on by a group of `g` lanes (a power of two, 2 ... 32, chosen per table from the items' sizes), so a warp takes 32 / g items at a
+// on by a group of `g` lanes (a power of two, 1 ... 32: its terms), so a warp takes 32 / g items at a
 // time; the items' sums meet per group of oracles in shared memory, as 16-bit halves (32-bit adds, no carries to fold).
-// tables[t] = (first item, items, g, round of the transcript step + 1 or 0).
+// tables[t] = (first item, items, log2 g, round of the transcript step + 1 or 0).
 __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const GkrBatchItem* __restrict__ items_base, const uint4* __restrict__ tables,
                                                                           int n_tables, const uint32_t* __restrict__ eq, qm31 lambda,
                                                                           const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
@@ -413,28 +446,42 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
     __shared__ struct alignas(16) { uint32_t digest[8], n_draws, degenerate, pad[2]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
     GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
     __shared__ uint32_t acc[2][GKR_GROUPS][16];
-    __shared__ GkrStepConst consts;
+    __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];  // of the tail's rounds, in order
+    __shared__ uint4 tabs[GKR_LAYER_MAX_ROUNDS + 1];
     static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // what the host made: there before the first launch of the chain
+    if (tid < n_tables) tabs[tid] = tables[tid];
+    const int round0 = (int)tables[0].w - 1;
+    if (round0 >= 0)
+        for (int i = tid; i < 16 * (n_rounds - round0); i += GKR_TAIL_THREADS) reinterpret_cast<uint4*>(consts)[i] = reinterpret_cast<const uint4*>(rc + round0)[i];
+    __syncthreads();
+    // Every thread's first item of the next table is on its way while the step of the round at hand runs.
+    GkrBatchItem ahead{};
+    auto fetch = [&](int t) {
+        if (t >= n_tables) return;
+        const uint32_t idx = (uint32_t)tid >> tabs[t].z;
+        if (idx < tabs[t].y) ahead = items_base[tabs[t].x + idx];
+    };
+    fetch(0);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // see gkr_batch_layer_kernel
     for (int i = tid; i < (int)(sizeof(head_words) / 4); i += GKR_TAIL_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = __ldcg(reinterpret_cast<const uint32_t*>(st) + i);
     for (int i = tid; i < 2 * GKR_GROUPS * 16; i += GKR_TAIL_THREADS) (&acc[0][0][0])[i] = 0u;
     __syncthreads();
     if (warp == 0) batch_step_open(sm, s, lane);
     for (int t = 0; t < n_tables; t++) {
-        const uint4 tb = tables[t];
+        const uint4 tb = tabs[t];
         const GkrBatchItem* items = items_base + tb.x;
-        const int n_items = (int)tb.y, g = (int)tb.z, per_pass = GKR_TAIL_THREADS / g, round = (int)tb.w - 1;
+        const int n_items = (int)tb.y, g_log = (int)tb.z, g = 1 << g_log, per_pass = GKR_TAIL_THREADS >> g_log, round = (int)tb.w - 1;
         const qm31 r = s.challenge;
-        if (round >= 0 && tid >= GKR_TAIL_THREADS - 64) reinterpret_cast<uint32_t*>(&consts)[tid - (GKR_TAIL_THREADS - 64)] = reinterpret_cast<const uint32_t*>(rc + round)[tid - (GKR_TAIL_THREADS - 64)];
         const int sub = tid & (g - 1);
         for (int base = 0; base < n_items; base += per_pass) {
-            const int idx = base + tid / g;
+            const int idx = base + (tid >> g_log);
             const bool live = idx < n_items;
             qm31 s0 = qm31_zero(), s2 = qm31_zero();
             GkrBatchItem it{};
             if (live) {
-                it = items[idx];
+                it = base == 0 ? ahead : items[idx];
                 if (it.mode == 2) {
                     if (sub < 2) fix_mask(it, sub, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
                 } else {
@@ -442,31 +489,9 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
                 }
             }
             if (round < 0) continue;
-            for (int off = g >> 1; off > 0; off >>= 1) {
-                s0 = qm31_add(s0, shflb(s0, (lane & ~(g - 1)) | ((sub + off) & (g - 1))));
-                s2 = qm31_add(s2, shflb(s2, (lane & ~(g - 1)) | ((sub + off) & (g - 1))));
-            }
-            // every lane of the group has its item's sums: the first two take them times alpha^k to the oracles' group
-            const bool adds = live && sub < 2 && it.mode != 2;
-            const qm31 v = qmul(sub == 0 ? s0 : s2, adds ? ldqb(alpha_pow, (uint32_t)it.slot) : qm31_zero());
-            const uint32_t group = adds ? (uint32_t)(it.slot >> 32) : 0u;
-            const unsigned who = __ballot_sync(0xffffffffu, adds);
-            if (!who) continue;
-            const uint32_t g0 = __shfl_sync(0xffffffffu, group, __ffs(who) - 1);
-            if (__all_sync(0xffffffffu, !adds || group == g0)) {  // one group in the warp: add up before going to memory
-                const qm31 a0 = warp_sum_m(adds && sub == 0 ? v : qm31_zero()), a2 = warp_sum_m(adds && sub == 1 ? v : qm31_zero());
-                uint32_t w = 0;
-#pragma unroll
-                for (int c = 0; c < 4; c++) { w = (lane >> 1) == c ? a0.c[c] : w; w = (lane >> 1) == 4 + c ? a2.c[c] : w; }
-                if (lane < 16) atomicAdd(&acc[round & 1][g0][lane], (lane & 1) ? w >> 16 : w & 0xffffu);
-            } else if (adds) {
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    atomicAdd(&acc[round & 1][group][8 * sub + 2 * c], v.c[c] & 0xffffu);
-                    atomicAdd(&acc[round & 1][group][8 * sub + 2 * c + 1], v.c[c] >> 16);
-                }
-            }
+            add_to_group(acc[round & 1], g, live, (uint32_t)it.slot, (uint32_t)(it.slot >> 32), alpha_pow, s0, s2);
         }
+        fetch(t + 1);
         __syncthreads();
         if (round >= 0) {
             if (warp == 0) {
@@ -476,7 +501,7 @@ __global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const 
 #pragma unroll
                     for (int c = 0; c < 4; c++)
                         v[z].c[c] = m31_reduce64(acc[round & 1][lane][8 * z + 2 * c] + ((uint64_t)acc[round & 1][lane][8 * z + 2 * c + 1] << 16));
-                batch_step(sm, s, consts, v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)round);
+                batch_step(sm, s, consts[round - round0], v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)round);
             } else if (warp == 1) {
 #pragma unroll
                 for (int c = 0; c < 16; c++) acc[(round + 1) & 1][lane][c] = 0u;
@@ -665,11 +690,11 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
     if (n_rounds > GKR_LAYER_MAX_ROUNDS) return set_error(ctx, ZKB_EINVAL, "gkr batch: %d rounds in a layer", n_rounds);
     DeviceGuard g(ctx);
     // The small rounds at the end of the layer go to one single-CTA launch: from the first table on after which every table
-    // is at most GKR_TAIL_MAX_UNITS units of work (a unit = what one thread does in a pass: eight entries of a fix): one unit
-    // per thread of the CTA.
+    // is at most GKR_TAIL_MAX_UNITS terms (a term: eight entries of a fix): one per thread of the CTA.
     constexpr size_t GKR_TAIL_MAX_UNITS = 512;
     plan.ctas.assign((size_t)n_rounds + 1, 0u);
-    plan.lanes.assign((size_t)n_rounds + 1, 2u);
+    plan.terms_log.assign((size_t)n_rounds + 1, 0);
+    plan.ctas_log.assign((size_t)n_rounds + 1, 0);
     plan.tail_from = n_rounds + 1;
     bool tail = true;
     if (const char* e = getenv("ZKB_GKR_ROUNDS")) tail = strcmp(e, "launches") != 0;
@@ -677,16 +702,18 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
         GkrBatchItem* const t = plan.items.data() + plan.table_at[j];
         const int nt = (int)(plan.table_at[j + 1] - plan.table_at[j]);
         if (!nt) return set_error(ctx, ZKB_EINVAL, "gkr batch: round %d of the layer has no work", j);
-        plan.ctas[j] = plan_blocks(t, nt);
-        size_t units = 0, widest = 1;
-        for (int q = 0; q < nt; q++) {
+        for (int q = 0; q < nt; q++)
             t[q].slot = (t[q].slot & 0xffffffffull) | (unsigned long long)(n_rounds - (int)plan.n_vars[t[q].slot & 0xffffffffull]) << 32;
-            const size_t u = t[q].mode == 0 ? t[q].n / 4 : t[q].mode == 1 ? t[q].n / 8 : 2;
-            units += u;
-            widest = std::max(widest, u);
-        }
-        while (plan.lanes[j] < 32 && plan.lanes[j] < widest) plan.lanes[j] *= 2;
-        tail = tail && units <= GKR_TAIL_MAX_UNITS;
+        // n_rounds - j variables are left: 2^(that - 1) terms an item, and two entries of a mask each at the end. From 2^8 terms on
+        // an item takes whole CTAs, a thread up to eight terms as long as that leaves four CTAs an SM.
+        const int terms = j < n_rounds ? n_rounds - j - 1 : 1;
+        const size_t at_one_each = (size_t)nt << std::max(terms - 8, 0);
+        int per_thread = 0;
+        while (per_thread < 3 && terms - 8 > per_thread && (at_one_each >> (per_thread + 1)) >= 4 * 148) per_thread++;
+        plan.terms_log[j] = terms;
+        plan.ctas_log[j] = std::max(terms - 8 - per_thread, 0);
+        plan.ctas[j] = terms < 8 ? (uint32_t)((((size_t)nt << terms) + 255) / 256) : (uint32_t)nt << plan.ctas_log[j];
+        tail = tail && ((size_t)nt << terms) <= GKR_TAIL_MAX_UNITS;
         if (tail) plan.tail_from = j;
     }
     void* d = nullptr;
@@ -743,7 +770,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         uint32_t* tb = &blob[o_tables + 4 * (size_t)(j - plan.tail_from)];
         tb[0] = (uint32_t)plan.table_at[j];
         tb[1] = (uint32_t)(plan.table_at[j + 1] - plan.table_at[j]);
-        tb[2] = plan.lanes[j];
+        tb[2] = (uint32_t)std::min(plan.terms_log[j], 5);
         tb[3] = j < n_rounds ? (uint32_t)j + 1u : 0u;
     }
     void* d_blob_v = nullptr;
@@ -777,7 +804,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         cfg.gridDim = dim3(ctas);
         cfg.blockDim = dim3(256);
         cfg.numAttrs = pdl && launched ? 1 : 0;  // the first launch follows a copy, not a kernel of this chain
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items + plan.table_at[j], (int)(plan.table_at[j + 1] - plan.table_at[j]), eq_evals, lam,
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items + plan.table_at[j], (int)(plan.table_at[j + 1] - plan.table_at[j]), plan.terms_log[j], plan.ctas_log[j], eq_evals, lam,
                                (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_blob + o_records, ctx->batch_tickets + GKR_BATCH_MAX_ITEMS,
                                j < n_rounds ? j : -1, n_rounds, host);
         launched = true;

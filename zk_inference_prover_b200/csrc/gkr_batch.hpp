@@ -67,7 +67,8 @@ struct GkrLayerPlan {
     std::vector<uint32_t> n_vars;    // per oracle: it is active in the rounds with at most so many variables left
     std::vector<GkrBatchItem> items; // table after table; table j: the fixes of round j - 1, the first sums of those entering in round j (slot = oracle)
     std::vector<size_t> table_at;    // n_rounds + 2
-    std::vector<uint32_t> ctas, lanes;  // from here on filled by gkr_batch_plan
+    std::vector<uint32_t> ctas;      // from here on filled by gkr_batch_plan: per table, its launch
+    std::vector<int> terms_log, ctas_log;
     int tail_from = 0;
     const GkrBatchItem* d_items = nullptr;
 };

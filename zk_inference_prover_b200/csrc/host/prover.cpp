@@ -198,19 +198,27 @@ struct MerkleProver {
             mp.layers.push_back(B200Backend::commit_on_layer(d, 0, nullptr, {}));
             return mp;
         }
-        std::vector<const BaseColumn*> sorted(columns);
-        std::stable_sort(sorted.begin(), sorted.end(), [](const BaseColumn* a, const BaseColumn* b) { return a->len() > b->len(); });
-        uint32_t max_log = sorted[0]->log_size();
+        uint32_t max_log = 0, min_log = 32;
+        size_t count[33] = {0};
+        for (auto c : columns) {
+            const uint32_t log = c->log_size();
+            count[log]++;
+            max_log = std::max(max_log, log);
+            min_log = std::min(min_log, log);
+        }
         mp.layers.resize(max_log + 1);
         mp.layer_col_ptrs.resize(max_log + 1);
-        size_t pos = 0;
+        for (uint32_t log = 0; log <= max_log; log++) mp.layer_col_ptrs[log].reserve(count[log]);
+        for (auto c : columns) mp.layer_col_ptrs[c->log_size()].push_back(c->ptr());
         for (uint32_t log = max_log + 1; log-- > 0;) {
-            std::vector<const BaseColumn*> layer_cols;
-            while (pos < sorted.size() && sorted[pos]->log_size() == log) layer_cols.push_back(sorted[pos++]);
-            for (auto c : layer_cols) mp.layer_col_ptrs[log].push_back(c->ptr());
             if (log == max_log && leaves) mp.layers[log] = std::move(*leaves);
-            else mp.layers[log] = B200Backend::commit_on_layer(d, log, log == max_log ? nullptr : &mp.layers[log + 1], layer_cols);
-            if (log > 0 && log <= 10 && pos == sorted.size()) {
+            else {
+                mp.layers[log] = HashColumn(d, (size_t)8 << log);
+                d.check(zkb_merkle_layer(d.ctx(), (int)log, log == max_log ? nullptr : mp.layers[log + 1].ptr(), mp.layer_col_ptrs[log].data(),
+                                         (int)mp.layer_col_ptrs[log].size(), 1, mp.layers[log].ptr()));
+            }
+            const bool all = log <= min_log;  // no columns left below
+            if (log > 0 && log <= 10 && all) {
                 // no columns left below: the rest of the tree is nodes only, built in one launch
                 std::vector<uint32_t*> lower;
                 for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
@@ -219,7 +227,12 @@ struct MerkleProver {
             }
             // The layers below this one that hold no column (down to the next layer that has one, or to the last ten, which
             // the launch above builds): up to nine of them per launch.
-            const uint32_t floor_log = pos == sorted.size() ? 10u : sorted[pos]->log_size() + 1;
+            uint32_t floor_log = 10u;
+            if (!all) {
+                uint32_t next = log - 1;
+                while (!count[next]) next--;
+                floor_log = next + 1;
+            }
             while (log > floor_log && log >= 9) {
                 const uint32_t levels = std::min<uint32_t>(9, log - floor_log);
                 std::vector<uint32_t*> outs;
@@ -227,7 +240,7 @@ struct MerkleProver {
                 d.check(zkb_merkle_levels(d.ctx(), (int)log, mp.layers[log].ptr(), (int)levels, outs.data(), 1));
                 log -= levels;
             }
-            if (log > 0 && log <= 10 && pos == sorted.size() && mp.layers[log - 1].len() == 0) {
+            if (log > 0 && log <= 10 && all && mp.layers[log - 1].len() == 0) {
                 std::vector<uint32_t*> lower;
                 for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
                 top(log, mp.layers[log].ptr(), lower.data());
@@ -664,22 +677,30 @@ struct PcsProof {
         void reserve(size_t) {}
         void push_back(uint32_t v) { if (n < cap) out[n] = v; n++; }
         template <class It> void insert(int, It b, It e) {
-            size_t k = (size_t)(e - b);
-            if (n + k <= cap && k) copy_words(out + n, &*b, k);
+            const size_t k = (size_t)(e - b);
+            if (n + k <= cap && k) {
+                if (k < LONG_RUN) memcpy(out + n, &*b, 4 * k);
+                else runs.push_back({out + n, &*b, k});
+            }
             n += k;
         }
-        // A run of many megabytes (the queried values of a wide tree) is copied by four threads: one core moves about
-        // 10 GB/s, and the proof of a composed segment is 50 MB.
-        static void copy_words(uint32_t* dst, const uint32_t* src, size_t k) {
-            if (k < ((size_t)2 << 20)) { memcpy(dst, src, k * 4); return; }
-            const size_t part = (k + 3) / 4;
-            std::thread th[3];
-            for (int t = 0; t < 3; t++) {
-                size_t lo = (size_t)(t + 1) * part, hi = std::min(k, lo + part);
-                th[t] = std::thread([=] { if (lo < hi) memcpy(dst + lo, src + lo, (hi - lo) * 4); });
-            }
-            memcpy(dst, src, std::min(k, part) * 4);
-            for (auto& t : th) t.join();
+        // Long runs (the queried values of a wide tree's layers; their source outlives the sink) are copied at the end, by four threads
+        // in equal parts: one core moves some 6 GB/s into fresh pages, and the proof of a composed segment is 26 MB and more.
+        static constexpr size_t LONG_RUN = 4096;
+        struct Run { uint32_t* dst; const uint32_t* src; size_t n; };
+        std::vector<Run> runs;
+        void finish() {
+            size_t total = 0;
+            for (auto& r : runs) total += r.n;
+            parallel_chunks(total, (size_t)1 << 17, [&](size_t lo, size_t hi, size_t) {
+                size_t at = 0;
+                for (auto& r : runs) {
+                    const size_t a = std::max(lo, at), b = std::min(hi, at + r.n);
+                    if (a < b) memcpy(r.dst + (a - at), r.src + (a - at), 4 * (b - a));
+                    at += r.n;
+                }
+            });
+            runs.clear();
         }
         size_t size() const { return n; }
     };
@@ -766,7 +787,14 @@ struct CommitmentSchemeProver {
         CommitmentTreeProver t;
         if (slab) t.coeff_slab = std::move(*slab);
         std::map<uint32_t, std::vector<size_t>> by_log;
-        for (size_t i = 0; i < columns.size(); i++) by_log[columns[i].log_size()].push_back(i);
+        {
+            size_t count[33] = {0};
+            for (auto& c : columns) count[c.log_size()]++;
+            std::vector<size_t>* of[33] = {nullptr};
+            for (uint32_t log = 0; log <= 32; log++)
+                if (count[log]) { of[log] = &by_log[log]; of[log]->reserve(count[log]); }
+            for (size_t i = 0; i < columns.size(); i++) of[columns[i].log_size()]->push_back(i);
+        }
         t.evals.resize(columns.size());
         HashColumn leaves;
         bool have_leaves = false;
@@ -805,22 +833,31 @@ struct CommitmentSchemeProver {
         } else {
             for (auto& g : by_log) {
                 if (are_coeffs) break;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
-                std::vector<BaseColumn*> cols;
-                for (auto i : g.second) cols.push_back(&columns[i]);
-                B200Backend::interpolate_columns(d, cols);
+                std::vector<uint32_t*> cols;
+                cols.reserve(g.second.size());
+                for (auto i : g.second) cols.push_back(columns[i].ptr());
+                d.check(zkb_ifft_cols(d.ctx(), cols.data(), (int)cols.size(), (int)g.first));
             }
             mark(0);
             for (auto& g : by_log) {
-                std::vector<const BaseColumn*> cols;
-                for (auto i : g.second) cols.push_back(&columns[i]);
-                t.eval_slabs.emplace_back();
-                auto ev_cols = B200Backend::evaluate_polynomials(d, cols, config.fri.log_blowup_factor, &t.eval_slabs.back());
-                for (size_t k = 0; k < g.second.size(); k++) t.evals[g.second[k]] = std::move(ev_cols[k]);
+                // one allocation for the extended columns of a size (16-byte aligned each)
+                const size_t nc = g.second.size(), n_out = (size_t)1 << (g.first + config.fri.log_blowup_factor);
+                const size_t stride = std::max<size_t>(n_out, 4);
+                t.eval_slabs.emplace_back(d, nc * stride);
+                std::vector<const uint32_t*> src(nc);
+                std::vector<uint32_t*> dst(nc);
+                for (size_t k = 0; k < nc; k++) {
+                    src[k] = columns[g.second[k]].ptr();
+                    dst[k] = t.eval_slabs.back().ptr() + k * stride;
+                    t.evals[g.second[k]] = BaseColumn::view(d, dst[k], n_out);
+                }
+                d.check(zkb_lde_cols(d.ctx(), src.data(), (int)nc, (int)g.first, dst.data(), (int)(g.first + config.fri.log_blowup_factor)));
             }
         }
         mark(1);
         t.coeffs = std::move(columns);
         std::vector<const BaseColumn*> refs;
+        refs.reserve(t.evals.size());
         for (auto& e : t.evals) refs.push_back(&e);
         t.commitment = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr);
         ch.mix_root(t.commitment.root(d));
@@ -1842,6 +1879,7 @@ int zkb_shard_pcs_finish(zkb_shard_pcs* h, const uint32_t* const* h_parts, const
         proof.fri = s.fri_proof;
         PcsProof::RawSink w{h_out, cap};
         proof.write(w);
+        w.finish();
         w.insert(w.end(), s.ch.digest().begin(), s.ch.digest().end());
         *n_words = w.size();
         if (w.size() > cap) throw Error(ZKB_EINVAL, "zkb_shard_pcs_finish: output buffer too small");
@@ -1859,6 +1897,7 @@ static void commit_input_trees(Device& dev, zkb_ctx* ctx, CommitmentSchemeProver
         if (d_cols) {
             for (int t = 0; t < n_trees; t++) {
                 std::vector<BaseColumn> columns;
+                columns.reserve((size_t)tree_ncols[t]);
                 for (int c = 0; c < tree_ncols[t]; c++, flat++)
                     columns.push_back(BaseColumn::view(dev, d_cols[flat], (size_t)1 << col_logs[flat]));
                 prover.commit_evals(std::move(columns), ch);
@@ -1971,6 +2010,7 @@ static int pcs_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, uint
         hc.reset(new HostClock("pcs.write"));
         PcsProof::RawSink w{h_out, cap};  // straight into the caller's buffer: a proof of many columns is tens of megabytes
         proof.write(w);
+        w.finish();
         w.insert(w.end(), ch.digest().begin(), ch.digest().end());
         *n_words = w.size();
         hc.reset();
