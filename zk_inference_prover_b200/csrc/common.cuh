@@ -42,6 +42,7 @@ struct zkb_ctx {
     // Batched GKR rounds (gkr_batch.cu): per-item tickets (zero between launches: the last CTA of an item clears its own)
     // and a pinned landing buffer for the per-item results; both allocated on first use.
     unsigned int* batch_tickets = nullptr;
+    int batch_grid = 0;  // CTAs of gkr_batch_layer_kernel that are resident at once
     uint32_t* h_batch = nullptr;
     bool fri_tail_ready = false;   // fri_tail.cu: the same
     bool res_ready = false;        // gkr_resident.cu: its kernels' attributes are set on this device

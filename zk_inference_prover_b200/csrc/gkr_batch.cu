@@ -7,9 +7,8 @@
 // size, and every item's eight result words (and, at the end of a layer, its two-entry mask) land in one
 // result array.
 //
-// A whole layer's sum-check is enqueued at once (gkr_batch_layer): the CTA that completes a round's launch goes on with the
-// transcript step (the batch's round polynomial, the channel, the challenge, the claims), the next launch reads the
-// challenge from device memory, and the small rounds at the end of a layer run in one single-CTA launch.
+// A whole layer's sum-check is one launch (gkr_batch_layer_begin): its CTAs take the rounds' tables one after the other, CTA 0 runs the
+// transcript step between them (the batch's round polynomial, the channel, the challenge, the claims).
 //
 //   mode 0  sum_as_poly_in_first_variable sums of the item's layer (first round of a layer's sum-check)
 //   mode 1  fix_first_variable with the round's challenge on every column, and the sums of the fixed layer
@@ -139,7 +138,6 @@ __device__ __forceinline__ void item_sums(const GkrBatchItem& it, size_t first, 
 // hashing alone, a launch with its step 27-40 us.)
 // What it can not tell is the length the combination keeps when its leading coefficient vanishes (that of its longest term, each
 // trimmed on its own): it raises a flag then, and the caller proves the batch again with the transcript on the host.
-constexpr int GKR_TAIL_THREADS = 512;
 constexpr int GKR_GROUPS = 32;  // rounds of a layer at most, so groups of oracles that enter together
 
 struct GkrStepConst {        // of a round; host-made
@@ -295,73 +293,246 @@ __device__ __forceinline__ void add_to_group(uint32_t (*acc)[16], int g, bool ad
     }
 }
 
-// One launch of a layer enqueued at once. All items of a round have the same number of terms, 2^terms_log: from 2^8 on an item is
-// 2^ctas_log whole CTAs, below it 2^terms_log neighbouring threads, so that a late round of hundreds of instances is a few full CTAs and
-// not hundreds with a handful of threads at work (582 instances: 22 us a round, now 12). A CTA's sums go to their groups'
-// accumulators; the CTA that finishes last goes on with the transcript step of round `step` (-1: the masks, two threads an item, and
-// the way to the host).
-__global__ void __launch_bounds__(256) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items, int n_items, int terms_log, int ctas_log,
-                                                              const uint32_t* __restrict__ eq, qm31 lambda,
-                                                              const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
-                                                              uint32_t* __restrict__ records, unsigned int* __restrict__ done, int step, int n_rounds, GkrLayerOut host) {
-    __shared__ uint32_t acc[GKR_GROUPS][16];
+// ---- a layer in one launch
+//
+// A cooperative launch of up to two CTAs an SM runs all tables of a layer. Measured with a launch per round: of the 26,500 cycles (14 us)
+// that every round of a small batch took, whatever its size, half were the fetching of code that the SM at hand had not run
+// yet (the pass 14,500 cycles cold and 6,300 warm, the transcript step 12,000 and 8,000) and the rest of the gap the launch
+// itself; a round in one CTA took 9.3 us warm. Here the code stays warm in every SM, CTA 0 keeps the transcript in shared memory and
+// what goes round in a round is a count of arrivals and a challenge.
+//
+// A pass has two forms. With many terms a thread takes whole terms (bound by their 18 products). With few, what counts is the length of
+// the chain: four lanes take a term, one for each of its four entries, and every product is half of a pair (product_pair): a
+// sixth of the instructions and six products one after the other.
+//
+// The waits end: every CTA is resident (the launch is refused otherwise), a CTA waits only for what the others do before they wait
+// themselves, and after SPIN_LIMIT polls (about a second) it gives up and leaves; the host then sees no layer number and reports it.
+constexpr int GKR_THREADS = 256;
+constexpr uint32_t SPIN_LIMIT = 1u << 21;
+
+struct alignas(16) GkrTable {
+    uint32_t first, n_items;  // its items
+    int terms_log;            // log2 of the terms an item has
+    int form;                 // 0: a thread per term, 1: four lanes per term, 2: masks, two threads an item
+    int run_log;              // form 0, items of 2^8 terms and more: a chunk is 2^run_log terms a thread
+    uint32_t chunks, ctas;    // pieces of work, CTAs that take them in turn
+    uint32_t later;           // the most CTAs a later table has
+};
+static_assert(sizeof(GkrTable) == 32, "GkrTable layout");
+
+struct alignas(16) GkrSync {  // zero at launch
+    uint32_t count[GKR_LAYER_MAX_ROUNDS + 1];   // CTAs done with the table
+    uint32_t slot[GKR_LAYER_MAX_ROUNDS + 1][4];  // the challenge the table folds with; the top bit of a word: it is there
+};
+
+struct qm31_pair { qm31 a, b; };
+__device__ __noinline__ qm31_pair product_pair(qm31 a0, qm31 a1, qm31 b0, qm31 b1) { return {qm31_mul(a0, a1), qm31_mul(b0, b1)}; }
+
+// The sums of `v` over the warp's lanes with even and odd `which` go to the group's accumulator; lanes that do not add hold `adds` false.
+__device__ __forceinline__ void add_quad_terms(uint32_t (*acc)[16], bool adds, int which, uint32_t group, qm31 v) {
+    const int lane = threadIdx.x & 31;
+    const unsigned who = __ballot_sync(0xffffffffu, adds);
+    if (!who) return;
+    const uint32_t g0 = __shfl_sync(0xffffffffu, group, __ffs(who) - 1);
+    if (__all_sync(0xffffffffu, !adds || group == g0)) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const uint32_t e = warp_sum_m31(adds && which == 0 ? v.c[c] : 0u), o = warp_sum_m31(adds && which == 1 ? v.c[c] : 0u);
+            w = (lane >> 1) == c ? e : w;
+            w = (lane >> 1) == 4 + c ? o : w;
+        }
+        if (lane < 16) atomicAdd(&acc[g0][lane], (lane & 1) ? w >> 16 : w & 0xffffu);
+    } else if (adds) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            atomicAdd(&acc[group][8 * which + 2 * c], v.c[c] & 0xffffu);
+            atomicAdd(&acc[group][8 * which + 2 * c + 1], v.c[c] >> 16);
+        }
+    }
+}
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int n_tables,
+                                                                         const uint32_t* __restrict__ eq, qm31 lambda, const uint32_t* __restrict__ alpha_pow,
+                                                                         GkrStepState* st, GkrSync* sync, const GkrStepConst* __restrict__ rc,
+                                                                         uint32_t* records, int n_rounds, GkrLayerOut host) {
+    __shared__ uint32_t sums[GKR_GROUPS][16];  // of the pass at hand; zero before it
+    __shared__ GkrTable tabs[GKR_LAYER_MAX_ROUNDS + 1];
+    __shared__ qm31 r_sh;
+    __shared__ bool gave_up;
+    // CTA 0 only: the transcript
     __shared__ GkrStepSm sm;
-    __shared__ GkrStepConst consts;
-    __shared__ bool last;
+    __shared__ struct alignas(16) { uint32_t digest[8], n_draws, degenerate, pad[2]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
+    GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
+    __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];
+    static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool packed = terms_log < 8;
-    const uint32_t flat = blockIdx.x * 256 + tid;
-    const uint32_t idx = packed ? flat >> terms_log : blockIdx.x >> ctas_log;
-    const uint32_t first = packed ? flat & ((1u << terms_log) - 1) : (blockIdx.x & ((1u << ctas_log) - 1)) * 256 + tid;
-    const bool live = idx < (uint32_t)n_items;
-    GkrBatchItem it{};
-    if (live) it = items[idx];
-    (&acc[0][0])[tid] = 0u;
-    (&acc[0][0])[256 + tid] = 0u;
-    // The launch may start while the one before it is still in its transcript step (programmatic dependent launch): its CTAs get
-    // here, with their items looked up, and wait for that grid to end before they touch anything it writes.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const qm31 r = ldqb(reinterpret_cast<const uint32_t*>(&st->challenge), 0);
-    const uint32_t oracle = (uint32_t)it.slot, group = (uint32_t)(it.slot >> 32);
-    if (step < 0) {
-        if (live) fix_mask(it, (int)first, r, host.masks + 16 * (size_t)oracle);
-        __threadfence_system();
-    } else {
-        qm31 s0 = qm31_zero(), s2 = qm31_zero();
-        if (live) item_sums_of(it, first, packed ? (size_t)1 << terms_log : (size_t)256 << ctas_log, r, eq, lambda, s0, s2);
-        __syncthreads();
-        add_to_group(acc, terms_log < 5 ? 1 << terms_log : 32, live, oracle, group, alpha_pow, s0, s2);
-        __syncthreads();
-        const uint32_t* const h = &acc[tid >> 3][2 * (tid & 7)];
-        const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
-        if (v) atomicAdd(&st->acc[step & 1][tid >> 3][tid & 7], v);
-        __threadfence();
+    const bool lead = blockIdx.x == 0;
+    for (int i = tid; i < 2 * n_tables; i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
+    for (int i = tid; i < GKR_GROUPS * 16; i += GKR_THREADS) (&sums[0][0])[i] = 0u;
+    if (tid == 0) gave_up = false;
+    if (lead) {
+        for (int i = tid; i < 16 * n_rounds; i += GKR_THREADS) reinterpret_cast<uint4*>(consts)[i] = reinterpret_cast<const uint4*>(rc)[i];
+        for (int i = tid; i < (int)(sizeof(head_words) / 4); i += GKR_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = reinterpret_cast<const uint32_t*>(st)[i];
     }
     __syncthreads();
-    if (tid == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
-    if (warp != 0) return;
-    __syncwarp();
-    if (!last) return;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __threadfence();
-    if (lane == 0) *done = 0u;
-    if (step < 0) {
-        layer_out_words(host, records, n_rounds, st, lane, 32);
-        __threadfence_system();
-        __syncwarp();
-        if (lane == 0) *host.flag = host.id;
-        return;
-    }
-    if (lane < 16) reinterpret_cast<uint4*>(&consts)[lane] = reinterpret_cast<const uint4*>(rc + step)[lane];
-    batch_step_open(sm, *st, lane);
-    unsigned long long a[8];
+    if (lead && warp == 0) batch_step_open(sm, s, lane);
+    for (int t = 0; t < n_tables; t++) {
+        const GkrTable tb = tabs[t];
+        if (blockIdx.x >= tb.ctas) {
+            if (blockIdx.x >= tb.later) return;
+            continue;
+        }
+        const GkrBatchItem* const items = items_base + tb.first;
+        const bool step = t < n_rounds;
+        // what does not depend on the challenge: the first piece's item, in the small form its factor of the sums
+        uint32_t chunk = blockIdx.x;
+        GkrBatchItem it{};
+        uint32_t term = 0;
+        bool live = false;
+        qm31 ea = qm31_zero();
+        auto look_up = [&]() {  // forms 1 and 2
+            const uint32_t flat = chunk * GKR_THREADS + tid;
+            const uint32_t at = tb.form == 1 ? flat >> 2 : flat;
+            term = at & ((1u << tb.terms_log) - 1);
+            live = (at >> tb.terms_log) < tb.n_items;
+            if (live) it = items[at >> tb.terms_log];
+            if (tb.form == 1 && live) ea = qmul(ldqb(eq, term), ldqb(alpha_pow, (uint32_t)it.slot));
+        };
+        if (tb.form != 0) look_up();
+        if (!lead && t > 0) {
+            if (tid < 4) {
+                uint32_t w = ld_acquire(&sync->slot[t][tid]);
+                for (uint32_t spin = 0; !(w >> 31) && spin < SPIN_LIMIT; spin++) w = ld_acquire(&sync->slot[t][tid]);
+                if (!(w >> 31)) gave_up = true;
+                r_sh.c[tid] = w & 0x7fffffffu;
+            }
+            __syncthreads();
+            if (gave_up) return;
+        }
+        const qm31 r = lead ? s.challenge : r_sh;
+        if (tb.form == 1) {
+            for (;;) {
+                const int q = lane & 3;
+                const uint32_t group = (uint32_t)(it.slot >> 32);
+                const size_t nt = (size_t)1 << tb.terms_log, o = 2 * ((size_t)(q >> 1) * nt + term) + (q & 1);
+                const bool nums = it.kind == ZKB_GKR_LOGUP_GENERIC || it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES, base = it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES;
+                qm31 x = qm31_zero(), u = qm31_one();  // the entry's denominator and numerator
+                if (live) {
+                    x = ldqb(it.den, o);
+                    if (nums) u = base ? qm31_from_m31(it.num[o]) : ldqb(it.num, o);
+                    if (it.mode == 1) {
+                        const qm31 x1 = ldqb(it.den, o + 4 * nt);
+                        const qm31 u1 = !nums ? u : base ? qm31_from_m31(it.num[o + 4 * nt]) : ldqb(it.num, o + 4 * nt);
+                        const qm31_pair p = product_pair(r, qm31_sub(x1, x), r, qm31_sub(u1, u));
+                        x = qm31_add(x, p.a);
+                        u = qm31_add(u, p.b);
+                        stqb(it.den_out, o, x);
+                        if (nums) stqb(it.num_out, o, u);
+                    }
+                }
+                // lanes 2 and 3 go on with the entries' values at two
+                const qm31 x0 = shflb(x, lane & ~2), u0 = shflb(u, lane & ~2);
+                if (q & 2) { x = qm31_sub(qm31_dbl(x), x0); u = qm31_sub(qm31_dbl(u), u0); }
+                const qm31 xp = shflb(x, lane ^ 1);
+                const qm31_pair p = product_pair(xp, u, x, xp);  // half of the numerator; the denominator
+                qm31 n = qm31_add(p.a, shflb(p.a, lane ^ 1));
+                const qm31 d = qmul(lambda, p.b);
+                const qm31 v = qmul(it.kind == ZKB_GKR_GRAND_PRODUCT ? p.b : qm31_add(n, d), ea);
+                add_quad_terms(sums, live && !(q & 1), q >> 1, group, v);
+                chunk += tb.ctas;
+                if (chunk >= tb.chunks) break;
+                look_up();
+            }
+        } else if (tb.form == 0) {
+            for (; chunk < tb.chunks; chunk += tb.ctas) {
+                qm31 s0 = qm31_zero(), s2 = qm31_zero();
+                const int whole = tb.terms_log - 8 - tb.run_log;  // log2 of an item's chunks
+                const uint32_t flat = chunk * GKR_THREADS + tid;
+                const uint32_t idx = tb.terms_log < 8 ? flat >> tb.terms_log : chunk >> whole;
+                live = idx < tb.n_items;
+                if (live) {
+                    it = items[idx];
+                    if (tb.terms_log < 8) item_sums_of(it, flat & ((1u << tb.terms_log) - 1), (size_t)1 << tb.terms_log, r, eq, lambda, s0, s2);
+                    else item_sums_of(it, (size_t)(chunk & ((1u << whole) - 1)) * GKR_THREADS + tid, (size_t)GKR_THREADS << whole, r, eq, lambda, s0, s2);
+                }
+                add_to_group(sums, tb.terms_log < 5 ? 1 << tb.terms_log : 32, live, (uint32_t)it.slot, (uint32_t)(it.slot >> 32), alpha_pow, s0, s2);
+            }
+        } else {
+            for (;;) {
+                if (live) fix_mask(it, (int)term, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
+                chunk += tb.ctas;
+                if (chunk >= tb.chunks) break;
+                look_up();
+            }
+        }
+        __syncthreads();
+        if (tb.ctas > 1) {
+            if (step) {
+                uint32_t* const h = &sums[tid >> 3][2 * (tid & 7)];
+                const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
+                h[0] = h[1] = 0u;
+                if (v) atomicAdd(&st->acc[t & 1][tid >> 3][tid & 7], v);
+                __threadfence();
+            } else {
+                __threadfence_system();
+            }
+            __syncthreads();
+            if (!lead) {
+                if (tid == 0) { __threadfence(); atomicAdd(&sync->count[t], 1u); }
+                continue;
+            }
+            if (tid == 0) {
+                uint32_t n = ld_acquire(&sync->count[t]);
+                for (uint32_t spin = 0; n != tb.ctas - 1 && spin < SPIN_LIMIT; spin++) n = ld_acquire(&sync->count[t]);
+                if (n != tb.ctas - 1) gave_up = true;
+            }
+            __syncthreads();
+            if (gave_up) return;
+        }
+        // CTA 0 from here on
+        if (!step) break;
+        if (warp == 0) {
+            qm31 v[2];
+            if (tb.ctas > 1) {
+                unsigned long long a[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        a[c] = __ldcg(&st->acc[step & 1][lane][c]);
-        st->acc[step & 1][lane][c] = 0ull;  // for the round after the next
+                for (int c = 0; c < 8; c++) {
+                    a[c] = __ldcg(&st->acc[t & 1][lane][c]);
+                    st->acc[t & 1][lane][c] = 0ull;  // for the round after the next
+                }
+                v[0] = acc_value(a);
+                v[1] = acc_value(a + 4);
+            } else {
+#pragma unroll
+                for (int z = 0; z < 2; z++)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) v[z].c[c] = m31_reduce64(sums[lane][8 * z + 2 * c] + ((uint64_t)sums[lane][8 * z + 2 * c + 1] << 16));
+#pragma unroll
+                for (int c = 0; c < 16; c++) sums[lane][c] = 0u;
+            }
+            batch_step(sm, s, consts[t], v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)t);
+            if (tb.later > 1) {
+                __threadfence();
+                __syncwarp();
+                if (lane < 4) *reinterpret_cast<volatile uint32_t*>(&sync->slot[t + 1][lane]) = s.challenge.c[lane] | 0x80000000u;
+            }
+        }
+        __syncthreads();
     }
-    batch_step(sm, *st, consts, acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)step);
-    batch_step_close(sm, st, st->degenerate, lane);
+    if (!lead) return;
+    if (warp == 0) batch_step_close(sm, st, s.degenerate, lane);
+    __threadfence();
+    __syncthreads();
+    layer_out_words(host, records, n_rounds, st, tid, GKR_THREADS);
+    __threadfence_system();
+    __syncthreads();
+    if (tid == 0) *host.flag = host.id;
 }
 
 // ---- a single round with its results to the host
@@ -428,94 +599,6 @@ __global__ void __launch_bounds__(256) gkr_batch_round_kernel(const GkrBatchItem
         if (threadIdx.x == 0) tickets[idx] = 0u;
         item_done(done, n_items, flag, round_id);
     }
-}
-
-// The small rounds of a layer in ONE launch. All active oracles of a round have the same number of variables left, so late
-// in a layer's sum-check (and in the layers near the outputs throughout) a round is a few thousand entries: a launch per
-// round then costs its launch, its first pass through cold instruction memory and its drain for a microsecond
-// of work. Here one CTA runs table after table (the fixes of a round and the first sums of the oracles that enter the next,
-// then the transcript step, as the launches of gkr_batch_layer do), with the transcript's state in shared memory. An item is worked
-// on by a group of `g` lanes (a power of two, 1 ... 32: its terms), so a warp takes 32 / g items at a
-// time; the items' sums meet per group of oracles in shared memory, as 16-bit halves (32-bit adds, no carries to fold).
-// tables[t] = (first item, items, log2 g, round of the transcript step + 1 or 0).
-__global__ void __launch_bounds__(GKR_TAIL_THREADS) gkr_batch_tail_kernel(const GkrBatchItem* __restrict__ items_base, const uint4* __restrict__ tables,
-                                                                          int n_tables, const uint32_t* __restrict__ eq, qm31 lambda,
-                                                                          const uint32_t* __restrict__ alpha_pow, GkrStepState* st, const GkrStepConst* __restrict__ rc,
-                                                                          uint32_t* __restrict__ records, int n_rounds, GkrLayerOut host) {
-    __shared__ GkrStepSm sm;
-    __shared__ struct alignas(16) { uint32_t digest[8], n_draws, degenerate, pad[2]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
-    GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
-    __shared__ uint32_t acc[2][GKR_GROUPS][16];
-    __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];  // of the tail's rounds, in order
-    __shared__ uint4 tabs[GKR_LAYER_MAX_ROUNDS + 1];
-    static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // what the host made: there before the first launch of the chain
-    if (tid < n_tables) tabs[tid] = tables[tid];
-    const int round0 = (int)tables[0].w - 1;
-    if (round0 >= 0)
-        for (int i = tid; i < 16 * (n_rounds - round0); i += GKR_TAIL_THREADS) reinterpret_cast<uint4*>(consts)[i] = reinterpret_cast<const uint4*>(rc + round0)[i];
-    __syncthreads();
-    // Every thread's first item of the next table is on its way while the step of the round at hand runs.
-    GkrBatchItem ahead{};
-    auto fetch = [&](int t) {
-        if (t >= n_tables) return;
-        const uint32_t idx = (uint32_t)tid >> tabs[t].z;
-        if (idx < tabs[t].y) ahead = items_base[tabs[t].x + idx];
-    };
-    fetch(0);
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // see gkr_batch_layer_kernel
-    for (int i = tid; i < (int)(sizeof(head_words) / 4); i += GKR_TAIL_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = __ldcg(reinterpret_cast<const uint32_t*>(st) + i);
-    for (int i = tid; i < 2 * GKR_GROUPS * 16; i += GKR_TAIL_THREADS) (&acc[0][0][0])[i] = 0u;
-    __syncthreads();
-    if (warp == 0) batch_step_open(sm, s, lane);
-    for (int t = 0; t < n_tables; t++) {
-        const uint4 tb = tabs[t];
-        const GkrBatchItem* items = items_base + tb.x;
-        const int n_items = (int)tb.y, g_log = (int)tb.z, g = 1 << g_log, per_pass = GKR_TAIL_THREADS >> g_log, round = (int)tb.w - 1;
-        const qm31 r = s.challenge;
-        const int sub = tid & (g - 1);
-        for (int base = 0; base < n_items; base += per_pass) {
-            const int idx = base + (tid >> g_log);
-            const bool live = idx < n_items;
-            qm31 s0 = qm31_zero(), s2 = qm31_zero();
-            GkrBatchItem it{};
-            if (live) {
-                it = base == 0 ? ahead : items[idx];
-                if (it.mode == 2) {
-                    if (sub < 2) fix_mask(it, sub, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
-                } else {
-                    item_sums_of(it, sub, g, r, eq, lambda, s0, s2);
-                }
-            }
-            if (round < 0) continue;
-            add_to_group(acc[round & 1], g, live, (uint32_t)it.slot, (uint32_t)(it.slot >> 32), alpha_pow, s0, s2);
-        }
-        fetch(t + 1);
-        __syncthreads();
-        if (round >= 0) {
-            if (warp == 0) {
-                qm31 v[2];
-#pragma unroll
-                for (int z = 0; z < 2; z++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        v[z].c[c] = m31_reduce64(acc[round & 1][lane][8 * z + 2 * c] + ((uint64_t)acc[round & 1][lane][8 * z + 2 * c + 1] << 16));
-                batch_step(sm, s, consts[round - round0], v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)round);
-            } else if (warp == 1) {
-#pragma unroll
-                for (int c = 0; c < 16; c++) acc[(round + 1) & 1][lane][c] = 0u;
-            }
-            __syncthreads();
-        }
-    }
-    if (warp == 0) batch_step_close(sm, st, s.degenerate, lane);
-    __threadfence();
-    __syncthreads();
-    layer_out_words(host, records, n_rounds, st, tid, GKR_TAIL_THREADS);
-    __threadfence_system();
-    __syncthreads();
-    if (tid == 0) *host.flag = host.id;
 }
 
 // The towers of all instances, ten levels a launch (gkr_tower.cuh); an item's layers lie one after the other from num_out / den_out
@@ -587,6 +670,10 @@ static int batch_buffers(zkb_ctx* ctx) {
     // tickets per item, then the launch's count of completed items
     ZKB_CUDA(ctx, cudaMalloc(&ctx->batch_tickets, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int)));
     ZKB_CUDA(ctx, cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream));
+    int sms = 0, per_sm = 0;
+    ZKB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    ZKB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gkr_batch_layer_kernel, GKR_THREADS, 0));
+    ctx->batch_grid = sms * std::min(per_sm, 2);
     ZKB_CUDA(ctx, cudaMallocHost(&ctx->h_batch, H_BATCH_WORDS * 4));
     ctx->h_batch[H_BATCH_FLAG] = 0;
     ctx->batch_round = 0;
@@ -689,32 +776,36 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
     if (plan.n_vars.size() > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
     if (n_rounds > GKR_LAYER_MAX_ROUNDS) return set_error(ctx, ZKB_EINVAL, "gkr batch: %d rounds in a layer", n_rounds);
     DeviceGuard g(ctx);
-    // The small rounds at the end of the layer go to one single-CTA launch: from the first table on after which every table
-    // is at most GKR_TAIL_MAX_UNITS terms (a term: eight entries of a fix): one per thread of the CTA.
-    constexpr size_t GKR_TAIL_MAX_UNITS = 512;
-    plan.ctas.assign((size_t)n_rounds + 1, 0u);
-    plan.terms_log.assign((size_t)n_rounds + 1, 0);
-    plan.ctas_log.assign((size_t)n_rounds + 1, 0);
-    plan.tail_from = n_rounds + 1;
-    bool tail = true;
-    if (const char* e = getenv("ZKB_GKR_ROUNDS")) tail = strcmp(e, "launches") != 0;
+    if (int rc = batch_buffers(ctx)) return rc;
+    const uint32_t grid = (uint32_t)ctx->batch_grid;
+    plan.tables.assign((sizeof(GkrTable) / 4) * ((size_t)n_rounds + 1), 0u);
+    GkrTable* const tables = reinterpret_cast<GkrTable*>(plan.tables.data());
+    uint32_t later = 0;
     for (int j = n_rounds; j >= 0; j--) {
         GkrBatchItem* const t = plan.items.data() + plan.table_at[j];
         const int nt = (int)(plan.table_at[j + 1] - plan.table_at[j]);
         if (!nt) return set_error(ctx, ZKB_EINVAL, "gkr batch: round %d of the layer has no work", j);
         for (int q = 0; q < nt; q++)
             t[q].slot = (t[q].slot & 0xffffffffull) | (unsigned long long)(n_rounds - (int)plan.n_vars[t[q].slot & 0xffffffffull]) << 32;
-        // n_rounds - j variables are left: 2^(that - 1) terms an item, and two entries of a mask each at the end. From 2^8 terms on
-        // an item takes whole CTAs, a thread up to eight terms as long as that leaves four CTAs an SM.
-        const int terms = j < n_rounds ? n_rounds - j - 1 : 1;
-        const size_t at_one_each = (size_t)nt << std::max(terms - 8, 0);
-        int per_thread = 0;
-        while (per_thread < 3 && terms - 8 > per_thread && (at_one_each >> (per_thread + 1)) >= 4 * 148) per_thread++;
-        plan.terms_log[j] = terms;
-        plan.ctas_log[j] = std::max(terms - 8 - per_thread, 0);
-        plan.ctas[j] = terms < 8 ? (uint32_t)((((size_t)nt << terms) + 255) / 256) : (uint32_t)nt << plan.ctas_log[j];
-        tail = tail && ((size_t)nt << terms) <= GKR_TAIL_MAX_UNITS;
-        if (tail) plan.tail_from = j;
+        GkrTable& tb = tables[j];
+        tb.first = (uint32_t)plan.table_at[j];
+        tb.n_items = (uint32_t)nt;
+        // n_rounds - j variables are left: 2^(that - 1) terms an item; at the end two entries of a mask each
+        tb.terms_log = j < n_rounds ? n_rounds - j - 1 : 1;
+        const size_t terms = (size_t)nt << tb.terms_log;
+        // Four lanes a term while that is at most two passes of the whole grid: a pass of this form is a third of the other's latency,
+        // and a third more work.
+        tb.form = j == n_rounds ? 2 : 4 * terms <= 2 * (size_t)grid * GKR_THREADS ? 1 : 0;
+        // Whole items of 2^8 terms and more: a thread takes up to eight terms for one reduction, as long as four pieces per CTA remain.
+        tb.run_log = 0;
+        if (tb.form == 0)
+            while (tb.run_log < 3 && tb.terms_log - 8 > tb.run_log && (terms >> (8 + tb.run_log + 1)) >= 4 * (size_t)grid) tb.run_log++;
+        const size_t chunks = tb.form == 0 && tb.terms_log >= 8 ? terms >> (8 + tb.run_log) : ((tb.form == 1 ? 4 * terms : terms) + GKR_THREADS - 1) / GKR_THREADS;
+        tb.chunks = (uint32_t)chunks;
+        // Up to two pieces stay in CTA 0: sending the sums and the challenge round costs as much as another pass.
+        tb.ctas = chunks <= 2 ? 1u : (uint32_t)std::min<size_t>(chunks, grid);
+        tb.later = later;
+        later = std::max(later, tb.ctas);
     }
     void* d = nullptr;
     if (int rc = stage_blob(ctx, plan.items.data(), plan.items.size() * sizeof(GkrBatchItem), &d)) return rc;
@@ -727,11 +818,11 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     DeviceGuard g(ctx);
     if (int rc = batch_buffers(ctx)) return rc;
     const size_t K = plan.n_vars.size();
-    const int n_rounds = plan.n_rounds, n_tail_tables = n_rounds + 1 - plan.tail_from;
-    // The staged block: the transcript's state, the powers of alpha, the rounds' constants, the tail's tables, room for the rounds'
-    // records (every part a multiple of four words).
-    const size_t o_state = 0, o_alpha = sizeof(GkrStepState) / 4, o_rounds = o_alpha + 4 * K, o_tables = o_rounds + (sizeof(GkrStepConst) / 4) * (size_t)n_rounds;
-    const size_t o_records = o_tables + 4 * ((size_t)n_rounds + 1);
+    const int n_rounds = plan.n_rounds;
+    // The staged block: the transcript's state, the CTAs' meeting place, the powers of alpha, the rounds' constants, the tables, room for
+    // the rounds' records (every part a multiple of four words).
+    const size_t o_state = 0, o_sync = sizeof(GkrStepState) / 4, o_alpha = o_sync + sizeof(GkrSync) / 4, o_rounds = o_alpha + 4 * K, o_tables = o_rounds + (sizeof(GkrStepConst) / 4) * (size_t)n_rounds;
+    const size_t o_records = o_tables + plan.tables.size();
     std::vector<uint32_t>& blob = ctx_blob();
     blob.assign(o_records + GKR_LAYER_OUT_WORDS * (size_t)n_rounds, 0u);
     auto q4 = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
@@ -766,13 +857,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         c.entering = j + 1 < n_rounds ? qm31_mul_m31(entering[j + 1], half_pow) : qm31_zero();
         c.round = (uint32_t)j;
     }
-    for (int j = plan.tail_from; j <= n_rounds; j++) {
-        uint32_t* tb = &blob[o_tables + 4 * (size_t)(j - plan.tail_from)];
-        tb[0] = (uint32_t)plan.table_at[j];
-        tb[1] = (uint32_t)(plan.table_at[j + 1] - plan.table_at[j]);
-        tb[2] = (uint32_t)std::min(plan.terms_log[j], 5);
-        tb[3] = j < n_rounds ? (uint32_t)j + 1u : 0u;
-    }
+    memcpy(&blob[o_tables], plan.tables.data(), 4 * plan.tables.size());
     void* d_blob_v = nullptr;
     if (int rc = stage_blob(ctx, blob.data(), blob.size() * 4, &d_blob_v)) return rc;
     uint32_t* d_blob = static_cast<uint32_t*>(d_blob_v);
@@ -785,52 +870,28 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     host.masks = host.channel + 12;
     host.flag = reinterpret_cast<volatile unsigned int*>(ctx->h_batch + H_BATCH_FLAG);
     host.id = ++ctx->batch_round;
-    cudaError_t e = cudaSuccess;
-    // Each launch but the first is a programmatic dependent of the one before it (ZKB_GKR_PDL=0: plain stream order).
-    const char* pdl_env = getenv("ZKB_GKR_PDL");
-    const bool pdl = !(pdl_env && pdl_env[0] == '0') && !ctx->prof_on;
+    const GkrTable* const h_tables = reinterpret_cast<const GkrTable*>(plan.tables.data());
+    ProfScope prof(ctx, "gkr_batch_layer_kernel");
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails
+    attr[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.dynamicSmemBytes = 0;
+    cfg.gridDim = dim3(std::max(h_tables[0].ctas, h_tables[0].later));
+    cfg.blockDim = dim3(GKR_THREADS);
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
-    bool launched = false;
-    for (int j = 0; j < plan.tail_from && e == cudaSuccess; j++) {
-        const uint32_t ctas = plan.ctas[j];
-        ProfScope prof(ctx, ctas <= 8 ? "gkr_batch_layer_kernel(<=8 CTAs)" : ctas <= 128 ? "gkr_batch_layer_kernel(<=128 CTAs)"
-                                 : ctas <= 2048 ? "gkr_batch_layer_kernel(<=2048 CTAs)" : "gkr_batch_layer_kernel(>2048 CTAs)");
-        cfg.gridDim = dim3(ctas);
-        cfg.blockDim = dim3(256);
-        cfg.numAttrs = pdl && launched ? 1 : 0;  // the first launch follows a copy, not a kernel of this chain
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items + plan.table_at[j], (int)(plan.table_at[j + 1] - plan.table_at[j]), plan.terms_log[j], plan.ctas_log[j], eq_evals, lam,
-                               (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_blob + o_records, ctx->batch_tickets + GKR_BATCH_MAX_ITEMS,
-                               j < n_rounds ? j : -1, n_rounds, host);
-        launched = true;
-    }
-    if (n_tail_tables && e == cudaSuccess) {
-        ProfScope prof(ctx, "gkr_batch_tail_kernel");
-        cfg.gridDim = dim3(1);
-        cfg.blockDim = dim3(GKR_TAIL_THREADS);
-        cfg.numAttrs = pdl && launched ? 1 : 0;
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_tail_kernel, plan.d_items, reinterpret_cast<const uint4*>(d_blob + o_tables), n_tail_tables, eq_evals, lam,
-                               (const uint32_t*)(d_blob + o_alpha), d_state, d_consts, d_blob + o_records, n_rounds, host);
-    }
-    if (e != cudaSuccess) {
-        cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream);
-        return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
-    }
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, reinterpret_cast<const GkrTable*>(d_blob + o_tables), n_rounds + 1, eq_evals, lam,
+                                             (const uint32_t*)(d_blob + o_alpha), d_state, reinterpret_cast<GkrSync*>(d_blob + o_sync), d_consts, d_blob + o_records, n_rounds,
+                                             host);
+    if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
     return ZKB_OK;
 }
 
 int gkr_batch_layer_end(zkb_ctx* ctx, const GkrLayerPlan& plan, GkrLayerResult& res) {
     DeviceGuard g(ctx);
     const cudaError_t e = batch_wait(ctx, ctx->batch_round);
-    if (e != cudaSuccess) {
-        cudaMemsetAsync(ctx->batch_tickets, 0, (GKR_BATCH_MAX_ITEMS + 1) * sizeof(unsigned int), ctx->stream);
-        return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
-    }
+    if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
     res.records = ctx->h_batch;
     res.channel = res.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
     res.masks = res.channel + 12;

@@ -38,16 +38,14 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
                     uint32_t* h_results);
 
 
-// ---- a layer's whole sum-check enqueued at once (no host round trip per round)
+// ---- a layer's whole sum-check in one launch (no host round trip per round)
 //
 // What runs in a round depends on the oracles' sizes only, never on the transcript, so the host describes every round of a
-// layer's sum-check up front and the device keeps the transcript between the launches. Launch j (0 <= j <= rounds) carries the
-// fixes of round j - 1 (mode 1 / 2 items, the challenge read from device memory) and the first sums of the oracles that
-// enter in round j (mode 0 items); the CTA that completes the launch goes on with the transcript step of round j: the
-// batch's round polynomial from all oracles' sums, mixed into the channel, the challenge drawn, every oracle's claim and
-// correction updated. The launches of the small rounds at the end of the layer are replaced by one single-CTA launch that
-// runs the same tables one after the other. One copy brings back the round polynomials, the challenges, the masks and the
-// channel (sumcheck.rs:96-176 inside gkr_prover.rs:669-844).
+// layer's sum-check up front and the device keeps the transcript. Table j (0 <= j <= rounds) holds the fixes of round j - 1 (mode 1 / 2
+// items) and the first sums of the oracles that enter in round j (mode 0 items); between two tables comes the transcript step of round
+// j: the batch's round polynomial from all oracles' sums, mixed into the channel, the challenge drawn, every oracle's claim and
+// correction updated. The launch leaves the round polynomials, the challenges, the masks and the channel in page-locked
+// memory (sumcheck.rs:96-176 inside gkr_prover.rs:669-844).
 struct GkrRoundConst {
     // The basis of the round's polynomials (all active oracles have n_rem variables left, so their round polynomials are
     // r0 L0 + r1 L1 + r2 L2 over one basis): e0a = eq(0, y) / prod, e2a = eq(2, y) / prod, L[i] the coefficients (low first)
@@ -67,9 +65,7 @@ struct GkrLayerPlan {
     std::vector<uint32_t> n_vars;    // per oracle: it is active in the rounds with at most so many variables left
     std::vector<GkrBatchItem> items; // table after table; table j: the fixes of round j - 1, the first sums of those entering in round j (slot = oracle)
     std::vector<size_t> table_at;    // n_rounds + 2
-    std::vector<uint32_t> ctas;      // from here on filled by gkr_batch_plan: per table, its launch
-    std::vector<int> terms_log, ctas_log;
-    int tail_from = 0;
+    std::vector<uint32_t> tables;    // filled by gkr_batch_plan: how the kernel takes them
     const GkrBatchItem* d_items = nullptr;
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
