@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "count_cache.cuh"
 
 namespace zk {
 
@@ -182,7 +183,7 @@ __global__ void selectors_kernel(const uint32_t* __restrict__ flags, const uint3
 // ---------------------------------------------------------------------------------------------------
 struct RsGroup { uint32_t n, leaf_col, width, un, flat; };
 struct RsSlot { uint32_t a_sm, a_ef, b_sm, b_ef, base, o_sm, o_ef, from_slot; };
-struct RsMult { uint32_t* m; uint32_t n; };
+using RsMult = CountTable;
 struct RsArgs {
     const uint32_t* wit;
     const RsGroup* groups;
@@ -191,25 +192,27 @@ struct RsArgs {
     const int32_t* smul3;
     const int32_t* const* un2;
     const uint32_t* out_slot;
-    const uint32_t* order;        // slot indices sorted by level
-    const uint32_t* level_start;  // n_levels + 1 offsets into `order`
+    const uint32_t* level_start;  // the slots lie level by level: n_levels + 1 offsets
     uint32_t* const* cols;
+    uint32_t* col0;               // evenly spaced columns: the first one, and the distance in words
+    long long col_step;
     uint32_t* out_pat;
     int32_t* out_nat;
     int32_t* in_nat;
     RsMult m_pow, m_norm, m_val, m_frac, m_smul;
     const RsMult* m_un;
     uint32_t* counts;
-    uint32_t n_norm, n_smul, n_val, log_rows, live, n_groups, n_leaves, n_slots, n_levels, kmax, out_w;
+    uint32_t n_norm, n_smul, n_val, log_rows, live, n_groups, n_leaves, n_slots, n_levels, kmax, out_w, teams, flush_every;
 };
 constexpr uint32_t RS_DMAX = 12, RS_UMIN = 260, RS_BIAS = 134, RS_POW_ROWS = RS_DMAX + 1 + RS_UMIN;
 
-// One lookup: bump the table's multiplicity, or count the lookup as off the table. Lanes of a warp that hit the same
-// entry (a padded row's leaves all hit entry 0) are merged into one atomic.
+// One lookup: bump the table's multiplicity, or count the lookup as off the table (OFF_TABLE is larger than any table).
 __device__ __forceinline__ void lookup(const RsMult& t, uint32_t idx, uint32_t& off) {
-    if (idx >= t.n) { off++; return; }  // OFF_TABLE is larger than any table
-    uint32_t peers = __match_any_sync(__activemask(), idx);
-    if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(t.m + idx, (uint32_t)__popc(peers));
+    if (idx >= t.n) off++; else count_in_memory(t.m, idx);
+}
+template <int LOG>
+__device__ __forceinline__ void lookup(uint32_t* cache, const RsMult& t, uint32_t idx, uint32_t& off) {
+    if (idx >= t.n) off++; else count_cached<LOG>(cache, t.m, idx);
 }
 __device__ __forceinline__ uint32_t value_index(long long sm, long long ef) {  // val_table's row order: zero, then (ef, m7, sign)
     if (sm == 0 && ef == 0) return 0;
@@ -227,85 +230,116 @@ __device__ __forceinline__ uint32_t signed_significand_index(long long v) {
     unsigned long long a = (unsigned long long)(v < 0 ? -v : v);
     return (a < 128 || a >= 256) ? OFF_TABLE : 1u + (v < 0 ? 128u : 0u) + (uint32_t)(a - 128);
 }
-// The column table is never written by the kernel: its entries are fetched through the read-only path, so that the loads
-// of a slot's fourteen column addresses are independent of the stores between them (a plain load would have to be
-// ordered after every earlier store, one address at a time).
-__device__ __forceinline__ uint32_t* column(uint32_t* const* cols, uint32_t c) {
-    return reinterpret_cast<uint32_t*>(__ldg(reinterpret_cast<const unsigned long long*>(cols) + c));
+// Where a column begins. A program's columns usually are one allocation, evenly spaced: their addresses are then computed. Otherwise
+// they come from the table, which the kernel never writes: through the read-only path, so that the loads of a slot's
+// fourteen column addresses are independent of the stores between them (a plain load would have to be ordered after every
+// earlier store, one address at a time).
+template <bool EVEN>
+__device__ __forceinline__ uint32_t* column(const RsArgs& a, uint32_t c) {
+    if (EVEN) return a.col0 + (long long)c * a.col_step;
+    return reinterpret_cast<uint32_t*>(__ldg(reinterpret_cast<const unsigned long long*>(a.cols) + c));
 }
 // An operand as the (significand, exponent) it encodes. A slot's output exponent is clamped to [0, 0xfe] on the way
 // out of the slot while its cell keeps the unclamped value, so the clamp applies to slot sources only.
-__device__ __forceinline__ void operand(uint32_t* const* cols, uint32_t i, uint32_t c_sm, uint32_t c_ef, bool from_slot, long long& sm, long long& ef) {
+template <bool EVEN>
+__device__ __forceinline__ void operand(const RsArgs& a, uint32_t i, uint32_t c_sm, uint32_t c_ef, bool from_slot, long long& sm, long long& ef) {
     if (c_sm == OFF_TABLE) { sm = 0; ef = 0; return; }
-    const uint32_t *p_sm = column(cols, c_sm), *p_ef = column(cols, c_ef);
+    const uint32_t *p_sm = column<EVEN>(a, c_sm), *p_ef = column<EVEN>(a, c_ef);
     sm = signed_of(p_sm[i]);
     long long e = signed_of(p_ef[i]);
     ef = e < 0 ? 0 : (from_slot && e > 0xfe) ? 0xfe : e;
 }
 
-// A CTA owns 32 consecutive committed rows: lane = row, so that every column access of a warp is one 128-byte line.
-// Its RS_LANES warps share the row's work: the leaves, then the slots level by level (a level holds the slots whose
-// operands are leaves or outputs of earlier levels; `order` lists the slots by level, `level_start` where each begins),
-// with a CTA barrier between levels, since a slot's operand may be a cell another warp of the CTA wrote.
-constexpr uint32_t RS_LANES = 8;
-template <bool MUL, bool STICKY>
-__global__ void __launch_bounds__(32 * RS_LANES) residual_stream_kernel(RsArgs a) {
+// A team of warps owns 32 consecutive committed rows at a time: lane = row, so that every column access of a warp is one 128-byte
+// line. The warps share the rows' work: the leaves, then the slots level by level (a level holds the slots whose operands are
+// leaves or outputs of earlier levels), with a barrier of the team between levels, since a slot's operand may be a cell
+// another warp of the team wrote.
+//
+// What bounded it were the counts (count_cache.cuh), then the latency of a slot, a chain of loads (its record, the operands' cells, a
+// row of the table) before its stores. So one CTA an SM keeps the counters and takes rows until none are left, in two teams of sixteen
+// warps; column addresses are computed where they can be (fourteen of them were 28 registers), four leaves are loaded at a time.
+// 2^15 rows of 128 additions: see RS_TIMES at the launch.
+constexpr uint32_t RS_LANES = 16, RS_TEAMS = 2, RS_LEAVES = 4;
+constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 12, RS_SMUL_LOG = 14;
+constexpr uint32_t RS_ADD_WORDS = (1u << RS_VAL_LOG) + (1u << RS_NORM_LOG) + (1u << RS_FRAC_LOG), RS_MUL_WORDS = (1u << RS_VAL_LOG) + (1u << RS_SMUL_LOG);
+template <bool MUL, bool STICKY, bool EVEN>
+__global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_kernel(const __grid_constant__ RsArgs a) {
     // The power table has 273 rows and every addition hits row DMAX with its larger operand: counted per CTA in shared
     // memory and added to the global array once at the end (one hot address would serialise every warp of the grid).
     __shared__ uint32_t pow_hist[RS_POW_ROWS];
-    if (!MUL) {
-        for (uint32_t k = threadIdx.x; k < RS_POW_ROWS; k += blockDim.x) pow_hist[k] = 0;
-        __syncthreads();
-    }
-    const uint32_t i = blockIdx.x * 32u + (threadIdx.x & 31u), t = threadIdx.x >> 5;
+    extern __shared__ uint32_t counts_sm[];
+    uint32_t *const val_counts = counts_sm, *const norm_counts = counts_sm + (1u << RS_VAL_LOG), *const frac_counts = norm_counts + (1u << RS_NORM_LOG);
+    uint32_t* const smul_counts = norm_counts;  // a program adds or multiplies
+    for (uint32_t k = threadIdx.x; k < (MUL ? RS_MUL_WORDS : RS_ADD_WORDS); k += blockDim.x) counts_sm[k] = 0;
+    for (uint32_t k = threadIdx.x; k < RS_POW_ROWS; k += blockDim.x) pow_hist[k] = 0;
+    __syncthreads();
+    auto flush = [&](uint32_t thread, uint32_t threads) {
+        count_flush<RS_VAL_LOG>(val_counts, a.m_val.m, thread, threads);
+        if (MUL) count_flush<RS_SMUL_LOG>(smul_counts, a.m_smul.m, thread, threads);
+        else {
+            count_flush<RS_NORM_LOG>(norm_counts, a.m_norm.m, thread, threads);
+            count_flush<RS_FRAC_LOG>(frac_counts, a.m_frac.m, thread, threads);
+        }
+    };
+    const uint32_t lanes = blockDim.x / (32u * a.teams), team = (threadIdx.x >> 5) / lanes, t = (threadIdx.x >> 5) - team * lanes;
+    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1u), "r"(32u * lanes) : "memory"); };
+    uint32_t off = 0, bad_exp = 0, un_off = 0, since_flush = 0;
+    for (uint32_t block = blockIdx.x * a.teams + team; (block << 5 >> a.log_rows) == 0; block += gridDim.x * a.teams) {
+    const uint32_t i = block * 32u + (threadIdx.x & 31u);
     const bool in_range = (i >> a.log_rows) == 0;
     const uint32_t j = in_range ? committed_to_natural(i, a.log_rows) : 0u;
     const bool live = j < a.live;
-    uint32_t off = 0, bad_exp = 0, un_off = 0;
-    uint32_t* const* cols = a.cols;
     const size_t leaf0 = (size_t)j * a.n_leaves;
 
     if (in_range)
     for (uint32_t g = 0; g < a.n_groups; g++) {
         const RsGroup gr = a.groups[g];
-        for (uint32_t k = t; k < gr.n; k += RS_LANES) {
-            const uint32_t pat = live ? __ldg(a.wit + leaf0 + gr.flat + k) : 0u;
-            // a bf16 pattern as (sm, ef); both zeros, infinities and NaNs collapse to (0, 0)
-            const uint32_t e = (pat >> 7) & 0xffu;
-            const bool finite = e != 0 && e != 0xffu;
-            const long long mag = 128 + (pat & 0x7fu);
-            const long long sm = finite ? ((pat >> 15) & 1u ? -mag : mag) : 0;
-            const uint32_t ef = finite ? e : 0u;
-            const uint32_t b = gr.leaf_col + k * gr.width;
-            uint32_t *c0 = column(cols, b), *c1 = column(cols, b + 1), *c2 = nullptr, *c3 = nullptr;
-            if (gr.un) { c2 = column(cols, b + 2); c3 = column(cols, b + 3); }
-            c0[i] = field_of(sm);
-            c1[i] = ef;
-            reinterpret_cast<int2*>(a.in_nat)[leaf0 + gr.flat + k] = make_int2((int)sm, (int)ef);  // natural row order
-            const uint32_t v = value_index(sm, ef);
-            if (gr.un == 0) { lookup(a.m_val, v, off); continue; }
-            lookup(a.m_un[gr.un - 1], v, off);
-            int2 img = make_int2(0, 0);  // the unary image, tabulated over the value table's rows
-            if (v < a.n_val) img = __ldg(reinterpret_cast<const int2*>(a.un2[gr.un - 1]) + v);
-            else un_off++;
-            c2[i] = field_of(img.x);
-            c3[i] = field_of(img.y);
+        for (uint32_t k0 = t * RS_LEAVES; k0 < gr.n; k0 += lanes * RS_LEAVES) {
+            uint32_t pats[RS_LEAVES];
+#pragma unroll
+            for (uint32_t u = 0; u < RS_LEAVES; u++) pats[u] = live && k0 + u < gr.n ? __ldg(a.wit + leaf0 + gr.flat + k0 + u) : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < RS_LEAVES; u++) {
+                const uint32_t k = k0 + u, pat = pats[u];
+                if (k >= gr.n) break;
+                // a bf16 pattern as (sm, ef); both zeros, infinities and NaNs collapse to (0, 0)
+                const uint32_t e = (pat >> 7) & 0xffu;
+                const bool finite = e != 0 && e != 0xffu;
+                const long long mag = 128 + (pat & 0x7fu);
+                const long long sm = finite ? ((pat >> 15) & 1u ? -mag : mag) : 0;
+                const uint32_t ef = finite ? e : 0u;
+                const uint32_t b = gr.leaf_col + k * gr.width;
+                column<EVEN>(a, b)[i] = field_of(sm);
+                column<EVEN>(a, b + 1)[i] = ef;
+                reinterpret_cast<int2*>(a.in_nat)[leaf0 + gr.flat + k] = make_int2((int)sm, (int)ef);  // natural row order
+                const uint32_t v = value_index(sm, ef);
+                if (gr.un == 0) { lookup<RS_VAL_LOG>(val_counts, a.m_val, v, off); continue; }
+                uint32_t *c2 = column<EVEN>(a, b + 2), *c3 = column<EVEN>(a, b + 3);
+                lookup(a.m_un[gr.un - 1], v, off);
+                int2 img = make_int2(0, 0);  // the unary image, tabulated over the value table's rows
+                if (v < a.n_val) img = __ldg(reinterpret_cast<const int2*>(a.un2[gr.un - 1]) + v);
+                else un_off++;
+                c2[i] = field_of(img.x);
+                c3[i] = field_of(img.y);
+            }
         }
     }
 
     for (uint32_t level = 0; level < a.n_levels; level++) {
-      __syncthreads();
+      team_sync();
       if (in_range)
-      for (uint32_t at = a.level_start[level] + t; at < a.level_start[level + 1]; at += RS_LANES) {
-        const RsSlot sl = a.slots[a.order[at]];
+      for (uint32_t at = a.level_start[level] + t; at < a.level_start[level + 1]; at += lanes) {
+        const RsSlot sl = a.slots[at];
         long long a_sm, a_ef, b_sm, b_ef, c_sm, c_ef;
-        operand(cols, i, sl.a_sm, sl.a_ef, sl.from_slot & 1u, a_sm, a_ef);
-        operand(cols, i, sl.b_sm, sl.b_ef, sl.from_slot & 2u, b_sm, b_ef);
+        operand<EVEN>(a, i, sl.a_sm, sl.a_ef, sl.from_slot & 1u, a_sm, a_ef);
+        operand<EVEN>(a, i, sl.b_sm, sl.b_ef, sl.from_slot & 2u, b_sm, b_ef);
         const uint32_t b = sl.base;
         constexpr uint32_t W = MUL ? 4u : (STICKY ? 14u : 13u);
-        uint32_t* cell[W];
+        uint32_t* held[W];
 #pragma unroll
-        for (uint32_t k = 0; k < W; k++) cell[k] = column(cols, b + k);
+        for (uint32_t k = 0; k < W; k++) held[k] = EVEN ? nullptr : column<EVEN>(a, b + k);
+        uint32_t* const first = EVEN ? column<EVEN>(a, b) + i : nullptr;
+        auto put = [&](uint32_t k, uint32_t v) { (EVEN ? first + (long long)k * a.col_step : held[k] + i)[0] = v; };
         if (!MUL) {
             // align both operands to the larger exponent (a shift of up to DMAX bits is kept, a smaller operand is dropped),
             // add, normalise the magnitude to a 9-bit M2 with its round-bit weight ph, round through the table
@@ -334,26 +368,26 @@ __global__ void __launch_bounds__(32 * RS_LANES) residual_stream_kernel(RsArgs a
             uint32_t m7n = 0, efn = 0, nzn = 0;
             if (ni < a.n_norm) { m7n = __ldg(a.norm3 + 3 * (size_t)ni); efn = __ldg(a.norm3 + 3 * (size_t)ni + 1); nzn = __ldg(a.norm3 + 3 * (size_t)ni + 2); }
             else off++;
-            lookup(a.m_norm, ni, off);
-            lookup(a.m_frac, ph == 0 ? (r == 0 ? 0u : OFF_TABLE) : ph + (uint32_t)r, off);
+            lookup<RS_NORM_LOG>(norm_counts, a.m_norm, ni, off);
+            lookup<RS_FRAC_LOG>(frac_counts, a.m_frac, ph == 0 ? (r == 0 ? 0u : OFF_TABLE) : ph + (uint32_t)r, off);
             c_sm = (long long)(128u * nzn + m7n) * (sg ? -1 : 1);
             c_ef = nzn == 1 ? (long long)efn + etop - RS_DMAX - RS_BIAS : 0;
             bad_exp += nzn == 1 && !(c_ef >= 1 && c_ef < 0xff);
-            cell[0][i] = field_of(fa);
-            cell[1][i] = field_of(fb);
-            cell[2][i] = field_of(etop);
-            cell[3][i] = field_of((long long)mag);
-            cell[4][i] = sg;
-            cell[5][i] = m2;
-            cell[6][i] = ph;
-            cell[7][i] = field_of((long long)r);
-            if (STICKY) cell[8][i] = st;
+            put(0, field_of(fa));
+            put(1, field_of(fb));
+            put(2, field_of(etop));
+            put(3, field_of((long long)mag));
+            put(4, sg);
+            put(5, m2);
+            put(6, ph);
+            put(7, field_of((long long)r));
+            if (STICKY) put(8, st);
             constexpr uint32_t kk = STICKY ? 9u : 8u;
-            cell[kk][i] = m7n;
-            cell[kk + 1][i] = efn;
-            cell[kk + 2][i] = nzn;
-            cell[kk + 3][i] = field_of(c_sm);
-            cell[kk + 4][i] = field_of(c_ef);
+            put(kk, m7n);
+            put(kk + 1, efn);
+            put(kk + 2, nzn);
+            put(kk + 3, field_of(c_sm));
+            put(kk + 4, field_of(c_ef));
         } else {
             // the signed significands' correctly rounded product and binade carry come from one table row
             const uint32_t ia = signed_significand_index(a_sm), ib = signed_significand_index(b_sm);
@@ -361,36 +395,42 @@ __global__ void __launch_bounds__(32 * RS_LANES) residual_stream_kernel(RsArgs a
             int32_t prod = 0, cy = 0, nzc = 0;
             if (si < a.n_smul) { prod = __ldg(a.smul3 + 3 * (size_t)si); cy = __ldg(a.smul3 + 3 * (size_t)si + 1); nzc = __ldg(a.smul3 + 3 * (size_t)si + 2); }
             else off++;
-            lookup(a.m_smul, si, off);
+            lookup<RS_SMUL_LOG>(smul_counts, a.m_smul, si, off);
             c_sm = prod;
             c_ef = nzc == 1 ? a_ef + b_ef + cy - 127 : 0;
             bad_exp += nzc == 1 && !(c_ef >= 1 && c_ef < 0xff);
-            cell[0][i] = field_of(c_sm);
-            cell[1][i] = (uint32_t)cy;
-            cell[2][i] = (uint32_t)nzc;
-            cell[3][i] = field_of(c_ef);
+            put(0, field_of(c_sm));
+            put(1, (uint32_t)cy);
+            put(2, (uint32_t)nzc);
+            put(3, field_of(c_ef));
         }
-        lookup(a.m_val, (c_ef >= 0 && c_ef < 0xff) ? value_index(c_sm, c_ef) : OFF_TABLE, off);  // the slot's own output is a looked-up pair too
+        lookup<RS_VAL_LOG>(val_counts, a.m_val, (c_ef >= 0 && c_ef < 0xff) ? value_index(c_sm, c_ef) : OFF_TABLE, off);  // the slot's own output is a looked-up pair too
       }
     }
-    __syncthreads();
+    team_sync();
 
     // what the bindings and the next component read, in natural row order
     if (in_range)
-    for (uint32_t k = t; k < a.out_w; k += RS_LANES) {
+    for (uint32_t k = t; k < a.out_w; k += lanes) {
         const RsSlot sl = a.slots[a.out_slot[k]];
-        const long long sm = signed_of(column(cols, sl.o_sm)[i]), e = signed_of(column(cols, sl.o_ef)[i]);
+        const long long sm = signed_of(column<EVEN>(a, sl.o_sm)[i]), e = signed_of(column<EVEN>(a, sl.o_ef)[i]);
         const uint32_t ef = (uint32_t)(e < 0 ? 0 : e > 0xfe ? 0xfe : e);
         uint32_t pat = 0;
         if (sm != 0) pat = ((sm < 0 ? 1u << 15 : 0u) | (ef << 7) | (uint32_t)((sm < 0 ? -sm : sm) - 128)) & 0xffffu;
         a.out_pat[(size_t)j * a.out_w + k] = pat;
         reinterpret_cast<int2*>(a.out_nat)[(size_t)j * a.out_w + k] = make_int2((int)sm, (int)e);
     }
-    if (!MUL) {
-        __syncthreads();
+    team_sync();  // the next rows' cells are other memory, but a warp must not be two passes ahead of its team's barrier
+    if (++since_flush == a.flush_every) {
+        flush(threadIdx.x - team * 32u * lanes, 32u * lanes);
+        since_flush = 0;
+    }
+    }
+    __syncthreads();
+    flush(threadIdx.x, blockDim.x);
+    if (!MUL)
         for (uint32_t k = threadIdx.x; k < RS_POW_ROWS && k < a.m_pow.n; k += blockDim.x)
             if (pow_hist[k]) atomicAdd(a.m_pow.m + k, pow_hist[k]);
-    }
     off = __reduce_add_sync(0xffffffffu, off);
     bad_exp = __reduce_add_sync(0xffffffffu, bad_exp);
     un_off = __reduce_add_sync(0xffffffffu, un_off);
@@ -557,13 +597,17 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
         }
         n_levels = std::max(n_levels, level[s] + 1u);
     }
-    std::vector<uint32_t> order, level_start(n_levels + 1, 0);
-    for (uint32_t l = 0; l < n_levels; l++) {
-        level_start[l] = (uint32_t)order.size();
-        for (uint32_t s = 0; s < p.n_slots; s++)
-            if (level[s] == l) order.push_back(s);
+    // the slots level by level, in their own order within a level (a counting sort)
+    std::vector<uint32_t> level_start(n_levels + 1, 0), place(p.n_slots), out_slot(p.out_w);
+    for (uint32_t s = 0; s < p.n_slots; s++) level_start[level[s] + 1]++;
+    for (uint32_t l = 0; l < n_levels; l++) level_start[l + 1] += level_start[l];
+    std::vector<uint32_t> next(level_start.begin(), level_start.end());
+    std::vector<zkb_rs_slot> slots(p.n_slots);
+    for (uint32_t s = 0; s < p.n_slots; s++) {
+        place[s] = next[level[s]]++;
+        slots[place[s]] = p.slots[s];
     }
-    level_start[n_levels] = (uint32_t)order.size();
+    for (uint32_t k = 0; k < p.out_w; k++) out_slot[k] = place[p.out_slot[k]];
     for (uint32_t u = 0; u < tables->n_un; u++) ZKB_CHECK_ARG(ctx, tables->un2[u] && ((uintptr_t)tables->un2[u] & 7) == 0 && mults->un[u].m);
     for (uint32_t k = 0; k < n_cols; k++) ZKB_CHECK_ARG(ctx, cols[k] != nullptr);
     DeviceGuard g(ctx);
@@ -573,9 +617,8 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     if (rc) return rc;
     static_assert(sizeof(zkb_rs_group) == sizeof(RsGroup) && sizeof(zkb_rs_slot) == sizeof(RsSlot) && sizeof(zkb_rs_mult) == sizeof(RsMult), "layout");
     if ((rc = stage_array(ctx, reinterpret_cast<const RsGroup*>(p.groups), p.n_groups, &a.groups))) return rc;
-    if ((rc = stage_array(ctx, reinterpret_cast<const RsSlot*>(p.slots), p.n_slots, &a.slots))) return rc;
-    if ((rc = stage_array(ctx, p.out_slot, p.out_w, &a.out_slot))) return rc;
-    if ((rc = stage_array(ctx, order.data(), order.size(), &a.order))) return rc;
+    if ((rc = stage_array(ctx, reinterpret_cast<const RsSlot*>(slots.data()), p.n_slots, &a.slots))) return rc;
+    if ((rc = stage_array(ctx, out_slot.data(), p.out_w, &a.out_slot))) return rc;
     if ((rc = stage_array(ctx, level_start.data(), level_start.size(), &a.level_start))) return rc;
     if ((rc = stage_array(ctx, tables->un2, tables->n_un, &a.un2))) return rc;
     if ((rc = stage_array(ctx, reinterpret_cast<const RsMult*>(mults->un), tables->n_un, &a.m_un))) return rc;
@@ -586,11 +629,29 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     a.n_norm = tables->norm3 ? tables->n_norm : 0; a.n_smul = tables->smul3 ? tables->n_smul : 0; a.n_val = tables->n_val;
     a.log_rows = log_rows; a.live = live_rows; a.n_groups = p.n_groups; a.n_leaves = (uint32_t)n_leaves; a.n_slots = p.n_slots;
     a.kmax = p.kmax; a.out_w = p.out_w; a.n_levels = n_levels;
-    const uint32_t rows = 1u << log_rows, grid = (rows + 31) / 32, threads = 32 * RS_LANES;
+    // evenly spaced columns need no table
+    bool even = true;
+    a.col0 = cols[0];
+    a.col_step = n_cols > 1 ? (long long)(reinterpret_cast<intptr_t>(cols[1]) - reinterpret_cast<intptr_t>(cols[0])) / 4 : 0;
+    for (uint32_t k = 0; k < n_cols && even; k++) even = cols[k] == cols[0] + (long long)k * a.col_step;
+    // 32 rows a team of warps; two teams a CTA and a CTA an SM where there are so many rows, sixteen warps a team (eight where a row
+    // has too little for them).
+    const uint32_t rows = 1u << log_rows, blocks = (rows + 31) / 32;
+    a.teams = blocks > 148 ? RS_TEAMS : 1u;
+    const uint32_t grid = std::min((blocks + a.teams - 1) / a.teams, 148u);
+    const uint32_t lanes = n_leaves + p.n_slots < 64 ? RS_LANES / 2 : RS_LANES, threads = 32 * lanes * a.teams;
+    // A counter holds 2^27 - 1: the teams send them to memory long before one could be full.
+    a.flush_every = (uint32_t)std::max<uint64_t>(1, ((uint64_t)1 << 24) / (32 * (n_leaves + p.n_slots)));
     ProfScope prof(ctx, "residual_stream_kernel");
-    if (p.kind == 1) residual_stream_kernel<true, false><<<grid, threads, 0, ctx->stream>>>(a);
-    else if (p.sticky) residual_stream_kernel<false, true><<<grid, threads, 0, ctx->stream>>>(a);
-    else residual_stream_kernel<false, false><<<grid, threads, 0, ctx->stream>>>(a);
+    cudaError_t e = cudaSuccess;
+    auto launch = [&](auto kernel, uint32_t words) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * words));
+        if (e == cudaSuccess) kernel<<<grid, threads, 4 * words, ctx->stream>>>(a);
+    };
+    if (p.kind == 1) even ? launch(residual_stream_kernel<true, false, true>, RS_MUL_WORDS) : launch(residual_stream_kernel<true, false, false>, RS_MUL_WORDS);
+    else if (p.sticky) even ? launch(residual_stream_kernel<false, true, true>, RS_ADD_WORDS) : launch(residual_stream_kernel<false, true, false>, RS_ADD_WORDS);
+    else even ? launch(residual_stream_kernel<false, false, true>, RS_ADD_WORDS) : launch(residual_stream_kernel<false, false, false>, RS_ADD_WORDS);
+    ZKB_CUDA(ctx, e);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
 }
