@@ -9,9 +9,11 @@
 // component is witness_gen_mat_row, prover/src/gadgets/dequant/trace.rs:503-690 (pow2 and chain arms).
 // The reference kernels' "mutate" arguments are deliberate defects for its negative controls; they are not
 // part of the operator and are not built here.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
+#include "count_cache.cuh"
 
 namespace zk {
 
@@ -129,12 +131,15 @@ __global__ void tables_patch_kernel(const uint32_t* __restrict__ idx, const uint
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Dequantize component. One thread owns one committed row and a tile of its slots; a warp therefore
+// Dequantize component. A thread takes one committed row and a tile of its slots at a time; a warp therefore
 // writes 128 consecutive bytes of every column it touches; the accumulators of a row's slots are
-// consecutive in memory, so a thread walks one or two sectors of them. Multiplicities:
-// the 8-bit range table is a shared-memory histogram flushed once per CTA; the three large tables take
-// warp-aggregated atomics (lanes hitting the same row add once).
+// consecutive in memory, so a thread walks one or two sectors of them. Multiplicities: the 8-bit range table is a
+// shared-memory histogram, the three large tables go through counters in shared memory too (count_cache.cuh), so one CTA an
+// SM takes units until none are left. 2^17 rows of 16 slots: 230 us with the large tables' counts as warp-merged atomics.
 // ---------------------------------------------------------------------------------------------------
+constexpr int DEQ_THREADS = 1024, DEQ_NORM_LOG = 13, DEQ_FRAC_LOG = 12, DEQ_MUL_LOG = 14;
+constexpr uint32_t DEQ_COUNT_WORDS = (1u << DEQ_NORM_LOG) + (1u << DEQ_FRAC_LOG), DEQ_CHAIN_WORDS = DEQ_COUNT_WORDS + (1u << DEQ_MUL_LOG);
+constexpr uint32_t DEQ_POINTERS = 6144;  // column addresses kept in shared memory (48 KB); a wider component reads them from the table
 struct DeqArgs {
     const int32_t *acc, *jx, *jw;
     const uint32_t *sx, *sw, *norm3, *mul2;
@@ -142,13 +147,8 @@ struct DeqArgs {
     uint32_t* const* pre;
     uint32_t *m_norm, *m_frac, *m_mul, *m_r8, *counts, *want;
     zkb_dequant_cfg c;
-    uint32_t slot_tile;
+    uint32_t slot_tile, tiles, flush_every;
 };
-
-__device__ __forceinline__ void bump_agg(uint32_t* m, uint32_t idx) {
-    uint32_t peers = __match_any_sync(__activemask(), idx);
-    if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(m + idx, (uint32_t)__popc(peers));
-}
 
 __device__ __forceinline__ uint32_t bf16_bits(uint32_t sg, uint32_t ef, uint32_t m7) { return ((sg << 15) | (ef << 7) | m7) & 0xffffu; }
 __device__ __forceinline__ double bf16_value(uint32_t bits) { return (double)__uint_as_float(bits << 16); }
@@ -167,32 +167,43 @@ __device__ __forceinline__ uint32_t bf16_round_f64(double x) {
 }
 
 template <int CHAIN>
-__global__ void __launch_bounds__(128) dequant_kernel(const DeqArgs a) {
-    extern __shared__ __align__(16) uint32_t r8_hist[];
+__global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_constant__ DeqArgs a) {
+    extern __shared__ __align__(16) uint32_t deq_sm[];
     const zkb_dequant_cfg& c = a.c;
-    for (uint32_t k = threadIdx.x; k < c.n_r8; k += blockDim.x) r8_hist[k] = 0;
-    // The column addresses of this CTA's slots, once per CTA: every store of every thread would otherwise start with a
-    // dependent read of the pointer table.
-    uint32_t** s_base = reinterpret_cast<uint32_t**>(r8_hist + ((c.n_r8 + 3u) & ~3u));  // [slot in tile][field]
-    uint32_t** s_pre = s_base + a.slot_tile * c.per_slot;                               // [slot in tile][scale column]
-    {
-        const uint32_t s0 = blockIdx.y * a.slot_tile, ns = min(c.per_row - s0, a.slot_tile);
-        for (uint32_t k = threadIdx.x; k < ns * c.per_slot; k += blockDim.x) s_base[k] = a.base[c.slot0 + s0 * c.per_slot + k];
-        for (uint32_t k = threadIdx.x; k < ns * c.chan_w; k += blockDim.x) s_pre[k] = a.pre[c.chan_w * s0 + k];
+    uint32_t *const norm_counts = deq_sm, *const frac_counts = deq_sm + (1u << DEQ_NORM_LOG), *const mul_counts = deq_sm + DEQ_COUNT_WORDS;
+    uint32_t* const r8_hist = deq_sm + (CHAIN ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS);
+    for (uint32_t k = threadIdx.x; k < (CHAIN ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS) + c.n_r8; k += blockDim.x) deq_sm[k] = 0;
+    // The column addresses, once per CTA: every store of every thread would otherwise start with a dependent read of the pointer table.
+    const uint32_t n_base = c.per_row * c.per_slot, n_pre = c.per_row * c.chan_w;
+    uint32_t* const* p_base = a.base + c.slot0;
+    uint32_t* const* p_pre = a.pre;
+    if (n_base + n_pre <= DEQ_POINTERS) {
+        uint32_t** const p = reinterpret_cast<uint32_t**>(r8_hist + ((c.n_r8 + 3u) & ~3u));  // [slot][field], then [slot][scale column]
+        for (uint32_t k = threadIdx.x; k < n_base + n_pre; k += blockDim.x) p[k] = k < n_base ? p_base[k] : p_pre[k - n_base];
+        p_base = p;
+        p_pre = p + n_base;
     }
     __syncthreads();
+    auto flush = [&] {
+        count_flush<DEQ_NORM_LOG>(norm_counts, a.m_norm, threadIdx.x, DEQ_THREADS);
+        count_flush<DEQ_FRAC_LOG>(frac_counts, a.m_frac, threadIdx.x, DEQ_THREADS);
+        if (CHAIN) count_flush<DEQ_MUL_LOG>(mul_counts, a.m_mul, threadIdx.x, DEQ_THREADS);
+    };
     const uint32_t rows = 1u << c.log_rows;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t off_table = 0, ref_bad = 0, no_row = 0;
-    if (i < rows) {
+    const uint64_t units = (uint64_t)rows * a.tiles;  // row by row within a tile of slots
+    uint32_t off_table = 0, ref_bad = 0, no_row = 0, since_flush = 0;
+    for (uint64_t unit0 = (uint64_t)blockIdx.x * DEQ_THREADS; unit0 < units; unit0 += (uint64_t)gridDim.x * DEQ_THREADS) {
+      const uint64_t unit = unit0 + threadIdx.x;
+      if (unit < units) {
+        const uint32_t i = (uint32_t)unit & (rows - 1u), tile = (uint32_t)(unit >> c.log_rows);
         const uint32_t j = coset_perm(i, c.log_rows);
         const uint32_t t = c.tokens - 1u - j / c.chunks, jm = j % c.chunks, b = c.chunks - 1u - jm;
-        const uint32_t s_begin = blockIdx.y * a.slot_tile, s_end = min(c.per_row, s_begin + a.slot_tile);
+        const uint32_t s_begin = tile * a.slot_tile, s_end = min(c.per_row, s_begin + a.slot_tile);
         uint32_t sx_m = 0, sx_e = 0;
         int jx_t = 0;
         if (CHAIN) { sx_m = __ldg(a.sx + 2u * t); sx_e = __ldg(a.sx + 2u * t + 1u); }
         else jx_t = __ldg(a.jx + t);
-        if (blockIdx.y == 0) {
+        if (tile == 0) {
             // the row's shared columns (the activation's scale) and the five selectors that close the preprocessed columns
             if (CHAIN) { a.base[c.sh0][i] = sx_m; a.base[c.sh1][i] = sx_e; }
             else a.base[c.sh0][i] = m31_of(jx_t);
@@ -206,8 +217,8 @@ __global__ void __launch_bounds__(128) dequant_kernel(const DeqArgs a) {
         const int32_t* acc_row = a.acc + (size_t)t * c.n_out + (size_t)b * c.per_row;
         for (uint32_t s = s_begin; s < s_end; s++) {
             const uint32_t ch = b * c.per_row + s;
-            uint32_t* const* col = s_base + (s - s_begin) * c.per_slot;  // col[field] is the slot's column of that field
-            uint32_t* const* pcol = s_pre + (s - s_begin) * c.chan_w;
+            uint32_t* const* col = p_base + s * c.per_slot;  // col[field] is the slot's column of that field
+            uint32_t* const* pcol = p_pre + s * c.chan_w;
             uint32_t sw_m = 0, sw_e = 0;
             int jw_c = 0;
             if (CHAIN) {
@@ -244,8 +255,8 @@ __global__ void __launch_bounds__(128) dequant_kernel(const DeqArgs a) {
             }
             if (ri >= c.n_norm || fi >= c.n_frac) { no_row++; continue; }
             const uint32_t n_m7 = __ldg(a.norm3 + 3u * ri), n_ef = __ldg(a.norm3 + 3u * ri + 1u), n_nz = __ldg(a.norm3 + 3u * ri + 2u);
-            bump_agg(a.m_norm, ri);
-            bump_agg(a.m_frac, fi);
+            count_cached<DEQ_NORM_LOG>(norm_counts, a.m_norm, ri);
+            count_cached<DEQ_FRAC_LOG>(frac_counts, a.m_frac, fi);
             col[c.f_sg][i] = sg;
             col[c.f_m2][i] = m2;
             col[c.f_ph][i] = ph;
@@ -281,7 +292,7 @@ __global__ void __launch_bounds__(128) dequant_kernel(const DeqArgs a) {
                     col[c.f_mul[3u * step + 0u]][i] = po;
                     col[c.f_mul[3u * step + 1u]][i] = ca;
                     col[c.f_mul[3u * step + 2u]][i] = m31_of(eo);
-                    if (n_nz == 1u) bump_agg(a.m_mul, mi);
+                    if (n_nz == 1u) count_cached<DEQ_MUL_LOG>(mul_counts, a.m_mul, mi);
                     if (eo >= 0 && eo < (long long)c.n_r8) atomicAdd(&r8_hist[eo], 1u); else off_table++;
                     m_in = po;
                     e_in = eo;
@@ -297,11 +308,17 @@ __global__ void __launch_bounds__(128) dequant_kernel(const DeqArgs a) {
                 }
             }
         }
+      }
+      if (++since_flush == a.flush_every) {
+          flush();
+          since_flush = 0;
+      }
     }
     if (off_table) atomicAdd(a.counts + 0, off_table);
     if (ref_bad) atomicAdd(a.counts + 1, ref_bad);
     if (no_row) atomicAdd(a.counts + 2, no_row);
     __syncthreads();
+    flush();
     for (uint32_t k = threadIdx.x; k < c.n_r8; k += blockDim.x)
         if (r8_hist[k]) atomicAdd(a.m_r8 + k, r8_hist[k]);
 }
@@ -369,18 +386,25 @@ int zkb_witness_dequant(zkb_ctx* ctx, const int32_t* acc, const int32_t* jx, con
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)pre_cols, (int)n_pre, &d_pre);
     if (rc) return rc;
-    const uint32_t rows = 1u << c.log_rows, gx = (rows + 127) / 128;
-    // Slots per thread. A slot is a chain of dependent table reads, so the kernel lives on the number of warps in flight:
-    // as few slots per thread as it takes to reach 32 CTAs (128 warps) per SM, and never more than four.
+    // Slots a unit: up to four, as long as every CTA has eight rounds of units (so that the last one counts little).
+    const uint32_t rows = 1u << c.log_rows;
     uint32_t slot_tile = c.per_row < 4 ? c.per_row : 4;
-    while (slot_tile > 1 && (uint64_t)gx * ((c.per_row + slot_tile - 1) / slot_tile) < 148u * 32u) slot_tile = (slot_tile + 1) / 2;
+    while (slot_tile > 1 && (uint64_t)rows * ((c.per_row + slot_tile - 1) / slot_tile) < 8ull * 148u * DEQ_THREADS) slot_tile = (slot_tile + 1) / 2;
+    const uint32_t tiles = (c.per_row + slot_tile - 1) / slot_tile;
+    // a counter holds 2^27 - 1, and a unit counts at most twice per slot
     DeqArgs a{acc, jx, jw, sx, sw, norm3, mul2, (uint32_t* const*)d_base, (uint32_t* const*)d_pre, m_norm, m_frac, m_mul, m_r8, counts,
-              want_out, c, slot_tile};
-    dim3 grid(gx, (c.per_row + slot_tile - 1) / slot_tile);
+              want_out, c, slot_tile, tiles, (1u << 26) / (DEQ_THREADS * 2u * slot_tile)};
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)rows * tiles + DEQ_THREADS - 1) / DEQ_THREADS, 148u);
+    const uint64_t pointers = (uint64_t)c.per_row * (c.per_slot + c.chan_w);
+    const size_t smem = (size_t)((c.variant == 1 ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS) + ((c.n_r8 + 3u) & ~3u)) * 4 + (pointers <= DEQ_POINTERS ? 8 * pointers : 0);
     ProfScope prof(ctx, "witness_dequant_kernel");
-    const size_t smem = (size_t)((c.n_r8 + 3u) & ~3u) * 4 + (size_t)slot_tile * (c.per_slot + c.chan_w) * sizeof(uint32_t*);
-    if (c.variant == 1) dequant_kernel<1><<<grid, 128, smem, ctx->stream>>>(a);
-    else dequant_kernel<0><<<grid, 128, smem, ctx->stream>>>(a);
+    auto launch = [&](auto kernel) {
+        // the most any call takes: another thread's call must not lower it in between
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * (DEQ_CHAIN_WORDS + 8192) + 8 * DEQ_POINTERS));
+        if (e == cudaSuccess) kernel<<<grid, DEQ_THREADS, smem, ctx->stream>>>(a);
+        return e;
+    };
+    ZKB_CUDA(ctx, c.variant == 1 ? launch(dequant_kernel<1>) : launch(dequant_kernel<0>));
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
 }
