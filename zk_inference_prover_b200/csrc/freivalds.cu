@@ -13,6 +13,7 @@
 // The Horner restarts at every group, so each group is scanned independently and acc_m is a prefix
 // sum over the groups' totals. Kernels: per-row inner products (coalesced column reads, results in
 // coset order), per-group scan, prefix over groups, split into coordinate columns.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -28,8 +29,25 @@ __device__ __forceinline__ uint32_t coset_perm(uint32_t i, uint32_t log_n) {
 }
 __device__ __forceinline__ uint32_t m31_of_i32(int v) { return v < 0 ? (uint32_t)(v + (int)P) : (uint32_t)v; }
 
+// Which rows a thread of the passes over all rows takes: i and rows - 1 - i. Their places in coset order are neighbours (an even row's
+// place is twice the reversal of i / 2, the mirrored odd one's the one after it), so what is read or written there, 16 bytes a
+// row, is a whole 32-byte sector at once; with one row a thread the halves of a sector came far apart in time and the memory
+// behind L2 saw them twice. The warps of a CTA take rows an eighth of the half apart, whose places are neighbours again.
+// block: of rows / 512 (at least one); false: no such row.
+__device__ __forceinline__ bool row_pair(uint32_t block, uint32_t rows, uint32_t& i) {
+    const uint32_t half = rows >> 1;
+    i = half >= 256u ? (threadIdx.x >> 5) * (half >> 3) + block * 32u + (threadIdx.x & 31u) : threadIdx.x;
+    return i < half;
+}
+static unsigned row_pair_blocks(size_t rows) { return rows >= 512 ? (unsigned)(rows / 512) : 1u; }
+
 // ---- F1: columns ------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) freivalds_scatter_kernel(const int8_t* __restrict__ qx, const int8_t* const* __restrict__ qw,
+// Consecutive threads' rows lie far apart in coset order (the permutation is a bit reversal), so every weight load touches 32 sectors a
+// warp: with one load a byte those, not the columns' stores, were the pass (16 of them a row and matrix). A row's weights of one
+// matrix are consecutive: they are loaded 16 at a time where their addresses allow it, else four. A CTA takes several pieces of rows, so
+// that its range histogram reaches memory once. 2^20 rows, 2 x 16 weights and an activation: 100 us before.
+constexpr int SCATTER_THREADS = 256;
+__global__ void __launch_bounds__(SCATTER_THREADS, 5) freivalds_scatter_kernel(const int8_t* __restrict__ qx, const int8_t* const* __restrict__ qw,
                                                                 const uint32_t* __restrict__ n_out, FGrid g, uint32_t pq, uint32_t pk,
                                                                 uint32_t n_in, uint32_t tokens, uint32_t n_mats,
                                                                 uint32_t* const* __restrict__ base_cols,
@@ -39,8 +57,11 @@ __global__ void __launch_bounds__(256) freivalds_scatter_kernel(const int8_t* __
     for (uint32_t t = threadIdx.x; t < table_len; t += blockDim.x) hist[t] = 0;
     __syncthreads();
     const uint32_t rows = 1u << g.log_rows;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < rows) {
+    for (uint32_t block = blockIdx.x; block < (rows >= 512u ? rows >> 9 : 1u); block += gridDim.x) {
+      uint32_t i0;
+      if (!row_pair(block, rows, i0)) continue;
+      for (uint32_t side = 0; side < 2; side++) {
+        const uint32_t i = side ? rows - 1u - i0 : i0;
         const uint32_t j = coset_perm(i, g.log_rows);
         const bool some = j >= g.lead;
         uint32_t k = 0, chunk = 0;
@@ -61,9 +82,36 @@ __global__ void __launch_bounds__(256) freivalds_scatter_kernel(const int8_t* __
         for (uint32_t m = 0; m < n_mats; m++) {
             const uint32_t no = n_out[m];
             const int8_t* __restrict__ w = qw[m] + (size_t)k * no;
-            for (uint32_t p = 0; p < pk; p++) {
-                uint32_t c = chunk * pk + p;
-                pre_cols[m * pk + p][i] = (some && c < no) ? m31_of_i32((int)w[c]) : 0u;
+            uint32_t* const* __restrict__ cols = pre_cols + m * pk;
+            const uint32_t c0 = chunk * pk, fit = (uint32_t)reinterpret_cast<uintptr_t>(qw[m]) | no | pk;  // aligned and whole: every load of the row is
+            if ((fit & 15u) == 0) {
+                for (uint32_t p = 0; p < pk; p += 16) {
+                    const uint4 x = some && c0 + p < no ? __ldg(reinterpret_cast<const uint4*>(w + c0 + p)) : make_uint4(0, 0, 0, 0);
+                    const uint32_t q[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (uint32_t u = 0; u < 16; u++) cols[p + u][i] = m31_of_i32((int)(int8_t)(q[u >> 2] >> (8 * (u & 3))));
+                }
+            } else {
+                // four at a time from aligned words; a word that is not wholly the matrix's comes in bytes
+                const uintptr_t lo = reinterpret_cast<uintptr_t>(qw[m]), hi = lo + (uintptr_t)g.groups * no;
+                auto word = [&](uintptr_t x) -> uint32_t {
+                    if (x >= lo && x + 4 <= hi) return __ldg(reinterpret_cast<const uint32_t*>(x));
+                    uint32_t v = 0;
+                    for (uint32_t u = 0; u < 4; u++)
+                        if (x + u >= lo && x + u < hi) v |= (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(x + u)) << (8 * u);
+                    return v;
+                };
+                const uintptr_t at = reinterpret_cast<uintptr_t>(w + c0);
+                const bool any = some && c0 < no;
+                uintptr_t x = at & ~(uintptr_t)3;
+                uint32_t cur = any ? word(x) : 0u;
+                for (uint32_t p = 0; p < pk; p += 4, x += 4) {
+                    const uint32_t next = any ? word(x + 4) : 0u, v = __funnelshift_r(cur, next, 8u * (uint32_t)(at & 3u));
+                    cur = next;
+#pragma unroll
+                    for (uint32_t u = 0; u < 4; u++)
+                        if (p + u < pk) cols[p + u][i] = (some && c0 + p + u < no) ? m31_of_i32((int)(int8_t)(v >> (8 * u))) : 0u;
+                }
             }
         }
         uint32_t* const* sel = pre_cols + n_mats * pk;
@@ -71,6 +119,7 @@ __global__ void __launch_bounds__(256) freivalds_scatter_kernel(const int8_t* __
         sel[1][i] = (some && chunk == 0) ? 1u : 0u;
         sel[2][i] = j > 0 ? 1u : 0u;
         sel[3][i] = j + 1 == rows ? 1u : 0u;
+      }
     }
     __syncthreads();
     for (uint32_t t = threadIdx.x; t < table_len; t += blockDim.x)
@@ -80,36 +129,47 @@ __global__ void __launch_bounds__(256) freivalds_scatter_kernel(const int8_t* __
 // ---- F2: inner products per row -----------------------------------------------------------------
 __device__ __forceinline__ uint64_t fold64f(uint64_t v) { return (v & P) + (v >> 31); }
 
-// lanes[l][j] (QM31, coset order): l = 0 is v_in, l = 1 + m is u_in of matrix m.
-__global__ void __launch_bounds__(256) freivalds_inner_kernel(const uint32_t* const* __restrict__ base_cols,
-                                                              const uint32_t* const* __restrict__ pre_cols,
-                                                              const uint4* __restrict__ s_pow, const uint4* __restrict__ rv_pow, FGrid g,
-                                                              uint32_t pq, uint32_t pk, uint32_t n_mats, uint4* __restrict__ lanes) {
-    const uint32_t rows = 1u << g.log_rows;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows) return;
-    const uint32_t j = coset_perm(i, g.log_rows);
-    const bool some = j >= g.lead;
-    {
-        uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        for (uint32_t p = 0; p < pq; p++) {
-            uint32_t x = m31_sub(base_cols[p][i], 128u);
-            uint4 c = s_pow[p];
-            a0 += (uint64_t)c.x * x; a1 += (uint64_t)c.y * x; a2 += (uint64_t)c.z * x; a3 += (uint64_t)c.w * x;
-            if ((p & 3) == 3) { a0 = fold64f(a0); a1 = fold64f(a1); a2 = fold64f(a2); a3 = fold64f(a3); }
+// lanes[l][j] (QM31, coset order): l = 0 is v_in, l = 1 + m is u_in of matrix m. Eight loads are on their way at a time (a load
+// a row, behind that of its column address, one after the other: 107 us at 2^20 rows of 33 columns).
+// sum of pow[p] (cols[p][row] - bias) for two rows
+struct RowSums { uint4 a, b; };
+__device__ __forceinline__ RowSums inner_pair(const uint32_t* const* __restrict__ cols, const uint4* __restrict__ pow, uint32_t n, uint32_t bias, uint32_t i, uint32_t i2) {
+    uint64_t a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0};
+    for (uint32_t p0 = 0; p0 < n; p0 += 4) {
+        uint32_t x[4], y[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const bool there = p0 + u < n;
+            const uint32_t* const col = there ? cols[p0 + u] : nullptr;
+            x[u] = there ? __ldcs(col + i) : bias;
+            y[u] = there ? __ldcs(col + i2) : bias;
         }
-        lanes[j] = some ? make_uint4(m31_reduce64(a0), m31_reduce64(a1), m31_reduce64(a2), m31_reduce64(a3)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {  // four products below 2^62 on top of a folded accumulator fit 64 bits
+            const uint4 c = p0 + u < n ? __ldg(pow + p0 + u) : make_uint4(0, 0, 0, 0);
+            const uint32_t v = m31_sub(x[u], bias), w = m31_sub(y[u], bias);
+            a[0] += (uint64_t)c.x * v; a[1] += (uint64_t)c.y * v; a[2] += (uint64_t)c.z * v; a[3] += (uint64_t)c.w * v;
+            b[0] += (uint64_t)c.x * w; b[1] += (uint64_t)c.y * w; b[2] += (uint64_t)c.z * w; b[3] += (uint64_t)c.w * w;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) { a[q] = fold64f(a[q]); b[q] = fold64f(b[q]); }
     }
-    for (uint32_t m = 0; m < n_mats; m++) {
-        uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        for (uint32_t p = 0; p < pk; p++) {
-            uint32_t x = pre_cols[m * pk + p][i];
-            uint4 c = rv_pow[p];
-            a0 += (uint64_t)c.x * x; a1 += (uint64_t)c.y * x; a2 += (uint64_t)c.z * x; a3 += (uint64_t)c.w * x;
-            if ((p & 3) == 3) { a0 = fold64f(a0); a1 = fold64f(a1); a2 = fold64f(a2); a3 = fold64f(a3); }
-        }
-        lanes[(size_t)(1 + m) * rows + j] =
-            some ? make_uint4(m31_reduce64(a0), m31_reduce64(a1), m31_reduce64(a2), m31_reduce64(a3)) : make_uint4(0, 0, 0, 0);
+    return {make_uint4(m31_reduce64(a[0]), m31_reduce64(a[1]), m31_reduce64(a[2]), m31_reduce64(a[3])),
+            make_uint4(m31_reduce64(b[0]), m31_reduce64(b[1]), m31_reduce64(b[2]), m31_reduce64(b[3]))};
+}
+__global__ void __launch_bounds__(256, 4) freivalds_inner_kernel(const uint32_t* const* __restrict__ base_cols,
+                                                                 const uint32_t* const* __restrict__ pre_cols,
+                                                                 const uint4* __restrict__ s_pow, const uint4* __restrict__ rv_pow, FGrid g,
+                                                                 uint32_t pq, uint32_t pk, uint32_t n_mats, uint4* __restrict__ lanes) {
+    const uint32_t rows = 1u << g.log_rows;
+    uint32_t i;
+    if (!row_pair(blockIdx.x, rows, i)) return;
+    const uint32_t i2 = rows - 1u - i, j = coset_perm(i, g.log_rows), j2 = coset_perm(i2, g.log_rows);
+    for (uint32_t l = 0; l <= n_mats; l++) {
+        const RowSums r = l ? inner_pair(pre_cols + (size_t)(l - 1) * pk, rv_pow, pk, 0u, i, i2) : inner_pair(base_cols, s_pow, pq, 128u, i, i2);
+        uint4* const out = lanes + (size_t)l * rows;
+        out[j] = j >= g.lead ? r.a : make_uint4(0, 0, 0, 0);
+        out[j2] = j2 >= g.lead ? r.b : make_uint4(0, 0, 0, 0);
     }
 }
 
@@ -117,161 +177,115 @@ __global__ void __launch_bounds__(256) freivalds_inner_kernel(const uint32_t* co
 __device__ __forceinline__ qm31 q_of(uint4 v) { return {{v.x, v.y, v.z, v.w}}; }
 __device__ __forceinline__ uint4 u_of(qm31 v) { return make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]); }
 
-// One thread per (group slot, lane): x_r = x_{r-1} step + in_r over the group's `chunks` rows.
-__global__ void __launch_bounds__(128) freivalds_group_scan_kernel(uint4* __restrict__ lanes, FGrid g, uint32_t n_lanes, qm31 s_step,
-                                                                   qm31 rv_step) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.groups * n_lanes) return;
-    const uint32_t lane = t / g.groups, slot = t % g.groups;
-    const qm31 step = lane == 0 ? s_step : rv_step;
-    uint4* __restrict__ p = lanes + ((size_t)lane << g.log_rows) + g.lead + (size_t)slot * g.chunks;
-    qm31 acc = q_of(p[0]);
-    for (uint32_t r = 1; r < g.chunks; r++) {
-        acc = qm31_add(qm31_mul(acc, step), q_of(p[r]));
-        p[r] = u_of(acc);
-    }
-}
-
-// The same recurrence with one WARP per group (groups of at most 256 rows): lane l takes rows 8l .. 8l+7, runs them from a
-// zero carry into registers, the lanes' (multiplier, value) pairs are combined by a shuffle scan of affine maps
-// ((A2, B2) o (A1, B1) = (A1 A2, B1 A2 + B2)), and each lane then adds its carry times the running power of the step. All
-// lanes of the group go through the same warp one after the other, so that the product u_m v of the group's last row
-// (what the prefix over groups sums) is at hand and is written to prod[m][slot]. One thread per (group, lane) walking 256
-// rows in sequence kept 6% of the warp slots busy and took as long as the pass over all the input columns.
+// x_r = x_{r-1} step + in_r over the group's `chunks` rows, one WARP a group, 256 rows at a time: lane l takes rows 8l .. 8l+7, runs
+// them from a zero carry into registers, the lanes' values are combined by a shuffle scan (a lane of eight rows multiplies what
+// comes before it by step^8, so the multipliers of the scan are constants), and each lane then adds its carry times the running power
+// of the step. All lanes (v, then the u_m) of the group go through the same warp one after the other, so that the product
+// u_m v of the group's last row (what the prefix over groups sums) is at hand and is written to prod[m][slot]. Bound by its products,
+// 22 a lane and eight rows (with the multipliers scanned too: 26). One thread per (group, lane) walking 256 rows in sequence
+// kept 6% of the warp slots busy and took as long as the pass over all the input columns.
 struct ScanSteps {
-    qm31 pw[2][9];  // pw[kind][k] = step^k for k = 0..8; kind 0 is lane 0 (v, step s^pq), kind 1 the lanes u_m (step rv^pk)
+    qm31 pw[2][9];    // pw[kind][k] = step^k for k = 0..8; kind 0 is lane 0 (v, step s^pq), kind 1 the lanes u_m (step rv^pk)
+    qm31 wide[2][6];  // step^(8 2^k)
 };
-__global__ void __launch_bounds__(256) freivalds_group_scan_warp_kernel(uint4* __restrict__ lanes, FGrid g, uint32_t n_mats, ScanSteps st,
-                                                                        uint4* __restrict__ prod) {
+__global__ void __launch_bounds__(256) freivalds_group_scan_kernel(uint4* __restrict__ lanes, FGrid g, uint32_t n_mats, const __grid_constant__ ScanSteps st,
+                                                                   uint4* __restrict__ prod) {
     const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (slot >= g.groups) return;
-    const uint32_t r0 = lane * 8u, n_here = r0 >= g.chunks ? 0u : (g.chunks - r0 < 8u ? g.chunks - r0 : 8u);
     qm31 v_last = qm31_zero();
     for (uint32_t l = 0; l <= n_mats; l++) {
         const qm31* pw = st.pw[l ? 1 : 0];
+        const qm31* wide = st.wide[l ? 1 : 0];
         const qm31 step = pw[1];
-        uint4* __restrict__ p = lanes + ((size_t)l << g.log_rows) + g.lead + (size_t)slot * g.chunks + r0;
-        qm31 y[8];
-        qm31 acc = qm31_zero();
+        uint4* __restrict__ p = lanes + ((size_t)l << g.log_rows) + g.lead + (size_t)slot * g.chunks;
+        qm31 end = qm31_zero();  // the value after the last row so far
+        for (uint32_t base = 0; base < g.chunks; base += 256, p += 256) {
+            const uint32_t left = g.chunks - base, r0 = lane * 8u, n_here = r0 >= left ? 0u : (left - r0 < 8u ? left - r0 : 8u);
+            qm31 y[8];
+            qm31 acc = qm31_zero();
 #pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (k < n_here) {
-                acc = qm31_add(qm31_mul(acc, step), q_of(p[k]));
-                y[k] = acc;
-            }
-        const qm31 mult = pw[n_here];  // this lane's map: x -> mult x + acc
-        // inclusive scan of the maps over the lanes
-        qm31 A = mult, B = acc;
+            for (uint32_t k = 0; k < 8; k++)
+                if (k < n_here) {
+                    acc = qm31_add(qm31_mul(acc, step), q_of(p[r0 + k]));
+                    y[k] = acc;
+                }
+            // The value after a lane's rows, exact for lanes whose rows before them are all there: only the last lane with rows may
+            // have fewer than eight, and nothing is taken from it or from the ones after.
+            qm31 B = lane == 0 && base ? qm31_add(acc, qm31_mul(end, pw[n_here])) : acc;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            qm31 a1, b1;
+            for (int k = 0; k < 5; k++) {
+                qm31 b1;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                a1.c[c] = __shfl_up_sync(0xffffffffu, A.c[c], off);
-                b1.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], off);
+                for (int c = 0; c < 4; c++) b1.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1 << k);
+                if ((int)lane >= (1 << k)) B = qm31_add(qm31_mul(b1, wide[k]), B);
             }
-            if ((int)lane >= off) {
-                B = qm31_add(qm31_mul(b1, A), B);
-                A = qm31_mul(a1, A);
-            }
+            qm31 carry;  // into this lane: the value at the end of the previous one
+#pragma unroll
+            for (int c = 0; c < 4; c++) carry.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1);
+            if (lane == 0) carry = end;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++)
+                if (k < n_here) {
+                    acc = qm31_add(y[k], qm31_mul(carry, pw[k + 1]));
+                    p[r0 + k] = u_of(acc);
+                }
+            const int from = (int)((left < 256u ? left : 256u) - 1u) >> 3;  // the lane of the last row
+#pragma unroll
+            for (int c = 0; c < 4; c++) end.c[c] = __shfl_sync(0xffffffffu, acc.c[c], from);
         }
-        // carry into this lane = the value at the end of the previous lane
-        qm31 carry;
-#pragma unroll
-        for (int c = 0; c < 4; c++) carry.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1);
-        if (lane == 0) carry = qm31_zero();
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (k < n_here) p[k] = u_of(qm31_add(y[k], qm31_mul(carry, pw[k + 1])));
-        // the group's last row is in the last lane that has rows; B of lane 31 is the value there either way
-        qm31 end;
-#pragma unroll
-        for (int c = 0; c < 4; c++) end.c[c] = __shfl_sync(0xffffffffu, B.c[c], 31);
         if (l == 0) v_last = end;
         else if (lane == 0) prod[(size_t)(l - 1) * g.groups + slot] = u_of(qm31_mul(end, v_last));
     }
 }
 
-// prefix[m][slot] = sum over slots <= slot of prod[m][slot]; one CTA, coalesced reads.
-__global__ void __launch_bounds__(1024) freivalds_prefix_prod_kernel(const uint4* __restrict__ prod, uint32_t groups, uint32_t n_mats,
-                                                                     uint4* __restrict__ prefix) {
-    __shared__ uint32_t warp_tot[32][4];
-    __shared__ uint32_t carry_s[4];
-    const int lane_id = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t m = 0; m < n_mats; m++) {
-        if (threadIdx.x < 4) carry_s[threadIdx.x] = 0;
-        __syncthreads();
-        for (uint32_t base = 0; base < groups; base += blockDim.x) {
-            const uint32_t slot = base + threadIdx.x;
-            qm31 x = slot < groups ? q_of(prod[(size_t)m * groups + slot]) : qm31_zero();
+// In place: prefix[m][slot] = sum over slots <= slot of what is there; a CTA a matrix, a thread a run of slots. The whole sum is the
+// matrix's claim: it goes to page-locked memory as well. (One CTA for all matrices, 1,024 slots at a time: 16 us for 2 x 4,096.)
+__global__ void __launch_bounds__(1024) freivalds_prefix_kernel(uint4* __restrict__ prefix, uint32_t groups, uint4* __restrict__ claims) {
+    __shared__ qm31 warp_tot[32];
+    const uint32_t run = (groups + 1023u) / 1024u, first = threadIdx.x * run, last = first + run < groups ? first + run : groups;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* __restrict__ p = prefix + (size_t)blockIdx.x * groups;
+    auto shift = [&](qm31 v, int off) {
+        qm31 o;
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                qm31 o;
+        for (int k = 0; k < 4; k++) o.c[k] = __shfl_up_sync(0xffffffffu, v.c[k], off);
+        return o;
+    };
+    qm31 sum = qm31_zero();
+#pragma unroll 4
+    for (uint32_t s = first; s < last; s++) sum = qm31_add(sum, q_of(p[s]));
+    auto scan = [&](qm31 x) {  // inclusive, over the warp
 #pragma unroll
-                for (int k = 0; k < 4; k++) o.c[k] = __shfl_up_sync(0xffffffffu, x.c[k], off);
-                if (lane_id >= off) x = qm31_add(x, o);
-            }
-            if (lane_id == 31)
-                for (int k = 0; k < 4; k++) warp_tot[warp][k] = x.c[k];
-            __syncthreads();
-            qm31 pre{{carry_s[0], carry_s[1], carry_s[2], carry_s[3]}};
-            for (int w = 0; w < warp; w++) pre = qm31_add(pre, qm31{{warp_tot[w][0], warp_tot[w][1], warp_tot[w][2], warp_tot[w][3]}});
-            x = qm31_add(x, pre);
-            if (slot < groups) prefix[(size_t)m * groups + slot] = u_of(x);
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1)
-                for (int k = 0; k < 4; k++) carry_s[k] = x.c[k];
-            __syncthreads();
+        for (int off = 1; off < 32; off <<= 1) {
+            const qm31 o = shift(x, off);
+            if (lane >= off) x = qm31_add(x, o);
         }
+        return x;
+    };
+    const qm31 mine = scan(sum);
+    if (lane == 31) warp_tot[warp] = mine;
+    __syncthreads();
+    if (warp == 0) warp_tot[lane] = scan(warp_tot[lane]);
+    __syncthreads();
+    qm31 acc = shift(mine, 1);
+    if (lane == 0) acc = qm31_zero();
+    if (warp) acc = qm31_add(acc, warp_tot[warp - 1]);
+    for (uint32_t s = first; s < last; s++) {
+        acc = qm31_add(acc, q_of(p[s]));
+        p[s] = u_of(acc);
     }
-}
-
-// One CTA: prefix[m][slot] = sum over slots <= slot of u_m[last row] * v[last row].
-__global__ void __launch_bounds__(1024) freivalds_prefix_kernel(const uint4* __restrict__ lanes, FGrid g, uint32_t n_mats,
-                                                                uint4* __restrict__ prefix) {
-    __shared__ uint32_t warp_tot[32][4];
-    __shared__ uint32_t carry_s[4];
-    const uint32_t rows = 1u << g.log_rows;
-    const int lane_id = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t m = 0; m < n_mats; m++) {
-        if (threadIdx.x < 4) carry_s[threadIdx.x] = 0;
-        __syncthreads();
-        for (uint32_t base = 0; base < g.groups; base += blockDim.x) {
-            uint32_t slot = base + threadIdx.x;
-            qm31 x = qm31_zero();
-            if (slot < g.groups) {
-                size_t last = (size_t)g.lead + (size_t)slot * g.chunks + g.chunks - 1;
-                x = qm31_mul(q_of(lanes[(size_t)(1 + m) * rows + last]), q_of(lanes[last]));
-            }
-            // inclusive scan inside the warp
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                qm31 o;
-#pragma unroll
-                for (int k = 0; k < 4; k++) o.c[k] = __shfl_up_sync(0xffffffffu, x.c[k], off);
-                if (lane_id >= off) x = qm31_add(x, o);
-            }
-            if (lane_id == 31)
-                for (int k = 0; k < 4; k++) warp_tot[warp][k] = x.c[k];
-            __syncthreads();
-            qm31 pre{{carry_s[0], carry_s[1], carry_s[2], carry_s[3]}};
-            for (int w = 0; w < warp; w++) pre = qm31_add(pre, qm31{{warp_tot[w][0], warp_tot[w][1], warp_tot[w][2], warp_tot[w][3]}});
-            x = qm31_add(x, pre);
-            if (slot < g.groups) prefix[(size_t)m * g.groups + slot] = u_of(x);
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1)
-                for (int k = 0; k < 4; k++) carry_s[k] = x.c[k];
-            __syncthreads();
-        }
-    }
+    if (first < last && last == groups) claims[blockIdx.x] = u_of(acc);
 }
 
 // out: (1 + 2 n_mats) secure columns of 4 coordinate columns each, committed order.
 __global__ void __launch_bounds__(256) freivalds_split_kernel(const uint4* __restrict__ lanes, const uint4* __restrict__ prefix, FGrid g,
                                                               uint32_t n_mats, uint32_t* const* __restrict__ out) {
     const uint32_t rows = 1u << g.log_rows;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows) return;
+    uint32_t i0;
+    if (!row_pair(blockIdx.x, rows, i0)) return;
+#pragma unroll
+    for (uint32_t side = 0; side < 2; side++) {
+    const uint32_t i = side ? rows - 1u - i0 : i0;
     const uint32_t j = coset_perm(i, g.log_rows);
     const bool some = j >= g.lead;
     uint32_t slot = 0;
@@ -293,6 +307,7 @@ __global__ void __launch_bounds__(256) freivalds_split_kernel(const uint4* __res
         }
         uint32_t* const* oa = out + 8 + 8 * m;
         oa[0][i] = a.x; oa[1][i] = a.y; oa[2][i] = a.z; oa[3][i] = a.w;
+    }
     }
 }
 
@@ -325,13 +340,15 @@ int zkb_freivalds_scatter(zkb_ctx* ctx, const int8_t* qx, const int8_t* const* q
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)qw, (int)n_mats, &d_qw);
     if (rc) return rc;
-    uint32_t* d_nout = ctx->scratch;
-    ZKB_CUDA(ctx, cudaMemcpyAsync(d_nout, h_n_out, n_mats * 4, cudaMemcpyHostToDevice, ctx->stream));
+    void* d_nout = nullptr;
+    rc = stage_blob(ctx, h_n_out, n_mats * 4, &d_nout);
+    if (rc) return rc;
     FGrid fg{grid->log_rows, grid->groups, grid->chunks, grid->lead};
     uint32_t rows = 1u << grid->log_rows;
     ProfScope prof(ctx, "freivalds_scatter_kernel");
-    freivalds_scatter_kernel<<<(rows + 255) / 256, 256, table_len * 4, ctx->stream>>>(
-        qx, (const int8_t* const*)d_qw, d_nout, fg, pq, pk, n_in, tokens, n_mats, (uint32_t* const*)d_base, (uint32_t* const*)d_pre,
+    const uint32_t grid_ctas = std::min(row_pair_blocks(rows), 148u * 8u);
+    freivalds_scatter_kernel<<<grid_ctas, SCATTER_THREADS, table_len * 4, ctx->stream>>>(
+        qx, (const int8_t* const*)d_qw, (const uint32_t*)d_nout, fg, pq, pk, n_in, tokens, n_mats, (uint32_t* const*)d_base, (uint32_t* const*)d_pre,
         m_r8, table_len, off_table);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
@@ -375,50 +392,29 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     FGrid fg{grid->log_rows, grid->groups, grid->chunks, grid->lead};
     {
         ProfScope prof(ctx, "freivalds_inner_kernel");
-        freivalds_inner_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, ctx->stream>>>(
+        freivalds_inner_kernel<<<row_pair_blocks(rows), 256, 0, ctx->stream>>>(
             (const uint32_t* const*)d_base, (const uint32_t* const*)d_pre, d_pows, d_pows + pq, fg, pq, pk, n_mats, lanes);
     }
-    if (grid->chunks <= 256) {
-        ScanSteps scan_steps;
-        for (int kind = 0; kind < 2; kind++) {
-            scan_steps.pw[kind][0] = qm31_one();
-            for (int k = 1; k <= 8; k++) scan_steps.pw[kind][k] = qm31_mul(scan_steps.pw[kind][k - 1], kind ? rv_step : s_step);
-        }
-        uint4* prod = nullptr;  // u_m v at each group's last row
-        e = cudaMallocAsync((void**)&prod, (size_t)n_mats * grid->groups * 16, ctx->stream);
-        if (e != cudaSuccess) {
-            cudaFreeAsync(lanes, ctx->stream);
-            cudaFreeAsync(prefix, ctx->stream);
-            return set_error(ctx, ZKB_ENOMEM, "zkb_freivalds_acc: %s", cudaGetErrorString(e));
-        }
-        {
-            ProfScope prof(ctx, "freivalds_group_scan_kernel");
-            freivalds_group_scan_warp_kernel<<<(unsigned)(((size_t)grid->groups * 32 + 255) / 256), 256, 0, ctx->stream>>>(
-                lanes, fg, n_mats, scan_steps, prod);
-        }
-        {
-            ProfScope prof(ctx, "freivalds_prefix_kernel");
-            freivalds_prefix_prod_kernel<<<1, 1024, 0, ctx->stream>>>(prod, grid->groups, n_mats, prefix);
-        }
-        cudaFreeAsync(prod, ctx->stream);
-    } else {
-        {
-            ProfScope prof(ctx, "freivalds_group_scan_kernel");
-            unsigned threads_total = grid->groups * n_lanes;
-            freivalds_group_scan_kernel<<<(threads_total + 127) / 128, 128, 0, ctx->stream>>>(lanes, fg, n_lanes, s_step, rv_step);
-        }
-        {
-            ProfScope prof(ctx, "freivalds_prefix_kernel");
-            freivalds_prefix_kernel<<<1, 1024, 0, ctx->stream>>>(lanes, fg, n_mats, prefix);
-        }
+    ScanSteps scan_steps;
+    for (int kind = 0; kind < 2; kind++) {
+        scan_steps.pw[kind][0] = qm31_one();
+        for (int k = 1; k <= 8; k++) scan_steps.pw[kind][k] = qm31_mul(scan_steps.pw[kind][k - 1], kind ? rv_step : s_step);
+        scan_steps.wide[kind][0] = scan_steps.pw[kind][8];
+        for (int k = 1; k < 6; k++) scan_steps.wide[kind][k] = qm31_mul(scan_steps.wide[kind][k - 1], scan_steps.wide[kind][k - 1]);
+    }
+    {
+        ProfScope prof(ctx, "freivalds_group_scan_kernel");
+        freivalds_group_scan_kernel<<<(unsigned)(((size_t)grid->groups * 32 + 255) / 256), 256, 0, ctx->stream>>>(lanes, fg, n_mats, scan_steps, prefix);
+    }
+    {
+        ProfScope prof(ctx, "freivalds_prefix_kernel");
+        freivalds_prefix_kernel<<<n_mats, 1024, 0, ctx->stream>>>(prefix, grid->groups, reinterpret_cast<uint4*>(ctx->h_small));
     }
     {
         ProfScope prof(ctx, "freivalds_split_kernel");
-        freivalds_split_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, ctx->stream>>>(lanes, prefix, fg, n_mats, (uint32_t* const*)d_out);
+        freivalds_split_kernel<<<row_pair_blocks(rows), 256, 0, ctx->stream>>>(lanes, prefix, fg, n_mats, (uint32_t* const*)d_out);
     }
     e = cudaGetLastError();
-    for (uint32_t m = 0; m < n_mats && e == cudaSuccess; m++)
-        e = cudaMemcpyAsync(ctx->h_small + 4 * m, prefix + (size_t)m * grid->groups + grid->groups - 1, 16, cudaMemcpyDeviceToHost, ctx->stream);
     cudaFreeAsync(lanes, ctx->stream);
     cudaFreeAsync(prefix, ctx->stream);
     if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "zkb_freivalds_acc: %s", cudaGetErrorString(e));
