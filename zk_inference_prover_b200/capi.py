@@ -108,6 +108,12 @@ def load_library():
         for name in EXPORTED_SYMBOLS + PROVER_SYMBOLS + AIR_SYMBOLS:
             if name not in ("zkb_last_error", "zkb_gkr_sum_noalloc_error"):
                 getattr(_lib, name).restype = C.c_int
+        # Calls made by the hundred (a tree layer by layer, a fold after the other): with their types declared the plain integers
+        # convert in half the time that a ctypes object apiece takes.
+        p, i = C.c_void_p, C.c_int
+        _lib.zkb_merkle_layer.argtypes = [p, i, p, p, i, i, p]
+        _lib.zkb_fold_line.argtypes = [p, p, p, i, p]
+        _lib.zkb_d2d.argtypes = [p, p, p, C.c_size_t]
     return _lib
 
 
@@ -328,6 +334,7 @@ class Context:
             raise ZkbError(rc, "zkb_init failed (is a CUDA device visible?)")
         self.h = h
         self.max_log_size = max_log_size
+        self._rooms = []  # see _room
 
     def close(self):
         if getattr(self, "h", None):
@@ -343,6 +350,21 @@ class Context:
     def _check(self, rc):
         if rc != 0:
             raise ZkbError(rc, self.lib.zkb_last_error(self.h).decode())
+
+    def _room(self, cap):
+        """A host buffer of at least `cap` words for a call's output. Up to two are kept between calls (one per thread that is in a
+        call): 64 MB fresh from the system cost their mapping and a fault per page written, more than a small proof's copy."""
+        try:
+            room = self._rooms.pop()
+        except IndexError:
+            room = None
+        return room if room is not None and room.size >= cap else np.empty(cap, np.uint32)
+
+    def _taken(self, room, n):
+        words = room[:n].copy()
+        if len(self._rooms) < 2 and room.size <= 1 << 24:
+            self._rooms.append(room)
+        return words
 
     # ---- memory
     def alloc(self, words):
@@ -447,7 +469,7 @@ class Context:
         self._check(self.lib.zkb_peer_copies_wait(self.h))
 
     def d2d(self, dst, src, nbytes):
-        self._check(self.lib.zkb_d2d(self.h, C.c_void_p(dst), C.c_void_p(src), C.c_size_t(nbytes)))
+        self._check(self.lib.zkb_d2d(self.h, dst, src, nbytes))
 
     def stream(self):
         s = C.c_void_p()
@@ -504,8 +526,10 @@ class Context:
 
     # ---- MerkleOps
     def merkle_layer(self, log_size, prev_ptr, col_ptrs, out_ptr, m31_out=True):
-        self._check(self.lib.zkb_merkle_layer(self.h, C.c_int(log_size), C.c_void_p(prev_ptr or None), _ptr_array(col_ptrs),
-                                              C.c_int(len(col_ptrs)), C.c_int(int(m31_out)), C.c_void_p(out_ptr)))
+        n = len(col_ptrs)
+        rc = self.lib.zkb_merkle_layer(self.h, log_size, prev_ptr or None, _ptr_array(col_ptrs) if n else None, n, int(m31_out), out_ptr)
+        if rc:
+            self._check(rc)
 
     def merkle_leaves_partial(self, log_size, col_ptrs, cols_before, total_cols, out_ptr, m31_out=True):
         arr = (C.c_void_p * len(col_ptrs))(*col_ptrs)
@@ -522,7 +546,7 @@ class Context:
     # ---- FriOps
     def fold_line(self, out4, in4, log_n, alpha):
         a = _u32(alpha)
-        self._check(self.lib.zkb_fold_line(self.h, _ptr_array(out4), _ptr_array(in4), C.c_int(log_n), a.ctypes.data_as(C.c_void_p)))
+        self._check(self.lib.zkb_fold_line(self.h, _ptr_array(out4), _ptr_array(in4), log_n, a.ctypes.data))
 
     def fold_circle_into_line(self, dst4, src4, log_n_src, alpha):
         a = _u32(alpha)
@@ -712,15 +736,15 @@ class Context:
 
     def _pcs(self, fn, trees_ptrs, logs, pow_bits, log_blowup, log_last_layer, n_queries, two_sample_every, cap, phases):
         prepared = trees_ptrs if isinstance(trees_ptrs, dict) else None
-        a = prepared or self.pcs_prepare(trees_ptrs, logs, cap)
+        a = prepared or self.pcs_prepare(trees_ptrs, logs, 1)
         cfg = PcsConfig(pow_bits, log_blowup, log_last_layer, n_queries)
-        out = a["out"]
+        out = a["out"] if prepared else self._room(cap)
         n = C.c_size_t()
         ph = np.zeros(len(PCS_PHASES), np.float32)
         self._check(fn(self.h, C.c_int(a["n_trees"]), a["ncols"].ctypes.data_as(C.c_void_p), a["ptrs"], a["logs"].ctypes.data_as(C.c_void_p),
-                       C.byref(cfg), C.c_int(two_sample_every), out.ctypes.data_as(C.c_void_p), C.c_size_t(out.size), C.byref(n),
+                       C.byref(cfg), C.c_int(two_sample_every), out.ctypes.data_as(C.c_void_p), C.c_size_t(out.size if prepared else cap), C.byref(n),
                        ph.ctypes.data_as(C.c_void_p) if phases else None))
-        words = out[:n.value] if prepared else out[:n.value].copy()
+        words = out[:n.value] if prepared else self._taken(out, n.value)
         return (words, dict(zip(PCS_PHASES, ph.tolist()))) if phases else words
 
     def pcs_prove_device(self, trees_ptrs, logs, pow_bits=10, log_blowup=1, log_last_layer=0, n_queries=3, two_sample_every=0,
@@ -751,7 +775,7 @@ class Context:
         cfg = PcsConfig(pow_bits, log_blowup, log_last_layer, n_queries)
         sc = _u32(prog.source.scalars if scalars is None else scalars)
         cs = _u32(claimed_sum) if claimed_sum is not None else None
-        out = np.empty(cap, np.uint32)
+        out = self._room(cap)
         n = C.c_size_t()
         oods = np.zeros(8, np.uint32)
         ph = (C.c_float * len(PCS_PHASES))()
@@ -769,7 +793,7 @@ class Context:
         if phases is not None:
             phases.update({k: float(ph[i]) for i, k in enumerate(PCS_PHASES)})
             phases["composition"] = float(comp_ms.value)
-        return out[:n.value].copy(), oods[:4].copy(), oods[4:].copy(), float(comp_ms.value)
+        return self._taken(out, n.value), oods[:4].copy(), oods[4:].copy(), float(comp_ms.value)
 
     def stark_prove_multi(self, components, trees, pow_bits=10, log_blowup=1, log_last_layer=0, n_queries=3, cap=1 << 24, phases=None,
                           host=False):
@@ -790,7 +814,7 @@ class Context:
             arr[i].claimed_sum = cs.ctypes.data if cs is not None else None
         ncols = np.array([len(t) for t in trees], dtype=np.int32)
         cfg = PcsConfig(pow_bits, log_blowup, log_last_layer, n_queries)
-        out = np.empty(cap, np.uint32)
+        out = self._room(cap)
         n = C.c_size_t()
         oods = np.zeros(8, np.uint32)
         ph = (C.c_float * len(PCS_PHASES))()
@@ -807,7 +831,7 @@ class Context:
         if phases is not None:
             phases.update({k: float(ph[i]) for i, k in enumerate(PCS_PHASES)})
             phases["composition"] = float(comp_ms.value)
-        return out[:n.value].copy(), oods[:4].copy(), oods[4:].copy(), float(comp_ms.value)
+        return self._taken(out, n.value), oods[:4].copy(), oods[4:].copy(), float(comp_ms.value)
 
     def gkr_prove_device(self, instances, seed, cap=1 << 22):
         """instances: list of (kind, num_ptr or 0, den_ptr, n_entries)."""
@@ -815,9 +839,9 @@ class Context:
         nums = (C.c_void_p * len(instances))(*[(n or None) for _, n, _, _ in instances])
         dens = (C.c_void_p * len(instances))(*[d for _, _, d, _ in instances])
         ns = np.array([n for _, _, _, n in instances], np.uint64)
-        out = np.empty(cap, np.uint32)
+        out = self._room(cap)
         nw = C.c_size_t()
         self._check(self.lib.zkb_gkr_prove_device(self.h, C.c_int(len(instances)), kinds.ctypes.data_as(C.c_void_p), nums, dens,
                                                   ns.ctypes.data_as(C.c_void_p), C.c_uint64(seed), out.ctypes.data_as(C.c_void_p),
                                                   C.c_size_t(cap), C.byref(nw)))
-        return out[:nw.value].copy()
+        return self._taken(out, nw.value)

@@ -5,7 +5,10 @@
 // hashed with Blake2s-256 (RFC 7693) and, for the M31 hasher, each digest word reduced mod 2^31-1
 // (core/vcs/blake2_hash.rs:111-118). One thread hashes one node: the column words ARE the message
 // words, so a 64-byte block is 16 coalesced loads (one per column) straight into registers.
+#include <algorithm>
+
 #include "blake2s.cuh"
+#include "channel.cuh"
 #include "common.cuh"
 
 namespace zk {
@@ -57,13 +60,74 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(int log_size, const u
     store_hash(out, i, h, m31_out != 0);
 }
 
-// The same node hash for layers of few rows and many columns (a segment's trees hold tens of thousands of columns of
+// The same node hash for layers of at most 2^13 nodes, four lanes to a node (b2s_compress_quad in channel.cuh). Such a layer is
+// bound by the latency of its compressions, and by fetching their code where it is one of a few: a quad issues a quarter of
+// a thread's instructions from a quarter of the code. A lane brings four of a block's sixteen words; a block's words
+// and the addresses of the next one's are on their way while the block before is hashed. A tree of 2^16 leaves built layer by
+// layer, with the next launch started early (below): 5.4 -> 4.2 us a layer.
+constexpr int QUAD_THREADS = 64, QUAD_MAX_LOG = 13;
+__global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log_size, const uint32_t* __restrict__ prev,
+                                                                         const uint32_t* const* __restrict__ cols, int ncols, int m31_out,
+                                                                         uint32_t* __restrict__ out) {
+    __shared__ uint32_t sched[40];
+    __shared__ alignas(16) uint32_t msg[QUAD_THREADS / 4][PAIR_WORDS];
+    const uint32_t node = blockIdx.x * (QUAD_THREADS / 4) + (threadIdx.x >> 2), l = threadIdx.x & 3u;
+    const bool live = (node >> log_size) == 0;
+    const uint32_t i = live ? node : 0u;
+    const int col_blocks = (ncols + 15) / 16, first = prev ? 0 : 1, end = prev || ncols ? 1 + col_blocks : 2;  // block 0: the children
+    const uint32_t* at[4] = {nullptr, nullptr, nullptr, nullptr};
+    uint32_t next[4] = {0u, 0u, 0u, 0u};
+    auto addresses = [&](int b) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int c = 16 * b + 4 * (int)l + u;
+            at[u] = c < ncols ? cols[c] : nullptr;
+        }
+    };
+    auto values = [&] {
+#pragma unroll
+        for (int u = 0; u < 4; u++) next[u] = at[u] ? __ldg(at[u] + i) : 0u;
+    };
+    quad_make_schedule(sched, threadIdx.x, QUAD_THREADS);
+    // A tree built layer by layer is a chain of launches of a microsecond or two: the next one may start now (programmatic dependent
+    // launch) and wait here for this grid to end.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    addresses(0);
+    uint4 cur = make_uint4(0u, 0u, 0u, 0u);
+    if (prev) cur = reinterpret_cast<const uint4*>(prev)[4 * (size_t)i + l];
+    values();
+    addresses(1);
+    __syncthreads();
+    const QuadConst k;
+    uint2 h = make_uint2(k.h0, k.h1);
+    uint32_t* const m = msg[threadIdx.x >> 2];
+#pragma unroll 1
+    for (int b = first; b < end; b++) {
+        if (b > 0) cur = make_uint4(next[0], next[1], next[2], next[3]);
+        *reinterpret_cast<uint4*>(m + 4 * l) = cur;
+        if (b > 0) {
+            values();
+            addresses(b + 1);
+        }
+        __syncwarp();
+        const bool last = b + 1 == end;
+        const uint32_t bytes = (prev ? 64u : 0u) + 4u * (uint32_t)(16 * b < ncols ? 16 * b : ncols);
+        h = b2s_compress_quad(h, m, sched, k, bytes, last ? 0xffffffffu : 0u);
+        __syncwarp();
+    }
+    if (live) {
+        out[8 * (size_t)node + l] = m31_out ? reduce_word_m31(h.x) : h.x;
+        out[8 * (size_t)node + 4 + l] = m31_out ? reduce_word_m31(h.y) : h.y;
+    }
+}
+
+// One thread a node for layers of few rows and many columns (a segment's trees hold tens of thousands of columns of
 // 2^8 ... 2^11 rows: a leaf is then a chain of up to 2,000 compressions on a few hundred threads, and what a thread waits for
 // is the memory latency of its next sixteen column words, not the arithmetic). A warp issues in order, so a word whose column
 // pointer has not arrived holds up the compression behind it: the loads therefore run two blocks deep. During the compression
 // of block b the sixteen words of block b + 1 are in flight (their pointers arrived during block b - 1) and so are the sixteen
-// pointers of block b + 2. (Spreading a compression over four lanes was tried for these layers and is slower: the four column
-// steps of a round are already independent instructions of one thread, and the lane exchanges add latency.)
+// pointers of block b + 2.
 __global__ void __launch_bounds__(256) merkle_layer_prefetch_kernel(int log_size, const uint32_t* __restrict__ prev,
                                                                     const uint32_t* const* __restrict__ cols, int ncols, int m31_out,
                                                                     uint32_t* __restrict__ out) {
@@ -208,83 +272,99 @@ __global__ void __launch_bounds__(256) merkle_levels_kernel(MerkleLevelsArgs a, 
 
 // Blake2sM31Channel on the device, for protocol loops whose next launch only needs a challenge
 // (FRI: mix the layer's root, draw the folding challenge). State: chan[0..8) = digest, chan[8] = n_draws.
-// mix_root is H(digest || root) (core/vcs/blake2_merkle.rs:53-58); draw_secure_felt hashes
-// digest || n_draws (LE) || 0x00 and retries while a word is >= 2p (core/channel/blake2s.rs:34-52,
-// 95-120); every digest word is reduced mod p.
-__device__ __forceinline__ void channel_mix_root_draw(uint32_t* __restrict__ chan, const uint32_t* root,
-                                                      uint32_t* __restrict__ alpha_out, uint32_t* __restrict__ root_copy) {
-    uint32_t h[8], m[16];
-    blake2s_init(h);
-#pragma unroll
-    for (int k = 0; k < 8; k++) { m[k] = chan[k]; m[8 + k] = root[k]; }
-    blake2s_compress(h, m, 64u, true);
-    uint32_t digest[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) digest[k] = reduce_word_m31(h[k]);
-    uint32_t n_draws = 0, u[8];
-    for (int attempt = 0; attempt < 64; attempt++) {  // the words are already below p: one pass in practice
-        blake2s_init(h);
-#pragma unroll
-        for (int k = 0; k < 8; k++) m[k] = digest[k];
-        m[8] = n_draws;
-#pragma unroll
-        for (int k = 9; k < 16; k++) m[k] = 0u;
-        blake2s_compress(h, m, 37u, true);
-        n_draws++;
-        bool ok = true;
-#pragma unroll
-        for (int k = 0; k < 8; k++) { u[k] = reduce_word_m31(h[k]); ok = ok && u[k] < 2u * P; }
-        if (ok) break;
-    }
-    if (root_copy) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) root_copy[k] = root[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 8; k++) chan[k] = digest[k];
-    chan[8] = n_draws;
-#pragma unroll
-    for (int k = 0; k < 4; k++) alpha_out[k] = u[k] >= P ? u[k] - P : u[k];
-}
+// mix_root is H(digest || root) (core/vcs/blake2_merkle.rs:53-58); draw_secure_felt is chan_step's.
 __global__ void channel_mix_root_draw_kernel(uint32_t* __restrict__ chan, const uint32_t* __restrict__ root,
                                              uint32_t* __restrict__ alpha_out, uint32_t* __restrict__ root_copy) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    channel_mix_root_draw(chan, root, alpha_out, root_copy);
+    __shared__ ChanSm ch;
+    __shared__ uint32_t felt[4];
+    const int lane = threadIdx.x;
+    chan_make_schedule(ch, lane, 32);
+    const uint32_t w = lane < 8 ? root[lane] : 0u;
+    ch.msg[lane] = lane < 8 ? chan[lane] : 0u;
+    __syncwarp();
+    if (lane < 8) {
+        ch.msg[8 + lane] = w;
+        if (root_copy) root_copy[lane] = w;
+    }
+    if (lane == 0) ch.n_draws = chan[8];
+    chan_step(ch, 8, 1, felt);
+    if (lane < 8) chan[lane] = ch.msg[lane];
+    if (lane == 8) chan[8] = ch.n_draws;
+    if (lane < 4) alpha_out[lane] = felt[lane];
 }
 
 // The last (at most ten) layers of a tree in one CTA. Every level is written to its layer array and kept in shared memory
 // for the next one (a level read back from global memory costs an L2 round trip on top of the compression; ten levels are a
-// chain of ten dependent hashes either way). When `chan` is given, the thread that wrote the root goes on with the channel
-// step of a FRI layer (mix the root, draw the folding challenge), which would otherwise be a launch of its own.
-// (Spreading a compression of the upper levels over four lanes, one G function each, was tried here and is slower: 35 us per
-// tree top against 20: the per-lane message schedule becomes divergent constant-memory reads and the state rotation shuffles
-// cost more than the shorter dependency chain saves.)
+// chain of ten dependent hashes either way, which is what bounds it). Levels of 2^8 and 2^9 nodes are a thread a node, bound by
+// issue; from 2^7 down a node is a quad's (channel.cuh), and the last four levels one warp's, without a CTA barrier. When `chan` is
+// given, that warp goes on with the channel step of a FRI layer (mix the root, draw the folding challenge), which would otherwise
+// be a launch of its own. With a thread a node throughout and the channel step on one thread: 19 us
+// for ten levels and the step, now 16 us.
 __global__ void __launch_bounds__(512) merkle_top_kernel(MerkleTopArgs a, int top_log, int m31_out, uint32_t* __restrict__ chan,
                                                          uint32_t* __restrict__ alpha_out, uint32_t* __restrict__ root_copy) {
-    __shared__ uint32_t sh[2][512][8];
-    for (int lg = top_log - 1; lg >= 0; lg--) {
-        const bool from_global = lg == top_log - 1;
-        const uint32_t(*src)[8] = sh[(lg + 1) & 1];
-        for (uint32_t i = threadIdx.x; i < (1u << lg); i += blockDim.x) {
+    __shared__ alignas(16) uint32_t sh[2][256 * PAIR_WORDS];
+    __shared__ ChanSm ch;
+    __shared__ uint32_t felt[4];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, l = tid & 3u;
+    chan_make_schedule(ch, (int)tid, (int)blockDim.x);
+    if (chan && tid < 32) {
+        ch.msg[tid] = tid < 8 ? chan[tid] : 0u;
+        if (tid == 0) ch.n_draws = chan[8];
+    }
+    int lg = top_log - 1;
+    if (top_log <= 8)
+        for (uint32_t i = tid; i < (2u << top_log); i += blockDim.x)
+            *reinterpret_cast<uint4*>(&sh[(lg + 1) & 1][(i >> 2) * PAIR_WORDS + (i & 3u) * 4u]) = reinterpret_cast<const uint4*>(a.layer[top_log])[i];
+    __syncthreads();
+#pragma unroll 1
+    for (; lg >= 8; lg--) {
+        if (tid < (1u << lg)) {
             uint32_t h[8], m[16];
             blake2s_init(h);
-            if (from_global) {
-                const uint4* p = reinterpret_cast<const uint4*>(a.layer[lg + 1] + 16 * (size_t)i);
-                uint4 x0 = p[0], x1 = p[1], x2 = p[2], x3 = p[3];
-                m[0] = x0.x; m[1] = x0.y; m[2] = x0.z; m[3] = x0.w; m[4] = x1.x; m[5] = x1.y; m[6] = x1.z; m[7] = x1.w;
-                m[8] = x2.x; m[9] = x2.y; m[10] = x2.z; m[11] = x2.w; m[12] = x3.x; m[13] = x3.y; m[14] = x3.z; m[15] = x3.w;
-            } else {
+            const uint4* p = lg == top_log - 1 ? reinterpret_cast<const uint4*>(a.layer[lg + 1] + 16 * (size_t)tid)
+                                               : reinterpret_cast<const uint4*>(&sh[(lg + 1) & 1][tid * PAIR_WORDS]);
 #pragma unroll
-                for (int k = 0; k < 8; k++) { m[k] = src[2 * i][k]; m[8 + k] = src[2 * i + 1][k]; }
+            for (int q = 0; q < 4; q++) {
+                const uint4 x = p[q];
+                m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
             }
             blake2s_compress(h, m, 64u, true);
 #pragma unroll
-            for (int k = 0; k < 8; k++) { h[k] = m31_out ? reduce_word_m31(h[k]) : h[k]; sh[lg & 1][i][k] = h[k]; }
-            store_hash(a.layer[lg], i, h, false);
+            for (int k = 0; k < 8; k++) h[k] = m31_out ? reduce_word_m31(h[k]) : h[k];
+            uint4* const o = reinterpret_cast<uint4*>(&sh[lg & 1][pair_at(tid)]);
+            o[0] = make_uint4(h[0], h[1], h[2], h[3]);
+            o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            store_hash(a.layer[lg], tid, h, false);
         }
         __syncthreads();
     }
-    if (chan && threadIdx.x == 0) channel_mix_root_draw(chan, sh[0][0], alpha_out, root_copy);
+    const QuadConst k;
+    const uint32_t node = tid >> 2;
+#pragma unroll 1
+    for (; lg >= 0; lg--) {
+        if (lg <= 3 && warp) return;
+        if (warp * 8u < (1u << lg)) {
+            uint2 h = b2s_compress_quad(make_uint2(k.h0, k.h1), &sh[(lg + 1) & 1][node * PAIR_WORDS], ch.sched, k, 64u, 0xffffffffu);
+            if (m31_out) h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
+            if (node < (1u << lg)) {
+                uint32_t *const o = &sh[lg & 1][pair_at(node)], *const g = a.layer[lg] + 8 * (size_t)node;
+                o[l] = g[l] = h.x;
+                o[4 + l] = g[4 + l] = h.y;
+            }
+        }
+        if (lg >= 4) __syncthreads();
+        else __syncwarp();
+    }
+    if (!chan) return;
+    if (lane < 8) {
+        const uint32_t w = sh[0][lane];
+        ch.msg[8 + lane] = w;
+        if (root_copy) root_copy[lane] = w;
+    }
+    chan_step(ch, 8, 1, felt);
+    if (lane < 8) chan[lane] = ch.msg[lane];
+    if (lane == 8) chan[8] = ch.n_draws;
+    if (lane < 4) alpha_out[lane] = felt[lane];
 }
 
 // Grind: thread `lo` tests nonce (hi << 32) | lo; the minimum passing lo is kept.
@@ -317,9 +397,23 @@ int zkb_merkle_layer(zkb_ctx* ctx, int log_size, const uint32_t* prev, const uin
         int rc = stage_ptrs(ctx, (const void* const*)cols, ncols, &d_cols);
         if (rc) return rc;
     }
-    size_t n = (size_t)1 << log_size;
-    unsigned threads = n < 256 ? 32 : 256;
-    unsigned blocks = (unsigned)((n + threads - 1) / threads);
+    const size_t n = (size_t)1 << log_size;
+    if (log_size <= QUAD_MAX_LOG) {
+        // up to here there are no more than two warps of quads a scheduler, so a node's latency is what counts
+        ProfScope prof(ctx, ncols >= 64 ? "merkle_layer_quad_kernel(>=64 columns)" : "merkle_layer_quad_kernel");
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)((4 * n + QUAD_THREADS - 1) / QUAD_THREADS));
+        cfg.blockDim = dim3(QUAD_THREADS);
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = ctx->prof_on ? 0 : 1;
+        ZKB_CUDA(ctx, cudaLaunchKernelEx(&cfg, merkle_layer_quad_kernel, log_size, prev, (const uint32_t* const*)d_cols, ncols, m31_out, out));
+        return ZKB_OK;
+    }
+    const unsigned threads = 256, blocks = (unsigned)(n / threads);
     if (ncols >= 64 && n <= ((size_t)1 << 17)) {
         // few rows (at 2^17 there are still only seven warps per scheduler), a long chain of compressions each: the next
         // block's loads are in flight during a compression; small CTAs so that the few rows spread over all SMs
@@ -396,7 +490,7 @@ static int merkle_top_impl(zkb_ctx* ctx, int top_log, const uint32_t* top_layer,
     }
     DeviceGuard g(ctx);
     ProfScope prof(ctx, "merkle_top_kernel");
-    merkle_top_kernel<<<1, top_log >= 10 ? 512 : (top_log >= 6 ? 1 << (top_log - 1) : 32), 0, ctx->stream>>>(a, top_log, m31_out, d_chan, d_alpha,
+    merkle_top_kernel<<<1, top_log >= 8 ? 512 : std::max(2 << top_log, 32), 0, ctx->stream>>>(a, top_log, m31_out, d_chan, d_alpha,
                                                                                                               d_root_copy);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;

@@ -29,13 +29,20 @@ struct alignas(16) ChanSm {
 };
 
 // Any set of threads; a barrier (of the warp or the CTA, whichever called) must follow.
-__device__ __forceinline__ void chan_make_schedule(ChanSm& s, int thread, int n_threads) {
+__device__ __forceinline__ void quad_make_schedule(uint32_t* sched, int thread, int n_threads) {
     for (int t = thread; t < 40; t += n_threads) {
         const uint8_t* sg = c_chan_sigma[t >> 2];
         const int l = t & 3, g = (l + 3) & 3;  // in the diagonal step the lane that keeps v[4 + l] runs diagonal l - 1
-        s.sched[t] = 4u * sg[2 * l] | (4u * sg[2 * l + 1]) << 8 | (4u * sg[8 + 2 * g]) << 16 | (4u * sg[9 + 2 * g]) << 24;
+        sched[t] = 4u * sg[2 * l] | (4u * sg[2 * l + 1]) << 8 | (4u * sg[8 + 2 * g]) << 16 | (4u * sg[9 + 2 * g]) << 24;
     }
 }
+
+__device__ __forceinline__ void chan_make_schedule(ChanSm& s, int thread, int n_threads) { quad_make_schedule(s.sched, thread, n_threads); }
+
+// Where quads keep hashes of a tree level in shared memory: a pair of siblings is the 16-word message of their parent, the pairs are 20
+// words apart (16-byte aligned, and the eight quads of a warp read their messages from different banks).
+constexpr int PAIR_WORDS = 20;
+__device__ __forceinline__ uint32_t pair_at(uint32_t node) { return (node >> 1) * PAIR_WORDS + (node & 1u) * 8u; }
 
 // What a lane of the quad knows of the hash for good: its words of the initial state, and masks for the byte count and the last flag.
 struct QuadConst {

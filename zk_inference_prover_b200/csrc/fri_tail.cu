@@ -3,7 +3,9 @@
 // (mix, draw the folding challenge) and the fold.
 //
 // What bounds it: dependency depth. A layer of 2^l values is a chain of l + 1 tree levels and two channel compressions, each some
-// 0.9 us; at 2^10 values the leaves and the level above them are another 9 us of one SM's hashing. As launches (fold and leaves, tree
+// 0.9 us; at 2^10 values the leaves and the level above them are another 9 us of one SM's hashing. Levels of up to 2^7 hashes are
+// four lanes a hash, and the last four and the channel one warp's, without CTA barriers (as in merkle_top_kernel): nine layers
+// from 2^9 values 95 -> 85 us. As launches (fold and leaves, tree
 // top with channel step) a layer also paid two launches, the gaps around them and a dozen allocations for its arrays: a ten-column
 // proof of 2^8 rows spent 190 us of device time in them and as much on the host. Layers stay in shared memory; what the decommitment
 // reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs.
@@ -15,19 +17,20 @@ namespace zk {
 
 constexpr int TAIL_THREADS = 512;
 constexpr size_t TAIL_N = (size_t)1 << FRI_TAIL_LOG;
+static_assert(TAIL_N / 2 <= TAIL_THREADS, "a layer folds to at most a value a thread");
 
 __device__ __forceinline__ uint32_t bitrev_bits(uint32_t i, int bits) { return bits ? __brev(i) >> (32 - bits) : 0u; }
 
-// Dynamic shared memory: two layers of values and two of hashes, word by word ([word][node]: a node's two children then lie next to
-// each other in every word's row, two-way bank conflicts instead of sixteen).
-constexpr size_t TAIL_SMEM = (2 * 4 + 2 * 8) * TAIL_N * 4;
+// Dynamic shared memory: two layers of values, word by word, and two of hashes, pair by pair (pair_at).
+constexpr size_t TAIL_PAIRS = TAIL_N / 2 * PAIR_WORDS, TAIL_SMEM = (2 * 4 * TAIL_N + 2 * TAIL_PAIRS) * 4;
 
 __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_constant__ FriTailArgs a, const uint32_t* __restrict__ itw) {
     extern __shared__ uint32_t dyn[];
     __shared__ ChanSm ch;
     __shared__ uint32_t alpha_w[4];
-    uint32_t *ev = dyn, *ev_next = ev + 4 * TAIL_N, *const ha = ev_next + 4 * TAIL_N, *const hb = ha + 8 * TAIL_N;
-    const int tid = threadIdx.x, lane = tid & 31;
+    uint32_t *ev = dyn, *ev_next = ev + 4 * TAIL_N, *const ha = ev_next + 4 * TAIL_N, *const hb = ha + TAIL_PAIRS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = tid & 3, quad = tid >> 2;
+    const QuadConst qc;
     chan_make_schedule(ch, tid, TAIL_THREADS);
     if (tid < 32) ch.msg[tid] = tid < 8 ? (a.chan ? a.chan[tid] : a.digest[tid]) : 0u;
     if (tid == 0) ch.n_draws = a.chan ? a.chan[8] : a.n_draws;
@@ -39,36 +42,62 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
     for (int k = 0; k < a.n_layers; k++) {
         const int log = a.first_log - k;
         uint32_t *cur = ha, *below = hb;
+        // the fold's twiddle (a layer folds to at most a value a thread) is on its way while the tree is hashed
+        const uint32_t half = 1u << (log - 1), mine = (uint32_t)tid < half ? (uint32_t)tid : 0u;
+        uint32_t t, ix;
+        if (a.circle && k == 0) half_coset_point(itw, log, mine, ix, t);
+        else t = itw[half + mine];  // T_log^-1 starts at 2^(log - 1)
         // leaves (level log) and nodes: one loop, so that the code of the hash is there once
 #pragma unroll 1
         for (int lv = log; lv >= 0; lv--) {
             uint32_t* const out = a.tree[k] + ((size_t)8 << lv);
             const bool leaf = lv == log;
-            for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
-                uint32_t h[8], m[16];
-                blake2s_init(h);
+            if (lv >= 8) {
+                for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
+                    uint32_t h[8], m[16];
+                    blake2s_init(h);
 #pragma unroll
-                for (int w = 0; w < 16; w++)
-                    m[w] = leaf ? (w < 4 ? ev[w * TAIL_N + i] : 0u) : below[(w & 7) * TAIL_N + 2 * i + (w >> 3)];
-                blake2s_compress(h, m, leaf ? 16u : 64u, true);
+                    for (int q = 0; q < 4; q++) {
+                        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                        if (!leaf) x = *reinterpret_cast<const uint4*>(below + PAIR_WORDS * i + 4 * q);
+                        else if (q == 0) x = make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
+                        m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
+                    }
+                    blake2s_compress(h, m, leaf ? 16u : 64u, true);
 #pragma unroll
-                for (int w = 0; w < 8; w++) {
-                    h[w] = reduce_word_m31(h[w]);
-                    cur[w * TAIL_N + i] = h[w];
+                    for (int w = 0; w < 8; w++) h[w] = reduce_word_m31(h[w]);
+                    const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
+                    uint4 *const c = reinterpret_cast<uint4*>(cur + pair_at(i)), *const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
+                    c[0] = o[0] = lo;
+                    c[1] = o[1] = hi;
                 }
-                uint4* const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
-                o[0] = make_uint4(h[0], h[1], h[2], h[3]);
-                o[1] = make_uint4(h[4], h[5], h[6], h[7]);
+            } else if (8 * warp < (1 << lv)) {
+                uint32_t* const m = below + PAIR_WORDS * quad;
+                const bool live = quad < (1 << lv);
+                if (leaf) {
+                    const uint32_t i = live ? quad : 0;
+                    *reinterpret_cast<uint4*>(m + 4 * l) = l ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
+                    __syncwarp();
+                }
+                uint2 h = b2s_compress_quad(make_uint2(qc.h0, qc.h1), m, ch.sched, qc, leaf ? 16u : 64u, 0xffffffffu);
+                h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
+                if (live) {
+                    uint32_t *const c = cur + pair_at(quad), *const o = out + 8 * quad;
+                    c[l] = o[l] = h.x;
+                    c[4 + l] = o[4 + l] = h.y;
+                }
             }
-            uint32_t* const t = cur;
+            uint32_t* const swap = cur;
             cur = below;
-            below = t;
-            __syncthreads();
+            below = swap;
+            if (lv >= 4) __syncthreads();
+            else if (warp == 0) __syncwarp();
+            else break;
         }
-        // the root is in below[.][0]: mix it in, draw the challenge
+        // the root is in warp 0's below[0, 8): mix it in, draw the challenge
         if (tid < 32) {
             if (lane < 8) {
-                const uint32_t w = below[lane * TAIL_N];
+                const uint32_t w = below[lane];
                 ch.msg[8 + lane] = w;
                 a.out[FRI_TAIL_ROOTS + 8 * k + lane] = w;
             }
@@ -76,12 +105,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
         }
         __syncthreads();
         const qm31 alpha{{alpha_w[0], alpha_w[1], alpha_w[2], alpha_w[3]}};
-        const uint32_t half = 1u << (log - 1);
         const size_t stride = log - 1 < 2 ? 4 : half;
-        for (uint32_t i = tid; i < half; i += TAIL_THREADS) {
-            uint32_t t, ix;
-            if (a.circle && k == 0) half_coset_point(itw, log, i, ix, t);
-            else t = itw[half + i];  // T_log^-1 starts at 2^(log - 1)
+        if ((uint32_t)tid < half) {
+            const uint32_t i = (uint32_t)tid;
             qm31 x, y;
 #pragma unroll
             for (int c = 0; c < 4; c++) { x.c[c] = ev[c * TAIL_N + 2 * i]; y.c[c] = ev[c * TAIL_N + 2 * i + 1]; }
@@ -89,9 +115,9 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
 #pragma unroll
             for (int c = 0; c < 4; c++) { ev_next[c * TAIL_N + i] = r.c[c]; a.evals[k][c * stride + i] = r.c[c]; }
         }
-        uint32_t* const t = ev;
+        uint32_t* const swap = ev;
         ev = ev_next;
-        ev_next = t;
+        ev_next = swap;
         __syncthreads();
     }
     if (tid >= 32) return;

@@ -250,7 +250,12 @@ struct MerkleProver {
         return mp;
     }
     Hash root(const Device& d) const {
-        if (!have_root) { root_cache = B200Backend::batch_at(d, layers[0], {0})[0]; have_root = true; }
+        if (!have_root) {
+            const uint32_t* h = nullptr;
+            d.check(zk::read_small(d.ctx(), layers[0].ptr(), 8, &h));
+            std::copy(h, h + 8, root_cache.begin());
+            have_root = true;
+        }
         return root_cache;
     }
     mutable Hash root_cache{};
