@@ -52,6 +52,10 @@ struct zkb_ctx {
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t fences[64] = {nullptr};
     cudaEvent_t copy_gate = nullptr;  // orders the copy stream after allocations made on `stream`
+    // side_stream.hpp: the stream that is not `stream` (the side one, or the main one between side_begin and side_end)
+    cudaStream_t other_stream = nullptr;
+    cudaEvent_t side_events[2] = {nullptr, nullptr};  // fork, join
+    bool on_side = false, side_pending = false;
     cudaStream_t peer_streams[4] = {nullptr, nullptr, nullptr, nullptr};  // device-to-device copies to other GPUs, side by side
     // Optional per-kernel timeline (zkb_profile_*): pairs of events around selected launches.
     bool prof_on = false;

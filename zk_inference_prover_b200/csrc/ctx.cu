@@ -1,9 +1,11 @@
 // Context lifetime, device memory helpers, the twiddle tower and small utilities.
 #include <cstdarg>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
+#include "side_stream.hpp"
 #include "gather_blocks.hpp"
 
 namespace zk {
@@ -21,6 +23,7 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...) {
 // The ring is used from its start again: earlier slots may still be in flight, so drain the stream, and forget what they held.
 static int stage_wrap(zkb_ctx* ctx) {
     ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (ctx->other_stream) ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->other_stream));
     ctx->ring_pos = 0;
     for (auto& t : ctx->staged) t.n = 0;
     return ZKB_OK;
@@ -72,10 +75,45 @@ int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out) {
     void** d = ctx->d_ring + ctx->ring_pos;
     memcpy(h, h_ptrs, (size_t)n * sizeof(void*));
     ZKB_CUDA(ctx, cudaMemcpyAsync(d, h, (size_t)n * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->staged[ctx->staged_next] = {ctx->ring_pos, (size_t)n};
-    ctx->staged_next = (ctx->staged_next + 1) % zkb_ctx::STAGED_TABLES;
+    if (!ctx->on_side) {  // a table copied on the side is not there yet for the work outside
+        ctx->staged[ctx->staged_next] = {ctx->ring_pos, (size_t)n};
+        ctx->staged_next = (ctx->staged_next + 1) % zkb_ctx::STAGED_TABLES;
+    }
     ctx->ring_pos += (size_t)n;
     *out = d;
+    return ZKB_OK;
+}
+
+int side_begin(zkb_ctx* ctx) {
+    DeviceGuard g(ctx);
+    if (!ctx->other_stream) {
+        // what goes there is long and narrow (chains of a few warps): its CTAs are placed before those of the wide work beside it
+        int low = 0, high = 0;
+        ZKB_CUDA(ctx, cudaDeviceGetStreamPriorityRange(&low, &high));
+        ZKB_CUDA(ctx, cudaStreamCreateWithPriority(&ctx->other_stream, cudaStreamNonBlocking, high));
+        for (auto& e : ctx->side_events) ZKB_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    ZKB_CUDA(ctx, cudaEventRecord(ctx->side_events[0], ctx->stream));
+    ZKB_CUDA(ctx, cudaStreamWaitEvent(ctx->other_stream, ctx->side_events[0], 0));
+    std::swap(ctx->stream, ctx->other_stream);
+    ctx->on_side = true;
+    return ZKB_OK;
+}
+int side_end(zkb_ctx* ctx) {
+    if (!ctx->on_side) return ZKB_OK;
+    DeviceGuard g(ctx);
+    std::swap(ctx->stream, ctx->other_stream);
+    ctx->on_side = false;
+    ctx->side_pending = true;
+    ZKB_CUDA(ctx, cudaEventRecord(ctx->side_events[1], ctx->other_stream));
+    return ZKB_OK;
+}
+int side_join(zkb_ctx* ctx) {
+    if (int rc = side_end(ctx)) return rc;
+    if (!ctx->side_pending) return ZKB_OK;
+    DeviceGuard g(ctx);
+    ctx->side_pending = false;
+    ZKB_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->side_events[1], 0));
     return ZKB_OK;
 }
 
@@ -262,6 +300,9 @@ int zkb_destroy(zkb_ctx* ctx) {
         if (ctx->fences[i]) cudaEventDestroy(ctx->fences[i]);
     if (ctx->copy_gate) cudaEventDestroy(ctx->copy_gate);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    for (auto e : ctx->side_events)
+        if (e) cudaEventDestroy(e);
+    if (ctx->other_stream) cudaStreamDestroy(ctx->other_stream);
     for (auto st : ctx->peer_streams)
         if (st) cudaStreamDestroy(st);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -275,6 +316,7 @@ int zkb_sync(zkb_ctx* ctx) {
     if (!ctx) return ZKB_EINVAL;
     DeviceGuard g(ctx);
     if (ctx->copy_stream) ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->copy_stream));
+    if (ctx->other_stream) ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->other_stream));
     // a kernel whose bounded wait ran out has set the error word; report it here, where the host waits anyway
     ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->h_small + SMALL_WORDS, ctx->dev_err, 4, cudaMemcpyDeviceToHost, ctx->stream));
     ZKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -653,6 +695,12 @@ int zkb_secure_powers(zkb_ctx* ctx, const uint32_t h_felt[4], size_t n, uint32_t
 }  // extern "C"
 
 namespace zk {
+
+int stage_table(zkb_ctx* ctx, const uint32_t* const* ptrs, int n) {
+    DeviceGuard g(ctx);
+    void** d = nullptr;
+    return stage_ptrs(ctx, (const void* const*)ptrs, n, &d);
+}
 
 int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t total_words, const uint32_t* const* word_addrs, size_t n_words,
                 const uint32_t* const* hash_addrs, size_t n_hashes, uint32_t* h_out) {

@@ -7,6 +7,9 @@ struct zkb_ctx;
 
 namespace zk {
 
+// A table of device addresses on the device, where operators that are given the same table soon after find it.
+int stage_table(zkb_ctx* ctx, const uint32_t* const* ptrs, int n);
+
 // out[out_off + i * ncols + c] = cols[c][idx[i]]: the rows idx[0..nidx) of ncols device columns, row-major.
 // cols and idx are host arrays (cols holds device pointers).
 struct GatherBlock {

@@ -26,6 +26,7 @@
 #include "../fri_tail.hpp"
 #include "../gather_blocks.hpp"
 #include "channel.hpp"
+#include "../side_stream.hpp"
 #include "../quot_lines.hpp"
 
 // Records a message on the context (defined with the context, ctx.cu).
@@ -179,6 +180,13 @@ struct MerkleProver {
     // the committed columns of each layer (device addresses, in commitment order), kept for the decommitment: sorting tens
     // of thousands of columns by size a second time costs milliseconds
     std::vector<std::vector<const uint32_t*>> layer_col_ptrs;
+
+    // The column tables of a tree's layers, copied to the device (commit and the decommitment find them there).
+    static void stage_tables(const Device& d, const std::vector<const BaseColumn*>& columns) {
+        std::vector<std::vector<const uint32_t*>> of(33);
+        for (auto c : columns) of[c->log_size()].push_back(c->ptr());
+        for (auto& p : of) if (!p.empty()) d.check(zk::stage_table(d.ctx(), p.data(), (int)p.size()));
+    }
 
     // `leaves`, when given, is the already hashed largest layer (see zkb_merkle_leaves_partial).
     // `chan_step`, when given, is a FRI layer's channel step (channel state, challenge slot, root copy; device addresses) to run
@@ -782,13 +790,39 @@ struct CommitmentSchemeProver {
         }
     }
 
+    // Trees committed one after the other with nothing drawn in between: their roots are read and mixed in at the end (mix_roots). One of
+    // them is hashed beside the work on the next ones, the first whose short layers hold so many columns that they are a chain of
+    // compressions on a handful of warps (20,000 columns of 2^11 rows: a millisecond and a half with most of the chip idle).
+    struct SeveralTrees {
+        bool more = true;  // trees come after this one
+        bool forked = false;
+    };
+    static bool narrow(const std::vector<BaseColumn>& evals) {
+        size_t cols[14] = {0}, chain = 0;
+        for (auto& e : evals)
+            if (e.log_size() <= 13) cols[e.log_size()]++;
+        for (size_t c : cols) chain += c / 16;
+        return chain >= 64;  // some 55 us; a fork and its join cost a few
+    }
+    void mix_roots(Channel& ch) {
+        zk::side_join(d.ctx());
+        GatherPlan plan;
+        for (auto& t : trees) plan.add_hash(t.commitment.layers[0].ptr());
+        if (!trees.empty()) plan.execute(d);
+        for (size_t k = 0; k < trees.size(); k++) {
+            trees[k].commitment.root_cache = plan.hash_at(k);
+            trees[k].commitment.have_root = true;
+            ch.mix_root(trees[k].commitment.root_cache);
+        }
+    }
+
     // TreeBuilder::extend_evals + commit (pcs/mod.rs:429-464) -> CommitmentTreeProver::new (:481-537).
     // `columns` are consumed: interpolated in place, per size group.
     // `fence_of` (optional, one entry per column) names the copy fence after which a column's values have
     // arrived from the host; columns are then interpolated and extended fence by fence, while later
     // columns are still in flight.
     void commit_evals(std::vector<BaseColumn> columns, Channel& ch, const std::vector<int>* fence_of = nullptr,
-                      BaseColumn* slab = nullptr, bool are_coeffs = false) {
+                      BaseColumn* slab = nullptr, bool are_coeffs = false, SeveralTrees* several = nullptr) {
         CommitmentTreeProver t;
         if (slab) t.coeff_slab = std::move(*slab);
         std::map<uint32_t, std::vector<size_t>> by_log;
@@ -864,8 +898,16 @@ struct CommitmentSchemeProver {
         std::vector<const BaseColumn*> refs;
         refs.reserve(t.evals.size());
         for (auto& e : t.evals) refs.push_back(&e);
-        t.commitment = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr);
-        ch.mix_root(t.commitment.root(d));
+        if (several && several->more && !several->forked && narrow(t.evals)) {
+            several->forked = true;
+            MerkleProver::stage_tables(d, refs);  // so that the decommitment finds them
+            d.check(zk::side_begin(d.ctx()));
+            t.commitment = MerkleProver::commit(d, refs);
+            d.check(zk::side_end(d.ctx()));
+        } else {
+            t.commitment = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr);
+        }
+        if (!several) ch.mix_root(t.commitment.root(d));
         mark(2);
         trees.push_back(std::move(t));
     }
@@ -1900,13 +1942,19 @@ static void commit_input_trees(Device& dev, zkb_ctx* ctx, CommitmentSchemeProver
                                uint32_t* const* d_cols, const uint32_t* const* h_cols, const uint32_t* col_logs, int total) {
         int flat = 0;
         if (d_cols) {
+            // (with phases to be timed one tree after the other: their marks are on one stream)
+            const bool together = n_trees > 1 && !prover.phase_ms;
+            CommitmentSchemeProver::SeveralTrees several;
+            zk::SideScope scope(ctx);
             for (int t = 0; t < n_trees; t++) {
+                several.more = t + 1 < n_trees;
                 std::vector<BaseColumn> columns;
                 columns.reserve((size_t)tree_ncols[t]);
                 for (int c = 0; c < tree_ncols[t]; c++, flat++)
                     columns.push_back(BaseColumn::view(dev, d_cols[flat], (size_t)1 << col_logs[flat]));
-                prover.commit_evals(std::move(columns), ch);
+                prover.commit_evals(std::move(columns), ch, nullptr, nullptr, false, together ? &several : nullptr);
             }
+            if (together) prover.mix_roots(ch);
         } else {
             // Host columns: every copy of every tree is enqueued on the copy stream first, with a fence
             // after each ~1/32 of the bytes, so that the transfer runs at link speed from start to end
