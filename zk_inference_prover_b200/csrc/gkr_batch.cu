@@ -163,6 +163,8 @@ struct GkrStepSm {
 };
 
 __device__ __noinline__ qm31 qmul(qm31 a, qm31 b) { return qm31_mul(a, b); }
+struct qm31_pair { qm31 a, b; };
+__device__ __noinline__ qm31_pair product_pair(qm31 a0, qm31 a1, qm31 b0, qm31 b1) { return {qm31_mul(a0, a1), qm31_mul(b0, b1)}; }
 __device__ __noinline__ void chan_step_b(ChanSm& s, int n, int draws, qm31* felts) { chan_step(s, n, draws, reinterpret_cast<uint32_t*>(felts)); }
 __device__ __forceinline__ qm31 shflb(qm31 v, int src) {
     qm31 r;
@@ -178,11 +180,14 @@ __device__ __forceinline__ qm31 warp_sum_m(qm31 v) {
 }
 
 // By one warp; sm.ch's schedule is made and its message holds the digest. st: the state, wherever it is (its accumulators are not
-// touched); s0, s2: lane g's group's sums; out: the round's record.
-__device__ void batch_step(GkrStepSm& sm, GkrStepState& st, const GkrStepConst& rc, qm31 s0, qm31 s2, uint32_t* out) {
+// touched); s0, s2: lane g's group's sums; out: the round's record. drawn() is called as soon as the challenge is in sm.r, before
+// what the next step needs of it is worked out.
+template <class Drawn>
+__device__ __forceinline__ void batch_step(GkrStepSm& sm, GkrStepState& st, const GkrStepConst& rc, qm31 s0, qm31 s2, uint32_t* out, Drawn drawn) {
     const int lane = threadIdx.x & 31, c4 = lane & 3;
     const qm31 corr = st.corr[lane];
-    const qm31 S0 = warp_sum_m(qmul(s0, corr)), S2 = warp_sum_m(qmul(s2, corr));
+    const qm31_pair w = product_pair(s0, corr, s2, corr);
+    const qm31 S0 = warp_sum_m(w.a), S2 = warp_sum_m(w.b);
     // coefficient c4: lanes 0-3 of the first sum, 4-7 of the second, 8-11 of the claim
     const int q = lane >> 2;
     const qm31 p = qmul(q == 0 ? S0 : q == 1 ? S2 : st.claim, q == 0 ? rc.A[c4] : q == 1 ? rc.B[c4] : rc.L1[c4]);
@@ -191,12 +196,13 @@ __device__ void batch_step(GkrStepSm& sm, GkrStepState& st, const GkrStepConst& 
     if (lane < 4) {
         sm.coef[lane] = act;
         stqb(sm.ch.msg + 8, lane, c);
-        stqb(out, lane, c);
     }
-    if (lane == 3 && qm31_is_zero(c)) st.degenerate = 1u;
-    if (lane == 0) out[16] = 4u;
     chan_step_b(sm.ch, 16, 1, &sm.r);
     const qm31 r = sm.r, y = rc.y, one = qm31_one();
+    drawn();
+    if (lane < 4) stqb(out, lane, c);
+    if (lane == 3 && qm31_is_zero(c)) st.degenerate = 1u;
+    if (lane == 0) out[16] = 4u;
     // (c3 r + c2) r^2 + (c1 r + c0), eq(r, y)
     qm31 x = r, z = r;
     if (lane == 0) x = sm.coef[3];
@@ -325,8 +331,6 @@ struct alignas(16) GkrSync {  // zero at launch
     uint32_t slot[GKR_LAYER_MAX_ROUNDS + 1][4];  // the challenge the table folds with; the top bit of a word: it is there
 };
 
-struct qm31_pair { qm31 a, b; };
-__device__ __noinline__ qm31_pair product_pair(qm31 a0, qm31 a1, qm31 b0, qm31 b1) { return {qm31_mul(a0, a1), qm31_mul(b0, b1)}; }
 
 // The sums of `v` over the warp's lanes with even and odd `which` go to the group's accumulator; lanes that do not add hold `adds` false.
 __device__ __forceinline__ void add_quad_terms(uint32_t (*acc)[16], bool adds, int which, uint32_t group, qm31 v) {
@@ -391,13 +395,14 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
         const GkrBatchItem* const items = items_base + tb.first;
         const bool step = t < n_rounds;
         // what does not depend on the challenge: the first piece's item, in the small form its factor of the sums
-        uint32_t chunk = blockIdx.x;
+        // CTA 0 has the last piece, its first warp the end of it: often there is nothing there, and that warp comes late (below).
+        uint32_t chunk = tb.form == 0 ? blockIdx.x : tb.ctas - 1u - blockIdx.x;
         GkrBatchItem it{};
         uint32_t term = 0;
         bool live = false;
         qm31 ea = qm31_zero();
         auto look_up = [&]() {  // forms 1 and 2
-            const uint32_t flat = chunk * GKR_THREADS + tid;
+            const uint32_t flat = chunk * GKR_THREADS + ((tid + GKR_THREADS - 32) & (GKR_THREADS - 1));
             const uint32_t at = tb.form == 1 ? flat >> 2 : flat;
             term = at & ((1u << tb.terms_log) - 1);
             live = (at >> tb.terms_log) < tb.n_items;
@@ -415,7 +420,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
             __syncthreads();
             if (gave_up) return;
         }
-        const qm31 r = lead ? s.challenge : r_sh;
+        const qm31 r = lead ? sm.r : r_sh;
         if (tb.form == 1) {
             for (;;) {
                 const int q = lane & 3;
@@ -472,7 +477,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
             }
         }
         __syncthreads();
-        if (tb.ctas > 1) {
+        if (!lead) {
             if (step) {
                 uint32_t* const h = &sums[tid >> 3][2 * (tid & 7)];
                 const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
@@ -483,10 +488,11 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
                 __threadfence_system();
             }
             __syncthreads();
-            if (!lead) {
-                if (tid == 0) { __threadfence(); atomicAdd(&sync->count[t], 1u); }
-                continue;
-            }
+            if (tid == 0) { __threadfence(); atomicAdd(&sync->count[t], 1u); }
+            continue;
+        }
+        // CTA 0 from here on; its own sums stay where they are
+        if (tb.ctas > 1) {
             if (tid == 0) {
                 uint32_t n = ld_acquire(&sync->count[t]);
                 for (uint32_t spin = 0; n != tb.ctas - 1 && spin < SPIN_LIMIT; spin++) n = ld_acquire(&sync->count[t]);
@@ -495,37 +501,33 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
             __syncthreads();
             if (gave_up) return;
         }
-        // CTA 0 from here on
         if (!step) break;
+        auto challenge_drawn = [] { asm volatile("bar.sync 1, %0;" ::"n"(GKR_THREADS) : "memory"); };
         if (warp == 0) {
-            qm31 v[2];
+            unsigned long long a[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) a[c] = tb.ctas > 1 ? __ldcg(&st->acc[t & 1][lane][c]) : 0ull;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                a[c] += (unsigned long long)sums[lane][2 * c] + ((unsigned long long)sums[lane][2 * c + 1] << 16);
+                sums[lane][2 * c] = sums[lane][2 * c + 1] = 0u;
+            }
+            batch_step(sm, s, consts[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, challenge_drawn);
             if (tb.ctas > 1) {
-                unsigned long long a[8];
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    a[c] = __ldcg(&st->acc[t & 1][lane][c]);
-                    st->acc[t & 1][lane][c] = 0ull;  // for the round after the next
-                }
-                v[0] = acc_value(a);
-                v[1] = acc_value(a + 4);
-            } else {
-#pragma unroll
-                for (int z = 0; z < 2; z++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) v[z].c[c] = m31_reduce64(sums[lane][8 * z + 2 * c] + ((uint64_t)sums[lane][8 * z + 2 * c + 1] << 16));
-#pragma unroll
-                for (int c = 0; c < 16; c++) sums[lane][c] = 0u;
+                for (int c = 0; c < 8; c++) st->acc[t & 1][lane][c] = 0ull;  // for the round after the next: seen with the next challenge
             }
-            batch_step(sm, s, consts[t], v[0], v[1], records + GKR_LAYER_OUT_WORDS * (size_t)t);
-            if (tb.later > 1) {
-                __threadfence();
-                __syncwarp();
-                if (lane < 4) *reinterpret_cast<volatile uint32_t*>(&sync->slot[t + 1][lane]) = s.challenge.c[lane] | 0x80000000u;
-            }
+        } else {
+            // Warp 1 sends the challenge. Its fence stands behind the barrier that put everybody's folded layers behind this point,
+            // and takes as long as a third of a compression: warp 0 hashes meanwhile, and the CTA goes on with the next table
+            // while it works out what the step after that needs.
+            if (warp == 1 && tb.later > 1) __threadfence();
+            challenge_drawn();
+            if (warp == 1 && lane < 4 && tb.later > 1) *reinterpret_cast<volatile uint32_t*>(&sync->slot[t + 1][lane]) = sm.r.c[lane] | 0x80000000u;
         }
-        __syncthreads();
     }
     if (!lead) return;
+    __syncthreads();
     if (warp == 0) batch_step_close(sm, st, s.degenerate, lane);
     __threadfence();
     __syncthreads();
@@ -802,8 +804,8 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
             while (tb.run_log < 3 && tb.terms_log - 8 > tb.run_log && (terms >> (8 + tb.run_log + 1)) >= 4 * (size_t)grid) tb.run_log++;
         const size_t chunks = tb.form == 0 && tb.terms_log >= 8 ? terms >> (8 + tb.run_log) : ((tb.form == 1 ? 4 * terms : terms) + GKR_THREADS - 1) / GKR_THREADS;
         tb.chunks = (uint32_t)chunks;
-        // Up to two pieces stay in CTA 0: sending the sums and the challenge round costs as much as another pass.
-        tb.ctas = chunks <= 2 ? 1u : (uint32_t)std::min<size_t>(chunks, grid);
+        // (sending the sums and the challenge round costs less than a second piece in CTA 0: 6,400 cycles against 8,500)
+        tb.ctas = (uint32_t)std::min<size_t>(chunks, grid);
         tb.later = later;
         later = std::max(later, tb.ctas);
     }

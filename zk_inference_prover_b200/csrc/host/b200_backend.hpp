@@ -153,21 +153,21 @@ struct Layer {
     }
 };
 
-// f(begin, end, chunk) over [0, n) on up to four host threads (the caller's among them; chunk = 0 ... 3) when every thread
+// f(begin, end, chunk) over [0, n) on up to MAX host threads (the caller's among them; chunk = 0 ... MAX - 1) when every thread
 // gets at least `min_per_thread` items: the per-column arithmetic of a proof over tens of thousands of columns (powers of
 // the random coefficient, line coefficients) is independent per item. An exception of any chunk is rethrown on the caller's
 // thread after all chunks have ended.
-template <class F>
+template <int MAX = 4, class F>
 inline void parallel_chunks(size_t n, size_t min_per_thread, F f) {
     size_t nt = min_per_thread ? n / min_per_thread : 1;
-    if (nt > 4) nt = 4;
+    if (nt > MAX) nt = MAX;
     if (nt <= 1) { f((size_t)0, n, (size_t)0); return; }
     const size_t per = (n + nt - 1) / nt;
-    std::exception_ptr failed[4];
+    std::exception_ptr failed[MAX];
     auto run = [&](size_t t) {
         try { f(t * per < n ? t * per : n, (t + 1) * per < n ? (t + 1) * per : n, t); } catch (...) { failed[t] = std::current_exception(); }
     };
-    std::thread th[3];
+    std::thread th[MAX - 1];
     for (size_t t = 1; t < nt; t++) th[t - 1] = std::thread(run, t);
     run(0);
     for (size_t t = 1; t < nt; t++) th[t - 1].join();

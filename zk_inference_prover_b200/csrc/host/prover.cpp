@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <iterator>
 #include <chrono>
+#include <future>
 #include <map>
 #include <memory>
 #include <numeric>
@@ -697,7 +698,7 @@ struct PcsProof {
             }
             n += k;
         }
-        // Long runs (the queried values of a wide tree's layers; their source outlives the sink) are copied at the end, by four threads
+        // Long runs (the queried values of a wide tree's layers; their source outlives the sink) are copied at the end, by eight threads
         // in equal parts: one core moves some 6 GB/s into fresh pages, and the proof of a composed segment is 26 MB and more.
         static constexpr size_t LONG_RUN = 4096;
         struct Run { uint32_t* dst; const uint32_t* src; size_t n; };
@@ -705,7 +706,7 @@ struct PcsProof {
         void finish() {
             size_t total = 0;
             for (auto& r : runs) total += r.n;
-            parallel_chunks(total, (size_t)1 << 17, [&](size_t lo, size_t hi, size_t) {
+            parallel_chunks<8>(total, (size_t)1 << 17, [&](size_t lo, size_t hi, size_t) {
                 size_t at = 0;
                 for (auto& r : runs) {
                     const size_t a = std::max(lo, at), b = std::min(hi, at + r.n);
@@ -1088,6 +1089,10 @@ struct CommitmentSchemeProver {
                     place_of[s] = (uint32_t)(g.first + g.count);
                     polys[g.first + g.count++] = t.coeffs[c].ptr();
                 }
+        // The quotient plan of tens of thousands of samples takes as long as hashing them does: it is made on another thread meanwhile.
+        const bool aside = n_samples >= 8192;
+        std::future<Numerators> planned;
+        if (aside) planned = std::async(std::launch::async, [&] { return plan_numerators(sp, place_of, lifting_log); });
         hc.reset(new HostClock("pcs.sample.eval"));
         BaseColumn d_values(d, 4 * n_samples);
         for (auto& g : groups) {
@@ -1097,9 +1102,16 @@ struct CommitmentSchemeProver {
             d.check(zk::eval_at_point_device(d.ctx(), polys.data() + g.first, (int)g.count, (int)g.log, pt, d_values.ptr() + 4 * g.first));
         }
         hc.reset(new HostClock("pcs.quot.plan"));
-        Numerators nu = plan_numerators(sp, place_of, lifting_log);
-        d.check(zk::numerator_stage(d.ctx(), nu.entries, nu.batches, nu.lines));
-        BaseColumn lines_block = BaseColumn::adopt(d, nu.lines.block);
+        Numerators nu;
+        BaseColumn lines_block;
+        auto stage = [&] {
+            d.check(zk::numerator_stage(d.ctx(), nu.entries, nu.batches, nu.lines));
+            lines_block = BaseColumn::adopt(d, nu.lines.block);
+        };
+        if (!aside) {
+            nu = plan_numerators(sp, place_of, lifting_log);
+            stage();
+        }
         hc.reset(new HostClock("pcs.sample.read"));
         qm31* h_values = reinterpret_cast<qm31*>(GatherPlan::arena(4 * n_samples));
         if (n_samples) d.check(zkb_d2h(d.ctx(), h_values, d_values.ptr(), 16 * n_samples));
@@ -1110,6 +1122,10 @@ struct CommitmentSchemeProver {
         hc.reset(new HostClock("pcs.quot.mix"));
         ch.mix_felts(values);
         qm31 random_coeff = ch.draw_secure_felt();
+        if (aside) {
+            nu = planned.get();
+            stage();
+        }
         hc.reset(new HostClock("pcs.quot.compute"));
         SecureColumnByCoords quotients = compute_fri_quotients(nu, random_coeff, h_values, d_values.ptr(), lifting_log);
         proof.sampled_values.first = std::move(sp.first);
