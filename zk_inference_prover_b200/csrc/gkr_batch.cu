@@ -848,7 +848,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         waiting = qm31_add(waiting, entering[j + 1]);  // all that enter after round j
         GkrStepConst& c = consts[j];
         const GkrRoundConst& rc = rounds[j];
-        const uint32_t half_pow = m31_inv(1u << (j + 1 < 31 ? j + 1 : 0));  // 2^-(j + 1)
+        const uint32_t half_pow = j + 1 < 31 ? 1u << (31 - (j + 1)) : 1u;  // 2^-(j + 1), as 2^31 = 1
         for (int t = 0; t < 4; t++) {
             c.A[t] = qm31_mul(q4(rc.e0a), qm31_sub(q4(rc.L[0][t]), q4(rc.L[1][t])));
             c.B[t] = qm31_mul(q4(rc.e2a), q4(rc.L[2][t]));
