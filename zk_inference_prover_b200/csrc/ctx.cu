@@ -185,8 +185,11 @@ __global__ void gather_words_kernel(const uint32_t* const* __restrict__ addrs, s
 }
 
 // Everything a read plan asks for (gather_plan). Thread t < n_cells: cell t of the blocks (their out_off ascending, found by
-// bisection); then a word per word address; then eight words per hash address.
-struct PlanBlock { const uint32_t* const* cols; uint32_t ncols, idx, out_off, pad; };  // idx: where its row indices start
+// bisection); then a word per word address; then eight words per hash address. The plan begins with the word addresses.
+struct PlanBlock { const uint32_t* const* cols; uint32_t ncols, idx, out_off, here; };  // idx: where its row indices start; here: cols is an offset into the plan
+__host__ __device__ __forceinline__ const uint32_t* const* plan_cols(const PlanBlock& b, const void* plan) {
+    return b.here ? reinterpret_cast<const uint32_t* const*>(static_cast<const char*>(plan) + reinterpret_cast<uintptr_t>(b.cols)) : b.cols;
+}
 __global__ void __launch_bounds__(256) gather_plan_kernel(const PlanBlock* __restrict__ blocks, int n_blocks, const uint32_t* __restrict__ idx, uint32_t n_cells,
                                                           const uint32_t* const* __restrict__ words, uint32_t n_words,
                                                           const uint32_t* const* __restrict__ hashes, uint32_t n_hashes, uint32_t* __restrict__ out) {
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(256) gather_plan_kernel(const PlanBlock* __res
         }
         const PlanBlock b = blocks[lo];
         const uint32_t e = t - b.out_off;
-        out[t] = b.cols[e % b.ncols][idx[b.idx + e / b.ncols]];
+        out[t] = plan_cols(b, words)[e % b.ncols][idx[b.idx + e / b.ncols]];
         return;
     }
     if (t < n_cells + n_words) {
@@ -707,22 +710,36 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
     const size_t results = total_words + n_words + 8 * n_hashes;
     if (results == 0) return ZKB_OK;
     DeviceGuard g(ctx);
-    size_t n_idx = 0;
-    for (int b = 0; b < n_blocks; b++) n_idx += (size_t)blocks[b].nidx;
-    // [word addresses | hash addresses | block descriptors | row indices]
-    const size_t at_hash = 8 * n_words, at_blocks = at_hash + 8 * n_hashes, at_idx = at_blocks + sizeof(PlanBlock) * (size_t)n_blocks;
+    // The column tables of short blocks (a FRI layer's four columns) travel in the plan; those of a tree's columns are the ones its
+    // commitment staged.
+    constexpr int OWN_COLS = 64;
+    size_t n_idx = 0, n_own = 0;
+    for (int b = 0; b < n_blocks; b++) {
+        n_idx += (size_t)blocks[b].nidx;
+        if (blocks[b].ncols <= OWN_COLS) n_own += (size_t)blocks[b].ncols;
+    }
+    // [word addresses | hash addresses | short tables | block descriptors | row indices]
+    const size_t at_hash = 8 * n_words, at_own = at_hash + 8 * n_hashes, at_blocks = at_own + 8 * n_own, at_idx = at_blocks + sizeof(PlanBlock) * (size_t)n_blocks;
     std::vector<unsigned char> blob(at_idx + 4 * n_idx);
     if (n_words) memcpy(blob.data(), word_addrs, 8 * n_words);
     if (n_hashes) memcpy(blob.data() + at_hash, hash_addrs, 8 * n_hashes);
     PlanBlock* pb = reinterpret_cast<PlanBlock*>(blob.data() + at_blocks);
     uint32_t* pi = reinterpret_cast<uint32_t*>(blob.data() + at_idx);
-    size_t first_idx = 0;
+    size_t first_idx = 0, own = 0;
     for (int b = 0; b < n_blocks; b++) {
-        void** cols;
-        if (int rc = stage_ptrs(ctx, (const void* const*)blocks[b].cols, blocks[b].ncols, &cols)) return rc;
-        if (blocks[b].nidx) memcpy(pi + first_idx, blocks[b].idx, 4 * (size_t)blocks[b].nidx);
-        pb[b] = {(const uint32_t* const*)cols, (uint32_t)blocks[b].ncols, (uint32_t)first_idx, (uint32_t)blocks[b].out_off, 0u};
-        first_idx += (size_t)blocks[b].nidx;
+        const GatherBlock& g = blocks[b];
+        void** cols = nullptr;
+        const bool here = g.ncols <= OWN_COLS;
+        if (here) {  // as an offset into the plan
+            memcpy(blob.data() + at_own + 8 * own, g.cols, 8 * (size_t)g.ncols);
+            cols = reinterpret_cast<void**>(at_own + 8 * own);
+            own += (size_t)g.ncols;
+        } else if (int rc = stage_ptrs(ctx, (const void* const*)g.cols, g.ncols, &cols)) {
+            return rc;
+        }
+        if (g.nidx) memcpy(pi + first_idx, g.idx, 4 * (size_t)g.nidx);
+        pb[b] = {(const uint32_t* const*)cols, (uint32_t)g.ncols, (uint32_t)first_idx, (uint32_t)g.out_off, here ? 1u : 0u};
+        first_idx += (size_t)g.nidx;
     }
     // a plan too long for the staging ring brings its own memory
     unsigned char *d_blob = nullptr, *d_own = nullptr;
@@ -748,7 +765,7 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
             for (int b = 0; b < n_blocks; b++) {
                 const size_t cells = (size_t)blocks[b].ncols * blocks[b].nidx;
                 if (cells)
-                    gather_multi_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, ctx->stream>>>(pb[b].cols, blocks[b].ncols, d_idx + pb[b].idx, blocks[b].nidx,
+                    gather_multi_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, ctx->stream>>>(plan_cols(pb[b], d_blob), blocks[b].ncols, d_idx + pb[b].idx, blocks[b].nidx,
                                                                                                   d_out + blocks[b].out_off);
             }
         }

@@ -8,6 +8,7 @@
 // the canonic circle domain of log size L uses the y of point i of Coset::half_odds(L-1).
 #include "blake2s.cuh"
 #include "common.cuh"
+#include "fri_tail.hpp"
 
 namespace zk {
 
@@ -123,8 +124,9 @@ __global__ void __launch_bounds__(256) fold_line_kernel4(Secure4 out, Secure4C i
     for (int k = 0; k < 4; k++) reinterpret_cast<uint4*>(out.c[k])[i4] = make_uint4(r[0].c[k], r[1].c[k], r[2].c[k], r[3].c[k]);
 }
 
+// (fresh: what is in dst counts as zero and is not read)
 __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
-                                                           const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw) {
+                                                           const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw, int fresh) {
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
     const size_t half = (size_t)1 << (log_n_src - 1);
@@ -135,13 +137,15 @@ __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C
     for (int e = 0; e < 4; e++) half_coset_point(itw, log_n_src, (uint32_t)(4 * i4 + e), ix, t[e]);
     qm31 f[4];
     fold_quad(src, i4, t, alpha, f);
-    uint4 d[4];
+    if (!fresh) {
+        uint4 d[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) d[k] = reinterpret_cast<const uint4*>(dst.c[k])[i4];
+        for (int k = 0; k < 4; k++) d[k] = reinterpret_cast<const uint4*>(dst.c[k])[i4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const qm31 de{{(&d[0].x)[e], (&d[1].x)[e], (&d[2].x)[e], (&d[3].x)[e]}};
-        f[e] = qm31_add(qm31_mul(de, alpha_sq), f[e]);
+        for (int e = 0; e < 4; e++) {
+            const qm31 de{{(&d[0].x)[e], (&d[1].x)[e], (&d[2].x)[e], (&d[3].x)[e]}};
+            f[e] = qm31_add(qm31_mul(de, alpha_sq), f[e]);
+        }
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) reinterpret_cast<uint4*>(dst.c[k])[i4] = make_uint4(f[0].c[k], f[1].c[k], f[2].c[k], f[3].c[k]);
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C
 
 __global__ void __launch_bounds__(256) fold_circle_kernel2(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
                                                            const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
-                                                           uint32_t* __restrict__ leaves) {
+                                                           uint32_t* __restrict__ leaves, int fresh) {
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
     const size_t half = (size_t)1 << (log_n_src - 1);
@@ -160,13 +164,17 @@ __global__ void __launch_bounds__(256) fold_circle_kernel2(Secure4 dst, Secure4C
     half_coset_point(itw, log_n_src, (uint32_t)(2 * i2 + 1), ix, iy1);
     qm31 f0, f1;
     fold_pair2(src, i2, iy0, iy1, alpha, f0, f1);
-    qm31 d0, d1;
+    qm31 r0 = f0, r1 = f1;
+    if (!fresh) {
+        qm31 d0, d1;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        uint2 v = reinterpret_cast<const uint2*>(dst.c[k])[i2];
-        d0.c[k] = v.x; d1.c[k] = v.y;
+        for (int k = 0; k < 4; k++) {
+            uint2 v = reinterpret_cast<const uint2*>(dst.c[k])[i2];
+            d0.c[k] = v.x; d1.c[k] = v.y;
+        }
+        r0 = qm31_add(qm31_mul(d0, alpha_sq), f0);
+        r1 = qm31_add(qm31_mul(d1, alpha_sq), f1);
     }
-    const qm31 r0 = qm31_add(qm31_mul(d0, alpha_sq), f0), r1 = qm31_add(qm31_mul(d1, alpha_sq), f1);
 #pragma unroll
     for (int k = 0; k < 4; k++) reinterpret_cast<uint2*>(dst.c[k])[i2] = make_uint2(r0.c[k], r1.c[k]);
     if (leaves) { store_leaf(leaves, 2 * i2, r0); store_leaf(leaves, 2 * i2 + 1, r1); }
@@ -192,7 +200,7 @@ __global__ void fold_small_kernel(Secure4 out, Secure4C in, int n_out, qm31 alph
 
 __global__ void __launch_bounds__(256) fold_circle_kernel(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
                                                           const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
-                                                          uint32_t* __restrict__ leaves = nullptr) {
+                                                          uint32_t* __restrict__ leaves, int fresh) {
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
     size_t half = (size_t)1 << (log_n_src - 1);
@@ -201,8 +209,8 @@ __global__ void __launch_bounds__(256) fold_circle_kernel(Secure4 dst, Secure4C 
     uint32_t ix, iy;
     half_coset_point(itw, log_n_src, (uint32_t)i, ix, iy);
     qm31 f = fold_pair(src, i, iy, alpha);
-    qm31 d{{dst.c[0][i], dst.c[1][i], dst.c[2][i], dst.c[3][i]}};
-    qm31 r = qm31_add(qm31_mul(d, alpha_sq), f);
+    qm31 r = f;
+    if (!fresh) r = qm31_add(qm31_mul(qm31{{dst.c[0][i], dst.c[1][i], dst.c[2][i], dst.c[3][i]}}, alpha_sq), f);
 #pragma unroll
     for (int k = 0; k < 4; k++) dst.c[k][i] = r.c[k];
     if (leaves) store_leaf(leaves, i, r);
@@ -259,7 +267,7 @@ static int fold_line_impl(zkb_ctx* ctx, uint32_t* const out[4], const uint32_t* 
 }
 
 static int fold_circle_impl(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t* const src[4], int log_n_src,
-                            const uint32_t* h_alpha, const uint32_t* d_alpha, uint32_t* leaves = nullptr) {
+                            const uint32_t* h_alpha, const uint32_t* d_alpha, uint32_t* leaves = nullptr, int fresh = 0) {
     if (!ctx) return ZKB_EINVAL;
     ZKB_CHECK_ARG(ctx, dst && src && (h_alpha || d_alpha) && log_n_src >= 1 && log_n_src <= ctx->max_log);
     ZKB_CHECK_ARG(ctx, ((uintptr_t)d_alpha & 15) == 0);
@@ -283,7 +291,7 @@ static int fold_circle_impl(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t
             cpoint p = host_point(((1u << (29 - hl)) + (j << (31 - hl))) & 0x7fffffffu);
             it[i] = m31_inv(p.y);
         }
-        fold_small_kernel<<<1, 32, 0, ctx->stream>>>(o, s, 1 << hl, alpha, d_alpha, 1, it[0], it[1], it[2], it[3]);
+        fold_small_kernel<<<1, 32, 0, ctx->stream>>>(o, s, 1 << hl, alpha, d_alpha, fresh ? 0 : 1, it[0], it[1], it[2], it[3]);
         ZKB_LAUNCH_CHECK(ctx);
         return ZKB_OK;
     }
@@ -294,13 +302,17 @@ static int fold_circle_impl(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t
     bool quad = wide && log_n_src >= 5 && !leaves;
     for (int k = 0; k < 4; k++) quad = quad && ((uintptr_t)dst[k] & 15) == 0;
     if (quad)
-        fold_circle_kernel4<<<(unsigned)((half / 4 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw);
+        fold_circle_kernel4<<<(unsigned)((half / 4 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, fresh);
     else if (wide)
-        fold_circle_kernel2<<<(unsigned)((half / 2 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves);
+        fold_circle_kernel2<<<(unsigned)((half / 2 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves, fresh);
     else
-        fold_circle_kernel<<<(unsigned)((half + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves);
+        fold_circle_kernel<<<(unsigned)((half + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves, fresh);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
+}
+
+int zk::fold_circle_fresh(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t* const src[4], int log_n_src, const uint32_t* d_alpha, uint32_t* leaves) {
+    return fold_circle_impl(ctx, dst, src, log_n_src, nullptr, d_alpha, leaves, 1);
 }
 
 extern "C" {

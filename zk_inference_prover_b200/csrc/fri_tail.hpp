@@ -36,6 +36,8 @@ inline size_t fri_tail_stride(int log) { return log < 2 ? 4 : (size_t)1 << log; 
 int fri_tail(zkb_ctx* ctx, const FriTailArgs& args);
 // The first nonces (several times 2^pow_bits of them) tested against the digest at prefixed; the smallest that passes goes to *best.
 int grind_first(zkb_ctx* ctx, const uint32_t* prefixed, int pow_bits, uint32_t* best);
+// zkb_fold_circle_into_line_dalpha (leaves: ..._leaves, or null) into a line that counts as zero: it is neither cleared first nor read.
+int fold_circle_fresh(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t* const src[4], int log_n_src, const uint32_t* d_alpha, uint32_t* leaves);
 // A few words to device memory through the staging ring: no synchronisation.
 int upload_small(zkb_ctx* ctx, uint32_t* dst, const uint32_t* h, size_t words);
 // `words` of device memory to the context's page-locked buffer and a synchronisation; *h is valid until the next such read.

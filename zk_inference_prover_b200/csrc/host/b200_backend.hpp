@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../../include/zkb200.h"
+#include "../fri_tail.hpp"
 #include "../m31.cuh"
 
 namespace b200 {
@@ -271,16 +272,13 @@ struct B200Backend {
         d.check(zkb_fold_line_dalpha(d.ctx(), o.data(), i.data(), (int)log_n, d_alpha));
         return out;
     }
+    // into a new line (what is in dst counts as zero)
     static void fold_circle_into_line(const Device& d, SecureColumnByCoords& dst, const SecureColumnByCoords& src, const uint32_t* d_alpha,
                                       HashColumn* leaves = nullptr) {
         auto o = dst.ptrs();
         auto i = src.cptrs();
-        if (leaves) {
-            *leaves = HashColumn(d, 8 * dst.len());
-            d.check(zkb_fold_circle_into_line_dalpha_leaves(d.ctx(), o.data(), i.data(), (int)src.columns[0].log_size(), d_alpha, leaves->ptr()));
-        } else {
-            d.check(zkb_fold_circle_into_line_dalpha(d.ctx(), o.data(), i.data(), (int)src.columns[0].log_size(), d_alpha));
-        }
+        if (leaves) *leaves = HashColumn(d, 8 * dst.len());
+        d.check(zk::fold_circle_fresh(d.ctx(), o.data(), i.data(), (int)src.columns[0].log_size(), d_alpha, leaves ? leaves->ptr() : nullptr));
     }
     // fold_line that also hashes the folded layer's Merkle leaves (the layer's four columns are its coordinates)
     static SecureColumnByCoords fold_line(const Device& d, const SecureColumnByCoords& eval, const uint32_t* d_alpha, HashColumn& leaves) {

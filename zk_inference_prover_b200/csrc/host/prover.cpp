@@ -450,7 +450,7 @@ struct FriProver {
                 for (int k = 0; k < 8; k++) st[k] = ch.digest()[k];
                 st[8] = ch.n_draws();
                 d.check(zk::upload_small(d.ctx(), chan, st, 16));
-                layer = SecureColumnByCoords(d, (size_t)1 << inner_log, true);
+                layer = SecureColumnByCoords(d, (size_t)1 << inner_log);
                 bool stepped = false;
                 MerkleProver::ChanStep step0{chan, alphas, roots};
                 fp.first_tree = MerkleProver::commit(d, column.refs(), nullptr, &step0, &stepped);
@@ -2266,6 +2266,14 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
         std::vector<std::vector<std::vector<int32_t>>> offsets((size_t)n_components);
         std::vector<std::vector<std::vector<CirclePointQ>>> points((size_t)n_trees + 1);
         for (int t = 0; t < n_trees; t++) points[t].resize((size_t)tree_ncols[t]);
+        std::map<int32_t, CirclePointQ> at_offset;  // a handful of distinct ones over all columns
+        auto mask_point = [&](int32_t off) {
+            auto it = at_offset.find(off);
+            if (it != at_offset.end()) return it->second;
+            // trace_step.mul_signed(off): the point of index off * 2^(31 - max_log_degree_bound) in the circle group
+            const cpoint st = host_circle_point(((uint32_t)off << (31 - max_log_degree_bound)) & 0x7fffffffu);
+            return at_offset[off] = point_add(oods, {qm31_from_m31(st.x), qm31_from_m31(st.y)});
+        };
         for (int k = 0; k < n_components; k++) {
             const zkb_air_program* prog = comps[k].prog;
             offsets[k].resize(prog->n_cols);
@@ -2276,11 +2284,7 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
                 }
             for (int t = 0; t < n_trees; t++)
                 for (uint32_t q = 0; q < cols_of(k, t); q++)
-                    for (int32_t off : offsets[k][prog->tree_base[t] + q]) {
-                        // trace_step.mul_signed(off): the point of index off * 2^(31 - max_log_degree_bound) in the circle group
-                        cpoint st = host_circle_point(((uint32_t)off << (31 - max_log_degree_bound)) & 0x7fffffffu);
-                        points[t][first[k][t] + q].push_back(point_add(oods, {qm31_from_m31(st.x), qm31_from_m31(st.y)}));
-                    }
+                    for (int32_t off : offsets[k][prog->tree_base[t] + q]) points[t][first[k][t] + q].push_back(mask_point(off));
         }
         points.back().assign(8, {oods});
         SamplePoints flat_points;
