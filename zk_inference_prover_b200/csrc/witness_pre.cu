@@ -202,7 +202,7 @@ struct RsArgs {
     RsMult m_pow, m_norm, m_val, m_frac, m_smul;
     const RsMult* m_un;
     uint32_t* counts;
-    uint32_t n_norm, n_smul, n_val, log_rows, live, n_groups, n_leaves, n_slots, n_levels, kmax, out_w, teams, flush_every;
+    uint32_t n_norm, n_smul, n_val, log_rows, live, n_groups, n_leaves, n_slots, n_levels, kmax, out_w, teams, flush_every, leaves_by_four, outs_by_four;
 };
 constexpr uint32_t RS_DMAX = 12, RS_UMIN = 260, RS_BIAS = 134, RS_POW_ROWS = RS_DMAX + 1 + RS_UMIN;
 
@@ -295,9 +295,18 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
     for (uint32_t g = 0; g < a.n_groups; g++) {
         const RsGroup gr = a.groups[g];
         for (uint32_t k0 = t * RS_LEAVES; k0 < gr.n; k0 += lanes * RS_LEAVES) {
+            // What is in natural row order lies n_leaves words apart from lane to lane: a sector a lane and access, whatever its width.
+            const size_t at = leaf0 + gr.flat + k0;
+            const bool four = a.leaves_by_four && k0 + RS_LEAVES <= gr.n;
             uint32_t pats[RS_LEAVES];
+            if (four) {
+                const uint4 p = live ? __ldg(reinterpret_cast<const uint4*>(a.wit + at)) : make_uint4(0u, 0u, 0u, 0u);
+                pats[0] = p.x; pats[1] = p.y; pats[2] = p.z; pats[3] = p.w;
+            } else {
 #pragma unroll
-            for (uint32_t u = 0; u < RS_LEAVES; u++) pats[u] = live && k0 + u < gr.n ? __ldg(a.wit + leaf0 + gr.flat + k0 + u) : 0u;
+                for (uint32_t u = 0; u < RS_LEAVES; u++) pats[u] = live && k0 + u < gr.n ? __ldg(a.wit + at + u) : 0u;
+            }
+            int2 held = make_int2(0, 0);
 #pragma unroll
             for (uint32_t u = 0; u < RS_LEAVES; u++) {
                 const uint32_t k = k0 + u, pat = pats[u];
@@ -305,13 +314,15 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
                 // a bf16 pattern as (sm, ef); both zeros, infinities and NaNs collapse to (0, 0)
                 const uint32_t e = (pat >> 7) & 0xffu;
                 const bool finite = e != 0 && e != 0xffu;
-                const long long mag = 128 + (pat & 0x7fu);
-                const long long sm = finite ? ((pat >> 15) & 1u ? -mag : mag) : 0;
+                const int mag = 128 + (int)(pat & 0x7fu);
+                const int sm = finite ? ((pat >> 15) & 1u ? -mag : mag) : 0;
                 const uint32_t ef = finite ? e : 0u;
                 const uint32_t b = gr.leaf_col + k * gr.width;
-                column<EVEN>(a, b)[i] = field_of(sm);
+                column<EVEN>(a, b)[i] = sm < 0 ? (uint32_t)(sm + (int)P) : (uint32_t)sm;
                 column<EVEN>(a, b + 1)[i] = ef;
-                reinterpret_cast<int2*>(a.in_nat)[leaf0 + gr.flat + k] = make_int2((int)sm, (int)ef);  // natural row order
+                if (!four) reinterpret_cast<int2*>(a.in_nat)[at + u] = make_int2(sm, (int)ef);
+                else if (u & 1) reinterpret_cast<int4*>(a.in_nat)[(at + u) >> 1] = make_int4(held.x, held.y, sm, (int)ef);
+                else held = make_int2(sm, (int)ef);
                 const uint32_t v = value_index(sm, ef);
                 if (gr.un == 0) { lookup<RS_VAL_LOG>(val_counts, a.m_val, v, off); continue; }
                 uint32_t *c2 = column<EVEN>(a, b + 2), *c3 = column<EVEN>(a, b + 3);
@@ -411,14 +422,30 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
 
     // what the bindings and the next component read, in natural row order
     if (in_range)
-    for (uint32_t k = t; k < a.out_w; k += lanes) {
-        const RsSlot sl = a.slots[a.out_slot[k]];
-        const long long sm = signed_of(column<EVEN>(a, sl.o_sm)[i]), e = signed_of(column<EVEN>(a, sl.o_ef)[i]);
-        const uint32_t ef = (uint32_t)(e < 0 ? 0 : e > 0xfe ? 0xfe : e);
-        uint32_t pat = 0;
-        if (sm != 0) pat = ((sm < 0 ? 1u << 15 : 0u) | (ef << 7) | (uint32_t)((sm < 0 ? -sm : sm) - 128)) & 0xffffu;
-        a.out_pat[(size_t)j * a.out_w + k] = pat;
-        reinterpret_cast<int2*>(a.out_nat)[(size_t)j * a.out_w + k] = make_int2((int)sm, (int)e);
+    for (uint32_t k0 = t * 4; k0 < a.out_w; k0 += lanes * 4) {
+        uint32_t pats[4];
+        int2 held = make_int2(0, 0);
+        const size_t at = (size_t)j * a.out_w + k0;
+        const bool four = a.outs_by_four;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            if (k0 + u >= a.out_w) break;
+            const RsSlot sl = a.slots[a.out_slot[k0 + u]];
+            const long long sm = signed_of(column<EVEN>(a, sl.o_sm)[i]), e = signed_of(column<EVEN>(a, sl.o_ef)[i]);
+            const uint32_t ef = (uint32_t)(e < 0 ? 0 : e > 0xfe ? 0xfe : e);
+            uint32_t pat = 0;
+            if (sm != 0) pat = ((sm < 0 ? 1u << 15 : 0u) | (ef << 7) | (uint32_t)((sm < 0 ? -sm : sm) - 128)) & 0xffffu;
+            pats[u] = pat;
+            if (!four) {
+                a.out_pat[at + u] = pat;
+                reinterpret_cast<int2*>(a.out_nat)[at + u] = make_int2((int)sm, (int)e);
+            } else if (u & 1) {
+                reinterpret_cast<int4*>(a.out_nat)[(at + u) >> 1] = make_int4(held.x, held.y, (int)sm, (int)e);
+            } else {
+                held = make_int2((int)sm, (int)e);
+            }
+        }
+        if (four) *reinterpret_cast<uint4*>(a.out_pat + at) = make_uint4(pats[0], pats[1], pats[2], pats[3]);
     }
     team_sync();  // the next rows' cells are other memory, but a warp must not be two passes ahead of its team's barrier
     if (++since_flush == a.flush_every) {
@@ -629,6 +656,11 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     a.n_norm = tables->norm3 ? tables->n_norm : 0; a.n_smul = tables->smul3 ? tables->n_smul : 0; a.n_val = tables->n_val;
     a.log_rows = log_rows; a.live = live_rows; a.n_groups = p.n_groups; a.n_leaves = (uint32_t)n_leaves; a.n_slots = p.n_slots;
     a.kmax = p.kmax; a.out_w = p.out_w; a.n_levels = n_levels;
+    // four leaves, or outputs, of a row in one access where all of them start on 16 bytes
+    bool by_four = n_leaves % 4 == 0 && ((uintptr_t)wit & 15) == 0 && ((uintptr_t)in_nat & 15) == 0;
+    for (uint32_t g = 0; g < p.n_groups; g++) by_four = by_four && p.groups[g].flat % 4 == 0;
+    a.leaves_by_four = by_four;
+    a.outs_by_four = p.out_w % 4 == 0 && ((uintptr_t)out_pat & 15) == 0 && ((uintptr_t)out_nat & 15) == 0;
     // evenly spaced columns need no table
     bool even = true;
     a.col0 = cols[0];
