@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
     quad_make_schedule(sched, threadIdx.x, QUAD_THREADS);
     // A tree built layer by layer is a chain of launches of a microsecond or two: the next one may start now (programmatic dependent
     // launch) and wait here for this grid to end.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    let_next_start();
+    follow_previous();
     addresses(0);
     uint4 cur = make_uint4(0u, 0u, 0u, 0u);
     if (prev) cur = reinterpret_cast<const uint4*>(prev)[4 * (size_t)i + l];
@@ -242,6 +242,7 @@ struct MerkleLevelsArgs {
 __global__ void __launch_bounds__(256) merkle_levels_kernel(MerkleLevelsArgs a, int levels, int m31_out) {
     __shared__ uint32_t sh[2][256][8];
     const size_t cta = blockIdx.x;
+    follow_previous();
     uint32_t h[8], m[16];
     {
         blake2s_init(h);
@@ -307,6 +308,8 @@ __global__ void __launch_bounds__(512) merkle_top_kernel(MerkleTopArgs a, int to
     __shared__ uint32_t felt[4];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, l = tid & 3u;
     chan_make_schedule(ch, (int)tid, (int)blockDim.x);
+    let_next_start();  // one CTA: whatever comes next finds room
+    follow_previous();
     if (chan && tid < 32) {
         ch.msg[tid] = tid < 8 ? chan[tid] : 0u;
         if (tid == 0) ch.n_draws = chan[8];
@@ -401,16 +404,8 @@ int zkb_merkle_layer(zkb_ctx* ctx, int log_size, const uint32_t* prev, const uin
     if (log_size <= QUAD_MAX_LOG) {
         // up to here there are no more than two warps of quads a scheduler, so a node's latency is what counts
         ProfScope prof(ctx, ncols >= 64 ? "merkle_layer_quad_kernel(>=64 columns)" : "merkle_layer_quad_kernel");
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)((4 * n + QUAD_THREADS - 1) / QUAD_THREADS));
-        cfg.blockDim = dim3(QUAD_THREADS);
-        cfg.stream = ctx->stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = ctx->prof_on ? 0 : 1;
-        ZKB_CUDA(ctx, cudaLaunchKernelEx(&cfg, merkle_layer_quad_kernel, log_size, prev, (const uint32_t* const*)d_cols, ncols, m31_out, out));
+        ZKB_CUDA(ctx, launch_following(ctx, merkle_layer_quad_kernel, (unsigned)((4 * n + QUAD_THREADS - 1) / QUAD_THREADS), QUAD_THREADS, log_size, prev,
+                                       (const uint32_t* const*)d_cols, ncols, m31_out, out));
         return ZKB_OK;
     }
     const unsigned threads = 256, blocks = (unsigned)(n / threads);
@@ -461,8 +456,7 @@ int zkb_merkle_levels(zkb_ctx* ctx, int child_log, const uint32_t* children, int
     }
     DeviceGuard g(ctx);
     ProfScope prof(ctx, "merkle_levels_kernel");
-    merkle_levels_kernel<<<1u << (child_log - 9), 256, 0, ctx->stream>>>(a, levels, m31_out);
-    ZKB_LAUNCH_CHECK(ctx);
+    ZKB_CUDA(ctx, launch_following(ctx, merkle_levels_kernel, 1u << (child_log - 9), 256u, a, levels, m31_out));
     return ZKB_OK;
 }
 
@@ -490,9 +484,7 @@ static int merkle_top_impl(zkb_ctx* ctx, int top_log, const uint32_t* top_layer,
     }
     DeviceGuard g(ctx);
     ProfScope prof(ctx, "merkle_top_kernel");
-    merkle_top_kernel<<<1, top_log >= 8 ? 512 : std::max(2 << top_log, 32), 0, ctx->stream>>>(a, top_log, m31_out, d_chan, d_alpha,
-                                                                                                              d_root_copy);
-    ZKB_LAUNCH_CHECK(ctx);
+    ZKB_CUDA(ctx, launch_following(ctx, merkle_top_kernel, 1u, top_log >= 8 ? 512u : (unsigned)std::max(2 << top_log, 32), a, top_log, m31_out, d_chan, d_alpha, d_root_copy));
     return ZKB_OK;
 }
 

@@ -89,6 +89,28 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...);
 #define ZKB_LAUNCH_CHECK(ctx) ZKB_CUDA(ctx, cudaGetLastError())
 
 // RAII guard making the context's device current for the duration of a call.
+// Launches a kernel that may start while the one before it on the stream is still running (programmatic dependent launch): it calls
+// follow_previous() before it touches anything an earlier launch writes or reads. For chains of launches of a few microseconds.
+// With a timeline being recorded, plainly.
+template <class... P, class... A>
+cudaError_t launch_following(zkb_ctx* ctx, void (*kernel)(P...), unsigned grid, unsigned block, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->prof_on ? 0 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void follow_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next launch may start: its CTAs take what room this grid leaves and wait in follow_previous.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 struct DeviceGuard {
     int prev = -1, dev;
     bool ok = true;

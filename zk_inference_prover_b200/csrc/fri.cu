@@ -83,6 +83,7 @@ __device__ __forceinline__ void fold_pair2(const Secure4C& in, size_t i2, uint32
 __global__ void __launch_bounds__(256) fold_line_kernel2(Secure4 out, Secure4C in, int log_n, qm31 alpha,
                                                          const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
                                                          uint32_t* __restrict__ leaves) {
+    follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const size_t half = (size_t)1 << (log_n - 1);
     const size_t i2 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -112,6 +113,7 @@ __device__ __forceinline__ void fold_quad(const Secure4C& in, size_t i4, const u
 
 __global__ void __launch_bounds__(256) fold_line_kernel4(Secure4 out, Secure4C in, int log_n, qm31 alpha,
                                                          const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw) {
+    follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const size_t half = (size_t)1 << (log_n - 1);
     const size_t i4 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(256) fold_line_kernel4(Secure4 out, Secure4C i
 // (fresh: what is in dst counts as zero and is not read)
 __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
                                                            const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw, int fresh) {
+    follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
     const size_t half = (size_t)1 << (log_n_src - 1);
@@ -154,6 +157,7 @@ __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C
 __global__ void __launch_bounds__(256) fold_circle_kernel2(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
                                                            const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
                                                            uint32_t* __restrict__ leaves, int fresh) {
+    follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
     const size_t half = (size_t)1 << (log_n_src - 1);
@@ -254,14 +258,16 @@ static int fold_line_impl(zkb_ctx* ctx, uint32_t* const out[4], const uint32_t* 
     bool wide = log_n >= 3;
     for (int k = 0; k < 4; k++) wide = wide && ((uintptr_t)in[k] & 15) == 0 && ((uintptr_t)out[k] & 7) == 0;
     ProfScope prof(ctx, "fold_line_kernel");
+    cudaError_t e = cudaSuccess;
     bool quad = wide && log_n >= 4 && !leaves;
     for (int k = 0; k < 4; k++) quad = quad && ((uintptr_t)out[k] & 15) == 0;
     if (quad)
-        fold_line_kernel4<<<(unsigned)((half / 4 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n, alpha, d_alpha, ctx->itw);
+        e = launch_following(ctx, fold_line_kernel4, (unsigned)((half / 4 + 255) / 256), 256u, o, s, log_n, alpha, d_alpha, ctx->itw);
     else if (wide)
-        fold_line_kernel2<<<(unsigned)((half / 2 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n, alpha, d_alpha, ctx->itw, leaves);
+        e = launch_following(ctx, fold_line_kernel2, (unsigned)((half / 2 + 255) / 256), 256u, o, s, log_n, alpha, d_alpha, ctx->itw, leaves);
     else
         fold_line_kernel<<<(unsigned)((half + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n, alpha, d_alpha, ctx->itw, leaves);
+    ZKB_CUDA(ctx, e);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
 }
@@ -299,14 +305,16 @@ static int fold_circle_impl(zkb_ctx* ctx, uint32_t* const dst[4], const uint32_t
     bool wide = log_n_src >= 4;
     for (int k = 0; k < 4; k++) wide = wide && ((uintptr_t)src[k] & 15) == 0 && ((uintptr_t)dst[k] & 7) == 0;
     ProfScope prof(ctx, "fold_circle_kernel");
+    cudaError_t e = cudaSuccess;
     bool quad = wide && log_n_src >= 5 && !leaves;
     for (int k = 0; k < 4; k++) quad = quad && ((uintptr_t)dst[k] & 15) == 0;
     if (quad)
-        fold_circle_kernel4<<<(unsigned)((half / 4 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, fresh);
+        e = launch_following(ctx, fold_circle_kernel4, (unsigned)((half / 4 + 255) / 256), 256u, o, s, log_n_src, alpha, d_alpha, ctx->itw, fresh);
     else if (wide)
-        fold_circle_kernel2<<<(unsigned)((half / 2 + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves, fresh);
+        e = launch_following(ctx, fold_circle_kernel2, (unsigned)((half / 2 + 255) / 256), 256u, o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves, fresh);
     else
         fold_circle_kernel<<<(unsigned)((half + 255) / 256), 256, 0, ctx->stream>>>(o, s, log_n_src, alpha, d_alpha, ctx->itw, leaves, fresh);
+    ZKB_CUDA(ctx, e);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
 }
