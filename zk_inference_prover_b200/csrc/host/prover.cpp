@@ -193,6 +193,9 @@ struct MerkleProver {
     // `chan_step`, when given, is a FRI layer's channel step (channel state, challenge slot, root copy; device addresses) to run
     // in the launch that builds the root; *chan_done says whether it ran (a tree of one node has no such launch).
     struct ChanStep { uint32_t *chan, *alpha, *root_copy; };
+    // The launch that ends a tree takes it from 2^8 hashes on: below, a hash is a quad's (blake2s.cu), and the two levels above cost
+    // the launch before it 2 us and this one, with the code for a thread a hash to fetch, 7.
+    static constexpr uint32_t TOP_LOG = 8;
     static MerkleProver commit(const Device& d, const std::vector<const BaseColumn*>& columns, HashColumn* leaves = nullptr,
                                const ChanStep* chan_step = nullptr, bool* chan_done = nullptr) {  // :39-64
         if (chan_done) *chan_done = false;
@@ -227,16 +230,16 @@ struct MerkleProver {
                                          (int)mp.layer_col_ptrs[log].size(), 1, mp.layers[log].ptr()));
             }
             const bool all = log <= min_log;  // no columns left below
-            if (log > 0 && log <= 10 && all) {
+            if (log > 0 && log <= TOP_LOG && all) {
                 // no columns left below: the rest of the tree is nodes only, built in one launch
                 std::vector<uint32_t*> lower;
                 for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
                 top(log, mp.layers[log].ptr(), lower.data());
                 break;
             }
-            // The layers below this one that hold no column (down to the next layer that has one, or to the last ten, which
+            // The layers below this one that hold no column (down to the next layer that has one, or to the last ones, which
             // the launch above builds): up to nine of them per launch.
-            uint32_t floor_log = 10u;
+            uint32_t floor_log = TOP_LOG;
             if (!all) {
                 uint32_t next = log - 1;
                 while (!count[next]) next--;
@@ -249,7 +252,7 @@ struct MerkleProver {
                 d.check(zkb_merkle_levels(d.ctx(), (int)log, mp.layers[log].ptr(), (int)levels, outs.data(), 1));
                 log -= levels;
             }
-            if (log > 0 && log <= 10 && all && mp.layers[log - 1].len() == 0) {
+            if (log > 0 && log <= TOP_LOG && all && mp.layers[log - 1].len() == 0) {
                 std::vector<uint32_t*> lower;
                 for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
                 top(log, mp.layers[log].ptr(), lower.data());
