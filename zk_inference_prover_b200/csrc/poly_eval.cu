@@ -95,6 +95,52 @@ __global__ void __launch_bounds__(256) eval_dot_kernel(const uint32_t* const* __
     }
 }
 
+// Columns of at most 2^10 coefficients: out[col] = sum_i cols[col][i] w_i with the weights in shared memory (made there, level by level:
+// ten products deep), a warp a column, CTAs over the columns until none are left. Bound by HBM where there are many columns; folding
+// a column as a tree of QM31 values in shared memory instead took ten times the arithmetic (65,000 columns of 2^8 to 2^10: 500 us).
+constexpr int EVAL_SHORT_LOG = 10;
+__global__ void __launch_bounds__(256) eval_short_kernel(const uint32_t* const* __restrict__ cols, int ncols, int log_n, const __grid_constant__ EvalFactors f,
+                                                         uint32_t* __restrict__ out) {
+    __shared__ uint4 w[1 << EVAL_SHORT_LOG];
+    const uint32_t n = 1u << log_n, lane = threadIdx.x & 31u;
+    if (threadIdx.x == 0) w[0] = make_uint4(1u, 0u, 0u, 0u);
+    for (int k = 0; k < log_n; k++) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < (1u << k); i += 256u) {
+            const uint4 x = w[i];
+            const qm31 r = qm31_mul(qm31{{x.x, x.y, x.z, x.w}}, f.m[k]);
+            w[(1u << k) + i] = make_uint4(r.c[0], r.c[1], r.c[2], r.c[3]);
+        }
+    }
+    __syncthreads();
+    for (int col = (int)(blockIdx.x * 8u + (threadIdx.x >> 5)); col < ncols; col += (int)(gridDim.x * 8u)) {
+        const uint32_t* __restrict__ c = cols[col];
+        uint64_t a[4] = {0, 0, 0, 0};
+#pragma unroll 2
+        for (uint32_t e = lane; e < n; e += 128u) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) v[u] = e + 32u * u < n ? __ldcs(c + e + 32u * u) : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; u++) {
+                const uint4 x = w[e + 32u * u < n ? e + 32u * u : 0u];
+                a[0] += (uint64_t)v[u] * x.x; a[1] += (uint64_t)v[u] * x.y;
+                a[2] += (uint64_t)v[u] * x.z; a[3] += (uint64_t)v[u] * x.w;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) a[q] = fold64_eval(a[q]);
+        }
+        uint32_t r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t x = m31_reduce64(a[q]);
+            const uint32_t lo = __reduce_add_sync(0xffffffffu, x & 0xffffu), hi = __reduce_add_sync(0xffffffffu, x >> 16);
+            r[q] = m31_reduce64(lo + ((uint64_t)hi << 16));
+        }
+        if (lane == 0) reinterpret_cast<uint4*>(out)[col] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
 // in: either a table of M31 columns (IS_BASE) or a dense [ncols][2^log_in] array of QM31.
 // out: dense [ncols][2^(log_in - chunk_log)] QM31.
 template <bool IS_BASE>
@@ -167,6 +213,12 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
         uint32_t* bufA = ctx->scratch + weights_words;
         uint32_t* bufB = bufA + half_words;
         uint32_t* const out = d_out + 4 * (size_t)c0;  // what the last kernel writes to
+        if (log_n <= EVAL_SHORT_LOG) {
+            ProfScope prof(ctx, "eval_short_kernel");
+            eval_short_kernel<<<(unsigned)((nc + 7) / 8 < 6 * 148 ? (nc + 7) / 8 : 6 * 148), 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, f, out);
+            ZKB_LAUNCH_CHECK(ctx);
+            continue;
+        }
         int log_cur = log_n, level = 0;
         if (use_dot) {
             size_t items = (partials_per_col + DOT_CHUNKS - 1) / DOT_CHUNKS * (size_t)nc;
