@@ -2,7 +2,7 @@
 one-launch tail (2^10 values) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
 the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit;
 batches whose towers take one launch (2^10 entries) and two; samples whose quotient lines are worked out on the host and on the
-device (from 512 on, in pieces of 1,024)."""
+device (from 512 on, in pieces of 1,024); a few instances on both sides of the choice of driver."""
 import pytest
 
 from util import m31_column, qm31_array
@@ -62,4 +62,19 @@ def test_pcs_proof_around_the_line_kernel(ctx, oracle, n_cols):
     kw = dict(pow_bits=0, log_blowup=1, log_last_layer=0, n_queries=3, two_sample_every=6)
     want = oracle.pcs_prove(trees, **kw)
     got = ctx.pcs_prove_host(trees, **kw)
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("n_inst,log_n", [(2, 12), (2, 13), (3, 12), (3, 13), (4, 5)])
+def test_gkr_few_instances_around_the_choice_of_driver(ctx, oracle, n_inst, log_n):
+    inst, dev, keep = [], [], []
+    for k in range(n_inst):
+        kind, n = (3, 0, 1, 3)[k], 1 << (log_n - k)
+        den = qm31_array(7600 + 10 * log_n + k, n, nonzero=True)
+        num = qm31_array(7700 + 10 * log_n + k, n) if kind == 1 else None
+        inst.append((kind, num, den))
+        keep.append((ctx.upload(num) if num is not None else None, ctx.upload(den)))
+        dev.append((kind, keep[-1][0].ptr if keep[-1][0] else 0, keep[-1][1].ptr, n))
+    want = oracle.gkr_prove(inst, 0x5EED0006, verify=True)
+    got = ctx.gkr_prove_device(dev, 0x5EED0006)
     assert len(got) == len(want) and (got == want).all()

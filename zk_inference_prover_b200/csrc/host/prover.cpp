@@ -2419,10 +2419,13 @@ int zkb_gkr_prove_device(zkb_ctx* ctx, int n_inst, const int* kinds, const uint3
         ch.mix_u64(seed);
         std::vector<uint32_t> w;
         // Two drivers give the same proof. With everything on the device a layer costs no host round trip, but its masks and claims are
-        // hashed there, some 2.3 us an instance, and an instance's passes are launches of their own: measured against the batch driver
-        // (one launch a round for all instances, masks hashed on the host), 0.45-0.75 of its time for two to four instances of 2^8 to
-        // 2^16 entries, equal at six, twice at sixteen. ZKB_GKR_DRIVER=resident|batch overrides the choice.
-        bool resident = gkr_resident_supported(n_inst, ns) && n_inst <= 4;
+        // hashed there, some 2.3 us an instance, its small layers are one CTA's and an instance's large rounds are launches of their
+        // own; the batch driver takes a layer's rounds of all instances in one launch and some 40 us of host time. Measured
+        // (resident / batch, us): one instance of 2^12 457 / 748, of 2^22 2,266 / 2,787; two of 2^12 710 / 760, of 2^14 1,023 / 1,004, of 2^20
+        // 2,691 / 2,176; three of 2^8 373 / 404, of 2^12 784 / 778; four of 2^8 425 / 405. ZKB_GKR_DRIVER=resident|batch overrides the choice.
+        uint64_t tallest = 0;
+        for (int i = 0; i < n_inst; i++) tallest = std::max(tallest, ns[i]);
+        bool resident = gkr_resident_supported(n_inst, ns) && (n_inst == 1 || (n_inst <= 3 && tallest <= (uint64_t)1 << 12));
         if (const char* pick = getenv("ZKB_GKR_DRIVER")) {
             if (!strcmp(pick, "resident")) resident = gkr_resident_supported(n_inst, ns);
             else if (!strcmp(pick, "batch")) resident = false;
