@@ -27,11 +27,12 @@ ZK_HD uint32_t m31_sub(uint32_t a, uint32_t b) { uint32_t d = a - b; return umin
 ZK_HD uint32_t m31_neg(uint32_t a) { return a ? P - a : 0u; }
 ZK_HD uint32_t m31_dbl(uint32_t a) { return m31_add(a, a); }
 
-// A 64-bit value below 4 p^2 (or any whose three parts below do not sum past 2^32) -> canonical residue. The three 31-bit parts
-// have weight one each; the middle one is a funnel shift on the device.
+// Any 64-bit value -> canonical residue. Its three parts of 31, 31 and 2 bits have weight one each; the middle one is a funnel shift
+// on the device. The top one is added after the fold: the two others are at most 2p < 2^32 and fold to at most p, so nothing is lost,
+// while all three at once reach 2^32 (at 3 * 2^62 - 1, say, which four products can add up to) and would wrap.
 ZK_HD uint32_t m31_reduce64(uint64_t v) {
-    uint32_t s = ((uint32_t)v & P) + ((uint32_t)(v >> 31) & P) + (uint32_t)(v >> 62);
-    s = (s & P) + (s >> 31);  // <= p + 1
+    uint32_t s = ((uint32_t)v & P) + ((uint32_t)(v >> 31) & P);
+    s = (s & P) + (s >> 31) + (uint32_t)(v >> 62);  // <= p + 3
     return umin32(s, s - P);
 }
 // Product of two canonical values.
