@@ -88,7 +88,6 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...);
 
 #define ZKB_LAUNCH_CHECK(ctx) ZKB_CUDA(ctx, cudaGetLastError())
 
-// RAII guard making the context's device current for the duration of a call.
 // Launches a kernel that may start while the one before it on the stream is still running (programmatic dependent launch): it calls
 // follow_previous() before it touches anything an earlier launch writes or reads. For chains of launches of a few microseconds.
 // With a timeline being recorded, plainly.
@@ -111,6 +110,7 @@ __device__ __forceinline__ void follow_previous() { asm volatile("griddepcontrol
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
+// RAII guard making the context's device current for the duration of a call.
 struct DeviceGuard {
     int prev = -1, dev;
     bool ok = true;
@@ -128,6 +128,11 @@ struct DeviceGuard {
 int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out);
 // The same ring for a block of bytes that the device reads as 16-byte vectors: starts on a 16-byte boundary.
 int stage_blob(zkb_ctx* ctx, const void* h_data, size_t bytes, void** out);
+constexpr size_t blob_slots(size_t bytes) { return (bytes + sizeof(void*) - 1) / sizeof(void*) + 1; }  // what it takes of the ring at most
+// The next `slots` slots are in one piece, after every table that is there now: by an operator that stages several tables, before the
+// first of them, with the sum of what it may stage. Without it a later table of the call could start the ring again and be written over
+// an earlier one, found there or just copied, that the call's kernel has yet to read. Refuses more than the ring holds.
+int stage_reserve(zkb_ctx* ctx, size_t slots);
 
 // Brackets a kernel launch with events when the timeline is on (see zkb_profile_begin).
 struct ProfScope {

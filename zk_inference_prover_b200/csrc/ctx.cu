@@ -1,10 +1,12 @@
 // Context lifetime, device memory helpers, the twiddle tower and small utilities.
+#include <climits>
 #include <cstdarg>
 #include <unordered_map>
 #include <utility>
 #include <vector>
 
 #include "common.cuh"
+#include "fri_tail.hpp"
 #include "side_stream.hpp"
 #include "gather_blocks.hpp"
 
@@ -27,6 +29,11 @@ static int stage_wrap(zkb_ctx* ctx) {
     ctx->ring_pos = 0;
     for (auto& t : ctx->staged) t.n = 0;
     return ZKB_OK;
+}
+
+int stage_reserve(zkb_ctx* ctx, size_t slots) {
+    if (slots > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_reserve: the tables of one call (%zu slots) exceed the staging ring", slots);
+    return ctx->ring_pos + slots > ctx->ring_cap ? stage_wrap(ctx) : ZKB_OK;
 }
 
 // Device memory of a proof's small arrays (tree layers, FRI layers, coordinate columns): a proof allocates hundreds of them, and
@@ -56,15 +63,13 @@ struct BlockCache {
 
 // Copies the table into the ring, unless the same table is still there from an earlier call: a tree's columns are named by the
 // interpolation, the extension, the hashing, the sampling, the numerators and the decommitment in turn, and a copy of a table in
-// between two kernels costs 2-3 us of the stream.
+// between two kernels costs 2-3 us of the stream. (What was handed out stays in place until the ring is used from its start again: an
+// operator with several tables has their room reserved first.)
 int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out) {
     if (n < 0 || (size_t)n > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_ptrs: %d pointers exceed the staging ring", n);
     if (n == 0) { *out = ctx->d_ring; return ZKB_OK; }
-    // Near the ring's end a table from its first half is not reused: a later table of the same operator (operators stage less than a
-    // quarter of the ring) might start the ring again and be written over it.
-    const size_t from = ctx->ring_pos > ctx->ring_cap / 4 * 3 ? ctx->ring_cap / 2 : 0;
     for (const auto& t : ctx->staged) {
-        if (t.n != (size_t)n || t.pos < from || ctx->h_ring[t.pos] != h_ptrs[0] || memcmp(ctx->h_ring + t.pos, h_ptrs, (size_t)n * sizeof(void*))) continue;
+        if (t.n != (size_t)n || ctx->h_ring[t.pos] != h_ptrs[0] || memcmp(ctx->h_ring + t.pos, h_ptrs, (size_t)n * sizeof(void*))) continue;
         *out = ctx->d_ring + t.pos;
         return ZKB_OK;
     }
@@ -117,7 +122,8 @@ int side_join(zkb_ctx* ctx) {
     return ZKB_OK;
 }
 
-int stage_blob(zkb_ctx* ctx, const void* h_data, size_t bytes, void** out) {
+// A block's place in the ring, its bytes copied to the page-locked side.
+static int stage_place(zkb_ctx* ctx, const void* h_data, size_t bytes, size_t* at) {
     const size_t slots = (bytes + sizeof(void*) - 1) / sizeof(void*);
     if (slots + 1 > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_blob: %zu bytes exceed the staging ring", bytes);
     size_t pos = (ctx->ring_pos + 1) & ~(size_t)1;  // slots are 8 bytes and the ring's base is aligned: even slots are 16-byte aligned
@@ -126,9 +132,22 @@ int stage_blob(zkb_ctx* ctx, const void* h_data, size_t bytes, void** out) {
         pos = 0;
     }
     memcpy(ctx->h_ring + pos, h_data, bytes);
-    ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->d_ring + pos, ctx->h_ring + pos, bytes, cudaMemcpyHostToDevice, ctx->stream));
     ctx->ring_pos = pos + slots;
+    *at = pos;
+    return ZKB_OK;
+}
+int stage_blob(zkb_ctx* ctx, const void* h_data, size_t bytes, void** out) {
+    size_t pos = 0;
+    if (int rc = stage_place(ctx, h_data, bytes, &pos)) return rc;
+    ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->d_ring + pos, ctx->h_ring + pos, bytes, cudaMemcpyHostToDevice, ctx->stream));
     *out = ctx->d_ring + pos;
+    return ZKB_OK;
+}
+int upload_small(zkb_ctx* ctx, uint32_t* dst, const uint32_t* h, size_t words) {
+    DeviceGuard g(ctx);
+    size_t pos = 0;
+    if (int rc = stage_place(ctx, h, words * 4, &pos)) return rc;
+    ZKB_CUDA(ctx, cudaMemcpyAsync(dst, ctx->h_ring + pos, words * 4, cudaMemcpyHostToDevice, ctx->stream));
     return ZKB_OK;
 }
 
@@ -712,15 +731,22 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
     DeviceGuard g(ctx);
     // The column tables of short blocks (a FRI layer's four columns) travel in the plan; those of a tree's columns are the ones its
     // commitment staged.
-    constexpr int OWN_COLS = 64;
-    size_t n_idx = 0, n_own = 0;
+    int own_cols = 64;
+    size_t n_idx = 0, n_own = 0, n_wide = 0;
     for (int b = 0; b < n_blocks; b++) {
         n_idx += (size_t)blocks[b].nidx;
-        if (blocks[b].ncols <= OWN_COLS) n_own += (size_t)blocks[b].ncols;
+        (blocks[b].ncols <= own_cols ? n_own : n_wide) += (size_t)blocks[b].ncols;
+    }
+    if (n_wide > ctx->ring_cap / 2) {  // too many to be in the ring together: all travel in the plan
+        own_cols = INT_MAX;
+        n_own += n_wide;
+        n_wide = 0;
     }
     // [word addresses | hash addresses | short tables | block descriptors | row indices]
     const size_t at_hash = 8 * n_words, at_own = at_hash + 8 * n_hashes, at_blocks = at_own + 8 * n_own, at_idx = at_blocks + sizeof(PlanBlock) * (size_t)n_blocks;
     std::vector<unsigned char> blob(at_idx + 4 * n_idx);
+    const bool in_ring = blob.size() <= sizeof(void*) * (ctx->ring_cap / 8);  // a longer plan brings its own memory
+    if (int rc = stage_reserve(ctx, n_wide + (in_ring ? blob_slots(blob.size()) : 0))) return rc;
     if (n_words) memcpy(blob.data(), word_addrs, 8 * n_words);
     if (n_hashes) memcpy(blob.data() + at_hash, hash_addrs, 8 * n_hashes);
     PlanBlock* pb = reinterpret_cast<PlanBlock*>(blob.data() + at_blocks);
@@ -729,7 +755,7 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
     for (int b = 0; b < n_blocks; b++) {
         const GatherBlock& g = blocks[b];
         void** cols = nullptr;
-        const bool here = g.ncols <= OWN_COLS;
+        const bool here = g.ncols <= own_cols;
         if (here) {  // as an offset into the plan
             memcpy(blob.data() + at_own + 8 * own, g.cols, 8 * (size_t)g.ncols);
             cols = reinterpret_cast<void**>(at_own + 8 * own);
@@ -741,12 +767,11 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
         pb[b] = {(const uint32_t* const*)cols, (uint32_t)g.ncols, (uint32_t)first_idx, (uint32_t)g.out_off, here ? 1u : 0u};
         first_idx += (size_t)g.nidx;
     }
-    // a plan too long for the staging ring brings its own memory
     unsigned char *d_blob = nullptr, *d_own = nullptr;
     uint32_t* d_out = nullptr;
     cudaError_t e = cudaSuccess;
     int rc = ZKB_OK;
-    if (blob.size() <= sizeof(void*) * (ctx->ring_cap / 8)) {
+    if (in_ring) {
         rc = stage_blob(ctx, blob.data(), blob.size(), (void**)&d_blob);
     } else {
         rc = zkb_malloc(ctx, blob.size(), (void**)&d_own);

@@ -318,7 +318,9 @@ int lde_cols_blocked(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols, int
     for (int c = 0; c < ncols; c++) ZKB_CHECK_ARG(ctx, (const void*)coeffs[c] != (const void*)out[c]);
     DeviceGuard g(ctx);
     void **d_src, **d_dst;
-    int rc = stage_ptrs(ctx, (const void* const*)coeffs, ncols, &d_src);
+    int rc = stage_reserve(ctx, 2 * (size_t)ncols);
+    if (rc) return rc;
+    rc = stage_ptrs(ctx, (const void* const*)coeffs, ncols, &d_src);
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)out, ncols, &d_dst);
     if (rc) return rc;

@@ -334,7 +334,9 @@ int zkb_freivalds_scatter(zkb_ctx* ctx, const int8_t* qx, const int8_t* const* q
     for (uint32_t m = 0; m < n_mats; m++) ZKB_CHECK_ARG(ctx, qw[m] != nullptr && (uint64_t)grid->chunks * pk >= h_n_out[m]);
     DeviceGuard g(ctx);
     void **d_base, **d_pre, **d_qw;
-    int rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)pq, &d_base);
+    int rc = stage_reserve(ctx, (size_t)pq + (size_t)n_mats * pk + 4 + n_mats + blob_slots(n_mats * 4));
+    if (rc) return rc;
+    rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)pq, &d_base);
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)pre_cols, (int)(n_mats * pk + 4), &d_pre);
     if (rc) return rc;
@@ -375,7 +377,9 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     // the powers go up through the pinned staging ring: no synchronisation with the work before
     void **d_base, **d_pre, **d_out;
     void* d_pw;
-    int rc = stage_blob(ctx, pows.data(), pows.size() * sizeof(qm31), &d_pw);
+    int rc = stage_reserve(ctx, blob_slots(pows.size() * sizeof(qm31)) + (size_t)pq + (size_t)n_mats * pk + (1 + 2 * (size_t)n_mats) * 4);
+    if (rc) return rc;
+    rc = stage_blob(ctx, pows.data(), pows.size() * sizeof(qm31), &d_pw);
     if (rc) return rc;
     uint4* d_pows = reinterpret_cast<uint4*>(d_pw);
     rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)pq, &d_base);

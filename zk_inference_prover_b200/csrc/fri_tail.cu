@@ -207,15 +207,6 @@ int grind_first(zkb_ctx* ctx, const uint32_t* prefixed, int pow_bits, uint32_t* 
     return ZKB_OK;
 }
 
-// (the ring's slots are 8 bytes; the copy is ordered on the stream like every use of dst)
-int upload_small(zkb_ctx* ctx, uint32_t* dst, const uint32_t* h, size_t words) {
-    DeviceGuard g(ctx);
-    void* staged = nullptr;
-    if (int rc = stage_blob(ctx, h, words * 4, &staged)) return rc;
-    ZKB_CUDA(ctx, cudaMemcpyAsync(dst, staged, words * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-    return ZKB_OK;
-}
-
 int read_small(zkb_ctx* ctx, const uint32_t* d, size_t words, const uint32_t** h) {
     ZKB_CHECK_ARG(ctx, words <= (size_t)SMALL_WORDS);
     DeviceGuard g(ctx);

@@ -773,6 +773,20 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
     return ZKB_OK;
 }
 
+// The block a layer's launch stages: the transcript's state, the CTAs' meeting place, the powers of alpha, the rounds' constants, the tables,
+// room for the rounds' records (every part a multiple of four words).
+struct LayerBlob { size_t sync, alpha, rounds, tables, records, words; };
+static LayerBlob layer_blob(const GkrLayerPlan& plan) {
+    LayerBlob o;
+    o.sync = sizeof(GkrStepState) / 4;
+    o.alpha = o.sync + sizeof(GkrSync) / 4;
+    o.rounds = o.alpha + 4 * plan.n_vars.size();
+    o.tables = o.rounds + (sizeof(GkrStepConst) / 4) * (size_t)plan.n_rounds;
+    o.records = o.tables + plan.tables.size();
+    o.words = o.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
+    return o;
+}
+
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
     const int n_rounds = plan.n_rounds;
     if (plan.n_vars.size() > GKR_BATCH_MAX_ITEMS) return set_error(ctx, ZKB_EINVAL, "gkr batch: more than %d instances", (int)GKR_BATCH_MAX_ITEMS);
@@ -809,8 +823,11 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
         tb.later = later;
         later = std::max(later, tb.ctas);
     }
+    // What the launch stages later must not come to lie over the items: room for both.
+    const size_t item_bytes = plan.items.size() * sizeof(GkrBatchItem);
+    if (int rc = stage_reserve(ctx, blob_slots(item_bytes) + blob_slots(4 * layer_blob(plan).words))) return rc;
     void* d = nullptr;
-    if (int rc = stage_blob(ctx, plan.items.data(), plan.items.size() * sizeof(GkrBatchItem), &d)) return rc;
+    if (int rc = stage_blob(ctx, plan.items.data(), item_bytes, &d)) return rc;
     plan.d_items = static_cast<const GkrBatchItem*>(d);
     return ZKB_OK;
 }
@@ -821,12 +838,9 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     if (int rc = batch_buffers(ctx)) return rc;
     const size_t K = plan.n_vars.size();
     const int n_rounds = plan.n_rounds;
-    // The staged block: the transcript's state, the CTAs' meeting place, the powers of alpha, the rounds' constants, the tables, room for
-    // the rounds' records (every part a multiple of four words).
-    const size_t o_state = 0, o_sync = sizeof(GkrStepState) / 4, o_alpha = o_sync + sizeof(GkrSync) / 4, o_rounds = o_alpha + 4 * K, o_tables = o_rounds + (sizeof(GkrStepConst) / 4) * (size_t)n_rounds;
-    const size_t o_records = o_tables + plan.tables.size();
+    const LayerBlob at = layer_blob(plan);
     std::vector<uint32_t>& blob = ctx_blob();
-    blob.assign(o_records + GKR_LAYER_OUT_WORDS * (size_t)n_rounds, 0u);
+    blob.assign(at.words, 0u);
     auto q4 = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
     // The oracles' claims by the round they enter in (group; those without variables never do), each times alpha^k. The claims come
     // scaled by 2^(rounds they wait), and a waiting oracle's claim halves every round (sumcheck.rs:115-125).
@@ -836,13 +850,13 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         qm31& v = entering[n_rounds - (int)plan.n_vars[k]];
         v = qm31_add(v, qm31_mul(q4(alpha_pow + 4 * k), q4(claims + 4 * k)));
     }
-    GkrStepState& st = *reinterpret_cast<GkrStepState*>(&blob[o_state]);
+    GkrStepState& st = *reinterpret_cast<GkrStepState*>(blob.data());
     memcpy(st.digest, chan, 32);
     st.n_draws = chan[8];
     st.claim = entering[0];
     for (auto& c : st.corr) c = qm31_one();
-    memcpy(&blob[o_alpha], alpha_pow, 16 * K);
-    GkrStepConst* const consts = reinterpret_cast<GkrStepConst*>(&blob[o_rounds]);
+    memcpy(&blob[at.alpha], alpha_pow, 16 * K);
+    GkrStepConst* const consts = reinterpret_cast<GkrStepConst*>(&blob[at.rounds]);
     qm31 waiting = qm31_zero();
     for (int j = n_rounds; j-- > 0;) {
         waiting = qm31_add(waiting, entering[j + 1]);  // all that enter after round j
@@ -859,12 +873,12 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         c.entering = j + 1 < n_rounds ? qm31_mul_m31(entering[j + 1], half_pow) : qm31_zero();
         c.round = (uint32_t)j;
     }
-    memcpy(&blob[o_tables], plan.tables.data(), 4 * plan.tables.size());
+    memcpy(&blob[at.tables], plan.tables.data(), 4 * plan.tables.size());
     void* d_blob_v = nullptr;
     if (int rc = stage_blob(ctx, blob.data(), blob.size() * 4, &d_blob_v)) return rc;
     uint32_t* d_blob = static_cast<uint32_t*>(d_blob_v);
-    GkrStepState* d_state = reinterpret_cast<GkrStepState*>(d_blob + o_state);
-    const GkrStepConst* d_consts = reinterpret_cast<const GkrStepConst*>(d_blob + o_rounds);
+    GkrStepState* d_state = reinterpret_cast<GkrStepState*>(d_blob);
+    const GkrStepConst* d_consts = reinterpret_cast<const GkrStepConst*>(d_blob + at.rounds);
     const qm31 lam = q4(h_lambda);
     GkrLayerOut host;
     host.records = ctx->h_batch;
@@ -883,8 +897,8 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     cfg.stream = ctx->stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, reinterpret_cast<const GkrTable*>(d_blob + o_tables), n_rounds + 1, eq_evals, lam,
-                                             (const uint32_t*)(d_blob + o_alpha), d_state, reinterpret_cast<GkrSync*>(d_blob + o_sync), d_consts, d_blob + o_records, n_rounds,
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, reinterpret_cast<const GkrTable*>(d_blob + at.tables), n_rounds + 1, eq_evals, lam,
+                                             (const uint32_t*)(d_blob + at.alpha), d_state, reinterpret_cast<GkrSync*>(d_blob + at.sync), d_consts, d_blob + at.records, n_rounds,
                                              host);
     if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
     return ZKB_OK;

@@ -385,10 +385,7 @@ int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<Numerat
                 sums[2 * b + 1] = qm31_add(sums[2 * b + 1], qm31_mul(p, conj_q(v)));
             }
         memcpy(&h[4 * n], e.col.data(), 4 * n);
-        void* staged = nullptr;  // read where the ring holds it (the accumulations that follow stage a small part of it)
-        if (int rc = stage_blob(ctx, h.data(), 20 * n, &staged)) return rc;
-        lines.d_c = static_cast<uint32_t*>(staged);
-        lines.d_col = lines.d_c + 4 * n;
+        if (int rc = upload_words(ctx, lines.d_c, h)) return rc;  // [c: 4 n][col: n], where the accumulations that follow read it
     } else {
         size_t n_chunks = 0;
         for (auto& b : batches) n_chunks += (b.count + LINE_CHUNK - 1) / LINE_CHUNK;

@@ -382,7 +382,9 @@ int zkb_witness_dequant(zkb_ctx* ctx, const int32_t* acc, const int32_t* jx, con
     else for (int k = 0; k < 6; k++) ZKB_CHECK_ARG(ctx, c.f_mul[k] < c.per_slot);
     DeviceGuard g(ctx);
     void **d_base, **d_pre;
-    int rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)n_base, &d_base);
+    int rc = stage_reserve(ctx, (size_t)n_base + n_pre);
+    if (rc) return rc;
+    rc = stage_ptrs(ctx, (const void* const*)base_cols, (int)n_base, &d_base);
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)pre_cols, (int)n_pre, &d_pre);
     if (rc) return rc;

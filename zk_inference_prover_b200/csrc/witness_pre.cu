@@ -475,8 +475,9 @@ using namespace zk;
 
 namespace {
 // Host arrays the kernels index (groups, slots, pointer tables) go up through the context's staging ring, 8 bytes a word.
+template <class T> size_t array_slots(size_t n) { return (n * sizeof(T) + 7) / 8 + 1; }
 template <class T> int stage_array(zkb_ctx* ctx, const T* src, size_t n, const T** out) {
-    std::vector<uint64_t> blob((n * sizeof(T) + 7) / 8 + 1, 0);
+    std::vector<uint64_t> blob(array_slots<T>(n), 0);
     if (n) memcpy(blob.data(), src, n * sizeof(T));
     void** d = nullptr;
     int rc = stage_ptrs(ctx, reinterpret_cast<const void* const*>(blob.data()), (int)blob.size(), &d);
@@ -503,7 +504,9 @@ int zkb_witness_pre_table(zkb_ctx* ctx, uint32_t kind, uint32_t log_rows, uint32
     ZKB_CHECK_ARG(ctx, real <= (1ull << log_rows));
     DeviceGuard g(ctx);
     void **d_cnt = nullptr, **d_cols = nullptr;
-    int rc = stage_ptrs(ctx, (const void* const*)cols, (int)n_cols, &d_cols);
+    int rc = stage_reserve(ctx, (size_t)n_cols + n_counters);
+    if (rc) return rc;
+    rc = stage_ptrs(ctx, (const void* const*)cols, (int)n_cols, &d_cols);
     if (rc) return rc;
     if (n_counters && m_col) {
         rc = stage_ptrs(ctx, (const void* const*)counters, (int)n_counters, &d_cnt);
@@ -640,7 +643,10 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     DeviceGuard g(ctx);
     RsArgs a{};
     void** d_cols = nullptr;
-    int rc = stage_ptrs(ctx, (const void* const*)cols, (int)n_cols, &d_cols);
+    int rc = stage_reserve(ctx, (size_t)n_cols + array_slots<RsGroup>(p.n_groups) + array_slots<RsSlot>(p.n_slots) + array_slots<uint32_t>(p.out_w) +
+                                    array_slots<uint32_t>(level_start.size()) + array_slots<uint32_t*>(tables->n_un) + array_slots<RsMult>(tables->n_un));
+    if (rc) return rc;
+    rc = stage_ptrs(ctx, (const void* const*)cols, (int)n_cols, &d_cols);
     if (rc) return rc;
     static_assert(sizeof(zkb_rs_group) == sizeof(RsGroup) && sizeof(zkb_rs_slot) == sizeof(RsSlot) && sizeof(zkb_rs_mult) == sizeof(RsMult), "layout");
     if ((rc = stage_array(ctx, reinterpret_cast<const RsGroup*>(p.groups), p.n_groups, &a.groups))) return rc;
