@@ -66,9 +66,9 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(int log_size, const u
 // and the addresses of the next one's are on their way while the block before is hashed. A tree of 2^16 leaves built layer by
 // layer, with the next launch started early (below): 5.4 -> 4.2 us a layer.
 constexpr int QUAD_THREADS = 64, QUAD_MAX_LOG = 13;
-__global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log_size, const uint32_t* __restrict__ prev,
+__global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log_size, const uint32_t* prev,
                                                                          const uint32_t* const* __restrict__ cols, int ncols, int m31_out,
-                                                                         uint32_t* __restrict__ out) {
+                                                                         uint32_t* out) {
     __shared__ uint32_t sched[40];
     __shared__ alignas(16) uint32_t msg[QUAD_THREADS / 4][PAIR_WORDS];
     const uint32_t node = blockIdx.x * (QUAD_THREADS / 4) + (threadIdx.x >> 2), l = threadIdx.x & 3u;
@@ -86,11 +86,12 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
     };
     auto values = [&] {
 #pragma unroll
-        for (int u = 0; u < 4; u++) next[u] = at[u] ? __ldg(at[u] + i) : 0u;
+        for (int u = 0; u < 4; u++) next[u] = at[u] ? at[u][i] : 0u;
     };
     quad_make_schedule(sched, threadIdx.x, QUAD_THREADS);
     // A tree built layer by layer is a chain of launches of a microsecond or two: the next one may start now (programmatic dependent
-    // launch) and wait here for this grid to end.
+    // launch) and wait here for this grid to end. (What that grid writes while this one already runs, the children and the columns, is
+    // read by plain loads: a read-only load is for memory that nobody writes during a kernel's life.)
     let_next_start();
     follow_previous();
     addresses(0);

@@ -89,7 +89,8 @@ int set_error(zkb_ctx* ctx, int code, const char* fmt, ...);
 #define ZKB_LAUNCH_CHECK(ctx) ZKB_CUDA(ctx, cudaGetLastError())
 
 // Launches a kernel that may start while the one before it on the stream is still running (programmatic dependent launch): it calls
-// follow_previous() before it touches anything an earlier launch writes or reads. For chains of launches of a few microseconds.
+// follow_previous() before it touches anything an earlier launch writes or reads, and takes what that launch may still be writing by
+// plain loads (no const __restrict__ parameter, no __ldg). For chains of launches of a few microseconds.
 // With a timeline being recorded, plainly.
 template <class... P, class... A>
 cudaError_t launch_following(zkb_ctx* ctx, void (*kernel)(P...), unsigned grid, unsigned block, A... args) {

@@ -29,8 +29,9 @@ __device__ __forceinline__ qm31 fold_pair(const Secure4C& in, size_t i, uint32_t
 }
 
 // The folding challenge comes by value or, when d_alpha is given, from device memory (written by the
-// channel kernel of the previous step, so that a whole FRI commit phase runs without a host round trip).
-__device__ __forceinline__ qm31 load_alpha(const uint32_t* __restrict__ d_alpha, qm31 alpha) {
+// channel kernel of the previous step, so that a whole FRI commit phase runs without a host round trip; a kernel that
+// is launched while that step runs must not read it as memory that nobody writes).
+__device__ __forceinline__ qm31 load_alpha(const uint32_t* d_alpha, qm31 alpha) {
     if (d_alpha) {
         uint4 v = *reinterpret_cast<const uint4*>(d_alpha);
         return qm31{{v.x, v.y, v.z, v.w}};
@@ -81,7 +82,7 @@ __device__ __forceinline__ void fold_pair2(const Secure4C& in, size_t i2, uint32
 }
 
 __global__ void __launch_bounds__(256) fold_line_kernel2(Secure4 out, Secure4C in, int log_n, qm31 alpha,
-                                                         const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
+                                                         const uint32_t* d_alpha, const uint32_t* __restrict__ itw,
                                                          uint32_t* __restrict__ leaves) {
     follow_previous();
     alpha = load_alpha(d_alpha, alpha);
@@ -112,7 +113,7 @@ __device__ __forceinline__ void fold_quad(const Secure4C& in, size_t i4, const u
 }
 
 __global__ void __launch_bounds__(256) fold_line_kernel4(Secure4 out, Secure4C in, int log_n, qm31 alpha,
-                                                         const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw) {
+                                                         const uint32_t* d_alpha, const uint32_t* __restrict__ itw) {
     follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const size_t half = (size_t)1 << (log_n - 1);
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(256) fold_line_kernel4(Secure4 out, Secure4C i
 
 // (fresh: what is in dst counts as zero and is not read)
 __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
-                                                           const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw, int fresh) {
+                                                           const uint32_t* d_alpha, const uint32_t* __restrict__ itw, int fresh) {
     follow_previous();
     alpha = load_alpha(d_alpha, alpha);
     const qm31 alpha_sq = qm31_sqr(alpha);
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C
 }
 
 __global__ void __launch_bounds__(256) fold_circle_kernel2(Secure4 dst, Secure4C src, int log_n_src, qm31 alpha,
-                                                           const uint32_t* __restrict__ d_alpha, const uint32_t* __restrict__ itw,
+                                                           const uint32_t* d_alpha, const uint32_t* __restrict__ itw,
                                                            uint32_t* __restrict__ leaves, int fresh) {
     follow_previous();
     alpha = load_alpha(d_alpha, alpha);
