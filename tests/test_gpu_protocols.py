@@ -171,6 +171,35 @@ def test_gkr_batch_with_round_polynomials_of_low_degree(ctx, oracle, monkeypatch
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("spec", [[(0, 9, 1), (3, 6, None), (1, 5, None), (0, 4, None)],   # the tallest is constant: degree nought until the others enter
+                                  [(0, 8, 0), (0, 6, None), (0, 6, None), (0, 5, None)],   # nothing but the constants of those that wait
+                                  [(0, 7, 0)] * 5,                                         # polynomials without a coefficient
+                                  [(1, 7, 1)] * 3 + [(0, 7, 1)] * 2,
+                                  [(3, 6, None), (0, 8, 1), (2, 8, None)]])
+def test_gkr_batch_of_constant_layers_is_proven_once(ctx, oracle, monkeypatch, spec):
+    """A batch whose round polynomials are of low degree takes the launches any other takes, one a layer with rounds, and gives the
+    oracle's words. (kind, log size, the value of every entry or None.)"""
+    monkeypatch.setenv("ZKB_GKR_DRIVER", "batch")
+    insts, keep, dev = [], [], []
+    for i, (kind, lg, value) in enumerate(spec):
+        kind, num, den = _instance(kind, lg, 5600 + 10 * i)
+        if value is not None:
+            den = np.zeros_like(den)
+            den[:, 0] = value
+            num = np.zeros_like(num) if num is not None else None
+        insts.append((kind, num, den))
+        keep += [ctx.upload(num) if num is not None else None, ctx.upload(den)]
+        dev.append((kind, keep[-2].ptr if keep[-2] else 0, keep[-1].ptr, den.shape[0]))
+    want = oracle.gkr_prove(insts, 0x5EED0015, verify=True)
+    got = ctx.gkr_prove_device(dev, 0x5EED0015)
+    assert len(got) == len(want) and (got == want).all()
+    ctx.profile_begin()
+    ctx.gkr_prove_device(dev, 0x5EED0015)
+    prof = ctx.profile_end()
+    assert prof["gkr_batch_layer_kernel"][1] == max(lg for _, lg, _ in spec) - 1
+    assert "gkr_batch_round_kernel" not in prof
+
+
 def test_two_contexts_on_two_threads_prove_side_by_side(zkb, oracle):
     """Several contexts may be used from different host threads at once (one thread per context): two threads, each with
     its own context, prove a PCS opening over many short columns and a GKR batch of 20 instances three times over while the

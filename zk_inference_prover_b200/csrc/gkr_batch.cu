@@ -136,8 +136,10 @@ __device__ __forceinline__ void item_sums(const GkrBatchItem& it, size_t first, 
 // The step is then one warp's work whatever the number of instances: two products, three compressions (channel.cuh), four products.
 // (The form it replaces kept a record per oracle, passed over all of them twice per round and hashed on one thread: 5.5 us of
 // hashing alone, a launch with its step 27-40 us.)
-// What it can not tell is the length the combination keeps when its leading coefficient vanishes (that of its longest term, each
-// trimmed on its own): it raises a flag then, and the caller proves the batch again with the transcript on the host.
+// The combination keeps the length of its longest term, each trimmed on its own (lookups/utils.rs:165-170 under sumcheck.rs:139-149). The
+// step trims the sum instead, which is the same unless the longest terms' leading coefficients, times powers of alpha, cancel. Alpha is
+// drawn after everything that fixes them, so they do with a chance of some K / 2^124 a round, and the proof is a valid one even then. A
+// batch of constant layers (padding instances, products of ones) so takes no longer than any other.
 constexpr int GKR_GROUPS = 32;  // rounds of a layer at most, so groups of oracles that enter together
 
 struct GkrStepConst {        // of a round; host-made
@@ -150,7 +152,7 @@ struct GkrStepConst {        // of a round; host-made
 static_assert(sizeof(GkrStepConst) == 256, "GkrStepConst layout");
 
 struct alignas(16) GkrStepState {
-    uint32_t digest[8], n_draws, degenerate, pad[2];  // degenerate: a leading coefficient vanished
+    uint32_t digest[8], n_draws, pad[3];
     qm31 challenge, claim;                            // claim: sum of alpha^k claim_k over the active oracles
     qm31 corr[GKR_GROUPS];
     unsigned long long acc[2][GKR_GROUPS][8];         // the groups' sums of the round at hand, and zeros for the next
@@ -193,16 +195,16 @@ __device__ __forceinline__ void batch_step(GkrStepSm& sm, GkrStepState& st, cons
     const qm31 p = qmul(q == 0 ? S0 : q == 1 ? S2 : st.claim, q == 0 ? rc.A[c4] : q == 1 ? rc.B[c4] : rc.L1[c4]);
     const qm31 act = qm31_add(qm31_add(p, shflb(p, (lane + 4) & 31)), shflb(p, (lane + 8) & 31));
     const qm31 c = lane == 0 ? qm31_add(act, rc.waiting) : act;
+    const int len = 32 - __clz(__ballot_sync(0xffffffffu, lane < 4 && !qm31_is_zero(c)));
     if (lane < 4) {
         sm.coef[lane] = act;
         stqb(sm.ch.msg + 8, lane, c);
     }
-    chan_step_b(sm.ch, 16, 1, &sm.r);
+    chan_step_b(sm.ch, 4 * len, 1, &sm.r);
     const qm31 r = sm.r, y = rc.y, one = qm31_one();
     drawn();
     if (lane < 4) stqb(out, lane, c);
-    if (lane == 3 && qm31_is_zero(c)) st.degenerate = 1u;
-    if (lane == 0) out[16] = 4u;
+    if (lane == 0) out[16] = (uint32_t)len;
     // (c3 r + c2) r^2 + (c1 r + c0), eq(r, y)
     qm31 x = r, z = r;
     if (lane == 0) x = sm.coef[3];
@@ -228,8 +230,8 @@ __device__ __forceinline__ void batch_step_open(GkrStepSm& sm, const GkrStepStat
     __syncwarp();
 }
 // The channel's state to where the next launch finds it.
-__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, GkrStepState* st, uint32_t degenerate, int lane) {
-    const uint32_t w = lane < 8 ? sm.ch.msg[lane] : lane == 8 ? sm.ch.n_draws : lane == 9 ? degenerate : 0u;
+__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, GkrStepState* st, int lane) {
+    const uint32_t w = lane < 8 ? sm.ch.msg[lane] : lane == 8 ? sm.ch.n_draws : 0u;
     if (lane < 12) reinterpret_cast<uint32_t*>(st)[lane] = w;
 }
 
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
     __shared__ bool gave_up;
     // CTA 0 only: the transcript
     __shared__ GkrStepSm sm;
-    __shared__ struct alignas(16) { uint32_t digest[8], n_draws, degenerate, pad[2]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
+    __shared__ struct alignas(16) { uint32_t digest[8], n_draws, pad[3]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
     GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
     __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];
     static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
@@ -528,7 +530,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
     }
     if (!lead) return;
     __syncthreads();
-    if (warp == 0) batch_step_close(sm, st, s.degenerate, lane);
+    if (warp == 0) batch_step_close(sm, st, lane);
     __threadfence();
     __syncthreads();
     layer_out_words(host, records, n_rounds, st, tid, GKR_THREADS);
@@ -911,7 +913,6 @@ int gkr_batch_layer_end(zkb_ctx* ctx, const GkrLayerPlan& plan, GkrLayerResult& 
     res.records = ctx->h_batch;
     res.channel = res.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
     res.masks = res.channel + 12;
-    res.degenerate = res.channel[9] != 0u;
     return ZKB_OK;
 }
 

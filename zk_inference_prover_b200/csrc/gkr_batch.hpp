@@ -76,11 +76,9 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
                           const uint32_t* eq_evals, const uint32_t h_lambda[4], const uint32_t chan[9]);
 
 // In the context's memory, until the next call: n_rounds x GKR_LAYER_OUT_WORDS, the channel as above, n_oracles x GKR_LAYER_MASK_WORDS
-// (of every oracle that had a round). degenerate: a round polynomial's leading coefficient vanished; the results do not follow
-// the transcript then and must be thrown away.
+// (of every oracle that had a round).
 struct GkrLayerResult {
     const uint32_t *records, *channel, *masks;
-    bool degenerate;
 };
 int gkr_batch_layer_end(zkb_ctx* ctx, const GkrLayerPlan& plan, GkrLayerResult& res);
 

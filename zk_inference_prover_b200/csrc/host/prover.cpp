@@ -1459,9 +1459,8 @@ static void plan_layer(const std::vector<BatchTower>& towers, int level, int n_r
     plan.table_at.push_back(plan.items.size());
 }
 
-// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream. host_rounds_only: the transcript of the rounds stays on
-// the host; otherwise *degenerate may be set, and the caller proves again that way (see gkr_batch.hpp).
-static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const std::vector<Layer>& input_layers, bool host_rounds_only, bool* degenerate) {
+// gkr_prover.rs:657-882 with sumcheck.rs:96-176. Returns the proof word stream.
+static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const std::vector<Layer>& input_layers) {
     const size_t n_inst = input_layers.size();
     std::unique_ptr<HostClock> hc(new HostClock("gkr.towers"));
     std::vector<BatchTower> towers(n_inst);  // gen_layers, :847-852
@@ -1517,7 +1516,7 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
     // description is staged as one block (an item per oracle and active round, 64 bytes each, and some 52 bytes per oracle): a batch of
     // thousands of tall instances would not fit the staging ring and takes the round-by-round path, which stages one round's items at a time.
     const char* rounds_env = getenv("ZKB_GKR_ROUNDS");
-    const bool never = host_rounds_only || (rounds_env && !strcmp(rounds_env, "host"));
+    const bool never = rounds_env && !strcmp(rounds_env, "host");
     auto on_device = [&](const zk::GkrLayerPlan& p) {
         return !never && p.n_rounds > 0 && p.n_rounds <= zk::GKR_LAYER_MAX_ROUNDS &&
                64 * p.items.size() + 64 * p.n_vars.size() + 256 * (size_t)p.n_rounds + 8192 <= ((size_t)2 << 20);
@@ -1592,7 +1591,6 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
             hc.reset(new HostClock("gkr.layer.wait"));
             zk::GkrLayerResult res;
             d.check(zk::gkr_batch_layer_end(d.ctx(), plan, res));
-            if (res.degenerate) { *degenerate = true; return {}; }
             HashWords digest;
             memcpy(digest.data(), res.channel, 32);
             ch.set_state(digest, res.channel[8]);
@@ -2440,13 +2438,7 @@ int zkb_gkr_prove_device(zkb_ctx* ctx, int n_inst, const int* kinds, const uint3
             for (int k = 0; k < 8; k++) hw[k] = dg[k];
             ch.set_state(hw, nd);
         } else {
-            bool degenerate = false;
-            const Channel before = ch;
-            w = gkr_prove_batch(dev, ch, layers(), false, &degenerate);
-            if (degenerate) {
-                ch = before;
-                w = gkr_prove_batch(dev, ch, layers(), true, &degenerate);
-            }
+            w = gkr_prove_batch(dev, ch, layers());
         }
         w.insert(w.end(), ch.digest().begin(), ch.digest().end());
         *n_words = w.size();
