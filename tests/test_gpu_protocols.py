@@ -145,6 +145,24 @@ def test_gkr_drivers_give_the_same_proof(ctx, oracle, monkeypatch, driver, spec)
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("rounds,kernels", [("", {"gkr_batch_layer_kernel": 12}),
+                                            ("launches", {"gkr_batch_layer_kernel": 90, "gkr_batch_step_kernel": 90}),
+                                            ("host", {"gkr_batch_round_kernel": 90})])
+def test_gkr_rounds_setting_chooses_the_launches(ctx, monkeypatch, rounds, kernels):
+    """13 layers, of 0 ... 12 rounds: a launch for the layer, or one for each of its tables (a round more than it has, where it has one)
+    and one for each step."""
+    monkeypatch.setenv("ZKB_GKR_ROUNDS", rounds)
+    keep, dev = [], []
+    for i, (kind, lg) in enumerate(_WIDE_BATCH):
+        kind, num, den = _instance(kind, lg, 5800 + 10 * i)
+        keep += [ctx.upload(num) if num is not None else None, ctx.upload(den)]
+        dev.append((kind, keep[-2].ptr if keep[-2] else 0, keep[-1].ptr, den.shape[0]))
+    ctx.profile_begin()
+    ctx.gkr_prove_device(dev, 0x5EED0004)
+    prof = ctx.profile_end()
+    assert {k: v[1] for k, v in prof.items() if k in ("gkr_batch_layer_kernel", "gkr_batch_step_kernel", "gkr_batch_round_kernel")} == kernels
+
+
 @pytest.mark.parametrize("rounds", ["", "launches", "host"])
 @pytest.mark.parametrize("spec", [[(1, 6)] * 3, [(1, 4), (0, 6), (1, 5), (0, 3)], [(1, 3)] * 20 + [(0, 7)], [(1, 12), (1, 12), (0, 12)]])
 def test_gkr_batch_with_round_polynomials_of_low_degree(ctx, oracle, monkeypatch, rounds, spec):

@@ -363,7 +363,9 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
     return v;
 }
 
-__global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int n_tables,
+// Tables [first, end) of the layer. rc: null where the transcript's steps are launches of their own (gkr_batch_step_kernel); no CTA then
+// keeps it, and the challenge is in its slot before the launch.
+__global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int first, int end,
                                                                          const uint32_t* __restrict__ eq, qm31 lambda, const uint32_t* __restrict__ alpha_pow,
                                                                          GkrStepState* st, GkrSync* sync, const GkrStepConst* __restrict__ rc,
                                                                          uint32_t* records, int n_rounds, GkrLayerOut host) {
@@ -378,8 +380,8 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
     __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];
     static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool lead = blockIdx.x == 0;
-    for (int i = tid; i < 2 * n_tables; i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
+    const bool lead = blockIdx.x == 0 && rc;
+    for (int i = tid; i < 2 * end; i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
     for (int i = tid; i < GKR_GROUPS * 16; i += GKR_THREADS) (&sums[0][0])[i] = 0u;
     if (tid == 0) gave_up = false;
     if (lead) {
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
     }
     __syncthreads();
     if (lead && warp == 0) batch_step_open(sm, s, lane);
-    for (int t = 0; t < n_tables; t++) {
+    for (int t = first; t < end; t++) {
         const GkrTable tb = tabs[t];
         if (blockIdx.x >= tb.ctas) {
             if (blockIdx.x >= tb.later) return;
@@ -537,6 +539,30 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
     __threadfence_system();
     __syncthreads();
     if (tid == 0) *host.flag = host.id;
+}
+
+// The step after table t < n_rounds by itself, one warp; after the last table, what goes to the host.
+__global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, GkrSync* sync, const GkrStepConst* __restrict__ rc, uint32_t* records, int t, int n_rounds,
+                                                            GkrLayerOut host) {
+    __shared__ GkrStepSm sm;
+    const int lane = threadIdx.x;
+    if (t == n_rounds) {
+        layer_out_words(host, records, n_rounds, st, lane, 32);
+        __threadfence_system();
+        __syncwarp();
+        if (lane == 0) *host.flag = host.id;
+        return;
+    }
+    unsigned long long a[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+        a[c] = st->acc[t & 1][lane][c];
+        st->acc[t & 1][lane][c] = 0ull;
+    }
+    batch_step_open(sm, *st, lane);
+    batch_step(sm, *st, rc[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, [] {});
+    if (lane < 4) sync->slot[t + 1][lane] = sm.r.c[lane] | 0x80000000u;
+    batch_step_close(sm, st, lane);
 }
 
 // ---- a single round with its results to the host
@@ -889,19 +915,41 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     host.flag = reinterpret_cast<volatile unsigned int*>(ctx->h_batch + H_BATCH_FLAG);
     host.id = ++ctx->batch_round;
     const GkrTable* const h_tables = reinterpret_cast<const GkrTable*>(plan.tables.data());
-    ProfScope prof(ctx, "gkr_batch_layer_kernel");
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails
-    attr[0].val.cooperative = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(std::max(h_tables[0].ctas, h_tables[0].later));
-    cfg.blockDim = dim3(GKR_THREADS);
-    cfg.stream = ctx->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, reinterpret_cast<const GkrTable*>(d_blob + at.tables), n_rounds + 1, eq_evals, lam,
-                                             (const uint32_t*)(d_blob + at.alpha), d_state, reinterpret_cast<GkrSync*>(d_blob + at.sync), d_consts, d_blob + at.records, n_rounds,
-                                             host);
+    const GkrTable* const d_tables = reinterpret_cast<const GkrTable*>(d_blob + at.tables);
+    const uint32_t* const d_alpha = d_blob + at.alpha;
+    uint32_t* const d_records = d_blob + at.records;
+    GkrSync* const d_sync = reinterpret_cast<GkrSync*>(d_blob + at.sync);
+    cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
+    if (!plan.launches) {
+        ProfScope prof(ctx, "gkr_batch_layer_kernel");
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails
+        attr[0].val.cooperative = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(std::max(h_tables[0].ctas, h_tables[0].later));
+        cfg.blockDim = dim3(GKR_THREADS);
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, d_tables, 0, n_rounds + 1, eq_evals, lam, d_alpha, d_state, d_sync, d_consts, d_records, n_rounds, host);
+    }
+    // Asked for, or the CTAs are not all resident at once (a share of the GPU's SMs): a launch per table and one per step, where nobody waits.
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        e = cudaSuccess;
+        for (int t = 0; t <= n_rounds && e == cudaSuccess; t++) {
+            {
+                ProfScope prof(ctx, "gkr_batch_layer_kernel");
+                gkr_batch_layer_kernel<<<h_tables[t].ctas, GKR_THREADS, 0, ctx->stream>>>(plan.d_items, d_tables, t, t + 1, eq_evals, lam, d_alpha, d_state, d_sync, nullptr,
+                                                                                          d_records, n_rounds, host);
+            }
+            {
+                ProfScope prof(ctx, "gkr_batch_step_kernel");
+                gkr_batch_step_kernel<<<1, 32, 0, ctx->stream>>>(d_state, d_sync, d_consts, d_records, t, n_rounds, host);
+            }
+            e = cudaGetLastError();
+        }
+    }
     if (e != cudaSuccess) return set_error(ctx, ZKB_ECUDA, "gkr batch layer: %s", cudaGetErrorString(e));
     return ZKB_OK;
 }

@@ -67,6 +67,7 @@ struct GkrLayerPlan {
     std::vector<size_t> table_at;    // n_rounds + 2
     std::vector<uint32_t> tables;    // filled by gkr_batch_plan: how the kernel takes them
     const GkrBatchItem* d_items = nullptr;
+    bool launches = false;           // the layer as a launch per table and one per transcript step
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
 
