@@ -2,7 +2,9 @@
 one-launch tail (2^10 values) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
 the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit;
 batches whose towers take one launch (2^10 entries) and two; samples whose quotient lines are worked out on the host and on the
-device (from 512 on, in pieces of 1,024); a few instances on both sides of the choice of driver."""
+device (from 512 on, in pieces of 1,024); trees hashed on a second stream, quotients planned on a second thread, decommitments in one
+launch and in several; a few instances on both sides of the choice of driver."""
+import numpy as np
 import pytest
 
 from util import m31_column, qm31_array
@@ -63,6 +65,32 @@ def test_pcs_proof_around_the_line_kernel(ctx, oracle, n_cols):
     want = oracle.pcs_prove(trees, **kw)
     got = ctx.pcs_prove_host(trees, **kw)
     assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("shape,kw", [
+    # a tree before the last whose short layers are a chain of 64 blocks of sixteen columns is hashed on a second stream: 63, 64, the first
+    # of two, one whose layers are not all short
+    ([[4] * 600 + [5] * 424, [6] * 8], dict(n_queries=20)),
+    ([[4] * 608 + [5] * 416, [6] * 8], dict(n_queries=20)),
+    ([[5] * 1100 + [3] * 40, [4] * 1100, [7] * 3], dict(pow_bits=2, log_blowup=2, n_queries=20, two_sample_every=7)),
+    ([[4] * 3, [13] * 2 + [12] * 1040, [14]], dict(n_queries=5)),
+    # 8,191 and 8,192 samples: from there on the quotient plan is made on another thread
+    ([[4] * 8189, [5] * 2], dict(n_queries=3)),
+    ([[4] * 8190, [5] * 2], dict(n_queries=3)),
+    # a decommitment of more than 2^20 cells: a launch per block
+    ([[7] * 8300, [8] * 2], dict(n_queries=250)),
+])
+def test_pcs_proof_of_many_device_columns(ctx, oracle, shape, kw):
+    kw = {"pow_bits": 0, "log_blowup": 1, **kw}
+    trees = [[m31_column(6700 + 100 * t + c, 1 << lg) for c, lg in enumerate(logs)] for t, logs in enumerate(shape)]
+    want = oracle.pcs_prove(trees, **kw)
+    flat = np.concatenate([c for t in trees for c in t])
+    at = np.cumsum([0] + [len(c) for t in trees for c in t])
+    for _ in range(2):  # the second pass finds tables, blocks and buffers of the first
+        buf = ctx.upload(flat)
+        ptrs = iter([buf.ptr + 4 * int(a) for a in at[:-1]])
+        got = ctx.pcs_prove_device([[next(ptrs) for _ in t] for t in trees], [lg for t in shape for lg in t], **kw)
+        assert len(got) == len(want) and (got == want).all()
 
 
 @pytest.mark.parametrize("n_inst,log_n", [(2, 12), (2, 13), (3, 12), (3, 13), (4, 5)])
