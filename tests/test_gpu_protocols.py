@@ -93,7 +93,7 @@ def _instance(kind, log_n, seed):
         [(2, 10), (3, 7), (0, 8), (1, 3)],      # mixed kinds and sizes in one batch
         [(3, 12), (3, 12), (2, 12)],
         [(2, 16)],
-        # more than 16 instances: the batch path, one launch per sum-check round for all instances (csrc/gkr_batch.cu)
+        # many instances: the batch path, one launch per layer for all instances (csrc/gkr_batch.cu)
         [(3, 9)] * 6 + [(3, 7)] * 5 + [(1, 8)] * 3 + [(2, 6), (0, 5), (3, 2), (2, 2), (1, 1), (3, 1), (0, 2), (0, 1)],
         [(3, 13)] * 20 + [(3, 11)] * 12 + [(2, 12), (1, 10)],
     ],
@@ -119,16 +119,18 @@ _MIXED_BATCH = [(3, 9)] * 6 + [(3, 7)] * 5 + [(1, 8)] * 3 + [(2, 6), (0, 5), (3,
 
 
 @pytest.mark.parametrize("driver,spec", [("resident", [(2, 10), (3, 7), (0, 8), (1, 3)]), ("resident", [(3, 12), (3, 12), (2, 12)]),
+                                         # several oracles in rounds that are launches of their own (layers of more than 2^13 entries)
+                                         ("resident", [(3, 15), (2, 15)]), ("resident", [(0, 14), (2, 16), (1, 15), (3, 13), (1, 1)]),
                                          ("batch", [(2, 11)]), ("batch", [(1, 6), (0, 6)]),
                                          # the batch driver's three ways through a layer's rounds: the transcript on the host and a
-                                         # round trip per round; on the device with a launch per round; on the device with the small
+                                         # round trip per round; on the device with two launches per round; on the device with all
                                          # rounds in one launch (the default, which the cases of the test above take)
                                          ("batch:host", _WIDE_BATCH), ("batch:host", _MIXED_BATCH),
                                          ("batch:launches", _WIDE_BATCH), ("batch:launches", _MIXED_BATCH), ("batch:launches", [(2, 11)]),
                                          ("batch", [(0, 15), (1, 14), (2, 15)])])
 def test_gkr_drivers_give_the_same_proof(ctx, oracle, monkeypatch, driver, spec):
-    """The library picks the device-resident transcript for one or two instances and the batched rounds otherwise;
-    ZKB_GKR_DRIVER forces either, and both must reproduce the oracle's proof for any batch they accept."""
+    """The library picks the device-resident transcript for one instance and for two or three short ones and the batched rounds
+    otherwise; ZKB_GKR_DRIVER forces either, and both must reproduce the oracle's proof for any batch they accept."""
     driver, _, rounds = driver.partition(":")
     monkeypatch.setenv("ZKB_GKR_DRIVER", driver)
     if rounds:
