@@ -67,6 +67,21 @@ def test_pcs_proof_around_the_line_kernel(ctx, oracle, n_cols):
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("log_n", [0, 1, 9, 10, 11, 12, 22])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_eval_at_point_around_its_kernels(ctx, oracle, log_n, shift):
+    # up to 2^10 coefficients a warp a column; above, chunks of 2^11 by 16-byte loads or, for columns that do not start on 16 bytes, folded
+    n = 1 << log_n
+    cols = [m31_column(6300 + 10 * log_n + c, n) for c in range(3)]
+    at = [c * (n + 4 - n % 4) + shift for c in range(3)]
+    flat = np.zeros(at[2] + n, np.uint32)
+    for a, c in zip(at, cols):
+        flat[a:a + n] = c
+    buf, point = ctx.upload(flat), qm31_array(6390, 2).ravel()
+    got = ctx.eval_at_point_cols([buf.ptr + 4 * a for a in at], log_n, point)
+    assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()
+
+
 @pytest.mark.parametrize("shape,kw", [
     # a tree before the last whose short layers are a chain of 64 blocks of sixteen columns is hashed on a second stream: 63, 64, the first
     # of two, one whose layers are not all short

@@ -190,17 +190,30 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
         f.m[k] = x;
         x = qm31_double_x(x);
     }
+    constexpr int MAX_COLS = 32768;  // columns a launch
+    if (log_n <= EVAL_SHORT_LOG) {
+        for (int c0 = 0; c0 < ncols; c0 += MAX_COLS) {
+            const int nc = ncols - c0 < MAX_COLS ? ncols - c0 : MAX_COLS;
+            void** d_cols;
+            if (int rc = stage_ptrs(ctx, (const void* const*)(coeffs + c0), nc, &d_cols)) return rc;
+            ProfScope prof(ctx, "eval_short_kernel");
+            eval_short_kernel<<<(unsigned)((nc + 7) / 8 < 6 * 148 ? (nc + 7) / 8 : 6 * 148), 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, f,
+                                                                                                                  d_out + 4 * (size_t)c0);
+            ZKB_LAUNCH_CHECK(ctx);
+        }
+        return ZKB_OK;
+    }
+    static_assert(EVAL_SHORT_LOG + 1 == EVAL_CHUNK_LOG, "what is left has a whole chunk");
     // Scratch: [weights: 2048 QM31] [ping] [pong]; columns go in batches whose partials fit.
-    bool use_dot = log_n >= EVAL_CHUNK_LOG;
+    bool use_dot = true;
     for (int c = 0; c < ncols; c++) use_dot = use_dot && ((uintptr_t)coeffs[c] & 15) == 0;  // 16-byte loads
-    int first_chunk = log_n < EVAL_CHUNK_LOG ? log_n : EVAL_CHUNK_LOG;
-    size_t partials_per_col = (size_t)1 << (log_n - first_chunk);
+    size_t partials_per_col = (size_t)1 << (log_n - EVAL_CHUNK_LOG);
     uint32_t* weights = ctx->scratch;
     const size_t weights_words = (size_t)4 << EVAL_CHUNK_LOG;
     size_t half_words = (ctx->scratch_words - weights_words) / 2;
     size_t max_cols = half_words / (4 * partials_per_col);
     ZKB_CHECK_ARG(ctx, max_cols >= 1);
-    if (max_cols > 32768) max_cols = 32768;
+    if (max_cols > MAX_COLS) max_cols = MAX_COLS;
     if (use_dot) {
         eval_weights_kernel<<<(1 << EVAL_CHUNK_LOG) / 256, 256, 0, ctx->stream>>>(f, EVAL_CHUNK_LOG, weights);
         ZKB_LAUNCH_CHECK(ctx);
@@ -213,28 +226,21 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
         uint32_t* bufA = ctx->scratch + weights_words;
         uint32_t* bufB = bufA + half_words;
         uint32_t* const out = d_out + 4 * (size_t)c0;  // what the last kernel writes to
-        if (log_n <= EVAL_SHORT_LOG) {
-            ProfScope prof(ctx, "eval_short_kernel");
-            eval_short_kernel<<<(unsigned)((nc + 7) / 8 < 6 * 148 ? (nc + 7) / 8 : 6 * 148), 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, f, out);
-            ZKB_LAUNCH_CHECK(ctx);
-            continue;
-        }
         int log_cur = log_n, level = 0;
         if (use_dot) {
             size_t items = (partials_per_col + DOT_CHUNKS - 1) / DOT_CHUNKS * (size_t)nc;
             unsigned grid = (unsigned)(items < 2 * 148 ? items : 2 * 148);
             ProfScope prof(ctx, "eval_dot_kernel");
-            eval_dot_kernel<<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, weights, log_n == first_chunk ? out : bufA);
+            eval_dot_kernel<<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, weights, log_n == EVAL_CHUNK_LOG ? out : bufA);
             ZKB_LAUNCH_CHECK(ctx);
         } else {
-            unsigned threads = first_chunk >= 9 ? 256 : 32;
             dim3 grid((unsigned)partials_per_col, nc);
-            eval_fold_kernel<true><<<grid, threads, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nullptr, log_cur,
-                                                                      first_chunk, level, f, log_n == first_chunk ? out : bufA);
+            eval_fold_kernel<true><<<grid, 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nullptr, log_cur, EVAL_CHUNK_LOG, level, f,
+                                                                  log_n == EVAL_CHUNK_LOG ? out : bufA);
             ZKB_LAUNCH_CHECK(ctx);
         }
-        log_cur -= first_chunk;
-        level += first_chunk;
+        log_cur -= EVAL_CHUNK_LOG;
+        level += EVAL_CHUNK_LOG;
         while (log_cur > 0) {
             int ch = log_cur < EVAL_CHUNK_LOG ? log_cur : EVAL_CHUNK_LOG;
             unsigned threads = ch >= 9 ? 256 : 32;
