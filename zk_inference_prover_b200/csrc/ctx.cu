@@ -38,7 +38,7 @@ int stage_reserve(zkb_ctx* ctx, size_t slots) {
 
 // Device memory of a proof's small arrays (tree layers, FRI layers, coordinate columns): a proof allocates hundreds of them, and
 // the stream-ordered allocator takes 0.6-0.8 us of host time for each allocation and each release (716 us of a ten-column proof
-// were 230 of them). Blocks of up to 2^BLOCK_MAX_LOG bytes are rounded up to a power of two and kept per size when they are freed,
+// were 230 of them). Blocks of up to 2^MAX_LOG bytes are rounded up to a power of two and kept per size when they are freed,
 // up to KEPT_BYTES in all; they go back to the pool beyond that, when an allocation fails and with the context. A context's work is
 // ordered on one stream, so a kept block is as reusable as one the pool would hand out on that stream.
 struct BlockCache {

@@ -1,14 +1,13 @@
 // GKR batches of many instances (the prover's reductions hold hundreds: one instance per component and
 // power-of-two share of its lookups, prover/src/gkr_key_tile.rs:34-55). prove_batch
 // (nitroo/crates/stwo/src/prover/lookups/gkr_prover.rs:657-882) runs ONE sum-check per layer over all
-// instances, so what every instance needs in a round is known together. Here a round of the whole batch is
-// one launch and one read-back, whatever the number of instances: a table of work items (one per instance)
-// says what to do with which arrays, a flat grid of CTAs is split over the items in proportion to their
-// size, and every item's eight result words (and, at the end of a layer, its two-entry mask) land in one
-// result array.
+// instances, so what every instance needs in a round is known together: a table of work items (one per
+// instance) says what to do with which arrays.
 //
 // A whole layer's sum-check is one launch (gkr_batch_layer_begin): its CTAs take the rounds' tables one after the other, CTA 0 runs the
-// transcript step between them (the batch's round polynomial, the channel, the challenge, the claims).
+// transcript step between them (the batch's round polynomial, the channel, the challenge, the claims). Where the transcript of the
+// rounds stays on the host, a round is a launch and a read-back (gkr_batch_round): a flat grid of CTAs is split over the items in
+// proportion to their size, and every item's eight result words (and, at the end of a layer, its two-entry mask) land in one array.
 //
 //   mode 0  sum_as_poly_in_first_variable sums of the item's layer (first round of a layer's sum-check)
 //   mode 1  fix_first_variable with the round's challenge on every column, and the sums of the fixed layer

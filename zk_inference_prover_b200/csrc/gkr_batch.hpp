@@ -1,4 +1,4 @@
-// One launch per sum-check round for a GKR batch of any number of instances (gkr_batch.cu); internal to the library.
+// A layer's sum-check, or one round of it, for a GKR batch of any number of instances in one launch (gkr_batch.cu); internal to the library.
 #pragma once
 #include <cstddef>
 #include <cstdint>

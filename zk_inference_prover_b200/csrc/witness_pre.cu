@@ -258,7 +258,8 @@ __device__ __forceinline__ void operand(const RsArgs& a, uint32_t i, uint32_t c_
 // What bounded it were the counts (count_cache.cuh), then the latency of a slot, a chain of loads (its record, the operands' cells, a
 // row of the table) before its stores. So one CTA an SM keeps the counters and takes rows until none are left, in two teams of sixteen
 // warps; column addresses are computed where they can be (fourteen of them were 28 registers), four leaves are loaded at a time.
-// 2^15 rows of 128 additions: see RS_TIMES at the launch.
+// 2^15 rows of 128 additions: 690 us with the counts as atomics in L2, 257 us with them in shared memory, 206 us with four leaves or
+// outputs of a row to an access.
 constexpr uint32_t RS_LANES = 16, RS_TEAMS = 2, RS_LEAVES = 4;
 constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 12, RS_SMUL_LOG = 14;
 constexpr uint32_t RS_ADD_WORDS = (1u << RS_VAL_LOG) + (1u << RS_NORM_LOG) + (1u << RS_FRAC_LOG), RS_MUL_WORDS = (1u << RS_VAL_LOG) + (1u << RS_SMUL_LOG);
