@@ -39,3 +39,19 @@ def test_more_columns_than_the_ring_holds_are_refused(zkb):
         ctx.lde_cols(_columns(src, n, 4), 2, _columns(out, n, 8), 3)
     assert not out.download().any()
     ctx.close()
+
+
+def test_a_decommitment_of_more_columns_than_the_ring_takes_together(zkb, oracle):
+    """600,001 columns of two sizes: each size's tables fit the ring, all of them do not, so the decommitment's plan brings them along."""
+    logs = [[3] * 300000 + [2] * 300000, [4]]
+    at = np.cumsum([0] + [1 << lg for tree in logs for lg in tree])
+    vals, flat = m31_column(78, int(at[-1])), range(len(at) - 1)
+    cols = [vals[at[i]:at[i + 1]] for i in flat]
+    kw = dict(pow_bits=0, log_blowup=1, n_queries=2)
+    want = oracle.pcs_prove([cols[:-1], cols[-1:]], **kw)
+    ctx = zkb.Context(device=0, max_log_size=8)
+    buf = ctx.upload(vals)
+    ptrs = [buf.ptr + 4 * int(at[i]) for i in flat]
+    got = ctx.pcs_prove_device([ptrs[:-1], ptrs[-1:]], [lg for tree in logs for lg in tree], **kw)
+    assert len(got) == len(want) and (got == want).all()
+    ctx.close()
