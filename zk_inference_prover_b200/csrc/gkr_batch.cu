@@ -709,7 +709,7 @@ static int batch_buffers(zkb_ctx* ctx) {
     return ZKB_OK;
 }
 
-// Waits for a launch to report `id`: a bounded spin on the host (about 20 ms), then the stream.
+// Waits for a launch to report `id`: a bounded spin on the host (2 10^7 polls, a second at most), then the stream.
 static cudaError_t batch_wait(zkb_ctx* ctx, unsigned int id) {
     volatile unsigned int* flag = reinterpret_cast<volatile unsigned int*>(ctx->h_batch + H_BATCH_FLAG);
     if (!ctx->prof_on)
