@@ -121,3 +121,15 @@ def test_gkr_few_instances_around_the_choice_of_driver(ctx, oracle, n_inst, log_
     want = oracle.gkr_prove(inst, 0x5EED0006, verify=True)
     got = ctx.gkr_prove_device(dev, 0x5EED0006)
     assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("child_log,levels", [(19, 9), (20, 3), (20, 4), (21, 9), (23, 7)])
+def test_merkle_levels_around_the_split_launches(ctx, oracle, child_log, levels):
+    # from 2^20 children on three levels a launch, the others in the next
+    below = m31_column(7800 + child_log, 8 << child_log).reshape(-1, 8)
+    buf = ctx.upload(below)
+    outs = [ctx.alloc(8 << (child_log - j)) for j in range(1, levels + 1)]
+    ctx.merkle_levels(child_log, buf.ptr, [o.ptr for o in outs])
+    for j, o in enumerate(outs, 1):
+        below = oracle.commit_on_layer(child_log - j, below, [], m31=True)
+        assert (o.download(shape=(-1, 8)) == below).all(), j

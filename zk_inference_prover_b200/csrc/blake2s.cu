@@ -236,6 +236,10 @@ struct MerkleTopArgs { uint32_t* layer[MERKLE_TOP_MAX_LOG + 1]; };  // layer[k]:
 // one compression per node whatever the launch shape; what this saves is a launch (and its drain and refill of the whole
 // GPU) per layer, for the layers between the leaves and the last ten, which merkle_top_kernel builds.
 constexpr int MERKLE_LEVELS_MAX = 9;
+// From 2^20 children on the GPU is full with three levels of whole warps (eight, four and two of them), and the six above, where a CTA has at most
+// one warp's work and waits for its latency, are left to the next launch: nine levels of 2^22 children in one launch are 227 us, 18.5 M
+// hashes a ms, the first three alone 152, 24.2 M. At 2^18 the six levels as a launch of their own (12 us) cost more than they save (9).
+constexpr int MERKLE_LEVELS_SPLIT_LOG = 20, MERKLE_LEVELS_SPLIT = 3;
 struct MerkleLevelsArgs {
     const uint32_t* children;             // 2^child_log hashes
     uint32_t* out[MERKLE_LEVELS_MAX + 1];  // out[j]: the layer j levels above the children (2^(child_log - j) hashes), j = 1..levels
@@ -243,6 +247,7 @@ struct MerkleLevelsArgs {
 __global__ void __launch_bounds__(256) merkle_levels_kernel(MerkleLevelsArgs a, int levels, int m31_out) {
     __shared__ uint32_t sh[2][256][8];
     const size_t cta = blockIdx.x;
+    let_next_start();
     follow_previous();
     uint32_t h[8], m[16];
     {
@@ -449,15 +454,17 @@ int zkb_merkle_levels(zkb_ctx* ctx, int child_log, const uint32_t* children, int
     if (!ctx) return ZKB_EINVAL;
     ZKB_CHECK_ARG(ctx, children != nullptr && out_layers != nullptr && ((uintptr_t)children & 15) == 0);
     ZKB_CHECK_ARG(ctx, levels >= 1 && levels <= MERKLE_LEVELS_MAX && child_log >= 9 && child_log <= 31 && child_log - levels >= 0);
-    MerkleLevelsArgs a{};
-    a.children = children;
-    for (int j = 1; j <= levels; j++) {
-        ZKB_CHECK_ARG(ctx, out_layers[j - 1] != nullptr && ((uintptr_t)out_layers[j - 1] & 15) == 0);
-        a.out[j] = out_layers[j - 1];
-    }
+    for (int j = 1; j <= levels; j++) ZKB_CHECK_ARG(ctx, out_layers[j - 1] != nullptr && ((uintptr_t)out_layers[j - 1] & 15) == 0);
     DeviceGuard g(ctx);
-    ProfScope prof(ctx, "merkle_levels_kernel");
-    ZKB_CUDA(ctx, launch_following(ctx, merkle_levels_kernel, 1u << (child_log - 9), 256u, a, levels, m31_out));
+    for (int done = 0; done < levels;) {
+        const int log = child_log - done, left = levels - done, take = log >= MERKLE_LEVELS_SPLIT_LOG ? std::min(left, MERKLE_LEVELS_SPLIT) : left;
+        MerkleLevelsArgs a{};
+        a.children = done ? out_layers[done - 1] : children;
+        for (int j = 1; j <= take; j++) a.out[j] = out_layers[done + j - 1];
+        ProfScope prof(ctx, "merkle_levels_kernel");
+        ZKB_CUDA(ctx, launch_following(ctx, merkle_levels_kernel, 1u << (log - 9), 256u, a, take, m31_out));
+        done += take;
+    }
     return ZKB_OK;
 }
 
