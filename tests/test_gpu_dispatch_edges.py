@@ -133,3 +133,14 @@ def test_merkle_levels_around_the_split_launches(ctx, oracle, child_log, levels)
     for j, o in enumerate(outs, 1):
         below = oracle.commit_on_layer(child_log - j, below, [], m31=True)
         assert (o.download(shape=(-1, 8)) == below).all(), j
+
+
+@pytest.mark.parametrize("n_cols,log_n,blowup,shift,two", [(63, 19, 1, 0, 0), (64, 19, 1, 0, 0), (64, 18, 2, 0, 5), (64, 19, 1, 1, 0), (2100, 13, 2, 0, 0), (100, 19, 1, 2, 3)])
+def test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, log_n, blowup, shift, two):
+    # 64 entries and 2^25 words saved: the numerators come from the coefficients, unless these do not start on 16 bytes
+    trees = [[m31_column(7900 + c, 1 << log_n) for c in range(n_cols)]]
+    kw = dict(pow_bits=0, log_blowup=blowup, log_last_layer=0, n_queries=3, two_sample_every=two)
+    want = oracle.pcs_prove(trees, **kw)
+    buf = ctx.upload(np.concatenate([np.zeros(shift, np.uint32)] + trees[0]))
+    got = ctx.pcs_prove_device([[buf.ptr + 4 * (shift + (c << log_n)) for c in range(n_cols)]], [log_n] * n_cols, **kw)
+    assert len(got) == len(want) and (got == want).all()

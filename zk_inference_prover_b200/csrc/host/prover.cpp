@@ -920,7 +920,7 @@ struct CommitmentSchemeProver {
     // the columns' sizes and the sample points only, so it is made and uploaded while the samples are evaluated and hashed.
     struct Numerators {
         struct Group { uint32_t log; size_t first_col, n_cols, first_batch, n_batches; };
-        std::vector<const uint32_t*> cols;  // by ascending size, in their own order within a size
+        std::vector<const uint32_t*> cols, coeffs;  // evaluations and coefficients, by ascending size, in their own order within a size
         std::vector<Group> groups;
         zk::NumeratorEntries entries;       // batch after batch
         std::vector<zk::NumeratorBatch> batches;
@@ -933,14 +933,17 @@ struct CommitmentSchemeProver {
         Numerators nu;
         nu.points = sp.points;
         const size_t n_cols = sp.first.size() - 1;
-        std::vector<const BaseColumn*> flat;
+        std::vector<const BaseColumn*> flat, flat_coeffs;
         std::vector<uint8_t> logs;
         flat.reserve(n_cols);
+        flat_coeffs.reserve(n_cols);
         logs.reserve(n_cols);
         size_t first_of[34] = {0};
         for (auto& t : trees)
-            for (auto& e : t.evals) {
+            for (size_t c = 0; c < t.evals.size(); c++) {
+                const BaseColumn& e = t.evals[c];
                 flat.push_back(&e);
+                flat_coeffs.push_back(&t.coeffs[c]);
                 logs.push_back((uint8_t)std::min<uint32_t>(e.log_size(), 32));
                 first_of[logs.back() + 1]++;
             }
@@ -975,6 +978,7 @@ struct CommitmentSchemeProver {
         std::vector<Raw> raw;
         raw.reserve(n_pows);
         nu.cols.reserve(n_cols);
+        nu.coeffs.reserve(n_cols);
         std::vector<uint32_t> batch_of;  // per point, within the size at hand; ~0: none yet
         for (size_t i = 0; i < n_cols;) {
             const uint32_t log = logs[order[i]];
@@ -984,6 +988,7 @@ struct CommitmentSchemeProver {
                 const uint32_t c = order[i];
                 const uint32_t col = (uint32_t)(nu.cols.size() - first_col);
                 nu.cols.push_back(flat[c]->ptr());
+                nu.coeffs.push_back(flat_coeffs[c]->ptr());
                 uint32_t pow = first_pow[c];
                 auto entry = [&](uint32_t point, size_t sample) {
                     if (point >= batch_of.size()) batch_of.resize(point + 1, ~0u);
@@ -1025,7 +1030,8 @@ struct CommitmentSchemeProver {
             for (size_t b = g.first_batch; b < g.first_batch + g.n_batches; b++) {
                 SecureColumnByCoords acc(d, (size_t)1 << g.log);
                 auto o = acc.ptrs();
-                d.check(zk::numerator_run(d.ctx(), nu.cols.data() + g.first_col, (int)g.n_cols, (int)g.log, nu.lines, nu.batches[b], o.data()));
+                d.check(zk::numerator_run(d.ctx(), nu.cols.data() + g.first_col, nu.coeffs.data() + g.first_col, (int)g.n_cols, (int)g.log,
+                                          (int)(g.log - config.fri.log_blowup_factor), nu.lines, nu.batches[b], o.data()));
                 accs.push_back({nu.points[nu.batch_point[b]], std::move(acc), nu.batches[b].first_linear});
             }
         hc.reset(new HostClock("pcs.quot.combine"));

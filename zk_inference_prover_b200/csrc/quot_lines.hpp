@@ -32,6 +32,8 @@ struct NumeratorLines {
 int numerator_stage(zkb_ctx* ctx, const NumeratorEntries& e, const std::vector<NumeratorBatch>& batches, NumeratorLines& lines);
 int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<NumeratorBatch>& batches, NumeratorLines& lines, qm31 random_coeff,
                     const qm31* h_values, const uint32_t* d_values);
-int numerator_run(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const NumeratorLines& lines, const NumeratorBatch& batch, uint32_t* const out[4]);
+// cols: the columns' 2^log_n evaluations; coeffs: the 2^log_coeff coefficients they are the extension of.
+int numerator_run(zkb_ctx* ctx, const uint32_t* const* cols, const uint32_t* const* coeffs, int ncols, int log_n, int log_coeff, const NumeratorLines& lines,
+                  const NumeratorBatch& batch, uint32_t* const out[4]);
 
 }  // namespace zk

@@ -32,12 +32,12 @@ constexpr int NUM_TILE = 128;
 template <int R>
 __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* const* __restrict__ cols,
                                                               const uint32_t* __restrict__ col_idx,
-                                                              const uint4* __restrict__ coeff_c, int k, qm31 b_sum,
+                                                              const uint4* __restrict__ coeff_c, int k, qm31 b_sum, int b_first,
                                                               size_t n, Secure4 out, int chunk = 0,
                                                               uint32_t* __restrict__ partial = nullptr) {
     // With `partial`, CTA row blockIdx.y takes the columns [y * chunk, (y + 1) * chunk) and leaves its reduced sums in
     // partial[(y * 4 + coordinate) * n + row]; quot_partial_sum_kernel adds the rows up. Short, wide groups (thousands of
-    // columns of a few hundred rows) would otherwise run on one or two CTAs.
+    // columns of a few hundred rows) would otherwise run on one or two CTAs. b_first: b_sum is taken off row 0 only.
     const int k_begin = partial ? (int)blockIdx.y * chunk : 0;
     const int k_end = partial ? (k_begin + chunk < k ? k_begin + chunk : k) : k;
     __shared__ const uint32_t* s_col[NUM_TILE];
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
 #pragma unroll
     for (int r = 0; r < R; r++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) res[r][q] = partial ? m31_reduce64(acc[r][q]) : m31_sub(m31_reduce64(acc[r][q]), b_sum.c[q]);
+        for (int q = 0; q < 4; q++) res[r][q] = partial ? m31_reduce64(acc[r][q]) : m31_sub(m31_reduce64(acc[r][q]), b_first && row0 + r ? 0u : b_sum.c[q]);
     if (partial) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
@@ -120,14 +120,14 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
 }
 
 // out[q][row] = sum over the S column chunks of partial[(s * 4 + q) * n + row], minus b_sum.
-__global__ void __launch_bounds__(256) quot_partial_sum_kernel(const uint32_t* __restrict__ partial, int S, size_t n, qm31 b_sum, Secure4 out) {
+__global__ void __launch_bounds__(256) quot_partial_sum_kernel(const uint32_t* __restrict__ partial, int S, size_t n, qm31 b_sum, int b_first, Secure4 out) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over 4 * n (coordinate-major)
     if (i >= 4 * n) return;
     const int q = (int)(i / n);
     const size_t row = i - (size_t)q * n;
     uint64_t acc = 0;
     for (int s = 0; s < S; s++) acc += partial[((size_t)s * 4 + q) * n + row];  // 31-bit terms: the 64-bit sum cannot overflow
-    out.c[q][row] = m31_sub(m31_reduce64(acc), b_sum.c[q]);
+    out.c[q][row] = m31_sub(m31_reduce64(acc), b_first && row ? 0u : b_sum.c[q]);
 }
 
 constexpr int MAX_ACCS = 8;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(256) quot_lines_kernel(const LineChunk* __rest
 
 // The kernels of one accumulation. d_cols: the columns' staged table; scratch_used: words of the scratch buffer that hold its inputs.
 static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const uint32_t* const* d_cols, const uint32_t* d_idx,
-                             const uint32_t* d_c, int k, qm31 b_sum, Secure4 o, size_t scratch_used) {
+                             const uint32_t* d_c, int k, qm31 b_sum, int b_first, Secure4 o, size_t scratch_used) {
     size_t n = (size_t)1 << log_n;
     bool wide = n >= 4;
     for (int q = 0; q < 4; q++) wide = wide && ((uintptr_t)o.c[q] & 15) == 0;
@@ -303,21 +303,21 @@ static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncol
         dim3 grid(row_blocks, (unsigned)S);
         if (wide)
             quot_numerators_kernel<4><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, n, o, chunk, partial);
+                                                                     b_sum, b_first, n, o, chunk, partial);
         else
             quot_numerators_kernel<2><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, n, o, chunk, partial);
+                                                                     b_sum, b_first, n, o, chunk, partial);
         ZKB_LAUNCH_CHECK(ctx);
-        quot_partial_sum_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, o);
+        quot_partial_sum_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, b_first, o);
         ZKB_LAUNCH_CHECK(ctx);
         return ZKB_OK;
     }
     if (wide)
         quot_numerators_kernel<4><<<(unsigned)((n / 4 + 255) / 256), 256, 0, ctx->stream>>>(
-            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
+            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, b_first, n, o);
     else
         quot_numerators_kernel<2><<<(unsigned)((n / 2 + 255) / 256), 256, 0, ctx->stream>>>(
-            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, n, o);
+            d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k, b_sum, b_first, n, o);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
 }
@@ -433,15 +433,40 @@ int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<Numerat
     return ZKB_OK;
 }
 
-int numerator_run(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, int log_n, const NumeratorLines& lines, const NumeratorBatch& batch, uint32_t* const out[4]) {
+// The combination of the columns' polynomials is itself a polynomial of their degree, so it can be taken of the coefficients, a
+// blow-up fewer of them, and extended: four columns' worth of transform in the place of most of the reading. (The constant comes off
+// coefficient 0, whose basis element is 1.) 256 columns of 2^20 at blow-up 4: 810 us from the evaluations, 229 + 86 from the coefficients.
+// The transform costs as much as reading 27 columns' evaluations at that height and its launches some 10 us, which is 50 MB, so
+// narrow or short groups are read as they are; so are coefficients that do not start on 16 bytes.
+static bool numerators_of_coeffs(const uint32_t* const* coeffs, int ncols, int log_n, int log_coeff, size_t k) {
+    if (k < 64 || (k << log_n) - (k << log_coeff) < ((size_t)1 << 25)) return false;
+    for (int c = 0; c < ncols; c++) if (((uintptr_t)coeffs[c] & 15) != 0) return false;
+    return true;
+}
+
+int numerator_run(zkb_ctx* ctx, const uint32_t* const* cols, const uint32_t* const* coeffs, int ncols, int log_n, int log_coeff, const NumeratorLines& lines,
+                  const NumeratorBatch& batch, uint32_t* const out[4]) {
     DeviceGuard g(ctx);
-    Secure4 o;
-    for (int q = 0; q < 4; q++) o.c[q] = out[q];
+    const bool of_coeffs = numerators_of_coeffs(coeffs, ncols, log_n, log_coeff, batch.count);
+    if (of_coeffs) {
+        cols = coeffs;
+        ZKB_CHECK_ARG(ctx, log_coeff >= 2 && log_coeff < log_n && log_n <= ctx->max_log);
+    }
     for (int c = 0; c < ncols; c++) ZKB_CHECK_ARG(ctx, cols[c] != nullptr && ((uintptr_t)cols[c] & 7) == 0);
     void** d_cols;
     if (int rc = stage_ptrs(ctx, (const void* const*)cols, ncols, &d_cols)) return rc;
-    return launch_numerators(ctx, cols, ncols, log_n, (const uint32_t* const*)d_cols, lines.d_col + batch.first, lines.d_c + 4 * batch.first, (int)batch.count,
-                             batch.b_sum, o, 0);
+    const size_t n = (size_t)1 << log_coeff;
+    uint32_t* combined = nullptr;
+    if (of_coeffs)
+        if (int rc = zkb_malloc(ctx, 16 * n, (void**)&combined)) return rc;
+    Secure4 o;
+    for (int q = 0; q < 4; q++) o.c[q] = of_coeffs ? combined + q * n : out[q];
+    int rc = launch_numerators(ctx, cols, ncols, of_coeffs ? log_coeff : log_n, (const uint32_t* const*)d_cols, lines.d_col + batch.first,
+                               lines.d_c + 4 * batch.first, (int)batch.count, batch.b_sum, of_coeffs ? 1 : 0, o, 0);
+    if (!of_coeffs) return rc;
+    if (rc == ZKB_OK) rc = zkb_lde_cols(ctx, o.c, 4, log_coeff, out, log_n);
+    zkb_free(ctx, combined);
+    return rc;
 }
 
 }  // namespace zk
@@ -476,7 +501,7 @@ int zkb_quot_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncols, in
         ZKB_CUDA(ctx, cudaMemcpyAsync(d_c, h_c, (size_t)k * 16, cudaMemcpyHostToDevice, ctx->stream));
         ZKB_CUDA(ctx, cudaMemcpyAsync(d_idx, h_col_idx, (size_t)k * 4, cudaMemcpyHostToDevice, ctx->stream));
     }
-    return launch_numerators(ctx, cols, ncols, log_n, (const uint32_t* const*)d_cols, d_idx, d_c, k, b_sum, o, (size_t)5 * k);
+    return launch_numerators(ctx, cols, ncols, log_n, (const uint32_t* const*)d_cols, d_idx, d_c, k, b_sum, 0, o, (size_t)5 * k);
 }
 
 int zkb_quot_combine(zkb_ctx* ctx, int n_acc, const uint32_t* const* acc_cols, const int* h_acc_log,
