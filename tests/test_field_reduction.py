@@ -80,3 +80,24 @@ def test_product_at_the_top_of_the_range_on_the_device(ctx):
     dst = ctx.alloc(4)
     ctx.mle_fix_qm31(src.ptr, 2, np.array(X, np.uint32), dst.ptr)
     assert dst.download().tolist() == _mul(X, Y)
+
+
+SIGNED = SHARED + """
+extern "C" unsigned mul_signed(unsigned v, unsigned t) { return m31_mul_signed(v, m31_twice_signed(t)); }
+extern "C" unsigned unsign(unsigned v) { return m31_unsign(v); }
+"""
+
+
+def test_signed_product_stays_in_range_and_in_its_class(tmp_path):
+    (tmp_path / "s.cpp").write_text(SIGNED)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", str(tmp_path / "s.so"), str(tmp_path / "s.cpp")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "s.so"))
+    lib.mul_signed.restype = lib.unsign.restype = ctypes.c_uint32
+    half = 1 << 30
+    rng = np.random.default_rng(3)
+    vs = [-P, 1 - P, 2 - P, -half - 1, -half, 1 - half, -1, 0, 1, half - 1, half, half + 1, P - 1, P] + [int(x) for x in rng.integers(-P, P + 1, 200)]
+    ts = [0, 1, half - 2, half - 1, half, half + 1, P - 2, P - 1] + [int(x) for x in rng.integers(0, P, 100)]
+    for v in vs:
+        for t in ts:
+            q = lib.mul_signed(ctypes.c_uint32(v & 0xffffffff), ctypes.c_uint32(t))
+            assert -P <= q - ((q >> 31) << 32) <= P - 1 and lib.unsign(ctypes.c_uint32(q)) == v * t % P

@@ -19,7 +19,7 @@ struct zkb_ctx {
     uint32_t* tw = nullptr;
     uint32_t* itw = nullptr;
     size_t tw_len = 0;
-    // The same two towers with every word doubled (2t < 2^32): what the radix-32 butterflies multiply by.
+    // The same two towers with every word as twice its signed representative (m31_twice_signed): what the radix-32 butterflies multiply by.
     uint32_t* tw2 = nullptr;
     uint32_t* itw2 = nullptr;
     // One word the kernels with bounded waits set when a wait ran out (0 = none); read by zkb_sync.

@@ -178,9 +178,9 @@ __global__ void twiddle_tower_kernel(uint32_t* __restrict__ tw, uint32_t* __rest
     itw[t] = m31_inv(p.x);
 }
 
-__global__ void double_words_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, size_t len) {
+__global__ void twice_signed_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, size_t len) {
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < len) out[t] = in[t] << 1;
+    if (t < len) out[t] = m31_twice_signed(in[t]);
 }
 
 __global__ void gather_multi_kernel(const uint32_t* const* __restrict__ cols, int ncols, const uint32_t* __restrict__ idx,
@@ -283,8 +283,8 @@ int zkb_init(int device, int max_log_size, zkb_ctx** out) {
     if (cudaMemcpyToSymbolAsync(c_gen_pow2, g, sizeof(g), 0, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess) return fail(ZKB_ECUDA);
     unsigned blocks = (unsigned)((ctx->tw_len + 255) / 256);
     twiddle_tower_kernel<<<blocks, 256, 0, ctx->stream>>>(ctx->tw, ctx->itw, ctx->tw_len);
-    double_words_kernel<<<blocks, 256, 0, ctx->stream>>>(ctx->tw, ctx->tw2, ctx->tw_len);
-    double_words_kernel<<<blocks, 256, 0, ctx->stream>>>(ctx->itw, ctx->itw2, ctx->tw_len);
+    twice_signed_kernel<<<blocks, 256, 0, ctx->stream>>>(ctx->tw, ctx->tw2, ctx->tw_len);
+    twice_signed_kernel<<<blocks, 256, 0, ctx->stream>>>(ctx->itw, ctx->itw2, ctx->tw_len);
     if (cudaGetLastError() != cudaSuccess) return fail(ZKB_ECUDA);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fail(ZKB_ECUDA);
     *out = ctx;

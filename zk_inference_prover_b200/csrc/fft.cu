@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256, 2) butterfly_ceiling_kernel(uint32_t* __r
 #pragma unroll
     for (int i = 0; i < 32; i++) v[i] = tower[(threadIdx.x * 32 + i) & 1023] >> 1;
     const uint32_t* const tb[5] = {tw, tw + 16, tw + 24, tw + 28, tw + 30};
-    for (int r = 0; r < rounds; r++) radix32_stage<false, false, true>(v, tb, 0, 0, 5);
+    for (int r = 0; r < rounds; r++) radix32_stage<false, false>(v, tb, 0, 0, 5);
     uint32_t acc = 0;
 #pragma unroll
     for (int i = 0; i < 32; i++) acc ^= v[i];

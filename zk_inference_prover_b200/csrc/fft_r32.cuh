@@ -15,8 +15,12 @@
 //   strided pass (lo >= 3): a CTA of 256 threads owns 1024 rows x 8 consecutive words; thread
 //     (tm = tid / 8, w = tid % 8); global accesses are runs of 32 bytes.
 //
-// The butterfly multiplies by a pre-doubled twiddle: with t2 = 2t, the 64-bit product t2 * v splits
-// as hi = (t v) >> 31 and lo / 2 = (t v) mod 2^31, whose sum is congruent to t v and below 2p.
+// The butterflies multiply signed representatives by doubled signed twiddles (m31_mul_signed). The bound of these passes is the integer
+// ALU pipe (two cycles an instruction, and a wide product takes it once beside the four cycles it takes on the FMA-heavy pipe), so what
+// counts is the ALU instructions of a butterfly: in the forward direction the product's fold, its reduction and that of `a` (a half-range
+// each), and nothing for the outputs where the next layer adds them: it reduces a sum from [0, 2p) and a difference from (-p, p) alike. Only
+// a sum that the next layer multiplies costs one more, to be signed. The inverse direction multiplies the difference unreduced.
+// In a register-only loop a warp's butterfly takes a scheduler 9.6 cycles forward and 8.6 inverse; with canonical values throughout both take 10.4.
 #pragma once
 #include <type_traits>
 
@@ -24,26 +28,28 @@
 
 namespace zk {
 
-__device__ __forceinline__ uint32_t m31_mul_dbl(uint32_t v, uint32_t t2) {
-    uint64_t p = (uint64_t)v * t2;
-    uint32_t s = (uint32_t)(p >> 32) + ((uint32_t)p >> 1);
-    return umin32(s, s - P);
-}
+// How a forward butterfly's `a` comes: signed, in [-p, p], or an unreduced sum, in [0, 2p). `b` is always signed.
+enum : int { IN_SIGNED = 0, IN_SUM = 1 };
+// What becomes of its outputs: both signed; left as the sum and the difference they are, for the next layer to reduce (IN_SUM, IN_SIGNED);
+// canonical.
+enum : int { OUT_SIGNED = 0, OUT_RAW = 1, OUT_CANONICAL = 2 };
 
 // Forward: (a, b) -> (a + t b, a - t b); with NEG the twiddle is -t.
-template <bool NEG>
+template <bool NEG, int IN, int OUT>
 __device__ __forceinline__ void bf_fwd(uint32_t& a, uint32_t& b, uint32_t t2) {
-    uint32_t s = m31_mul_dbl(b, t2);
-    uint32_t x = m31_add(a, s), y = m31_sub(a, s);
-    a = NEG ? y : x;
-    b = NEG ? x : y;
+    static_assert(!NEG || OUT != OUT_RAW, "the next layer would take the difference for the sum");
+    const uint32_t r = m31_unsign(m31_mul_signed(b, t2)), c = IN == IN_SUM ? m31_reduce_sum(a) : m31_unsign(a);
+    const uint32_t sum = OUT == OUT_CANONICAL ? m31_reduce_sum(c + r) : OUT == OUT_SIGNED ? c + r - P : c + r;
+    const uint32_t diff = OUT == OUT_CANONICAL ? m31_unsign(c - r) : c - r;
+    a = NEG ? diff : sum;
+    b = NEG ? sum : diff;
 }
-// Inverse: (a, b) -> (a + b, (a - b) t); with NEG the twiddle is -t.
+// Inverse, canonical in and out: (a, b) -> (a + b, (a - b) t); with NEG the twiddle is -t.
 template <bool NEG>
 __device__ __forceinline__ void bf_inv(uint32_t& a, uint32_t& b, uint32_t t2) {
-    uint32_t d = NEG ? m31_sub(b, a) : m31_sub(a, b);
+    const uint32_t d = NEG ? b - a : a - b;
     a = m31_add(a, b);
-    b = m31_mul_dbl(d, t2);
+    b = m31_unsign(m31_mul_signed(d, t2));
 }
 
 // CNT consecutive twiddles, fetched with the widest loads (the tables are aligned to their length).
@@ -63,47 +69,68 @@ __device__ __forceinline__ void load_tw(const uint32_t* __restrict__ p, uint32_t
     }
 }
 
+// Layer JJ of N_LAYERS on the registers' index p (values v[(p << SUB) + j], j < 2^SUB): pairs p with p + 2^JJ, with the twiddles
+// t[p >> (JJ + 1)]. ALL: the stage's layers above ran right before, so that a forward `a` comes as they left it, and the layer below follows.
+template <bool INVERSE, bool ALL, int JJ, int N_LAYERS, int SUB, int LAST_OUT>
+__device__ __forceinline__ void register_layer(uint32_t (&v)[32], const uint32_t (&t)[16]) {
+#pragma unroll
+    for (int h = 0; h < ((1 << (N_LAYERS - 1)) >> JJ); h++) {
+#pragma unroll
+        for (int l = 0; l < (1 << JJ); l++) {
+            const int p0 = (h << (JJ + 1)) | l, p1 = p0 | (1 << JJ);
+#pragma unroll
+            for (int j = 0; j < (1 << SUB); j++) {
+                uint32_t &a = v[(p0 << SUB) + j], &b = v[(p1 << SUB) + j];
+                if constexpr (INVERSE) {
+                    bf_inv<false>(a, b, t[h]);
+                } else {
+                    const bool sum_in = ALL && JJ + 1 < N_LAYERS && !(h & 1);             // bit JJ + 1 of p0 is clear
+                    const bool raw_out = ALL && JJ > 0 && !((l >> (JJ > 0 ? JJ - 1 : 0)) & 1);  // bit JJ - 1 is: the next layer's `a`s
+                    constexpr int OUT = JJ == 0 ? LAST_OUT : (int)OUT_SIGNED;
+                    if (sum_in && raw_out) bf_fwd<false, IN_SUM, OUT_RAW>(a, b, t[h]);
+                    else if (sum_in) bf_fwd<false, IN_SUM, OUT>(a, b, t[h]);
+                    else if (raw_out) bf_fwd<false, IN_SIGNED, OUT_RAW>(a, b, t[h]);
+                    else bf_fwd<false, IN_SIGNED, OUT>(a, b, t[h]);
+                }
+            }
+        }
+    }
+}
+
 // Five layers on 32 registers. Layer jj pairs p with p + 2^jj and uses the 16 >> jj twiddles at
 // tb[jj] (global or shared memory): tb[jj][p >> (jj+1)].
 // Layers outside [act_lo, act_hi) (window-local numbering, this stage starts at `first`) are skipped.
 // When CIRCLE, layer jj = 0 is the circle layer (global layer 0): its twiddles are [y, -y, -x, x]
-// for each pair (x, y) of the eight layer-1 twiddles at tb[0] (cpu/circle.rs:312-332).
-// With DBL the table already holds doubled twiddles (2t) and nothing is shifted here.
-template <bool INVERSE, bool CIRCLE, bool DBL = false>
-__device__ __forceinline__ void radix32_stage(uint32_t (&v)[32], const uint32_t* const (&tb)[5], int first, int act_lo, int act_hi) {
+// for each pair (x, y) of the eight layer-1 twiddles at tb[0] (cpu/circle.rs:312-332), and the forward direction's outputs are
+// canonical; otherwise they are signed.
+template <bool INVERSE, bool CIRCLE, bool ALL>
+__device__ __forceinline__ void radix32_layers(uint32_t (&v)[32], const uint32_t* const (&tb)[5], int first, int act_lo, int act_hi) {
     uint32_t t[16];
     auto layer = [&](auto JJ) {
         constexpr int jj = decltype(JJ)::value;
-        if (first + jj < act_lo || first + jj >= act_hi) return;
+        if (!ALL && (first + jj < act_lo || first + jj >= act_hi)) return;
         if constexpr (CIRCLE && jj == 0) {
             load_tw<8>(tb[0], t);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const uint32_t x2 = DBL ? t[2 * q] : t[2 * q] << 1, y2 = DBL ? t[2 * q + 1] : t[2 * q + 1] << 1;
-                if (INVERSE) {
-                    bf_inv<false>(v[8 * q + 0], v[8 * q + 1], y2);
-                    bf_inv<true>(v[8 * q + 2], v[8 * q + 3], y2);
-                    bf_inv<true>(v[8 * q + 4], v[8 * q + 5], x2);
-                    bf_inv<false>(v[8 * q + 6], v[8 * q + 7], x2);
+                const uint32_t x2 = t[2 * q], y2 = t[2 * q + 1];
+                uint32_t* const w = v + 8 * q;
+                if constexpr (INVERSE) {
+                    bf_inv<false>(w[0], w[1], y2);
+                    bf_inv<true>(w[2], w[3], y2);
+                    bf_inv<true>(w[4], w[5], x2);
+                    bf_inv<false>(w[6], w[7], x2);
                 } else {
-                    bf_fwd<false>(v[8 * q + 0], v[8 * q + 1], y2);
-                    bf_fwd<true>(v[8 * q + 2], v[8 * q + 3], y2);
-                    bf_fwd<true>(v[8 * q + 4], v[8 * q + 5], x2);
-                    bf_fwd<false>(v[8 * q + 6], v[8 * q + 7], x2);
+                    constexpr int SUM = ALL ? IN_SUM : IN_SIGNED;
+                    bf_fwd<false, SUM, OUT_CANONICAL>(w[0], w[1], y2);
+                    bf_fwd<true, IN_SIGNED, OUT_CANONICAL>(w[2], w[3], y2);
+                    bf_fwd<true, SUM, OUT_CANONICAL>(w[4], w[5], x2);
+                    bf_fwd<false, IN_SIGNED, OUT_CANONICAL>(w[6], w[7], x2);
                 }
             }
         } else {
             load_tw<(16 >> jj)>(tb[jj], t);
-#pragma unroll
-            for (int h = 0; h < (16 >> jj); h++) {
-                const uint32_t t2 = DBL ? t[h] : t[h] << 1;
-#pragma unroll
-                for (int l = 0; l < (1 << jj); l++) {
-                    const int p0 = (h << (jj + 1)) | l, p1 = p0 | (1 << jj);
-                    if (INVERSE) bf_inv<false>(v[p0], v[p1], t2);
-                    else bf_fwd<false>(v[p0], v[p1], t2);
-                }
-            }
+            register_layer<INVERSE, ALL, jj, 5, 0, OUT_SIGNED>(v, t);
         }
     };
     if (INVERSE) {
@@ -113,6 +140,11 @@ __device__ __forceinline__ void radix32_stage(uint32_t (&v)[32], const uint32_t*
         layer(std::integral_constant<int, 4>{}); layer(std::integral_constant<int, 3>{}); layer(std::integral_constant<int, 2>{});
         layer(std::integral_constant<int, 1>{}); layer(std::integral_constant<int, 0>{});
     }
+}
+template <bool INVERSE, bool CIRCLE>
+__device__ __forceinline__ void radix32_stage(uint32_t (&v)[32], const uint32_t* const (&tb)[5], int first, int act_lo, int act_hi) {
+    if (act_lo <= first && act_hi >= first + 5) radix32_layers<INVERSE, CIRCLE, true>(v, tb, first, act_lo, act_hi);
+    else radix32_layers<INVERSE, CIRCLE, false>(v, tb, first, act_lo, act_hi);
 }
 
 // ---- asynchronous global -> shared copies (16 bytes each), grouped and waited on per thread
@@ -247,7 +279,7 @@ __global__ void __launch_bounds__(32 * R32_CONTIG_WARPS, 16 / R32_CONTIG_WARPS)
         if (!INVERSE) {
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
-            radix32_stage<false, false, true>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
+            radix32_stage<false, false>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) s[R32_PITCH * p + tm] = v[p];  // the words this lane read itself
             __syncwarp();
@@ -256,7 +288,7 @@ __global__ void __launch_bounds__(32 * R32_CONTIG_WARPS, 16 / R32_CONTIG_WARPS)
                 uint4 x = row[q];
                 v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
             }
-            radix32_stage<false, true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
+            radix32_stage<false, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int q = 0; q < 8; q++) row[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             __syncwarp();
@@ -273,13 +305,13 @@ __global__ void __launch_bounds__(32 * R32_CONTIG_WARPS, 16 / R32_CONTIG_WARPS)
                 uint4 x = row[q];
                 v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
             }
-            radix32_stage<true, true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
+            radix32_stage<true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int q = 0; q < 8; q++) row[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             __syncwarp();
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
-            radix32_stage<true, false, true>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
+            radix32_stage<true, false>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) dst[base + tm + 32 * p] = scale ? m31_mul(v[p], scale) : v[p];
         }
@@ -308,34 +340,25 @@ constexpr int R32_WIDE_TW = 256;         // [0,128) [128,192) [192,224): layers 
 __host__ __device__ constexpr size_t r32_wide_smem() { return (size_t)(2 * R32_WIDE_TILE + R32_WIDE_TW) * sizeof(uint32_t); }
 
 // Three layers over the row index q of v[4 q + j] (eight rows x four words). tw0: 4, tw1: 2, tw2: 1 doubled twiddles.
-template <bool INVERSE>
-__device__ __forceinline__ void radix8x4_stage(uint32_t (&v)[32], const uint32_t* tw0, const uint32_t* tw1, const uint32_t* tw2,
-                                               int act_lo, int act_hi) {
+template <bool INVERSE, bool ALL>
+__device__ __forceinline__ void radix8x4_layers(uint32_t (&v)[32], const uint32_t* tw0, const uint32_t* tw1, const uint32_t* tw2, int act_lo, int act_hi) {
+    uint32_t t[16];
     auto layer = [&](auto JJ, const uint32_t* tw) {
         constexpr int jj = decltype(JJ)::value;
-        if (jj < act_lo || jj >= act_hi) return;
-        uint32_t t[4];
-        if constexpr (jj == 0) { uint4 x = *reinterpret_cast<const uint4*>(tw); t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w; }
-        else if constexpr (jj == 1) { uint2 x = *reinterpret_cast<const uint2*>(tw); t[0] = x.x; t[1] = x.y; }
-        else t[0] = tw[0];
-#pragma unroll
-        for (int h = 0; h < (4 >> jj); h++) {
-#pragma unroll
-            for (int l = 0; l < (1 << jj); l++) {
-                const int q0 = (h << (jj + 1)) | l, q1 = q0 | (1 << jj);
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    if (INVERSE) bf_inv<false>(v[4 * q0 + j], v[4 * q1 + j], t[h]);
-                    else bf_fwd<false>(v[4 * q0 + j], v[4 * q1 + j], t[h]);
-                }
-            }
-        }
+        if (!ALL && (jj < act_lo || jj >= act_hi)) return;
+        load_tw<(4 >> jj)>(tw, t);
+        register_layer<INVERSE, ALL, jj, 3, 2, OUT_SIGNED>(v, t);
     };
     if (INVERSE) {
         layer(std::integral_constant<int, 0>{}, tw0); layer(std::integral_constant<int, 1>{}, tw1); layer(std::integral_constant<int, 2>{}, tw2);
     } else {
         layer(std::integral_constant<int, 2>{}, tw2); layer(std::integral_constant<int, 1>{}, tw1); layer(std::integral_constant<int, 0>{}, tw0);
     }
+}
+template <bool INVERSE>
+__device__ __forceinline__ void radix8x4_stage(uint32_t (&v)[32], const uint32_t* tw0, const uint32_t* tw1, const uint32_t* tw2, int act_lo, int act_hi) {
+    if (act_lo <= 0 && act_hi >= 3) radix8x4_layers<INVERSE, true>(v, tw0, tw1, tw2, act_lo, act_hi);
+    else radix8x4_layers<INVERSE, false>(v, tw0, tw1, tw2, act_lo, act_hi);
 }
 
 template <bool INVERSE>
@@ -423,7 +446,7 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
         if (!INVERSE) {
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[32 * (warp + 8 * p) + lane];
-            radix32_stage<false, false, true>(v, tb_uni, 3, ps.act_lo, ps.act_hi);
+            radix32_stage<false, false>(v, tb_uni, 3, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) s[32 * (warp + 8 * p) + lane] = v[p];  // the words this thread read itself
             __syncthreads();
@@ -450,7 +473,7 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
             __syncthreads();
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[32 * (warp + 8 * p) + lane];
-            radix32_stage<true, false, true>(v, tb_uni, 3, ps.act_lo, ps.act_hi);
+            radix32_stage<true, false>(v, tb_uni, 3, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) dst[(base | ((warp + 8 * p) << ps.lo)) + lane] = scale ? m31_mul(v[p], scale) : v[p];
         }
@@ -521,8 +544,15 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
             const int pos = R32_PITCH * (o >> 5) + (o & 31);
             uint32_t x0 = s[pos], x1 = s[BLK + pos], x2 = s[2 * BLK + pos], x3 = s[3 * BLK + pos];
             if (!INVERSE) {
-                if (on11) { bf_fwd<false>(x0, x2, t11); bf_fwd<false>(x1, x3, t11); }
-                if (on10) { bf_fwd<false>(x0, x1, t10a); bf_fwd<false>(x2, x3, t10b); }
+                if (on10 && on11) {
+                    bf_fwd<false, IN_SIGNED, OUT_RAW>(x0, x2, t11);
+                    bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1, x3, t11);
+                    bf_fwd<false, IN_SUM, OUT_SIGNED>(x0, x1, t10a);
+                    bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2, x3, t10b);
+                } else {
+                    if (on11) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0, x2, t11); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1, x3, t11); }
+                    if (on10) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0, x1, t10a); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2, x3, t10b); }
+                }
                 s[pos] = x0; s[BLK + pos] = x1; s[2 * BLK + pos] = x2; s[3 * BLK + pos] = x3;
             } else {
                 if (on10) { bf_inv<false>(x0, x1, t10a); bf_inv<false>(x2, x3, t10b); }
@@ -557,7 +587,7 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
             __syncthreads();
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
-            radix32_stage<false, false, true>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
+            radix32_stage<false, false>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) s[R32_PITCH * p + tm] = v[p];
             __syncwarp();
@@ -566,7 +596,7 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
                 uint4 x = row[q];
                 v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
             }
-            radix32_stage<false, true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
+            radix32_stage<false, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int q = 0; q < 8; q++) row[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             __syncwarp();
@@ -583,13 +613,13 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
                 uint4 x = row[q];
                 v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
             }
-            radix32_stage<true, true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
+            radix32_stage<true, true>(v, tb_lane, 0, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int q = 0; q < 8; q++) row[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             __syncwarp();
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
-            radix32_stage<true, false, true>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
+            radix32_stage<true, false>(v, tb_uni, 5, ps.act_lo, ps.act_hi);
 #pragma unroll
             for (int p = 0; p < 32; p++) s[R32_PITCH * p + tm] = v[p];
             __syncthreads();

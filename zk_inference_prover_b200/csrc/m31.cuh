@@ -42,6 +42,20 @@ ZK_HD uint32_t m31_mul(uint32_t a, uint32_t b) {
     return umin32(s, s - P);
 }
 ZK_HD uint32_t m31_sqr(uint32_t a) { return m31_mul(a, a); }
+
+// Signed representatives. A word read as a signed integer in [-p, p - 1] stands for its residue; one add-and-minimum brings it back to
+// [0, p) (m31_unsign), and a product takes it, or p, as it is.
+//
+// t2 is twice the representative of a factor in [-(2^30 - 1), 2^30 - 1] (m31_twice_signed). With v t2 + 2^31 = h 2^32 + l, l even,
+// v t = h 2^31 + l / 2 - 2^30, congruent to h - 2^30 + l / 2: one product with the constant in its addend, one shift-and-add. For v in
+// [-p, p] that lies in [-p, p - 1], since |v t2| <= (2^31 - 1) (2^31 - 2) puts h in [-2^30 + 1, 2^30 - 1].
+ZK_HD uint32_t m31_twice_signed(uint32_t t) { return 2 * t + (t >> 30 ? 2u : 0u); }
+ZK_HD uint32_t m31_mul_signed(uint32_t v, uint32_t t2) {
+    const int64_t p = (int64_t)(int32_t)v * (int32_t)t2 + (((int64_t)1 << 31) - ((int64_t)1 << 62));
+    return (uint32_t)((uint64_t)p >> 32) + ((uint32_t)p >> 1);
+}
+ZK_HD uint32_t m31_unsign(uint32_t v) { return umin32(v, v + P); }      // [-p, p - 1] -> [0, p)
+ZK_HD uint32_t m31_reduce_sum(uint32_t v) { return umin32(v, v - P); }  // [0, 2p - 1] -> [0, p)
 ZK_HD uint32_t m31_sqn(uint32_t v, int n) { for (int i = 0; i < n; i++) v = m31_sqr(v); return v; }
 // v^(p-2): 37 multiplications, the addition chain of m31.rs:192-200.
 ZK_HD uint32_t m31_inv(uint32_t v) {
