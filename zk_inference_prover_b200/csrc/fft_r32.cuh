@@ -381,6 +381,10 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
     const size_t stride = stationary ? gridDim.x / n_a : gridDim.x;
     size_t item = stationary ? blockIdx.x / n_a : blockIdx.x;
     const uint32_t a_fixed = blockIdx.x % n_a;
+    // A thread's addresses are one and a step, unless the source is shorter than the window (an extension of few coefficients) or the
+    // destination lies in row blocks: an address apiece is a tenth of a pass's instructions.
+    const bool whole_rows = (src_mask >> (ps.lo + 7)) != 0;
+    const size_t row_step = (size_t)32 << ps.lo;
 
     auto decode = [&](size_t it, uint32_t& col, uint32_t& a) {
         uint32_t wb;
@@ -401,11 +405,14 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
         uint32_t col, a;
         const uint32_t base = decode(it, col, a);
         const uint32_t* __restrict__ src = src_cols[col];
+        const uint32_t m = threadIdx.x >> 3, q = threadIdx.x & 7;  // 16-byte chunks: rows m + 32 k, part q
+        if (whole_rows) {
+            const uint32_t* p = src + ((base & src_mask) | (m << ps.lo) | (q << 2));
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t ch = k * 256 + threadIdx.x;  // 16-byte chunk: row ch / 8, part ch % 8
-            const uint32_t m = ch >> 3, q = ch & 7;
-            cp_async16(buf + 32 * m + 4 * q, src + ((base | (m << ps.lo) | (q << 2)) & src_mask));
+            for (int k = 0; k < 8; k++, p += row_step) cp_async16(buf + 1024 * k + 4 * threadIdx.x, p);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) cp_async16(buf + 1024 * k + 4 * threadIdx.x, src + ((base | ((m + 32 * k) << ps.lo) | (q << 2)) & src_mask));
         }
     };
     auto load_twiddles = [&](uint32_t a) {
@@ -456,10 +463,16 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
                 v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
             }
             radix8x4_stage<false>(v, tw + 4 * R, tw + 128 + 2 * R, tw + 192 + R, ps.act_lo, ps.act_hi);
+            if (rb.log >= 31) {
+                uint32_t* p = dst + ((base | ((8 * R) << ps.lo)) + 4 * c);
 #pragma unroll
-            for (int q = 0; q < 8; q++)
-                *reinterpret_cast<uint4*>(dst + blocked(base | ((8 * R + q) << ps.lo), rb) + 4 * c) =
-                    make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                for (int q = 0; q < 8; q++, p += row_step / 32) *reinterpret_cast<uint4*>(p) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    *reinterpret_cast<uint4*>(dst + blocked(base | ((8 * R + q) << ps.lo), rb) + 4 * c) =
+                        make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            }
         } else {
 #pragma unroll
             for (int q = 0; q < 8; q++) {
@@ -474,8 +487,9 @@ __global__ void __launch_bounds__(256, R32_WIDE_CTAS)
 #pragma unroll
             for (int p = 0; p < 32; p++) v[p] = s[32 * (warp + 8 * p) + lane];
             radix32_stage<true, false>(v, tb_uni, 3, ps.act_lo, ps.act_hi);
+            uint32_t* at = dst + ((base | (warp << ps.lo)) + lane);
 #pragma unroll
-            for (int p = 0; p < 32; p++) dst[(base | ((warp + 8 * p) << ps.lo)) + lane] = scale ? m31_mul(v[p], scale) : v[p];
+            for (int p = 0; p < 32; p++, at += row_step / 4) *at = scale ? m31_mul(v[p], scale) : v[p];
         }
         cur ^= 1;
     }
@@ -508,6 +522,10 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
     const size_t total = (size_t)ncols << unit_bits, stride = gridDim.x;
     size_t item = blockIdx.x;
 
+    // of the twiddles of layers 3..9, which a thread has one chunk of: where it lies in the tower for unit 0, and the layer's units' distance
+    const int jj_above = tid < 127 ? 9 - (31 - __clz(127 - tid)) : 9;
+    const uint32_t tw_above = (1u << (dom_log - jj_above - 1)) + 4 * (tid - (128 - (512 >> (jj_above - 1))));
+    const int tw_shift = 11 - jj_above;
     auto prefetch = [&](int b, size_t it) {
         uint32_t* buf = buf0 + b * BUF;
         const uint32_t* __restrict__ src = src_cols[it >> unit_bits];
@@ -515,24 +533,26 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
         const uint32_t base = un << 12;
         // an in-place pass over a column laid out in row blocks reads the unit where the pass before it wrote it
         const uint32_t* __restrict__ usrc = src_blocked ? src + blocked(base, rb) - base : src;
+        // 16-byte chunks k * NT + tid: block ch / 256, row (ch / 8) % 32, part ch % 8
+        uint32_t* const to = buf + R32_PITCH * (tid >> 3) + 4 * (tid & 7);
+        if (src_mask >= 4095u) {
+            const uint32_t* const p = usrc + ((base & src_mask) + 4 * tid);
 #pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int ch = k * NT + tid;  // 16-byte chunk: block ch / 256, row (ch / 8) % 32, part ch % 8
-            const int blk = ch >> 8, r = (ch >> 3) & 31, q = ch & 7;
-            cp_async16(buf + blk * BLK + R32_PITCH * r + 4 * q, usrc + ((base + (blk << 10) + 32 * r + 4 * q) & src_mask));
-        }
-        uint32_t* tw = tw0 + b * R32_C12_TW;
+            for (int k = 0; k < 8; k++) cp_async16(to + (k >> 1) * BLK + (k & 1) * 16 * R32_PITCH, p + 4 * NT * k);
+        } else {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int ch = k * NT + tid;  // chunk of layers 1..9: layer jj holds 256 >> (jj - 1) chunks
-            if (ch < 511) {
-                const int jj = 9 - (31 - __clz(511 - ch));
-                const int cc = ch - (512 - (512 >> (jj - 1)));
-                cp_async16(tw + 4 * ch, tower + (1u << (dom_log - jj - 1)) + (un << (11 - jj)) + 4 * cc);
-            }
+            for (int k = 0; k < 8; k++) cp_async16(to + (k >> 1) * BLK + (k & 1) * 16 * R32_PITCH, usrc + ((base + 4 * (k * NT + tid)) & src_mask));
         }
-        if (tid < 2) cp_async4(tw + 2044 + tid, tower + (1u << (dom_log - 11)) + (un << 1) + tid);
-        else if (tid == 2) cp_async4(tw + 2046, tower + (1u << (dom_log - 12)) + un);
+        // chunks of layers 1..9: layer jj holds 256 >> (jj - 1), so a thread has two of layer 1, one of layer 2, one of those above
+        uint32_t* tw = tw0 + b * R32_C12_TW + 4 * tid;
+        const uint32_t* const t1 = tower + ((1u << (dom_log - 2)) + (un << 10) + 4 * tid);
+        cp_async16(tw, t1);
+        cp_async16(tw + 4 * NT, t1 + 4 * NT);
+        cp_async16(tw + 8 * NT, tower + ((1u << (dom_log - 3)) + (un << 9) + 4 * tid));
+        if (tid < 127) cp_async16(tw + 12 * NT, tower + (tw_above + (un << tw_shift)));
+        else if (tid == 127) cp_async4(tw + 12 * NT, tower + ((1u << (dom_log - 11)) + (un << 1)));
+        if (tid == 0) cp_async4(tw0 + b * R32_C12_TW + 2045, tower + ((1u << (dom_log - 11)) + (un << 1) + 1));
+        else if (tid == 32) cp_async4(tw0 + b * R32_C12_TW + 2046, tower + ((1u << (dom_log - 12)) + un));
     };
     // Layers 10 and 11 on the four blocks' words at offset o of a block.
     auto cross_blocks = [&](uint32_t* s, const uint32_t* tw, uint32_t* out, uint32_t out_scale) {
