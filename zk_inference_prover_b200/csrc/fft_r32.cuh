@@ -554,32 +554,40 @@ __global__ void __launch_bounds__(32 * R32_C12_WARPS, 4)
         if (tid == 0) cp_async4(tw0 + b * R32_C12_TW + 2045, tower + ((1u << (dom_log - 11)) + (un << 1) + 1));
         else if (tid == 32) cp_async4(tw0 + b * R32_C12_TW + 2046, tower + ((1u << (dom_log - 12)) + un));
     };
-    // Layers 10 and 11 on the four blocks' words at offset o of a block.
+    // Layers 10 and 11 on the four blocks' words at the same offset of a block, four words to an access.
     auto cross_blocks = [&](uint32_t* s, const uint32_t* tw, uint32_t* out, uint32_t out_scale) {
         const bool on10 = 10 >= ps.act_lo && 10 < ps.act_hi, on11 = 11 >= ps.act_lo && 11 < ps.act_hi;
         const uint32_t t10a = tw[2044], t10b = tw[2045], t11 = tw[2046];
+        uint32_t* const at = s + R32_PITCH * (tid >> 3) + 4 * (tid & 7);
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int o = tid + NT * i;
-            const int pos = R32_PITCH * (o >> 5) + (o & 31);
-            uint32_t x0 = s[pos], x1 = s[BLK + pos], x2 = s[2 * BLK + pos], x3 = s[3 * BLK + pos];
-            if (!INVERSE) {
-                if (on10 && on11) {
-                    bf_fwd<false, IN_SIGNED, OUT_RAW>(x0, x2, t11);
-                    bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1, x3, t11);
-                    bf_fwd<false, IN_SUM, OUT_SIGNED>(x0, x1, t10a);
-                    bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2, x3, t10b);
+        for (int i = 0; i < 2; i++) {
+            uint4* const c[4] = {reinterpret_cast<uint4*>(at + 16 * R32_PITCH * i), reinterpret_cast<uint4*>(at + 16 * R32_PITCH * i + BLK),
+                                 reinterpret_cast<uint4*>(at + 16 * R32_PITCH * i + 2 * BLK), reinterpret_cast<uint4*>(at + 16 * R32_PITCH * i + 3 * BLK)};
+            const uint4 l0 = *c[0], l1 = *c[1], l2 = *c[2], l3 = *c[3];
+            uint32_t x0[4] = {l0.x, l0.y, l0.z, l0.w}, x1[4] = {l1.x, l1.y, l1.z, l1.w}, x2[4] = {l2.x, l2.y, l2.z, l2.w}, x3[4] = {l3.x, l3.y, l3.z, l3.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (!INVERSE) {
+                    if (on10 && on11) {
+                        bf_fwd<false, IN_SIGNED, OUT_RAW>(x0[j], x2[j], t11);
+                        bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1[j], x3[j], t11);
+                        bf_fwd<false, IN_SUM, OUT_SIGNED>(x0[j], x1[j], t10a);
+                        bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2[j], x3[j], t10b);
+                    } else {
+                        if (on11) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0[j], x2[j], t11); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1[j], x3[j], t11); }
+                        if (on10) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0[j], x1[j], t10a); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2[j], x3[j], t10b); }
+                    }
                 } else {
-                    if (on11) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0, x2, t11); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x1, x3, t11); }
-                    if (on10) { bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x0, x1, t10a); bf_fwd<false, IN_SIGNED, OUT_SIGNED>(x2, x3, t10b); }
+                    if (on10) { bf_inv<false>(x0[j], x1[j], t10a); bf_inv<false>(x2[j], x3[j], t10b); }
+                    if (on11) { bf_inv<false>(x0[j], x2[j], t11); bf_inv<false>(x1[j], x3[j], t11); }
+                    if (out_scale) { x0[j] = m31_mul(x0[j], out_scale); x1[j] = m31_mul(x1[j], out_scale); x2[j] = m31_mul(x2[j], out_scale); x3[j] = m31_mul(x3[j], out_scale); }
                 }
-                s[pos] = x0; s[BLK + pos] = x1; s[2 * BLK + pos] = x2; s[3 * BLK + pos] = x3;
-            } else {
-                if (on10) { bf_inv<false>(x0, x1, t10a); bf_inv<false>(x2, x3, t10b); }
-                if (on11) { bf_inv<false>(x0, x2, t11); bf_inv<false>(x1, x3, t11); }
-                if (out_scale) { x0 = m31_mul(x0, out_scale); x1 = m31_mul(x1, out_scale); x2 = m31_mul(x2, out_scale); x3 = m31_mul(x3, out_scale); }
-                out[o] = x0; out[1024 + o] = x1; out[2048 + o] = x2; out[3072 + o] = x3;
             }
+            uint4* const to = reinterpret_cast<uint4*>(out + 512 * i + 4 * tid);
+            *(INVERSE ? to : c[0]) = make_uint4(x0[0], x0[1], x0[2], x0[3]);
+            *(INVERSE ? to + 256 : c[1]) = make_uint4(x1[0], x1[1], x1[2], x1[3]);
+            *(INVERSE ? to + 512 : c[2]) = make_uint4(x2[0], x2[1], x2[2], x2[3]);
+            *(INVERSE ? to + 768 : c[3]) = make_uint4(x3[0], x3[1], x3[2], x3[3]);
         }
     };
 
