@@ -89,6 +89,10 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
         for (int u = 0; u < 4; u++) next[u] = at[u] ? at[u][i] : 0u;
     };
     quad_make_schedule(sched, threadIdx.x, QUAD_THREADS);
+    __syncthreads();
+    uint32_t* const m = msg[threadIdx.x >> 2];
+    const QuadWords word(m, sched);
+    const QuadConst k;
     // A tree built layer by layer is a chain of launches of a microsecond or two: the next one may start now (programmatic dependent
     // launch) and wait here for this grid to end. (What that grid writes while this one already runs, the children and the columns, is
     // read by plain loads: a read-only load is for memory that nobody writes during a kernel's life.)
@@ -99,22 +103,19 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
     if (prev) cur = reinterpret_cast<const uint4*>(prev)[4 * (size_t)i + l];
     values();
     addresses(1);
-    __syncthreads();
-    const QuadConst k;
     uint2 h = make_uint2(k.h0, k.h1);
-    uint32_t* const m = msg[threadIdx.x >> 2];
 #pragma unroll 1
     for (int b = first; b < end; b++) {
         if (b > 0) cur = make_uint4(next[0], next[1], next[2], next[3]);
         *reinterpret_cast<uint4*>(m + 4 * l) = cur;
+        __syncwarp();
         if (b > 0) {
             values();
             addresses(b + 1);
         }
-        __syncwarp();
         const bool last = b + 1 == end;
         const uint32_t bytes = (prev ? 64u : 0u) + 4u * (uint32_t)(16 * b < ncols ? 16 * b : ncols);
-        h = b2s_compress_quad(h, m, sched, k, bytes, last ? 0xffffffffu : 0u);
+        h = b2s_compress_quad(h, word, k, bytes, last ? 0xffffffffu : 0u);
         __syncwarp();
     }
     if (live) {
@@ -303,11 +304,10 @@ __global__ void channel_mix_root_draw_kernel(uint32_t* __restrict__ chan, const 
 // The last (at most ten) layers of a tree in one CTA. Every level is written to its layer array and kept in shared memory
 // for the next one (a level read back from global memory costs an L2 round trip on top of the compression; ten levels are a
 // chain of ten dependent hashes either way, which is what bounds it). Levels of 2^8 and 2^9 nodes are a thread a node, bound by
-// issue; from 2^7 down a node is a quad's (channel.cuh), and the last four levels one warp's, without a CTA barrier. When `chan` is
-// given, that warp goes on with the channel step of a FRI layer (mix the root, draw the folding challenge), which would otherwise
-// be a launch of its own. With a thread a node throughout and the channel step on one thread: 19 us
-// for ten levels and the step, now 16 us.
-__global__ void __launch_bounds__(512) merkle_top_kernel(MerkleTopArgs a, int top_log, int m31_out, uint32_t* __restrict__ chan,
+// issue; from 2^7 down a node is a quad's (channel.cuh). When `chan` is
+// given, the last warp goes on with the channel step of a FRI layer (mix the root, draw the folding challenge), which would otherwise
+// be a launch of its own. Eight levels and the step: 14.0 us with the schedule looked up in shared memory and a handful of branches a level, now 12.7.
+__global__ void __launch_bounds__(512, 1) merkle_top_kernel(const __grid_constant__ MerkleTopArgs a, int top_log, int m31_out, uint32_t* __restrict__ chan,
                                                          uint32_t* __restrict__ alpha_out, uint32_t* __restrict__ root_copy) {
     __shared__ alignas(16) uint32_t sh[2][256 * PAIR_WORDS];
     __shared__ ChanSm ch;
@@ -347,23 +347,32 @@ __global__ void __launch_bounds__(512) merkle_top_kernel(MerkleTopArgs a, int to
         }
         __syncthreads();
     }
+    // A hash's way to the next level is shared memory and a barrier; it goes to the layer's array behind that. A warp without a hash at a level
+    // has none further up and leaves; quads of the last warp without one hash what is there, for nobody. (Every branch on the way is
+    // some 25 cycles of a level's 1,400.)
     const QuadConst k;
     const uint32_t node = tid >> 2;
+    QuadWords word(&sh[0][node * PAIR_WORDS], ch.sched);
+    uint32_t* const parent = &sh[0][pair_at(node)] + l;
+    if (warp * 8u >= (1u << lg)) return;
 #pragma unroll 1
-    for (; lg >= 0; lg--) {
-        if (lg <= 3 && warp) return;
-        if (warp * 8u < (1u << lg)) {
-            uint2 h = b2s_compress_quad(make_uint2(k.h0, k.h1), &sh[(lg + 1) & 1][node * PAIR_WORDS], ch.sched, k, 64u, 0xffffffffu);
-            if (m31_out) h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
-            if (node < (1u << lg)) {
-                uint32_t *const o = &sh[lg & 1][pair_at(node)], *const g = a.layer[lg] + 8 * (size_t)node;
-                o[l] = g[l] = h.x;
-                o[4 + l] = g[4 + l] = h.y;
-            }
+    while (true) {
+        uint32_t* const g = a.layer[lg] + 8 * (size_t)node + l;
+        uint32_t* const o = parent + (lg & 1) * (256 * PAIR_WORDS);
+        const bool live = node < (1u << lg);
+        word.at = ((lg + 1) & 1) * (uint32_t)sizeof(sh[0]);
+        uint2 h = b2s_compress_quad(make_uint2(k.h0, k.h1), word, k, 64u, 0xffffffffu);
+        if (m31_out) h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
+        o[0] = h.x;
+        o[4] = h.y;
+        __syncthreads();
+        if (live) {
+            g[0] = h.x;
+            g[4] = h.y;
         }
-        if (lg >= 4) __syncthreads();
-        else __syncwarp();
+        if (--lg < 0 || warp * 8u >= (1u << lg)) break;
     }
+    if (warp) return;
     if (!chan) return;
     if (lane < 8) {
         const uint32_t w = sh[0][lane];

@@ -39,6 +39,32 @@ __device__ __forceinline__ void quad_make_schedule(uint32_t* sched, int thread, 
 
 __device__ __forceinline__ void chan_make_schedule(ChanSm& s, int thread, int n_threads) { quad_make_schedule(s.sched, thread, n_threads); }
 
+// Where a lane finds its message words, in the order it takes them (word 4 r + u is the u-th of round r). By the schedule in shared memory,
+// wherever the message is:
+struct ScheduledWords {
+    const uint32_t *m, *sched;
+    __device__ __forceinline__ uint32_t operator()(int i) const {
+        const uint32_t off = sched[(i & ~3) + (threadIdx.x & 3)] >> (8 * (i & 3)) & 255u;
+        return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(m) + off);
+    }
+};
+// By addresses in registers, for a kernel whose quads keep to one place, or to places `at` bytes apart: an instruction and a load less a word,
+// and forty registers.
+struct QuadWords {
+    uint32_t address[40], at = 0;
+    // sched: quad_make_schedule's, behind a barrier
+    __device__ __forceinline__ QuadWords(const uint32_t* m, const uint32_t* sched) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(m);
+#pragma unroll
+        for (int r = 0; r < 10; r++) {
+            const uint32_t pk = sched[4 * r + (threadIdx.x & 3)];
+#pragma unroll
+            for (int u = 0; u < 4; u++) address[4 * r + u] = base + ((pk >> (8 * u)) & 255u);
+        }
+    }
+    __device__ __forceinline__ uint32_t operator()(int i) const { return *reinterpret_cast<const uint32_t*>(__cvta_shared_to_generic(address[i] + at)); }
+};
+
 // Where quads keep hashes of a tree level in shared memory: a pair of siblings is the 16-word message of their parent, the pairs are 20
 // words apart (16-byte aligned, and the eight quads of a warp read their messages from different banks).
 constexpr int PAIR_WORDS = 20;
@@ -59,12 +85,12 @@ struct QuadConst {
 };
 
 // Warp-collective compression: lane l of every quad holds h[l] in .x and h[4 + l] in .y. last: all ones for the last block.
-__device__ __forceinline__ uint2 b2s_compress_quad(uint2 h, const uint32_t* m, const uint32_t* sched, const QuadConst& k, uint32_t t, uint32_t last) {
+template <class Words>
+__device__ __forceinline__ uint2 b2s_compress_quad(uint2 h, const Words& word, const QuadConst& k, uint32_t t, uint32_t last) {
     const unsigned full = 0xffffffffu;
     const int l = threadIdx.x & 3, q = threadIdx.x & 28;
     const int up = q | ((l + 3) & 3), dn = q | ((l + 1) & 3);
     uint32_t a = h.x, b = h.y, c = k.c, d = k.d ^ (t & k.t_mask) ^ (last & k.last_mask);
-    auto word = [&](uint32_t off) { return *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(m) + (off & 255u)); };
 #define CHAN_HALF_G(rot1, rot2, x) \
     a = (a + (x)) + b;             \
     d = rot1(d ^ a);               \
@@ -84,8 +110,7 @@ __device__ __forceinline__ uint2 b2s_compress_quad(uint2 h, const uint32_t* m, c
     }
 #pragma unroll
     for (int r = 0; r < 10; r++) {
-        const uint32_t pk = sched[4 * r + l];
-        const uint32_t x0 = word(pk), x1 = word(pk >> 8), x2 = word(pk >> 16), x3 = word(pk >> 24);
+        const uint32_t x0 = word(4 * r), x1 = word(4 * r + 1), x2 = word(4 * r + 2), x3 = word(4 * r + 3);
         CHAN_HALF_G(rotr16, rotr12, x0)
         CHAN_HALF_G_X(x1, up, dn)
         CHAN_HALF_G(rotr16, rotr12, x2)
@@ -116,7 +141,7 @@ __device__ __forceinline__ void chan_step(ChanSm& s, int n, int draws, uint32_t*
     __syncwarp();
 #pragma unroll 1
     for (; block < end; block++) {
-        h = b2s_compress_quad(h, m, s.sched, k, block == 0 ? 64u : block == 1 ? total : 37u, block == 0 ? 0u : 0xffffffffu);
+        h = b2s_compress_quad(h, ScheduledWords{m, s.sched}, k, block == 0 ? 64u : block == 1 ? total : 37u, block == 0 ? 0u : 0xffffffffu);
         const uint32_t rx = reduce_word_m31(h.x), ry = reduce_word_m31(h.y);
         const bool first = block == 0, mixed = block == 1;
         h.x = first ? h.x : k.h0;

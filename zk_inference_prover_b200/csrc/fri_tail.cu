@@ -3,9 +3,9 @@
 // (mix, draw the folding challenge) and the fold.
 //
 // What bounds it: dependency depth. A layer of 2^l values is a chain of l + 1 tree levels and two channel compressions, each some
-// 0.9 us; at 2^10 values the leaves and the level above them are another 9 us of one SM's hashing. Levels of up to 2^7 hashes are
-// four lanes a hash, and the last four and the channel one warp's, without CTA barriers (as in merkle_top_kernel): nine layers
-// from 2^9 values 95 -> 85 us. As launches (fold and leaves, tree
+// 0.75 us; at 2^10 values the leaves and the level above them are another 9 us of one SM's hashing. Levels of up to 2^7 hashes are
+// four lanes a hash, their message's addresses in registers and no branch but the loop's on a hash's way to the next level: eight layers from
+// 2^10 values 91 -> 86 us. As launches (fold and leaves, tree
 // top with channel step) a layer also paid two launches, the gaps around them and a dozen allocations for its arrays: a ten-column
 // proof of 2^8 rows spent 190 us of device time in them and as much on the host. Layers stay in shared memory; what the decommitment
 // reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs.
@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
         ev[c * TAIL_N + r] = a.src[c][r];
     }
     __syncthreads();
+    QuadWords word(ha + PAIR_WORDS * quad, ch.sched);
     for (int k = 0; k < a.n_layers; k++) {
         const int log = a.first_log - k;
         uint32_t *cur = ha, *below = hb;
@@ -48,51 +49,66 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
         if (a.circle && k == 0) half_coset_point(itw, log, mine, ix, t);
         else t = itw[half + mine];  // T_log^-1 starts at 2^(log - 1)
         // leaves (level log) and nodes: one loop, so that the code of the hash is there once
+        int lv = log;
 #pragma unroll 1
-        for (int lv = log; lv >= 0; lv--) {
+        for (; lv >= 8; lv--) {
             uint32_t* const out = a.tree[k] + ((size_t)8 << lv);
             const bool leaf = lv == log;
-            if (lv >= 8) {
-                for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
-                    uint32_t h[8], m[16];
-                    blake2s_init(h);
+            for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
+                uint32_t h[8], m[16];
+                blake2s_init(h);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-                        if (!leaf) x = *reinterpret_cast<const uint4*>(below + PAIR_WORDS * i + 4 * q);
-                        else if (q == 0) x = make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
-                        m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
-                    }
-                    blake2s_compress(h, m, leaf ? 16u : 64u, true);
+                for (int q = 0; q < 4; q++) {
+                    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                    if (!leaf) x = *reinterpret_cast<const uint4*>(below + PAIR_WORDS * i + 4 * q);
+                    else if (q == 0) x = make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
+                    m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
+                }
+                blake2s_compress(h, m, leaf ? 16u : 64u, true);
 #pragma unroll
-                    for (int w = 0; w < 8; w++) h[w] = reduce_word_m31(h[w]);
-                    const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
-                    uint4 *const c = reinterpret_cast<uint4*>(cur + pair_at(i)), *const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
-                    c[0] = o[0] = lo;
-                    c[1] = o[1] = hi;
-                }
-            } else if (8 * warp < (1 << lv)) {
-                uint32_t* const m = below + PAIR_WORDS * quad;
-                const bool live = quad < (1 << lv);
-                if (leaf) {
-                    const uint32_t i = live ? quad : 0;
-                    *reinterpret_cast<uint4*>(m + 4 * l) = l ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
-                    __syncwarp();
-                }
-                uint2 h = b2s_compress_quad(make_uint2(qc.h0, qc.h1), m, ch.sched, qc, leaf ? 16u : 64u, 0xffffffffu);
-                h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
-                if (live) {
-                    uint32_t *const c = cur + pair_at(quad), *const o = out + 8 * quad;
-                    c[l] = o[l] = h.x;
-                    c[4 + l] = o[4 + l] = h.y;
-                }
+                for (int w = 0; w < 8; w++) h[w] = reduce_word_m31(h[w]);
+                const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
+                uint4 *const c = reinterpret_cast<uint4*>(cur + pair_at(i)), *const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
+                c[0] = o[0] = lo;
+                c[1] = o[1] = hi;
             }
             uint32_t* const swap = cur;
             cur = below;
             below = swap;
-            if (lv >= 4) __syncthreads();
-            else if (warp == 0) __syncwarp();
-            else break;
+            __syncthreads();
+        }
+        // From 2^7 hashes down four lanes a hash, as in merkle_top_kernel; warps that have one meet at a barrier of their own, the others wait for
+        // the challenge.
+        if (lv == log && 8 * warp < (1 << lv)) {
+            const uint32_t i = quad < (1 << lv) ? quad : 0;
+            *reinterpret_cast<uint4*>(below + PAIR_WORDS * quad + 4 * l) = l ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
+            __syncwarp();
+        }
+        if (8 * warp < (1 << lv)) {
+            uint32_t* const parent = ha + pair_at(quad) + l;
+            uint32_t* const mine_out = a.tree[k] + 8 * quad + l;
+            const uint32_t apart = (uint32_t)TAIL_PAIRS;
+            uint32_t side = below == ha ? 0u : 1u;  // which of the two the messages are in
+#pragma unroll 1
+            while (true) {
+                uint32_t* const o = mine_out + ((size_t)8 << lv);
+                const bool live = quad < (1 << lv);
+                const int meet = lv >= 3 ? 4 << lv : 32;
+                word.at = side * (apart * 4u);
+                side ^= 1u;
+                uint32_t* const c = parent + side * apart;
+                uint2 h = b2s_compress_quad(make_uint2(qc.h0, qc.h1), word, qc, lv == log ? 16u : 64u, 0xffffffffu);
+                h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
+                c[0] = h.x;
+                c[4] = h.y;
+                asm volatile("bar.sync 1, %0;" ::"r"(meet) : "memory");
+                if (live) {
+                    o[0] = h.x;
+                    o[4] = h.y;
+                }
+                if (--lv < 0 || 8 * warp >= (1 << lv)) break;
+            }
+            below = side ? hb : ha;
         }
         // the root is in warp 0's below[0, 8): mix it in, draw the challenge
         if (tid < 32) {
@@ -158,7 +174,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
         if (lane < 16) block[lane] = lane == 0 ? 0x12345678u : lane < 4 ? 0u : lane < 12 ? shifted : lane == 12 ? a.pow_bits : 0u;
         __syncwarp();
         const QuadConst q;
-        const uint2 h = b2s_compress_quad(make_uint2(q.h0, q.h1), block, ch.sched, q, 52u, 0xffffffffu);
+        const uint2 h = b2s_compress_quad(make_uint2(q.h0, q.h1), ScheduledWords{block, ch.sched}, q, 52u, 0xffffffffu);
         if (lane < 4) { a.out[16 + lane] = reduce_word_m31(h.x); a.out[20 + lane] = reduce_word_m31(h.y); }
     }
     if (lane < 8) a.out[lane] = ch.msg[lane];
