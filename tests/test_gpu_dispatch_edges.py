@@ -144,3 +144,28 @@ def test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, lo
     buf = ctx.upload(np.concatenate([np.zeros(shift, np.uint32)] + trees[0]))
     got = ctx.pcs_prove_device([[buf.ptr + 4 * (shift + (c << log_n)) for c in range(n_cols)]], [log_n] * n_cols, **kw)
     assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("log_n,n_cols", [(1, 40), (2, 31), (2, 32), (5, 600), (9, 33), (10, 1500), (13, 100), (19, 34)])
+def test_numerators_split_over_columns(ctx, oracle, log_n, n_cols):
+    # from 32 entries on and as long as the rows alone do not fill the GPU, in pieces of sixteen columns and more; 24 pieces are added up by
+    # eight warps
+    cols = [m31_column(8000 + c, 1 << log_n) for c in range(n_cols)]
+    point, values, rands = oracle.secure_circle_mul(24680), qm31_array(8101, n_cols), qm31_array(8102, n_cols)
+    want, _ = oracle.quot_numerators(cols, point, np.arange(n_cols, dtype=np.uint32), values, rands)
+    lc = np.stack([oracle.line_coeffs(point, values[k], rands[k]) for k in range(n_cols)])
+    bufs, outs = [ctx.upload(c) for c in cols], [ctx.alloc(1 << log_n) for _ in range(4)]
+    ctx.quot_numerators([b.ptr for b in bufs], log_n, np.arange(n_cols, dtype=np.uint32), lc[:, 1, :], lc[:, 2, :], [o.ptr for o in outs])
+    assert (np.stack([o.download() for o in outs]) == want).all()
+
+
+@pytest.mark.parametrize("n_acc", [1, 2, 3, 4, 5, 9])
+@pytest.mark.parametrize("log_n", [3, 4, 9])
+def test_quotients_combined_several_rows_a_thread(ctx, oracle, n_acc, log_n):
+    accs = [([m31_column(8200 + 10 * a + q, 1 << (log_n - a % 3)) for q in range(4)], log_n - a % 3) for a in range(n_acc)]
+    first, points = qm31_array(8300, n_acc), np.stack([oracle.secure_circle_mul(13579 + 977 * a) for a in range(n_acc)])
+    want = oracle.quot_combine([np.stack(c) for c, _ in accs], first, points, log_n)
+    keep = [[ctx.upload(x) for x in c] for c, _ in accs]
+    outs = [ctx.alloc(1 << log_n) for _ in range(4)]
+    ctx.quot_combine([b.ptr for k in keep for b in k], [lg for _, lg in accs], first, points, log_n, [o.ptr for o in outs])
+    assert (np.stack([o.download() for o in outs]) == want).all()

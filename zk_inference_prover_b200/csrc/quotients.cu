@@ -10,6 +10,7 @@
 // with p the row's domain point (prover/backend/cpu/quotients.rs:47-75). p comes from the twiddle
 // tower; the CM31 inverses of one row are taken with one M31 inversion (Montgomery's trick on the
 // norms), which is exact because inverses are unique.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -68,9 +69,9 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
     for (int tile0 = k_begin; tile0 < k_end; tile0 += NUM_TILE) {
         const int tk = k_end - tile0 < NUM_TILE ? k_end - tile0 : NUM_TILE;
         __syncthreads();
-        if ((int)threadIdx.x < tk) {
-            s_col[threadIdx.x] = cols[col_idx[tile0 + threadIdx.x]];
-            s_c[threadIdx.x] = coeff_c[tile0 + threadIdx.x];
+        for (int t = (int)threadIdx.x; t < tk; t += (int)blockDim.x) {
+            s_col[t] = cols[col_idx[tile0 + t]];
+            s_c[t] = coeff_c[tile0 + t];
         }
         __syncthreads();
         if (!live) continue;
@@ -119,14 +120,26 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
     }
 }
 
-// out[q][row] = sum over the S column chunks of partial[(s * 4 + q) * n + row], minus b_sum.
+// out[q][row] = sum over the S column chunks of partial[(s * 4 + q) * n + row], minus b_sum. PARTS warps share 32 of the 4 n words, a run of
+// chunks each: short groups have hundreds of chunks (one thread a word walked them for 18 us), tall ones a few and many words.
+template <int PARTS>
 __global__ void __launch_bounds__(256) quot_partial_sum_kernel(const uint32_t* __restrict__ partial, int S, size_t n, qm31 b_sum, int b_first, Secure4 out) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // over 4 * n (coordinate-major)
+    __shared__ uint64_t sums[8][32];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t i = ((size_t)blockIdx.x * (8 / PARTS) + warp / PARTS) * 32 + lane;  // over 4 * n (coordinate-major)
+    uint64_t acc = 0;
+    if (i < 4 * n)
+        for (int s = (int)(warp % PARTS); s < S; s += PARTS) acc += partial[(size_t)s * 4 * n + i];  // 31-bit terms: the 64-bit sum cannot overflow
+    if (PARTS > 1) {
+        sums[warp][lane] = acc;
+        __syncthreads();
+        if (warp % PARTS) return;
+#pragma unroll
+        for (int w = 1; w < PARTS; w++) acc += sums[warp + w][lane];
+    }
     if (i >= 4 * n) return;
     const int q = (int)(i / n);
     const size_t row = i - (size_t)q * n;
-    uint64_t acc = 0;
-    for (int s = 0; s < S; s++) acc += partial[((size_t)s * 4 + q) * n + row];  // 31-bit terms: the 64-bit sum cannot overflow
     out.c[q][row] = m31_sub(m31_reduce64(acc), b_first && row ? 0u : b_sum.c[q]);
 }
 
@@ -142,48 +155,61 @@ struct CombineArgs {
 
 // Rows [row_begin, row_begin + n_rows) of the lifting domain; the accumulations and `out` are indexed from row_begin
 // (a row shard holds only its own rows; the whole domain is row_begin = 0, n_rows = 2^lifting_log).
-__global__ void __launch_bounds__(256) quot_combine_kernel(CombineArgs a, int lifting_log, Secure4 out,
+//
+// Bound by its products, 37 of a row's 60 those of an inversion: a thread takes ROWS neighbouring rows of up to ACCS accumulations and inverts the
+// product of their norms once. One accumulation over 2^23 rows, a row a thread: 230 us, four: 115.
+template <int ACCS, int ROWS>
+__global__ void __launch_bounds__(256) quot_combine_kernel(const __grid_constant__ CombineArgs a, int lifting_log, Secure4 out,
                                                            const uint32_t* __restrict__ tw, size_t row_begin, size_t n_rows) {
-    const size_t local = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t local = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * ROWS;
     if (local >= n_rows) return;
-    const size_t row = row_begin + local;
-    uint32_t px, py;
-    half_coset_point(tw, lifting_log, (uint32_t)(row >> 1), px, py);
-    if (row & 1) py = m31_neg(py);  // odd rows hold the conjugate point
-    cm31 den[MAX_ACCS];
-    uint32_t norm[MAX_ACCS], pref[MAX_ACCS];
-    uint32_t run = 1u;
+    const size_t row0 = row_begin + local;
+    cm31 den[ACCS * ROWS];
+    uint32_t norm[ACCS * ROWS], pref[ACCS * ROWS], py[ROWS];
+    uint32_t run = 1u, px = 0u;
 #pragma unroll
-    for (int z = 0; z < MAX_ACCS; z++) {
-        if (z < a.n_acc) {
-            cm31 dx = {m31_sub(a.prx[z].a, px), a.prx[z].b};
-            cm31 dy = {m31_sub(a.pry[z].a, py), a.pry[z].b};
-            den[z] = cm31_sub(cm31_mul(dx, a.piy[z]), cm31_mul(dy, a.pix[z]));
-            norm[z] = m31_reduce64((uint64_t)den[z].a * den[z].a + (uint64_t)den[z].b * den[z].b);
-            pref[z] = run;
-            run = m31_mul(run, norm[z]);
+    for (int r = 0; r < ROWS; r++) {
+        if (ROWS == 1 || !(r & 1)) half_coset_point(tw, lifting_log, (uint32_t)((row0 + r) >> 1), px, py[r]);
+        if (ROWS > 1 && (r & 1)) py[r] = m31_neg(py[r - 1]);  // odd rows hold the conjugate point; several rows start on an even one
+        if (ROWS == 1 && (row0 & 1)) py[r] = m31_neg(py[r]);
+#pragma unroll
+        for (int z = 0; z < ACCS; z++) {
+            if (z < a.n_acc) {
+                const int k = r * ACCS + z;
+                cm31 dx = {m31_sub(a.prx[z].a, px), a.prx[z].b};
+                cm31 dy = {m31_sub(a.pry[z].a, py[r]), a.pry[z].b};
+                den[k] = cm31_sub(cm31_mul(dx, a.piy[z]), cm31_mul(dy, a.pix[z]));
+                norm[k] = m31_reduce64((uint64_t)den[k].a * den[k].a + (uint64_t)den[k].b * den[k].b);
+                pref[k] = run;
+                run = m31_mul(run, norm[k]);
+            }
         }
     }
     uint32_t inv = m31_inv(run);
-    qm31 q = qm31_zero();
 #pragma unroll
-    for (int z = MAX_ACCS - 1; z >= 0; z--) {
-        if (z < a.n_acc) {
-            uint32_t ninv = m31_mul(inv, pref[z]);
-            inv = m31_mul(inv, norm[z]);
-            cm31 dinv = {m31_mul(den[z].a, ninv), m31_mul(m31_neg(den[z].b), ninv)};
-            const size_t li = ((row >> (a.log_ratio[z] + 1)) << 1) + (row & 1) - (((row_begin >> (a.log_ratio[z] + 1)) << 1));
-            qm31 num{{a.acc[z][0][li], a.acc[z][1][li], a.acc[z][2][li], a.acc[z][3][li]}};
-            num = qm31_sub(num, qm31_mul_m31(a.first_lin[z], py));
-            q = qm31_add(q, qm31_mul_cm31(num, dinv));
+    for (int r = ROWS - 1; r >= 0; r--) {
+        const size_t row = row0 + r;
+        qm31 q = qm31_zero();
+#pragma unroll
+        for (int z = ACCS - 1; z >= 0; z--) {
+            if (z < a.n_acc) {
+                const int k = r * ACCS + z;
+                uint32_t ninv = m31_mul(inv, pref[k]);
+                inv = m31_mul(inv, norm[k]);
+                cm31 dinv = {m31_mul(den[k].a, ninv), m31_mul(m31_neg(den[k].b), ninv)};
+                const size_t li = ((row >> (a.log_ratio[z] + 1)) << 1) + (row & 1) - (((row_begin >> (a.log_ratio[z] + 1)) << 1));
+                qm31 num{{a.acc[z][0][li], a.acc[z][1][li], a.acc[z][2][li], a.acc[z][3][li]}};
+                num = qm31_sub(num, qm31_mul_m31(a.first_lin[z], py[r]));
+                q = qm31_add(q, qm31_mul_cm31(num, dinv));
+            }
         }
-    }
-    if (!a.first) {
-        qm31 o{{out.c[0][local], out.c[1][local], out.c[2][local], out.c[3][local]}};
-        q = qm31_add(q, o);
-    }
+        if (!a.first) {
+            qm31 o{{out.c[0][local + r], out.c[1][local + r], out.c[2][local + r], out.c[3][local + r]}};
+            q = qm31_add(q, o);
+        }
 #pragma unroll
-    for (int k = 0; k < 4; k++) out.c[k][local] = q.c[k];
+        for (int k = 0; k < 4; k++) out.c[k][local + r] = q.c[k];
+    }
 }
 
 // Slow path for lifting domains of log size 1 and 2, whose points are not in the tower.
@@ -291,24 +317,29 @@ static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncol
     for (int q = 0; q < 4; q++) wide = wide && ((uintptr_t)o.c[q] & 15) == 0;
     for (int c = 0; c < ncols; c++) wide = wide && ((uintptr_t)cols[c] & 15) == 0;
     ProfScope prof(ctx, "quot_numerators_kernel");
-    // Few rows and many columns: split the columns over the grid's second dimension.
-    const unsigned row_blocks = (unsigned)((n / (wide ? 4 : 2) + 255) / 256);
+    // Few rows: the columns are split over the grid's second dimension, so that some 148 x 4 CTAs' worth of threads have loads on their way, sixteen
+    // columns each at least. A thread walks its columns four at a time, a trip to memory each: a hundred columns of 2^13 rows on
+    // eight CTAs were 35 us, of 2^17 rows 41; split, and added up, 10 + 4 and 18 + 8. Groups of fewer than 1,024 rows take narrower CTAs.
+    const size_t per = wide ? 4 : 2;
+    const unsigned threads = n / per >= 256 ? 256u : n / per >= 32 ? (unsigned)(n / per) : 32u;
+    const unsigned row_blocks = (unsigned)((n / per + threads - 1) / threads);
     const size_t scratch_free = ctx->scratch_words - scratch_used;
-    if (row_blocks < 148u && k >= 8 * NUM_TILE && 4 * n * 2 <= scratch_free) {
-        int S = (int)((2u * 148u + row_blocks - 1) / row_blocks);            // about two CTAs per SM
-        int chunk = ((k + S - 1) / S + NUM_TILE - 1) / NUM_TILE * NUM_TILE;  // whole tiles of columns
+    int S = std::min((k + 15) / 16, (int)(148u * 1024u / (row_blocks * threads)));
+    S = std::min<size_t>(S, (scratch_free - 4) / (4 * n));
+    if (S >= 2 && k >= 32) {
+        const int chunk = ((k + S - 1) / S + 3) / 4 * 4;
         S = (k + chunk - 1) / chunk;
-        while ((size_t)S * 4 * n + 4 > scratch_free) { chunk += NUM_TILE; S = (k + chunk - 1) / chunk; }
         uint32_t* partial = ctx->scratch + scratch_used + ((4 - (scratch_used & 3)) & 3);  // 16-byte aligned
         dim3 grid(row_blocks, (unsigned)S);
         if (wide)
-            quot_numerators_kernel<4><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, b_first, n, o, chunk, partial);
+            quot_numerators_kernel<4><<<grid, threads, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
+                                                                         b_sum, b_first, n, o, chunk, partial);
         else
-            quot_numerators_kernel<2><<<grid, 256, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
-                                                                     b_sum, b_first, n, o, chunk, partial);
+            quot_numerators_kernel<2><<<grid, threads, 0, ctx->stream>>>(d_cols, d_idx, reinterpret_cast<const uint4*>(d_c), k,
+                                                                         b_sum, b_first, n, o, chunk, partial);
         ZKB_LAUNCH_CHECK(ctx);
-        quot_partial_sum_kernel<<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, b_first, o);
+        if (S >= 24) quot_partial_sum_kernel<8><<<(unsigned)((4 * n + 31) / 32), 256, 0, ctx->stream>>>(partial, S, n, b_sum, b_first, o);
+        else quot_partial_sum_kernel<1><<<(unsigned)((4 * n + 255) / 256), 256, 0, ctx->stream>>>(partial, S, n, b_sum, b_first, o);
         ZKB_LAUNCH_CHECK(ctx);
         return ZKB_OK;
     }
@@ -556,7 +587,12 @@ int zkb_quot_combine_rows(zkb_ctx* ctx, int n_acc, const uint32_t* const* acc_co
             quot_combine_small_kernel<<<1, 32, 0, ctx->stream>>>(args, lifting_log, o, p0.x, p0.y, p1.x, p1.y);
         } else {
             ProfScope prof(ctx, "quot_combine_kernel");
-            quot_combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(args, lifting_log, o, ctx->tw, row_begin, n_rows);
+            // the rows are a multiple of four but in a shard of two
+            auto launch = [&](auto kernel, int rows) { kernel<<<(unsigned)((n / rows + 255) / 256), 256, 0, ctx->stream>>>(args, lifting_log, o, ctx->tw, row_begin, n_rows); };
+            if (n % 4 || args.n_acc > 4) launch(quot_combine_kernel<MAX_ACCS, 1>, 1);
+            else if (args.n_acc == 1) launch(quot_combine_kernel<1, 4>, 4);
+            else if (args.n_acc == 2) launch(quot_combine_kernel<2, 4>, 4);
+            else launch(quot_combine_kernel<4, 2>, 2);
         }
         ZKB_LAUNCH_CHECK(ctx);
     }
