@@ -169,3 +169,12 @@ def test_quotients_combined_several_rows_a_thread(ctx, oracle, n_acc, log_n):
     outs = [ctx.alloc(1 << log_n) for _ in range(4)]
     ctx.quot_combine([b.ptr for k in keep for b in k], [lg for _, lg in accs], first, points, log_n, [o.ptr for o in outs])
     assert (np.stack([o.download() for o in outs]) == want).all()
+
+
+@pytest.mark.parametrize("log_n,n_cols", [(14, 2), (15, 1), (15, 300), (16, 150), (17, 5), (17, 300), (18, 299)])
+def test_eval_at_point_in_runs_of_chunks(ctx, oracle, log_n, n_cols):
+    # from 2^15 coefficients on: runs of sixteen chunks, of 32 and 64 where there are two for every SM
+    cols = [m31_column(8400 + 7 * log_n + c, 1 << log_n) for c in range(n_cols)]
+    bufs, point = [ctx.upload(c) for c in cols], qm31_array(8390, 2).ravel()
+    got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
+    assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()

@@ -21,13 +21,14 @@ constexpr int EVAL_MAX_LEVELS = 32;
 
 struct EvalFactors { qm31 m[EVAL_MAX_LEVELS]; };
 
-// weights[i] = prod over set bits k of i of m_k, i < 2^EVAL_CHUNK_LOG.
-__global__ void eval_weights_kernel(EvalFactors f, int bits, uint32_t* __restrict__ weights) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (1u << bits)) return;
+// weights[i] = prod over set bits k of i of m_k, i < 2^EVAL_CHUNK_LOG, and behind them the same of the run_bits factors that follow.
+__global__ void eval_weights_kernel(EvalFactors f, int run_bits, uint32_t* __restrict__ weights) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, n = 1u << EVAL_CHUNK_LOG;
+    if (i >= n + (1u << run_bits)) return;
+    const int first = i < n ? 0 : EVAL_CHUNK_LOG, bits = i < n ? EVAL_CHUNK_LOG : run_bits;
     qm31 w = qm31_one();
     for (int k = 0; k < bits; k++)
-        if ((i >> k) & 1u) w = qm31_mul(w, f.m[k]);
+        if (((i < n ? i : i - n) >> k) & 1u) w = qm31_mul(w, f.m[first + k]);
     reinterpret_cast<uint4*>(weights)[i] = make_uint4(w.c[0], w.c[1], w.c[2], w.c[3]);
 }
 
@@ -92,6 +93,82 @@ __global__ void __launch_bounds__(256) eval_dot_kernel(const uint32_t* const* __
             }
         }
         __syncthreads();
+    }
+}
+
+// The same for runs of 2^run_log chunks: out[col][run] = sum_e weights[e] sum_g weights[2048 + g] cols[col][2048 (2^run_log run + g) + e].
+// eval_dot_kernel is bound by what a chunk costs beside its products, the reduction of four words over the CTA; here a thread keeps the inner sums of
+// its eight elements through a run (64-bit sums folded every four chunks) and the weights and the reduction come once a run. 256 columns of
+// 2^20: 396 us with a reduction a chunk, 229 with one in 64.
+constexpr int RUN_MIN_LOG = 4, RUN_MAX_LOG = 6, RUN_CTAS = 2;
+__global__ void __launch_bounds__(256, RUN_CTAS) eval_runs_kernel(const uint32_t* const* __restrict__ cols, int ncols, int log_n, int run_log,
+                                                                  const uint32_t* __restrict__ weights, uint32_t* __restrict__ out) {
+    __shared__ uint4 of_chunk[1 << RUN_MAX_LOG];
+    __shared__ uint32_t red[2][4][2][8];  // [run mod 2][component][lo/hi][warp]
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const uint4* const w = reinterpret_cast<const uint4*>(weights);
+    if (t < (1 << run_log)) of_chunk[t] = w[(1 << EVAL_CHUNK_LOG) + t];
+    __syncthreads();
+    const int runs_log = log_n - EVAL_CHUNK_LOG - run_log;
+    const size_t items = (size_t)ncols << runs_log;
+    const int chunks = 1 << run_log;
+    int side = 0;
+    for (size_t item = blockIdx.x; item < items; item += gridDim.x, side ^= 1) {
+        const uint4* __restrict__ c = reinterpret_cast<const uint4*>(cols[item >> runs_log] + ((item & (((size_t)1 << runs_log) - 1)) << (EVAL_CHUNK_LOG + run_log))) + t;
+        uint64_t a[8][4];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) a[u][q] = 0;
+        uint4 next[4];  // two chunks
+#pragma unroll
+        for (int g = 0; g < 4; g++) next[g] = __ldcs(c + 256 * g);
+        for (int g0 = 0; g0 < chunks; g0 += 4) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                uint4 v[4];
+#pragma unroll
+                for (int g = 0; g < 4; g++) v[g] = next[g];
+                c += 1024;
+                if (g0 + 2 * h + 2 < chunks) {
+#pragma unroll
+                    for (int g = 0; g < 4; g++) next[g] = __ldcs(c + 256 * g);
+                }
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    const uint4 f = of_chunk[g0 + 2 * h + g], x = v[2 * g], y = v[2 * g + 1];
+                    const uint32_t e[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        a[u][0] += (uint64_t)e[u] * f.x; a[u][1] += (uint64_t)e[u] * f.y;
+                        a[u][2] += (uint64_t)e[u] * f.z; a[u][3] += (uint64_t)e[u] * f.w;
+                    }
+                }
+            }
+            // four 62-bit products on top of a folded (< 2^34) sum fit in 64 bits
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) a[u][q] = fold64_eval(a[u][q]);
+        }
+        qm31 r = qm31_zero();
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const uint4 x = w[(u >> 2) * 1024 + 4 * t + (u & 3)];
+            r = qm31_add(r, qm31_mul(qm31{{m31_reduce64(a[u][0]), m31_reduce64(a[u][1]), m31_reduce64(a[u][2]), m31_reduce64(a[u][3])}}, qm31{{x.x, x.y, x.z, x.w}}));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t lo = __reduce_add_sync(0xffffffffu, r.c[k] & 0xffffu), hi = __reduce_add_sync(0xffffffffu, r.c[k] >> 16);
+            if (lane == 0) { red[side][k][0][warp] = lo; red[side][k][1][warp] = hi; }
+        }
+        __syncthreads();  // (what the run before the last left in the same place was read before the last run's barrier)
+        if (t < 4) {
+            uint64_t lo = 0, hi = 0;
+#pragma unroll
+            for (int wv = 0; wv < 8; wv++) { lo += red[side][t][0][wv]; hi += red[side][t][1][wv]; }
+            out[4 * item + t] = m31_reduce64(lo + (hi << 16));
+        }
     }
 }
 
@@ -204,18 +281,23 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
         return ZKB_OK;
     }
     static_assert(EVAL_SHORT_LOG + 1 == EVAL_CHUNK_LOG, "what is left has a whole chunk");
-    // Scratch: [weights: 2048 QM31] [ping] [pong]; columns go in batches whose partials fit.
+    // Scratch: [weights: 2048 and 64 QM31] [ping] [pong]; columns go in batches whose partials fit.
     bool use_dot = true;
     for (int c = 0; c < ncols; c++) use_dot = use_dot && ((uintptr_t)coeffs[c] & 15) == 0;  // 16-byte loads
-    size_t partials_per_col = (size_t)1 << (log_n - EVAL_CHUNK_LOG);
+    // Runs of sixteen chunks and more, as long as there are two for every SM (shorter ones cost more in products with the weights than they save).
+    int run_log = log_n - EVAL_CHUNK_LOG < RUN_MAX_LOG ? log_n - EVAL_CHUNK_LOG : RUN_MAX_LOG;
+    while (run_log > RUN_MIN_LOG && ((size_t)ncols << (log_n - EVAL_CHUNK_LOG - run_log)) < RUN_CTAS * 148u) run_log--;
+    if (!use_dot || run_log < RUN_MIN_LOG) run_log = 0;
+    const int chunk_log = EVAL_CHUNK_LOG + run_log;
+    size_t partials_per_col = (size_t)1 << (log_n - chunk_log);
     uint32_t* weights = ctx->scratch;
-    const size_t weights_words = (size_t)4 << EVAL_CHUNK_LOG;
+    const size_t weights_words = ((size_t)4 << EVAL_CHUNK_LOG) + ((size_t)4 << RUN_MAX_LOG);
     size_t half_words = (ctx->scratch_words - weights_words) / 2;
     size_t max_cols = half_words / (4 * partials_per_col);
     ZKB_CHECK_ARG(ctx, max_cols >= 1);
     if (max_cols > MAX_COLS) max_cols = MAX_COLS;
     if (use_dot) {
-        eval_weights_kernel<<<(1 << EVAL_CHUNK_LOG) / 256, 256, 0, ctx->stream>>>(f, EVAL_CHUNK_LOG, weights);
+        eval_weights_kernel<<<(1 << EVAL_CHUNK_LOG) / 256 + 1, 256, 0, ctx->stream>>>(f, run_log, weights);
         ZKB_LAUNCH_CHECK(ctx);
     }
     for (int c0 = 0; c0 < ncols; c0 += (int)max_cols) {
@@ -227,7 +309,13 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
         uint32_t* bufB = bufA + half_words;
         uint32_t* const out = d_out + 4 * (size_t)c0;  // what the last kernel writes to
         int log_cur = log_n, level = 0;
-        if (use_dot) {
+        if (run_log) {
+            const size_t items = partials_per_col * (size_t)nc;
+            ProfScope prof(ctx, "eval_runs_kernel");
+            eval_runs_kernel<<<(unsigned)(items < RUN_CTAS * 148u ? items : RUN_CTAS * 148u), 256, 0, ctx->stream>>>((const uint32_t* const*)d_cols, nc, log_n, run_log, weights,
+                                                                                                               log_n == chunk_log ? out : bufA);
+            ZKB_LAUNCH_CHECK(ctx);
+        } else if (use_dot) {
             size_t items = (partials_per_col + DOT_CHUNKS - 1) / DOT_CHUNKS * (size_t)nc;
             unsigned grid = (unsigned)(items < 2 * 148 ? items : 2 * 148);
             ProfScope prof(ctx, "eval_dot_kernel");
@@ -239,8 +327,8 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
                                                                   log_n == EVAL_CHUNK_LOG ? out : bufA);
             ZKB_LAUNCH_CHECK(ctx);
         }
-        log_cur -= EVAL_CHUNK_LOG;
-        level += EVAL_CHUNK_LOG;
+        log_cur -= chunk_log;
+        level += chunk_log;
         while (log_cur > 0) {
             int ch = log_cur < EVAL_CHUNK_LOG ? log_cur : EVAL_CHUNK_LOG;
             unsigned threads = ch >= 9 ? 256 : 32;
