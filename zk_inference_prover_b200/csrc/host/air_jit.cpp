@@ -37,7 +37,7 @@ __device__ __forceinline__ u32 m31_neg(u32 a) { return a ? P - a : 0u; }
 __device__ __forceinline__ u32 m31_reduce64(u64 v) {
     u32 lo = (u32)v, hi = (u32)(v >> 32);
     u32 s = (lo & P) + (((hi << 1) | (lo >> 31)) & P);
-    s = (s & P) + (s >> 31) + (hi >> 30);
+    s = umin32(s, s - P) + (hi >> 30);
     return umin32(s, s - P);
 }
 __device__ __forceinline__ u32 m31_mul(u32 a, u32 b) {

@@ -28,11 +28,11 @@ ZK_HD uint32_t m31_neg(uint32_t a) { return a ? P - a : 0u; }
 ZK_HD uint32_t m31_dbl(uint32_t a) { return m31_add(a, a); }
 
 // Any 64-bit value -> canonical residue. Its three parts of 31, 31 and 2 bits have weight one each; the middle one is a funnel shift
-// on the device. The top one is added after the fold: the two others are at most 2p < 2^32 and fold to at most p, so nothing is lost,
-// while all three at once reach 2^32 (at 3 * 2^62 - 1, say, which four products can add up to) and would wrap.
+// on the device. The top one is added once the two others, at most 2p < 2^32, are back at most p: all three at once reach 2^32 (at
+// 3 * 2^62 - 1, say, which four products can add up to) and would wrap. Either subtraction is one add-and-minimum.
 ZK_HD uint32_t m31_reduce64(uint64_t v) {
     uint32_t s = ((uint32_t)v & P) + ((uint32_t)(v >> 31) & P);
-    s = (s & P) + (s >> 31) + (uint32_t)(v >> 62);  // <= p + 3
+    s = umin32(s, s - P) + (uint32_t)(v >> 62);  // <= p + 3
     return umin32(s, s - P);
 }
 // Product of two canonical values.
