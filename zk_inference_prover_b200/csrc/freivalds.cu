@@ -127,8 +127,6 @@ __global__ void __launch_bounds__(SCATTER_THREADS, 5) freivalds_scatter_kernel(c
 }
 
 // ---- F2: inner products per row -----------------------------------------------------------------
-__device__ __forceinline__ uint64_t fold64f(uint64_t v) { return (v & P) + (v >> 31); }
-
 // lanes[l][j] (QM31, coset order): l = 0 is v_in, l = 1 + m is u_in of matrix m. Eight loads are on their way at a time (a load
 // a row, behind that of its column address, one after the other: 107 us at 2^20 rows of 33 columns).
 // sum of pow[p] (cols[p][row] - bias) for two rows
@@ -152,7 +150,7 @@ __device__ __forceinline__ RowSums inner_pair(const uint32_t* const* __restrict_
             b[0] += (uint64_t)c.x * w; b[1] += (uint64_t)c.y * w; b[2] += (uint64_t)c.z * w; b[3] += (uint64_t)c.w * w;
         }
 #pragma unroll
-        for (int q = 0; q < 4; q++) { a[q] = fold64f(a[q]); b[q] = fold64f(b[q]); }
+        for (int q = 0; q < 4; q++) { a[q] = m31_fold64(a[q]); b[q] = m31_fold64(b[q]); }
     }
     return {make_uint4(m31_reduce64(a[0]), m31_reduce64(a[1]), m31_reduce64(a[2]), m31_reduce64(a[3])),
             make_uint4(m31_reduce64(b[0]), m31_reduce64(b[1]), m31_reduce64(b[2]), m31_reduce64(b[3]))};

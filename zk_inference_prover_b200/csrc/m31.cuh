@@ -27,12 +27,21 @@ ZK_HD uint32_t m31_sub(uint32_t a, uint32_t b) { uint32_t d = a - b; return umin
 ZK_HD uint32_t m31_neg(uint32_t a) { return a ? P - a : 0u; }
 ZK_HD uint32_t m31_dbl(uint32_t a) { return m31_add(a, a); }
 
-// Any 64-bit value -> canonical residue. Its three parts of 31, 31 and 2 bits have weight one each; the middle one is a funnel shift
-// on the device. The top one is added once the two others, at most 2p < 2^32, are back at most p: all three at once reach 2^32 (at
-// 3 * 2^62 - 1, say, which four products can add up to) and would wrap. Either subtraction is one add-and-minimum.
+// Any 64-bit value to one below 2^34 of the same class: 2^32 = 2 (mod p), so the upper word enters doubled. On the device that is one wide
+// multiply-add on the FMA pipe; masks, shifts and carries in its place are five instructions on the ALU pipe, which bounds field arithmetic here.
+ZK_HD uint64_t m31_fold64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+    uint64_t t;
+    asm("mad.wide.u32 %0, %1, 2, %2;" : "=l"(t) : "r"((uint32_t)(v >> 32)), "l"((uint64_t)(uint32_t)v));
+    return t;
+#else
+    return (v >> 32) * 2 + (uint32_t)v;
+#endif
+}
+// Any 64-bit value -> canonical residue. The fold leaves at most 3 (2^32 - 1), whose parts of 31 and 3 bits add up to at most p + 5.
 ZK_HD uint32_t m31_reduce64(uint64_t v) {
-    uint32_t s = ((uint32_t)v & P) + ((uint32_t)(v >> 31) & P);
-    s = umin32(s, s - P) + (uint32_t)(v >> 62);  // <= p + 3
+    const uint64_t t = m31_fold64(v);
+    const uint32_t s = ((uint32_t)t & P) + (uint32_t)(t >> 31);
     return umin32(s, s - P);
 }
 // Product of two canonical values.

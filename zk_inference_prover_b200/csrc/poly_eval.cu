@@ -32,8 +32,6 @@ __global__ void eval_weights_kernel(EvalFactors f, int run_bits, uint32_t* __res
     reinterpret_cast<uint4*>(weights)[i] = make_uint4(w.c[0], w.c[1], w.c[2], w.c[3]);
 }
 
-__device__ __forceinline__ uint64_t fold64_eval(uint64_t v) { return (v & P) + (v >> 31); }
-
 // out[col][chunk] = sum_{e < 2048} cols[col][2048 chunk + e] * weights[e]
 // Thread t owns elements 4t..4t+3 and 1024+4t..1024+4t+3 of every chunk (two 16-byte loads) and keeps
 // their eight weights in registers. DOT_CHUNKS chunks are in flight per iteration; their per-warp sums
@@ -72,7 +70,7 @@ __global__ void __launch_bounds__(256) eval_dot_kernel(const uint32_t* const* __
             for (int u = 0; u < 8; u++) {
                 a0 += (uint64_t)e[u] * w[u].x; a1 += (uint64_t)e[u] * w[u].y;
                 a2 += (uint64_t)e[u] * w[u].z; a3 += (uint64_t)e[u] * w[u].w;
-                if (u == 3) { a0 = fold64_eval(a0); a1 = fold64_eval(a1); a2 = fold64_eval(a2); a3 = fold64_eval(a3); }
+                if (u == 3) { a0 = m31_fold64(a0); a1 = m31_fold64(a1); a2 = m31_fold64(a2); a3 = m31_fold64(a3); }
             }
             const uint32_t r[4] = {m31_reduce64(a0), m31_reduce64(a1), m31_reduce64(a2), m31_reduce64(a3)};
 #pragma unroll
@@ -99,7 +97,7 @@ __global__ void __launch_bounds__(256) eval_dot_kernel(const uint32_t* const* __
 // The same for runs of 2^run_log chunks: out[col][run] = sum_e weights[e] sum_g weights[2048 + g] cols[col][2048 (2^run_log run + g) + e].
 // eval_dot_kernel is bound by what a chunk costs beside its products, the reduction of four words over the CTA; here a thread keeps the inner sums of
 // its eight elements through a run (64-bit sums folded every four chunks) and the weights and the reduction come once a run. 256 columns of
-// 2^20: 396 us with a reduction a chunk, 229 with one in 64.
+// 2^20: 396 us with a reduction a chunk, 210 with one in 64.
 constexpr int RUN_MIN_LOG = 4, RUN_MAX_LOG = 6, RUN_CTAS = 2;
 __global__ void __launch_bounds__(256, RUN_CTAS) eval_runs_kernel(const uint32_t* const* __restrict__ cols, int ncols, int log_n, int run_log,
                                                                   const uint32_t* __restrict__ weights, uint32_t* __restrict__ out) {
@@ -149,7 +147,7 @@ __global__ void __launch_bounds__(256, RUN_CTAS) eval_runs_kernel(const uint32_t
 #pragma unroll
             for (int u = 0; u < 8; u++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) a[u][q] = fold64_eval(a[u][q]);
+                for (int q = 0; q < 4; q++) a[u][q] = m31_fold64(a[u][q]);
         }
         qm31 r = qm31_zero();
 #pragma unroll
@@ -205,7 +203,7 @@ __global__ void __launch_bounds__(256) eval_short_kernel(const uint32_t* const* 
                 a[2] += (uint64_t)v[u] * x.z; a[3] += (uint64_t)v[u] * x.w;
             }
 #pragma unroll
-            for (int q = 0; q < 4; q++) a[q] = fold64_eval(a[q]);
+            for (int q = 0; q < 4; q++) a[q] = m31_fold64(a[q]);
         }
         uint32_t r[4];
 #pragma unroll

@@ -22,9 +22,6 @@ namespace zk {
 struct Secure4 { uint32_t* c[4]; };
 struct Secure4C { const uint32_t* c[4]; };
 
-// Partially folds a 64-bit accumulator to below 2^34 without changing its residue.
-__device__ __forceinline__ uint64_t fold64(uint64_t v) { return (v & P) + (v >> 31); }
-
 // R consecutive rows per thread (one 8- or 16-byte load per column). The column addresses and the
 // coefficients of a tile of columns are resolved once per CTA into shared memory, so the inner loop
 // is one independent streaming load per column and 4 R multiply-adds: the kernel is bound by HBM.
@@ -86,7 +83,7 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
 #pragma unroll
             for (int r = 0; r < R; r++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) acc[r][q] = fold64(acc[r][q]);
+                for (int q = 0; q < 4; q++) acc[r][q] = m31_fold64(acc[r][q]);
         }
         for (; j < tk; j++) {  // at most 3 tail products
             uint32_t v[R];
@@ -96,7 +93,7 @@ __global__ void __launch_bounds__(256) quot_numerators_kernel(const uint32_t* co
 #pragma unroll
         for (int r = 0; r < R; r++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) acc[r][q] = fold64(acc[r][q]);
+            for (int q = 0; q < 4; q++) acc[r][q] = m31_fold64(acc[r][q]);
     }
     if (!live) return;
     uint32_t res[R][4];
@@ -466,7 +463,7 @@ int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<Numerat
 
 // The combination of the columns' polynomials is itself a polynomial of their degree, so it can be taken of the coefficients, a
 // blow-up fewer of them, and extended: four columns' worth of transform in the place of most of the reading. (The constant comes off
-// coefficient 0, whose basis element is 1.) 256 columns of 2^20 at blow-up 4: 810 us from the evaluations, 229 + 86 from the coefficients.
+// coefficient 0, whose basis element is 1.) 256 columns of 2^20 at blow-up 4: 810 us from the evaluations, 206 + 86 from the coefficients.
 // The transform costs as much as reading 27 columns' evaluations at that height and its launches some 10 us, which is 50 MB, so
 // narrow or short groups are read as they are; so are coefficients that do not start on 16 bytes.
 static bool numerators_of_coeffs(const uint32_t* const* coeffs, int ncols, int log_n, int log_coeff, size_t k) {
