@@ -58,6 +58,17 @@ def test_oracle_claims_are_the_freivalds_identity(oracle, tokens, n_in, n_outs, 
         assert (cols[8 + 8 * m:12 + 8 * m, last] == claims[m]).all()
 
 
+# groups of 32 to 256 rows, a power of two, in sixteen blocks of coset order and more (with and without lead rows), and what lies around that
+BLOCKS = [(5, 16, [70, 33], 32), (5, 15, [70], 32), (8, 12, [300], 64), (40, 100, [256, 100, 31], 256), (3, 17, [600], 128), (2, 20, [520], 512), (9, 8, [64], 32),
+          (9, 60, [64], 33)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,n_in,n_outs,chunks", BLOCKS)
+def test_freivalds_device_matches_oracle_in_blocks(ctx, oracle, tokens, n_in, n_outs, chunks):
+    test_freivalds_device_matches_oracle(ctx, oracle, tokens, n_in, n_outs, chunks)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("tokens,n_in,n_outs,chunks", [(5, 6, [7, 5], 4), (3, 8, [8], 2), (9, 4, [4, 6, 2], 3), (1, 16, [5], 1),
                                                       (32, 64, [64, 48, 64], 16), (17, 128, [96], 64)])

@@ -171,6 +171,79 @@ __global__ void __launch_bounds__(256, 4) freivalds_inner_kernel(const uint32_t*
     }
 }
 
+// The same, four rows a thread: two neighbours and the two that mirror them, whose places in coset order are two whole sectors. What a column costs
+// beside its products (its address, the power, the checks) is paid for four rows, column addresses and powers come from shared memory,
+// and the activations' bias is taken off the finished sums. 2^20 rows of 33 columns: 24 instructions a row and column, 52 us; now 15 and
+// 42.
+constexpr uint32_t INNER_TILE = 64;
+__global__ void __launch_bounds__(256, 4) freivalds_inner_quad_kernel(const uint32_t* const* __restrict__ base_cols, const uint32_t* const* __restrict__ pre_cols,
+                                                                      const uint4* __restrict__ s_pow, const uint4* __restrict__ rv_pow, FGrid g, uint32_t pq,
+                                                                      uint32_t pk, uint32_t n_mats, qm31 bias, uint4* __restrict__ lanes) {
+    __shared__ const uint32_t* s_col[INNER_TILE];
+    __shared__ uint4 s_c[INNER_TILE];
+    const uint32_t rows = 1u << g.log_rows, n_threads = rows >> 2;  // at least 256
+    const uint32_t i = 2u * ((threadIdx.x >> 5) * (n_threads >> 3) + blockIdx.x * 32u + (threadIdx.x & 31u)), i2 = rows - 2u - i;
+    for (uint32_t l = 0; l <= n_mats; l++) {
+        const uint32_t* const* __restrict__ cols = l ? pre_cols + (size_t)(l - 1) * pk : base_cols;
+        const uint4* __restrict__ pow = l ? rv_pow : s_pow;
+        const uint32_t n = l ? pk : pq;
+        uint64_t a[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) a[r][q] = 0;
+        auto add = [&](const uint4& c, const uint2& x, const uint2& y) {
+            const uint32_t e[4] = {x.x, x.y, y.x, y.y};
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                a[r][0] += (uint64_t)c.x * e[r]; a[r][1] += (uint64_t)c.y * e[r]; a[r][2] += (uint64_t)c.z * e[r]; a[r][3] += (uint64_t)c.w * e[r];
+            }
+        };
+        // four products below 2^62 on top of a folded sum fit 64 bits
+        auto fold = [&] {
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) a[r][q] = m31_fold64(a[r][q]);
+        };
+        for (uint32_t tile = 0; tile < n; tile += INNER_TILE) {
+            const uint32_t here = n - tile < INNER_TILE ? n - tile : INNER_TILE;
+            __syncthreads();
+            if (threadIdx.x < here) {
+                s_col[threadIdx.x] = cols[tile + threadIdx.x];
+                s_c[threadIdx.x] = pow[tile + threadIdx.x];
+            }
+            __syncthreads();
+            uint32_t p = 0;
+            for (; p + 4 <= here; p += 4) {
+                uint2 x[4], y[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) {
+                    x[u] = __ldcs(reinterpret_cast<const uint2*>(s_col[p + u] + i));
+                    y[u] = __ldcs(reinterpret_cast<const uint2*>(s_col[p + u] + i2));
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 4; u++) add(s_c[p + u], x[u], y[u]);
+                fold();
+            }
+            for (; p < here; p++) add(s_c[p], __ldcs(reinterpret_cast<const uint2*>(s_col[p] + i)), __ldcs(reinterpret_cast<const uint2*>(s_col[p] + i2)));
+            fold();
+        }
+        uint4* const out = lanes + (size_t)l * rows;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const uint32_t j = coset_perm(r < 2 ? i + r : i2 + r - 2, g.log_rows);
+            uint32_t w[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t v = m31_reduce64(a[r][q]);
+                w[q] = l ? v : m31_sub(v, bias.c[q]);
+            }
+            out[j] = j >= g.lead ? make_uint4(w[0], w[1], w[2], w[3]) : make_uint4(0, 0, 0, 0);
+        }
+    }
+}
+
 // ---- F3: per-group Horner, prefix over groups, split ------------------------------------------------
 __device__ __forceinline__ qm31 q_of(uint4 v) { return {{v.x, v.y, v.z, v.w}}; }
 __device__ __forceinline__ uint4 u_of(qm31 v) { return make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]); }
@@ -186,53 +259,141 @@ struct ScanSteps {
     qm31 pw[2][9];    // pw[kind][k] = step^k for k = 0..8; kind 0 is lane 0 (v, step s^pq), kind 1 the lanes u_m (step rv^pk)
     qm31 wide[2][6];  // step^(8 2^k)
 };
+// `left` rows of a group (at most 256 are taken), by a warp; end: the value before them, on return that after the last of them.
+// get(r): row r's input; put(r, x): its value. IN_PLACE: get reads what put wrote cheaply, so the sums from a zero carry are kept there
+// instead of in 32 registers.
+template <bool IN_PLACE, class Get, class Put>
+__device__ __forceinline__ void scan_rows(uint32_t left, bool first, const qm31* pw, const qm31* wide, qm31& end, Get get, Put put) {
+    const uint32_t lane = threadIdx.x & 31u, r0 = lane * 8u, n_here = r0 >= left ? 0u : (left - r0 < 8u ? left - r0 : 8u);
+    const qm31 step = pw[1];
+    qm31 y[IN_PLACE ? 1 : 8];
+    qm31 acc = qm31_zero();
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++)
+        if (k < n_here) {
+            acc = qm31_add(qm31_mul(acc, step), q_of(get(r0 + k)));
+            if (IN_PLACE) put(r0 + k, u_of(acc));
+            else y[IN_PLACE ? 0 : k] = acc;
+        }
+    // The value after a lane's rows, exact for lanes whose rows before them are all there: only the last lane with rows may
+    // have fewer than eight, and nothing is taken from it or from the ones after.
+    qm31 B = lane == 0 && !first ? qm31_add(acc, qm31_mul(end, pw[n_here])) : acc;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        qm31 b1;
+#pragma unroll
+        for (int c = 0; c < 4; c++) b1.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1 << k);
+        if ((int)lane >= (1 << k)) B = qm31_add(qm31_mul(b1, wide[k]), B);
+    }
+    qm31 carry;  // into this lane: the value at the end of the previous one
+#pragma unroll
+    for (int c = 0; c < 4; c++) carry.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1);
+    if (lane == 0) carry = end;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; k++)
+        if (k < n_here) {
+            acc = qm31_add(IN_PLACE ? q_of(get(r0 + k)) : y[IN_PLACE ? 0 : k], qm31_mul(carry, pw[k + 1]));
+            put(r0 + k, u_of(acc));
+        }
+    const int from = (int)((left < 256u ? left : 256u) - 1u) >> 3;  // the lane of the last row
+#pragma unroll
+    for (int c = 0; c < 4; c++) end.c[c] = __shfl_sync(0xffffffffu, acc.c[c], from);
+}
 __global__ void __launch_bounds__(256) freivalds_group_scan_kernel(uint4* __restrict__ lanes, FGrid g, uint32_t n_mats, const __grid_constant__ ScanSteps st,
                                                                    uint4* __restrict__ prod) {
     const uint32_t slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (slot >= g.groups) return;
     qm31 v_last = qm31_zero();
     for (uint32_t l = 0; l <= n_mats; l++) {
-        const qm31* pw = st.pw[l ? 1 : 0];
-        const qm31* wide = st.wide[l ? 1 : 0];
-        const qm31 step = pw[1];
-        uint4* __restrict__ p = lanes + ((size_t)l << g.log_rows) + g.lead + (size_t)slot * g.chunks;
+        uint4* p = lanes + ((size_t)l << g.log_rows) + g.lead + (size_t)slot * g.chunks;
         qm31 end = qm31_zero();  // the value after the last row so far
-        for (uint32_t base = 0; base < g.chunks; base += 256, p += 256) {
-            const uint32_t left = g.chunks - base, r0 = lane * 8u, n_here = r0 >= left ? 0u : (left - r0 < 8u ? left - r0 : 8u);
-            qm31 y[8];
-            qm31 acc = qm31_zero();
-#pragma unroll
-            for (uint32_t k = 0; k < 8; k++)
-                if (k < n_here) {
-                    acc = qm31_add(qm31_mul(acc, step), q_of(p[r0 + k]));
-                    y[k] = acc;
-                }
-            // The value after a lane's rows, exact for lanes whose rows before them are all there: only the last lane with rows may
-            // have fewer than eight, and nothing is taken from it or from the ones after.
-            qm31 B = lane == 0 && base ? qm31_add(acc, qm31_mul(end, pw[n_here])) : acc;
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                qm31 b1;
-#pragma unroll
-                for (int c = 0; c < 4; c++) b1.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1 << k);
-                if ((int)lane >= (1 << k)) B = qm31_add(qm31_mul(b1, wide[k]), B);
-            }
-            qm31 carry;  // into this lane: the value at the end of the previous one
-#pragma unroll
-            for (int c = 0; c < 4; c++) carry.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1);
-            if (lane == 0) carry = end;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; k++)
-                if (k < n_here) {
-                    acc = qm31_add(y[k], qm31_mul(carry, pw[k + 1]));
-                    p[r0 + k] = u_of(acc);
-                }
-            const int from = (int)((left < 256u ? left : 256u) - 1u) >> 3;  // the lane of the last row
-#pragma unroll
-            for (int c = 0; c < 4; c++) end.c[c] = __shfl_sync(0xffffffffu, acc.c[c], from);
-        }
+        for (uint32_t base = 0; base < g.chunks; base += 256, p += 256)
+            scan_rows<false>(g.chunks - base, base == 0, st.pw[l ? 1 : 0], st.wide[l ? 1 : 0], end, [&](uint32_t r) { return p[r]; }, [&](uint32_t r, uint4 x) { p[r] = x; });
         if (l == 0) v_last = end;
         else if (lane == 0) prod[(size_t)(l - 1) * g.groups + slot] = u_of(qm31_mul(end, v_last));
+    }
+}
+
+// Scan and split in one, where a group is 2^b rows, 32 to 256 of them: then it is an aligned block of coset order, and in committed order the
+// blocks whose numbers, bits reversed, are neighbours lie next to each other: with c = (row in the block, bits reversed) 2^L + c_low, c_low the
+// block's number reversed, an even row is at 2 c and an odd one at 2 n - 1 - 2 c. A CTA takes the blocks c0 ... c0 + 7 (A) and their complements (B),
+// a warp each; for an even row r and either of the two segments below, sixteen consecutive words hold eight blocks' values at row r and eight
+// of the others' at row 2^b - 1 - r, so a lane's values cross shared memory once and go out in whole 64-byte pieces. 2^20 rows, 256 to a
+// group, v and two u: scan and split one after the other 44 + 32 us, this and the accumulators' columns 51 + 8.
+constexpr int SCAN_OUT_THREADS = 512, SCAN_OUT_GROUPS = SCAN_OUT_THREADS / 32;
+constexpr uint32_t SCAN_OUT_PITCH = 256 + 32;  // of a group in shared memory: a gap every eight rows, which the lanes write at a time
+constexpr size_t SCAN_OUT_SMEM = (size_t)SCAN_OUT_GROUPS * SCAN_OUT_PITCH * 16;
+__global__ void __launch_bounds__(SCAN_OUT_THREADS, 2) freivalds_scan_out_kernel(const uint4* __restrict__ lanes, FGrid g, uint32_t chunk_log, uint32_t n_mats,
+                                                                                 const __grid_constant__ ScanSteps st, uint4* __restrict__ prod,
+                                                                                 uint32_t* const* __restrict__ out) {
+    extern __shared__ uint4 tile[];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, L = g.log_rows - chunk_log, mask = (1u << L) - 1u, c0 = blockIdx.x * 8u;
+    const uint32_t c_low = warp < 8 ? c0 + warp : mask - (c0 + warp - 8u), block = __brev(c_low) >> (32 - L);
+    const uint32_t lead_blocks = g.lead >> chunk_log;
+    uint4* const mine = tile + warp * SCAN_OUT_PITCH;
+    auto at = [](uint32_t r) { return r + (r >> 3); };
+    qm31 v_last = qm31_zero();
+    for (uint32_t l = 0; l <= n_mats; l++) {
+        qm31 end = qm31_zero();
+        const uint4* const rows_in = lanes + ((size_t)l << g.log_rows) + ((size_t)block << chunk_log);
+        uint4 in[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            if (32u * k + lane < g.chunks) in[k] = rows_in[32u * k + lane];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            if (32u * k + lane < g.chunks) mine[at(32u * k + lane)] = in[k];
+        __syncwarp();
+        scan_rows<true>(g.chunks, true, st.pw[l ? 1 : 0], st.wide[l ? 1 : 0], end, [&](uint32_t r) { return mine[at(r)]; }, [&](uint32_t r, uint4 x) { mine[at(r)] = x; });
+        if (l == 0) v_last = end;
+        else if (lane == 0 && block >= lead_blocks) prod[(size_t)(l - 1) * g.groups + block - lead_blocks] = u_of(qm31_mul(end, v_last));
+        __syncthreads();
+        uint32_t* const* const o = out + (l ? 8 * l - 4 : 0);
+        uint32_t *const o0 = o[0], *const o1 = o[1], *const o2 = o[2], *const o3 = o[3];
+        for (uint32_t k = threadIdx.x; k < 16u * g.chunks; k += SCAN_OUT_THREADS) {
+            const uint32_t w = k & 15u, t = w >> 1, odd = w & 1u, seg = (k >> 4) & 1u, h = k >> 5, r = __brev(h) >> (32 - chunk_log);
+            const uint32_t from = seg == odd ? (seg ? 7u - t : t) : 8u + (seg ? 7u - t : t);  // A in even words of the first segment, odd ones of the second
+            const uint32_t row = odd ? g.chunks - 1u - r : r;
+            const uint4 x = tile[from * SCAN_OUT_PITCH + at(row)];
+            const size_t i = 2u * ((h << L) + (seg ? mask - (c0 + 7u) : c0)) + w;
+            o0[i] = x.x; o1[i] = x.y; o2[i] = x.z; o3[i] = x.w;
+        }
+        __syncthreads();
+    }
+}
+// The accumulators' columns for the same grids: the prefix up to the row's block, in its last row (odd, the odd words' first) with it. Where a row
+// lies in committed order modulo 2^(L + 1) says which block it is of: a thread has the prefixes of four neighbouring places and writes them to
+// every row of its share.
+constexpr uint32_t ACC_RUN = 16;
+__global__ void __launch_bounds__(128) freivalds_acc_columns_kernel(const uint4* __restrict__ prefix, FGrid g, uint32_t chunk_log, uint32_t n_mats, uint32_t* const* __restrict__ out) {
+    const uint32_t L = g.log_rows - chunk_log, low = 4u * (blockIdx.x * blockDim.x + threadIdx.x), lead_blocks = g.lead >> chunk_log;
+    if (low >> (L + 1)) return;
+    const uint32_t half = g.chunks >> 1, h0 = blockIdx.y * ACC_RUN, h1 = h0 + ACC_RUN < half ? h0 + ACC_RUN : half;
+    uint32_t upto[4];  // slots in the sum of a place's rows
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+        const uint32_t block = coset_perm(low + u, g.log_rows) >> chunk_log;
+        upto[u] = block < lead_blocks ? 0u : block - lead_blocks;
+    }
+    for (uint32_t m = 0; m < n_mats; m++) {
+        const uint4* const pre = prefix + (size_t)m * g.groups;
+        auto sum = [&](uint32_t n) { return n ? pre[n - 1u] : make_uint4(0, 0, 0, 0); };
+        uint32_t* const* const o = out + 8 + 8 * m;
+        uint32_t *const o0 = o[0] + low, *const o1 = o[1] + low, *const o2 = o[2] + low, *const o3 = o[3] + low;
+        auto write = [&](size_t h, uint4 a, uint4 b, uint4 c, uint4 d) {
+            const size_t i = h << (L + 1);
+            *reinterpret_cast<uint4*>(o0 + i) = make_uint4(a.x, b.x, c.x, d.x);
+            *reinterpret_cast<uint4*>(o1 + i) = make_uint4(a.y, b.y, c.y, d.y);
+            *reinterpret_cast<uint4*>(o2 + i) = make_uint4(a.z, b.z, c.z, d.z);
+            *reinterpret_cast<uint4*>(o3 + i) = make_uint4(a.w, b.w, c.w, d.w);
+        };
+        const uint4 a = sum(upto[0]), b = sum(upto[1]), c = sum(upto[2]), d = sum(upto[3]);
+        for (uint32_t h = h0; h < h1; h++)
+            if (h) write(h, a, b, c, d);
+        if (h0 == 0) {
+            const uint32_t b1 = coset_perm(low + 1u, g.log_rows) >> chunk_log, d1 = coset_perm(low + 3u, g.log_rows) >> chunk_log;
+            write(0, a, sum(b1 < lead_blocks ? 0u : upto[1] + 1u), c, sum(d1 < lead_blocks ? 0u : upto[3] + 1u));
+        }
     }
 }
 
@@ -386,13 +547,31 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     if (rc) return rc;
     rc = stage_ptrs(ctx, (const void* const*)out_cols, (int)((1 + 2 * n_mats) * 4), &d_out);
     if (rc) return rc;
+    auto aligned = [](const uint32_t* const* p, size_t n) {
+        for (size_t k = 0; k < n; k++) if ((uintptr_t)p[k] & 15) return false;
+        return true;
+    };
+    // a group is an aligned block of coset order: lead is the rest of a power of two, so it is a multiple of chunks too
+    const uint32_t chunk_log = 31u - (uint32_t)__builtin_clz(grid->chunks);
+    const bool blocks = grid->chunks == 1u << chunk_log && chunk_log >= 5 && chunk_log <= 8 && grid->log_rows >= chunk_log + 4 && aligned(out_cols, (1 + 2 * (size_t)n_mats) * 4);
+    if (blocks) ZKB_CUDA(ctx, cudaFuncSetAttribute(freivalds_scan_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_OUT_SMEM));
     // work buffers from the stream-ordered pool: lanes in coset order, prefix over groups
     uint4 *lanes = nullptr, *prefix = nullptr;
     ZKB_CUDA(ctx, cudaMallocAsync((void**)&lanes, (size_t)n_lanes * rows * 16, ctx->stream));
     cudaError_t e = cudaMallocAsync((void**)&prefix, (size_t)n_mats * grid->groups * 16, ctx->stream);
     if (e != cudaSuccess) { cudaFreeAsync(lanes, ctx->stream); return set_error(ctx, ZKB_ENOMEM, "zkb_freivalds_acc: %s", cudaGetErrorString(e)); }
     FGrid fg{grid->log_rows, grid->groups, grid->chunks, grid->lead};
-    {
+    auto even = [](const uint32_t* const* p, size_t n) {
+        for (size_t k = 0; k < n; k++) if ((uintptr_t)p[k] & 7) return false;
+        return true;
+    };
+    if (rows >= 1024 && even(base_cols, pq) && even(pre_cols, (size_t)n_mats * pk)) {
+        qm31 bias = qm31_zero();
+        for (uint32_t p = 0; p < pq; p++) bias = qm31_add(bias, qm31_mul_m31(pows[p], 128u));
+        ProfScope prof(ctx, "freivalds_inner_quad_kernel");
+        freivalds_inner_quad_kernel<<<(unsigned)(rows / 1024), 256, 0, ctx->stream>>>(
+            (const uint32_t* const*)d_base, (const uint32_t* const*)d_pre, d_pows, d_pows + pq, fg, pq, pk, n_mats, bias, lanes);
+    } else {
         ProfScope prof(ctx, "freivalds_inner_kernel");
         freivalds_inner_kernel<<<row_pair_blocks(rows), 256, 0, ctx->stream>>>(
             (const uint32_t* const*)d_base, (const uint32_t* const*)d_pre, d_pows, d_pows + pq, fg, pq, pk, n_mats, lanes);
@@ -404,7 +583,11 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
         scan_steps.wide[kind][0] = scan_steps.pw[kind][8];
         for (int k = 1; k < 6; k++) scan_steps.wide[kind][k] = qm31_mul(scan_steps.wide[kind][k - 1], scan_steps.wide[kind][k - 1]);
     }
-    {
+    if (blocks) {
+        ProfScope prof(ctx, "freivalds_scan_out_kernel");
+        freivalds_scan_out_kernel<<<1u << (grid->log_rows - chunk_log - 4), SCAN_OUT_THREADS, SCAN_OUT_SMEM, ctx->stream>>>(lanes, fg, chunk_log, n_mats, scan_steps, prefix,
+                                                                                                                     (uint32_t* const*)d_out);
+    } else {
         ProfScope prof(ctx, "freivalds_group_scan_kernel");
         freivalds_group_scan_kernel<<<(unsigned)(((size_t)grid->groups * 32 + 255) / 256), 256, 0, ctx->stream>>>(lanes, fg, n_mats, scan_steps, prefix);
     }
@@ -412,7 +595,11 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
         ProfScope prof(ctx, "freivalds_prefix_kernel");
         freivalds_prefix_kernel<<<n_mats, 1024, 0, ctx->stream>>>(prefix, grid->groups, reinterpret_cast<uint4*>(ctx->h_small));
     }
-    {
+    if (blocks) {
+        ProfScope prof(ctx, "freivalds_acc_columns_kernel");
+        const dim3 ctas((unsigned)(((2u << (grid->log_rows - chunk_log)) / 4 + 127) / 128), (grid->chunks / 2 + ACC_RUN - 1) / ACC_RUN);
+        freivalds_acc_columns_kernel<<<ctas, 128, 0, ctx->stream>>>(prefix, fg, chunk_log, n_mats, (uint32_t* const*)d_out);
+    } else {
         ProfScope prof(ctx, "freivalds_split_kernel");
         freivalds_split_kernel<<<row_pair_blocks(rows), 256, 0, ctx->stream>>>(lanes, prefix, fg, n_mats, (uint32_t* const*)d_out);
     }
