@@ -178,3 +178,17 @@ def test_eval_at_point_in_runs_of_chunks(ctx, oracle, log_n, n_cols):
     bufs, point = [ctx.upload(c) for c in cols], qm31_array(8390, 2).ravel()
     got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
     assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()
+
+
+@pytest.mark.parametrize("log_n,n_cols", [(4, 3), (5, 1), (5, 33), (6, 17), (7, 9), (8, 5), (8, 700), (9, 2), (9, 301)])
+@pytest.mark.parametrize("blowup", [1, 2, 4])
+def test_transforms_of_short_columns(ctx, oracle, log_n, n_cols, blowup):
+    # 2^5 to 2^9 words: several columns to a warp, the last warp's not all there; extensions into that range and out of it
+    vals = np.stack([m31_column(8600 + c, 1 << log_n) for c in range(n_cols)])
+    cols = [ctx.upload(v) for v in vals]
+    ctx.ifft_cols([c.ptr for c in cols], log_n)
+    coeffs = oracle.interpolate_cols(vals, log_n)
+    assert (np.stack([c.download() for c in cols]) == coeffs).all()
+    outs = [ctx.alloc(1 << (log_n + blowup)) for _ in range(n_cols)]
+    ctx.lde_cols([c.ptr for c in cols], log_n, [o.ptr for o in outs], log_n + blowup)
+    assert (np.stack([o.download() for o in outs]) == oracle.evaluate_cols(coeffs, log_n, log_n + blowup)).all()

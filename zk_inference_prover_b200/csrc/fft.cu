@@ -131,7 +131,7 @@ __global__ void fft_small_kernel(uint32_t* const* __restrict__ dst_cols, const u
 
 // One launch of the plan.
 struct FftStep {
-    int kind;  // 0: generic, 1: radix-32 contiguous (10 layers), 3: contiguous over 12 layers, 4: wide strided (8 layers)
+    int kind;  // 0: generic, 1: radix-32 contiguous (10 layers), 2: short columns whole, 3: contiguous over 12 layers, 4: wide strided (8 layers)
     FftPass generic;
     R32Pass r32;
 };
@@ -140,9 +140,13 @@ struct FftStep {
 // From 2^12 words up (16-byte aligned columns): the twelve-layer contiguous pass, then wide strided passes
 // of up to eight layers (their window slides down over layers already done when the array is short; those
 // layers are switched off). 2^10 and 2^11 words: the ten-layer contiguous pass and a generic pass for the
-// rest. Everything else goes through the generic pass.
+// rest. 2^5 to 2^9 words: one launch that takes several columns a warp. Everything else goes through the generic pass.
 static std::vector<FftStep> plan_steps(int nl, int log_n, bool aligned) {
     std::vector<FftStep> v;
+    if (log_n >= 5 && log_n < 10 && aligned && nl > 0) {
+        v.push_back({2, {}, {0, 0, nl}});
+        return v;
+    }
     if (log_n < 10 || !aligned) {
         int kb = log_n < FFT_CONTIG_LOG ? log_n : FFT_CONTIG_LOG;
         int kf = nl < kb ? nl : kb;
@@ -165,11 +169,8 @@ static std::vector<FftStep> plan_steps(int nl, int log_n, bool aligned) {
         int covered = nl < 10 ? nl : 10;
         v.push_back({1, {}, {0, 0, covered}});
         if (covered < nl) {  // log_n = 11, one layer left
-            int take = nl - covered;
-            int logw = FFT_MAX_TILE_LOG - take;
-            if (logw > 5) logw = 5;
-            if (logw > covered) logw = covered;
-            v.push_back({0, {covered, take, take, logw}, {}});
+            // its two halves in one tile: a CTA a column (as 32 tiles of 64 words, 4,700 columns were 81 us, now TT)
+            v.push_back({0, {covered, 1, 1, covered}, {}});
         }
         return v;
     }
@@ -211,16 +212,17 @@ static int launch_step(zkb_ctx* ctx, uint32_t* const* d_dst, const uint32_t* con
     // The opt-in shared-memory size is a per-device function attribute and the SM count differs between
     // devices, so both are looked up once per device (under a lock: contexts on several devices may be
     // driven from several host threads).
-    const int which = st.kind == 1 ? 0 : st.kind == 3 ? 1 : 2;
-    const size_t smem = which == 0 ? r32_contig_smem(INVERSE) : which == 1 ? r32_c12_smem() : r32_wide_smem();
+    const int which = st.kind == 1 ? 0 : st.kind == 3 ? 1 : st.kind == 2 ? 3 : 2;
+    const size_t smem = which == 0 ? r32_contig_smem(INVERSE) : which == 1 ? r32_c12_smem() : which == 3 ? r32_short_smem() : r32_wide_smem();
     const void* fn = which == 0   ? (const void*)fft_r32_contig_kernel<INVERSE>
                      : which == 1 ? (const void*)fft_r32_contig12_kernel<INVERSE>
+                     : which == 3 ? (const void*)fft_r32_short_kernel<INVERSE>
                                   : (const void*)fft_r32_wide_kernel<INVERSE>;
-    const int threads = which == 0 ? 32 * R32_CONTIG_WARPS : which == 1 ? 32 * R32_C12_WARPS : 256;
+    const int threads = which == 0 || which == 3 ? 32 * R32_CONTIG_WARPS : which == 1 ? 32 * R32_C12_WARPS : 256;
     int ctas = 0, n_sms = 0;
     {
         static std::mutex mu;
-        static int s_ctas[R32_MAX_DEVICES][3][2];  // [device][kernel][forward/inverse]; 0 = not set up
+        static int s_ctas[R32_MAX_DEVICES][4][2];  // [device][kernel][forward/inverse]; 0 = not set up
         static int s_sms[R32_MAX_DEVICES];
         ZKB_CHECK_ARG(ctx, ctx->device >= 0 && ctx->device < R32_MAX_DEVICES);
         std::lock_guard<std::mutex> lock(mu);
@@ -236,6 +238,7 @@ static int launch_step(zkb_ctx* ctx, uint32_t* const* d_dst, const uint32_t* con
     }
     size_t items = which == 0   ? (((size_t)ncols << (log_n - 10)) + R32_CONTIG_WARPS - 1) / R32_CONTIG_WARPS
                    : which == 1 ? ((size_t)ncols << (log_n - 12))
+                   : which == 3 ? ((((size_t)ncols + ((size_t)1 << (10 - log_n)) - 1) >> (10 - log_n)) + R32_CONTIG_WARPS - 1) / R32_CONTIG_WARPS
                                 : ((size_t)ncols << (log_n - 13));
     size_t max_ctas = (size_t)n_sms * ctas;
     unsigned grid = (unsigned)(items < max_ctas ? items : max_ctas);
@@ -247,7 +250,9 @@ static int launch_step(zkb_ctx* ctx, uint32_t* const* d_dst, const uint32_t* con
     const uint32_t* tower = INVERSE ? ctx->itw2 : ctx->tw2;
     ProfScope prof(ctx, which == 2 ? (INVERSE ? "fft_r32_wide_kernel<inverse>" : "fft_r32_wide_kernel<forward>")
                                    : (INVERSE ? "fft_r32_contig_kernel<inverse>" : "fft_r32_contig_kernel<forward>"));
-    if (which == 0)
+    if (which == 3)
+        fft_r32_short_kernel<INVERSE><<<grid, threads, smem, ctx->stream>>>(d_dst, d_src, src_mask, ncols, dom_log, st.r32.act_hi, tower, scale);
+    else if (which == 0)
         fft_r32_contig_kernel<INVERSE><<<grid, threads, smem, ctx->stream>>>(d_dst, d_src, src_mask, ncols, log_n, dom_log, st.r32, tower, scale);
     else if (which == 1)
         fft_r32_contig12_kernel<INVERSE><<<grid, threads, smem, ctx->stream>>>(d_dst, d_src, src_mask, ncols, log_n, dom_log, st.r32, tower, scale,

@@ -321,6 +321,105 @@ __global__ void __launch_bounds__(32 * R32_CONTIG_WARPS, 16 / R32_CONTIG_WARPS)
     cp_async_wait<0>();
 }
 
+// The same for whole columns of 2^5 .. 2^9 words (dom_log), as many of them to a warp's 1024 words as fit: the layers above the column's are switched
+// off and every unit has the same twiddles. Segments have tens of thousands of such columns; a CTA a column and a barrier a layer
+// was 92 us for 29,000 of 2^8, this 22.
+template <bool INVERSE>
+__global__ void __launch_bounds__(32 * R32_CONTIG_WARPS, 16 / R32_CONTIG_WARPS)
+    fft_r32_short_kernel(uint32_t* const* __restrict__ dst_cols, const uint32_t* const* __restrict__ src_cols, uint32_t src_mask, int ncols, int dom_log,
+                         int act_hi, const uint32_t* __restrict__ tower, uint32_t scale) {
+    extern __shared__ __align__(16) uint32_t dyn_smem[];
+    const int warp = threadIdx.x >> 5, tm = threadIdx.x & 31;
+    constexpr int BUF = R32_PITCH * 32;
+    uint32_t* const buf0 = dyn_smem + (2 * warp) * BUF;
+    uint32_t* const tw = dyn_smem + 2 * R32_CONTIG_WARPS * BUF;
+    // twiddle k of a layer's run is that of the column's pair k mod their number; layout as in the pass above
+    for (int k = threadIdx.x; k < 511; k += 32 * R32_CONTIG_WARPS) {
+        const int up = k < 480 ? 0 : 1;
+        int jj, h;
+        if (up) { uniform_slot(k - 480, jj, h); jj += 5; }
+        else { jj = 1 + (k >= 256) + (k >= 384) + (k >= 448); h = k - (512 - (1024 >> jj)); }
+        if (jj < dom_log) tw[k] = tower[(1u << (dom_log - jj - 1)) + (h & ((1u << (dom_log - jj - 1)) - 1u))];
+    }
+    __syncthreads();
+    const int per_log = 10 - dom_log, row_log = dom_log - 5;  // columns a unit, rows of 32 words a column
+    const int units = (ncols + (1 << per_log) - 1) >> per_log, stride = (int)gridDim.x * R32_CONTIG_WARPS;
+    auto column = [&](int unit, int row) { return (unit << per_log) + (row >> row_log); };
+    auto offset = [&](int row) { return (uint32_t)(row & ((1 << row_log) - 1)) << 5; };
+    auto prefetch = [&](int b, int unit) {
+        uint32_t* buf = buf0 + b * BUF;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int r = k * 4 + (tm >> 3), q = tm & 7, col = column(unit, r);
+            cp_async16(buf + r * R32_PITCH + (q << 2), src_cols[col < ncols ? col : ncols - 1] + ((offset(r) + q * 4) & src_mask));
+        }
+    };
+    const uint32_t* const tb_uni[5] = {tw + 480, tw + 496, tw + 504, tw + 508, tw + 510};
+    const uint32_t* const tb_lane[5] = {tw + 8 * tm, tw + 8 * tm, tw + 256 + 4 * tm, tw + 384 + 2 * tm, tw + 448 + tm};
+    int cur = 0, unit = (int)blockIdx.x * R32_CONTIG_WARPS + warp;
+    if (unit < units) prefetch(0, unit);
+    cp_async_commit();
+    for (; unit < units; unit += stride) {
+        if (unit + stride < units) prefetch(cur ^ 1, unit + stride);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncwarp();
+        uint32_t* __restrict__ s = buf0 + cur * BUF;
+        uint4* const row = reinterpret_cast<uint4*>(s + R32_PITCH * tm);
+        uint32_t v[32];
+        auto load_rows = [&] {
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const uint4 x = row[q];
+                v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+            }
+        };
+        auto store_rows = [&] {
+#pragma unroll
+            for (int q = 0; q < 8; q++) row[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            __syncwarp();
+        };
+        if (!INVERSE) {
+            if (act_hi > 5) {
+#pragma unroll
+                for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
+                radix32_stage<false, false>(v, tb_uni, 5, 0, act_hi);
+#pragma unroll
+                for (int p = 0; p < 32; p++) s[R32_PITCH * p + tm] = v[p];
+                __syncwarp();
+            }
+            load_rows();
+            radix32_stage<false, true>(v, tb_lane, 0, 0, act_hi);
+        } else {
+            load_rows();
+            radix32_stage<true, true>(v, tb_lane, 0, 0, act_hi);
+            if (act_hi > 5) {
+                store_rows();
+#pragma unroll
+                for (int p = 0; p < 32; p++) v[p] = s[R32_PITCH * p + tm];
+                radix32_stage<true, false>(v, tb_uni, 5, 0, act_hi);
+#pragma unroll
+                for (int p = 0; p < 32; p++) s[R32_PITCH * p + tm] = scale ? m31_mul(v[p], scale) : v[p];
+                __syncwarp();
+            } else if (scale) {
+#pragma unroll
+                for (int p = 0; p < 32; p++) v[p] = m31_mul(v[p], scale);
+            }
+        }
+        if (!INVERSE || act_hi <= 5) store_rows();
+        const int j = tm >> 3, c = tm & 7;
+#pragma unroll
+        for (int st = 0; st < 8; st++) {
+            const int r = 4 * st + j, col = column(unit, r);
+            if (col < ncols) *reinterpret_cast<uint4*>(dst_cols[col] + offset(r) + 4 * c) = *reinterpret_cast<const uint4*>(s + R32_PITCH * r + 4 * c);
+        }
+        __syncwarp();  // the exchange reads are done before this buffer is refilled
+        cur ^= 1;
+    }
+    cp_async_wait<0>();
+}
+__host__ __device__ constexpr size_t r32_short_smem() { return (size_t)(2 * R32_CONTIG_WARPS * R32_PITCH * 32 + R32_TW_CONTIG) * sizeof(uint32_t); }
+
 // ---------------------------------------------------------------------------------------------------------
 // Wide strided pass: window bits [lo, lo+8), lo >= 5. A CTA of 256 threads owns a tile of 256 rows x 32
 // consecutive words, so every global access is a full 128-byte line (a row of the tile), in both directions.
