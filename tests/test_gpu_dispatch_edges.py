@@ -192,3 +192,15 @@ def test_transforms_of_short_columns(ctx, oracle, log_n, n_cols, blowup):
     outs = [ctx.alloc(1 << (log_n + blowup)) for _ in range(n_cols)]
     ctx.lde_cols([c.ptr for c in cols], log_n, [o.ptr for o in outs], log_n + blowup)
     assert (np.stack([o.download() for o in outs]) == oracle.evaluate_cols(coeffs, log_n, log_n + blowup)).all()
+
+
+@pytest.mark.parametrize("with_prev", [False, True])
+@pytest.mark.parametrize("log_size,ncols", [(0, 64), (3, 63), (3, 65), (4, 80), (5, 81), (6, 95), (7, 96), (13, 64), (13, 97), (14, 64), (2, 1000)])
+def test_merkle_layers_of_many_columns(ctx, oracle, log_size, ncols, with_prev):
+    # from 64 columns on, up to 2^13 nodes, a warp brings the blocks of sixteen nodes: even and odd numbers of blocks, whole and partial last ones
+    cols = [m31_column(8700 + c, 1 << log_size) for c in range(ncols)]
+    prev = m31_column(8690, 16 << log_size).reshape(-1, 8) if with_prev else None
+    bufs, pb, out = [ctx.upload(c) for c in cols], ctx.upload(prev) if with_prev else None, ctx.alloc(8 << log_size)
+    for m31 in (False, True):
+        ctx.merkle_layer(log_size, pb.ptr if pb else 0, [b.ptr for b in bufs], out.ptr, m31_out=m31)
+        assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, prev, cols, m31=m31)).all()

