@@ -101,3 +101,30 @@ def test_signed_product_stays_in_range_and_in_its_class(tmp_path):
         for t in ts:
             q = lib.mul_signed(ctypes.c_uint32(v & 0xffffffff), ctypes.c_uint32(t))
             assert -P <= q - ((q >> 31) << 32) <= P - 1 and lib.unsign(ctypes.c_uint32(q)) == v * t % P
+
+
+SUMS = SHARED + """
+static qm31 q(const unsigned* a) { return {{a[0], a[1], a[2], a[3]}}; }
+extern "C" void sums(const unsigned* x, const unsigned* y, const unsigned* z, int n, unsigned* o) {
+    qm31_sum s = qm31_sum_zero();
+    for (int k = 0; k < n; k++) s.add_product(q(x), q(y));
+    const qm31 r[4] = {qm31_mul_add(q(x), q(y), q(z)), qm31_dot2(q(x), q(y), q(z), q(y)), qm31_dot2_m31(q(x), y[0], q(z), y[1]), s.value()};
+    for (int k = 0; k < 16; k++) o[k] = r[k / 4].c[k % 4];
+}
+"""
+
+
+def test_sums_of_products_at_the_top_of_the_range(tmp_path):
+    (tmp_path / "s.cpp").write_text(SUMS)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", str(tmp_path / "s.so"), str(tmp_path / "s.cpp")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "s.so"))
+    rng = np.random.default_rng(4)
+    top, word = [P - 1] * 4, lambda v: np.array(v, np.uint32).ctypes.data_as(ctypes.c_void_p)
+    cases = [(X, Y, top), (top, top, top), ([0, 0, 0, 0], top, top), ([P - 1, 0, P - 1, 0], [P - 1, P - 1, 0, P - 1], [0] * 4)]
+    cases += [tuple([int(v) for v in rng.integers(0, P, 4)] for _ in range(3)) for _ in range(200)]
+    for x, y, z in cases:
+        out = np.zeros(16, np.uint32)
+        lib.sums(word(x), word(y), word(z), 5, out.ctypes.data_as(ctypes.c_void_p))
+        xy, zy = _mul(x, y), _mul(z, y)
+        want = [(a + b) % P for a, b in zip(xy, z)] + [(a + b) % P for a, b in zip(xy, zy)] + [(a * y[0] + b * y[1]) % P for a, b in zip(x, z)] + [5 * a % P for a in xy]
+        assert out.tolist() == want

@@ -271,19 +271,19 @@ __device__ __forceinline__ void scan_rows(uint32_t left, bool first, const qm31*
 #pragma unroll
     for (uint32_t k = 0; k < 8; k++)
         if (k < n_here) {
-            acc = qm31_add(qm31_mul(acc, step), q_of(get(r0 + k)));
+            acc = qm31_mul_add(acc, step, q_of(get(r0 + k)));
             if (IN_PLACE) put(r0 + k, u_of(acc));
             else y[IN_PLACE ? 0 : k] = acc;
         }
     // The value after a lane's rows, exact for lanes whose rows before them are all there: only the last lane with rows may
     // have fewer than eight, and nothing is taken from it or from the ones after.
-    qm31 B = lane == 0 && !first ? qm31_add(acc, qm31_mul(end, pw[n_here])) : acc;
+    qm31 B = lane == 0 && !first ? qm31_mul_add(end, pw[n_here], acc) : acc;
 #pragma unroll
     for (int k = 0; k < 5; k++) {
         qm31 b1;
 #pragma unroll
         for (int c = 0; c < 4; c++) b1.c[c] = __shfl_up_sync(0xffffffffu, B.c[c], 1 << k);
-        if ((int)lane >= (1 << k)) B = qm31_add(qm31_mul(b1, wide[k]), B);
+        if ((int)lane >= (1 << k)) B = qm31_mul_add(b1, wide[k], B);
     }
     qm31 carry;  // into this lane: the value at the end of the previous one
 #pragma unroll
@@ -292,7 +292,7 @@ __device__ __forceinline__ void scan_rows(uint32_t left, bool first, const qm31*
 #pragma unroll
     for (uint32_t k = 0; k < 8; k++)
         if (k < n_here) {
-            acc = qm31_add(IN_PLACE ? q_of(get(r0 + k)) : y[IN_PLACE ? 0 : k], qm31_mul(carry, pw[k + 1]));
+            acc = qm31_mul_add(carry, pw[k + 1], IN_PLACE ? q_of(get(r0 + k)) : y[IN_PLACE ? 0 : k]);
             put(r0 + k, u_of(acc));
         }
     const int from = (int)((left < 256u ? left : 256u) - 1u) >> 3;  // the lane of the last row

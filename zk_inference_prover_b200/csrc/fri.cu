@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256) fold_circle_kernel4(Secure4 dst, Secure4C
 #pragma unroll
         for (int e = 0; e < 4; e++) {
             const qm31 de{{(&d[0].x)[e], (&d[1].x)[e], (&d[2].x)[e], (&d[3].x)[e]}};
-            f[e] = qm31_add(qm31_mul(de, alpha_sq), f[e]);
+            f[e] = qm31_mul_add(de, alpha_sq, f[e]);
         }
     }
 #pragma unroll
@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(256) fold_circle_kernel2(Secure4 dst, Secure4C
             uint2 v = reinterpret_cast<const uint2*>(dst.c[k])[i2];
             d0.c[k] = v.x; d1.c[k] = v.y;
         }
-        r0 = qm31_add(qm31_mul(d0, alpha_sq), f0);
-        r1 = qm31_add(qm31_mul(d1, alpha_sq), f1);
+        r0 = qm31_mul_add(d0, alpha_sq, f0);
+        r1 = qm31_mul_add(d1, alpha_sq, f1);
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) reinterpret_cast<uint2*>(dst.c[k])[i2] = make_uint2(r0.c[k], r1.c[k]);
@@ -197,7 +197,7 @@ __global__ void fold_small_kernel(Secure4 out, Secure4C in, int n_out, qm31 alph
     qm31 r = fold_pair(in, i, its[i], alpha);
     if (accumulate) {
         qm31 d{{out.c[0][i], out.c[1][i], out.c[2][i], out.c[3][i]}};
-        r = qm31_add(qm31_mul(d, alpha_sq), r);
+        r = qm31_mul_add(d, alpha_sq, r);
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) out.c[k][i] = r.c[k];

@@ -31,10 +31,10 @@ __global__ void __launch_bounds__(256) next_layer_kernel(const uint32_t* __restr
         n = qm31_add(d0, d1);
     } else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) {
         uint2 m = reinterpret_cast<const uint2*>(num)[i];
-        n = qm31_add(qm31_mul_m31(d1, m.x), qm31_mul_m31(d0, m.y));
+        n = qm31_dot2_m31(d1, m.x, d0, m.y);
     } else {
         qm31 n0 = ldq(num, 2 * i), n1 = ldq(num, 2 * i + 1);
-        n = qm31_add(qm31_mul(d1, n0), qm31_mul(d0, n1));
+        n = qm31_dot2(d1, n0, d0, n1);
     }
     stq(num_out, i, n);
     stq(den_out, i, qm31_mul(d0, d1));
@@ -77,14 +77,14 @@ __global__ void __launch_bounds__(256) gkr_sum_kernel(const uint32_t* __restrict
                 uint2 a = reinterpret_cast<const uint2*>(num)[i];
                 uint2 b = reinterpret_cast<const uint2*>(num)[n_terms + i];
                 uint32_t n20 = m31_sub(m31_dbl(b.x), a.x), n21 = m31_sub(m31_dbl(b.y), a.y);
-                n0 = qm31_add(qm31_mul_m31(d01, a.x), qm31_mul_m31(d00, a.y));
-                n2 = qm31_add(qm31_mul_m31(d21, n20), qm31_mul_m31(d20, n21));
+                n0 = qm31_dot2_m31(d01, a.x, d00, a.y);
+                n2 = qm31_dot2_m31(d21, n20, d20, n21);
             } else {
                 qm31 n00 = ldq(num, 2 * i), n01 = ldq(num, 2 * i + 1);
                 qm31 n10 = ldq(num, 2 * (n_terms + i)), n11 = ldq(num, 2 * (n_terms + i) + 1);
                 qm31 n20 = qm31_sub(qm31_dbl(n10), n00), n21 = qm31_sub(qm31_dbl(n11), n01);
-                n0 = qm31_add(qm31_mul(d01, n00), qm31_mul(d00, n01));
-                n2 = qm31_add(qm31_mul(d21, n20), qm31_mul(d20, n21));
+                n0 = qm31_dot2(d01, n00, d00, n01);
+                n2 = qm31_dot2(d21, n20, d20, n21);
             }
             t0 = qm31_add(n0, qm31_mul(lambda, qm31_mul(d00, d01)));
             t2 = qm31_add(n2, qm31_mul(lambda, qm31_mul(d20, d21)));
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) mle_fix_qm31_kernel(const uint32_t* __res
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= half) return;
     qm31 a = ldq(in, i), b = ldq(in, i + half);
-    stq(out, i, qm31_add(qm31_mul(r, qm31_sub(b, a)), a));
+    stq(out, i, qm31_mul_add(r, qm31_sub(b, a), a));
 }
 __global__ void __launch_bounds__(256) mle_fix_m31_kernel(const uint32_t* __restrict__ in, size_t half, qm31 r,
                                                           uint32_t* __restrict__ out) {

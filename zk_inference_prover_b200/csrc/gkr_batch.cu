@@ -38,7 +38,7 @@ __device__ __forceinline__ qm31 ldqb(const uint32_t* p, size_t i) {
 __device__ __forceinline__ void stqb(uint32_t* p, size_t i, qm31 v) {
     reinterpret_cast<uint4*>(p)[i] = make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]);
 }
-__device__ __forceinline__ qm31 foldb(qm31 r, qm31 a, qm31 b) { return qm31_add(qm31_mul(r, qm31_sub(b, a)), a); }
+__device__ __forceinline__ qm31 foldb(qm31 r, qm31 a, qm31 b) { return qm31_mul_add(r, qm31_sub(b, a), a); }
 __device__ __forceinline__ qm31 fold_m31(qm31 r, uint32_t a, uint32_t b) {
     qm31 v = qm31_mul_m31(r, m31_sub(b, a));
     v.c[0] = m31_add(v.c[0], a);
@@ -69,16 +69,19 @@ __device__ __forceinline__ void term(const qm31 d[4], const qm31 nu[4], qm31 lam
         n2 = qm31_add(d20, d21);
     } else {
         qm31 n20 = qm31_sub(qm31_dbl(nu[2]), nu[0]), n21 = qm31_sub(qm31_dbl(nu[3]), nu[1]);
-        n0 = qm31_add(qm31_mul(d[1], nu[0]), qm31_mul(d[0], nu[1]));
-        n2 = qm31_add(qm31_mul(d21, n20), qm31_mul(d20, n21));
+        // n0 d1 + n1 d0 + lambda d0 d1 as (n0 + lambda d0) d1 + n1 d0
+        t0 = qm31_dot2(qm31_mul_add(lambda, d[0], nu[0]), d[1], nu[1], d[0]);
+        t2 = qm31_dot2(qm31_mul_add(lambda, d20, n20), d21, n21, d20);
+        return;
     }
-    t0 = qm31_add(n0, qm31_mul(lambda, qm31_mul(d[0], d[1])));
-    t2 = qm31_add(n2, qm31_mul(lambda, qm31_mul(d20, d21)));
+    t0 = qm31_mul_add(lambda, qm31_mul(d[0], d[1]), n0);
+    t2 = qm31_mul_add(lambda, qm31_mul(d20, d21), n2);
 }
 
 template <int KIND>
 __device__ __forceinline__ void item_sums(const GkrBatchItem& it, size_t first, size_t stride, qm31 r, const uint32_t* __restrict__ eq, qm31 lambda,
                                           qm31& s0, qm31& s2) {
+    qm31_sum a0 = qm31_sum_zero(), a2 = qm31_sum_zero();
     if (it.mode == 0) {
         const size_t nt = it.n / 4;  // entries (0, i, b) at 2i + b, (1, i, b) at 2(nt + i) + b
         for (size_t i = first; i < nt; i += stride) {
@@ -93,8 +96,8 @@ __device__ __forceinline__ void item_sums(const GkrBatchItem& it, size_t first, 
             qm31 t0, t2;
             term<KIND>(d, nu, lambda, t0, t2);
             qm31 e = ldqb(eq, i);
-            s0 = qm31_add(s0, qm31_mul(e, t0));
-            s2 = qm31_add(s2, qm31_mul(e, t2));
+            a0.add_product(e, t0);
+            a2.add_product(e, t2);
         }
     } else {
         const size_t half = it.n / 2, nt = half / 4;
@@ -116,10 +119,12 @@ __device__ __forceinline__ void item_sums(const GkrBatchItem& it, size_t first, 
             qm31 t0, t2;
             term<KIND>(d, nu, lambda, t0, t2);
             qm31 e = ldqb(eq, i);
-            s0 = qm31_add(s0, qm31_mul(e, t0));
-            s2 = qm31_add(s2, qm31_mul(e, t2));
+            a0.add_product(e, t0);
+            a2.add_product(e, t2);
         }
     }
+    s0 = qm31_add(s0, a0.value());
+    s2 = qm31_add(s2, a2.value());
 }
 
 // ---- the transcript step of a round, for a layer enqueued at once

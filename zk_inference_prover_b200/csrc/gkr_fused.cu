@@ -20,7 +20,7 @@ __device__ __forceinline__ qm31 ldq2(const uint32_t* __restrict__ p, size_t i) {
 __device__ __forceinline__ void stq2(uint32_t* __restrict__ p, size_t i, qm31 v) {
     reinterpret_cast<uint4*>(p)[i] = make_uint4(v.c[0], v.c[1], v.c[2], v.c[3]);
 }
-__device__ __forceinline__ qm31 fold_q(qm31 r, qm31 a, qm31 b) { return qm31_add(qm31_mul(r, qm31_sub(b, a)), a); }
+__device__ __forceinline__ qm31 fold_q(qm31 r, qm31 a, qm31 b) { return qm31_mul_add(r, qm31_sub(b, a), a); }
 
 __device__ __forceinline__ qm31 warp_sum2(qm31 v) {
 #pragma unroll
@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(256) fold_sum_kernel(const uint32_t* __restric
                 n2 = qm31_add(d20, d21);
             } else {
                 qm31 n20 = qm31_sub(qm31_dbl(nu[2]), nu[0]), n21 = qm31_sub(qm31_dbl(nu[3]), nu[1]);
-                n0 = qm31_add(qm31_mul(d[1], nu[0]), qm31_mul(d[0], nu[1]));
-                n2 = qm31_add(qm31_mul(d21, n20), qm31_mul(d20, n21));
+                n0 = qm31_dot2(d[1], nu[0], d[0], nu[1]);
+                n2 = qm31_dot2(d21, n20, d20, n21);
             }
             t0 = qm31_add(n0, qm31_mul(lambda, qm31_mul(d[0], d[1])));
             t2 = qm31_add(n2, qm31_mul(lambda, qm31_mul(d20, d21)));

@@ -191,7 +191,7 @@ __device__ __forceinline__ qm31 step_level(TrSm& t, const uint4 e, uint32_t basi
     char* const base = reinterpret_cast<char*>(&t);
     const qm31 x = ldq_r(base + e.x, 0);
     const qm31 z = qm31_add(ldq_r(base + (e.y & 0xffffu) + e.w * basis_off, 0), ldq_r(base + (e.y >> 16), 0));
-    const qm31 m = qm31_add(qm31_mul(x, z), ldq_r(base + (e.z & 0xffffu), 0));
+    const qm31 m = qm31_mul_add(x, z, ldq_r(base + (e.z & 0xffffu), 0));
     stq_r(base + (e.z >> 16), 0, m);
     __syncwarp();
     return m;
@@ -365,11 +365,11 @@ __device__ __forceinline__ void tr_update(TrSm& t, const qm31* B, uint32_t basis
 template <int KIND>
 __device__ __forceinline__ qm31 term_at(qm31 d0, qm31 d1, qm31 n0, qm31 n1, qm31 lambda) {
     if (KIND == ZKB_GKR_GRAND_PRODUCT) return qm31_mul(d0, d1);
-    if (KIND == ZKB_GKR_LOGUP_SINGLES) return qm31_add(qm31_add(d0, d1), qm31_mul(lambda, qm31_mul(d0, d1)));
-    return qm31_add(qm31_mul(qm31_add(n0, qm31_mul(lambda, d0)), d1), qm31_mul(n1, d0));
+    if (KIND == ZKB_GKR_LOGUP_SINGLES) return qm31_mul_add(lambda, qm31_mul(d0, d1), qm31_add(d0, d1));
+    return qm31_dot2(qm31_mul_add(lambda, d0, n0), d1, n1, d0);
 }
 __device__ __forceinline__ qm31 at_two(qm31 v0, qm31 v1) { return qm31_sub(qm31_dbl(v1), v0); }
-__device__ __forceinline__ qm31 fold_q(qm31 r, qm31 a, qm31 b) { return qm31_add(qm31_mul(r, qm31_sub(b, a)), a); }
+__device__ __forceinline__ qm31 fold_q(qm31 r, qm31 a, qm31 b) { return qm31_mul_add(r, qm31_sub(b, a), a); }
 __device__ __forceinline__ qm31 fold_m(qm31 r, uint32_t a, uint32_t b) {
     qm31 v = qm31_mul_m31(r, m31_sub(b, a));
     v.c[0] = m31_add(v.c[0], a);
@@ -478,17 +478,17 @@ __global__ void __launch_bounds__(ROUND_THREADS, 2) res_round_kernel(const __gri
     const size_t n_chunks = a.nt >> a.chunk_log;
     for (size_t ck = blockIdx.x; ck < n_chunks; ck += gridDim.x) {
         const size_t begin = ck << a.chunk_log;
-        qm31 c0 = qm31_zero(), c2 = qm31_zero();
+        qm31_sum c0 = qm31_sum_zero(), c2 = qm31_sum_zero();
         for (size_t i = begin + tid; i < begin + ((size_t)1 << a.chunk_log); i += ROUND_THREADS) {
             qm31 t0, t2;
             const qm31 e = ldq_r(a.eq_low, i & ((1u << EQ_LOW) - 1));
             pass_term<KIND, FOLD, true>(a.num, a.den, a.num_out, a.den_out, a.nt, i, r, lambda, t0, t2);
-            c0 = qm31_add(c0, qm31_mul(e, t0));
-            c2 = qm31_add(c2, qm31_mul(e, t2));
+            c0.add_product(e, t0);
+            c2.add_product(e, t2);
         }
         const qm31 eh = ldq_r(a.eq_high, begin >> EQ_LOW);
-        s0 = qm31_add(s0, qm31_mul(eh, c0));
-        s2 = qm31_add(s2, qm31_mul(eh, c2));
+        s0 = qm31_add(s0, qm31_mul(eh, c0.value()));
+        s2 = qm31_add(s2, qm31_mul(eh, c2.value()));
     }
     s0 = warp_sum_q(s0);
     s2 = warp_sum_q(s2);

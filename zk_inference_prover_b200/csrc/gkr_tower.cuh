@@ -13,8 +13,8 @@ template <int KIND>
 __device__ __forceinline__ void tower_pair(qm31 n0, qm31 n1, qm31 d0, qm31 d1, qm31& n, qm31& d) {
     d = qm31_mul(d0, d1);
     if (KIND == ZKB_GKR_LOGUP_SINGLES) n = qm31_add(d0, d1);
-    else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) n = qm31_add(qm31_mul_m31(d1, n0.c[0]), qm31_mul_m31(d0, n1.c[0]));
-    else if (KIND == ZKB_GKR_LOGUP_GENERIC) n = qm31_add(qm31_mul(d1, n0), qm31_mul(d0, n1));
+    else if (KIND == ZKB_GKR_LOGUP_MULTIPLICITIES) n = qm31_dot2_m31(d1, n0.c[0], d0, n1.c[0]);
+    else if (KIND == ZKB_GKR_LOGUP_GENERIC) n = qm31_dot2(d1, n0, d0, n1);
     else n = qm31_zero();
 }
 __device__ __forceinline__ qm31 tower_ld(const void* p, size_t i) {

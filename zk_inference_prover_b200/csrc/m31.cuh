@@ -116,17 +116,51 @@ ZK_HD bool qm31_is_zero(qm31 x) { return (x.c[0] | x.c[1] | x.c[2] | x.c[3]) == 
 // (A + B u)(C + D u) = (AC + (2+i) BD) + (AD + BC) u, qm31.rs:80-88. (2+i) D = e0 + e1 i is formed first, so that every output
 // coordinate is four 62-bit products and one fold: folding BD before it is multiplied by 2+i is two folds more, on the longest
 // path (233 -> 319 G products/s over all SMs, latency 188 -> 163 cycles). Subtracted products take p - x for x. 4 p^2 < 2^64.
-ZK_HD qm31 qm31_mul(qm31 x, qm31 y) {
+// What is in r (at most 2^34 a coordinate) is added: 4 p^2 = 2^64 - 2^34 + 4.
+ZK_HD void qm31_add_products(uint64_t (&r)[4], qm31 x, qm31 y) {
     const uint32_t e0 = m31_sub(m31_dbl(y.c[2]), y.c[3]), e1 = m31_add(y.c[2], m31_dbl(y.c[3]));
     const uint32_t n1 = P - x.c[1], n3 = P - x.c[3];
     const uint64_t x0 = x.c[0], x1 = x.c[1], x2 = x.c[2], x3 = x.c[3];
-    uint64_t r0 = x0 * y.c[0] + (uint64_t)n1 * y.c[1] + x2 * e0 + (uint64_t)n3 * e1;
-    uint64_t r1 = x0 * y.c[1] + x1 * y.c[0] + x2 * e1 + x3 * e0;
-    uint64_t r2 = x0 * y.c[2] + (uint64_t)n1 * y.c[3] + x2 * y.c[0] + (uint64_t)n3 * y.c[1];
-    uint64_t r3 = x0 * y.c[3] + x1 * y.c[2] + x2 * y.c[1] + x3 * y.c[0];
-    return {{m31_reduce64(r0), m31_reduce64(r1), m31_reduce64(r2), m31_reduce64(r3)}};
+    r[0] += x0 * y.c[0] + (uint64_t)n1 * y.c[1] + x2 * e0 + (uint64_t)n3 * e1;
+    r[1] += x0 * y.c[1] + x1 * y.c[0] + x2 * e1 + x3 * e0;
+    r[2] += x0 * y.c[2] + (uint64_t)n1 * y.c[3] + x2 * y.c[0] + (uint64_t)n3 * y.c[1];
+    r[3] += x0 * y.c[3] + x1 * y.c[2] + x2 * y.c[1] + x3 * y.c[0];
+}
+ZK_HD qm31 qm31_reduce64(const uint64_t (&r)[4]) { return {{m31_reduce64(r[0]), m31_reduce64(r[1]), m31_reduce64(r[2]), m31_reduce64(r[3])}}; }
+ZK_HD qm31 qm31_mul(qm31 x, qm31 y) {
+    uint64_t r[4] = {0, 0, 0, 0};
+    qm31_add_products(r, x, y);
+    return qm31_reduce64(r);
+}
+// x y + z: the addition is an operand of the first multiply-add
+ZK_HD qm31 qm31_mul_add(qm31 x, qm31 y, qm31 z) {
+    uint64_t r[4] = {z.c[0], z.c[1], z.c[2], z.c[3]};
+    qm31_add_products(r, x, y);
+    return qm31_reduce64(r);
 }
 ZK_HD qm31 qm31_sqr(qm31 x) { return qm31_mul(x, x); }
+// A sum of secure products, its coordinates folded (< 2^34) and not reduced. Adding a product costs its sixteen multiply-adds and four folds; the
+// reductions and additions that a product and a sum of its own would take, half of their ALU instructions, come once at the end.
+struct qm31_sum {
+    uint64_t c[4];
+    ZK_HD void add_product(qm31 x, qm31 y) {
+        qm31_add_products(c, x, y);
+        for (int k = 0; k < 4; k++) c[k] = m31_fold64(c[k]);
+    }
+    ZK_HD qm31 value() const { return qm31_reduce64(c); }
+};
+ZK_HD qm31_sum qm31_sum_zero() { return {{0, 0, 0, 0}}; }
+// x0 y0 + x1 y1
+ZK_HD qm31 qm31_dot2(qm31 x0, qm31 y0, qm31 x1, qm31 y1) {
+    qm31_sum s = qm31_sum_zero();
+    s.add_product(x0, y0);
+    qm31_add_products(s.c, x1, y1);
+    return s.value();
+}
+ZK_HD qm31 qm31_dot2_m31(qm31 x0, uint32_t y0, qm31 x1, uint32_t y1) {
+    return {{m31_reduce64((uint64_t)x0.c[0] * y0 + (uint64_t)x1.c[0] * y1), m31_reduce64((uint64_t)x0.c[1] * y0 + (uint64_t)x1.c[1] * y1),
+             m31_reduce64((uint64_t)x0.c[2] * y0 + (uint64_t)x1.c[2] * y1), m31_reduce64((uint64_t)x0.c[3] * y0 + (uint64_t)x1.c[3] * y1)}};
+}
 ZK_HD qm31 qm31_mul_cm31(qm31 x, cm31 y) {
     cm31 a = cm31_mul({x.c[0], x.c[1]}, y), b = cm31_mul({x.c[2], x.c[3]}, y);
     return {{a.a, a.b, b.a, b.b}};
