@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(int log_size, const u
     store_hash(out, i, h, m31_out != 0);
 }
 
-// The same node hash for layers of at most 2^13 nodes, four lanes to a node (b2s_compress_quad in channel.cuh). Such a layer is
+// The same node hash for layers of at most 2^13 nodes and fewer than 64 columns, four lanes to a node (b2s_compress_quad in channel.cuh). Such a layer is
 // bound by the latency of its compressions, and by fetching their code where it is one of a few: a quad issues a quarter of
 // a thread's instructions from a quarter of the code. A lane brings four of a block's sixteen words; a block's words
 // and the addresses of the next one's are on their way while the block before is hashed. A tree of 2^16 leaves built layer by

@@ -18,7 +18,7 @@
 //     result, and, by the CTA that finishes last, the transcript step; the next launch is a programmatic dependent of it.
 //   * eq(., point) is never written out for these: the terms are taken in chunks of at most 2^11 with one factor in common,
 //     eq = A[low 11 bits] B[the rest], so a pass reads a table of 32 KB and multiplies by B once per chunk.
-// Measured (one instance): 2^10 fractions 906 -> 318 us, 2^24 fractions 7.95 -> 3.61 ms. Of the latter's 276 rounds the chain kernel takes
+// Measured (one instance): 2^10 fractions 906 -> 314 us, 2^24 fractions 7.95 -> 3.36 ms. Of the latter's 276 rounds the chain kernel takes
 // 199 in 1.60 ms, 8 us each with the layers' begins and ends; 77 are launches.
 #include <algorithm>
 #include <vector>
