@@ -58,9 +58,11 @@ def test_oracle_claims_are_the_freivalds_identity(oracle, tokens, n_in, n_outs, 
         assert (cols[8 + 8 * m:12 + 8 * m, last] == claims[m]).all()
 
 
-# groups of 32 to 256 rows, a power of two, in sixteen blocks of coset order and more (with and without lead rows), and what lies around that
+# groups of 32 to 256 rows, a power of two (with and without lead rows), and what lies around that; then 2^19 rows, where the inner products go from two
+# rows a thread to four at eight columns a matrix and from one tile of columns to two above 64, and where scan and split go in one with groups
+# of 256 rows and at most a quarter of lead rows (the last two: the quarter, and one group less)
 BLOCKS = [(5, 16, [70, 33], 32), (5, 15, [70], 32), (8, 12, [300], 64), (40, 100, [256, 100, 31], 256), (3, 17, [600], 128), (2, 20, [520], 512), (9, 8, [64], 32),
-          (9, 60, [64], 33)]
+          (9, 60, [64], 33), (9, 2048, [1792, 100], 256), (300, 2047, [2048, 100], 256), (3, 2600, [8500], 128), (3, 1536, [300, 300, 20], 256), (3, 1535, [2048], 256)]
 
 
 @pytest.mark.gpu

@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) freivalds_group_scan_kernel(uint4* __rest
     }
 }
 
-// Scan and split in one, where a group is 2^b rows, 32 to 256 of them: then it is an aligned block of coset order, and in committed order the
+// Scan and split in one, where a group is 2^b rows, at most 256 of them (the call takes it for 256): then it is an aligned block of coset order, and in committed order the
 // blocks whose numbers, bits reversed, are neighbours lie next to each other: with c = (row in the block, bits reversed) 2^L + c_low, c_low the
 // block's number reversed, an even row is at 2 c and an odd one at 2 n - 1 - 2 c. A CTA takes the blocks c0 ... c0 + 7 (A) and their complements (B),
 // a warp each; for an even row r and either of the two segments below, sixteen consecutive words hold eight blocks' values at row r and eight
@@ -553,7 +553,11 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     };
     // a group is an aligned block of coset order: lead is the rest of a power of two, so it is a multiple of chunks too
     const uint32_t chunk_log = 31u - (uint32_t)__builtin_clz(grid->chunks);
-    const bool blocks = grid->chunks == 1u << chunk_log && chunk_log >= 5 && chunk_log <= 8 && grid->log_rows >= chunk_log + 4 && aligned(out_cols, (1 + 2 * (size_t)n_mats) * 4);
+    // Scan and split in one takes 2^19 rows and more, 256 to a group, at most a quarter of them lead rows, which it goes through too. Two passes -> one, the
+    // whole call and the scatter before it at 2^20 rows without lead, two matrices of 16 columns: 208 -> 191 us. The call alone with a quarter of
+    // lead rows: 2^20 144.8 -> 143.1, 2^19 100.7 -> 98.7. What is smaller or has shorter groups stays with two passes, which have a warp a group
+    // and no barriers: 2^18 rows 77 -> 88, 2^20 rows with 128, 64 and 32 to a group 172 -> 178, 224 -> 241 and 336 -> 394.
+    const bool blocks = grid->chunks == 256 && grid->log_rows >= 19 && grid->lead <= rows / 4 && aligned(out_cols, (1 + 2 * (size_t)n_mats) * 4);
     if (blocks) ZKB_CUDA(ctx, cudaFuncSetAttribute(freivalds_scan_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_OUT_SMEM));
     // work buffers from the stream-ordered pool: lanes in coset order, prefix over groups
     uint4 *lanes = nullptr, *prefix = nullptr;
@@ -565,7 +569,10 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
         for (size_t k = 0; k < n; k++) if ((uintptr_t)p[k] & 7) return false;
         return true;
     };
-    if (rows >= 1024 && even(base_cols, pq) && even(pre_cols, (size_t)n_mats * pk)) {
+    // Four rows a thread from 2^19 rows (512 CTAs) and eight columns a matrix on. The whole call, two rows a thread -> four: 2^20 rows, one matrix of 40
+    // columns 132 -> 120 us, three of 8 175 -> 172; 2^19, three of 8 116 -> 112. Two rows a thread keep what is smaller, where the chip isn't full
+    // (2^18, three of 8: 82.7 -> 82.9; 2^16: 69.1 -> 71.3) or a thread has few columns to share its work (2^20, three of 1: 190 -> 196).
+    if (rows >= (1u << 19) && pk >= 8 && even(base_cols, pq) && even(pre_cols, (size_t)n_mats * pk)) {
         qm31 bias = qm31_zero();
         for (uint32_t p = 0; p < pq; p++) bias = qm31_add(bias, qm31_mul_m31(pows[p], 128u));
         ProfScope prof(ctx, "freivalds_inner_quad_kernel");
