@@ -60,7 +60,7 @@ def test_oracle_claims_are_the_freivalds_identity(oracle, tokens, n_in, n_outs, 
 
 # groups of 32 to 256 rows, a power of two (with and without lead rows), and what lies around that; then 2^19 rows, where the inner products go from two
 # rows a thread to four at eight columns a matrix and from one tile of columns to two above 64, and where scan and split go in one with groups
-# of 256 rows and at most a quarter of lead rows (the last two: the quarter, and one group less)
+# of 256 rows (the last two: with a quarter of lead rows, and a group more of them)
 BLOCKS = [(5, 16, [70, 33], 32), (5, 15, [70], 32), (8, 12, [300], 64), (40, 100, [256, 100, 31], 256), (3, 17, [600], 128), (2, 20, [520], 512), (9, 8, [64], 32),
           (9, 60, [64], 33), (9, 2048, [1792, 100], 256), (300, 2047, [2048, 100], 256), (3, 2600, [8500], 128), (3, 1536, [300, 300, 20], 256), (3, 1535, [2048], 256)]
 
@@ -97,4 +97,34 @@ def test_freivalds_device_matches_oracle(ctx, oracle, tokens, n_in, n_outs, chun
     out = [ctx.alloc(rows) for _ in range((1 + 2 * n_mats) * 4)]
     claims = ctx.freivalds_acc([b.ptr for b in base], [p.ptr for p in pre[:n_mats * pk]], grid, pq, pk, n_mats, s, rv, [o.ptr for o in out])
     assert (np.stack([o.download() for o in out]) == want_cols).all()
+    assert (claims == want_claims).all()
+
+
+# 2^19 rows, 256 to a group: the one pass over scan and split with few lead rows, with almost half of them and with columns that it does not take, the
+# four-row inner products with columns on 8 bytes and without; 2^20 rows; shorter groups. shift: words by which the columns miss 16 bytes
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,n_in,n_outs,chunks,shift_in,shift_out", [
+    (9, 1100, [2048, 300], 256, 0, 0), (300, 1025, [2048], 256, 2, 0), (3, 2049, [300], 256, 0, 0), (3, 2047, [2048], 256, 1, 0), (3, 2047, [2048], 256, 0, 1),
+    (3, 1536, [2048, 2000], 256, 1, 1), (3, 1536, [2048], 256, 3, 2), (3, 4095, [1024], 128, 1, 2)])
+def test_freivalds_accumulators_at_2_19_rows(ctx, oracle, tokens, n_in, n_outs, chunks, shift_in, shift_out):
+    qx, qws = _case(13, tokens, n_in, n_outs)
+    grid, pq, pk = layout(n_in, max(n_outs), tokens, chunks)
+    rows, n_mats = 1 << grid[0], len(qws)
+    base, pre, _, _ = oracle.freivalds_columns(qx, qws, grid, pq, pk)
+    s, rv = qm31_array(33, 1)[0], qm31_array(34, 1)[0]
+    want_cols, want_claims = oracle.freivalds_acc(base, pre, n_mats, grid, pq, pk, s, rv)
+
+    def at(shift, words):  # on the device, `shift` words behind a 16-byte boundary, in one buffer
+        buf = ctx.upload(np.concatenate([np.zeros(shift, np.uint32)] + [np.concatenate([w, np.zeros(4, np.uint32)]) for w in words]))
+        return buf, [buf.ptr + 4 * (shift + k * (rows + 4)) for k in range(len(words))]
+
+    keep_b, d_base = at(shift_in, base)
+    keep_p, d_pre = at(shift_in, pre[:n_mats * pk])
+    keep_o, d_out = at(shift_out, np.zeros_like(want_cols))
+    ctx.profile_begin()
+    claims = ctx.freivalds_acc(d_base, d_pre, grid, pq, pk, n_mats, s, rv, d_out)
+    ran = ctx.profile_end()
+    assert ("freivalds_scan_out_kernel" in ran) == (chunks == 256 and shift_out == 0)
+    assert ("freivalds_inner_quad_kernel" in ran) == (pk >= 8 and shift_in % 2 == 0)
+    assert (keep_o.download()[shift_out:].reshape(-1, rows + 4)[:, :rows] == want_cols).all()
     assert (claims == want_claims).all()

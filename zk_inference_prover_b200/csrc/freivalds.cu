@@ -314,46 +314,50 @@ __global__ void __launch_bounds__(256) freivalds_group_scan_kernel(uint4* __rest
     }
 }
 
-// Scan and split in one, where a group is 2^b rows, at most 256 of them (the call takes it for 256): then it is an aligned block of coset order, and in committed order the
-// blocks whose numbers, bits reversed, are neighbours lie next to each other: with c = (row in the block, bits reversed) 2^L + c_low, c_low the
-// block's number reversed, an even row is at 2 c and an odd one at 2 n - 1 - 2 c. A CTA takes the blocks c0 ... c0 + 7 (A) and their complements (B),
-// a warp each; for an even row r and either of the two segments below, sixteen consecutive words hold eight blocks' values at row r and eight
-// of the others' at row 2^b - 1 - r, so a lane's values cross shared memory once and go out in whole 64-byte pieces. 2^20 rows, 256 to a
-// group, v and two u: scan and split one after the other 44 + 32 us, this and the accumulators' columns 51 + 8.
+// Scan and split in one, where a group is 256 rows, what a warp scans at a time: then it is an aligned block of coset order, and in committed
+// order the blocks whose numbers, bits reversed, are neighbours lie next to each other: with c = (row in the block, bits reversed) 2^L + c_low, c_low
+// the block's number reversed, an even row is at 2 c and an odd one at 2 n - 1 - 2 c. A CTA takes the blocks c0 ... c0 + 7 (A) and their complements
+// (B), a warp each; for an even row r and either of the two segments below, sixteen consecutive words hold eight blocks' values at row r and eight
+// of the others' at row 255 - r, so a lane's values cross shared memory once and go out in whole 64-byte pieces. A block of lead rows is zeros and is
+// not scanned. 2^20 rows, v and two u: scan and split one after the other 45 + 35 us, this and the accumulators' columns 47 + 10.
+constexpr uint32_t BLOCK_LOG = 8, BLOCK_ROWS = 1u << BLOCK_LOG;
 constexpr int SCAN_OUT_THREADS = 512, SCAN_OUT_GROUPS = SCAN_OUT_THREADS / 32;
-constexpr uint32_t SCAN_OUT_PITCH = 256 + 32;  // of a group in shared memory: a gap every eight rows, which the lanes write at a time
+constexpr uint32_t SCAN_OUT_PITCH = BLOCK_ROWS + 32;  // of a group in shared memory: a gap every eight rows, which the lanes write at a time
 constexpr size_t SCAN_OUT_SMEM = (size_t)SCAN_OUT_GROUPS * SCAN_OUT_PITCH * 16;
-__global__ void __launch_bounds__(SCAN_OUT_THREADS, 2) freivalds_scan_out_kernel(const uint4* __restrict__ lanes, FGrid g, uint32_t chunk_log, uint32_t n_mats,
+__global__ void __launch_bounds__(SCAN_OUT_THREADS, 2) freivalds_scan_out_kernel(const uint4* __restrict__ lanes, FGrid g, uint32_t n_mats,
                                                                                  const __grid_constant__ ScanSteps st, uint4* __restrict__ prod,
                                                                                  uint32_t* const* __restrict__ out) {
     extern __shared__ uint4 tile[];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, L = g.log_rows - chunk_log, mask = (1u << L) - 1u, c0 = blockIdx.x * 8u;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, L = g.log_rows - BLOCK_LOG, mask = (1u << L) - 1u, c0 = blockIdx.x * 8u;
     const uint32_t c_low = warp < 8 ? c0 + warp : mask - (c0 + warp - 8u), block = __brev(c_low) >> (32 - L);
-    const uint32_t lead_blocks = g.lead >> chunk_log;
+    const uint32_t lead_blocks = g.lead >> BLOCK_LOG;
+    const bool live = block >= lead_blocks;
     uint4* const mine = tile + warp * SCAN_OUT_PITCH;
     auto at = [](uint32_t r) { return r + (r >> 3); };
+    if (!live)
+        for (uint32_t k = lane; k < SCAN_OUT_PITCH; k += 32u) mine[k] = make_uint4(0, 0, 0, 0);
     qm31 v_last = qm31_zero();
     for (uint32_t l = 0; l <= n_mats; l++) {
-        qm31 end = qm31_zero();
-        const uint4* const rows_in = lanes + ((size_t)l << g.log_rows) + ((size_t)block << chunk_log);
-        uint4 in[8];
+        if (live) {
+            qm31 end = qm31_zero();
+            const uint4* const rows_in = lanes + ((size_t)l << g.log_rows) + ((size_t)block << BLOCK_LOG);
+            uint4 in[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (32u * k + lane < g.chunks) in[k] = rows_in[32u * k + lane];
+            for (uint32_t k = 0; k < 8; k++) in[k] = rows_in[32u * k + lane];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; k++)
-            if (32u * k + lane < g.chunks) mine[at(32u * k + lane)] = in[k];
-        __syncwarp();
-        scan_rows<true>(g.chunks, true, st.pw[l ? 1 : 0], st.wide[l ? 1 : 0], end, [&](uint32_t r) { return mine[at(r)]; }, [&](uint32_t r, uint4 x) { mine[at(r)] = x; });
-        if (l == 0) v_last = end;
-        else if (lane == 0 && block >= lead_blocks) prod[(size_t)(l - 1) * g.groups + block - lead_blocks] = u_of(qm31_mul(end, v_last));
+            for (uint32_t k = 0; k < 8; k++) mine[at(32u * k + lane)] = in[k];
+            __syncwarp();
+            scan_rows<true>(BLOCK_ROWS, true, st.pw[l ? 1 : 0], st.wide[l ? 1 : 0], end, [&](uint32_t r) { return mine[at(r)]; }, [&](uint32_t r, uint4 x) { mine[at(r)] = x; });
+            if (l == 0) v_last = end;
+            else if (lane == 0) prod[(size_t)(l - 1) * g.groups + block - lead_blocks] = u_of(qm31_mul(end, v_last));
+        }
         __syncthreads();
         uint32_t* const* const o = out + (l ? 8 * l - 4 : 0);
         uint32_t *const o0 = o[0], *const o1 = o[1], *const o2 = o[2], *const o3 = o[3];
-        for (uint32_t k = threadIdx.x; k < 16u * g.chunks; k += SCAN_OUT_THREADS) {
-            const uint32_t w = k & 15u, t = w >> 1, odd = w & 1u, seg = (k >> 4) & 1u, h = k >> 5, r = __brev(h) >> (32 - chunk_log);
+        for (uint32_t k = threadIdx.x; k < 16u * BLOCK_ROWS; k += SCAN_OUT_THREADS) {
+            const uint32_t w = k & 15u, t = w >> 1, odd = w & 1u, seg = (k >> 4) & 1u, h = k >> 5, r = __brev(h) >> (32 - BLOCK_LOG);
             const uint32_t from = seg == odd ? (seg ? 7u - t : t) : 8u + (seg ? 7u - t : t);  // A in even words of the first segment, odd ones of the second
-            const uint32_t row = odd ? g.chunks - 1u - r : r;
+            const uint32_t row = odd ? BLOCK_ROWS - 1u - r : r;
             const uint4 x = tile[from * SCAN_OUT_PITCH + at(row)];
             const size_t i = 2u * ((h << L) + (seg ? mask - (c0 + 7u) : c0)) + w;
             o0[i] = x.x; o1[i] = x.y; o2[i] = x.z; o3[i] = x.w;
@@ -365,14 +369,15 @@ __global__ void __launch_bounds__(SCAN_OUT_THREADS, 2) freivalds_scan_out_kernel
 // lies in committed order modulo 2^(L + 1) says which block it is of: a thread has the prefixes of four neighbouring places and writes them to
 // every row of its share.
 constexpr uint32_t ACC_RUN = 16;
-__global__ void __launch_bounds__(128) freivalds_acc_columns_kernel(const uint4* __restrict__ prefix, FGrid g, uint32_t chunk_log, uint32_t n_mats, uint32_t* const* __restrict__ out) {
-    const uint32_t L = g.log_rows - chunk_log, low = 4u * (blockIdx.x * blockDim.x + threadIdx.x), lead_blocks = g.lead >> chunk_log;
+static_assert(BLOCK_ROWS / 2 % ACC_RUN == 0, "whole runs");
+__global__ void __launch_bounds__(128) freivalds_acc_columns_kernel(const uint4* __restrict__ prefix, FGrid g, uint32_t n_mats, uint32_t* const* __restrict__ out) {
+    const uint32_t L = g.log_rows - BLOCK_LOG, low = 4u * (blockIdx.x * blockDim.x + threadIdx.x), lead_blocks = g.lead >> BLOCK_LOG;
     if (low >> (L + 1)) return;
-    const uint32_t half = g.chunks >> 1, h0 = blockIdx.y * ACC_RUN, h1 = h0 + ACC_RUN < half ? h0 + ACC_RUN : half;
+    const uint32_t h0 = blockIdx.y * ACC_RUN;
     uint32_t upto[4];  // slots in the sum of a place's rows
 #pragma unroll
     for (uint32_t u = 0; u < 4; u++) {
-        const uint32_t block = coset_perm(low + u, g.log_rows) >> chunk_log;
+        const uint32_t block = coset_perm(low + u, g.log_rows) >> BLOCK_LOG;
         upto[u] = block < lead_blocks ? 0u : block - lead_blocks;
     }
     for (uint32_t m = 0; m < n_mats; m++) {
@@ -388,10 +393,10 @@ __global__ void __launch_bounds__(128) freivalds_acc_columns_kernel(const uint4*
             *reinterpret_cast<uint4*>(o3 + i) = make_uint4(a.w, b.w, c.w, d.w);
         };
         const uint4 a = sum(upto[0]), b = sum(upto[1]), c = sum(upto[2]), d = sum(upto[3]);
-        for (uint32_t h = h0; h < h1; h++)
+        for (uint32_t h = h0; h < h0 + ACC_RUN; h++)
             if (h) write(h, a, b, c, d);
         if (h0 == 0) {
-            const uint32_t b1 = coset_perm(low + 1u, g.log_rows) >> chunk_log, d1 = coset_perm(low + 3u, g.log_rows) >> chunk_log;
+            const uint32_t b1 = coset_perm(low + 1u, g.log_rows) >> BLOCK_LOG, d1 = coset_perm(low + 3u, g.log_rows) >> BLOCK_LOG;
             write(0, a, sum(b1 < lead_blocks ? 0u : upto[1] + 1u), c, sum(d1 < lead_blocks ? 0u : upto[3] + 1u));
         }
     }
@@ -551,13 +556,13 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
         for (size_t k = 0; k < n; k++) if ((uintptr_t)p[k] & 15) return false;
         return true;
     };
-    // a group is an aligned block of coset order: lead is the rest of a power of two, so it is a multiple of chunks too
-    const uint32_t chunk_log = 31u - (uint32_t)__builtin_clz(grid->chunks);
-    // Scan and split in one takes 2^19 rows and more, 256 to a group, at most a quarter of them lead rows, which it goes through too. Two passes -> one, the
-    // whole call and the scatter before it at 2^20 rows without lead, two matrices of 16 columns: 208 -> 191 us. The call alone with a quarter of
-    // lead rows: 2^20 144.8 -> 143.1, 2^19 100.7 -> 98.7. What is smaller or has shorter groups stays with two passes, which have a warp a group
-    // and no barriers: 2^18 rows 77 -> 88, 2^20 rows with 128, 64 and 32 to a group 172 -> 178, 224 -> 241 and 336 -> 394.
-    const bool blocks = grid->chunks == 256 && grid->log_rows >= 19 && grid->lead <= rows / 4 && aligned(out_cols, (1 + 2 * (size_t)n_mats) * 4);
+    // Scan and split in one takes groups of 256 rows, what a warp scans at a time, from 2^19 rows on (two CTAs on nearly every SM): a group is an aligned
+    // block of coset order, since lead, the rest of a power of two, is a multiple of 256 too. Two passes -> one, this call alone, two matrices of 16
+    // columns: 2^19 rows without lead 100.7 -> 93.1 us, with half of it lead 93.4 -> 89.6; 2^20 157.6 -> 138.8 and 133.5 -> 124.2; 2^22 506 -> 413 and
+    // 427 -> 350. One matrix of two columns gains 4 to 20 %, three of 16 5 to 21 %. Below, a CTA's barriers have no other CTA's work to hide behind
+    // and two passes, a warp a group without any, are ahead: 2^18 77.0 -> 83.6, 2^16 68.3 -> 79.0. So they are with shorter groups, where a CTA has as many
+    // barriers for fewer rows (with the block's size a parameter, 2^20 rows of 128, 64 and 32 to a group: 172 -> 178, 224 -> 241, 336 -> 394).
+    const bool blocks = grid->chunks == BLOCK_ROWS && grid->log_rows >= 19 && aligned(out_cols, (1 + 2 * (size_t)n_mats) * 4);
     if (blocks) ZKB_CUDA(ctx, cudaFuncSetAttribute(freivalds_scan_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_OUT_SMEM));
     // work buffers from the stream-ordered pool: lanes in coset order, prefix over groups
     uint4 *lanes = nullptr, *prefix = nullptr;
@@ -592,8 +597,7 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     }
     if (blocks) {
         ProfScope prof(ctx, "freivalds_scan_out_kernel");
-        freivalds_scan_out_kernel<<<1u << (grid->log_rows - chunk_log - 4), SCAN_OUT_THREADS, SCAN_OUT_SMEM, ctx->stream>>>(lanes, fg, chunk_log, n_mats, scan_steps, prefix,
-                                                                                                                     (uint32_t* const*)d_out);
+        freivalds_scan_out_kernel<<<1u << (grid->log_rows - BLOCK_LOG - 4), SCAN_OUT_THREADS, SCAN_OUT_SMEM, ctx->stream>>>(lanes, fg, n_mats, scan_steps, prefix, (uint32_t* const*)d_out);
     } else {
         ProfScope prof(ctx, "freivalds_group_scan_kernel");
         freivalds_group_scan_kernel<<<(unsigned)(((size_t)grid->groups * 32 + 255) / 256), 256, 0, ctx->stream>>>(lanes, fg, n_mats, scan_steps, prefix);
@@ -604,8 +608,8 @@ int zkb_freivalds_acc(zkb_ctx* ctx, const uint32_t* const* base_cols, const uint
     }
     if (blocks) {
         ProfScope prof(ctx, "freivalds_acc_columns_kernel");
-        const dim3 ctas((unsigned)(((2u << (grid->log_rows - chunk_log)) / 4 + 127) / 128), (grid->chunks / 2 + ACC_RUN - 1) / ACC_RUN);
-        freivalds_acc_columns_kernel<<<ctas, 128, 0, ctx->stream>>>(prefix, fg, chunk_log, n_mats, (uint32_t* const*)d_out);
+        const dim3 ctas(((2u << (grid->log_rows - BLOCK_LOG)) / 4 + 127) / 128, BLOCK_ROWS / 2 / ACC_RUN);
+        freivalds_acc_columns_kernel<<<ctas, 128, 0, ctx->stream>>>(prefix, fg, n_mats, (uint32_t* const*)d_out);
     } else {
         ProfScope prof(ctx, "freivalds_split_kernel");
         freivalds_split_kernel<<<row_pair_blocks(rows), 256, 0, ctx->stream>>>(lanes, prefix, fg, n_mats, (uint32_t* const*)d_out);
