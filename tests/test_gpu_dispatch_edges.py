@@ -173,7 +173,7 @@ def test_quotients_combined_several_rows_a_thread(ctx, oracle, n_acc, log_n):
 
 @pytest.mark.parametrize("log_n,n_cols", [(14, 2), (15, 1), (15, 300), (16, 150), (17, 5), (17, 300), (18, 299)])
 def test_eval_at_point_in_runs_of_chunks(ctx, oracle, log_n, n_cols):
-    # from 2^15 coefficients on: runs of sixteen chunks, of 32 and 64 where there are two for every SM
+    # one run of sixteen chunks a column, runs of sixteen, and of 32 and 64 where there are two for every SM
     cols = [m31_column(8400 + 7 * log_n + c, 1 << log_n) for c in range(n_cols)]
     bufs, point = [ctx.upload(c) for c in cols], qm31_array(8390, 2).ravel()
     got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
@@ -204,3 +204,15 @@ def test_merkle_layers_of_many_columns(ctx, oracle, log_size, ncols, with_prev):
     for m31 in (False, True):
         ctx.merkle_layer(log_size, pb.ptr if pb else 0, [b.ptr for b in bufs], out.ptr, m31_out=m31)
         assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, prev, cols, m31=m31)).all()
+
+
+
+@pytest.mark.parametrize("log_n,n_cols,runs", [(15, 1, True), (16, 39, False), (16, 40, True), (18, 9, False), (18, 10, True), (20, 2, False), (20, 3, True)])
+def test_eval_at_point_where_runs_begin(ctx, oracle, log_n, n_cols, runs):
+    # one run a column, or eighty runs of sixteen chunks
+    cols = [m31_column(8450 + c, 1 << log_n) for c in range(n_cols)]
+    bufs, point = [ctx.upload(c) for c in cols], qm31_array(8395, 2).ravel()
+    ctx.profile_begin()
+    got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
+    assert ("eval_runs_kernel" in ctx.profile_end()) == runs
+    assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()

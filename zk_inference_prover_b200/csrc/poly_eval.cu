@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) eval_dot_kernel(const uint32_t* const* __
 // eval_dot_kernel is bound by what a chunk costs beside its products, the reduction of four words over the CTA; here a thread keeps the inner sums of
 // its eight elements through a run (64-bit sums folded every four chunks) and the weights and the reduction come once a run. 256 columns of
 // 2^20: 396 us with a reduction a chunk, 210 with one in 64.
-constexpr int RUN_MIN_LOG = 4, RUN_MAX_LOG = 6, RUN_CTAS = 2;
+constexpr int RUN_MIN_LOG = 4, RUN_MAX_LOG = 6, RUN_CTAS = 2, RUN_MIN_RUNS = 80;
 __global__ void __launch_bounds__(256, RUN_CTAS) eval_runs_kernel(const uint32_t* const* __restrict__ cols, int ncols, int log_n, int run_log,
                                                                   const uint32_t* __restrict__ weights, uint32_t* __restrict__ out) {
     __shared__ uint4 of_chunk[1 << RUN_MAX_LOG];
@@ -282,10 +282,14 @@ int eval_at_point_device(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols,
     // Scratch: [weights: 2048 and 64 QM31] [ping] [pong]; columns go in batches whose partials fit.
     bool use_dot = true;
     for (int c = 0; c < ncols; c++) use_dot = use_dot && ((uintptr_t)coeffs[c] & 15) == 0;  // 16-byte loads
-    // Runs of sixteen chunks and more, as long as there are two for every SM (shorter ones cost more in products with the weights than they save).
+    // Runs of sixteen chunks, longer as long as there are two for every SM (shorter ones cost more in products with the weights than they save). Fewer
+    // than 80 of sixteen are a handful of CTAs that walk them one chunk after the other; four chunks a CTA are faster there, unless a column is one run
+    // and the launch that folds the runs falls away. The whole call, four chunks -> runs, columns not in L2: 8 of 2^18 (64 runs) 39.1 -> 40.3 us, 10
+    // (80) 42.0 -> 41.0, 16 (128) 45.6 -> 41.4; 33 of 2^16 (66) 42.6 -> 43.4, 40 (80) 44.5 -> 44.1, 64 (128) 51 -> 47; 1 of 2^20 (32) 38.2 -> 39.0, 4 (128)
+    // 49.5 -> 40.2. One run a column, 4 of 2^15: 38.6 -> 36.7, 64: 45.7 -> 43.3.
     int run_log = log_n - EVAL_CHUNK_LOG < RUN_MAX_LOG ? log_n - EVAL_CHUNK_LOG : RUN_MAX_LOG;
     while (run_log > RUN_MIN_LOG && ((size_t)ncols << (log_n - EVAL_CHUNK_LOG - run_log)) < RUN_CTAS * 148u) run_log--;
-    if (!use_dot || run_log < RUN_MIN_LOG) run_log = 0;
+    if (!use_dot || run_log < RUN_MIN_LOG || (log_n > EVAL_CHUNK_LOG + RUN_MIN_LOG && ((size_t)ncols << (log_n - EVAL_CHUNK_LOG - RUN_MIN_LOG)) < RUN_MIN_RUNS)) run_log = 0;
     const int chunk_log = EVAL_CHUNK_LOG + run_log;
     size_t partials_per_col = (size_t)1 << (log_n - chunk_log);
     uint32_t* weights = ctx->scratch;
