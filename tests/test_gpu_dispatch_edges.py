@@ -197,7 +197,7 @@ def test_transforms_of_short_columns(ctx, oracle, log_n, n_cols, blowup):
 @pytest.mark.parametrize("with_prev", [False, True])
 @pytest.mark.parametrize("log_size,ncols", [(0, 64), (3, 63), (3, 65), (4, 80), (5, 81), (6, 95), (7, 96), (13, 64), (13, 97), (14, 64), (2, 1000)])
 def test_merkle_layers_of_many_columns(ctx, oracle, log_size, ncols, with_prev):
-    # from 64 columns on, up to 2^13 nodes, a warp brings the blocks of sixteen nodes: even and odd numbers of blocks, whole and partial last ones
+    # many columns: a warp brings the blocks of sixteen nodes; even and odd numbers of blocks, whole and partial last ones
     cols = [m31_column(8700 + c, 1 << log_size) for c in range(ncols)]
     prev = m31_column(8690, 16 << log_size).reshape(-1, 8) if with_prev else None
     bufs, pb, out = [ctx.upload(c) for c in cols], ctx.upload(prev) if with_prev else None, ctx.alloc(8 << log_size)
@@ -216,3 +216,15 @@ def test_eval_at_point_where_runs_begin(ctx, oracle, log_n, n_cols, runs):
     got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
     assert ("eval_runs_kernel" in ctx.profile_end()) == runs
     assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()
+
+
+
+@pytest.mark.parametrize("log_size,ncols,chain", [(0, 95, False), (0, 96, True), (8, 95, False), (11, 95, False), (11, 96, True), (11, 129, True), (12, 1535, False),
+                                                  (12, 1536, True), (13, 143, False), (13, 144, True)])
+def test_merkle_layers_where_the_loader_warp_begins(ctx, oracle, log_size, ncols, chain):
+    cols = [m31_column(9000 + c, 1 << log_size) for c in range(ncols)]
+    bufs, out = [ctx.upload(c) for c in cols], ctx.alloc(8 << log_size)
+    ctx.profile_begin()
+    ctx.merkle_layer(log_size, 0, [b.ptr for b in bufs], out.ptr, m31_out=True)
+    assert ("merkle_layer_chain_kernel" in ctx.profile_end()) == chain
+    assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, None, cols, m31=True)).all()

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256) merkle_layer_kernel(int log_size, const u
     store_hash(out, i, h, m31_out != 0);
 }
 
-// The same node hash for layers of at most 2^13 nodes and fewer than 64 columns, four lanes to a node (b2s_compress_quad in channel.cuh). Such a layer is
+// The same node hash for layers of at most 2^13 nodes and few columns (chain_min_cols), four lanes to a node (b2s_compress_quad in channel.cuh). Such a layer is
 // bound by the latency of its compressions, and by fetching their code where it is one of a few: a quad issues a quarter of
 // a thread's instructions from a quarter of the code. A lane brings four of a block's sixteen words; a block's words
 // and the addresses of the next one's are on their way while the block before is hashed. A tree of 2^16 leaves built layer by
@@ -128,7 +128,13 @@ __global__ void __launch_bounds__(QUAD_THREADS) merkle_layer_quad_kernel(int log
 // their blocks, so that a hash meets no load from memory and none of the instructions around one (some 250 of 1,500 cycles a
 // block). While block k is hashed the loader puts block k + 1 into the other buffer, its words asked for two blocks before and
 // their columns' addresses three; one CTA barrier a block.
-constexpr int CHAIN_NODES = 16, CHAIN_THREADS = 4 * CHAIN_NODES + 32, CHAIN_MIN_COLS = 64;
+constexpr int CHAIN_NODES = 16, CHAIN_THREADS = 4 * CHAIN_NODES + 32;
+// From how many columns on. The third warp costs a start of its own and a barrier a block, which some six blocks make up for; where a CTA shares its SM
+// with another, from 2^12 nodes on, it shares schedulers too and takes longer to. Quads -> chain, a layer alone, columns not in L2: 2^8 nodes of 64
+// columns 10.3 -> 10.7 us, 80 10.5 -> 10.7, 96 11.2 -> 10.7, 256 18.8 -> 17.6, 4,096 203 -> 176; 2^11 of 80 10.6 -> 10.8, 96 11.4 -> 11.0, 1,024 55.7 -> 53.4;
+// 2^12 of 256 19.1 -> 21.0, 512 32.4 -> 33.2, 1,024 57.3 -> 57.4, 2,048 106.3 -> 105.2, 16,000 777 -> 764; 2^13 of 128 14.8 -> 16.0, 144 18.4 -> 16.5, 300 25.6 ->
+// 25.1, 4,096 244 -> 224.
+static int chain_min_cols(int log_size) { return log_size <= 11 ? 96 : log_size == 12 ? 1536 : 144; }
 __global__ void __launch_bounds__(CHAIN_THREADS) merkle_layer_chain_kernel(int log_size, const uint32_t* prev, const uint32_t* const* __restrict__ cols, int ncols,
                                                                            int m31_out, uint32_t* out) {
     __shared__ uint32_t sched[40];
@@ -496,7 +502,7 @@ int zkb_merkle_layer(zkb_ctx* ctx, int log_size, const uint32_t* prev, const uin
         if (rc) return rc;
     }
     const size_t n = (size_t)1 << log_size;
-    if (log_size <= QUAD_MAX_LOG && ncols >= CHAIN_MIN_COLS) {
+    if (log_size <= QUAD_MAX_LOG && ncols >= chain_min_cols(log_size)) {
         ProfScope prof(ctx, "merkle_layer_chain_kernel");
         ZKB_CUDA(ctx, launch_following(ctx, merkle_layer_chain_kernel, (unsigned)((n + CHAIN_NODES - 1) / CHAIN_NODES), CHAIN_THREADS, log_size, prev,
                                        (const uint32_t* const*)d_cols, ncols, m31_out, out));
