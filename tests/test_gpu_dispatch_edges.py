@@ -148,8 +148,7 @@ def test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, lo
 
 @pytest.mark.parametrize("log_n,n_cols", [(1, 40), (2, 31), (2, 32), (5, 600), (9, 33), (10, 1500), (13, 100), (19, 34)])
 def test_numerators_split_over_columns(ctx, oracle, log_n, n_cols):
-    # from 32 entries on and as long as the rows alone do not fill the GPU, in pieces of sixteen columns and more; 24 pieces are added up by
-    # eight warps
+    # as long as the rows alone do not fill the GPU, in pieces of sixteen columns and more; 24 pieces are added up by eight warps
     cols = [m31_column(8000 + c, 1 << log_n) for c in range(n_cols)]
     point, values, rands = oracle.secure_circle_mul(24680), qm31_array(8101, n_cols), qm31_array(8102, n_cols)
     want, _ = oracle.quot_numerators(cols, point, np.arange(n_cols, dtype=np.uint32), values, rands)
@@ -228,3 +227,10 @@ def test_merkle_layers_where_the_loader_warp_begins(ctx, oracle, log_size, ncols
     ctx.merkle_layer(log_size, 0, [b.ptr for b in bufs], out.ptr, m31_out=True)
     assert ("merkle_layer_chain_kernel" in ctx.profile_end()) == chain
     assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, None, cols, m31=True)).all()
+
+
+
+@pytest.mark.parametrize("log_n,n_cols", [(1, 48), (2, 47), (2, 48), (13, 47), (13, 48), (17, 47), (17, 49), (18, 111), (18, 112)])
+def test_numerators_where_the_split_begins(ctx, oracle, log_n, n_cols):
+    # 48 entries; 112 where the rows leave room for two pieces
+    test_numerators_split_over_columns(ctx, oracle, log_n, n_cols)

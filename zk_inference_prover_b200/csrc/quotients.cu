@@ -317,13 +317,16 @@ static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncol
     // Few rows: the columns are split over the grid's second dimension, so that some 148 x 4 CTAs' worth of threads have loads on their way, sixteen
     // columns each at least. A thread walks its columns four at a time, a trip to memory each: a hundred columns of 2^13 rows on
     // eight CTAs were 35 us, of 2^17 rows 41; split, and added up, 10 + 4 and 18 + 8. Groups of fewer than 1,024 rows take narrower CTAs.
+    // The pieces' sums are a launch more and as many bytes as eight columns a piece: whole -> split, 40 columns of 2^6 rows 12.7 -> 13.4 us, 2^13
+    // 18.5 -> 16.0, 2^17 20.0 -> 21.6; 48 columns 13.9 -> 13.8, 21.5 -> 16.0 and 22.7 -> 21.8. Where the rows leave room for two pieces only (2^18): 80 columns
+    // 35.1 -> 36.5, 100 41.4 -> 41.3, 112 45.6 -> 44.0, 200 75.4 -> 62.7.
     const size_t per = wide ? 4 : 2;
     const unsigned threads = n / per >= 256 ? 256u : n / per >= 32 ? (unsigned)(n / per) : 32u;
     const unsigned row_blocks = (unsigned)((n / per + threads - 1) / threads);
     const size_t scratch_free = ctx->scratch_words - scratch_used;
     int S = std::min((k + 15) / 16, (int)(148u * 1024u / (row_blocks * threads)));
     S = std::min<size_t>(S, (scratch_free - 4) / (4 * n));
-    if (S >= 2 && k >= 32) {
+    if (S >= 2 && k >= (S == 2 ? 112 : 48)) {
         const int chunk = ((k + S - 1) / S + 3) / 4 * 4;
         S = (k + chunk - 1) / chunk;
         uint32_t* partial = ctx->scratch + scratch_used + ((4 - (scratch_used & 3)) & 3);  // 16-byte aligned
