@@ -230,7 +230,7 @@ def test_merkle_layers_where_the_loader_warp_begins(ctx, oracle, log_size, ncols
 
 
 
-@pytest.mark.parametrize("log_n,n_cols", [(1, 48), (2, 47), (2, 48), (13, 47), (13, 48), (17, 47), (17, 49), (18, 111), (18, 112)])
+@pytest.mark.parametrize("log_n,n_cols", [(1, 40), (2, 39), (2, 41), (13, 39), (13, 40), (16, 40), (17, 47), (17, 49), (18, 111), (18, 112)])
 def test_numerators_where_the_split_begins(ctx, oracle, log_n, n_cols):
-    # 48 entries; 112 where the rows leave room for two pieces
+    # 40 entries; 48 and 112 where the rows leave room for four pieces and for two
     test_numerators_split_over_columns(ctx, oracle, log_n, n_cols)

@@ -317,16 +317,17 @@ static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncol
     // Few rows: the columns are split over the grid's second dimension, so that some 148 x 4 CTAs' worth of threads have loads on their way, sixteen
     // columns each at least. A thread walks its columns four at a time, a trip to memory each: a hundred columns of 2^13 rows on
     // eight CTAs were 35 us, of 2^17 rows 41; split, and added up, 10 + 4 and 18 + 8. Groups of fewer than 1,024 rows take narrower CTAs.
-    // The pieces' sums are a launch more and as many bytes as eight columns a piece: whole -> split, 40 columns of 2^6 rows 12.7 -> 13.4 us, 2^13
-    // 18.5 -> 16.0, 2^17 20.0 -> 21.6; 48 columns 13.9 -> 13.8, 21.5 -> 16.0 and 22.7 -> 21.8. Where the rows leave room for two pieces only (2^18): 80 columns
-    // 35.1 -> 36.5, 100 41.4 -> 41.3, 112 45.6 -> 44.0, 200 75.4 -> 62.7.
+    // The pieces' sums are a launch more and as many bytes as eight columns a piece: whole -> split, 32 columns of 2^9 rows 13.2 -> 14.1 us, 2^13
+    // 10.8 -> 13.2, 40 columns 13.5 -> 13.6 and 18.5 -> 16.0. Where the rows leave room for four pieces (2^17): 40 columns 20.0 -> 21.6, 48 22.7 -> 21.8; for two
+    // (2^18): 80 35.1 -> 36.5, 100 41.4 -> 41.3, 112 45.6 -> 44.0, 200 75.4 -> 62.7.
     const size_t per = wide ? 4 : 2;
     const unsigned threads = n / per >= 256 ? 256u : n / per >= 32 ? (unsigned)(n / per) : 32u;
     const unsigned row_blocks = (unsigned)((n / per + threads - 1) / threads);
     const size_t scratch_free = ctx->scratch_words - scratch_used;
-    int S = std::min((k + 15) / 16, (int)(148u * 1024u / (row_blocks * threads)));
+    const int room = (int)(148u * 1024u / (row_blocks * threads));
+    int S = std::min((k + 15) / 16, room);
     S = std::min<size_t>(S, (scratch_free - 4) / (4 * n));
-    if (S >= 2 && k >= (S == 2 ? 112 : 48)) {
+    if (S >= 2 && k >= (room == 2 ? 112 : room <= 4 ? 48 : 40)) {
         const int chunk = ((k + S - 1) / S + 3) / 4 * 4;
         S = (k + chunk - 1) / chunk;
         uint32_t* partial = ctx->scratch + scratch_used + ((4 - (scratch_used & 3)) & 3);  // 16-byte aligned
