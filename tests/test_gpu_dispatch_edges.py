@@ -234,3 +234,23 @@ def test_merkle_layers_where_the_loader_warp_begins(ctx, oracle, log_size, ncols
 def test_numerators_where_the_split_begins(ctx, oracle, log_n, n_cols):
     # 40 entries; 48 and 112 where the rows leave room for four pieces and for two
     test_numerators_split_over_columns(ctx, oracle, log_n, n_cols)
+
+
+
+@pytest.mark.parametrize("n_acc", [1, 2, 3, 4, 5, 9])
+@pytest.mark.parametrize("log_n,row_begin,n_rows", [(16, 0, 1 << 16), (17, 0, 1 << 17), (18, 1 << 16, (1 << 17) + 2), (18, 1 << 16, (1 << 17) + 4), (18, 8, (1 << 17) - 2), (4, 8, 2)])
+def test_quotients_of_many_rows_combined(ctx, oracle, n_acc, log_n, row_begin, n_rows):
+    # from 2^17 rows on several a thread, a shard's rows too unless they are not a multiple of four
+    import ctypes as C
+
+    accs = [([m31_column(9100 + 10 * a + q, 1 << (log_n - a % 3)) for q in range(4)], log_n - a % 3) for a in range(n_acc)]
+    first, points = qm31_array(9200, n_acc), np.stack([oracle.secure_circle_mul(24680 + 977 * a) for a in range(n_acc)])
+    want = oracle.quot_combine([np.stack(c) for c, _ in accs], first, points, log_n)[:, row_begin:row_begin + n_rows]
+    keep = [ctx.upload(x[row_begin >> (log_n - lg):]) for c, lg in accs for x in c]  # a shard holds its own rows
+    outs = [ctx.alloc(n_rows) for _ in range(4)]
+    ptrs = lambda bufs: (C.c_void_p * len(bufs))(*[b.ptr for b in bufs])
+    logs = np.array([lg for _, lg in accs], np.int32)
+    at = lambda a: np.ascontiguousarray(a).ctypes.data_as(C.c_void_p)
+    first, points = np.ascontiguousarray(first, np.uint32), np.ascontiguousarray(points, np.uint32)
+    ctx._check(ctx.lib.zkb_quot_combine_rows(ctx.h, C.c_int(n_acc), ptrs(keep), at(logs), at(first), at(points), C.c_int(log_n), C.c_size_t(row_begin), C.c_size_t(n_rows), ptrs(outs)))
+    assert (np.stack([o.download() for o in outs]) == want).all()

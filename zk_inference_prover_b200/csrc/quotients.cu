@@ -588,9 +588,11 @@ int zkb_quot_combine_rows(zkb_ctx* ctx, int n_acc, const uint32_t* const* acc_co
             quot_combine_small_kernel<<<1, 32, 0, ctx->stream>>>(args, lifting_log, o, p0.x, p0.y, p1.x, p1.y);
         } else {
             ProfScope prof(ctx, "quot_combine_kernel");
-            // the rows are a multiple of four but in a shard of two
             auto launch = [&](auto kernel, int rows) { kernel<<<(unsigned)((n / rows + 255) / 256), 256, 0, ctx->stream>>>(args, lifting_log, o, ctx->tw, row_begin, n_rows); };
-            if (n % 4 || args.n_acc > 4) launch(quot_combine_kernel<MAX_ACCS, 1>, 1);
+            // Several rows a thread from 2^17 rows on: below, where a row a thread does not fill the GPU, they only make the chain longer. One accumulation
+            // over 2^16 rows: 8.2 us a row a thread, 8.8 four; two 8.8 and 10.6, four 10.7 and 10.8 (over 2^10 7.1 and 8.8, 7.8 and 10.5, 8.7 and 10.8); over 2^17
+            // 10.4 and 8.8, 10.7 and 10.6, 14.6 and 12.7.
+            if (n < ((size_t)1 << 17) || n % 4 || args.n_acc > 4) launch(quot_combine_kernel<MAX_ACCS, 1>, 1);
             else if (args.n_acc == 1) launch(quot_combine_kernel<1, 4>, 4);
             else if (args.n_acc == 2) launch(quot_combine_kernel<2, 4>, 4);
             else launch(quot_combine_kernel<4, 2>, 2);
