@@ -137,7 +137,7 @@ def test_merkle_levels_around_the_split_launches(ctx, oracle, child_log, levels)
 
 @pytest.mark.parametrize("n_cols,log_n,blowup,shift,two", [(63, 19, 1, 0, 0), (64, 19, 1, 0, 0), (64, 18, 2, 0, 5), (64, 19, 1, 1, 0), (2100, 13, 2, 0, 0), (100, 19, 1, 2, 3)])
 def test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, log_n, blowup, shift, two):
-    # 64 entries and 2^25 words saved: the numerators come from the coefficients, unless these do not start on 16 bytes
+    # wide and tall groups' numerators come from the coefficients, unless these do not start on 16 bytes
     trees = [[m31_column(7900 + c, 1 << log_n) for c in range(n_cols)]]
     kw = dict(pow_bits=0, log_blowup=blowup, log_last_layer=0, n_queries=3, two_sample_every=two)
     want = oracle.pcs_prove(trees, **kw)
@@ -254,3 +254,10 @@ def test_quotients_of_many_rows_combined(ctx, oracle, n_acc, log_n, row_begin, n
     first, points = np.ascontiguousarray(first, np.uint32), np.ascontiguousarray(points, np.uint32)
     ctx._check(ctx.lib.zkb_quot_combine_rows(ctx.h, C.c_int(n_acc), ptrs(keep), at(logs), at(first), at(points), C.c_int(log_n), C.c_size_t(row_begin), C.c_size_t(n_rows), ptrs(outs)))
     assert (np.stack([o.download() for o in outs]) == want).all()
+
+
+
+@pytest.mark.parametrize("n_cols,log_n,blowup,shift,two", [(247, 17, 1, 0, 0), (248, 17, 1, 0, 0), (248, 17, 1, 1, 0), (248, 17, 1, 2, 3), (104, 18, 2, 0, 5)])
+def test_pcs_proof_where_the_numerators_of_coefficients_begin(ctx, oracle, n_cols, log_n, blowup, shift, two):
+    # 24 M words and 28 columns of evaluations saved: 248 columns of 2^17 at blow-up 2
+    test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, log_n, blowup, shift, two)

@@ -468,10 +468,13 @@ int numerator_lines(zkb_ctx* ctx, const NumeratorEntries& e, std::vector<Numerat
 // The combination of the columns' polynomials is itself a polynomial of their degree, so it can be taken of the coefficients, a
 // blow-up fewer of them, and extended: four columns' worth of transform in the place of most of the reading. (The constant comes off
 // coefficient 0, whose basis element is 1.) 256 columns of 2^20 at blow-up 4: 810 us from the evaluations, 206 + 86 from the coefficients.
-// The transform costs as much as reading 27 columns' evaluations at that height and its launches some 10 us, which is 50 MB, so
-// narrow or short groups are read as they are; so are coefficients that do not start on 16 bytes.
+// The transform of four columns costs some 17 us and as much as reading 21 columns' evaluations; the line lies a quarter above that, at 24 M words and 28
+// columns saved, where nothing measured is slower. Numerators and transforms of a proof from the evaluations -> from the coefficients, blow-up 2: 64 columns of
+// 2^19 498 -> 505 us, of 2^20 945 -> 943, 150 of 2^18 560 -> 565 (all left as they were), 256 of 2^17 483 -> 475, 4,500 of 2^13 476 -> 467; blow-up 4: 64 of 2^18
+// 417 -> 422 and 100 of 2^17 326 -> 327 (left), 256 of 2^16 406 -> 383, 200 of 2^17 611 -> 581; blow-up 16: 100 of 2^20 2,380 -> 2,231. Coefficients that do not
+// start on 16 bytes are left too.
 static bool numerators_of_coeffs(const uint32_t* const* coeffs, int ncols, int log_n, int log_coeff, size_t k) {
-    if (k < 64 || (k << log_n) - (k << log_coeff) < ((size_t)1 << 25)) return false;
+    if ((k << log_n) - (k << log_coeff) < ((size_t)24 << 20) + ((size_t)28 << log_n)) return false;
     for (int c = 0; c < ncols; c++) if (((uintptr_t)coeffs[c] & 15) != 0) return false;
     return true;
 }
