@@ -248,8 +248,11 @@ static int launch_step(zkb_ctx* ctx, uint32_t* const* d_dst, const uint32_t* con
         if (grid >= n_a) grid -= grid % n_a;
     }
     const uint32_t* tower = INVERSE ? ctx->itw2 : ctx->tw2;
-    ProfScope prof(ctx, which == 2 ? (INVERSE ? "fft_r32_wide_kernel<inverse>" : "fft_r32_wide_kernel<forward>")
-                                   : (INVERSE ? "fft_r32_contig_kernel<inverse>" : "fft_r32_contig_kernel<forward>"));
+    static const char* const names[4][2] = {{"fft_r32_contig_kernel<forward>", "fft_r32_contig_kernel<inverse>"},
+                                            {"fft_r32_contig12_kernel<forward>", "fft_r32_contig12_kernel<inverse>"},
+                                            {"fft_r32_wide_kernel<forward>", "fft_r32_wide_kernel<inverse>"},
+                                            {"fft_r32_short_kernel<forward>", "fft_r32_short_kernel<inverse>"}};
+    ProfScope prof(ctx, names[which][INVERSE]);
     if (which == 3)
         fft_r32_short_kernel<INVERSE><<<grid, threads, smem, ctx->stream>>>(d_dst, d_src, src_mask, ncols, dom_log, st.r32.act_hi, tower, scale);
     else if (which == 0)
