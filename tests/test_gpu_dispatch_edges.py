@@ -182,7 +182,7 @@ def test_eval_at_point_in_runs_of_chunks(ctx, oracle, log_n, n_cols):
 @pytest.mark.parametrize("log_n,n_cols", [(4, 3), (5, 1), (5, 33), (6, 17), (7, 9), (8, 5), (8, 700), (9, 2), (9, 301)])
 @pytest.mark.parametrize("blowup", [1, 2, 4])
 def test_transforms_of_short_columns(ctx, oracle, log_n, n_cols, blowup):
-    # 2^5 to 2^9 words: several columns to a warp, the last warp's not all there; extensions into that range and out of it
+    # 2^5 to 2^9 words: a CTA a column and, of many columns, several to a warp, the last warp's not all there; extensions into that range and out of it
     vals = np.stack([m31_column(8600 + c, 1 << log_n) for c in range(n_cols)])
     cols = [ctx.upload(v) for v in vals]
     ctx.ifft_cols([c.ptr for c in cols], log_n)
@@ -261,3 +261,19 @@ def test_quotients_of_many_rows_combined(ctx, oracle, n_acc, log_n, row_begin, n
 def test_pcs_proof_where_the_numerators_of_coefficients_begin(ctx, oracle, n_cols, log_n, blowup, shift, two):
     # 24 M words and 28 columns of evaluations saved: 248 columns of 2^17 at blow-up 2
     test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, log_n, blowup, shift, two)
+
+
+
+@pytest.mark.parametrize("log_n,n_cols,short", [(5, 2047, False), (5, 2048, True), (6, 2051, True), (7, 2049, True), (8, 1023, False), (8, 1024, True), (9, 511, False), (9, 513, True)])
+def test_transforms_where_short_columns_share_a_warp(ctx, oracle, log_n, n_cols, short):
+    vals = np.stack([m31_column(9300 + c, 1 << log_n) for c in range(n_cols)])
+    flat = ctx.upload(vals)
+    ptrs = [flat.ptr + 4 * (c << log_n) for c in range(n_cols)]
+    ctx.profile_begin()
+    ctx.ifft_cols(ptrs, log_n)
+    assert any("short" in name for name in ctx.profile_end()) == short
+    coeffs = oracle.interpolate_cols(vals, log_n)
+    assert (flat.download(shape=vals.shape) == coeffs).all()
+    outs = ctx.alloc(n_cols << (log_n + 1))
+    ctx.lde_cols(ptrs, log_n, [outs.ptr + 4 * (c << (log_n + 1)) for c in range(n_cols)], log_n + 1)
+    assert (outs.download(shape=(n_cols, -1)) == oracle.evaluate_cols(coeffs, log_n, log_n + 1)).all()

@@ -140,10 +140,14 @@ struct FftStep {
 // From 2^12 words up (16-byte aligned columns): the twelve-layer contiguous pass, then wide strided passes
 // of up to eight layers (their window slides down over layers already done when the array is short; those
 // layers are switched off). 2^10 and 2^11 words: the ten-layer contiguous pass and a generic pass for the
-// rest. 2^5 to 2^9 words: one launch that takes several columns a warp. Everything else goes through the generic pass.
-static std::vector<FftStep> plan_steps(int nl, int log_n, bool aligned) {
+// rest. 2^5 to 2^9 words, many columns: one launch that takes several columns a warp. Everything else goes through the generic pass.
+//
+// Several columns a warp take 2,048 columns and more or 2^18 words and more: fewer leave the GPU idle either way, and a CTA a column starts sooner than a
+// warp fills its tables. Interpolation, a CTA a column -> several a warp: ten columns of 2^5 4.3 -> 4.8 us, of 2^6 5.1 -> 5.9, of 2^8 6.4 -> 6.1; 300 of 2^7 5.5 ->
+// 6.7; 2,000 of 2^5, 2^6 and 2^7 5.3 -> 5.4, 6.3 -> 6.4 and 6.7 -> 6.6, 4,000 of 2^6 7.1 -> 6.1; 800 of 2^8 6.7 -> 6.9, 1,200 8.0 -> 7.1; 400 of 2^9 7.5 -> 7.4, 600 8.4 -> 7.0.
+static std::vector<FftStep> plan_steps(int nl, int log_n, bool aligned, int ncols) {
     std::vector<FftStep> v;
-    if (log_n >= 5 && log_n < 10 && aligned && nl > 0) {
+    if (log_n >= 5 && log_n < 10 && aligned && nl > 0 && (ncols >= 2048 || ((size_t)ncols << log_n) >= ((size_t)1 << 18))) {
         v.push_back({2, {}, {0, 0, nl}});
         return v;
     }
@@ -343,7 +347,7 @@ int lde_cols_blocked(zkb_ctx* ctx, const uint32_t* const* coeffs, int ncols, int
     for (int c = 0; c < ncols; c++) aligned = aligned && (((uintptr_t)out[c] | (uintptr_t)coeffs[c]) & 15) == 0;
     if (log_n < 2) aligned = false;  // the staged copies move 16 bytes at a time
     if (!plain) ZKB_CHECK_ARG(ctx, aligned && lde_blocked_supported(log_n, log_out, blk_log) && (blk_stride & 3u) == 0);
-    auto steps = plan_steps(log_n, log_out, aligned);
+    auto steps = plan_steps(log_n, log_out, aligned, ncols);
     uint32_t src_mask = (1u << log_n) - 1u;
     // ZKB_LDE_CHUNK=k runs all passes over k columns at a time, so that the array between two passes (2^log_out
     // words per column) is still in the L2 cache when the next pass reads it. Off by default: at 256 x 2^22 the
@@ -420,7 +424,7 @@ int zkb_ifft_cols(zkb_ctx* ctx, uint32_t* const* cols, int ncols, int log_n) {
     }
     bool aligned = true;
     for (int c = 0; c < ncols; c++) aligned = aligned && ((uintptr_t)cols[c] & 15) == 0;
-    auto steps = plan_steps(log_n, log_n, aligned);
+    auto steps = plan_steps(log_n, log_n, aligned, ncols);
     uint32_t n_inv = m31_inv(1u << log_n);
     for (size_t p = 0; p < steps.size(); p++) {
         rc = launch_step<true>(ctx, dc, (const uint32_t* const*)dc, 0xffffffffu, ncols, log_n, log_n, steps[p],
