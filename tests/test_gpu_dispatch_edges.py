@@ -205,7 +205,6 @@ def test_merkle_layers_of_many_columns(ctx, oracle, log_size, ncols, with_prev):
         assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, prev, cols, m31=m31)).all()
 
 
-
 @pytest.mark.parametrize("log_n,n_cols,runs", [(15, 1, True), (16, 39, False), (16, 40, True), (18, 9, False), (18, 10, True), (20, 2, False), (20, 3, True)])
 def test_eval_at_point_where_runs_begin(ctx, oracle, log_n, n_cols, runs):
     # one run a column, or eighty runs of sixteen chunks
@@ -215,7 +214,6 @@ def test_eval_at_point_where_runs_begin(ctx, oracle, log_n, n_cols, runs):
     got = ctx.eval_at_point_cols([b.ptr for b in bufs], log_n, point)
     assert ("eval_runs_kernel" in ctx.profile_end()) == runs
     assert (got == np.stack([oracle.eval_at_point(c, point) for c in cols])).all()
-
 
 
 @pytest.mark.parametrize("log_size,ncols,chain", [(0, 95, False), (0, 96, True), (8, 95, False), (11, 95, False), (11, 96, True), (11, 129, True), (12, 1535, False),
@@ -229,12 +227,10 @@ def test_merkle_layers_where_the_loader_warp_begins(ctx, oracle, log_size, ncols
     assert (out.download(shape=(-1, 8)) == oracle.commit_on_layer(log_size, None, cols, m31=True)).all()
 
 
-
 @pytest.mark.parametrize("log_n,n_cols", [(1, 40), (2, 39), (2, 41), (13, 39), (13, 40), (16, 40), (17, 47), (17, 49), (18, 111), (18, 112)])
 def test_numerators_where_the_split_begins(ctx, oracle, log_n, n_cols):
     # 40 entries; 48 and 112 where the rows leave room for four pieces and for two
     test_numerators_split_over_columns(ctx, oracle, log_n, n_cols)
-
 
 
 @pytest.mark.parametrize("n_acc", [1, 2, 3, 4, 5, 9])
@@ -256,12 +252,10 @@ def test_quotients_of_many_rows_combined(ctx, oracle, n_acc, log_n, row_begin, n
     assert (np.stack([o.download() for o in outs]) == want).all()
 
 
-
 @pytest.mark.parametrize("n_cols,log_n,blowup,shift,two", [(247, 17, 1, 0, 0), (248, 17, 1, 0, 0), (248, 17, 1, 1, 0), (248, 17, 1, 2, 3), (104, 18, 2, 0, 5)])
 def test_pcs_proof_where_the_numerators_of_coefficients_begin(ctx, oracle, n_cols, log_n, blowup, shift, two):
     # 24 M words and 28 columns of evaluations saved: 248 columns of 2^17 at blow-up 2
     test_pcs_proof_around_the_numerators_of_coefficients(ctx, oracle, n_cols, log_n, blowup, shift, two)
-
 
 
 @pytest.mark.parametrize("log_n,n_cols,short", [(5, 2047, False), (5, 2048, True), (6, 2051, True), (7, 2049, True), (8, 1023, False), (8, 1024, True), (9, 511, False), (9, 513, True)])
