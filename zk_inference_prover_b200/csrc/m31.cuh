@@ -116,7 +116,7 @@ ZK_HD bool qm31_is_zero(qm31 x) { return (x.c[0] | x.c[1] | x.c[2] | x.c[3]) == 
 // (A + B u)(C + D u) = (AC + (2+i) BD) + (AD + BC) u, qm31.rs:80-88. (2+i) D = e0 + e1 i is formed first, so that every output
 // coordinate is four 62-bit products and one fold: folding BD before it is multiplied by 2+i is two folds more, on the longest
 // path (233 -> 319 G products/s over all SMs, latency 188 -> 163 cycles). Subtracted products take p - x for x. 4 p^2 < 2^64.
-// What is in r (at most 2^34 a coordinate) is added: 4 p^2 = 2^64 - 2^34 + 4.
+// What is in r is added: a canonical word or a folded sum, at most 3 (2^32 - 1) = 2^34 - 2^32 - 3; 4 p^2 = 2^64 - 2^34 + 4.
 ZK_HD void qm31_add_products(uint64_t (&r)[4], qm31 x, qm31 y) {
     const uint32_t e0 = m31_sub(m31_dbl(y.c[2]), y.c[3]), e1 = m31_add(y.c[2], m31_dbl(y.c[3]));
     const uint32_t n1 = P - x.c[1], n3 = P - x.c[3];
@@ -139,7 +139,7 @@ ZK_HD qm31 qm31_mul_add(qm31 x, qm31 y, qm31 z) {
     return qm31_reduce64(r);
 }
 ZK_HD qm31 qm31_sqr(qm31 x) { return qm31_mul(x, x); }
-// A sum of secure products, its coordinates folded (< 2^34) and not reduced. Adding a product costs its sixteen multiply-adds and four folds; the
+// A sum of secure products, its coordinates folded (at most 3 (2^32 - 1)) and not reduced. Adding a product costs its sixteen multiply-adds and four folds; the
 // reductions and additions that a product and a sum of its own would take, half of their ALU instructions, come once at the end.
 struct qm31_sum {
     uint64_t c[4];
