@@ -269,7 +269,8 @@ def algorithmic_bytes(ncols, n, N):
         "interpolate": 8.0 * n * ncols,                 # read n + write n per column
         "extend": (4.0 * n + 4.0 * N) * ncols,          # read n coefficients, write N evaluations
         "merkle_leaves": 4.0 * ncols * N + 32.0 * N,    # read every evaluation, write one hash per row
-        "quot_numerators": 4.0 * ncols * N + 16.0 * N,  # one sample batch
+        "quot_numerators": 4.0 * ncols * N + 16.0 * N,  # one sample batch, of the evaluations
+        "quot_numerators_of_coefficients": 4.0 * ncols * n + 16.0 * n,  # the same of the coefficients; four columns are extended after it
     }
 
 
@@ -407,37 +408,42 @@ def run_ours(args, rank, world, local_rank):
         per = {k: v / args.steps for k, v in phases.items()}
         peak, peak_kind = measured_hbm_peak()
         ab = algorithmic_bytes(ncols, n, N)
+        # Wide, tall groups have their quotient numerators combined from the coefficients, and the four columns of the combination extended: these
+        # are among the timeline's forward transforms, and counted with them.
+        numerators = "quot_numerators_kernel(coefficients)" if "quot_numerators_kernel(coefficients)" in kernels else "quot_numerators_kernel"
+        numerator_bytes = ab["quot_numerators_of_coefficients" if "(" in numerators else "quot_numerators"]
+        extended = ncols + (4 if "(" in numerators else 0)
         # dominant operator: the LDE (two launches: the strided radix-32 pass, then the contiguous one)
         fwd = [(k, v) for k, v in kernels.items() if "forward" in k]
         lde_ms = sum(v[0] for _, v in fwd)
-        achieved = ab["extend"] / (lde_ms * 1e-3) / 1e9 if lde_ms else None
+        achieved = ab["extend"] / ncols * extended / (lde_ms * 1e-3) / 1e9 if lde_ms else None
         kern = {k: {"ms": round(v[0], 4), "launches": v[1]} for k, v in sorted(kernels.items(), key=lambda kv: -kv[1][0])}
         # DRAM traffic of the two LDE launches: ncu's dram__bytes_read + dram__bytes_write on 32 columns of this shape
-        # (137 + 482 MB for the wide pass, 569 + 479 MB for the twelve-layer contiguous pass), scaled by the column
+        # (137 + 479 MB for the wide pass, 566 + 480 MB for the twelve-layer contiguous pass), scaled by the column
         # count; a figure from a past capture, not measured in this run.
-        traffic = 1666.6e6 / 32 * ncols if (log_n, args.log_blowup) == (20, 2) else None
+        traffic = 1662e6 / 32 * extended if (log_n, args.log_blowup) == (20, 2) else None
         # The passes are bound by instruction issue: report them against the measured rate of the butterfly
         # arithmetic alone (the library's register-only butterfly kernel, timed in this run at this clock).
-        butterflies = ncols * (N // 2) * log_n  # the layers above the coefficient count only copy
+        butterflies = extended * (N // 2) * log_n  # the layers above the coefficient count only copy
         ceiling = ctx.fft_arith_ceiling()
         issue = {"bound": "instruction issue", "achieved": butterflies / (lde_ms * 1e-3) if lde_ms else None, "peak": ceiling,
                  "unit": "butterflies/s", "frac": butterflies / (lde_ms * 1e-3) / ceiling if lde_ms else None,
                  "peak_kind": "measured in this run: the same radix-32 butterfly stages on registers only, no global traffic, 2 CTAs x 256 threads per SM",
-                 "note": "about 10.5 machine instructions per butterfly at one instruction per cycle per scheduler saturate the "
-                         "ALU and FMA-heavy pipes together"}
-        roofline = {"bound": "hbm", "kernel": "+".join(k for k, _ in fwd) + " (the launches of one LDE)",
+                 "note": "a forward butterfly is 6.5 machine instructions, the passes run 7.7-7.9 for each (addresses, twiddles, exchanges); the "
+                         "ALU and FMA-heavy pipes take one every two cycles"}
+        roofline = {"bound": "hbm", "kernel": "+".join(k for k, _ in fwd) + f" (the launches that extend {extended} columns)",
                     "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak if achieved else None,
                     "traffic": traffic, "traffic_source": "ncu capture on 32 of the columns, scaled by the column count (an estimate for this run)",
                     "peak_kind": peak_kind, "issue": issue,
                     "note": "achieved = algorithmic bytes (read 2^log_size, write 2^(log_size+log_blowup) words per column) / the "
-                            "CUDA-event time of the two launches; the kernels are instruction-issue bound (see `issue`), DRAM at "
+                            "CUDA-event time of the launches; the kernels are instruction-issue bound (see `issue`), DRAM at "
                             "25-40% of peak; the 2.5x traffic is the array between the two passes",
                     "per_phase_ms": per, "kernels_one_step": kern,
                     "per_operator_gbs": {
                         "interpolate": ab["interpolate"] / (sum(v[0] for k, v in kernels.items() if "inverse" in k) * 1e-3) / 1e9,
                         "extend": achieved,
                         "merkle_leaves": ab["merkle_leaves"] / (kernels.get("merkle_layer_kernel(leaves)", (1e9, 1))[0] * 1e-3) / 1e9,
-                        "quot_numerators": ab["quot_numerators"] / (kernels.get("quot_numerators_kernel", (1e9, 1))[0] * 1e-3) / 1e9,
+                        "quot_numerators": numerator_bytes / (kernels.get(numerators, (1e9, 1))[0] * 1e-3) / 1e9,
                         **standalone}}
         roofline["per_operator_frac_of_hbm_peak"] = {k: v / peak for k, v in roofline["per_operator_gbs"].items()}
         roofline["same_bytes_by_device_copy_gbs"] = copy_ceiling  # one cudaMemcpyAsync D2D per launch, same byte counts

@@ -313,7 +313,7 @@ static int launch_numerators(zkb_ctx* ctx, const uint32_t* const* cols, int ncol
     bool wide = n >= 4;
     for (int q = 0; q < 4; q++) wide = wide && ((uintptr_t)o.c[q] & 15) == 0;
     for (int c = 0; c < ncols; c++) wide = wide && ((uintptr_t)cols[c] & 15) == 0;
-    ProfScope prof(ctx, "quot_numerators_kernel");
+    ProfScope prof(ctx, b_first ? "quot_numerators_kernel(coefficients)" : "quot_numerators_kernel");
     // Few rows: the columns are split over the grid's second dimension, so that some 148 x 4 CTAs' worth of threads have loads on their way, sixteen
     // columns each at least. A thread walks its columns four at a time, a trip to memory each: a hundred columns of 2^13 rows on
     // eight CTAs were 35 us, of 2^17 rows 41; split, and added up, 10 + 4 and 18 + 8. Groups of fewer than 1,024 rows take narrower CTAs.
