@@ -42,6 +42,22 @@ def test_gkr_single_instance_around_the_chain(ctx, oracle, kind, log_n):
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("kind,log_n,value", [(k, n, None) for k in (0, 1, 2, 3) for n in (4, 5, 11)] + [(0, 2, 1), (0, 7, 0), (0, 11, 1), (1, 3, 1), (1, 10, 1), (1, 11, 0)])
+def test_gkr_single_instance_a_round_ahead(ctx, oracle, kind, log_n, value):
+    """Layers that are taken whole, the one above them, and constant ones, whose round polynomials are of low degree or nothing."""
+    n = 1 << log_n
+    den = qm31_array(7000 + log_n, n, nonzero=True)
+    num = qm31_array(7100 + log_n, n) if kind == 1 else m31_column(7200 + log_n, n) if kind == 2 else None
+    if value is not None:
+        den = np.zeros_like(den)
+        den[:, 0] = value
+        num = np.zeros_like(num) if num is not None else None
+    want = oracle.gkr_prove([(kind, num, den)], 0x5EED0016, verify=True)
+    nb, db = ctx.upload(num) if num is not None else None, ctx.upload(den)
+    got = ctx.gkr_prove_device([(kind, nb.ptr if nb else 0, db.ptr, n)], 0x5EED0016)
+    assert len(got) == len(want) and (got == want).all()
+
+
 @pytest.mark.parametrize("log_n", [2, 9, 10, 11, 12])
 def test_gkr_batch_around_the_tower_launches(ctx, oracle, log_n):
     inst, dev, keep = [], [], []

@@ -10,16 +10,19 @@
 // kept off that chain:
 //   * Layers of at most 2^13 entries run in ONE CTA (res_chain_kernel): from the first fold on they live in its shared memory,
 //     and as many whole layers as are small follow one another in the same launch, so a round costs no launch and no trip to L2.
-//   * What a round polynomial depends on beside the two sums is prepared while the data warps work on the layer: the basis
-//     polynomials of all rounds of a layer while its claims are mixed in, the claims, the corrections and the coefficients' share
-//     that does not depend on the sums (one warp) while the others fold. Between the sums and the hash there is one
-//     multiplication.
+//   * One oracle's rounds of at most 2^8 terms are worked out a round ahead (look_work): while a round's polynomial is hashed the other warps make
+//     the next one as a function of the challenge to come. Between a challenge and the next hash are two products. The next layer's arrays and basis
+//     are made ready under the hash of the mask, its first sums, linear in lambda, under the hash of the claims.
+//   * In the other rounds what a polynomial depends on beside the two sums is prepared while the data warps work on the layer: the basis polynomials
+//     of all rounds of a layer while its claims are mixed in, the claims, the corrections and the coefficients' share that does not depend on the sums
+//     (one warp) while the others fold.
 //   * Rounds on larger layers are one launch each (res_round_kernel): the fold by the round before's challenge, the sums of the
 //     result, and, by the CTA that finishes last, the transcript step; the next launch is a programmatic dependent of it.
 //   * eq(., point) is never written out for these: the terms are taken in chunks of at most 2^11 with one factor in common,
 //     eq = A[low 11 bits] B[the rest], so a pass reads a table of 32 KB and multiplies by B once per chunk.
-// Measured (one instance): 2^10 fractions 906 -> 314 us, 2^24 fractions 7.95 -> 3.36 ms. Of the latter's 276 rounds the chain kernel takes
-// 199 in 1.60 ms, 8 us each with the layers' begins and ends; 77 are launches.
+// Measured (one instance): 2^10 fractions 906 -> 317 -> 224 us, 2^24 fractions 7.95 -> 3.37 -> 3.21 ms (the last steps: rounds a round ahead, 12,000 ->
+// 5,150 cycles each, of which the three compressions take 3,900; a layer's begin and end 22,000 -> 9,500). Code that runs once a layer is cold: some five
+// cycles an instruction, so what is not on the transcript's path is better simple than short.
 #include <algorithm>
 #include <vector>
 
@@ -107,6 +110,9 @@ struct alignas(16) TrSm {
     // the round after before its correction, the challenge and one minus it, the prefix product, intermediate values, zero
     qm31 A[8], H[2], next_h[2], r, omr, pcur, tmp[5], zero, sink[32];
     uint32_t n_vars[RES_MAX_INST];            // variables of the layer's oracles
+    // rounds worked out ahead (look_rounds): the next polynomial's coefficients as cubics in the challenge, low first; the sums they are made
+    // of; the challenges of this round and the last (and the two polynomials); the first round's sums (solo_begin)
+    qm31 look_coef[2][4], ahead[16], look_sums[12], look_r[2], first_sums[32];
 };
 
 // Any set of threads; a barrier must follow (and precede tr_store's readers).
@@ -134,47 +140,37 @@ __device__ __forceinline__ void tr_store(const TrSm& t, ResState* st, int thread
 // b = (1 - y) / (1 - 2y), i.e. it is r0 L0 + r1 L1 + r2 L2; r0 = sum0 corr e0a, r2 = sum2 corr e2a with e0a = eq(0, y) / a and
 // e2a = eq(2, y) / a, a = prod_{i <= n - k} eq(0, y_i). The inversions (of a, 1 - 2y, 1 - y, y, 1 - 3y; those of b, 1 - b and 2 - b
 // follow) are one per thread.
-__device__ __forceinline__ void basis_inverses(const TrSm& t, qm31* inv, int nv, int thread, int n_threads) {
-    for (int i = thread; i < 5 * nv; i += n_threads) {
-        const int j = i / 5, w = i % 5;  // round j: nv - j variables left; ood has nv entries
-        const qm31 y = t.s.ood[j], omy = one_minus(y);
-        qm31 v = t.s.prefix[j + 1];
-        if (w == 1) v = one_minus(qm31_dbl(y));
-        if (w == 2) v = omy;
-        if (w == 3) v = y;
-        if (w == 4) v = qm31_sub(omy, qm31_dbl(y));
-        inv[i] = qm31_inv(v);
+// Rounds [first, n) of a layer, ys: their variables, prefix: the products before them.
+__device__ __forceinline__ void basis_inverses(const qm31* ys, qm31* prefix, qm31* inv, int first, int n, int thread, int n_threads) {
+    for (int i = 5 * first + thread; i < 5 * n; i += n_threads) {
+        const int j = i / 5, w = i % 5;
+        const qm31 y = ldq_r(ys, j), omy = one_minus(y), y2 = qm31_dbl(y);
+        const qm31 a = qm31_mul(ldq_r(prefix, j), omy);
+        if (w == 0) stq_r(prefix, j + 1, a);  // (what is there already, but for the last one)
+        stq_r(inv, i, qm31_inv(w == 0 ? a : w == 1 ? one_minus(y2) : w == 2 ? omy : w == 3 ? y : qm31_sub(omy, y2)));
     }
 }
-__device__ __forceinline__ void basis_rounds(const TrSm& t, const qm31* inv, qm31* basis, int nv, int thread, int n_threads) {
-    for (int i = thread; i < BASIS_Q * nv; i += n_threads) {
-        const int j = i / BASIS_Q, w = i % BASIS_Q;
+// Every value is (p0 + p1 b) q, of lanes that all do the same: L1 = -t(t-2)(t-b) / (1-b), L2 = t(t-1)(t-b) / 2(2-b), L0 = -(t-1)(t-2)(t-b) / 2b, low
+// coefficients first; 1/b = d / (1-y), -1/(1-b) = d / y, 1/(2-b) = d / (1-3y) with d = 1 - 2y. By whole warps.
+__device__ __forceinline__ void basis_rounds(const qm31* ys, const qm31* inv, qm31* basis, int first, int n, int thread, int n_threads) {
+    for (int i0 = BASIS_Q * first + (thread & ~31); i0 < BASIS_Q * n; i0 += n_threads) {
+        const int i = i0 + (thread & 31), j = min(i / BASIS_Q, n - 1), w = i % BASIS_Q, c = w & 3;
         const qm31* iv = inv + 5 * j;
-        const qm31 y = t.s.ood[j], omy = one_minus(y), d = one_minus(qm31_dbl(y));
-        qm31 v = w == 14 ? y : omy;
-        if (w < 12) {
-            const int c = w & 3;
-            const qm31 b = qmul(omy, iv[1]), b2 = qm31_dbl(b);
-            auto small = [](uint32_t m) { return qm31_from_m31(m); };
-            // L1 = -t(t-2)(t-b) / (1-b), L2 = t(t-1)(t-b) / 2(2-b), L0 = -(t-1)(t-2)(t-b) / 2b, low coefficients first;
-            // 1/b = d / (1-y), -1/(1-b) = d / y, 1/(2-b) = d / (1-3y)
-            const qm31 p1 = c == 0 ? qm31_zero() : c == 1 ? b2 : c == 2 ? qm31_neg(qm31_add(small(2), b)) : qm31_one();
-            if (w >= 8) {
-                const qm31 p2 = c == 0 ? qm31_zero() : c == 1 ? b : c == 2 ? qm31_neg(qm31_add(qm31_one(), b)) : qm31_one();
-                v = qm31_mul_m31(qmul(p2, qmul(d, iv[4])), 1u << 30);
-            } else {
-                v = qmul(p1, qmul(d, iv[3]));
-                if (w < 4) {
-                    const qm31 p0 = c == 0 ? b2 : c == 1 ? qm31_neg(qm31_add(small(2), qm31_add(b2, b))) : c == 2 ? qm31_add(small(3), b) : qm31_neg(qm31_one());
-                    v = qm31_sub(qm31_mul_m31(qmul(p0, qmul(d, iv[2])), 1u << 30), v);
-                }
-            }
-        } else if (w == 12) {
-            v = qmul(omy, iv[0]);
-        } else if (w == 13) {
-            v = qmul(qm31_neg(qm31_sub(omy, qm31_dbl(y))), iv[0]);  // eq(2, y) = 3y - 1
-        }
-        basis[i] = v;
+        const qm31 y = ldq_r(ys, j), omy = one_minus(y), y2 = qm31_dbl(y), d = one_minus(y2);
+        const qm31 b = qm31_mul(omy, ldq_r(iv, 1)), q = qm31_mul(d, ldq_r(iv, w < 4 ? 2 : w < 8 ? 3 : 4)), b2 = qm31_dbl(b);
+        auto small = [](uint32_t m) { return qm31_from_m31(m); };
+        // the polynomials' numerators: t(t-2)(t-b), t(t-1)(t-b) and -(t-1)(t-2)(t-b)
+        const qm31 p1 = c == 0 ? qm31_zero() : c == 1 ? b2 : c == 2 ? qm31_neg(qm31_add(small(2), b)) : qm31_one();
+        const qm31 p2 = c == 0 ? qm31_zero() : c == 1 ? b : c == 2 ? qm31_neg(qm31_add(qm31_one(), b)) : qm31_one();
+        const qm31 p0 = c == 0 ? b2 : c == 1 ? qm31_neg(qm31_add(small(2), qm31_add(b2, b))) : c == 2 ? qm31_add(small(3), b) : qm31_neg(qm31_one());
+        // eq(0, y) / a and eq(2, y) / a, eq(2, y) = 3y - 1
+        const qm31 x = w < 4 ? p0 : w < 8 ? p1 : w < 12 ? p2 : w == 12 ? omy : qm31_neg(qm31_sub(omy, y2));
+        qm31 v = qm31_mul(x, w < 12 ? q : ldq_r(iv, 0));
+        if (w < 4 || (w >= 8 && w < 12)) v = qm31_mul_m31(v, 1u << 30);
+        const qm31 l1 = shfl_q(v, (thread + 4) & 31);
+        if (w < 4) v = qm31_sub(v, l1);
+        if (w >= 14) v = w == 14 ? y : omy;
+        if (i < BASIS_Q * n) stq_r(basis, i, v);
     }
 }
 
@@ -321,11 +317,11 @@ __device__ __forceinline__ void tr_prepare(TrSm& t, const qm31* B, uint32_t basi
     }
 }
 // The round polynomial of the batch from the oracles' sums (sumcheck.rs:139-149), mixed into the channel, and the round's
-// challenge. poly: POLY_WORDS words of the proof. parts: the one oracle's sums as two addends per node, or NULL.
-__device__ __forceinline__ void tr_round(TrSm& t, const qm31* B, int K, uint32_t n_rem, int round, uint32_t* poly, const qm31* parts) {
-    const int lane = threadIdx.x & 31, node = (lane >> 2) & 1;
+// challenge. poly: POLY_WORDS words of the proof.
+__device__ __forceinline__ void tr_round(TrSm& t, const qm31* B, int K, uint32_t n_rem, int round, uint32_t* poly) {
+    const int lane = threadIdx.x & 31;
     qm31 p;
-    if (K == 1) p = qm31_mul(parts ? qm31_add(parts[node], parts[2 + node]) : ldq_r(t.s.sums[0], node), t.A[lane & 7]);
+    if (K == 1) p = qm31_mul(ldq_r(t.s.sums[0], (lane >> 2) & 1), t.A[lane & 7]);
     else p = many_coefficients(t, B, K, n_rem);
     const qm31 c = qm31_add(qm31_add(p, shfl_q(p, (lane + 4) & 31)), t.base[lane & 3]);
     if (lane < 4) {
@@ -539,7 +535,7 @@ __global__ void __launch_bounds__(ROUND_THREADS, 2) res_round_kernel(const __gri
         tr_open_channel(tr, lane);
         if (lane == 0) tr.pcur = tr.s.prefix_next[a.round];
         tr_prepare(tr, sm.basis, 0u, a.n_oracles, (uint32_t)a.n_rem);
-        tr_round(tr, sm.basis, a.n_oracles, (uint32_t)a.n_rem, a.round, a.poly, nullptr);
+        tr_round(tr, sm.basis, a.n_oracles, (uint32_t)a.n_rem, a.round, a.poly);
         tr_close_channel(tr, lane);
         tr_update(tr, sm.basis, 0u, a.n_oracles, (uint32_t)a.n_rem, a.round, false);
     }
@@ -727,7 +723,7 @@ __device__ __forceinline__ qm31 small_unit(int kind, const void* num, const void
     }
     return warp_sum_q(s);
 }
-// The same once numerators have been changed for m = n + (lambda / 2) d: products m0 d1 and m1 d0 (a grand product: d0 d1).
+// The same for one oracle, whose numerators have been changed for m = n + (lambda / 2) d: products m0 d1 and m1 d0 (a grand product: d0 d1).
 __device__ __forceinline__ qm31 small_unit_m(bool product, const void* m, const void* den, uint32_t nt, uint32_t i, int node, int part, const void* eq) {
     qm31 s = qm31_zero();
     if (i < nt && !(product && part)) {
@@ -742,6 +738,371 @@ __device__ __forceinline__ qm31 small_unit_m(bool product, const void* m, const 
     return s;
 }
 
+// ---- the small rounds of one oracle, a round ahead of the transcript
+//
+// A layer fixed at r is linear in r and a term is a product of two of its entries, so the next round's sums are quadratic in this round's
+// challenge: S(r) = C0 + C1 r + C2 r^2, and with the correction, linear in r, and the claim, this round's cubic at r, the coefficients of the
+// next polynomial are cubics in r. Their coefficients are worked out while the first warp hashes this round's polynomial; when it
+// has the challenge it has the next polynomial two products later and hashes on. The layer itself is fixed under the next hash. What was on a
+// round's path and no longer is: the fold, the sums and three levels of products, with the barriers between them.
+//
+// A round:
+//   warp 0          next polynomial from `ahead`, its hash, the challenge
+//   LOOK_WARPS      the layer fixed at the last challenge; then six sums, two warps each (the second for passes of more than 32 terms): two
+//                   nodes (t = 0, 2) x the term at r = 0, at r = 1 and its leading coefficient
+//   the last one    correction at the last challenge besides; `ahead` from the sums and the polynomial being hashed
+// Warp 0 has its scheduler to itself: what other warps issue there is taken from its turns (three compressions 3,930 -> 4,600 cycles).
+constexpr int LOOK_WARPS = 12;
+constexpr uint32_t LOOK_TERMS = 256;  // passes of more terms take longer this way than the hash they would hide under
+static_assert(RES_WARPS == 16, "twelve warps are not on warp 0's scheduler");
+// The barriers: a polynomial is there (warp 0 to the helper), the layer is fixed (the twelve), the sums are there (the twelve to the helper), so is the last
+// round's basis (solo_last_basis to the helper). Warp 0 and the twelve meet when a challenge is there: what is due by then (`ahead`, the mask) is.
+__device__ __forceinline__ void look_poly_set() { asm volatile("bar.arrive 3, 64;" ::: "memory"); }
+__device__ __forceinline__ void look_poly_wait() { asm volatile("bar.sync 3, 64;" ::: "memory"); }
+__device__ __forceinline__ void look_fixed() { asm volatile("bar.sync 4, %0;" ::"n"(32 * LOOK_WARPS) : "memory"); }
+__device__ __forceinline__ void look_sums_set() { asm volatile("bar.arrive 5, %0;" ::"n"(32 * LOOK_WARPS) : "memory"); }
+__device__ __forceinline__ void look_sums_wait() { asm volatile("bar.sync 5, %0;" ::"n"(32 * LOOK_WARPS) : "memory"); }
+__device__ __forceinline__ void look_basis_set() { asm volatile("bar.arrive 7, 64;" ::: "memory"); }
+__device__ __forceinline__ void look_basis_wait() { asm volatile("bar.sync 7, 64;" ::: "memory"); }
+__device__ __forceinline__ void look_challenge() { asm volatile("bar.sync 6, %0;" ::"n"(32 * (LOOK_WARPS + 1)) : "memory"); }
+
+// A layer that is taken whole this way.
+__device__ __forceinline__ bool is_solo(const ChainLayer& L) {
+    return L.flags == (CHAIN_BEGIN | CHAIN_ROUNDS | CHAIN_END) && L.n_oracles == 1 && L.nv > 0 && (1u << (L.nv - 1)) <= LOOK_TERMS;
+}
+// The work areas of two such layers, of at most 4 LOOK_TERMS entries a column: while one ends the next is fetched.
+constexpr uint32_t SOLO_BYTES = 64 * LOOK_TERMS;
+constexpr int SOLO_BASIS_WARPS = 5;
+static_assert(4 * SOLO_BYTES <= CHAIN_WORK_BYTES, "two layers of two columns");
+__device__ __forceinline__ void solo_done() { asm volatile("bar.sync 9, %0;" ::"n"(RES_THREADS) : "memory"); }
+
+// A product by y, a coordinate a lane (its two low bits): four multiply-adds and a reduction, where a lane that makes all four takes sixteen and four.
+struct slice_by {
+    uint32_t m[4];
+    __device__ __forceinline__ slice_by(qm31 y) {
+        const int k = threadIdx.x & 3;
+        const uint32_t e0 = m31_sub(m31_dbl(y.c[2]), y.c[3]), e1 = m31_add(y.c[2], m31_dbl(y.c[3]));
+        m[0] = k == 0 ? y.c[0] : k == 1 ? y.c[1] : k == 2 ? y.c[2] : y.c[3];
+        m[1] = k == 0 ? P - y.c[1] : k == 1 ? y.c[0] : k == 2 ? P - y.c[3] : y.c[2];
+        m[2] = k == 0 ? e0 : k == 1 ? e1 : k == 2 ? y.c[0] : y.c[1];
+        m[3] = k == 0 ? P - e1 : k == 1 ? e0 : k == 2 ? P - y.c[1] : y.c[0];
+    }
+    // coordinate k of x y, and the word z added (qm31_add_products has the bound)
+    __device__ __forceinline__ uint32_t mul_add(qm31 x, uint32_t z) const {
+        return m31_reduce64(z + (uint64_t)x.c[0] * m[0] + (uint64_t)x.c[1] * m[1] + (uint64_t)x.c[2] * m[2] + (uint64_t)x.c[3] * m[3]);
+    }
+};
+// The value whose coordinates are in lanes first ... first + 3.
+__device__ __forceinline__ qm31 gather_q(uint32_t v, int first) {
+    qm31 r;
+#pragma unroll
+    for (int c = 0; c < 4; c++) r.c[c] = __shfl_sync(0xffffffffu, v, first + c);
+    return r;
+}
+
+// Where one_lead starts and ends.
+enum : int { LEAD_BEGIN = 1, LEAD_ROUNDS = 2, LEAD_SUMS = 4 };
+
+// Warp 0, for a layer with one oracle. LEAD_BEGIN: its claims into the channel, lambda (gkr_prover.rs:669-735). LEAD_ROUNDS: rounds round0 ... nv - 1, from the sums of round0's units in red (LEAD_SUMS) or, with the begin, from `ahead` at lambda; the
+// mask into the channel, the next layer's last coordinate and claims (gkr_prover.rs:745-800). The mask's hash is the loop's last turn, so that the
+// code of the hash is there once. With both it goes on to the layers after this one while they are taken whole; returns the layer it stopped at.
+__device__ __noinline__ int one_lead(TrSm& t, const ChainLayer* bufs, int d, int n_layers, int what, int round0, const qm31* red, uint32_t units, const unsigned char* num,
+                                     const unsigned char* den) {
+    const int lane = threadIdx.x & 31;
+    const QuadWords words(t.ch.msg, t.ch.sched);
+    const QuadConst qc;
+    for (;;) {
+        const ChainLayer& L = bufs[d & 1];
+        const int nv = L.nv, inst = L.inst[0];
+        const bool product = L.kind[0] == ZKB_GKR_GRAND_PRODUCT;
+        const uint32_t area = what & LEAD_SUMS ? 0u : (d & 1) * SOLO_BYTES;
+        qm31 r = qm31_zero(), mask = r;
+        uint32_t c = 0u;  // lane = 4 k + coordinate (and 16 more): coefficient k of the round's polynomial
+        if (what & LEAD_SUMS) {
+            const qm31 v = (uint32_t)lane < units ? red[lane] : qm31_zero();
+            const qm31 s0 = warp_sum_q((lane & 1) ? qm31_zero() : v), s2 = warp_sum_q((lane & 1) ? v : qm31_zero());
+            const qm31 p = qmul((lane & 4) ? s2 : s0, t.A[lane & 7]);
+            const qm31 q = qm31_add(qm31_add(p, shfl_q(p, (lane + 4) & 31)), t.base[lane & 3]);  // coefficient `lane` in lanes 0-3
+            const qm31 mine = shfl_q(q, (lane >> 2) & 3);
+            c = (lane & 3) == 0 ? mine.c[0] : (lane & 3) == 1 ? mine.c[1] : (lane & 3) == 2 ? mine.c[2] : mine.c[3];
+        }
+        for (int round = what & LEAD_BEGIN ? -1 : round0;; round++) {
+            unsigned nonzero = 0xffffu;  // the words mixed in
+            if (round >= 0 && round < nv) {
+                if (!(round == round0 && (what & LEAD_SUMS))) {
+                    // (d3 r + d2) r^2 + (d1 r + d0): the low half in lanes 0-15, the high one in 16-31
+                    const int at = (lane & 12) + (lane >> 4) * 2;
+                    const qm31 d1 = ldq_r(t.ahead, at + 1);
+                    const uint32_t d0 = t.ahead[at].c[lane & 3];
+                    const slice_by by(r);
+                    const uint32_t m = by.mul_add(d1, d0), r2 = by.mul_add(r, 0u);
+                    c = slice_by(gather_q(r2, 0)).mul_add(gather_q(m, 16 + (lane & 12)), m);
+                }
+                if (lane < 16) t.ch.msg[8 + lane] = c;
+                nonzero = __ballot_sync(0xffffffffu, lane < 16 && c != 0u);
+                if (!(nonzero & 0xff00u)) {  // two coefficients or fewer
+                    __syncwarp();
+                    chan_copy_digest(t.ch);
+                    if (lane < 8) t.ch.msg[24 + lane] = c;
+                }
+            } else if (round < 0) {
+                const int n = 4 * (int)t.s.n_claims[inst];
+                nonzero = (1u << n) - 1u;
+                chan_copy_digest(t.ch);
+                if (lane < n) t.ch.msg[24 + lane] = reinterpret_cast<const uint32_t*>(t.s.claims[inst])[lane];
+            } else {
+                // two entries a column (num0, num1, den0, den1; a grand product has the denominators only)
+                const void* const col = (product || (lane & 2) ? den : num) + area;
+                mask = fold_q(r, ldq_r(col, lane & 1), ldq_r(col, (lane & 1) + 2));
+                if (product) {
+                    nonzero = 0xffu;
+                    chan_copy_digest(t.ch);
+                }
+                if (lane < (product ? 2 : 4)) stq_r(t.ch.msg + (product ? 24 : 8), lane, mask);
+            }
+            __syncwarp();
+            const uint32_t v = chan_round(
+                t.ch, words, qc, (nonzero & 0xff00u) != 0u, round < 0 ? 1u : 0u,  // (alpha, the first draw of a begin, is the power of nothing here)
+                [&] { return 32u + 16u * (uint32_t)((35 - __clz(nonzero)) >> 2); },    // whole coefficients, up to the last that is not zero
+                [&] {
+                    if (round >= 0 && round < nv) {
+                        if (lane < 16) t.look_coef[round & 1][lane >> 2].c[lane & 3] = c;
+                        __syncwarp();
+                        if (nv - round >= 2) look_poly_set();
+                    } else if (round == nv && lane < 4) {
+                        stq_r(L.masks, lane, lane < (product ? 2 : 4) ? mask : qm31_zero());
+                    }
+                });
+            if (round < nv && lane < 4) t.look_r[round & 1].c[lane] = v;
+            r = gather_q(v, 0);
+            __syncwarp();
+            if (round == nv) break;
+            if (round < 0) {
+                if (lane == 0) {
+                    t.s.lambda = r;
+                    t.s.prefix_next[0] = t.pcur = t.s.apow[0] = t.s.corr[0] = qm31_one();
+                }
+                __syncwarp();
+                if (!(what & LEAD_ROUNDS)) {  // the claim, for rounds that are not worked out ahead
+                    const qm31 sc = qm31_add(qmul(product ? qm31_zero() : t.s.claims[inst][1], r), t.s.claims[inst][0]);
+                    if (lane == 0) t.s.sc[0] = sc;
+                    __syncwarp();
+                    return d;
+                }
+            }
+            look_challenge();
+        }
+        const qm31 claim = fold_q(r, shfl_q(mask, 2 * (lane & 1)), shfl_q(mask, 2 * (lane & 1) + 1));
+        if (lane < (product ? 1 : 2)) stq_r(t.s.claims[inst], lane, claim);
+        if (lane == 0) {
+            t.s.n_claims[inst] = product ? 1u : 2u;
+            t.s.challenge = t.s.ood[nv] = r;
+        }
+        __syncwarp();
+        if (what & LEAD_SUMS) return d;
+        solo_done();
+        if (++d == n_layers || !is_solo(bufs[d & 1])) return d;
+    }
+}
+
+// A layer's entries into the work area, numerators as they are.
+__device__ __forceinline__ void solo_fetch(const ChainLayer& L, unsigned char* num, unsigned char* den, uint32_t thread, uint32_t n_threads) {
+    const int kind = L.kind[0];
+    for (uint32_t e = thread; e < (2u << L.nv); e += n_threads) {
+        stq_r(den, e, ldq_r(L.den[0], e));
+        if (kind != ZKB_GKR_GRAND_PRODUCT)
+            stq_r(num, e, kind == ZKB_GKR_LOGUP_GENERIC ? ldq_r(L.num[0], e) : qm31_from_m31(kind == ZKB_GKR_LOGUP_MULTIPLICITIES ? L.num[0][e] : 1u));
+    }
+}
+
+// The twelve: rounds round0 ... nv - 1. num, den: the layer, 2^(nv - round0 + 1) entries, numerators as small_unit_m has them; `begins`: numerators
+// as they are, lambda is the first challenge. next (or null), then: the layer after this one, whose description goes to next_buf. If it is taken whole, its
+// arrays (to next_num, next_den) and all of its basis but for the last round are made ready while the mask is hashed.
+__device__ __forceinline__ void look_work(TrSm& t, qm31* basis, qm31* inv, int nv, int round0, bool begins, bool product, unsigned char* num, unsigned char* den, const void* eq,
+                                          uint32_t* polys, const ChainLayer* next, ChainLayer* next_buf, unsigned char* next_num, unsigned char* next_den) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t w = (uint32_t)((warp >> 2) * 3 + (warp & 3) - 1), sum = w % 6, node = sum & 1, at_r = sum >> 1, half = w / 6;
+    const bool helper = w == LOOK_WARPS - 1, keeper = w == LOOK_WARPS - 2;  // (the keeper: the point and its prefix products, the polynomials into the proof)
+    // the helper: lane = 16 node + 4 c + k has that node's share of the coefficient of r^k in coefficient c of the next polynomial
+    const int hn = lane >> 4, c = (lane >> 2) & 3, k = lane & 3;
+    qm31 corr = begins ? qm31_one() : t.s.corr[0], a0 = qm31_zero(), a1 = a0, l1 = a0, half_lambda = begins ? a0 : qm31_mul_m31(t.s.lambda, 1u << 30);
+    for (int round = round0; round <= nv; round++) {
+        const uint32_t n_rem = (uint32_t)(nv - round), n_out = 2u << n_rem;
+        if (helper && n_rem >= 2) {  // what does not depend on the challenge; the next correction is corr (w0 + w1 r)
+            if (n_rem == 2 && begins) look_basis_wait();
+            const qm31 *B = basis + BASIS_Q * round, *N = B + BASIS_Q;
+            const qm31 w0 = ldq_r(B, 15), g = qm31_mul(ldq_r(N, 12 + hn), ldq_r(N, 8 * hn + c));
+            a0 = qm31_mul(g, w0);
+            a1 = qm31_mul(g, qm31_sub(ldq_r(B, 14), w0));
+            l1 = ldq_r(N, 4 + c);
+        }
+        if (round > round0) {
+            look_challenge();
+            const qm31 r = ldq_r(t.look_r, (round & 1) ^ 1);
+            if (n_rem) {
+                for (uint32_t i = 32 * w + lane; i < (product ? n_out : 2 * n_out); i += 32 * LOOK_WARPS) {
+                    unsigned char* const p = i < n_out ? den : num;
+                    const uint32_t e = i & (n_out - 1);
+                    stq_r(p, e, fold_q(r, ldq_r(p, e), ldq_r(p, e + n_out)));
+                }
+                look_fixed();
+            }
+            if (helper && n_rem >= 2) {  // eq(r, y) in two parts
+                const qm31* L = basis + BASIS_Q * (round - 1);
+                const qm31 m = qm31_mul((lane & 1) ? one_minus(r) : r, ldq_r(L, 14 + (lane & 1)));
+                corr = qm31_mul(corr, qm31_add(m, shfl_q(m, lane ^ 1)));
+            }
+            if (keeper) {
+                const qm31 p = qmul(ldq_r(t.s.prefix_next, round - 1), one_minus(r));
+                __syncwarp();
+                if (lane == 0) { stq_r(t.s.prefix_next, round, p); stq_r(t.s.assign, round - 1, r); }
+                const qm31 v = ldq_r(t.look_coef[(round & 1) ^ 1], lane & 3);
+                const int len = 32 - __clz(__ballot_sync(0xffffffffu, lane < 4 && !qm31_is_zero(v)));
+                uint32_t* const poly = polys + (size_t)POLY_WORDS * (round - 1);
+                if (lane < 4) stq_r(poly, lane, v);
+                if (lane == 0) poly[16] = (uint32_t)len;
+                __syncwarp();
+            }
+            if (n_rem == 0) {
+                look_fixed();  // behind the keeper
+                if (keeper && lane <= nv) {
+                    if (lane < nv) t.s.ood[lane] = t.s.assign[lane];
+                    t.s.prefix[lane] = t.s.prefix_next[lane];
+                }
+                if (!next || !is_solo(*next_buf)) break;
+                if (w < SOLO_BASIS_WARPS) {
+                    basis_inverses(t.s.assign, t.s.prefix_next, inv, 0, nv, 32 * w + lane, 32 * SOLO_BASIS_WARPS);
+                    asm volatile("bar.sync 1, %0;" ::"n"(32 * SOLO_BASIS_WARPS) : "memory");
+                    basis_rounds(t.s.assign, inv, basis, 0, nv, 32 * w + lane, 32 * SOLO_BASIS_WARPS);
+                } else {
+                    solo_fetch(*next_buf, next_num, next_den, 32 * (w - SOLO_BASIS_WARPS) + lane, 32 * (LOOK_WARPS - SOLO_BASIS_WARPS));
+                }
+                break;
+            }
+        } else if (begins) {
+            look_challenge();
+            half_lambda = qm31_mul_m31(ldq_r(t.look_r, 1), 1u << 30);
+            if (n_rem >= 2 && !product) {
+                for (uint32_t e = 32 * w + lane; e < n_out; e += 32 * LOOK_WARPS) stq_r(num, e, qm31_mul_add(half_lambda, ldq_r(den, e), ldq_r(num, e)));
+                look_fixed();
+            }
+        }
+        if (keeper && begins && next && round == round0)  // the next layer's description: read after the next challenge
+            for (int i = lane; i < (int)(sizeof(ChainLayer) / 16); i += 32) reinterpret_cast<uint4*>(next_buf)[i] = __ldg(reinterpret_cast<const uint4*>(next) + i);
+        if (n_rem < 2) {  // what is left is folded to the mask by warp 0: numerators as they are again
+            if (!helper) continue;
+            if (lane < 4 && !product && !(begins && nv == 1)) stq_r(num, lane, qm31_sub(ldq_r(num, lane), qm31_mul(half_lambda, ldq_r(den, lane))));
+            continue;
+        }
+        const uint32_t nt = n_out >> 3;
+        qm31 s = qm31_zero();
+        for (uint32_t i = 32 * half + lane; i < nt; i += 64) {
+            auto fixed = [&](const void* p, uint32_t b, uint32_t h) {  // the half that stays at r = h
+                const uint32_t o = h * 4 * nt + 2 * i + b;
+                const qm31 v0 = ldq_r(p, o);
+                return node ? at_two(v0, ldq_r(p, o + 2 * nt)) : v0;
+            };
+            auto at = [&](const void* p, uint32_t b) {
+                const qm31 v = fixed(p, b, at_r ? 1u : 0u);
+                return at_r == 2 ? qm31_sub(v, fixed(p, b, 0u)) : v;
+            };
+            const qm31 d0 = at(den, 0), d1 = at(den, 1);
+            s = qm31_add(s, qm31_mul(ldq_r(eq, i), product ? qm31_mul(d0, d1) : qm31_dot2(at(num, 0), d1, at(num, 1), d0)));
+        }
+        if (nt >= 16) s = warp_sum_q(s);
+        else for (uint32_t off = nt >> 1; off; off >>= 1) s = qm31_add(s, shfl_q(s, lane + off));
+        if (lane == 0) stq_r(t.look_sums, w, s);
+        __syncwarp();
+        if (!helper) {
+            look_sums_set();
+            continue;
+        }
+        const qm31 b0 = qm31_mul(corr, a0), b1 = qm31_mul(corr, a1);
+        look_poly_wait();
+        const qm31 q = hn ? qm31_zero() : qm31_mul(ldq_r(t.look_coef[round & 1], k), l1);  // this round's polynomial at r is the next claim
+        look_sums_wait();
+        auto sums = [&](int at) { return qm31_add(ldq_r(t.look_sums, hn + 2 * at), ldq_r(t.look_sums, hn + 2 * at + 6)); };
+        const qm31 s0 = sums(0), s2 = sums(2), mid = qm31_sub(sums(1), qm31_add(s0, s2));
+        const qm31 lo = k == 0 ? s0 : k == 1 ? mid : k == 2 ? s2 : qm31_zero(), hi = k == 0 ? qm31_zero() : k == 1 ? s0 : k == 2 ? mid : s2;
+        const qm31 v = qm31_add(qm31_dot2(b0, lo, b1, hi), q), o = qm31_add(v, shfl_q(v, lane ^ 16));
+        if (lane < 16) stq_r(t.ahead, lane, o);
+    }
+}
+
+// The basis of a layer's last round, whose variable is the challenge that the layer before ended with: by a warp of its own, under the begin.
+__device__ __forceinline__ void solo_last_basis(TrSm& t, qm31* basis, qm31* inv, int nv) {
+    const int lane = threadIdx.x & 31;
+    basis_inverses(t.s.ood, t.s.prefix, inv, nv - 1, nv, lane, 32);
+    __syncwarp();
+    basis_rounds(t.s.ood, inv, basis, nv - 1, nv, lane, 32);
+    __syncwarp();
+    look_basis_set();
+}
+
+// The begin of a small layer by the twelve, while warp 0 hashes the claims and draws lambda: the layer into the work area (unless it is there, and its basis
+// with it), eq(., point), and the first round's sums, linear in lambda: `ahead` has the first polynomial at lambda. lo, hi: 32 entries each.
+static_assert(2 * (LOOK_TERMS / 32) * 2 <= 32, "first_sums");
+__device__ __forceinline__ void solo_begin(TrSm& t, const ChainLayer& L, qm31* basis, qm31* inv, unsigned char* num, unsigned char* den, void* eq, qm31* lo, qm31* hi,
+                                           bool ready) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = (warp >> 2) * 3 + (warp & 3) - 1, nv = L.nv, ny = nv - 1;
+    const bool product = L.kind[0] == ZKB_GKR_GRAND_PRODUCT;
+    const uint32_t nt = 1u << ny, blocks = (nt + 31) >> 5;
+    if (w >= LOOK_WARPS - 2) {
+        // eq = lo[low five bits] hi[the rest]; the first variable's share is 1 - y
+        const bool high = w == LOOK_WARPS - 1;
+        const int lo_bits = ny < 5 ? ny : 5, bits = high ? ny - lo_bits : lo_bits, first = high ? lo_bits : 0;
+        auto f = [&](int b) {
+            const qm31 y = ldq_r(t.s.ood, b < bits ? ny - first - b : 0);
+            return b >= bits ? qm31_one() : (lane >> b) & 1 ? y : one_minus(y);
+        };
+        const qm31 v = qm31_mul(qm31_mul(f(0), f(1)), qm31_mul(f(2), f(3)));
+        stq_r(high ? hi : lo, lane, qm31_mul(v, high ? one_minus(ldq_r(t.s.ood, 0)) : f(4)));
+    } else if (!ready) {
+        if (w < SOLO_BASIS_WARPS) {
+            basis_inverses(t.s.ood, t.s.prefix, inv, 0, nv - 1, 32 * w + lane, 32 * SOLO_BASIS_WARPS);
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * SOLO_BASIS_WARPS) : "memory");
+            basis_rounds(t.s.ood, inv, basis, 0, nv - 1, 32 * w + lane, 32 * SOLO_BASIS_WARPS);
+        } else {
+            solo_fetch(L, num, den, 32 * (w - SOLO_BASIS_WARPS) + lane, 32 * (LOOK_WARPS - 2 - SOLO_BASIS_WARPS));
+        }
+    }
+    look_fixed();
+    // 32 terms at one node a turn, its share without lambda (n0 d1 + n1 d0) or with it (d0 d1)
+    for (uint32_t job = w; job < 4 * blocks; job += LOOK_WARPS) {
+        const bool with = job & 1, node = job & 2;
+        const uint32_t i = 32 * (job >> 2) + lane;
+        qm31_sum x = qm31_sum_zero();
+        if (i < nt && !(with && product)) {
+            const qm31 e = qm31_mul(ldq_r(lo, i & 31), ldq_r(hi, i >> 5));
+            if (!with && !node) stq_r(eq, i, e);
+            auto at = [&](const void* p, uint32_t b) {
+                const qm31 v0 = ldq_r(p, 2 * i + b);
+                return node ? at_two(v0, ldq_r(p, 2 * (nt + i) + b)) : v0;
+            };
+            const qm31 d0 = at(den, 0), d1 = at(den, 1), e0 = qm31_mul(e, d0);
+            x.add_product(e0, with || product ? d1 : at(num, 1));
+            if (!with && !product) x.add_product(qm31_mul(e, d1), at(num, 0));
+        }
+        const qm31 s = warp_sum_q(x.value());
+        if (lane == 0) stq_r(t.first_sums, job, s);
+    }
+    __syncwarp();
+    if (w < LOOK_WARPS - 1) {
+        look_sums_set();
+        return;
+    }
+    // look_work's helper; lanes as there
+    if (nv == 1) look_basis_wait();
+    const int hn = lane >> 4, c = (lane >> 2) & 3, k = lane & 3;
+    const qm31 a = qm31_mul(ldq_r(basis, 12 + hn), ldq_r(basis, 8 * hn + c)), l1 = ldq_r(basis, 4 + c);
+    const qm31 claim = k < (product ? 1 : 2) && !hn ? ldq_r(t.s.claims[L.inst[0]], k) : qm31_zero();
+    look_sums_wait();
+    qm31 s = qm31_zero();
+    for (uint32_t p = 0; p < blocks; p++) s = qm31_add(s, ldq_r(t.first_sums, 4 * p + 2 * hn + (k & 1)));
+    const qm31 v = qm31_dot2(k < 2 ? s : qm31_zero(), a, claim, l1), o = qm31_add(v, shfl_q(v, lane ^ 16));
+    if (lane < 16) stq_r(t.ahead, lane, o);
+}
+
 struct ResInit { uint32_t digest[8], n_draws; int use; };  // use: the proof's first launch starts from this channel, not from *st
 __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st, const ChainLayer* __restrict__ layers, int n_layers, ResInit init) {
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -749,8 +1110,8 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
     TrSm& tr = sm.tr;
     qm31* const basis = sm.basis;
     __shared__ ChainLayer layer_buf[2];  // the layer at hand and the next one
-    __shared__ qm31 inv[RES_MAX_VARS * 5];
-    __shared__ qm31 red[RES_MAX_INST][32];  // per oracle: a warp's two sums (warps x 2), or the units of a small pass
+    __shared__ alignas(16) qm31 inv[RES_MAX_VARS * 5];
+    __shared__ alignas(16) qm31 red[RES_MAX_INST][32];  // per oracle: a warp's two sums (warps x 2), or the units of a small pass
     void* const eq = dyn;
     unsigned char* const work = dyn + CHAIN_EQ_BYTES;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -780,14 +1141,41 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
         const int K = L.n_oracles, nv = L.nv, ny = nv - 1;
         if (tid == 0 && L.round_start) tr.pcur = tr.s.prefix_next[L.round_start];
         if (tid < K) tr.n_vars[tid] = L.n_vars[tid];
+        const bool one = K == 1 && nv > 0;  // the first layer, of no variables, has the instances that start
+        if (is_solo(L)) {
+            unsigned char *const den = work, *const num = work + 2 * SOLO_BYTES;
+            if (warp == 0) {
+                d = one_lead(tr, layer_buf, d, n_layers, LEAD_BEGIN | LEAD_ROUNDS, 0, nullptr, 0, num, den);
+            } else {
+                bool ready = false;
+                do {
+                    const ChainLayer& S = layer_buf[d & 1];
+                    const uint32_t here = (d & 1) * SOLO_BYTES, there = SOLO_BYTES - here;
+                    if (warp & 3) {
+                        solo_begin(tr, S, basis, inv, num + here, den + here, eq, red[0], red[1], ready);
+                        look_work(tr, basis, inv, S.nv, 0, true, S.kind[0] == ZKB_GKR_GRAND_PRODUCT, num + here, den + here, eq, S.polys, d + 1 < n_layers ? layers + d + 1 : nullptr,
+                                  &layer_buf[(d + 1) & 1], num + there, den + there);
+                    } else if (warp == 4) {
+                        solo_last_basis(tr, basis, inv, S.nv);
+                    }
+                    solo_done();
+                    ready = true;
+                } while (++d < n_layers && is_solo(layer_buf[d & 1]));
+            }
+            d--;
+            continue;
+        }
         if (warp == 0) {
-            if (L.flags & CHAIN_BEGIN) tr_begin(tr, L);
+            if (L.flags & CHAIN_BEGIN) {
+                if (one) one_lead(tr, layer_buf, d, n_layers, LEAD_BEGIN, 0, nullptr, 0, nullptr, nullptr);
+                else tr_begin(tr, L);
+            }
         } else if (tid < 32 + BASIS_THREADS) {
             const int th = tid - 32;
             if (L.flags & CHAIN_BEGIN) {
-                basis_inverses(tr, inv, nv, th, BASIS_THREADS);
+                basis_inverses(tr.s.ood, tr.s.prefix, inv, 0, nv, th, BASIS_THREADS);
                 basis_bar();
-                basis_rounds(tr, inv, basis, nv, th, BASIS_THREADS);
+                basis_rounds(tr.s.ood, inv, basis, 0, nv, th, BASIS_THREADS);
                 basis_bar();
                 if (!(L.flags & CHAIN_ROUNDS))  // the rounds on launches of their own come next and read it from memory
                     for (int i = th; i < BASIS_Q * nv; i += BASIS_THREADS) L.basis[i] = basis[i];
@@ -812,10 +1200,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
         auto den_work = [&](int k) { return L.work_global ? reinterpret_cast<void*>(L.den_work[k]) : static_cast<void*>(work + L.den_work[k]); };
         auto num_work = [&](int k) { return L.work_global ? reinterpret_cast<void*>(L.num_work[k]) : static_cast<void*>(work + L.num_work[k]); };
         if (L.flags & CHAIN_ROUNDS) {
-            // one oracle: where its layer is, and whether small folds (below) have begun
-            struct { const void *num, *den; int kind; bool folds; } one = {L.num[0], L.den[0], L.kind[0], false};
+            // one oracle: where its layer is
+            struct { const void *num, *den; int kind; } at = {L.num[0], L.den[0], L.kind[0]};
             const bool one_product = L.kind[0] == ZKB_GKR_GRAND_PRODUCT;
-            const qm31 half_lambda = qm31_mul_m31(tr.s.lambda, 1u << 30);
             for (int round = L.round_start; round <= nv; round++) {
                 // Pass of this round: the oracles that were active before are fixed at the last challenge; those and the ones that
                 // enter now give their sums (none after the last round). The second warp brings claims and corrections up to date
@@ -824,43 +1211,46 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
                 const qm31 r = tr.s.challenge, lambda = tr.s.lambda;
                 const bool sums = round < nv;
                 const uint32_t nt = sums ? 1u << (n_rem - 1) : 0u;
-                const bool small = nt <= CHAIN_SMALL;
+                const bool small = nt <= (K == 1 ? LOOK_TERMS : CHAIN_SMALL);
                 if (warp == 1) {
                     if (round > L.round_start) tr_update(tr, basis + BASIS_Q * (round - 1), 16u * BASIS_Q * (round - 1), K, n_rem + 1, round - 1, true);
                     else if (sums) tr_prepare(tr, basis + BASIS_Q * round, 16u * BASIS_Q * round, K, n_rem);
                 }
-                if (K == 1 && small) {
-                    if (warp < 2) {
-                    } else if (one.folds && n_rem) {  // later folds: an entry of either column per thread
-                        const uint32_t e_out = 2u << n_rem, log_e = n_rem + 1;
-                        for (uint32_t i = tid - 64u; i < (one_product ? 1u : 2u) * e_out; i += RES_THREADS - 64u) {
-                            unsigned char* const p = work + (i >> log_e ? L.num_work[0] : 0u);
-                            const uint32_t e = i & (e_out - 1);
-                            stq_r(p, e, fold_q(r, ldq_r(p, e), ldq_r(p, e + e_out)));
-                        }
-                    } else if (tr.n_vars[0] > n_rem) {
-                        // the first small fold, which changes n for m = n + (lambda / 2) d (a term is then m0 d1 + m1 d0), and the
-                        // last one, which leaves the mask: n again
-                        const uint32_t e_out = 2u << n_rem;
-                        for (uint32_t e = tid - 64u; e < e_out; e += RES_THREADS - 64u) {
-                            const qm31 d = fold_q(r, ldq_r(one.den, e), ldq_r(one.den, e + e_out));
-                            qm31 n = qm31_one();
-                            if (one.kind == ZKB_GKR_LOGUP_MULTIPLICITIES && !one.folds) {
-                                const uint32_t* m = static_cast<const uint32_t*>(one.num);
-                                n = fold_m(r, m[e], m[e + e_out]);
-                            } else if (one.kind == ZKB_GKR_LOGUP_GENERIC || one.folds) {
-                                if (!one_product) n = fold_q(r, ldq_r(one.num, e), ldq_r(one.num, e + e_out));
+                if (K == 1 && small && sums) {
+                    // The layer goes to the work area, fixed at the last challenge if it has had one, with n changed for m = n + (lambda / 2) d: a
+                    // term is then m0 d1 + m1 d0.
+                    const bool fold = round > 0;
+                    const qm31 half_lambda = qm31_mul_m31(lambda, 1u << 30);
+                    unsigned char* const num_to = work + L.num_work[0];
+                    if (warp >= 2) {
+                        const uint32_t n_out = 2u << n_rem;
+                        for (uint32_t e = tid - 64u; e < n_out; e += RES_THREADS - 64u) {
+                            qm31 d = ldq_r(at.den, e), n = qm31_one();
+                            if (fold) d = fold_q(r, d, ldq_r(at.den, e + n_out));
+                            if (at.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) {
+                                const uint32_t* m = static_cast<const uint32_t*>(at.num);
+                                n = fold ? fold_m(r, m[e], m[e + n_out]) : qm31_from_m31(m[e]);
+                            } else if (at.kind == ZKB_GKR_LOGUP_GENERIC) {
+                                n = ldq_r(at.num, e);
+                                if (fold) n = fold_q(r, n, ldq_r(at.num, e + n_out));
                             }
                             stq_r(work, e, d);
-                            if (!one_product) {
-                                const qm31 hd = qm31_mul(half_lambda, d);
-                                stq_r(work + L.num_work[0], e, !n_rem ? (one.folds ? qm31_sub(n, hd) : n) : qm31_add(n, hd));
-                            }
+                            if (!one_product) stq_r(num_to, e, qm31_add(n, qm31_mul(half_lambda, d)));
                         }
                     }
-                    if (tr.n_vars[0] > n_rem) { one.den = work; one.num = work + L.num_work[0]; one.folds = true; }
+                    __syncthreads();
+                    // by the warps after the first two, whose instruction caches hold the transcript
+                    const uint32_t units = 4 * ((nt + 31) / 32);
+                    for (uint32_t w = (warp + RES_WARPS - 2) & (RES_WARPS - 1); w < units; w += RES_WARPS) {
+                        const qm31 v = small_unit_m(one_product, num_to, work, nt, 32 * (w >> 2) + lane, w & 1, (w >> 1) & 1, eq);
+                        if (lane == 0) red[0][w] = v;
+                    }
+                    __syncthreads();
+                    if (warp == 0) one_lead(tr, layer_buf, d, n_layers, LEAD_ROUNDS | LEAD_SUMS, round, red[0], units, num_to, work);
+                    else if (warp & 3) look_work(tr, basis, inv, nv, round, false, one_product, num_to, work, eq, L.polys, nullptr, nullptr, nullptr, nullptr);
+                    break;
                 }
-                for (int k = small && (warp < 2 || K == 1) ? K : 0; k < K; k++) {
+                for (int k = small && warp < 2 ? K : 0; k < K; k++) {
                     const uint32_t vars = tr.n_vars[k];
                     const bool fold = vars > n_rem, fresh = round == L.round_start || vars == n_rem + 1;  // fresh: nothing folded here yet
                     if (!fold && (vars < n_rem || small)) continue;
@@ -898,9 +1288,9 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
                     s2 = warp_sum_q(s2);
                     if (lane == 0) { red[k][2 * warp] = s0; red[k][2 * warp + 1] = s2; }
                     if (K == 1 && fold) {
-                        one.den = den_w;
-                        one.num = num_w;
-                        if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) one.kind = ZKB_GKR_LOGUP_GENERIC;
+                        at.den = den_w;
+                        at.num = num_w;
+                        if (kind == ZKB_GKR_LOGUP_MULTIPLICITIES) at.kind = ZKB_GKR_LOGUP_GENERIC;
                     }
                 }
                 __syncthreads();
@@ -909,28 +1299,19 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
                 if (small) {
                     // by the warps after the first two, whose instruction caches hold the transcript
                     units = 4 * ((nt + 31) / 32);
-                    if (K == 1) {
-                        for (uint32_t w = (warp + RES_WARPS - 2) & (RES_WARPS - 1); w < units; w += RES_WARPS) {
-                            const uint32_t i = 32 * (w >> 2) + lane;
-                            const qm31 v = one.folds ? small_unit_m(one_product, one.num, one.den, nt, i, w & 1, (w >> 1) & 1, eq)
-                                                     : small_unit(one.kind, one.num, one.den, nt, i, w & 1, (w >> 1) & 1, lambda, eq);
-                            if (lane == 0) red[0][w] = v;
-                        }
-                    } else {
-                        for (uint32_t u = (warp + RES_WARPS - 2) & (RES_WARPS - 1); u < units * K; u += RES_WARPS) {
-                            const int k = u / units, w = u % units;
-                            if (tr.n_vars[k] < n_rem) continue;
-                            const bool folded = tr.n_vars[k] > n_rem;
-                            const void* den = folded ? den_work(k) : static_cast<const void*>(L.den[k]);
-                            const void* num = folded ? num_work(k) : static_cast<const void*>(L.num[k]);
-                            const int kind = folded && L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES ? (int)ZKB_GKR_LOGUP_GENERIC : L.kind[k];
-                            const qm31 v = small_unit(kind, num, den, nt, 32 * (w >> 2) + lane, w & 1, (w >> 1) & 1, lambda, eq);
-                            if (lane == 0) red[k][w] = v;
-                        }
+                    for (uint32_t u = (warp + RES_WARPS - 2) & (RES_WARPS - 1); u < units * K; u += RES_WARPS) {
+                        const int k = u / units, w = u % units;
+                        if (tr.n_vars[k] < n_rem) continue;
+                        const bool folded = tr.n_vars[k] > n_rem;
+                        const void* den = folded ? den_work(k) : static_cast<const void*>(L.den[k]);
+                        const void* num = folded ? num_work(k) : static_cast<const void*>(L.num[k]);
+                        const int kind = folded && L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES ? (int)ZKB_GKR_LOGUP_GENERIC : L.kind[k];
+                        const qm31 v = small_unit(kind, num, den, nt, 32 * (w >> 2) + lane, w & 1, (w >> 1) & 1, lambda, eq);
+                        if (lane == 0) red[k][w] = v;
                     }
                     __syncthreads();
                 }
-                if (warp == 0 && (K > 1 || units > 4)) {  // one oracle with four units: tr_round adds them itself
+                if (warp == 0) {
                     for (int k = 0; k < K; k++) {
                         if (tr.n_vars[k] < n_rem) continue;
                         const qm31 v = (uint32_t)lane < units ? red[k][lane] : qm31_zero();
@@ -939,11 +1320,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1) res_chain_kernel(ResState* st,
                     }
                     __syncwarp();
                 }
-                if (warp == 0) tr_round(tr, basis + BASIS_Q * round, K, n_rem, round, L.polys + (size_t)POLY_WORDS * round, K == 1 && units == 4 ? red[0] : nullptr);
+                if (warp == 0) tr_round(tr, basis + BASIS_Q * round, K, n_rem, round, L.polys + (size_t)POLY_WORDS * round);
                 __syncthreads();
             }
         }
-        if ((L.flags & CHAIN_END) && warp == 0) {
+        if ((L.flags & CHAIN_END) && warp == 0 && !one) {
             tr_end(tr, L, [&](int k) { return L.n_vars[k] && L.kind[k] == ZKB_GKR_LOGUP_MULTIPLICITIES ? (int)ZKB_GKR_LOGUP_GENERIC : L.kind[k]; },
                    [&](int k) { return L.n_vars[k] ? num_work(k) : static_cast<const void*>(L.num[k]); },
                    [&](int k) { return L.n_vars[k] ? den_work(k) : static_cast<const void*>(L.den[k]); });
@@ -1106,6 +1487,7 @@ int gkr_prove_resident(zkb_ctx* ctx, std::vector<Layer> input_layers, uint32_t d
             L.den_work[k] = smem; smem += bytes;
             if (L.kind[k] != ZKB_GKR_GRAND_PRODUCT) { L.num_work[k] = smem; smem += bytes; }
         }
+        if (K == 1 && L.kind[0] != ZKB_GKR_GRAND_PRODUCT) L.num_work[0] = CHAIN_WORK_BYTES / 2;  // (a small layer goes there whole)
         L.work_global = smem > CHAIN_WORK_BYTES ? 1 : 0;
         if (L.work_global)  // several tall oracles at once: in place for the towers' layers, the folded copies for the inputs
             for (int k = 0; k < K; k++) {
