@@ -191,6 +191,30 @@ __device__ __forceinline__ void chan_copy_digest(ChanSm& s) {
     if (lane < 8) s.msg[16 + lane] = s.msg[lane];
 }
 
+// A product by y, a coordinate a lane (its two low bits): four multiply-adds and a reduction, where a lane that makes all four takes sixteen and four.
+struct slice_by {
+    uint32_t m[4];
+    __device__ __forceinline__ slice_by(qm31 y) {
+        const int k = threadIdx.x & 3;
+        const uint32_t e0 = m31_sub(m31_dbl(y.c[2]), y.c[3]), e1 = m31_add(y.c[2], m31_dbl(y.c[3]));
+        m[0] = k == 0 ? y.c[0] : k == 1 ? y.c[1] : k == 2 ? y.c[2] : y.c[3];
+        m[1] = k == 0 ? P - y.c[1] : k == 1 ? y.c[0] : k == 2 ? P - y.c[3] : y.c[2];
+        m[2] = k == 0 ? e0 : k == 1 ? e1 : k == 2 ? y.c[0] : y.c[1];
+        m[3] = k == 0 ? P - e1 : k == 1 ? e0 : k == 2 ? P - y.c[1] : y.c[0];
+    }
+    // coordinate k of x y, and the word z added (qm31_add_products has the bound)
+    __device__ __forceinline__ uint32_t mul_add(qm31 x, uint32_t z) const {
+        return m31_reduce64(z + (uint64_t)x.c[0] * m[0] + (uint64_t)x.c[1] * m[1] + (uint64_t)x.c[2] * m[2] + (uint64_t)x.c[3] * m[3]);
+    }
+};
+// The value whose coordinates are in lanes first ... first + 3.
+__device__ __forceinline__ qm31 gather_q(uint32_t v, int first) {
+    qm31 r;
+#pragma unroll
+    for (int c = 0; c < 4; c++) r.c[c] = __shfl_sync(0xffffffffu, v, first + c);
+    return r;
+}
+
 // Sum mod p of one word over the warp, the same value in every lane: two integer warp reductions of 16-bit halves.
 __device__ __forceinline__ uint32_t warp_sum_m31(uint32_t v) {
     const uint32_t lo = __reduce_add_sync(0xffffffffu, v & 0xffffu), hi = __reduce_add_sync(0xffffffffu, v >> 16);

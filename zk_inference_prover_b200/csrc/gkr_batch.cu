@@ -159,13 +159,25 @@ struct alignas(16) GkrStepState {
     uint32_t digest[8], n_draws, pad[3];
     qm31 challenge, claim;                            // claim: sum of alpha^k claim_k over the active oracles
     qm31 corr[GKR_GROUPS];
-    unsigned long long acc[2][GKR_GROUPS][8];         // the groups' sums of the round at hand, and zeros for the next
 };
 static_assert(sizeof(GkrStepState) % 16 == 0, "GkrStepState layout");
 
-struct GkrStepSm {
+// The groups' sums of the round at hand, and zeros for the next: [2][groups][24] 64-bit words. Of a round whose challenge is known its two sums (t =
+// 0, t = 2); of one that is worked out ahead (look_pass) three pairs.
+constexpr int ACC_WORDS = 24;
+struct GkrAcc {
+    unsigned long long* words;
+    int groups;
+    __device__ __forceinline__ unsigned long long* at(int round, int group) const { return words + (size_t)ACC_WORDS * ((round & 1) * groups + group); }
+};
+
+struct alignas(16) GkrStepSm {
     ChanSm ch;
     qm31 coef[4], r;
+    // rounds worked out ahead: the next polynomial (but for what the waiting oracles add) as cubics in the challenge, low first; the groups' sums with
+    // their corrections, of two nodes at three points; the sums of the oracles that enter next; of this round and the last the polynomial,
+    // with and without the waiting, and the challenge
+    qm31 ahead[16], look_sums[6], look_enter[2], look_coef[2][4], look_sent[2][4], look_r[2];
 };
 
 __device__ __noinline__ qm31 qmul(qm31 a, qm31 b) { return qm31_mul(a, b); }
@@ -185,19 +197,22 @@ __device__ __forceinline__ qm31 warp_sum_m(qm31 v) {
     return r;
 }
 
-// By one warp; sm.ch's schedule is made and its message holds the digest. st: the state, wherever it is (its accumulators are not
-// touched); s0, s2: lane g's group's sums; out: the round's record. drawn() is called as soon as the challenge is in sm.r, before
-// what the next step needs of it is worked out.
-template <class Drawn>
-__device__ __forceinline__ void batch_step(GkrStepSm& sm, GkrStepState& st, const GkrStepConst& rc, qm31 s0, qm31 s2, uint32_t* out, Drawn drawn) {
+// Coefficient (lane & 3) of the round's polynomial but for what the waiting oracles add. By one warp; s0, s2: lane g's group's sums.
+__device__ __forceinline__ qm31 batch_coefficients(const GkrStepState& st, const GkrStepConst& rc, qm31 corr, qm31 s0, qm31 s2) {
     const int lane = threadIdx.x & 31, c4 = lane & 3;
-    const qm31 corr = st.corr[lane];
     const qm31_pair w = product_pair(s0, corr, s2, corr);
     const qm31 S0 = warp_sum_m(w.a), S2 = warp_sum_m(w.b);
     // coefficient c4: lanes 0-3 of the first sum, 4-7 of the second, 8-11 of the claim
     const int q = lane >> 2;
     const qm31 p = qmul(q == 0 ? S0 : q == 1 ? S2 : st.claim, q == 0 ? rc.A[c4] : q == 1 ? rc.B[c4] : rc.L1[c4]);
-    const qm31 act = qm31_add(qm31_add(p, shflb(p, (lane + 4) & 31)), shflb(p, (lane + 8) & 31));
+    return qm31_add(qm31_add(p, shflb(p, (lane + 4) & 31)), shflb(p, (lane + 8) & 31));
+}
+// By one warp; sm.ch's schedule is made and its message holds the digest. st: the state, wherever it is; s0, s2: lane g's group's sums; out: the
+// round's record. drawn() is called as soon as the challenge is in sm.r, before what the next step needs of it is worked out.
+template <class Drawn>
+__device__ __forceinline__ void batch_step(GkrStepSm& sm, GkrStepState& st, const GkrStepConst& rc, qm31 s0, qm31 s2, uint32_t* out, Drawn drawn) {
+    const int lane = threadIdx.x & 31;
+    const qm31 corr = st.corr[lane], act = batch_coefficients(st, rc, corr, s0, s2);
     const qm31 c = lane == 0 ? qm31_add(act, rc.waiting) : act;
     const int len = 32 - __clz(__ballot_sync(0xffffffffu, lane < 4 && !qm31_is_zero(c)));
     if (lane < 4) {
@@ -276,7 +291,7 @@ __device__ __forceinline__ void item_sums_of(const GkrBatchItem& it, size_t firs
 // The terms of `g` neighbouring lanes (a power of two up to 32) are one item's: they are added up, taken times the item's power of
 // alpha and added to its group's sums in shared memory, as 16-bit halves (32-bit adds, no carries to fold; 2^16 terms fit). By
 // whole warps; adds: the lane belongs to an item.
-__device__ __forceinline__ void add_to_group(uint32_t (*acc)[16], int g, bool adds, uint32_t oracle, uint32_t group, const uint32_t* __restrict__ alpha_pow, qm31 s0, qm31 s2) {
+__device__ __forceinline__ void add_to_group(uint32_t (*acc)[2 * ACC_WORDS], int g, bool adds, uint32_t oracle, uint32_t group, const uint32_t* __restrict__ alpha_pow, qm31 s0, qm31 s2) {
     const int lane = threadIdx.x & 31, sub = lane & (g - 1);
     const qm31 a = adds ? ldqb(alpha_pow, oracle) : qm31_zero();
     for (int off = g >> 1; off > 0; off >>= 1) {
@@ -307,7 +322,7 @@ __device__ __forceinline__ void add_to_group(uint32_t (*acc)[16], int g, bool ad
 
 // ---- a layer in one launch
 //
-// A cooperative launch of up to two CTAs an SM runs all tables of a layer. Measured with a launch per round: of the 26,500 cycles (14 us)
+// A cooperative launch of up to a CTA an SM runs all tables of a layer. Measured with a launch per round: of the 26,500 cycles (14 us)
 // that every round of a small batch took, whatever its size, half were the fetching of code that the SM at hand had not run
 // yet (the pass 14,500 cycles cold and 6,300 warm, the transcript step 12,000 and 8,000) and the rest of the gap the launch
 // itself; a round in one CTA took 9.3 us warm. Here the code stays warm in every SM, CTA 0 keeps the transcript in shared memory and
@@ -319,14 +334,17 @@ __device__ __forceinline__ void add_to_group(uint32_t (*acc)[16], int g, bool ad
 //
 // The waits end: every CTA is resident (the launch is refused otherwise), a CTA waits only for what the others do before they wait
 // themselves, and after SPIN_LIMIT polls (about a second) it gives up and leaves; the host then sees no layer number and reports it.
-constexpr int GKR_THREADS = 256;
+constexpr int GKR_THREADS_LOG = 9, GKR_THREADS = 1 << GKR_THREADS_LOG;
+constexpr int LOOK_MIN_LOG = 7;                  // the fewest threads (log2) that a CTA is given work for
 constexpr uint32_t SPIN_LIMIT = 1u << 21;
+
+constexpr int EQ_TABLES = 3;                     // of five bits of a term's index each
 
 struct alignas(16) GkrTable {
     uint32_t first, n_items;  // its items
     int terms_log;            // log2 of the terms an item has
-    int form;                 // 0: a thread per term, 1: four lanes per term, 2: masks, two threads an item
-    int run_log;              // form 0, items of 2^8 terms and more: a chunk is 2^run_log terms a thread
+    int form;                 // 0: a thread per term, 1: four lanes per term, 2: masks, two threads an item; 3: a pass of a round ahead, 4: the last of them
+    int run_log;              // form 0, items of 2^GKR_THREADS_LOG terms and more: a chunk is 2^run_log terms a thread; the other forms: a chunk is 2^run_log threads
     uint32_t chunks, ctas;    // pieces of work, CTAs that take them in turn
     uint32_t later;           // the most CTAs a later table has
 };
@@ -335,11 +353,13 @@ static_assert(sizeof(GkrTable) == 32, "GkrTable layout");
 struct alignas(16) GkrSync {  // zero at launch
     uint32_t count[GKR_LAYER_MAX_ROUNDS + 1];   // CTAs done with the table
     uint32_t slot[GKR_LAYER_MAX_ROUNDS + 1][4];  // the challenge the table folds with; the top bit of a word: it is there
+    uint32_t look_count[GKR_LAYER_MAX_ROUNDS + 1];  // CTAs done with a pass of a round ahead
 };
+static_assert(sizeof(GkrSync) % 16 == 0, "GkrSync layout");
 
 
 // The sums of `v` over the warp's lanes with even and odd `which` go to the group's accumulator; lanes that do not add hold `adds` false.
-__device__ __forceinline__ void add_quad_terms(uint32_t (*acc)[16], bool adds, int which, uint32_t group, qm31 v) {
+__device__ __forceinline__ void add_quad_terms(uint32_t (*acc)[2 * ACC_WORDS], bool adds, int which, uint32_t group, qm31 v) {
     const int lane = threadIdx.x & 31;
     const unsigned who = __ballot_sync(0xffffffffu, adds);
     if (!who) return;
@@ -367,32 +387,245 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
     return v;
 }
 
-// Tables [first, end) of the layer. rc: null where the transcript's steps are launches of their own (gkr_batch_step_kernel); no CTA then
+// ---- the small rounds, a round ahead of the transcript
+//
+// A round is a chain: the challenge goes out, the CTAs fold and sum, their sums come back (together some 9,000 cycles however small the round), the
+// transcript's three compressions follow (4,400). A layer fixed at r is linear in r and a term is a product of two entries, so a group's sums of the next
+// round are quadratic in this round's challenge, and its correction is linear. From round look_from on, then, the CTAs work on the round after the one that is being
+// hashed: they fold with the challenge before, and bring back the next round's sums at r = 0, at r = 1 and their leading coefficient; warps of CTA 0 make
+// of those the next polynomial as cubics in the challenge to come. When the challenge is there the next polynomial is two products away. The two chains
+// run beside each other: 16,000 cycles a round before, 9,500 now (34 instances of 2^13).
+//
+// CTA 0 keeps the transcript and takes no pieces: warp 0 hashes, six warps take a node and point each, one makes the polynomial of them. Those are on other
+// schedulers than warp 0, and the CTA has its SM to itself (a CTA an SM: with two of half the size the hash beside a worker took 5,700 cycles instead of 4,200).
+constexpr int LOOK_SUM_WARPS = 6, LOOK_LAST_WARP = 9;
+static_assert(GKR_THREADS / 32 > LOOK_LAST_WARP, "the warps of CTA 0");
+__device__ __forceinline__ int look_value(int warp) { return warp == LOOK_LAST_WARP ? LOOK_SUM_WARPS : warp < 8 && (warp & 3) ? warp - 1 - (warp >> 2) : -1; }  // 1-3, 5-7
+
+// What a pass does for an item: the layer is there / fix it at the challenge first / it enters in the next round (nothing but its sums then).
+enum : uint32_t { LOOK_AS_IS = 0, LOOK_FIX = 1, LOOK_ENTERS = 2 };
+
+__device__ __forceinline__ bool wait_count(const uint32_t* count, uint32_t want) {
+    uint32_t n = ld_acquire(count);
+    for (uint32_t spin = 0; n != want && spin < SPIN_LIMIT; spin++) n = ld_acquire(count);
+    return n == want;
+}
+
+// One entry of a layer: its denominator and numerator (one where the kind has none, zero for a grand product).
+struct entry { qm31 d, n; };
+__device__ __forceinline__ entry load_entry(const GkrBatchItem& it, size_t e) {
+    entry v{ldqb(it.den, e), qm31_zero()};
+    if (it.kind == ZKB_GKR_LOGUP_SINGLES) v.n = qm31_one();
+    if (it.kind == ZKB_GKR_LOGUP_GENERIC) v.n = ldqb(it.num, e);
+    if (it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) v.n = qm31_from_m31(it.num[e]);
+    return v;
+}
+// The entry fixed at r, also where the folded layer goes. half: entries of that.
+__device__ __forceinline__ entry fix_entry(const GkrBatchItem& it, size_t e, size_t half, qm31 r) {
+    const entry v0 = load_entry(it, e), v1 = load_entry(it, e + half);
+    const qm31_pair p = product_pair(r, qm31_sub(v1.d, v0.d), r, qm31_sub(v1.n, v0.n));
+    const entry v{qm31_add(v0.d, p.a), qm31_add(v0.n, p.b)};
+    stqb(it.den_out, e, v.d);
+    if (it.kind == ZKB_GKR_LOGUP_GENERIC || it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) stqb(it.num_out, e, v.n);
+    return v;
+}
+
+// Eight lanes a term of the next round, one for each of its entries: bit 2 the variable this round fixes, bit 1 the next round's, bit 0 the pair. A term is
+// n0 d1 + n1 d0 + lambda d0 d1 = m0 d1 + m1 d0 with m = n + k d, k = lambda / 2 (a grand product's d0 d1 with n = 0, k = 1 / 2). Lanes 0 and 2 end with the term at r
+// = 0, 4 and 6 with it at r = 1, 5 and 7 with its leading coefficient. ea: eq times the oracle's power of alpha.
+__device__ __forceinline__ void look_term(uint32_t (*acc)[2 * ACC_WORDS], const GkrBatchItem& it, bool live, uint32_t term, int terms_log, qm31 r, qm31 half_lambda, qm31 ea) {
+    const int lane = threadIdx.x & 31, q = lane & 7;
+    const size_t nt = (size_t)1 << terms_log, e = (size_t)(q >> 2) * 4 * nt + (size_t)((q >> 1) & 1) * 2 * nt + 2 * (size_t)term + (q & 1);
+    live = live && !(it.mode == LOOK_ENTERS && (q & 4));
+    entry v{qm31_zero(), qm31_zero()};
+    if (live) v = it.mode == LOOK_FIX ? fix_entry(it, e, 8 * nt, r) : load_entry(it, e);
+    qm31 x = v.d, m = qm31_add(v.n, qmul(it.kind == ZKB_GKR_GRAND_PRODUCT ? qm31_from_m31(1u << 30) : half_lambda, x));
+    const qm31 x0 = shflb(x, lane & ~2), m0 = shflb(m, lane & ~2);
+    if (q & 2) { x = qm31_sub(qm31_dbl(x), x0); m = qm31_sub(qm31_dbl(m), m0); }
+    const qm31 xp = shflb(x, lane ^ 1);
+    const qm31 xp0 = shflb(xp, lane & ~4), mm0 = shflb(m, lane & ~4);
+    const qm31_pair p = product_pair(m, xp, qm31_sub(m, mm0), qm31_sub(xp, xp0));
+    const qm31 a = qm31_add(p.a, shflb(p.a, lane ^ 1)), b = qm31_add(p.b, shflb(p.b, lane ^ 1));
+    const bool adds = live && (it.mode == LOOK_ENTERS ? !(q & 1) : q != 1 && q != 3);
+    qm31 t = qmul((q & 1) ? b : a, ea);
+    // value 2 point + node
+    const uint32_t value = 2 * ((q >> 2) + (q & 1)) + ((q >> 1) & 1), group = (uint32_t)(it.slot >> 32);
+    const unsigned who = __ballot_sync(0xffffffffu, adds);
+    if (!who) return;
+    const uint32_t g0 = __shfl_sync(0xffffffffu, group, __ffs(who) - 1);
+    bool mine = adds;
+    if (__all_sync(0xffffffffu, !adds || group == g0)) {  // one group in the warp: the same value's lanes first
+        if (!adds) t = qm31_zero();
+        t = qm31_add(t, shflb(t, lane ^ 8));
+        t = qm31_add(t, shflb(t, lane ^ 16));
+        mine = lane < 8 && (who & (0x01010101u << lane)) != 0u;
+    }
+    if (mine) {
+        uint32_t* const at = &acc[adds ? group : g0][8 * value];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            atomicAdd(at + 2 * c, t.c[c] & 0xffffu);
+            atomicAdd(at + 2 * c + 1, t.c[c] >> 16);
+        }
+    }
+}
+
+// Warp 0 of CTA 0: the rounds from `from` on. act0: coefficient (lane & 3) of the first one's polynomial. `met` is the meeting with the other warps
+// once a round: the challenge is there, and so is `ahead`.
+__device__ __forceinline__ void look_met() { asm volatile("bar.sync 1, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 2)) : "memory"); }
+__device__ __noinline__ void look_lead(GkrStepSm& sm, const GkrStepConst* consts, int from, int n_rounds, qm31 act0) {
+    const int lane = threadIdx.x & 31, c4 = lane & 3;
+    const QuadWords words(sm.ch.msg, sm.ch.sched);
+    const QuadConst qc;
+    const qm31 mine = shflb(act0, (lane >> 2) & 3);
+    uint32_t act = c4 == 0 ? mine.c[0] : c4 == 1 ? mine.c[1] : c4 == 2 ? mine.c[2] : mine.c[3];  // lane = 4 k + coordinate: coefficient k
+    qm31 r = qm31_zero();
+    for (int round = from;; round++) {
+        if (round > from) {
+            // (d3 r + d2) r^2 + (d1 r + d0): the low half in lanes 0-15, the high one in 16-31
+            const int at = (lane & 12) + (lane >> 4) * 2;
+            const qm31 d1 = ldqb(reinterpret_cast<const uint32_t*>(sm.ahead), at + 1);
+            const uint32_t d0 = sm.ahead[at].c[c4];
+            const slice_by by(r);
+            const uint32_t m = by.mul_add(d1, d0), r2 = by.mul_add(r, 0u);
+            act = slice_by(gather_q(r2, 0)).mul_add(gather_q(m, 16 + (lane & 12)), m);
+        }
+        const uint32_t c = lane < 4 ? m31_add(act, consts[round].waiting.c[lane]) : act;
+        if (lane < 16) sm.ch.msg[8 + lane] = c;
+        const unsigned nonzero = __ballot_sync(0xffffffffu, lane < 16 && c != 0u);
+        if (!(nonzero & 0xff00u)) {  // two coefficients or fewer
+            __syncwarp();
+            chan_copy_digest(sm.ch);
+            if (lane < 8) sm.ch.msg[24 + lane] = c;
+        }
+        __syncwarp();
+        const uint32_t v = chan_round(
+            sm.ch, words, qc, (nonzero & 0xff00u) != 0u, 0u, [&] { return 32u + 16u * (uint32_t)((35 - __clz(nonzero)) >> 2); },
+            [&] {
+                if (lane < 16) {
+                    sm.look_coef[round & 1][lane >> 2].c[c4] = act;
+                    sm.look_sent[round & 1][lane >> 2].c[c4] = c;
+                }
+                __syncwarp();
+                if (round + 1 < n_rounds) asm volatile("bar.arrive 3, 64;" ::: "memory");
+            });
+        if (lane < 4) sm.look_r[round & 1].c[lane] = v;
+        r = gather_q(v, 0);
+        __syncwarp();
+        look_met();
+        if (round + 1 == n_rounds) return;
+    }
+}
+// The warps of CTA 0 with a look_value. Returns whether a wait has run out.
+__device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* consts, const GkrTable* looks, const GkrStepState& s, const GkrAcc acc, GkrSync* sync, int from,
+                                             int n_rounds, uint32_t* records) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (lane >> 2) & 3, k = lane & 3, hn = lane >> 4;
+    const bool last_warp = warp == LOOK_LAST_WARP;
+    const int value = look_value(warp), node = value & 1;
+    qm31 corr = s.corr[lane];  // group `lane`'s
+    bool gave_up = false;
+    auto record = [&](int round) {  // by warp 2
+        const uint32_t* const sent = sm.look_sent[round & 1][0].c;
+        uint32_t* const out = records + GKR_LAYER_OUT_WORDS * (size_t)round;
+        const uint32_t w = lane < 16 ? sent[lane] : 0u;
+        const unsigned nonzero = __ballot_sync(0xffffffffu, w != 0u);
+        if (lane < 16) out[lane] = w;
+        if (lane == 16) out[16] = (uint32_t)((35 - __clz(nonzero)) >> 2);
+        if (lane >= 20 && lane < 24) out[lane] = sm.look_r[round & 1].c[lane - 20];
+    };
+    for (int round = from; round < n_rounds; round++) {
+        const bool next = round + 1 < n_rounds;
+        const GkrStepConst &rc = consts[round], &rn = consts[next ? round + 1 : round];
+        const GkrTable& tb = looks[round];
+        const qm31 w0 = qm31_sub(qm31_one(), rc.y), w1 = qm31_sub(rc.y, w0);  // the next correction is corr (w0 + w1 r)
+        if (!last_warp) {
+            if (round > from) {
+                const qm31 r = sm.look_r[(round & 1) ^ 1], y = consts[round - 1].y, omy = qm31_sub(qm31_one(), y);
+                const qm31_pair p = product_pair(r, y, qm31_sub(qm31_one(), r), omy);
+                const qm31 up = qmul(corr, qm31_add(p.a, p.b));
+                if (lane < round) corr = up;
+                if (warp == 2) record(round - 1);
+            }
+            if (!gave_up && tb.ctas && !wait_count(&sync->look_count[round], tb.ctas)) gave_up = true;
+            gave_up = __any_sync(0xffffffffu, gave_up);
+            if (next) {
+                unsigned long long* const a = acc.at(round + 1, lane) + 4 * value;
+                const bool mine = lane < acc.groups && !gave_up;
+                ulonglong2 lo = make_ulonglong2(0ull, 0ull), hi = lo;
+                if (mine) { lo = __ldcg(reinterpret_cast<const ulonglong2*>(a)); hi = __ldcg(reinterpret_cast<const ulonglong2*>(a) + 1); }
+                const qm31 v{{m31_reduce64(lo.x), m31_reduce64(lo.y), m31_reduce64(hi.x), m31_reduce64(hi.y)}};
+                const qm31 sum = warp_sum_m(lane <= round ? qmul(v, corr) : qm31_zero());
+                if (lane == round + 1 && value < 2) sm.look_enter[node] = v;
+                if (lane == 0) sm.look_sums[value] = sum;
+                __syncwarp();
+                asm volatile("bar.arrive 2, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 1)) : "memory");
+                if (mine) reinterpret_cast<ulonglong2*>(a)[0] = reinterpret_cast<ulonglong2*>(a)[1] = make_ulonglong2(0ull, 0ull);  // for the round after the next
+            }
+            __threadfence();  // what the CTAs have folded, and the zeros, before the challenge that follows
+        } else if (next) {
+            // lane = 16 node + 4 c + k: that node's share of the coefficient of r^k in coefficient c
+            const qm31 a = hn ? rn.B[c] : rn.A[c], a0 = qmul(a, w0), a1 = k == 0 ? a : qmul(a, w1), l1 = rn.L1[c];
+            asm volatile("bar.sync 3, 64;" ::: "memory");  // this round's polynomial: its value at r, and what enters, is the next claim
+            const qm31 claim = hn ? qm31_zero() : k == 0 ? qm31_add(sm.look_coef[round & 1][0], rc.entering) : sm.look_coef[round & 1][k];
+            const qm31 q = qmul(claim, l1);
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 1)) : "memory");
+            const qm31 s0 = sm.look_sums[hn], s1 = sm.look_sums[2 + hn], s2 = sm.look_sums[4 + hn], mid = qm31_sub(s1, qm31_add(s0, s2));
+            const qm31 lo = k == 0 ? s0 : k == 1 ? mid : k == 2 ? s2 : qm31_zero(), hi = k == 0 ? sm.look_enter[hn] : k == 1 ? s0 : k == 2 ? mid : s2;
+            const qm31_pair p = product_pair(a0, lo, a1, hi);
+            qm31 v = qm31_add(qm31_add(p.a, p.b), q);
+            v = qm31_add(v, shflb(v, lane ^ 16));
+            if (lane < 16) sm.ahead[lane] = v;
+        }
+        look_met();
+        if (warp == 1 && lane < 4 && !gave_up) *reinterpret_cast<volatile uint32_t*>(&sync->slot[round + 1][lane]) = sm.look_r[round & 1].c[lane] | 0x80000000u;
+    }
+    if (warp == 2) record(n_rounds - 1);
+    return gave_up;
+}
+
+// Tables [first, end) of the layer; then, where look_from >= 0, the rounds from that on ahead of the transcript (the tables behind the n_rounds + 1 of the others) and
+// the masks; end is look_from + 1. rc: null where the transcript's steps are launches of their own (gkr_batch_step_kernel); no CTA then
 // keeps it, and the challenge is in its slot before the launch.
-__global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int first, int end,
+__global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int first, int end,
                                                                          const uint32_t* __restrict__ eq, qm31 lambda, const uint32_t* __restrict__ alpha_pow,
-                                                                         GkrStepState* st, GkrSync* sync, const GkrStepConst* __restrict__ rc,
+                                                                         GkrStepState* st, GkrAcc acc, GkrSync* sync, const GkrStepConst* __restrict__ rc, int look_from,
                                                                          uint32_t* records, int n_rounds, GkrLayerOut host) {
-    __shared__ uint32_t sums[GKR_GROUPS][16];  // of the pass at hand; zero before it
-    __shared__ GkrTable tabs[GKR_LAYER_MAX_ROUNDS + 1];
-    __shared__ qm31 r_sh;
+    __shared__ uint32_t sums[GKR_GROUPS][2 * ACC_WORDS];  // of the pass at hand; zero before it
+    __shared__ GkrTable tabs[2 * GKR_LAYER_MAX_ROUNDS + 1];
+    __shared__ qm31 r_sh, eq_tab[EQ_TABLES][32];
     __shared__ bool gave_up;
     // CTA 0 only: the transcript
     __shared__ GkrStepSm sm;
-    __shared__ struct alignas(16) { uint32_t digest[8], n_draws, pad[3]; qm31 challenge, claim, corr[GKR_GROUPS]; } head_words;
-    GkrStepState& s = *reinterpret_cast<GkrStepState*>(&head_words);  // the state up to its accumulators, which stay below
+    __shared__ GkrStepState s;
     __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];
-    static_assert(sizeof(head_words) == offsetof(GkrStepState, acc), "the head of GkrStepState");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool lead = blockIdx.x == 0 && rc;
-    for (int i = tid; i < 2 * end; i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
-    for (int i = tid; i < GKR_GROUPS * 16; i += GKR_THREADS) (&sums[0][0])[i] = 0u;
+    for (int i = tid; i < 2 * (look_from >= 0 ? 2 * n_rounds + 1 : end); i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
+    for (int i = tid; i < GKR_GROUPS * 2 * ACC_WORDS; i += GKR_THREADS) (&sums[0][0])[i] = 0u;
     if (tid == 0) gave_up = false;
     if (lead) {
         for (int i = tid; i < 16 * n_rounds; i += GKR_THREADS) reinterpret_cast<uint4*>(consts)[i] = reinterpret_cast<const uint4*>(rc)[i];
-        for (int i = tid; i < (int)(sizeof(head_words) / 4); i += GKR_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = reinterpret_cast<const uint32_t*>(st)[i];
+        for (int i = tid; i < (int)(sizeof(s) / 4); i += GKR_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = reinterpret_cast<const uint32_t*>(st)[i];
+    }
+    // eq(., point) of a term's index: from a table, or, where there is none, as a product over the index's bits, five to a table of a warp's making
+    // (bit k goes with coordinate n_rounds - 1 - k; the first coordinate's share is 1 - y)
+    if (!eq && warp < EQ_TABLES) {
+        auto factor = [&](int b) {
+            const int bit = 5 * warp + b;
+            const qm31 y = bit < n_rounds - 1 ? rc[n_rounds - 1 - bit].y : qm31_zero();
+            return (lane >> b) & 1 ? y : qm31_sub(qm31_one(), y);
+        };
+        qm31 v = factor(4);
+        if (warp == 0) v = qmul(v, qm31_sub(qm31_one(), rc[0].y));
+        const qm31_pair p = product_pair(factor(0), factor(1), factor(2), factor(3));
+        eq_tab[warp][lane] = qmul(v, qmul(p.a, p.b));
     }
     __syncthreads();
+    auto eq_at = [&](uint32_t i) {
+        if (eq) return ldqb(eq, i);
+        const qm31 low = qmul(eq_tab[0][i & 31], eq_tab[1][(i >> 5) & 31]);
+        return qmul(low, eq_tab[2][i >> 10]);
+    };
     if (lead && warp == 0) batch_step_open(sm, s, lane);
     for (int t = first; t < end; t++) {
         const GkrTable tb = tabs[t];
@@ -410,12 +643,12 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
         bool live = false;
         qm31 ea = qm31_zero();
         auto look_up = [&]() {  // forms 1 and 2
-            const uint32_t flat = chunk * GKR_THREADS + ((tid + GKR_THREADS - 32) & (GKR_THREADS - 1));
+            const uint32_t mine = (tid + GKR_THREADS - 32) & (GKR_THREADS - 1), flat = (chunk << tb.run_log) + mine;
             const uint32_t at = tb.form == 1 ? flat >> 2 : flat;
             term = at & ((1u << tb.terms_log) - 1);
-            live = (at >> tb.terms_log) < tb.n_items;
+            live = (at >> tb.terms_log) < tb.n_items && !(mine >> tb.run_log);
             if (live) it = items[at >> tb.terms_log];
-            if (tb.form == 1 && live) ea = qmul(ldqb(eq, term), ldqb(alpha_pow, (uint32_t)it.slot));
+            if (tb.form == 1 && live) ea = qmul(eq_at(term), ldqb(alpha_pow, (uint32_t)it.slot));
         };
         if (tb.form != 0) look_up();
         if (!lead && t > 0) {
@@ -465,13 +698,13 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
         } else if (tb.form == 0) {
             for (; chunk < tb.chunks; chunk += tb.ctas) {
                 qm31 s0 = qm31_zero(), s2 = qm31_zero();
-                const int whole = tb.terms_log - 8 - tb.run_log;  // log2 of an item's chunks
+                const int whole = tb.terms_log - GKR_THREADS_LOG - tb.run_log;  // log2 of an item's chunks
                 const uint32_t flat = chunk * GKR_THREADS + tid;
-                const uint32_t idx = tb.terms_log < 8 ? flat >> tb.terms_log : chunk >> whole;
+                const uint32_t idx = tb.terms_log < GKR_THREADS_LOG ? flat >> tb.terms_log : chunk >> whole;
                 live = idx < tb.n_items;
                 if (live) {
                     it = items[idx];
-                    if (tb.terms_log < 8) item_sums_of(it, flat & ((1u << tb.terms_log) - 1), (size_t)1 << tb.terms_log, r, eq, lambda, s0, s2);
+                    if (tb.terms_log < GKR_THREADS_LOG) item_sums_of(it, flat & ((1u << tb.terms_log) - 1), (size_t)1 << tb.terms_log, r, eq, lambda, s0, s2);
                     else item_sums_of(it, (size_t)(chunk & ((1u << whole) - 1)) * GKR_THREADS + tid, (size_t)GKR_THREADS << whole, r, eq, lambda, s0, s2);
                 }
                 add_to_group(sums, tb.terms_log < 5 ? 1 << tb.terms_log : 32, live, (uint32_t)it.slot, (uint32_t)(it.slot >> 32), alpha_pow, s0, s2);
@@ -486,44 +719,55 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
         }
         __syncthreads();
         if (!lead) {
-            if (step) {
+            if (step && tid < 8 * GKR_GROUPS) {
                 uint32_t* const h = &sums[tid >> 3][2 * (tid & 7)];
                 const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
                 h[0] = h[1] = 0u;
-                if (v) atomicAdd(&st->acc[t & 1][tid >> 3][tid & 7], v);
+                if (v) atomicAdd(acc.at(t, tid >> 3) + (tid & 7), v);
                 __threadfence();
-            } else {
-                __threadfence_system();
             }
+            if (!step) __threadfence_system();
             __syncthreads();
             if (tid == 0) { __threadfence(); atomicAdd(&sync->count[t], 1u); }
             continue;
         }
         // CTA 0 from here on; its own sums stay where they are
+        const bool ahead = t == look_from;  // (its own part of the layer is then read by others before there is a challenge)
+        if (ahead && tid == 0) { __threadfence(); atomicAdd(&sync->count[t], 1u); }
         if (tb.ctas > 1) {
-            if (tid == 0) {
-                uint32_t n = ld_acquire(&sync->count[t]);
-                for (uint32_t spin = 0; n != tb.ctas - 1 && spin < SPIN_LIMIT; spin++) n = ld_acquire(&sync->count[t]);
-                if (n != tb.ctas - 1) gave_up = true;
-            }
+            if (tid == 0 && !wait_count(&sync->count[t], tb.ctas - (ahead ? 0u : 1u))) gave_up = true;
             __syncthreads();
             if (gave_up) return;
         }
         if (!step) break;
         auto challenge_drawn = [] { asm volatile("bar.sync 1, %0;" ::"n"(GKR_THREADS) : "memory"); };
+        if (ahead && warp) {
+            if (look_value(warp) >= 0 && look_helpers(sm, consts, tabs + n_rounds + 1, s, acc, sync, look_from, n_rounds, records)) gave_up = true;
+            break;
+        }
         if (warp == 0) {
             unsigned long long a[8];
+            const bool theirs = tb.ctas > 1 && lane < acc.groups;
 #pragma unroll
-            for (int c = 0; c < 8; c++) a[c] = tb.ctas > 1 ? __ldcg(&st->acc[t & 1][lane][c]) : 0ull;
+            for (int c = 0; c < 8; c++) a[c] = theirs ? __ldcg(acc.at(t, lane) + c) : 0ull;
 #pragma unroll
             for (int c = 0; c < 8; c++) {
                 a[c] += (unsigned long long)sums[lane][2 * c] + ((unsigned long long)sums[lane][2 * c + 1] << 16);
                 sums[lane][2 * c] = sums[lane][2 * c + 1] = 0u;
             }
-            batch_step(sm, s, consts[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, challenge_drawn);
-            if (tb.ctas > 1) {
+            if (ahead) {
+                if (theirs) {
 #pragma unroll
-                for (int c = 0; c < 8; c++) st->acc[t & 1][lane][c] = 0ull;  // for the round after the next: seen with the next challenge
+                    for (int c = 0; c < 8; c++) acc.at(t, lane)[c] = 0ull;
+                    __threadfence();
+                }
+                look_lead(sm, consts, look_from, n_rounds, batch_coefficients(s, consts[t], s.corr[lane], acc_value(a), acc_value(a + 4)));
+                break;
+            }
+            batch_step(sm, s, consts[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, challenge_drawn);
+            if (theirs) {
+#pragma unroll
+                for (int c = 0; c < 8; c++) acc.at(t, lane)[c] = 0ull;  // for the round after the next: seen with the next challenge
             }
         } else {
             // Warp 1 sends the challenge. Its fence stands behind the barrier that put everybody's folded layers behind this point,
@@ -534,8 +778,74 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
             if (warp == 1 && lane < 4 && tb.later > 1) *reinterpret_cast<volatile uint32_t*>(&sync->slot[t + 1][lane]) = sm.r.c[lane] | 0x80000000u;
         }
     }
+    if (look_from >= 0 && !lead) {
+        const GkrTable* const looks = tabs + n_rounds + 1;
+        const qm31 half_lambda = qm31_mul_m31(lambda, 1u << 30);
+        const uint32_t block = blockIdx.x - 1;
+        for (int t = look_from; t <= n_rounds; t++) {
+            const GkrTable tb = t < n_rounds ? looks[t] : tabs[n_rounds];
+            if (block >= tb.ctas) {
+                if (block >= tb.later) return;
+                continue;
+            }
+            const GkrBatchItem* const items = items_base + tb.first;
+            const int lanes_log = tb.form == 3 ? 3 : tb.form == 4 ? 2 : 0;  // lanes a term (form 3), an item (4), of two threads an item (2)
+            uint32_t chunk = block, term = 0;
+            GkrBatchItem it{};
+            bool live = false;
+            qm31 ea = qm31_zero();
+            auto look_up = [&]() {
+                const uint32_t at = ((chunk << tb.run_log) + tid) >> lanes_log, item = at >> tb.terms_log;
+                term = at & ((1u << tb.terms_log) - 1);
+                live = item < tb.n_items && !(tid >> tb.run_log);
+                if (live) it = items[item];
+                if (tb.form == 3 && live) ea = qmul(eq_at(term), ldqb(alpha_pow, (uint32_t)it.slot));
+            };
+            look_up();
+            if (t > look_from) {
+                if (tid < 4) {
+                    uint32_t w = ld_acquire(&sync->slot[t][tid]);
+                    for (uint32_t spin = 0; !(w >> 31) && spin < SPIN_LIMIT; spin++) w = ld_acquire(&sync->slot[t][tid]);
+                    if (!(w >> 31)) gave_up = true;
+                    r_sh.c[tid] = w & 0x7fffffffu;
+                }
+            } else if (t > 0 && tid == 0 && !wait_count(&sync->count[t], tabs[t].ctas)) {  // the layer as the table before left it
+                gave_up = true;
+            }
+            __syncthreads();
+            if (gave_up) return;
+            const qm31 r = r_sh;
+            for (;;) {
+                if (tid >> tb.run_log) {  // (whole warps)
+                } else if (tb.form == 3) look_term(sums, it, live, term, tb.terms_log, r, half_lambda, ea);
+                else if (live && tb.form == 4) fix_entry(it, tid & 3, 4, r);
+                else if (live) fix_mask(it, (int)term, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
+                chunk += tb.ctas;
+                if (chunk >= tb.chunks) break;
+                look_up();
+            }
+            __syncthreads();
+            if (tb.form == 3)
+                for (int i = tid; i < ACC_WORDS * acc.groups; i += GKR_THREADS) {
+                    uint32_t* const h = &sums[0][0] + 2 * i;
+                    const unsigned long long v = (unsigned long long)h[0] + ((unsigned long long)h[1] << 16);
+                    h[0] = h[1] = 0u;
+                    if (v) atomicAdd(acc.at(t + 1, 0) + i, v);
+                }
+            if (t == n_rounds) __threadfence_system();
+            __syncthreads();
+            if (tid == 0) { __threadfence(); atomicAdd(t < n_rounds ? &sync->look_count[t] : &sync->count[t], 1u); }
+        }
+        return;
+    }
     if (!lead) return;
     __syncthreads();
+    if (gave_up) return;
+    if (look_from >= 0) {
+        if (tid == 0 && !wait_count(&sync->count[n_rounds], tabs[n_rounds].ctas)) gave_up = true;
+        __syncthreads();
+        if (gave_up) return;
+    }
     if (warp == 0) batch_step_close(sm, st, lane);
     __threadfence();
     __syncthreads();
@@ -546,7 +856,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 2) gkr_batch_layer_kernel(const G
 }
 
 // The step after table t < n_rounds by itself, one warp; after the last table, what goes to the host.
-__global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, GkrSync* sync, const GkrStepConst* __restrict__ rc, uint32_t* records, int t, int n_rounds,
+__global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, GkrAcc acc, GkrSync* sync, const GkrStepConst* __restrict__ rc, uint32_t* records, int t, int n_rounds,
                                                             GkrLayerOut host) {
     __shared__ GkrStepSm sm;
     const int lane = threadIdx.x;
@@ -560,8 +870,8 @@ __global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, Gk
     unsigned long long a[8];
 #pragma unroll
     for (int c = 0; c < 8; c++) {
-        a[c] = st->acc[t & 1][lane][c];
-        st->acc[t & 1][lane][c] = 0ull;
+        a[c] = lane < acc.groups ? acc.at(t, lane)[c] : 0ull;
+        if (lane < acc.groups) acc.at(t, lane)[c] = 0ull;
     }
     batch_step_open(sm, *st, lane);
     batch_step(sm, *st, rc[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, [] {});
@@ -707,7 +1017,7 @@ static int batch_buffers(zkb_ctx* ctx) {
     int sms = 0, per_sm = 0;
     ZKB_CUDA(ctx, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     ZKB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gkr_batch_layer_kernel, GKR_THREADS, 0));
-    ctx->batch_grid = sms * std::min(per_sm, 2);
+    ctx->batch_grid = sms * std::min(per_sm, 1);
     ZKB_CUDA(ctx, cudaMallocHost(&ctx->h_batch, H_BATCH_WORDS * 4));
     ctx->h_batch[H_BATCH_FLAG] = 0;
     ctx->batch_round = 0;
@@ -807,16 +1117,81 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
 
 // The block a layer's launch stages: the transcript's state, the CTAs' meeting place, the powers of alpha, the rounds' constants, the tables,
 // room for the rounds' records (every part a multiple of four words).
-struct LayerBlob { size_t sync, alpha, rounds, tables, records, words; };
+struct LayerBlob { size_t acc, sync, alpha, rounds, tables, records, words; };
 static LayerBlob layer_blob(const GkrLayerPlan& plan) {
     LayerBlob o;
-    o.sync = sizeof(GkrStepState) / 4;
+    o.acc = sizeof(GkrStepState) / 4;
+    o.sync = o.acc + 2 * 2 * ACC_WORDS * (size_t)plan.n_rounds;
     o.alpha = o.sync + sizeof(GkrSync) / 4;
     o.rounds = o.alpha + 4 * plan.n_vars.size();
     o.tables = o.rounds + (sizeof(GkrStepConst) / 4) * (size_t)plan.n_rounds;
     o.records = o.tables + plan.tables.size();
     o.words = o.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
     return o;
+}
+
+// The rounds that are taken ahead of the transcript: from the first whose table takes four lanes a term. Larger ones are bound by their products, of which this
+// way has twice as many. Their tables go behind the others, and the items that are used into look_items.
+static GkrTable* tables_of(GkrLayerPlan& plan) { return reinterpret_cast<GkrTable*>(plan.tables.data()); }
+static void plan_look(GkrLayerPlan& plan, uint32_t grid) {
+    const int n = plan.n_rounds;
+    GkrTable* tables = tables_of(plan);
+    int from = 0;
+    while (from < n && tables[from].form != 1) from++;
+    plan.look_from = -1;
+    if (plan.launches || from + 2 > n || grid < 2) return;
+    plan.look_from = from;
+    plan.tables.resize((sizeof(GkrTable) / 4) * (2 * (size_t)n + 1), 0u);
+    tables = tables_of(plan);
+    std::vector<GkrBatchItem>& out = plan.look_items;
+    auto table = [&](int j) { return std::make_pair(plan.items.begin() + plan.table_at[j], plan.items.begin() + plan.table_at[j + 1]); };
+    out.assign(plan.items.begin(), table(from).second);
+    auto add = [&](const GkrBatchItem& it, uint32_t mode) {
+        out.push_back(it);
+        out.back().mode = mode;
+    };
+    for (int j = from; j <= n; j++) {
+        GkrTable& tb = tables[j < n ? n + 1 + j : n];
+        tb.first = (uint32_t)out.size();
+        for (auto it = table(j).first; it != table(j).second; ++it) {
+            if (j == n) { add(*it, it->mode); continue; }
+            if (j == n - 1) {  // eight entries to four; those that enter now are folded with the last challenge
+                if (it->mode == 1) add(*it, LOOK_FIX);
+                continue;
+            }
+            if (it->mode == 1 && j > from) { add(*it, LOOK_FIX); continue; }
+            add(*it, LOOK_AS_IS);
+            GkrBatchItem& as_is = out.back();
+            if (it->mode == 1) {  // as table `from` has left it
+                as_is.den = as_is.den_out;
+                as_is.num = as_is.num_out;
+                if (as_is.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) as_is.kind = ZKB_GKR_LOGUP_GENERIC;
+            }
+        }
+        if (j < n - 1)
+            for (auto it = table(j + 1).first; it != table(j + 1).second; ++it)
+                if (it->mode == 0) add(*it, LOOK_ENTERS);
+        tb.n_items = (uint32_t)(out.size() - tb.first);
+        tb.terms_log = j == n ? 1 : j == n - 1 ? 0 : n - j - 2;
+        tb.form = j == n ? 2 : j == n - 1 ? 4 : 3;
+        const size_t lanes = ((size_t)tb.n_items << tb.terms_log) << (tb.form == 3 ? 3 : tb.form == 4 ? 2 : 0);
+        // as few warps a CTA as there are CTAs for: a pass of a warp a scheduler takes 2,300 cycles, of four 5,100
+        tb.run_log = LOOK_MIN_LOG;
+        while (tb.run_log < GKR_THREADS_LOG && ((lanes + (1u << tb.run_log) - 1) >> tb.run_log) > grid - 1) tb.run_log++;
+        tb.chunks = (uint32_t)((lanes + (1u << tb.run_log) - 1) >> tb.run_log);
+        tb.ctas = std::min(tb.chunks, grid - 1);
+    }
+    uint32_t later = 0;
+    for (int j = n; j >= from; j--) {
+        GkrTable& tb = tables[j < n ? n + 1 + j : n];
+        tb.later = later;
+        later = std::max(later, tb.ctas);
+    }
+    later++;  // CTA 0 takes none of them
+    for (int j = from; j >= 0; j--) {
+        tables[j].later = later;
+        later = std::max(later, tables[j].ctas);
+    }
 }
 
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
@@ -844,28 +1219,37 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
         // Four lanes a term while that is at most two passes of the whole grid: a pass of this form is a third of the other's latency,
         // and a third more work.
         tb.form = j == n_rounds ? 2 : 4 * terms <= 2 * (size_t)grid * GKR_THREADS ? 1 : 0;
-        // Whole items of 2^8 terms and more: a thread takes up to eight terms for one reduction, as long as four pieces per CTA remain.
+        // Whole items of 2^GKR_THREADS_LOG terms and more: a thread takes up to eight terms for one reduction, as long as four pieces per CTA remain.
         tb.run_log = 0;
         if (tb.form == 0)
-            while (tb.run_log < 3 && tb.terms_log - 8 > tb.run_log && (terms >> (8 + tb.run_log + 1)) >= 4 * (size_t)grid) tb.run_log++;
-        const size_t chunks = tb.form == 0 && tb.terms_log >= 8 ? terms >> (8 + tb.run_log) : ((tb.form == 1 ? 4 * terms : terms) + GKR_THREADS - 1) / GKR_THREADS;
+            while (tb.run_log < 3 && tb.terms_log - GKR_THREADS_LOG > tb.run_log && (terms >> (GKR_THREADS_LOG + tb.run_log + 1)) >= 4 * (size_t)grid) tb.run_log++;
+        if (tb.form) {
+            const size_t lanes = tb.form == 1 ? 4 * terms : terms;
+            for (tb.run_log = LOOK_MIN_LOG; tb.run_log < GKR_THREADS_LOG && ((lanes + (1u << tb.run_log) - 1) >> tb.run_log) > grid;) tb.run_log++;
+        }
+        const size_t chunks = tb.form == 0 && tb.terms_log >= GKR_THREADS_LOG ? terms >> (GKR_THREADS_LOG + tb.run_log) : tb.form == 0 ? (terms + GKR_THREADS - 1) / GKR_THREADS : ((tb.form == 1 ? 4 * terms : terms) + (1u << tb.run_log) - 1) >> tb.run_log;
         tb.chunks = (uint32_t)chunks;
         // (sending the sums and the challenge round costs less than a second piece in CTA 0: 6,400 cycles against 8,500)
         tb.ctas = (uint32_t)std::min<size_t>(chunks, grid);
         tb.later = later;
         later = std::max(later, tb.ctas);
     }
+    plan_look(plan, grid);
+    // Rounds that take four and eight lanes a term can work eq out: a term a thread would take two products more for each of its six.
+    plan.needs_eq = plan.look_from != 0 || tables_of(plan)[0].terms_log > 5 * EQ_TABLES;
+    const std::vector<GkrBatchItem>& items = plan.look_from >= 0 ? plan.look_items : plan.items;
     // What the launch stages later must not come to lie over the items: room for both.
-    const size_t item_bytes = plan.items.size() * sizeof(GkrBatchItem);
+    const size_t item_bytes = items.size() * sizeof(GkrBatchItem);
     if (int rc = stage_reserve(ctx, blob_slots(item_bytes) + blob_slots(4 * layer_blob(plan).words))) return rc;
     void* d = nullptr;
-    if (int rc = stage_blob(ctx, plan.items.data(), item_bytes, &d)) return rc;
+    if (int rc = stage_blob(ctx, items.data(), item_bytes, &d)) return rc;
     plan.d_items = static_cast<const GkrBatchItem*>(d);
     return ZKB_OK;
 }
 
-int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
+int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
                           const uint32_t* eq_evals, const uint32_t h_lambda[4], const uint32_t chan[9]) {
+    ZKB_CHECK_ARG(ctx, eq_evals || !plan.needs_eq);
     DeviceGuard g(ctx);
     if (int rc = batch_buffers(ctx)) return rc;
     const size_t K = plan.n_vars.size();
@@ -923,6 +1307,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
     const uint32_t* const d_alpha = d_blob + at.alpha;
     uint32_t* const d_records = d_blob + at.records;
     GkrSync* const d_sync = reinterpret_cast<GkrSync*>(d_blob + at.sync);
+    const GkrAcc acc{reinterpret_cast<unsigned long long*>(d_blob + at.acc), n_rounds};
     cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
     if (!plan.launches) {
         ProfScope prof(ctx, "gkr_batch_layer_kernel");
@@ -935,21 +1320,27 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t
         cfg.stream = ctx->stream;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, d_tables, 0, n_rounds + 1, eq_evals, lam, d_alpha, d_state, d_sync, d_consts, d_records, n_rounds, host);
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, d_tables, 0, plan.look_from >= 0 ? plan.look_from + 1 : n_rounds + 1, plan.needs_eq ? eq_evals : nullptr, lam, d_alpha, d_state, acc,
+                               d_sync, d_consts, plan.look_from, d_records, n_rounds, host);
     }
     // Asked for, or the CTAs are not all resident at once (a share of the GPU's SMs): a launch per table and one per step, where nobody waits.
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
         (void)cudaGetLastError();
+        if (plan.look_from >= 0) {  // other tables and items then
+            plan.launches = true;
+            if (int rc = gkr_batch_plan(ctx, plan)) return rc;
+            return GKR_BATCH_AGAIN;
+        }
         e = cudaSuccess;
         for (int t = 0; t <= n_rounds && e == cudaSuccess; t++) {
             {
                 ProfScope prof(ctx, "gkr_batch_layer_kernel");
-                gkr_batch_layer_kernel<<<h_tables[t].ctas, GKR_THREADS, 0, ctx->stream>>>(plan.d_items, d_tables, t, t + 1, eq_evals, lam, d_alpha, d_state, d_sync, nullptr,
-                                                                                          d_records, n_rounds, host);
+                gkr_batch_layer_kernel<<<h_tables[t].ctas, GKR_THREADS, 0, ctx->stream>>>(plan.d_items, d_tables, t, t + 1, eq_evals, lam, d_alpha, d_state, acc, d_sync, nullptr,
+                                                                                          -1, d_records, n_rounds, host);
             }
             {
                 ProfScope prof(ctx, "gkr_batch_step_kernel");
-                gkr_batch_step_kernel<<<1, 32, 0, ctx->stream>>>(d_state, d_sync, d_consts, d_records, t, n_rounds, host);
+                gkr_batch_step_kernel<<<1, 32, 0, ctx->stream>>>(d_state, acc, d_sync, d_consts, d_records, t, n_rounds, host);
             }
             e = cudaGetLastError();
         }

@@ -66,14 +66,19 @@ struct GkrLayerPlan {
     std::vector<GkrBatchItem> items; // table after table; table j: the fixes of round j - 1, the first sums of those entering in round j (slot = oracle)
     std::vector<size_t> table_at;    // n_rounds + 2
     std::vector<uint32_t> tables;    // filled by gkr_batch_plan: how the kernel takes them
+    int look_from = -1;              // and from which round on the rounds are taken ahead of the transcript, with which items (-1: none, and `items`)
+    std::vector<GkrBatchItem> look_items;
+    bool needs_eq = true;            // whether begin wants the table of eq(., point)
     const GkrBatchItem* d_items = nullptr;
     bool launches = false;           // the layer as a launch per table and one per transcript step
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
 
 // alpha_pow[k] = alpha^k; claims[k]: oracle k's claim before the first round (4 words each). chan: digest (8 words) and n_draws.
-// Enqueues the layer; gkr_batch_layer_end waits for it. Only gkr_batch_plan may come between the two.
-int gkr_batch_layer_begin(zkb_ctx* ctx, const GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
+// Enqueues the layer; gkr_batch_layer_end waits for it. Only gkr_batch_plan may come between the two. GKR_BATCH_AGAIN: the launch was refused and the plan is
+// another one now (launches, which needs the table); call again.
+constexpr int GKR_BATCH_AGAIN = -1000;
+int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alpha_pow, const uint32_t* claims, const GkrRoundConst* rounds,
                           const uint32_t* eq_evals, const uint32_t h_lambda[4], const uint32_t chan[9]);
 
 // In the context's memory, until the next call: n_rounds x GKR_LAYER_OUT_WORDS, the channel as above, n_oracles x GKR_LAYER_MASK_WORDS

@@ -776,30 +776,6 @@ constexpr int SOLO_BASIS_WARPS = 5;
 static_assert(4 * SOLO_BYTES <= CHAIN_WORK_BYTES, "two layers of two columns");
 __device__ __forceinline__ void solo_done() { asm volatile("bar.sync 9, %0;" ::"n"(RES_THREADS) : "memory"); }
 
-// A product by y, a coordinate a lane (its two low bits): four multiply-adds and a reduction, where a lane that makes all four takes sixteen and four.
-struct slice_by {
-    uint32_t m[4];
-    __device__ __forceinline__ slice_by(qm31 y) {
-        const int k = threadIdx.x & 3;
-        const uint32_t e0 = m31_sub(m31_dbl(y.c[2]), y.c[3]), e1 = m31_add(y.c[2], m31_dbl(y.c[3]));
-        m[0] = k == 0 ? y.c[0] : k == 1 ? y.c[1] : k == 2 ? y.c[2] : y.c[3];
-        m[1] = k == 0 ? P - y.c[1] : k == 1 ? y.c[0] : k == 2 ? P - y.c[3] : y.c[2];
-        m[2] = k == 0 ? e0 : k == 1 ? e1 : k == 2 ? y.c[0] : y.c[1];
-        m[3] = k == 0 ? P - e1 : k == 1 ? e0 : k == 2 ? P - y.c[1] : y.c[0];
-    }
-    // coordinate k of x y, and the word z added (qm31_add_products has the bound)
-    __device__ __forceinline__ uint32_t mul_add(qm31 x, uint32_t z) const {
-        return m31_reduce64(z + (uint64_t)x.c[0] * m[0] + (uint64_t)x.c[1] * m[1] + (uint64_t)x.c[2] * m[2] + (uint64_t)x.c[3] * m[3]);
-    }
-};
-// The value whose coordinates are in lanes first ... first + 3.
-__device__ __forceinline__ qm31 gather_q(uint32_t v, int first) {
-    qm31 r;
-#pragma unroll
-    for (int c = 0; c < 4; c++) r.c[c] = __shfl_sync(0xffffffffu, v, first + c);
-    return r;
-}
-
 // Where one_lead starts and ends.
 enum : int { LEAD_BEGIN = 1, LEAD_ROUNDS = 2, LEAD_SUMS = 4 };
 

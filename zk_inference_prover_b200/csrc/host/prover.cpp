@@ -1549,8 +1549,13 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
         // EqEvals::generate, :235-247
         hc.reset(new HostClock("gkr.layer.eq_evals"));
         SecureMle eq_evals;
-        if (ood_point.empty()) eq_evals = B200Backend::gen_eq_evals(d, {}, qm31_one());
-        else eq_evals = B200Backend::gen_eq_evals(d, std::vector<qm31>(ood_point.begin() + 1, ood_point.end()), eq1(qm31_zero(), ood_point[0]));
+        bool have_eq = false;
+        auto make_eq = [&] {
+            if (ood_point.empty()) eq_evals = B200Backend::gen_eq_evals(d, {}, qm31_one());
+            else eq_evals = B200Backend::gen_eq_evals(d, std::vector<qm31>(ood_point.begin() + 1, ood_point.end()), eq1(qm31_zero(), ood_point[0]));
+            have_eq = true;
+        };
+        if (on_device(plan) ? plan.needs_eq : nv > 0) make_eq();
         hc.reset(new HostClock("gkr.layer.claims"));
         for (size_t i : inst) {
             if (towers[i].log == n_remaining) {  // its output layer: one entry per column
@@ -1593,7 +1598,11 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
             uint32_t chan[9];
             memcpy(chan, ch.digest().data(), 32);
             chan[8] = ch.n_draws();
-            d.check(zk::gkr_batch_layer_begin(d.ctx(), plan, alpha_pow[0].c, sc_claims[0].c, consts.data(), eq_evals.words.ptr(), lambda.c, chan));
+            for (;;) {
+                const int rc = zk::gkr_batch_layer_begin(d.ctx(), plan, alpha_pow[0].c, sc_claims[0].c, consts.data(), have_eq ? eq_evals.words.ptr() : nullptr, lambda.c, chan);
+                if (rc != zk::GKR_BATCH_AGAIN) { d.check(rc); break; }
+                make_eq();
+            }
             hc.reset();
             if (layer + 1 < n_layers) make_next(layer + 1);
             hc.reset(new HostClock("gkr.layer.wait"));
