@@ -5,9 +5,11 @@ import numpy as np
 import pytest
 
 from test_freivalds import test_freivalds_device_matches_oracle as freivalds_matches_oracle
+from test_witness_gen import run_dequant
 from test_witness_gen import test_dequant_matches_oracle as dequant_matches_oracle
 from test_witness_pre import run_residual_stream
 from zk_inference_prover_b200 import witness_cases as wc
+from zk_inference_prover_b200.witness_cases import dequant_case
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +63,35 @@ def test_residual_stream_edges(ctx, oracle, even, shape, n, log_rows, live_rows,
 @pytest.mark.parametrize("variant,tokens,chunks,per_row", [(1, 4, 4, 330), (0, 2, 4, 500), (1, 64, 64, 1)])
 def test_dequant_edges(ctx, oracle, variant, tokens, chunks, per_row):
     dequant_matches_oracle(ctx, oracle, variant, tokens, chunks, per_row, 16, 1, 1, False)
+
+
+@pytest.mark.parametrize("log_rows,kmax,change", [(6, 21, None), (5, 13, "table"), (5, 13, "operands"), (14, 13, None)])
+def test_residual_stream_wide_values(ctx, oracle, log_rows, kmax, change):
+    """Tables too large for a counter a row; table rows and operands that 32 bits do not hold the sum of; rows for more passes than teams."""
+    case = wc.residual_stream_case(5 + log_rows, "pairs", 16, log_rows, (1 << log_rows) - 3, un=(1, 2) if change == "operands" else (0, 0), kind=0, sticky=True, kmax=kmax, spread=9)
+    rng = np.random.default_rng(log_rows)
+    if change == "table":
+        rows = case["norm3"].reshape(-1, 3)
+        at = rng.integers(1, len(rows), len(rows) // 2)
+        rows[at, rng.integers(0, 3, at.size)] = rng.choice(np.array([255, 256, 65535, 65536, 1 << 20], np.uint32), at.size)
+    if change == "operands":
+        for images in case["un2"]:
+            at = rng.integers(0, images.size, images.size // 2)
+            images[at] = rng.choice(np.array([0, 131071, 131072, -131072, -131073, 1 << 20, (1 << 30) - 1, -(1 << 29)], np.int64), at.size)
+            images[1::2] = rng.choice(np.array([0, 1, 254, 300, (1 << 20) - 1, 1 << 20, 1 << 29], np.int64), images.size // 2)
+    got, want = run_residual_stream(ctx, case), oracle.witness_residual_stream(case)
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("variant,per_row,kmax,wide_row", [(1, 7, 16, False), (1, 8, 13, False), (1, 8, 13, True), (0, 16, 13, False)])
+def test_dequant_tables_in_shared_memory(ctx, oracle, variant, per_row, kmax, wide_row):
+    """Slots enough a thread block for the tables to be brought there; a row that does not fit a word keeps them in memory."""
+    case = dequant_case(7 + per_row, variant, 256, 256, per_row, kmax, 1, 0, False)
+    if wide_row:
+        case["norm3"].reshape(-1, 3)[300] = (256, 65536, 1)
+    got = run_dequant(ctx, case)
+    want = oracle.witness_dequant(case["acc"], case["jx"], case["jw"], case["sx"], case["sw"], case["norm3"], case["mul2"], case["n_base"], case["n_pre"], case["cfg"])
+    want["want"][:] = 0
+    for k in ("counts", "m_norm", "m_frac", "m_mul", "m_r8", "pre", "base"):
+        assert np.array_equal(got[k], want[k]), k

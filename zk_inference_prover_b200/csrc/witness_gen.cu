@@ -135,11 +135,16 @@ __global__ void tables_patch_kernel(const uint32_t* __restrict__ idx, const uint
 // writes 128 consecutive bytes of every column it touches; the accumulators of a row's slots are
 // consecutive in memory, so a thread walks one or two sectors of them. Multiplicities: the 8-bit range table is a
 // shared-memory histogram, the three large tables go through counters in shared memory too (count_cache.cuh), so one CTA an
-// SM takes units until none are left. 2^17 rows of 16 slots: 230 us with the large tables' counts as warp-merged atomics.
+// SM takes units until none are left. A random row of a table in memory is a line a lane, so the LSU's data path was what bounded it (79 % busy): where a CTA has slots
+// enough, the normalisation table is in shared memory, a word a row, and the product table, 16 bits a row. 2^17 rows of 16 slots: 230 us with the large
+// tables' counts as warp-merged atomics, 88 us with the counters, 67 us with the tables, a counter a row of the fraction table and 32-bit arithmetic.
 // ---------------------------------------------------------------------------------------------------
-constexpr int DEQ_THREADS = 1024, DEQ_NORM_LOG = 13, DEQ_FRAC_LOG = 12, DEQ_MUL_LOG = 14;
+constexpr int DEQ_THREADS = 1024, DEQ_NORM_LOG = 13, DEQ_FRAC_LOG = 14, DEQ_MUL_LOG = 14;
 constexpr uint32_t DEQ_COUNT_WORDS = (1u << DEQ_NORM_LOG) + (1u << DEQ_FRAC_LOG), DEQ_CHAIN_WORDS = DEQ_COUNT_WORDS + (1u << DEQ_MUL_LOG);
-constexpr uint32_t DEQ_POINTERS = 6144;  // column addresses kept in shared memory (48 KB); a wider component reads them from the table
+// From how many slots a CTA on the tables are brought to shared memory too, which takes some 3 us. 2^17 rows of 16 slots, 14,000 a CTA: 83 us without,
+// 70 with; of four, 3,500: 29.7, 27.9; 2^14 rows of 16, 1,800: 19.0, 20.7.
+constexpr uint32_t DEQ_STAGE_SLOTS = 3072;
+constexpr uint32_t DEQ_SMEM = 227 * 1024;  // counters first, then the normalisation table and the column addresses as far as there is room for each
 struct DeqArgs {
     const int32_t *acc, *jx, *jw;
     const uint32_t *sx, *sw, *norm3, *mul2;
@@ -147,7 +152,7 @@ struct DeqArgs {
     uint32_t* const* pre;
     uint32_t *m_norm, *m_frac, *m_mul, *m_r8, *counts, *want;
     zkb_dequant_cfg c;
-    uint32_t slot_tile, tiles, flush_every;
+    uint32_t slot_tile, tiles, flush_every, pointers_staged, norm_staged, mul_staged;
 };
 
 __device__ __forceinline__ uint32_t bf16_bits(uint32_t sg, uint32_t ef, uint32_t m7) { return ((sg << 15) | (ef << 7) | m7) & 0xffffu; }
@@ -166,24 +171,54 @@ __device__ __forceinline__ uint32_t bf16_round_f64(double x) {
     return bf16_bits((uint32_t)(u >> 63), (uint32_t)(e + 127), (uint32_t)keep);
 }
 
+// The same of 32 bits: two folds are a selection there.
+__device__ __forceinline__ uint32_t m31_of_word(int32_t v) {
+    if (v == INT32_MIN) return P - 1u;  // -(p + 1)
+    const uint32_t u = v < 0 ? (uint32_t)v + P : (uint32_t)v;
+    return u == P ? 0u : u;
+}
+__device__ __forceinline__ uint32_t m31_of_small(long long v) { return v == (int32_t)v ? m31_of_word((int32_t)v) : m31_of(v); }
+
 template <int CHAIN>
 __global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_constant__ DeqArgs a) {
     extern __shared__ __align__(16) uint32_t deq_sm[];
     const zkb_dequant_cfg& c = a.c;
     uint32_t *const norm_counts = deq_sm, *const frac_counts = deq_sm + (1u << DEQ_NORM_LOG), *const mul_counts = deq_sm + DEQ_COUNT_WORDS;
     uint32_t* const r8_hist = deq_sm + (CHAIN ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS);
-    for (uint32_t k = threadIdx.x; k < (CHAIN ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS) + c.n_r8; k += blockDim.x) deq_sm[k] = 0;
+    const bool norm_whole = count_is_whole<DEQ_NORM_LOG>({a.m_norm, c.n_norm}), frac_whole = count_is_whole<DEQ_FRAC_LOG>({a.m_frac, c.n_frac});
+    const bool mul_whole = count_is_whole<DEQ_MUL_LOG>({a.m_mul, c.n_mul});
+    count_clear<DEQ_NORM_LOG>(norm_counts, norm_whole, threadIdx.x, DEQ_THREADS);
+    count_clear<DEQ_FRAC_LOG>(frac_counts, frac_whole, threadIdx.x, DEQ_THREADS);
+    if (CHAIN) count_clear<DEQ_MUL_LOG>(mul_counts, mul_whole, threadIdx.x, DEQ_THREADS);
+    for (uint32_t k = threadIdx.x; k < c.n_r8; k += DEQ_THREADS) r8_hist[k] = 0;
+    uint32_t* more = r8_hist + ((c.n_r8 + 3u) & ~3u);
     // The column addresses, once per CTA: every store of every thread would otherwise start with a dependent read of the pointer table.
     const uint32_t n_base = c.per_row * c.per_slot, n_pre = c.per_row * c.chan_w;
     uint32_t* const* p_base = a.base + c.slot0;
     uint32_t* const* p_pre = a.pre;
-    if (n_base + n_pre <= DEQ_POINTERS) {
-        uint32_t** const p = reinterpret_cast<uint32_t**>(r8_hist + ((c.n_r8 + 3u) & ~3u));  // [slot][field], then [slot][scale column]
+    if (a.pointers_staged) {
+        uint32_t** const p = reinterpret_cast<uint32_t**>(more);  // [slot][field], then [slot][scale column]
         for (uint32_t k = threadIdx.x; k < n_base + n_pre; k += blockDim.x) p[k] = k < n_base ? p_base[k] : p_pre[k - n_base];
         p_base = p;
         p_pre = p + n_base;
+        more += 2 * (n_base + n_pre);
     }
-    __syncthreads();
+    bool fits = a.norm_staged;
+    if (fits)
+        for (uint32_t k = threadIdx.x; k < c.n_norm; k += DEQ_THREADS) fits = pack_norm(a.norm3, k, more[k]) && fits;
+    const uint32_t* const norm_sm = __syncthreads_and(fits) ? more : nullptr;
+    const uint16_t* mul_sm = nullptr;
+    if (CHAIN && a.mul_staged) {
+        uint16_t* const rows16 = reinterpret_cast<uint16_t*>(more + (a.norm_staged ? c.n_norm : 0u));
+        fits = true;
+#pragma unroll 4
+        for (uint32_t k = threadIdx.x; k < c.n_mul; k += DEQ_THREADS) {
+            const uint32_t po = __ldg(a.mul2 + 2u * k), ca = __ldg(a.mul2 + 2u * k + 1u);
+            rows16[k] = (uint16_t)(po | ca << 15);
+            fits = fits && po < 32768u && ca < 2u;
+        }
+        if (__syncthreads_and(fits)) mul_sm = rows16;
+    }
     auto flush = [&] {
         count_flush<DEQ_NORM_LOG>(norm_counts, a.m_norm, threadIdx.x, DEQ_THREADS);
         count_flush<DEQ_FRAC_LOG>(frac_counts, a.m_frac, threadIdx.x, DEQ_THREADS);
@@ -230,20 +265,19 @@ __global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_co
                 jw_c = __ldg(a.jw + ch);
                 pcol[0][i] = m31_of(jw_c);
             }
-            const long long av = __ldg(acc_row + s);
-            col[c.f_acc][i] = m31_of(av);
-            const uint32_t sg = av < 0;
-            const unsigned long long mag = (unsigned long long)(av < 0 ? -av : av);
+            const int32_t av = __ldg(acc_row + s);
+            const uint32_t sg = av < 0, mag = sg ? 0u - (uint32_t)av : (uint32_t)av;
+            col[c.f_acc][i] = m31_of_word(av);
             // mag = m2 * ph + r with a 9-bit extended significand m2 (prover/src/bf16.rs:300-316)
             uint32_t m2 = 0, ph = 0, st = 0, k = 0;
-            unsigned long long r = 0;
+            uint32_t r = 0;
             if (mag) {
-                uint32_t bits = 64u - (uint32_t)__clzll((long long)mag);
+                const uint32_t bits = 32u - (uint32_t)__clz((int)mag);
                 k = bits > 9u ? bits - 9u : 0u;
-                ph = 1u << (k & 31u);
-                m2 = (uint32_t)(mag >> k);
-                r = mag & ((1ull << k) - 1ull);
-                st = (r != 0ull) && c.sticky;
+                ph = 1u << k;
+                m2 = mag >> k;
+                r = mag & (ph - 1u);
+                st = r != 0u && c.sticky;
             }
             // row indices of the normalisation and fraction tables (prover/src/layer.rs:2042-2068)
             uint32_t ri = NONE, fi = NONE;
@@ -251,17 +285,23 @@ __global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_co
                 if (!mag) ri = 0;
                 else if (m2 < 256u) ri = m2;  // then k = 0, ph = 1, r = 0
                 else ri = 256u + (k * 256u + (m2 - 256u)) * (1u + c.sticky) + st;
-                fi = ph + (uint32_t)r;
+                fi = ph + r;
             }
             if (ri >= c.n_norm || fi >= c.n_frac) { no_row++; continue; }
-            const uint32_t n_m7 = __ldg(a.norm3 + 3u * ri), n_ef = __ldg(a.norm3 + 3u * ri + 1u), n_nz = __ldg(a.norm3 + 3u * ri + 2u);
-            count_cached<DEQ_NORM_LOG>(norm_counts, a.m_norm, ri);
-            count_cached<DEQ_FRAC_LOG>(frac_counts, a.m_frac, fi);
+            uint32_t n_m7, n_ef, n_nz;
+            if (norm_sm) {
+                const uint32_t w = norm_sm[ri];
+                n_m7 = w & 255u; n_ef = w >> 8 & 65535u; n_nz = w >> 24;
+            } else {
+                n_m7 = __ldg(a.norm3 + 3u * ri); n_ef = __ldg(a.norm3 + 3u * ri + 1u); n_nz = __ldg(a.norm3 + 3u * ri + 2u);
+            }
+            count_cached<DEQ_NORM_LOG>(norm_counts, a.m_norm, ri, norm_whole);
+            count_cached<DEQ_FRAC_LOG>(frac_counts, a.m_frac, fi, frac_whole);
             col[c.f_sg][i] = sg;
             col[c.f_m2][i] = m2;
             col[c.f_ph][i] = ph;
             if (c.sticky) col[c.f_st][i] = st;
-            col[c.f_r][i] = (uint32_t)r;
+            col[c.f_r][i] = r;
             col[c.f_m7][i] = n_m7;
             col[c.f_ef][i] = n_ef;
             col[c.f_nz][i] = n_nz;
@@ -269,7 +309,7 @@ __global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_co
             if (!CHAIN) {
                 const long long shift = (long long)jx_t + jw_c;
                 const long long eo = n_nz == 1u ? (long long)n_ef + shift : 0;
-                col[c.f_eo][i] = m31_of(eo);
+                col[c.f_eo][i] = m31_of_small(eo);
                 if (eo >= 0 && eo < (long long)c.n_r8) atomicAdd(&r8_hist[eo], 1u); else off_table++;
                 got = bf16_bits(sg, (uint32_t)(eo > 0 ? eo : 0), n_m7);
                 if (c.do_ref) {
@@ -287,12 +327,13 @@ __global__ void __launch_bounds__(DEQ_THREADS, 1) dequant_kernel(const __grid_co
                     const uint32_t mi = m_in * 128u + ms;
                     if (mi >= c.n_mul) { no_row++; break; }
                     uint32_t po = 0, ca = 0;
-                    if (n_nz == 1u) { po = __ldg(a.mul2 + 2u * mi); ca = __ldg(a.mul2 + 2u * mi + 1u); }
+                    if (n_nz == 1u && mul_sm) { po = mul_sm[mi] & 32767u; ca = mul_sm[mi] >> 15; }
+                    else if (n_nz == 1u) { po = __ldg(a.mul2 + 2u * mi); ca = __ldg(a.mul2 + 2u * mi + 1u); }
                     const long long eo = n_nz == 1u ? e_in + es - 127 + (long long)ca : 0;
                     col[c.f_mul[3u * step + 0u]][i] = po;
                     col[c.f_mul[3u * step + 1u]][i] = ca;
-                    col[c.f_mul[3u * step + 2u]][i] = m31_of(eo);
-                    if (n_nz == 1u) count_cached<DEQ_MUL_LOG>(mul_counts, a.m_mul, mi);
+                    col[c.f_mul[3u * step + 2u]][i] = m31_of_small(eo);
+                    if (n_nz == 1u) count_cached<DEQ_MUL_LOG>(mul_counts, a.m_mul, mi, mul_whole);
                     if (eo >= 0 && eo < (long long)c.n_r8) atomicAdd(&r8_hist[eo], 1u); else off_table++;
                     m_in = po;
                     e_in = eo;
@@ -395,14 +436,19 @@ int zkb_witness_dequant(zkb_ctx* ctx, const int32_t* acc, const int32_t* jx, con
     const uint32_t tiles = (c.per_row + slot_tile - 1) / slot_tile;
     // a counter holds 2^27 - 1, and a unit counts at most twice per slot
     DeqArgs a{acc, jx, jw, sx, sw, norm3, mul2, (uint32_t* const*)d_base, (uint32_t* const*)d_pre, m_norm, m_frac, m_mul, m_r8, counts,
-              want_out, c, slot_tile, tiles, (1u << 26) / (DEQ_THREADS * 2u * slot_tile)};
+              want_out, c, slot_tile, tiles, (1u << 26) / (DEQ_THREADS * 2u * slot_tile), 0u, 0u, 0u};
     const uint32_t grid = (uint32_t)std::min<uint64_t>(((uint64_t)rows * tiles + DEQ_THREADS - 1) / DEQ_THREADS, 148u);
     const uint64_t pointers = (uint64_t)c.per_row * (c.per_slot + c.chan_w);
-    const size_t smem = (size_t)((c.variant == 1 ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS) + ((c.n_r8 + 3u) & ~3u)) * 4 + (pointers <= DEQ_POINTERS ? 8 * pointers : 0);
+    uint64_t smem = (uint64_t)((c.variant == 1 ? DEQ_CHAIN_WORDS : DEQ_COUNT_WORDS) + ((c.n_r8 + 3u) & ~3u)) * 4;
+    auto room_for = [&](uint64_t bytes) { return smem + bytes <= DEQ_SMEM ? (smem += bytes, 1u) : 0u; };
+    a.pointers_staged = room_for(8 * pointers);
+    const bool many = (uint64_t)rows * c.per_row >= (uint64_t)grid * DEQ_STAGE_SLOTS;
+    a.norm_staged = many ? room_for(4ull * c.n_norm) : 0u;
+    a.mul_staged = many && c.variant == 1 ? room_for(2ull * c.n_mul) : 0u;
     ProfScope prof(ctx, "witness_dequant_kernel");
     auto launch = [&](auto kernel) {
         // the most any call takes: another thread's call must not lower it in between
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * (DEQ_CHAIN_WORDS + 8192) + 8 * DEQ_POINTERS));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEQ_SMEM);
         if (e == cudaSuccess) kernel<<<grid, DEQ_THREADS, smem, ctx->stream>>>(a);
         return e;
     };

@@ -211,18 +211,20 @@ __device__ __forceinline__ void lookup(const RsMult& t, uint32_t idx, uint32_t& 
     if (idx >= t.n) off++; else count_in_memory(t.m, idx);
 }
 template <int LOG>
-__device__ __forceinline__ void lookup(uint32_t* cache, const RsMult& t, uint32_t idx, uint32_t& off) {
-    if (idx >= t.n) off++; else count_cached<LOG>(cache, t.m, idx);
+__device__ __forceinline__ void lookup(uint32_t* cache, const RsMult& t, uint32_t idx, uint32_t& off, bool whole = false) {
+    if (idx >= t.n) off++; else count_cached<LOG>(cache, t.m, idx, whole);
 }
-__device__ __forceinline__ uint32_t value_index(long long sm, long long ef) {  // val_table's row order: zero, then (ef, m7, sign)
+template <class I>
+__device__ __forceinline__ uint32_t value_index(I sm, I ef) {  // val_table's row order: zero, then (ef, m7, sign)
     if (sm == 0 && ef == 0) return 0;
-    unsigned long long a = (unsigned long long)(sm < 0 ? -sm : sm);
+    const I a = sm < 0 ? -sm : sm;
     if (ef <= 0 || ef >= 0xff || a < 128 || a >= 256) return OFF_TABLE;
     return 1u + (((uint32_t)ef - 1u) * 128u + (uint32_t)(a - 128)) * 2u + (sm < 0 ? 1u : 0u);
 }
-__device__ __forceinline__ uint32_t pow_index(long long u) {  // [0, DMAX], then [-UMIN, -1]
-    if (u >= 0 && u <= (long long)RS_DMAX) return (uint32_t)u;
-    if (u < 0 && u >= -(long long)RS_UMIN) return RS_DMAX + (uint32_t)(-u);
+template <class I>
+__device__ __forceinline__ uint32_t pow_index(I u) {  // [0, DMAX], then [-UMIN, -1]
+    if (u >= 0 && u <= (I)RS_DMAX) return (uint32_t)u;
+    if (u < 0 && u >= -(I)RS_UMIN) return RS_DMAX + (uint32_t)(-u);
     return OFF_TABLE;
 }
 __device__ __forceinline__ uint32_t signed_significand_index(long long v) {
@@ -239,15 +241,73 @@ __device__ __forceinline__ uint32_t* column(const RsArgs& a, uint32_t c) {
     if (EVEN) return a.col0 + (long long)c * a.col_step;
     return reinterpret_cast<uint32_t*>(__ldg(reinterpret_cast<const unsigned long long*>(a.cols) + c));
 }
-// An operand as the (significand, exponent) it encodes. A slot's output exponent is clamped to [0, 0xfe] on the way
+// A cell as the exponent it encodes, negative ones as 0: no larger than 2^31 for any word, so no sign is needed.
+__device__ __forceinline__ uint32_t exponent_of(uint32_t v) { return v <= P / 2 ? v : v < P ? 0u : v - P; }
+// An operand's words: its significand cell, and the exponent it encodes. A slot's output exponent is clamped to [0, 0xfe] on the way
 // out of the slot while its cell keeps the unclamped value, so the clamp applies to slot sources only.
+struct RsOperand {
+    uint32_t sm, ef;
+    __device__ __forceinline__ int small_sm() const { return (int)(sm <= P / 2 ? sm : sm - P); }  // of an operand that is_small
+    __device__ __forceinline__ bool is_small() const { return (uint32_t)(small_sm() + (1 << 17)) < (2u << 17) && ef < (1u << 20); }
+};
 template <bool EVEN>
-__device__ __forceinline__ void operand(const RsArgs& a, uint32_t i, uint32_t c_sm, uint32_t c_ef, bool from_slot, long long& sm, long long& ef) {
-    if (c_sm == OFF_TABLE) { sm = 0; ef = 0; return; }
-    const uint32_t *p_sm = column<EVEN>(a, c_sm), *p_ef = column<EVEN>(a, c_ef);
-    sm = signed_of(p_sm[i]);
-    long long e = signed_of(p_ef[i]);
-    ef = e < 0 ? 0 : (from_slot && e > 0xfe) ? 0xfe : e;
+__device__ __forceinline__ RsOperand operand(const RsArgs& a, uint32_t i, uint32_t c_sm, uint32_t c_ef, bool from_slot) {
+    if (c_sm == OFF_TABLE) return {0u, 0u};
+    const uint32_t e = exponent_of(column<EVEN>(a, c_ef)[i]);
+    return {column<EVEN>(a, c_sm)[i], from_slot ? umin32(e, 0xfeu) : e};
+}
+
+// What an addition writes and which rows of the tables it looks up.
+struct RsAddition { uint32_t fa, fb, etop, mag, sg, m2, ph, r, st, m7, ef, nz, c_sm, c_ef, pa, pb, ni, frac, val, lost, bad_exp; };
+// Both operands aligned to the larger exponent (a shift of up to DMAX bits is kept, a smaller operand is dropped), added, the magnitude normalised
+// to a 9-bit M2 with its round-bit weight ph, rounded through the table. In 32 bits for operands that are small (a significand below 2^17 times
+// 2^DMAX) and table rows of less than 2^16, which are all that well-formed tables and cells hold; false for other rows. In 64 bits for any.
+template <class I, bool STICKY>
+__device__ __forceinline__ bool add_slot(const RsArgs& a, I a_sm, I a_ef, I b_sm, I b_ef, RsAddition& o) {
+    constexpr bool WIDE = sizeof(I) == 8;
+    const I etop = a_ef > b_ef ? a_ef : b_ef, ua = a_ef - etop + (I)RS_DMAX, ub = b_ef - etop + (I)RS_DMAX;
+    o.pa = pow_index(ua);
+    o.pb = pow_index(ub);
+    o.fa = ua >= 0 ? 1u << ua : 0u;
+    o.fb = ub >= 0 ? 1u << ub : 0u;
+    const I acc = a_sm * (I)o.fa + b_sm * (I)o.fb, mag = acc < 0 ? -acc : acc;
+    I r = 0;
+    uint32_t k = 0;
+    o.sg = acc < 0;
+    o.m2 = o.ph = o.st = o.lost = 0;
+    if (mag) {
+        const uint32_t bits = WIDE ? 64u - (uint32_t)__clzll((long long)mag) : 32u - (uint32_t)__clz((int)mag);
+        k = bits > 9u ? bits - 9u : 0u;
+        if (k > a.kmax) o.lost = 1;  // a round-bit weight the table does not carry
+        else { o.ph = 1u << k; o.m2 = (uint32_t)(mag >> k); r = mag & (((I)1 << k) - 1); o.st = STICKY && r != 0; }
+    }
+    // the normalisation table's row: zero row, 255 exact small magnitudes, then (k, m2, st) ascending
+    if (o.m2 == 0 && o.ph == 0) o.ni = 0;
+    else if (o.ph == 1 && o.m2 < 256u) o.ni = o.m2;
+    else if (o.m2 >= 256u && o.m2 < 512u) o.ni = 256u + (k * 256u + (o.m2 - 256u)) * (STICKY ? 2u : 1u) + o.st;
+    else o.ni = OFF_TABLE;
+    o.m7 = o.ef = o.nz = 0;
+    if (o.ni >= a.n_norm) o.lost++;
+    else {
+        o.m7 = __ldg(a.norm3 + 3 * (size_t)o.ni); o.ef = __ldg(a.norm3 + 3 * (size_t)o.ni + 1); o.nz = __ldg(a.norm3 + 3 * (size_t)o.ni + 2);
+        if (!WIDE && (o.m7 >= 1u << 16 || o.ef >= 1u << 16 || o.nz >= 256u)) return false;
+    }
+    o.frac = o.ph == 0 ? (r == 0 ? 0u : OFF_TABLE) : o.ph + (uint32_t)r;
+    const I c_sm = (I)(128u * o.nz + o.m7) * (o.sg ? -1 : 1), c_ef = o.nz == 1 ? (I)o.ef + etop - (I)(RS_DMAX + RS_BIAS) : 0;
+    o.bad_exp = o.nz == 1 && !(c_ef >= 1 && c_ef < 0xff);
+    o.val = (c_ef >= 0 && c_ef < 0xff) ? value_index(c_sm, c_ef) : OFF_TABLE;  // the slot's own output is a looked-up pair too
+    if (WIDE) {
+        o.etop = field_of(etop); o.mag = field_of(mag); o.r = field_of(r); o.c_sm = field_of(c_sm); o.c_ef = field_of(c_ef);
+    } else {
+        o.etop = (uint32_t)etop; o.mag = (uint32_t)mag; o.r = (uint32_t)r;
+        o.c_sm = c_sm < 0 ? (uint32_t)(c_sm + (I)P) : (uint32_t)c_sm;
+        o.c_ef = c_ef < 0 ? (uint32_t)(c_ef + (I)P) : (uint32_t)c_ef;
+    }
+    return true;
+}
+template <bool STICKY>
+__device__ __noinline__ void add_slot_wide(const RsArgs& a, RsOperand x, RsOperand y, RsAddition* o) {
+    add_slot<long long, STICKY>(a, signed_of(x.sm), (long long)x.ef, signed_of(y.sm), (long long)y.ef, *o);
 }
 
 // A team of warps owns 32 consecutive committed rows at a time: lane = row, so that every column access of a warp is one 128-byte
@@ -256,22 +316,31 @@ __device__ __forceinline__ void operand(const RsArgs& a, uint32_t i, uint32_t c_
 // another warp of the team wrote.
 //
 // What bounded it were the counts (count_cache.cuh), then the latency of a slot, a chain of loads (its record, the operands' cells, a
-// row of the table) before its stores. So one CTA an SM keeps the counters and takes rows until none are left, in two teams of sixteen
-// warps; column addresses are computed where they can be (fourteen of them were 28 registers), four leaves are loaded at a time.
-// 2^15 rows of 128 additions: 690 us with the counts as atomics in L2, 257 us with them in shared memory, 206 us with four leaves or
-// outputs of a row to an access.
+// row of the table) before its stores, then its instructions, 990 a slot with its two leaves. So one CTA an SM keeps the counters and takes rows until none
+// are left, in two teams of sixteen warps; column addresses are computed where they can be (fourteen of them were 28 registers), four leaves are loaded at a
+// time, additions are worked out in 32 bits, the power table's one busy row is counted in a register, tables that have a counter a row need no tags (of the
+// fraction table's 2^14 rows a third of the lookups went to memory while they shared 2^12 counters), a slot's operands are asked for a slot before.
+// 2^15 rows of 128 additions: 690 us with the counts as atomics in L2, 257 us with them in shared memory, 204 us with four leaves or outputs of a row to
+// an access, 170 us as it is now (650 instructions a slot, issue slots at 46 %, the LSU's data path too). The normalisation table in shared memory, a word
+// a row, gained nothing (173). 2^13 rows: 53 -> 48 us; four teams of eight warps instead of two of sixteen: 193.
 constexpr uint32_t RS_LANES = 16, RS_TEAMS = 2, RS_LEAVES = 4;
-constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 12, RS_SMUL_LOG = 14;
+constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 14, RS_SMUL_LOG = 14;
 constexpr uint32_t RS_ADD_WORDS = (1u << RS_VAL_LOG) + (1u << RS_NORM_LOG) + (1u << RS_FRAC_LOG), RS_MUL_WORDS = (1u << RS_VAL_LOG) + (1u << RS_SMUL_LOG);
 template <bool MUL, bool STICKY, bool EVEN>
 __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_kernel(const __grid_constant__ RsArgs a) {
-    // The power table has 273 rows and every addition hits row DMAX with its larger operand: counted per CTA in shared
-    // memory and added to the global array once at the end (one hot address would serialise every warp of the grid).
+    // The power table has 273 rows and every addition hits row DMAX with its larger operand: that row is counted in a register, the others per CTA in
+    // shared memory, and added to the global array once at the end.
     __shared__ uint32_t pow_hist[RS_POW_ROWS];
-    extern __shared__ uint32_t counts_sm[];
+    extern __shared__ __align__(16) uint32_t counts_sm[];
     uint32_t *const val_counts = counts_sm, *const norm_counts = counts_sm + (1u << RS_VAL_LOG), *const frac_counts = norm_counts + (1u << RS_NORM_LOG);
     uint32_t* const smul_counts = norm_counts;  // a program adds or multiplies
-    for (uint32_t k = threadIdx.x; k < (MUL ? RS_MUL_WORDS : RS_ADD_WORDS); k += blockDim.x) counts_sm[k] = 0;
+    const bool norm_whole = count_is_whole<RS_NORM_LOG>(a.m_norm), frac_whole = count_is_whole<RS_FRAC_LOG>(a.m_frac);
+    count_clear<RS_VAL_LOG>(val_counts, false, threadIdx.x, blockDim.x);
+    if (MUL) count_clear<RS_SMUL_LOG>(smul_counts, false, threadIdx.x, blockDim.x);
+    else {
+        count_clear<RS_NORM_LOG>(norm_counts, norm_whole, threadIdx.x, blockDim.x);
+        count_clear<RS_FRAC_LOG>(frac_counts, frac_whole, threadIdx.x, blockDim.x);
+    }
     for (uint32_t k = threadIdx.x; k < RS_POW_ROWS; k += blockDim.x) pow_hist[k] = 0;
     __syncthreads();
     auto flush = [&](uint32_t thread, uint32_t threads) {
@@ -284,8 +353,9 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
     };
     const uint32_t lanes = blockDim.x / (32u * a.teams), team = (threadIdx.x >> 5) / lanes, t = (threadIdx.x >> 5) - team * lanes;
     auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1u), "r"(32u * lanes) : "memory"); };
-    uint32_t off = 0, bad_exp = 0, un_off = 0, since_flush = 0;
-    for (uint32_t block = blockIdx.x * a.teams + team; (block << 5 >> a.log_rows) == 0; block += gridDim.x * a.teams) {
+    uint32_t off = 0, bad_exp = 0, un_off = 0, top = 0, since_flush = 0;
+    // (a CTA's first team takes its rows before any CTA's second: what is left for a last pass is one team's a CTA)
+    for (uint32_t block = blockIdx.x + gridDim.x * team; (block << 5 >> a.log_rows) == 0; block += gridDim.x * a.teams) {
     const uint32_t i = block * 32u + (threadIdx.x & 31u);
     const bool in_range = (i >> a.log_rows) == 0;
     const uint32_t j = in_range ? committed_to_natural(i, a.log_rows) : 0u;
@@ -324,7 +394,7 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
                 if (!four) reinterpret_cast<int2*>(a.in_nat)[at + u] = make_int2(sm, (int)ef);
                 else if (u & 1) reinterpret_cast<int4*>(a.in_nat)[(at + u) >> 1] = make_int4(held.x, held.y, sm, (int)ef);
                 else held = make_int2(sm, (int)ef);
-                const uint32_t v = value_index(sm, ef);
+                const uint32_t v = value_index(sm, (int)ef);
                 if (gr.un == 0) { lookup<RS_VAL_LOG>(val_counts, a.m_val, v, off); continue; }
                 uint32_t *c2 = column<EVEN>(a, b + 2), *c3 = column<EVEN>(a, b + 3);
                 lookup(a.m_un[gr.un - 1], v, off);
@@ -339,84 +409,67 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
 
     for (uint32_t level = 0; level < a.n_levels; level++) {
       team_sync();
-      if (in_range)
-      for (uint32_t at = a.level_start[level] + t; at < a.level_start[level + 1]; at += lanes) {
-        const RsSlot sl = a.slots[at];
-        long long a_sm, a_ef, b_sm, b_ef, c_sm, c_ef;
-        operand<EVEN>(a, i, sl.a_sm, sl.a_ef, sl.from_slot & 1u, a_sm, a_ef);
-        operand<EVEN>(a, i, sl.b_sm, sl.b_ef, sl.from_slot & 2u, b_sm, b_ef);
-        const uint32_t b = sl.base;
-        constexpr uint32_t W = MUL ? 4u : (STICKY ? 14u : 13u);
-        uint32_t* held[W];
-#pragma unroll
-        for (uint32_t k = 0; k < W; k++) held[k] = EVEN ? nullptr : column<EVEN>(a, b + k);
+      if (!in_range) continue;
+      // A slot's operands are cells of levels before: the next slot's are on their way while this one is worked out, and the record after it.
+      const uint32_t end = a.level_start[level + 1];
+      uint32_t at = a.level_start[level] + t;
+      if (at >= end) continue;
+      RsSlot sl = a.slots[at];
+      RsOperand x = operand<EVEN>(a, i, sl.a_sm, sl.a_ef, sl.from_slot & 1u), y = operand<EVEN>(a, i, sl.b_sm, sl.b_ef, sl.from_slot & 2u);
+      uint32_t b = sl.base;
+      if (at + lanes < end) sl = a.slots[at + lanes];
+      while (true) {
+        RsOperand next_x{0u, 0u}, next_y{0u, 0u};
+        const uint32_t next_b = sl.base;
+        if (at + lanes < end) {
+            next_x = operand<EVEN>(a, i, sl.a_sm, sl.a_ef, sl.from_slot & 1u);
+            next_y = operand<EVEN>(a, i, sl.b_sm, sl.b_ef, sl.from_slot & 2u);
+        }
+        if (at + 2 * lanes < end) sl = a.slots[at + 2 * lanes];
         uint32_t* const first = EVEN ? column<EVEN>(a, b) + i : nullptr;
-        auto put = [&](uint32_t k, uint32_t v) { (EVEN ? first + (long long)k * a.col_step : held[k] + i)[0] = v; };
+        auto put = [&](uint32_t k, uint32_t v) { (EVEN ? first + (long long)k * a.col_step : column<EVEN>(a, b + k) + i)[0] = v; };
         if (!MUL) {
-            // align both operands to the larger exponent (a shift of up to DMAX bits is kept, a smaller operand is dropped),
-            // add, normalise the magnitude to a 9-bit M2 with its round-bit weight ph, round through the table
-            const long long etop = a_ef > b_ef ? a_ef : b_ef;
-            const long long ua = a_ef - etop + RS_DMAX, ub = b_ef - etop + RS_DMAX;
-            const uint32_t pa = pow_index(ua), pb = pow_index(ub);
-            if (pa < a.m_pow.n) atomicAdd(pow_hist + pa, 1u); else off++;
-            if (pb < a.m_pow.n) atomicAdd(pow_hist + pb, 1u); else off++;
-            const long long fa = (pa != OFF_TABLE && ua >= 0) ? (1LL << ua) : 0, fb = (pb != OFF_TABLE && ub >= 0) ? (1LL << ub) : 0;
-            const long long acc = a_sm * fa + b_sm * fb;
-            const uint32_t sg = acc < 0;
-            const unsigned long long mag = (unsigned long long)(acc < 0 ? -acc : acc);
-            uint32_t m2 = 0, ph = 0, st = 0, k = 0;
-            unsigned long long r = 0;
-            if (mag) {
-                const uint32_t bits = 64u - (uint32_t)__clzll((long long)mag);
-                k = bits > 9u ? bits - 9u : 0u;
-                if (k > a.kmax) off++;  // a round-bit weight the table does not carry
-                else { ph = 1u << k; m2 = (uint32_t)(mag >> k); r = mag & ((1ull << k) - 1ull); st = STICKY && r != 0; }
+            RsAddition o;
+            if (!(x.is_small() && y.is_small() && add_slot<int, STICKY>(a, x.small_sm(), (int)x.ef, y.small_sm(), (int)y.ef, o))) {
+                RsAddition wide;
+                add_slot_wide<STICKY>(a, x, y, &wide);
+                o = wide;
             }
-            uint32_t ni;  // the normalisation table's row: zero row, 255 exact small magnitudes, then (k, m2, st) ascending
-            if (m2 == 0 && ph == 0) ni = 0;
-            else if (ph == 1 && m2 < 256u) ni = m2;
-            else if (m2 >= 256u && m2 < 512u) ni = 256u + (k * 256u + (m2 - 256u)) * (STICKY ? 2u : 1u) + st;
-            else ni = OFF_TABLE;
-            uint32_t m7n = 0, efn = 0, nzn = 0;
-            if (ni < a.n_norm) { m7n = __ldg(a.norm3 + 3 * (size_t)ni); efn = __ldg(a.norm3 + 3 * (size_t)ni + 1); nzn = __ldg(a.norm3 + 3 * (size_t)ni + 2); }
-            else off++;
-            lookup<RS_NORM_LOG>(norm_counts, a.m_norm, ni, off);
-            lookup<RS_FRAC_LOG>(frac_counts, a.m_frac, ph == 0 ? (r == 0 ? 0u : OFF_TABLE) : ph + (uint32_t)r, off);
-            c_sm = (long long)(128u * nzn + m7n) * (sg ? -1 : 1);
-            c_ef = nzn == 1 ? (long long)efn + etop - RS_DMAX - RS_BIAS : 0;
-            bad_exp += nzn == 1 && !(c_ef >= 1 && c_ef < 0xff);
-            put(0, field_of(fa));
-            put(1, field_of(fb));
-            put(2, field_of(etop));
-            put(3, field_of((long long)mag));
-            put(4, sg);
-            put(5, m2);
-            put(6, ph);
-            put(7, field_of((long long)r));
-            if (STICKY) put(8, st);
             constexpr uint32_t kk = STICKY ? 9u : 8u;
-            put(kk, m7n);
-            put(kk + 1, efn);
-            put(kk + 2, nzn);
-            put(kk + 3, field_of(c_sm));
-            put(kk + 4, field_of(c_ef));
+            put(0, o.fa); put(1, o.fb); put(2, o.etop); put(3, o.mag); put(4, o.sg); put(5, o.m2); put(6, o.ph); put(7, o.r);
+            if (STICKY) put(8, o.st);
+            put(kk, o.m7); put(kk + 1, o.ef); put(kk + 2, o.nz); put(kk + 3, o.c_sm); put(kk + 4, o.c_ef);
+            off += o.lost;
+            bad_exp += o.bad_exp;
+            for (const uint32_t u : {o.pa, o.pb}) {
+                if (u >= a.m_pow.n) off++;
+                else if (u == RS_DMAX) top++;
+                else atomicAdd(pow_hist + u, 1u);
+            }
+            lookup<RS_NORM_LOG>(norm_counts, a.m_norm, o.ni, off, norm_whole);
+            lookup<RS_FRAC_LOG>(frac_counts, a.m_frac, o.frac, off, frac_whole);
+            lookup<RS_VAL_LOG>(val_counts, a.m_val, o.val, off);
         } else {
             // the signed significands' correctly rounded product and binade carry come from one table row
-            const uint32_t ia = signed_significand_index(a_sm), ib = signed_significand_index(b_sm);
+            const uint32_t ia = signed_significand_index(signed_of(x.sm)), ib = signed_significand_index(signed_of(y.sm));
             const uint32_t si = (ia == OFF_TABLE || ib == OFF_TABLE) ? OFF_TABLE : ia * 257u + ib;
             int32_t prod = 0, cy = 0, nzc = 0;
             if (si < a.n_smul) { prod = __ldg(a.smul3 + 3 * (size_t)si); cy = __ldg(a.smul3 + 3 * (size_t)si + 1); nzc = __ldg(a.smul3 + 3 * (size_t)si + 2); }
             else off++;
             lookup<RS_SMUL_LOG>(smul_counts, a.m_smul, si, off);
-            c_sm = prod;
-            c_ef = nzc == 1 ? a_ef + b_ef + cy - 127 : 0;
+            const long long c_sm = prod, c_ef = nzc == 1 ? (long long)x.ef + y.ef + cy - 127 : 0;
             bad_exp += nzc == 1 && !(c_ef >= 1 && c_ef < 0xff);
             put(0, field_of(c_sm));
             put(1, (uint32_t)cy);
             put(2, (uint32_t)nzc);
             put(3, field_of(c_ef));
+            lookup<RS_VAL_LOG>(val_counts, a.m_val, (c_ef >= 0 && c_ef < 0xff) ? value_index(c_sm, c_ef) : OFF_TABLE, off);
         }
-        lookup<RS_VAL_LOG>(val_counts, a.m_val, (c_ef >= 0 && c_ef < 0xff) ? value_index(c_sm, c_ef) : OFF_TABLE, off);  // the slot's own output is a looked-up pair too
+        at += lanes;
+        if (at >= end) break;
+        x = next_x;
+        y = next_y;
+        b = next_b;
       }
     }
     team_sync();
@@ -432,10 +485,12 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
         for (uint32_t u = 0; u < 4; u++) {
             if (k0 + u >= a.out_w) break;
             const RsSlot sl = a.slots[a.out_slot[k0 + u]];
-            const long long sm = signed_of(column<EVEN>(a, sl.o_sm)[i]), e = signed_of(column<EVEN>(a, sl.o_ef)[i]);
-            const uint32_t ef = (uint32_t)(e < 0 ? 0 : e > 0xfe ? 0xfe : e);
+            // (as words: of the magnitude the low bits count, and what is below 0 is known from the cell)
+            const uint32_t c_sm = column<EVEN>(a, sl.o_sm)[i], c_ef = column<EVEN>(a, sl.o_ef)[i];
+            const uint32_t sm = c_sm > P / 2 ? c_sm - P : c_sm, e = c_ef > P / 2 ? c_ef - P : c_ef;
+            const bool negative = c_sm > P / 2 && c_sm < P;
             uint32_t pat = 0;
-            if (sm != 0) pat = ((sm < 0 ? 1u << 15 : 0u) | (ef << 7) | (uint32_t)((sm < 0 ? -sm : sm) - 128)) & 0xffffu;
+            if (sm != 0) pat = ((negative ? 1u << 15 : 0u) | (umin32(exponent_of(c_ef), 0xfeu) << 7) | ((negative ? 0u - sm : sm) - 128u)) & 0xffffu;
             pats[u] = pat;
             if (!four) {
                 a.out_pat[at + u] = pat;
@@ -459,10 +514,12 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
     if (!MUL)
         for (uint32_t k = threadIdx.x; k < RS_POW_ROWS && k < a.m_pow.n; k += blockDim.x)
             if (pow_hist[k]) atomicAdd(a.m_pow.m + k, pow_hist[k]);
+    top = __reduce_add_sync(0xffffffffu, top);
     off = __reduce_add_sync(0xffffffffu, off);
     bad_exp = __reduce_add_sync(0xffffffffu, bad_exp);
     un_off = __reduce_add_sync(0xffffffffu, un_off);
     if ((threadIdx.x & 31u) == 0) {
+        if (top) atomicAdd(a.m_pow.m + RS_DMAX, top);
         if (off) atomicAdd(a.counts, off);
         if (bad_exp) atomicAdd(a.counts + 1, bad_exp);
         if (un_off) atomicAdd(a.counts + 2, un_off);
@@ -684,7 +741,8 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     ProfScope prof(ctx, "residual_stream_kernel");
     cudaError_t e = cudaSuccess;
     auto launch = [&](auto kernel, uint32_t words) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * words));
+        // the most any call takes: another thread's call must not lower it in between
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * (p.kind == 1 ? RS_MUL_WORDS : RS_ADD_WORDS)));
         if (e == cudaSuccess) kernel<<<grid, threads, 4 * words, ctx->stream>>>(a);
     };
     if (p.kind == 1) even ? launch(residual_stream_kernel<true, false, true>, RS_MUL_WORDS) : launch(residual_stream_kernel<true, false, false>, RS_MUL_WORDS);
