@@ -58,6 +58,21 @@ def test_gkr_single_instance_a_round_ahead(ctx, oracle, kind, log_n, value):
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("log_n,n_inst", [(5, 431), (5, 432), (5, 433), (9, 365), (9, 377)])
+def test_gkr_batch_around_what_a_launch_carries(ctx, oracle, log_n, n_inst):
+    """16 + 64 rounds + 4 instances words of a layer's description: 2,000 at most go with the launch, more are copied."""
+    inst, dev, keep = [], [], []
+    for i in range(n_inst):
+        n = 1 << (log_n if i == 3 else 2 + i % 3)
+        den = qm31_array(7300 + i, n, nonzero=True)
+        inst.append((3, None, den))
+        keep.append(ctx.upload(den))
+        dev.append((3, 0, keep[-1].ptr, n))
+    want = oracle.gkr_prove(inst, 0x5EED0017, verify=True)
+    got = ctx.gkr_prove_device(dev, 0x5EED0017)
+    assert len(got) == len(want) and (got == want).all()
+
+
 @pytest.mark.parametrize("log_n", [2, 9, 10, 11, 12])
 def test_gkr_batch_around_the_tower_launches(ctx, oracle, log_n):
     inst, dev, keep = [], [], []

@@ -162,6 +162,20 @@ struct alignas(16) GkrStepState {
 };
 static_assert(sizeof(GkrStepState) % 16 == 0, "GkrStepState layout");
 
+// What of a layer's description depends on the transcript, in words: the channel (digest, n_draws), the first claim, the rounds' constants, the powers of
+// alpha. It is known last, so the launch carries it as a parameter where it fits (a copy before the launch is 3 us of host time, and
+// the launch behind it starts later: 34 instances of 2^10 ... 2^13 983 -> 950 us a proof); for many instances it is staged and copied.
+constexpr size_t OPEN_CLAIM = 12, OPEN_CONSTS = 16, OPEN_WORDS = 2000;
+struct alignas(16) GkrLayerOpen {
+    uint32_t words[OPEN_WORDS];
+};
+__host__ __device__ inline size_t open_alpha(int n_rounds) { return OPEN_CONSTS + 64 * (size_t)n_rounds; }
+// Word i of the state that a layer begins with.
+__device__ __forceinline__ uint32_t open_state_word(const uint32_t* open, int i) {
+    constexpr int claim = offsetof(GkrStepState, claim) / 4, corr = offsetof(GkrStepState, corr) / 4;
+    return i < 9 ? open[i] : i >= claim && i < claim + 4 ? open[OPEN_CLAIM + i - claim] : i >= corr && !((i - corr) & 3) ? 1u : 0u;
+}
+
 // The groups' sums of the round at hand, and zeros for the next: [2][groups][24] 64-bit words. Of a round whose challenge is known its two sums (t =
 // 0, t = 2); of one that is worked out ahead (look_pass) three pairs.
 constexpr int ACC_WORDS = 24;
@@ -584,12 +598,12 @@ __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* 
 }
 
 // Tables [first, end) of the layer; then, where look_from >= 0, the rounds from that on ahead of the transcript (the tables behind the n_rounds + 1 of the others) and
-// the masks; end is look_from + 1. rc: null where the transcript's steps are launches of their own (gkr_batch_step_kernel); no CTA then
-// keeps it, and the challenge is in its slot before the launch.
+// the masks; end is look_from + 1. keeps_transcript: zero where the transcript's steps are launches of their own (gkr_batch_step_kernel); no CTA then
+// keeps it, and the challenge is in its slot before the launch. copied: what the launch does not carry (GkrLayerOpen), or null.
 __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const GkrBatchItem* __restrict__ items_base, const GkrTable* __restrict__ tables, int first, int end,
-                                                                         const uint32_t* __restrict__ eq, qm31 lambda, const uint32_t* __restrict__ alpha_pow,
-                                                                         GkrStepState* st, GkrAcc acc, GkrSync* sync, const GkrStepConst* __restrict__ rc, int look_from,
-                                                                         uint32_t* records, int n_rounds, GkrLayerOut host) {
+                                                                         const uint32_t* __restrict__ eq, qm31 lambda, const __grid_constant__ GkrLayerOpen carried,
+                                                                         const uint32_t* copied, GkrStepState* st, GkrAcc acc, GkrSync* sync, int keeps_transcript,
+                                                                         int look_from, uint32_t* records, int n_rounds, GkrLayerOut host) {
     __shared__ uint32_t sums[GKR_GROUPS][2 * ACC_WORDS];  // of the pass at hand; zero before it
     __shared__ GkrTable tabs[2 * GKR_LAYER_MAX_ROUNDS + 1];
     __shared__ qm31 r_sh, eq_tab[EQ_TABLES][32];
@@ -599,13 +613,16 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
     __shared__ GkrStepState s;
     __shared__ GkrStepConst consts[GKR_LAYER_MAX_ROUNDS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool lead = blockIdx.x == 0 && rc;
+    const bool lead = blockIdx.x == 0 && keeps_transcript;
+    const uint32_t* const open = copied ? copied : carried.words;
+    const GkrStepConst* const rc = reinterpret_cast<const GkrStepConst*>(open + OPEN_CONSTS);
+    const uint32_t* const alpha_pow = open + open_alpha(n_rounds);
     for (int i = tid; i < 2 * (look_from >= 0 ? 2 * n_rounds + 1 : end); i += GKR_THREADS) reinterpret_cast<uint4*>(tabs)[i] = reinterpret_cast<const uint4*>(tables)[i];
     for (int i = tid; i < GKR_GROUPS * 2 * ACC_WORDS; i += GKR_THREADS) (&sums[0][0])[i] = 0u;
     if (tid == 0) gave_up = false;
     if (lead) {
         for (int i = tid; i < 16 * n_rounds; i += GKR_THREADS) reinterpret_cast<uint4*>(consts)[i] = reinterpret_cast<const uint4*>(rc)[i];
-        for (int i = tid; i < (int)(sizeof(s) / 4); i += GKR_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = reinterpret_cast<const uint32_t*>(st)[i];
+        for (int i = tid; i < (int)(sizeof(s) / 4); i += GKR_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = open_state_word(open, i);
     }
     // eq(., point) of a term's index: from a table, or, where there is none, as a product over the index's bits, five to a table of a warp's making
     // (bit k goes with coordinate n_rounds - 1 - k; the first coordinate's share is 1 - y)
@@ -856,10 +873,15 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
 }
 
 // The step after table t < n_rounds by itself, one warp; after the last table, what goes to the host.
-__global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, GkrAcc acc, GkrSync* sync, const GkrStepConst* __restrict__ rc, uint32_t* records, int t, int n_rounds,
+__global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, GkrAcc acc, GkrSync* sync, const uint32_t* __restrict__ open, uint32_t* records, int t, int n_rounds,
                                                             GkrLayerOut host) {
     __shared__ GkrStepSm sm;
     const int lane = threadIdx.x;
+    const GkrStepConst* const rc = reinterpret_cast<const GkrStepConst*>(open + OPEN_CONSTS);
+    if (t == 0) {
+        for (int i = lane; i < (int)(sizeof(*st) / 4); i += 32) reinterpret_cast<uint32_t*>(st)[i] = open_state_word(open, i);
+        __syncwarp();
+    }
     if (t == n_rounds) {
         layer_out_words(host, records, n_rounds, st, lane, 32);
         __threadfence_system();
@@ -1115,20 +1137,19 @@ int gkr_batch_round(zkb_ctx* ctx, GkrBatchItem* items, int n_items, const uint32
     return ZKB_OK;
 }
 
-// The block a layer's launch stages: the transcript's state, the CTAs' meeting place, the powers of alpha, the rounds' constants, the tables,
-// room for the rounds' records (every part a multiple of four words).
-struct LayerBlob { size_t acc, sync, alpha, rounds, tables, records, words; };
+// What is staged with a layer's items, in words: room for the transcript's state, the CTAs' meeting place (zero), the tables, room for the rounds' records (every
+// part a multiple of four words).
+struct LayerBlob { size_t acc, sync, tables, records, words; };
 static LayerBlob layer_blob(const GkrLayerPlan& plan) {
     LayerBlob o;
     o.acc = sizeof(GkrStepState) / 4;
     o.sync = o.acc + 2 * 2 * ACC_WORDS * (size_t)plan.n_rounds;
-    o.alpha = o.sync + sizeof(GkrSync) / 4;
-    o.rounds = o.alpha + 4 * plan.n_vars.size();
-    o.tables = o.rounds + (sizeof(GkrStepConst) / 4) * (size_t)plan.n_rounds;
+    o.tables = o.sync + sizeof(GkrSync) / 4;
     o.records = o.tables + plan.tables.size();
     o.words = o.records + GKR_LAYER_OUT_WORDS * (size_t)plan.n_rounds;
     return o;
 }
+static size_t open_words(const GkrLayerPlan& plan) { return open_alpha(plan.n_rounds) + 4 * plan.n_vars.size(); }
 
 // The rounds that are taken ahead of the transcript: from the first whose table takes four lanes a term. Larger ones are bound by their products, of which this
 // way has twice as many. Their tables go behind the others, and the items that are used into look_items.
@@ -1238,12 +1259,18 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
     // Rounds that take four and eight lanes a term can work eq out: a term a thread would take two products more for each of its six.
     plan.needs_eq = plan.look_from != 0 || tables_of(plan)[0].terms_log > 5 * EQ_TABLES;
     const std::vector<GkrBatchItem>& items = plan.look_from >= 0 ? plan.look_items : plan.items;
-    // What the launch stages later must not come to lie over the items: room for both.
-    const size_t item_bytes = items.size() * sizeof(GkrBatchItem);
-    if (int rc = stage_reserve(ctx, blob_slots(item_bytes) + blob_slots(4 * layer_blob(plan).words))) return rc;
+    // What the launch stages later must not come to lie over this: room for both.
+    const size_t item_words = items.size() * (sizeof(GkrBatchItem) / 4);
+    const LayerBlob at = layer_blob(plan);
+    if (int rc = stage_reserve(ctx, blob_slots(4 * (item_words + at.words)) + blob_slots(4 * open_words(plan)))) return rc;
+    std::vector<uint32_t>& blob = ctx_blob();
+    blob.assign(item_words + at.words, 0u);
+    memcpy(blob.data(), items.data(), 4 * item_words);
+    memcpy(&blob[item_words + at.tables], plan.tables.data(), 4 * plan.tables.size());
     void* d = nullptr;
-    if (int rc = stage_blob(ctx, items.data(), item_bytes, &d)) return rc;
+    if (int rc = stage_blob(ctx, blob.data(), 4 * blob.size(), &d)) return rc;
     plan.d_items = static_cast<const GkrBatchItem*>(d);
+    plan.d_blob = static_cast<uint32_t*>(d) + item_words;
     return ZKB_OK;
 }
 
@@ -1255,8 +1282,11 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
     const size_t K = plan.n_vars.size();
     const int n_rounds = plan.n_rounds;
     const LayerBlob at = layer_blob(plan);
+    const bool carries = !plan.launches && open_words(plan) <= OPEN_WORDS;
+    GkrLayerOpen carried;
     std::vector<uint32_t>& blob = ctx_blob();
-    blob.assign(at.words, 0u);
+    if (!carries) blob.assign(open_words(plan), 0u);
+    uint32_t* const open = carries ? carried.words : blob.data();
     auto q4 = [](const uint32_t* w) { return qm31{{w[0], w[1], w[2], w[3]}}; };
     // The oracles' claims by the round they enter in (group; those without variables never do), each times alpha^k. The claims come
     // scaled by 2^(rounds they wait), and a waiting oracle's claim halves every round (sumcheck.rs:115-125).
@@ -1266,13 +1296,10 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
         qm31& v = entering[n_rounds - (int)plan.n_vars[k]];
         v = qm31_add(v, qm31_mul(q4(alpha_pow + 4 * k), q4(claims + 4 * k)));
     }
-    GkrStepState& st = *reinterpret_cast<GkrStepState*>(blob.data());
-    memcpy(st.digest, chan, 32);
-    st.n_draws = chan[8];
-    st.claim = entering[0];
-    for (auto& c : st.corr) c = qm31_one();
-    memcpy(&blob[at.alpha], alpha_pow, 16 * K);
-    GkrStepConst* const consts = reinterpret_cast<GkrStepConst*>(&blob[at.rounds]);
+    memcpy(open, chan, 36);
+    memcpy(open + OPEN_CLAIM, entering[0].c, 16);
+    memcpy(open + open_alpha(n_rounds), alpha_pow, 16 * K);
+    GkrStepConst* const consts = reinterpret_cast<GkrStepConst*>(open + OPEN_CONSTS);
     qm31 waiting = qm31_zero();
     for (int j = n_rounds; j-- > 0;) {
         waiting = qm31_add(waiting, entering[j + 1]);  // all that enter after round j
@@ -1289,12 +1316,16 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
         c.entering = j + 1 < n_rounds ? qm31_mul_m31(entering[j + 1], half_pow) : qm31_zero();
         c.round = (uint32_t)j;
     }
-    memcpy(&blob[at.tables], plan.tables.data(), 4 * plan.tables.size());
-    void* d_blob_v = nullptr;
-    if (int rc = stage_blob(ctx, blob.data(), blob.size() * 4, &d_blob_v)) return rc;
-    uint32_t* d_blob = static_cast<uint32_t*>(d_blob_v);
+    uint32_t* const d_blob = plan.d_blob;
+    const uint32_t* d_open = nullptr;
+    auto copy_open = [&]() -> int {
+        void* d = nullptr;
+        const int rc = stage_blob(ctx, open, 4 * open_words(plan), &d);
+        d_open = static_cast<const uint32_t*>(d);
+        return rc;
+    };
+    if (!carries) if (int rc = copy_open()) return rc;
     GkrStepState* d_state = reinterpret_cast<GkrStepState*>(d_blob);
-    const GkrStepConst* d_consts = reinterpret_cast<const GkrStepConst*>(d_blob + at.rounds);
     const qm31 lam = q4(h_lambda);
     GkrLayerOut host;
     host.records = ctx->h_batch;
@@ -1304,7 +1335,6 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
     host.id = ++ctx->batch_round;
     const GkrTable* const h_tables = reinterpret_cast<const GkrTable*>(plan.tables.data());
     const GkrTable* const d_tables = reinterpret_cast<const GkrTable*>(d_blob + at.tables);
-    const uint32_t* const d_alpha = d_blob + at.alpha;
     uint32_t* const d_records = d_blob + at.records;
     GkrSync* const d_sync = reinterpret_cast<GkrSync*>(d_blob + at.sync);
     const GkrAcc acc{reinterpret_cast<unsigned long long*>(d_blob + at.acc), n_rounds};
@@ -1320,8 +1350,8 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
         cfg.stream = ctx->stream;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, d_tables, 0, plan.look_from >= 0 ? plan.look_from + 1 : n_rounds + 1, plan.needs_eq ? eq_evals : nullptr, lam, d_alpha, d_state, acc,
-                               d_sync, d_consts, plan.look_from, d_records, n_rounds, host);
+        e = cudaLaunchKernelEx(&cfg, gkr_batch_layer_kernel, plan.d_items, d_tables, 0, plan.look_from >= 0 ? plan.look_from + 1 : n_rounds + 1, plan.needs_eq ? eq_evals : nullptr, lam, carried, d_open, d_state, acc,
+                               d_sync, 1, plan.look_from, d_records, n_rounds, host);
     }
     // Asked for, or the CTAs are not all resident at once (a share of the GPU's SMs): a launch per table and one per step, where nobody waits.
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
@@ -1331,16 +1361,17 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
             if (int rc = gkr_batch_plan(ctx, plan)) return rc;
             return GKR_BATCH_AGAIN;
         }
+        if (!d_open) if (int rc = copy_open()) return rc;
         e = cudaSuccess;
         for (int t = 0; t <= n_rounds && e == cudaSuccess; t++) {
             {
                 ProfScope prof(ctx, "gkr_batch_layer_kernel");
-                gkr_batch_layer_kernel<<<h_tables[t].ctas, GKR_THREADS, 0, ctx->stream>>>(plan.d_items, d_tables, t, t + 1, eq_evals, lam, d_alpha, d_state, acc, d_sync, nullptr,
+                gkr_batch_layer_kernel<<<h_tables[t].ctas, GKR_THREADS, 0, ctx->stream>>>(plan.d_items, d_tables, t, t + 1, eq_evals, lam, carried, d_open, d_state, acc, d_sync, 0,
                                                                                           -1, d_records, n_rounds, host);
             }
             {
                 ProfScope prof(ctx, "gkr_batch_step_kernel");
-                gkr_batch_step_kernel<<<1, 32, 0, ctx->stream>>>(d_state, acc, d_sync, d_consts, d_records, t, n_rounds, host);
+                gkr_batch_step_kernel<<<1, 32, 0, ctx->stream>>>(d_state, acc, d_sync, d_open, d_records, t, n_rounds, host);
             }
             e = cudaGetLastError();
         }

@@ -69,7 +69,8 @@ struct GkrLayerPlan {
     int look_from = -1;              // and from which round on the rounds are taken ahead of the transcript, with which items (-1: none, and `items`)
     std::vector<GkrBatchItem> look_items;
     bool needs_eq = true;            // whether begin wants the table of eq(., point)
-    const GkrBatchItem* d_items = nullptr;
+    const GkrBatchItem* d_items = nullptr;  // staged by gkr_batch_plan, and what else does not depend on the transcript
+    uint32_t* d_blob = nullptr;
     bool launches = false;           // the layer as a launch per table and one per transcript step
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
