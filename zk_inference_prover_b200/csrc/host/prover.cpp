@@ -182,13 +182,6 @@ struct MerkleProver {
     // of thousands of columns by size a second time costs milliseconds
     std::vector<std::vector<const uint32_t*>> layer_col_ptrs;
 
-    // The column tables of a tree's layers, copied to the device (commit and the decommitment find them there).
-    static void stage_tables(const Device& d, const std::vector<const BaseColumn*>& columns) {
-        std::vector<std::vector<const uint32_t*>> of(33);
-        for (auto c : columns) of[c->log_size()].push_back(c->ptr());
-        for (auto& p : of) if (!p.empty()) d.check(zk::stage_table(d.ctx(), p.data(), (int)p.size()));
-    }
-
     // `leaves`, when given, is the already hashed largest layer (see zkb_merkle_leaves_partial).
     // `chan_step`, when given, is a FRI layer's channel step (channel state, challenge slot, root copy; device addresses) to run
     // in the launch that builds the root; *chan_done says whether it ran (a tree of one node has no such launch).
@@ -197,70 +190,7 @@ struct MerkleProver {
     // the launch before it 2 us and this one, with the code for a thread a hash to fetch, 7.
     static constexpr uint32_t TOP_LOG = 8;
     static MerkleProver commit(const Device& d, const std::vector<const BaseColumn*>& columns, HashColumn* leaves = nullptr,
-                               const ChanStep* chan_step = nullptr, bool* chan_done = nullptr) {  // :39-64
-        if (chan_done) *chan_done = false;
-        auto top = [&](uint32_t log, uint32_t* top_layer, uint32_t** lower) {
-            if (chan_step && log >= 1) {
-                d.check(zkb_merkle_top_channel(d.ctx(), (int)log, top_layer, lower, 1, chan_step->chan, chan_step->alpha, chan_step->root_copy));
-                if (chan_done) *chan_done = true;
-            } else d.check(zkb_merkle_top(d.ctx(), (int)log, top_layer, lower, 1));
-        };
-        MerkleProver mp;
-        if (columns.empty()) {
-            mp.layers.push_back(B200Backend::commit_on_layer(d, 0, nullptr, {}));
-            return mp;
-        }
-        uint32_t max_log = 0, min_log = 32;
-        size_t count[33] = {0};
-        for (auto c : columns) {
-            const uint32_t log = c->log_size();
-            count[log]++;
-            max_log = std::max(max_log, log);
-            min_log = std::min(min_log, log);
-        }
-        mp.layers.resize(max_log + 1);
-        mp.layer_col_ptrs.resize(max_log + 1);
-        for (uint32_t log = 0; log <= max_log; log++) mp.layer_col_ptrs[log].reserve(count[log]);
-        for (auto c : columns) mp.layer_col_ptrs[c->log_size()].push_back(c->ptr());
-        for (uint32_t log = max_log + 1; log-- > 0;) {
-            if (log == max_log && leaves) mp.layers[log] = std::move(*leaves);
-            else {
-                mp.layers[log] = HashColumn(d, (size_t)8 << log);
-                d.check(zkb_merkle_layer(d.ctx(), (int)log, log == max_log ? nullptr : mp.layers[log + 1].ptr(), mp.layer_col_ptrs[log].data(),
-                                         (int)mp.layer_col_ptrs[log].size(), 1, mp.layers[log].ptr()));
-            }
-            const bool all = log <= min_log;  // no columns left below
-            if (log > 0 && log <= TOP_LOG && all) {
-                // no columns left below: the rest of the tree is nodes only, built in one launch
-                std::vector<uint32_t*> lower;
-                for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
-                top(log, mp.layers[log].ptr(), lower.data());
-                break;
-            }
-            // The layers below this one that hold no column (down to the next layer that has one, or to the last ones, which
-            // the launch above builds): up to nine of them per launch.
-            uint32_t floor_log = TOP_LOG;
-            if (!all) {
-                uint32_t next = log - 1;
-                while (!count[next]) next--;
-                floor_log = next + 1;
-            }
-            while (log > floor_log && log >= 9) {
-                const uint32_t levels = std::min<uint32_t>(9, log - floor_log);
-                std::vector<uint32_t*> outs;
-                for (uint32_t j = 1; j <= levels; j++) { mp.layers[log - j] = HashColumn(d, (size_t)8 << (log - j)); outs.push_back(mp.layers[log - j].ptr()); }
-                d.check(zkb_merkle_levels(d.ctx(), (int)log, mp.layers[log].ptr(), (int)levels, outs.data(), 1));
-                log -= levels;
-            }
-            if (log > 0 && log <= TOP_LOG && all && mp.layers[log - 1].len() == 0) {
-                std::vector<uint32_t*> lower;
-                for (uint32_t k = 0; k < log; k++) { mp.layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(mp.layers[k].ptr()); }
-                top(log, mp.layers[log].ptr(), lower.data());
-                break;
-            }
-        }
-        return mp;
-    }
+                               const ChanStep* chan_step = nullptr, bool* chan_done = nullptr);  // :39-64
     Hash root(const Device& d) const {
         if (!have_root) {
             const uint32_t* h = nullptr;
@@ -318,6 +248,88 @@ struct MerkleProver {
         return pm;
     }
 };
+
+// A tree from its largest layer down, as far as its columns are there: a layer's columns have to be enqueued only when it is hashed.
+struct MerkleBuilder {
+    const Device& d;
+    MerkleProver tree;
+    int next = -1;         // the layer to hash next; negative: the tree is whole
+    size_t count[33];      // columns of each layer
+    uint32_t min_log = 32;
+
+    MerkleBuilder(const Device& dev, const size_t (&columns)[33]) : d(dev) {
+        for (int log = 0; log <= 32; log++) {
+            count[log] = columns[log];
+            if (!count[log]) continue;
+            next = log;
+            min_log = std::min(min_log, (uint32_t)log);
+        }
+        if (next < 0) {
+            tree.layers.push_back(B200Backend::commit_on_layer(d, 0, nullptr, {}));
+            return;
+        }
+        tree.layers.resize((size_t)next + 1);
+        tree.layer_col_ptrs.resize((size_t)next + 1);
+    }
+    // The layer at `next`, whose columns are in tree.layer_col_ptrs, and what follows from it in the same launches.
+    void hash_next(HashColumn* leaves = nullptr, const MerkleProver::ChanStep* chan_step = nullptr, bool* chan_done = nullptr) {
+        constexpr uint32_t TOP_LOG = MerkleProver::TOP_LOG;
+        auto& layers = tree.layers;
+        uint32_t log = (uint32_t)next;
+        auto top = [&] {  // the rest of the tree is nodes only, built in one launch
+            std::vector<uint32_t*> lower;
+            for (uint32_t k = 0; k < log; k++) { layers[k] = HashColumn(d, (size_t)8 << k); lower.push_back(layers[k].ptr()); }
+            if (chan_step && log >= 1) {
+                d.check(zkb_merkle_top_channel(d.ctx(), (int)log, layers[log].ptr(), lower.data(), 1, chan_step->chan, chan_step->alpha, chan_step->root_copy));
+                if (chan_done) *chan_done = true;
+            } else d.check(zkb_merkle_top(d.ctx(), (int)log, layers[log].ptr(), lower.data(), 1));
+            next = -1;
+        };
+        const bool first = (size_t)log + 1 == layers.size();
+        if (first && leaves) layers[log] = std::move(*leaves);
+        else {
+            layers[log] = HashColumn(d, (size_t)8 << log);
+            d.check(zkb_merkle_layer(d.ctx(), (int)log, first ? nullptr : layers[log + 1].ptr(), tree.layer_col_ptrs[log].data(), (int)tree.layer_col_ptrs[log].size(), 1,
+                                     layers[log].ptr()));
+        }
+        const bool all = log <= min_log;  // no columns left below
+        if (log > 0 && log <= TOP_LOG && all) return top();
+        // The layers below this one that hold no column (down to the next layer that has one, or to the last ones, which
+        // the launch above builds): up to nine of them per launch.
+        uint32_t floor_log = TOP_LOG;
+        if (!all) {
+            uint32_t below = log - 1;
+            while (!count[below]) below--;
+            floor_log = below + 1;
+        }
+        while (log > floor_log && log >= 9) {
+            const uint32_t levels = std::min<uint32_t>(9, log - floor_log);
+            std::vector<uint32_t*> outs;
+            for (uint32_t j = 1; j <= levels; j++) { layers[log - j] = HashColumn(d, (size_t)8 << (log - j)); outs.push_back(layers[log - j].ptr()); }
+            d.check(zkb_merkle_levels(d.ctx(), (int)log, layers[log].ptr(), (int)levels, outs.data(), 1));
+            log -= levels;
+        }
+        if (log > 0 && log <= TOP_LOG && all && layers[log - 1].len() == 0) return top();
+        next = (int)log - 1;
+    }
+    // ... and on to the next layer with columns.
+    void hash_to_columns() {
+        do hash_next();
+        while (next >= 0 && !count[next]);
+    }
+};
+
+inline MerkleProver MerkleProver::commit(const Device& d, const std::vector<const BaseColumn*>& columns, HashColumn* leaves, const ChanStep* chan_step, bool* chan_done) {
+    if (chan_done) *chan_done = false;
+    size_t count[33] = {0};
+    for (auto c : columns) count[c->log_size()]++;
+    MerkleBuilder builder(d, count);
+    auto& cols = builder.tree.layer_col_ptrs;
+    for (size_t log = 0; log < cols.size(); log++) cols[log].reserve(count[log]);
+    for (auto c : columns) cols[c->log_size()].push_back(c->ptr());
+    while (builder.next >= 0) builder.hash_next(leaves, chan_step, chan_done);
+    return std::move(builder.tree);
+}
 
 // ------------------------------------------------------------------ FRI (STWO/prover/fri.rs:87-467)
 struct FriConfig {
@@ -671,6 +683,14 @@ struct SamplePoints {
     }
     void end_column() { first.push_back(point_of.size()); }
 };
+// What is evaluated where: a group of columns of one size at one point (doubled as often as its columns are shorter than the tallest), its values one after the
+// other in the value array, sample s's at place_of[s]. Made of the trees and of which points are which, not of where they are.
+struct SamplePlan {
+    struct Group { uint32_t log, point, doublings; size_t first, count; };
+    std::vector<Group> groups;
+    std::vector<uint32_t> place_of;
+    std::vector<const uint32_t*> polys;
+};
 struct SampledValues {
     std::vector<size_t> tree_first{0};  // the trees' first columns
     std::vector<size_t> first{0};       // the columns' first values
@@ -795,29 +815,30 @@ struct CommitmentSchemeProver {
     }
 
     // Trees committed one after the other with nothing drawn in between: their roots are read and mixed in at the end (mix_roots). One of
-    // them is hashed beside the work on the next ones, the first whose short layers hold so many columns that they are a chain of
+    // them ends beside the work on the next ones, the first whose short layers hold so many columns that they are a chain of
     // compressions on a handful of warps (20,000 columns of 2^11 rows: a millisecond and a half with most of the chip idle).
     struct SeveralTrees {
         bool more = true;  // trees come after this one
         bool forked = false;
     };
-    static bool narrow(const std::vector<BaseColumn>& evals) {
-        size_t cols[14] = {0}, chain = 0;
-        for (auto& e : evals)
-            if (e.log_size() <= 13) cols[e.log_size()]++;
-        for (size_t c : cols) chain += c / 16;
+    static constexpr uint32_t NARROW_LOG = 13;  // the tallest such layer
+    static bool narrow(const size_t (&columns)[33]) {
+        size_t chain = 0;
+        for (uint32_t log = 0; log <= NARROW_LOG; log++) chain += columns[log] / 16;
         return chain >= 64;  // some 55 us; a fork and its join cost a few
     }
     void mix_roots(Channel& ch) {
         zk::side_join(d.ctx());
-        GatherPlan plan;
-        for (auto& t : trees) plan.add_hash(t.commitment.layers[0].ptr());
-        if (!trees.empty()) plan.execute(d);
-        for (size_t k = 0; k < trees.size(); k++) {
-            trees[k].commitment.root_cache = plan.hash_at(k);
-            trees[k].commitment.have_root = true;
-            ch.mix_root(trees[k].commitment.root_cache);
+        if (trees.size() > 1) {
+            GatherPlan plan;
+            for (auto& t : trees) plan.add_hash(t.commitment.layers[0].ptr());
+            plan.execute(d);
+            for (size_t k = 0; k < trees.size(); k++) {
+                trees[k].commitment.root_cache = plan.hash_at(k);
+                trees[k].commitment.have_root = true;
+            }
         }
+        for (auto& t : trees) ch.mix_root(t.commitment.root(d));
     }
 
     // TreeBuilder::extend_evals + commit (pcs/mod.rs:429-464) -> CommitmentTreeProver::new (:481-537).
@@ -841,7 +862,8 @@ struct CommitmentSchemeProver {
         t.evals.resize(columns.size());
         HashColumn leaves;
         bool have_leaves = false;
-        if (fence_of && !columns.empty()) {
+        const bool hashes_later = fence_of && !columns.empty();
+        if (hashes_later) {
             mark(0);
             // One column size: the leaf layer is hashed run by run (whole Blake2s blocks of 16 columns) as the
             // extended columns appear, instead of after the last one.
@@ -874,41 +896,75 @@ struct CommitmentSchemeProver {
             }
             if (incremental) { hash_ready(true); have_leaves = true; }
         } else {
-            for (auto& g : by_log) {
-                if (are_coeffs) break;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
-                std::vector<uint32_t*> cols;
-                cols.reserve(g.second.size());
-                for (auto i : g.second) cols.push_back(columns[i].ptr());
-                d.check(zkb_ifft_cols(d.ctx(), cols.data(), (int)cols.size(), (int)g.first));
+            // From the tallest columns down, each size interpolated, extended and hashed before the next: a segment's short columns are tens of thousands,
+            // which take the host longer to write down than the device to transform, and the device has the tall ones' hashes meanwhile.
+            const uint32_t blowup = config.fri.log_blowup_factor;
+            struct Size { uint32_t log; const std::vector<size_t>* of; };
+            std::vector<Size> sizes;
+            size_t count[33] = {0};
+            for (auto g = by_log.rbegin(); g != by_log.rend(); ++g) {
+                sizes.push_back({g->first, &g->second});
+                count[g->first + blowup] = g->second.size();
             }
-            mark(0);
-            for (auto& g : by_log) {
+            MerkleBuilder builder(d, count);
+            auto interpolate = [&](const Size& g) {
+                if (are_coeffs) return;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
+                std::vector<uint32_t*> cols;
+                cols.reserve(g.of->size());
+                for (auto i : *g.of) cols.push_back(columns[i].ptr());
+                d.check(zkb_ifft_cols(d.ctx(), cols.data(), (int)cols.size(), (int)g.log));
+            };
+            auto extend = [&](const Size& g) {
                 // one allocation for the extended columns of a size (16-byte aligned each)
-                const size_t nc = g.second.size(), n_out = (size_t)1 << (g.first + config.fri.log_blowup_factor);
+                const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup);
                 const size_t stride = std::max<size_t>(n_out, 4);
                 t.eval_slabs.emplace_back(d, nc * stride);
                 std::vector<const uint32_t*> src(nc);
                 std::vector<uint32_t*> dst(nc);
                 for (size_t k = 0; k < nc; k++) {
-                    src[k] = columns[g.second[k]].ptr();
+                    src[k] = columns[(*g.of)[k]].ptr();
                     dst[k] = t.eval_slabs.back().ptr() + k * stride;
-                    t.evals[g.second[k]] = BaseColumn::view(d, dst[k], n_out);
                 }
-                d.check(zkb_lde_cols(d.ctx(), src.data(), (int)nc, (int)g.first, dst.data(), (int)(g.first + config.fri.log_blowup_factor)));
+                d.check(zkb_lde_cols(d.ctx(), src.data(), (int)nc, (int)g.log, dst.data(), (int)(g.log + blowup)));
+                for (size_t k = 0; k < nc; k++) t.evals[(*g.of)[k]] = BaseColumn::view(d, dst[k], n_out);
+                builder.tree.layer_col_ptrs[g.log + blowup].assign(dst.begin(), dst.end());
+            };
+            if (phase_ms) {  // phase after phase, to be timed
+                for (auto& g : sizes) interpolate(g);
+                mark(0);
+                for (auto& g : sizes) extend(g);
+                mark(1);
+                while (builder.next >= 0) builder.hash_next();
+            } else {
+                const bool fork = several && several->more && !several->forked && narrow(count);
+                size_t k = 0;
+                for (; k < sizes.size() && !(fork && sizes[k].log + blowup <= NARROW_LOG); k++) {
+                    interpolate(sizes[k]);
+                    extend(sizes[k]);
+                    builder.hash_to_columns();
+                }
+                if (k < sizes.size()) {
+                    several->forked = true;
+                    for (size_t j = k; j < sizes.size(); j++) interpolate(sizes[j]);
+                    for (size_t j = k; j < sizes.size(); j++) extend(sizes[j]);
+                    // so that the decommitment finds them: a table copied on the side is not there for the work outside
+                    for (size_t j = k; j < sizes.size(); j++) {
+                        const auto& cols = builder.tree.layer_col_ptrs[sizes[j].log + blowup];
+                        d.check(zk::stage_table(d.ctx(), cols.data(), (int)cols.size()));
+                    }
+                    d.check(zk::side_begin(d.ctx()));
+                    while (builder.next >= 0) builder.hash_next();
+                    d.check(zk::side_end(d.ctx()));
+                }
             }
+            t.commitment = std::move(builder.tree);
         }
-        mark(1);
         t.coeffs = std::move(columns);
-        std::vector<const BaseColumn*> refs;
-        refs.reserve(t.evals.size());
-        for (auto& e : t.evals) refs.push_back(&e);
-        if (several && several->more && !several->forked && narrow(t.evals)) {
-            several->forked = true;
-            MerkleProver::stage_tables(d, refs);  // so that the decommitment finds them
-            d.check(zk::side_begin(d.ctx()));
-            t.commitment = MerkleProver::commit(d, refs);
-            d.check(zk::side_end(d.ctx()));
-        } else {
+        if (hashes_later) {
+            mark(1);
+            std::vector<const BaseColumn*> refs;
+            refs.reserve(t.evals.size());
+            for (auto& e : t.evals) refs.push_back(&e);
             t.commitment = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr);
         }
         if (!several) ch.mix_root(t.commitment.root(d));
@@ -1054,61 +1110,67 @@ struct CommitmentSchemeProver {
         return B200Backend::compute_quotients_and_combine(d, per_point, lifting_log);
     }
 
-    // pcs/mod.rs:168-419
-    PcsProof prove_values(SamplePoints sp, Channel& ch) {
-        PcsProof proof;
-        uint32_t lifting_log = trees.back().max_log();
+    // batch out-of-domain evaluation: one call per (coefficient size, transformed point) group (pcs/mod.rs:187-265)
+    SamplePlan plan_samples(const SamplePoints& sp, size_t n_points) const {
+        HostClock hc("pcs.sample.group");
         // Every column is lifted to the height of the LAST tree (pcs/mod.rs:180: in a proof it is the composition tree, which
         // is the tallest); a taller column in an earlier tree has no lift.
+        const uint32_t lifting_log = trees.back().max_log();
         for (auto& t : trees)
             if (!t.evals.empty() && t.max_log() > lifting_log)
                 throw Error(ZKB_EINVAL, "pcs: the last tree must hold the tallest column (every column is lifted to its height)");
-        // batch out-of-domain evaluation: one call per (coefficient size, transformed point) group (:187-265); the values of a group
-        // lie one after the other in the value array, place_of[s] is sample s's
-        std::unique_ptr<HostClock> hc(new HostClock("pcs.sample.group"));
+        SamplePlan plan;
         const size_t n_samples = sp.point_of.size();
-        struct Group { uint32_t log; CirclePointQ pt; size_t first, count; };
-        std::vector<Group> groups;
-        std::vector<int> group_of(sp.points.size() * 64, -1);  // by (point, doublings)
-        std::vector<uint32_t> sample_group(n_samples), place_of(n_samples);
+        std::vector<int> group_of(n_points * 64, -1);  // by (point, doublings)
+        std::vector<uint32_t> sample_group(n_samples);
+        plan.place_of.resize(n_samples);
+        plan.polys.resize(n_samples);
         size_t flat = 0;
-        for (auto& t : trees) {
-            proof.sampled_values.tree_first.push_back(flat + t.coeffs.size());
+        for (auto& t : trees)
             for (size_t c = 0; c < t.coeffs.size(); c++, flat++) {
-                const uint32_t coeff_log = t.coeffs[c].log_size(), shift = lifting_log - t.evals[c].log_size();
+                const uint32_t shift = lifting_log - t.evals[c].log_size();
                 for (size_t s = sp.first[flat]; s < sp.first[flat + 1]; s++) {
                     int& g = group_of[sp.point_of[s] * 64 + shift];
                     if (g < 0) {
-                        g = (int)groups.size();
-                        groups.push_back({coeff_log, point_repeated_double(sp.points[sp.point_of[s]], shift), 0, 0});
+                        g = (int)plan.groups.size();
+                        plan.groups.push_back({t.coeffs[c].log_size(), sp.point_of[s], shift, 0, 0});
                     }
                     sample_group[s] = (uint32_t)g;
-                    groups[g].count++;
+                    plan.groups[g].count++;
                 }
             }
-        }
         size_t at = 0;
-        for (auto& g : groups) { g.first = at; at += g.count; g.count = 0; }
-        std::vector<const uint32_t*> polys(n_samples);
+        for (auto& g : plan.groups) { g.first = at; at += g.count; g.count = 0; }
         flat = 0;
         for (auto& t : trees)
             for (size_t c = 0; c < t.coeffs.size(); c++, flat++)
                 for (size_t s = sp.first[flat]; s < sp.first[flat + 1]; s++) {
-                    Group& g = groups[sample_group[s]];
-                    place_of[s] = (uint32_t)(g.first + g.count);
-                    polys[g.first + g.count++] = t.coeffs[c].ptr();
+                    SamplePlan::Group& g = plan.groups[sample_group[s]];
+                    plan.place_of[s] = (uint32_t)(g.first + g.count);
+                    plan.polys[g.first + g.count++] = t.coeffs[c].ptr();
                 }
+        return plan;
+    }
+
+    // pcs/mod.rs:168-419
+    PcsProof prove_values(SamplePoints sp, const SamplePlan& sample_plan, Channel& ch) {
+        PcsProof proof;
+        const uint32_t lifting_log = trees.back().max_log();
+        const size_t n_samples = sp.point_of.size();
+        const std::vector<uint32_t>& place_of = sample_plan.place_of;
+        for (auto& t : trees) proof.sampled_values.tree_first.push_back(proof.sampled_values.tree_first.back() + t.coeffs.size());
         // The quotient plan of tens of thousands of samples takes as long as hashing them does: it is made on another thread meanwhile.
         const bool aside = n_samples >= 8192;
         std::future<Numerators> planned;
         if (aside) planned = std::async(std::launch::async, [&] { return plan_numerators(sp, place_of, lifting_log); });
-        hc.reset(new HostClock("pcs.sample.eval"));
+        std::unique_ptr<HostClock> hc(new HostClock("pcs.sample.eval"));
         BaseColumn d_values(d, 4 * n_samples);
-        for (auto& g : groups) {
+        for (auto& g : sample_plan.groups) {
+            const CirclePointQ p = point_repeated_double(sp.points[g.point], g.doublings);
             uint32_t pt[8];
-            memcpy(pt, g.pt.x.c, 16);
-            memcpy(pt + 4, g.pt.y.c, 16);
-            d.check(zk::eval_at_point_device(d.ctx(), polys.data() + g.first, (int)g.count, (int)g.log, pt, d_values.ptr() + 4 * g.first));
+            memcpy(pt, p.x.c, 16);
+            memcpy(pt + 4, p.y.c, 16);
+            d.check(zk::eval_at_point_device(d.ctx(), sample_plan.polys.data() + g.first, (int)g.count, (int)g.log, pt, d_values.ptr() + 4 * g.first));
         }
         hc.reset(new HostClock("pcs.quot.plan"));
         Numerators nu;
@@ -2017,12 +2079,14 @@ int zkb_shard_pcs_finish(zkb_shard_pcs* h, const uint32_t* const* h_parts, const
 
 // Commits the caller's trees in order (TreeBuilder::extend_evals + commit per tree), from device columns or from host
 // columns with the upload overlapped.
+// meanwhile: what the host has to do that does not depend on the roots; where the trees are on the device it is done while they are hashed.
+template <class Meanwhile>
 static void commit_input_trees(Device& dev, zkb_ctx* ctx, CommitmentSchemeProver& prover, Channel& ch, int n_trees, const int* tree_ncols,
-                               uint32_t* const* d_cols, const uint32_t* const* h_cols, const uint32_t* col_logs, int total) {
+                               uint32_t* const* d_cols, const uint32_t* const* h_cols, const uint32_t* col_logs, int total, Meanwhile meanwhile) {
         int flat = 0;
         if (d_cols) {
             // (with phases to be timed one tree after the other: their marks are on one stream)
-            const bool together = n_trees > 1 && !prover.phase_ms;
+            const bool together = !prover.phase_ms;
             CommitmentSchemeProver::SeveralTrees several;
             zk::SideScope scope(ctx);
             for (int t = 0; t < n_trees; t++) {
@@ -2033,6 +2097,7 @@ static void commit_input_trees(Device& dev, zkb_ctx* ctx, CommitmentSchemeProver
                     columns.push_back(BaseColumn::view(dev, d_cols[flat], (size_t)1 << col_logs[flat]));
                 prover.commit_evals(std::move(columns), ch, nullptr, nullptr, false, together ? &several : nullptr);
             }
+            meanwhile();
             if (together) prover.mix_roots(ch);
         } else {
             // Host columns: every copy of every tree is enqueued on the copy stream first, with a fence
@@ -2088,6 +2153,7 @@ static void commit_input_trees(Device& dev, zkb_ctx* ctx, CommitmentSchemeProver
                     if (close) { flush(fence); since = 0; if (fence < 63) fence++; }
                 }
                 for (int t = 0; t < n_trees; t++) prover.commit_evals(std::move(tree_cols[t]), ch, &tree_fences[t], &slabs[t]);
+                meanwhile();
             } catch (...) {
                 zkb_sync(ctx);
                 throw;
@@ -2111,33 +2177,40 @@ static int pcs_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, uint
         Channel ch;
         config.mix_into(ch);
         CommitmentSchemeProver prover(dev, config, h_phase_ms);
+        // Which column is sampled where: all at the out-of-domain point, drawn from the roots, some one trace step back from it too. Points are told apart
+        // by their distance from that one.
+        SamplePoints points;
+        std::vector<cpoint> distance{host_circle_point(0)};
+        SamplePlan sample_plan;
         {
             HostClock hcc("pcs.commit_trees");
-            commit_input_trees(dev, ctx, prover, ch, n_trees, tree_ncols, d_cols, h_cols, col_logs, total);
-        }
-        int flat = 0;
-        CirclePointQ oods = get_random_point(ch);
-        SamplePoints points;
-        points.point_of.reserve((size_t)total);
-        points.first.reserve((size_t)total + 1);
-        const uint32_t at_oods = points.intern(oods);
-        uint32_t step_back[32];  // per column size, the place of its second point
-        for (auto& k : step_back) k = ~0u;
-        for (flat = 0; flat < total; flat++) {
-            if (two_sample_every && flat % two_sample_every == 0) {
-                uint32_t& k = step_back[col_logs[flat]];
-                if (k == ~0u) {
-                    // one trace step back: the conjugate of the step of CanonicCoset(col_log)
-                    cpoint st = host_circle_point(1u << (31 - col_logs[flat]));
-                    k = points.intern(point_add(oods, {qm31_from_m31(st.x), qm31_from_m31(m31_neg(st.y))}));
+            commit_input_trees(dev, ctx, prover, ch, n_trees, tree_ncols, d_cols, h_cols, col_logs, total, [&] {
+                points.point_of.reserve(2 * (size_t)total);
+                points.first.reserve((size_t)total + 1);
+                uint32_t step_back[33];  // per column size, the place of its second point
+                for (auto& k : step_back) k = ~0u;
+                for (int flat = 0; flat < total; flat++) {
+                    if (two_sample_every && flat % two_sample_every == 0) {
+                        uint32_t& k = step_back[col_logs[flat]];
+                        if (k == ~0u) {
+                            // the conjugate of the step of CanonicCoset(col_log)
+                            const cpoint st = host_circle_point(1u << (31 - col_logs[flat])), back{st.x, m31_neg(st.y)};
+                            for (k = 0; k < distance.size() && (distance[k].x != back.x || distance[k].y != back.y);) k++;
+                            if (k == distance.size()) distance.push_back(back);
+                        }
+                        points.point_of.push_back(k);
+                    }
+                    points.point_of.push_back(0);
+                    points.end_column();
                 }
-                points.point_of.push_back(k);
-            }
-            points.point_of.push_back(at_oods);
-            points.end_column();
+                sample_plan = prover.plan_samples(points, distance.size());
+            });
         }
+        const CirclePointQ oods = get_random_point(ch);
+        points.points.push_back(oods);
+        for (size_t k = 1; k < distance.size(); k++) points.points.push_back(point_add(oods, {qm31_from_m31(distance[k].x), qm31_from_m31(distance[k].y)}));
         std::unique_ptr<HostClock> hc(new HostClock("pcs.prove_values"));
-        PcsProof proof = prover.prove_values(std::move(points), ch);
+        PcsProof proof = prover.prove_values(std::move(points), sample_plan, ch);
         prover.finish_timing();
         hc.reset(new HostClock("pcs.write"));
         PcsProof::RawSink w{h_out, cap};  // straight into the caller's buffer: a proof of many columns is tens of megabytes
@@ -2207,7 +2280,7 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
         Channel ch;
         config.mix_into(ch);
         CommitmentSchemeProver prover(dev, config, h_phase_ms);
-        commit_input_trees(dev, ctx, prover, ch, n_trees, tree_ncols, d_cols, h_cols, col_logs.data(), total);
+        commit_input_trees(dev, ctx, prover, ch, n_trees, tree_ncols, d_cols, h_cols, col_logs.data(), total, [] {});
 
         // ---- composition polynomial
         const qm31 random_coeff = ch.draw_secure_felt();
@@ -2311,7 +2384,8 @@ static int stark_prove_impl(zkb_ctx* ctx, int n_trees, const int* tree_ncols, ui
                 for (auto& p : column) flat_points.point_of.push_back(flat_points.intern(p));
                 flat_points.end_column();
             }
-        PcsProof proof = prover.prove_values(std::move(flat_points), ch);
+        const SamplePlan sample_plan = prover.plan_samples(flat_points, flat_points.points.size());
+        PcsProof proof = prover.prove_values(std::move(flat_points), sample_plan, ch);
         prover.finish_timing();
         if (composition_ms) dev.check(zkb_event_elapsed_ms(ctx, 28, 29, composition_ms));
 
