@@ -65,12 +65,20 @@ struct BlockCache {
 // interpolation, the extension, the hashing, the sampling, the numerators and the decommitment in turn, and a copy of a table in
 // between two kernels costs 2-3 us of the stream. (What was handed out stays in place until the ring is used from its start again: an
 // operator with several tables has their room reserved first.)
+static const zkb_ctx::StagedTable* find_staged(const zkb_ctx* ctx, const void* const* h_ptrs, size_t n) {
+    for (const auto& t : ctx->staged)
+        if (t.n == n && ctx->h_ring[t.pos] == h_ptrs[0] && !memcmp(ctx->h_ring + t.pos, h_ptrs, n * sizeof(void*))) return &t;
+    return nullptr;
+}
+static void remember_staged(zkb_ctx* ctx, size_t pos, size_t n) {
+    ctx->staged[ctx->staged_next] = {pos, n};
+    ctx->staged_next = (ctx->staged_next + 1) % zkb_ctx::STAGED_TABLES;
+}
 int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out) {
     if (n < 0 || (size_t)n > ctx->ring_cap) return set_error(ctx, ZKB_EINVAL, "stage_ptrs: %d pointers exceed the staging ring", n);
     if (n == 0) { *out = ctx->d_ring; return ZKB_OK; }
-    for (const auto& t : ctx->staged) {
-        if (t.n != (size_t)n || ctx->h_ring[t.pos] != h_ptrs[0] || memcmp(ctx->h_ring + t.pos, h_ptrs, (size_t)n * sizeof(void*))) continue;
-        *out = ctx->d_ring + t.pos;
+    if (const auto* t = find_staged(ctx, h_ptrs, (size_t)n)) {
+        *out = ctx->d_ring + t->pos;
         return ZKB_OK;
     }
     if (ctx->ring_pos + (size_t)n > ctx->ring_cap) {
@@ -80,10 +88,7 @@ int stage_ptrs(zkb_ctx* ctx, const void* const* h_ptrs, int n, void*** out) {
     void** d = ctx->d_ring + ctx->ring_pos;
     memcpy(h, h_ptrs, (size_t)n * sizeof(void*));
     ZKB_CUDA(ctx, cudaMemcpyAsync(d, h, (size_t)n * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
-    if (!ctx->on_side) {  // a table copied on the side is not there yet for the work outside
-        ctx->staged[ctx->staged_next] = {ctx->ring_pos, (size_t)n};
-        ctx->staged_next = (ctx->staged_next + 1) % zkb_ctx::STAGED_TABLES;
-    }
+    if (!ctx->on_side) remember_staged(ctx, ctx->ring_pos, (size_t)n);  // a table copied on the side is not there yet for the work outside
     ctx->ring_pos += (size_t)n;
     *out = d;
     return ZKB_OK;
@@ -722,6 +727,27 @@ int stage_table(zkb_ctx* ctx, const uint32_t* const* ptrs, int n) {
     DeviceGuard g(ctx);
     void** d = nullptr;
     return stage_ptrs(ctx, (const void* const*)ptrs, n, &d);
+}
+
+int stage_tables(zkb_ctx* ctx, const std::pair<const uint32_t* const*, size_t>* tables, size_t n_tables) {
+    if (ctx->on_side) return ZKB_OK;  // whoever wants one copies it
+    DeviceGuard g(ctx);
+    size_t total = 0;
+    for (size_t k = 0; k < n_tables; k++) total += tables[k].second;
+    if (total > ctx->ring_cap / 2) return ZKB_OK;
+    if (int rc = stage_reserve(ctx, total)) return rc;
+    const size_t first = ctx->ring_pos;
+    for (size_t k = 0; k < n_tables; k++) {
+        const void* const* const p = (const void* const*)tables[k].first;
+        const size_t n = tables[k].second;
+        if (!n || find_staged(ctx, p, n)) continue;
+        memcpy(ctx->h_ring + ctx->ring_pos, p, n * sizeof(void*));
+        remember_staged(ctx, ctx->ring_pos, n);
+        ctx->ring_pos += n;
+    }
+    if (ctx->ring_pos > first)
+        ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->d_ring + first, ctx->h_ring + first, (ctx->ring_pos - first) * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
+    return ZKB_OK;
 }
 
 int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t total_words, const uint32_t* const* word_addrs, size_t n_words,

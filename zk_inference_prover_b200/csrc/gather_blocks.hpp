@@ -2,6 +2,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 struct zkb_ctx;
 
@@ -9,6 +10,8 @@ namespace zk {
 
 // A table of device addresses on the device, where operators that are given the same table soon after find it.
 int stage_table(zkb_ctx* ctx, const uint32_t* const* ptrs, int n);
+// Several in one copy.
+int stage_tables(zkb_ctx* ctx, const std::pair<const uint32_t* const*, size_t>* tables, size_t n_tables);
 
 // out[out_off + i * ncols + c] = cols[c][idx[i]]: the rows idx[0..nidx) of ncols device columns, row-major.
 // cols and idx are host arrays (cols holds device pointers).

@@ -899,54 +899,66 @@ struct CommitmentSchemeProver {
             // From the tallest columns down, each size interpolated, extended and hashed before the next: a segment's short columns are tens of thousands,
             // which take the host longer to write down than the device to transform, and the device has the tall ones' hashes meanwhile.
             const uint32_t blowup = config.fri.log_blowup_factor;
-            struct Size { uint32_t log; const std::vector<size_t>* of; };
+            struct Size { uint32_t log; const std::vector<size_t>* of; std::vector<uint32_t*> coeffs, evals; };
             std::vector<Size> sizes;
             size_t count[33] = {0};
             for (auto g = by_log.rbegin(); g != by_log.rend(); ++g) {
-                sizes.push_back({g->first, &g->second});
+                sizes.push_back({g->first, &g->second, {}, {}});
                 count[g->first + blowup] = g->second.size();
             }
             MerkleBuilder builder(d, count);
-            auto interpolate = [&](const Size& g) {
-                if (are_coeffs) return;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
-                std::vector<uint32_t*> cols;
-                cols.reserve(g.of->size());
-                for (auto i : *g.of) cols.push_back(columns[i].ptr());
-                d.check(zkb_ifft_cols(d.ctx(), cols.data(), (int)cols.size(), (int)g.log));
-            };
-            auto extend = [&](const Size& g) {
-                // one allocation for the extended columns of a size (16-byte aligned each)
-                const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup);
-                const size_t stride = std::max<size_t>(n_out, 4);
-                t.eval_slabs.emplace_back(d, nc * stride);
-                std::vector<const uint32_t*> src(nc);
-                std::vector<uint32_t*> dst(nc);
-                for (size_t k = 0; k < nc; k++) {
-                    src[k] = columns[(*g.of)[k]].ptr();
-                    dst[k] = t.eval_slabs.back().ptr() + k * stride;
+            // The tables of several sizes of few columns go to the device in one copy: a copy between two kernels of a few microseconds costs as much as one.
+            size_t prepared = 0;
+            auto prepare = [&](size_t k) {
+                if (k < prepared) return;
+                std::vector<std::pair<const uint32_t* const*, size_t>> tables;
+                for (size_t n = 0; prepared < sizes.size() && (prepared == k || n + sizes[prepared].of->size() <= 4096) && tables.size() < 24; prepared++) {
+                    Size& g = sizes[prepared];
+                    const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup), stride = std::max<size_t>(n_out, 4);
+                    n += nc;
+                    // one allocation for the extended columns of a size (16-byte aligned each)
+                    t.eval_slabs.emplace_back(d, nc * stride);
+                    g.coeffs.resize(nc);
+                    g.evals.resize(nc);
+                    for (size_t c = 0; c < nc; c++) {
+                        g.coeffs[c] = columns[(*g.of)[c]].ptr();
+                        g.evals[c] = t.eval_slabs.back().ptr() + c * stride;
+                    }
+                    tables.push_back({g.coeffs.data(), nc});
+                    tables.push_back({g.evals.data(), nc});
                 }
-                d.check(zkb_lde_cols(d.ctx(), src.data(), (int)nc, (int)g.log, dst.data(), (int)(g.log + blowup)));
-                for (size_t k = 0; k < nc; k++) t.evals[(*g.of)[k]] = BaseColumn::view(d, dst[k], n_out);
-                builder.tree.layer_col_ptrs[g.log + blowup].assign(dst.begin(), dst.end());
+                d.check(zk::stage_tables(d.ctx(), tables.data(), tables.size()));
+            };
+            auto interpolate = [&](size_t k) {
+                prepare(k);
+                if (are_coeffs) return;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
+                d.check(zkb_ifft_cols(d.ctx(), sizes[k].coeffs.data(), (int)sizes[k].coeffs.size(), (int)sizes[k].log));
+            };
+            auto extend = [&](size_t k) {
+                Size& g = sizes[k];
+                const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup);
+                d.check(zkb_lde_cols(d.ctx(), g.coeffs.data(), (int)nc, (int)g.log, g.evals.data(), (int)(g.log + blowup)));
+                for (size_t c = 0; c < nc; c++) t.evals[(*g.of)[c]] = BaseColumn::view(d, g.evals[c], n_out);
+                builder.tree.layer_col_ptrs[g.log + blowup].assign(g.evals.begin(), g.evals.end());
             };
             if (phase_ms) {  // phase after phase, to be timed
-                for (auto& g : sizes) interpolate(g);
+                for (size_t k = 0; k < sizes.size(); k++) interpolate(k);
                 mark(0);
-                for (auto& g : sizes) extend(g);
+                for (size_t k = 0; k < sizes.size(); k++) extend(k);
                 mark(1);
                 while (builder.next >= 0) builder.hash_next();
             } else {
                 const bool fork = several && several->more && !several->forked && narrow(count);
                 size_t k = 0;
                 for (; k < sizes.size() && !(fork && sizes[k].log + blowup <= NARROW_LOG); k++) {
-                    interpolate(sizes[k]);
-                    extend(sizes[k]);
+                    interpolate(k);
+                    extend(k);
                     builder.hash_to_columns();
                 }
                 if (k < sizes.size()) {
                     several->forked = true;
-                    for (size_t j = k; j < sizes.size(); j++) interpolate(sizes[j]);
-                    for (size_t j = k; j < sizes.size(); j++) extend(sizes[j]);
+                    for (size_t j = k; j < sizes.size(); j++) interpolate(j);
+                    for (size_t j = k; j < sizes.size(); j++) extend(j);
                     // so that the decommitment finds them: a table copied on the side is not there for the work outside
                     for (size_t j = k; j < sizes.size(); j++) {
                         const auto& cols = builder.tree.layer_col_ptrs[sizes[j].log + blowup];
