@@ -408,13 +408,18 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
 // round are quadratic in this round's challenge, and its correction is linear. From round look_from on, then, the CTAs work on the round after the one that is being
 // hashed: they fold with the challenge before, and bring back the next round's sums at r = 0, at r = 1 and their leading coefficient; warps of CTA 0 make
 // of those the next polynomial as cubics in the challenge to come. When the challenge is there the next polynomial is two products away. The two chains
-// run beside each other: 16,000 cycles a round before, 9,500 now (34 instances of 2^13).
+// run beside each other: 16,000 cycles a round before, 9,500 after (34 instances of 2^13). The CTAs' chain is the longer one (hash and challenge 5,000), so what can
+// stand beside it does: the fence before the next challenge, and the loads of the next pass's entries, which are there some 2,000 cycles before the
+// challenge they are fixed at (34 instances 904 -> 868 us a proof, micro segment 14.56 -> 14.37 ms). The sums' words counting the CTAs themselves, instead of a
+// count behind a fence, gained nothing more (857 of 895 us).
 //
-// CTA 0 keeps the transcript and takes no pieces: warp 0 hashes, six warps take a node and point each, one makes the polynomial of them. Those are on other
+// CTA 0 keeps the transcript and takes no pieces: warp 0 hashes, six warps take a node and point each, one makes the polynomial of them, one sends the challenge. Those are on other
 // schedulers than warp 0, and the CTA has its SM to itself (a CTA an SM: with two of half the size the hash beside a worker took 5,700 cycles instead of 4,200).
-constexpr int LOOK_SUM_WARPS = 6, LOOK_LAST_WARP = 9;
-static_assert(GKR_THREADS / 32 > LOOK_LAST_WARP, "the warps of CTA 0");
-__device__ __forceinline__ int look_value(int warp) { return warp == LOOK_LAST_WARP ? LOOK_SUM_WARPS : warp < 8 && (warp & 3) ? warp - 1 - (warp >> 2) : -1; }  // 1-3, 5-7
+constexpr int LOOK_SUM_WARPS = 6, LOOK_LAST_WARP = 9, LOOK_SEND_WARP = 10;
+static_assert(GKR_THREADS / 32 > LOOK_SEND_WARP, "the warps of CTA 0");
+__device__ __forceinline__ int look_value(int warp) {  // 1-3, 5-7
+    return warp == LOOK_LAST_WARP || warp == LOOK_SEND_WARP ? LOOK_SUM_WARPS : warp < 8 && (warp & 3) ? warp - 1 - (warp >> 2) : -1;
+}
 
 // What a pass does for an item: the layer is there / fix it at the challenge first / it enters in the next round (nothing but its sums then).
 enum : uint32_t { LOOK_AS_IS = 0, LOOK_FIX = 1, LOOK_ENTERS = 2 };
@@ -434,9 +439,8 @@ __device__ __forceinline__ entry load_entry(const GkrBatchItem& it, size_t e) {
     if (it.kind == ZKB_GKR_LOGUP_MULTIPLICITIES) v.n = qm31_from_m31(it.num[e]);
     return v;
 }
-// The entry fixed at r, also where the folded layer goes. half: entries of that.
-__device__ __forceinline__ entry fix_entry(const GkrBatchItem& it, size_t e, size_t half, qm31 r) {
-    const entry v0 = load_entry(it, e), v1 = load_entry(it, e + half);
+// The entry fixed at r, also where the folded layer goes: v0, v1 are entries e and e + half of the layer, half the entries of the folded one.
+__device__ __forceinline__ entry fix_entry(const GkrBatchItem& it, size_t e, entry v0, entry v1, qm31 r) {
     const qm31_pair p = product_pair(r, qm31_sub(v1.d, v0.d), r, qm31_sub(v1.n, v0.n));
     const entry v{qm31_add(v0.d, p.a), qm31_add(v0.n, p.b)};
     stqb(it.den_out, e, v.d);
@@ -447,12 +451,19 @@ __device__ __forceinline__ entry fix_entry(const GkrBatchItem& it, size_t e, siz
 // Eight lanes a term of the next round, one for each of its entries: bit 2 the variable this round fixes, bit 1 the next round's, bit 0 the pair. A term is
 // n0 d1 + n1 d0 + lambda d0 d1 = m0 d1 + m1 d0 with m = n + k d, k = lambda / 2 (a grand product's d0 d1 with n = 0, k = 1 / 2). Lanes 0 and 2 end with the term at r
 // = 0, 4 and 6 with it at r = 1, 5 and 7 with its leading coefficient. ea: eq times the oracle's power of alpha.
-__device__ __forceinline__ void look_term(uint32_t (*acc)[2 * ACC_WORDS], const GkrBatchItem& it, bool live, uint32_t term, int terms_log, qm31 r, qm31 half_lambda, qm31 ea) {
+__device__ __forceinline__ size_t look_entry(uint32_t term, int terms_log) {  // this lane's
+    const int q = threadIdx.x & 7;
+    const size_t nt = (size_t)1 << terms_log;
+    return (size_t)(q >> 2) * 4 * nt + (size_t)((q >> 1) & 1) * 2 * nt + 2 * (size_t)term + (q & 1);
+}
+__device__ __forceinline__ bool look_live(const GkrBatchItem& it) { return !(it.mode == LOOK_ENTERS && (threadIdx.x & 4)); }
+// v0: the lane's entry, v1: the one it is fixed with, where there is one
+__device__ __forceinline__ void look_term(uint32_t (*acc)[2 * ACC_WORDS], const GkrBatchItem& it, bool live, uint32_t term, int terms_log, entry v0, entry v1, qm31 r,
+                                          qm31 half_lambda, qm31 ea) {
     const int lane = threadIdx.x & 31, q = lane & 7;
-    const size_t nt = (size_t)1 << terms_log, e = (size_t)(q >> 2) * 4 * nt + (size_t)((q >> 1) & 1) * 2 * nt + 2 * (size_t)term + (q & 1);
-    live = live && !(it.mode == LOOK_ENTERS && (q & 4));
+    live = live && look_live(it);
     entry v{qm31_zero(), qm31_zero()};
-    if (live) v = it.mode == LOOK_FIX ? fix_entry(it, e, 8 * nt, r) : load_entry(it, e);
+    if (live) v = it.mode == LOOK_FIX ? fix_entry(it, look_entry(term, terms_log), v0, v1, r) : v0;
     qm31 x = v.d, m = qm31_add(v.n, qmul(it.kind == ZKB_GKR_GRAND_PRODUCT ? qm31_from_m31(1u << 30) : half_lambda, x));
     const qm31 x0 = shflb(x, lane & ~2), m0 = shflb(m, lane & ~2);
     if (q & 2) { x = qm31_sub(qm31_dbl(x), x0); m = qm31_sub(qm31_dbl(m), m0); }
@@ -486,7 +497,7 @@ __device__ __forceinline__ void look_term(uint32_t (*acc)[2 * ACC_WORDS], const 
 
 // Warp 0 of CTA 0: the rounds from `from` on. act0: coefficient (lane & 3) of the first one's polynomial. `met` is the meeting with the other warps
 // once a round: the challenge is there, and so is `ahead`.
-__device__ __forceinline__ void look_met() { asm volatile("bar.sync 1, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 2)) : "memory"); }
+__device__ __forceinline__ void look_met() { asm volatile("bar.sync 1, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 3)) : "memory"); }
 __device__ __noinline__ void look_lead(GkrStepSm& sm, const GkrStepConst* consts, int from, int n_rounds, qm31 act0) {
     const int lane = threadIdx.x & 31, c4 = lane & 3;
     const QuadWords words(sm.ch.msg, sm.ch.sched);
@@ -534,7 +545,7 @@ __device__ __noinline__ void look_lead(GkrStepSm& sm, const GkrStepConst* consts
 __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* consts, const GkrTable* looks, const GkrStepState& s, const GkrAcc acc, GkrSync* sync, int from,
                                              int n_rounds, uint32_t* records) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = (lane >> 2) & 3, k = lane & 3, hn = lane >> 4;
-    const bool last_warp = warp == LOOK_LAST_WARP;
+    const bool last_warp = warp == LOOK_LAST_WARP, sends = warp == LOOK_SEND_WARP;
     const int value = look_value(warp), node = value & 1;
     qm31 corr = s.corr[lane];  // group `lane`'s
     bool gave_up = false;
@@ -552,7 +563,13 @@ __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* 
         const GkrStepConst &rc = consts[round], &rn = consts[next ? round + 1 : round];
         const GkrTable& tb = looks[round];
         const qm31 w0 = qm31_sub(qm31_one(), rc.y), w1 = qm31_sub(rc.y, w0);  // the next correction is corr (w0 + w1 r)
-        if (!last_warp) {
+        if (sends) {
+            // What the CTAs have folded, and the zeros of the round before, have to be there before the challenge that follows: the fence, some 700 cycles,
+            // stands beside the sums' way to the next polynomial.
+            if (!gave_up && tb.ctas && !wait_count(&sync->look_count[round], tb.ctas)) gave_up = true;
+            gave_up = __any_sync(0xffffffffu, gave_up);
+            __threadfence();
+        } else if (!last_warp) {
             if (round > from) {
                 const qm31 r = sm.look_r[(round & 1) ^ 1], y = consts[round - 1].y, omy = qm31_sub(qm31_one(), y);
                 const qm31_pair p = product_pair(r, y, qm31_sub(qm31_one(), r), omy);
@@ -575,7 +592,6 @@ __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* 
                 asm volatile("bar.arrive 2, %0;" ::"n"(32 * (LOOK_SUM_WARPS + 1)) : "memory");
                 if (mine) reinterpret_cast<ulonglong2*>(a)[0] = reinterpret_cast<ulonglong2*>(a)[1] = make_ulonglong2(0ull, 0ull);  // for the round after the next
             }
-            __threadfence();  // what the CTAs have folded, and the zeros, before the challenge that follows
         } else if (next) {
             // lane = 16 node + 4 c + k: that node's share of the coefficient of r^k in coefficient c
             const qm31 a = hn ? rn.B[c] : rn.A[c], a0 = qmul(a, w0), a1 = k == 0 ? a : qmul(a, w1), l1 = rn.L1[c];
@@ -591,7 +607,7 @@ __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* 
             if (lane < 16) sm.ahead[lane] = v;
         }
         look_met();
-        if (warp == 1 && lane < 4 && !gave_up) *reinterpret_cast<volatile uint32_t*>(&sync->slot[round + 1][lane]) = sm.look_r[round & 1].c[lane] | 0x80000000u;
+        if (sends && lane < 4 && !gave_up) *reinterpret_cast<volatile uint32_t*>(&sync->slot[round + 1][lane]) = sm.look_r[round & 1].c[lane] | 0x80000000u;
     }
     if (warp == 2) record(n_rounds - 1);
     return gave_up;
@@ -819,6 +835,20 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
                 if (tb.form == 3 && live) ea = qmul(eq_at(term), ldqb(alpha_pow, (uint32_t)it.slot));
             };
             look_up();
+            entry v0{qm31_zero(), qm31_zero()}, v1 = v0;
+            auto load = [&] {
+                if (!live || !look_live(it)) return;
+                const size_t e = look_entry(term, tb.terms_log);
+                v0 = load_entry(it, e);
+                if (it.mode == LOOK_FIX) v1 = load_entry(it, e + ((size_t)8 << tb.terms_log));
+            };
+            // The layer is whole when the pass before is counted, some 2,000 cycles before the challenge: the first piece's entries are on their way then.
+            const bool early = tb.form == 3 && t > look_from;
+            if (early) {
+                if (tid == 0 && !wait_count(&sync->look_count[t - 1], looks[t - 1].ctas)) gave_up = true;
+                __syncthreads();
+                load();
+            }
             if (t > look_from) {
                 if (tid < 4) {
                     uint32_t w = ld_acquire(&sync->slot[t][tid]);
@@ -834,8 +864,10 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
             const qm31 r = r_sh;
             for (;;) {
                 if (tid >> tb.run_log) {  // (whole warps)
-                } else if (tb.form == 3) look_term(sums, it, live, term, tb.terms_log, r, half_lambda, ea);
-                else if (live && tb.form == 4) fix_entry(it, tid & 3, 4, r);
+                } else if (tb.form == 3) {
+                    if (!early || chunk != block) load();
+                    look_term(sums, it, live, term, tb.terms_log, v0, v1, r, half_lambda, ea);
+                } else if (live && tb.form == 4) fix_entry(it, tid & 3, load_entry(it, tid & 3), load_entry(it, (tid & 3) + 4), r);
                 else if (live) fix_mask(it, (int)term, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
                 chunk += tb.ctas;
                 if (chunk >= tb.chunks) break;
