@@ -302,3 +302,13 @@ def test_transforms_where_short_columns_share_a_warp(ctx, oracle, log_n, n_cols,
     outs = ctx.alloc(n_cols << (log_n + 1))
     ctx.lde_cols(ptrs, log_n, [outs.ptr + 4 * (c << (log_n + 1)) for c in range(n_cols)], log_n + 1)
     assert (outs.download(shape=(n_cols, -1)) == oracle.evaluate_cols(coeffs, log_n, log_n + 1)).all()
+
+
+@pytest.mark.parametrize("log_rows,kw", [(9, {}), (10, {}), (10, dict(log_last_layer=2)), (11, {}), (13, dict(log_last_layer=9)), (15, {}), (16, {}), (17, {}), (17, dict(log_last_layer=14))])
+def test_fri_layers_of_many_ctas(ctx, oracle, log_rows, kw):
+    """First layers of 2^10 ... 2^18 values: none, some and all of the middle ones in one launch, the last one above and below where that ends."""
+    trees = [[m31_column(9100 + log_rows, 1 << log_rows), m31_column(9200, 1 << (log_rows - 3))], [m31_column(9300 + log_rows, 1 << log_rows)]]
+    kw = dict(pow_bits=4, log_blowup=1, n_queries=9, **kw)
+    want = oracle.pcs_prove(trees, **kw)
+    got = ctx.pcs_prove_host(trees, **kw)
+    assert len(got) == len(want) and (got == want).all()

@@ -45,6 +45,7 @@ struct zkb_ctx {
     int batch_grid = 0;  // CTAs of gkr_batch_layer_kernel that are resident at once
     uint32_t* h_batch = nullptr;
     bool fri_tail_ready = false;   // fri_tail.cu: the same
+    bool fri_mid_ready = false;   // fri_tail.cu: the same
     bool res_ready = false;        // gkr_resident.cu: its kernels' attributes are set on this device
     unsigned int batch_round = 0;  // sequence number of the last batched round launched
     cudaEvent_t events[64] = {nullptr};

@@ -17,19 +17,90 @@ namespace zk {
 
 constexpr int TAIL_THREADS = 512;
 constexpr size_t TAIL_N = (size_t)1 << FRI_TAIL_LOG;
-static_assert(TAIL_N / 2 <= TAIL_THREADS, "a layer folds to at most a value a thread");
+static_assert(TAIL_N / 2 <= TAIL_THREADS && TAIL_N >= 256, "a layer folds to at most a value a thread; the messages of 128 quads have room");
 
 __device__ __forceinline__ uint32_t bitrev_bits(uint32_t i, int bits) { return bits ? __brev(i) >> (32 - bits) : 0u; }
 
 // Dynamic shared memory: two layers of values, word by word, and two of hashes, pair by pair (pair_at).
 constexpr size_t TAIL_PAIRS = TAIL_N / 2 * PAIR_WORDS, TAIL_SMEM = (2 * 4 * TAIL_N + 2 * TAIL_PAIRS) * 4;
 
+// The levels lv ... 0 of a tree, or of a subtree, by a CTA of TAIL_THREADS: leaves from ev where lv is leaf_lv (coordinate c of leaf i at ev[c * ev_stride + i]), else nodes of the
+// pairs at `below`, which is ha or hb; one loop, so that the code of the hash is there once. Hash i of a level goes to out(level) + 8 i too. Returns
+// where warp 0 finds the root; the other warps may still be on their way.
+template <class Out>
+__device__ __forceinline__ uint32_t* hash_levels(uint32_t* const ha, uint32_t* const hb, uint32_t* below, const uint32_t* ev, size_t ev_stride, int lv, int leaf_lv, QuadWords& word,
+                                                 const QuadConst& qc, Out out) {
+    const int tid = threadIdx.x, warp = tid >> 5, l = tid & 3, quad = tid >> 2;
+    uint32_t* cur = below == ha ? hb : ha;
+    auto leaf_word = [&](int c, uint32_t i) { return ev[c * ev_stride + i]; };
+#pragma unroll 1
+    for (; lv >= 8; lv--) {
+        uint32_t* const o_level = out(lv);
+        const bool leaf = lv == leaf_lv;
+        for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
+            uint32_t h[8], m[16];
+            blake2s_init(h);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                if (!leaf) x = *reinterpret_cast<const uint4*>(below + PAIR_WORDS * i + 4 * q);
+                else if (q == 0) x = make_uint4(leaf_word(0, i), leaf_word(1, i), leaf_word(2, i), leaf_word(3, i));
+                m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
+            }
+            blake2s_compress(h, m, leaf ? 16u : 64u, true);
+#pragma unroll
+            for (int w = 0; w < 8; w++) h[w] = reduce_word_m31(h[w]);
+            const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
+            uint4 *const c = reinterpret_cast<uint4*>(cur + pair_at(i)), *const o = reinterpret_cast<uint4*>(o_level + 8 * (size_t)i);
+            c[0] = o[0] = lo;
+            c[1] = o[1] = hi;
+        }
+        uint32_t* const swap = cur;
+        cur = below;
+        below = swap;
+        __syncthreads();
+    }
+    // From 2^7 hashes down four lanes a hash, as in merkle_top_kernel; warps that have one meet at a barrier of their own, the others wait for
+    // the challenge.
+    if (lv == leaf_lv && 8 * warp < (1 << lv)) {
+        const uint32_t i = quad < (1 << lv) ? quad : 0;
+        *reinterpret_cast<uint4*>(below + PAIR_WORDS * quad + 4 * l) = l ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(leaf_word(0, i), leaf_word(1, i), leaf_word(2, i), leaf_word(3, i));
+        __syncwarp();
+    }
+    if (8 * warp < (1 << lv)) {
+        uint32_t* const parent = ha + pair_at(quad) + l;
+        const uint32_t apart = (uint32_t)(hb - ha);
+        uint32_t side = below == ha ? 0u : 1u;  // which of the two the messages are in
+#pragma unroll 1
+        while (true) {
+            uint32_t* const o = out(lv) + 8 * quad + l;
+            const bool live = quad < (1 << lv);
+            const int meet = lv >= 3 ? 4 << lv : 32;
+            word.at = side * (apart * 4u);
+            side ^= 1u;
+            uint32_t* const c = parent + side * apart;
+            uint2 h = b2s_compress_quad(make_uint2(qc.h0, qc.h1), word, qc, lv == leaf_lv ? 16u : 64u, 0xffffffffu);
+            h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
+            c[0] = h.x;
+            c[4] = h.y;
+            asm volatile("bar.sync 1, %0;" ::"r"(meet) : "memory");
+            if (live) {
+                o[0] = h.x;
+                o[4] = h.y;
+            }
+            if (--lv < 0 || 8 * warp >= (1 << lv)) break;
+        }
+        below = side ? hb : ha;
+    }
+    return below;
+}
+
 __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_constant__ FriTailArgs a, const uint32_t* __restrict__ itw) {
     extern __shared__ uint32_t dyn[];
     __shared__ ChanSm ch;
     __shared__ uint32_t alpha_w[4];
     uint32_t *ev = dyn, *ev_next = ev + 4 * TAIL_N, *const ha = ev_next + 4 * TAIL_N, *const hb = ha + TAIL_PAIRS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l = tid & 3, quad = tid >> 2;
+    const int tid = threadIdx.x, lane = tid & 31, quad = tid >> 2;
     const QuadConst qc;
     chan_make_schedule(ch, tid, TAIL_THREADS);
     if (tid < 32) ch.msg[tid] = tid < 8 ? (a.chan ? a.chan[tid] : a.digest[tid]) : 0u;
@@ -42,74 +113,12 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
     QuadWords word(ha + PAIR_WORDS * quad, ch.sched);
     for (int k = 0; k < a.n_layers; k++) {
         const int log = a.first_log - k;
-        uint32_t *cur = ha, *below = hb;
         // the fold's twiddle (a layer folds to at most a value a thread) is on its way while the tree is hashed
         const uint32_t half = 1u << (log - 1), mine = (uint32_t)tid < half ? (uint32_t)tid : 0u;
         uint32_t t, ix;
         if (a.circle && k == 0) half_coset_point(itw, log, mine, ix, t);
         else t = itw[half + mine];  // T_log^-1 starts at 2^(log - 1)
-        // leaves (level log) and nodes: one loop, so that the code of the hash is there once
-        int lv = log;
-#pragma unroll 1
-        for (; lv >= 8; lv--) {
-            uint32_t* const out = a.tree[k] + ((size_t)8 << lv);
-            const bool leaf = lv == log;
-            for (uint32_t i = tid; i < (1u << lv); i += TAIL_THREADS) {
-                uint32_t h[8], m[16];
-                blake2s_init(h);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    uint4 x = make_uint4(0u, 0u, 0u, 0u);
-                    if (!leaf) x = *reinterpret_cast<const uint4*>(below + PAIR_WORDS * i + 4 * q);
-                    else if (q == 0) x = make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
-                    m[4 * q] = x.x; m[4 * q + 1] = x.y; m[4 * q + 2] = x.z; m[4 * q + 3] = x.w;
-                }
-                blake2s_compress(h, m, leaf ? 16u : 64u, true);
-#pragma unroll
-                for (int w = 0; w < 8; w++) h[w] = reduce_word_m31(h[w]);
-                const uint4 lo = make_uint4(h[0], h[1], h[2], h[3]), hi = make_uint4(h[4], h[5], h[6], h[7]);
-                uint4 *const c = reinterpret_cast<uint4*>(cur + pair_at(i)), *const o = reinterpret_cast<uint4*>(out + 8 * (size_t)i);
-                c[0] = o[0] = lo;
-                c[1] = o[1] = hi;
-            }
-            uint32_t* const swap = cur;
-            cur = below;
-            below = swap;
-            __syncthreads();
-        }
-        // From 2^7 hashes down four lanes a hash, as in merkle_top_kernel; warps that have one meet at a barrier of their own, the others wait for
-        // the challenge.
-        if (lv == log && 8 * warp < (1 << lv)) {
-            const uint32_t i = quad < (1 << lv) ? quad : 0;
-            *reinterpret_cast<uint4*>(below + PAIR_WORDS * quad + 4 * l) = l ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(ev[i], ev[TAIL_N + i], ev[2 * TAIL_N + i], ev[3 * TAIL_N + i]);
-            __syncwarp();
-        }
-        if (8 * warp < (1 << lv)) {
-            uint32_t* const parent = ha + pair_at(quad) + l;
-            uint32_t* const mine_out = a.tree[k] + 8 * quad + l;
-            const uint32_t apart = (uint32_t)TAIL_PAIRS;
-            uint32_t side = below == ha ? 0u : 1u;  // which of the two the messages are in
-#pragma unroll 1
-            while (true) {
-                uint32_t* const o = mine_out + ((size_t)8 << lv);
-                const bool live = quad < (1 << lv);
-                const int meet = lv >= 3 ? 4 << lv : 32;
-                word.at = side * (apart * 4u);
-                side ^= 1u;
-                uint32_t* const c = parent + side * apart;
-                uint2 h = b2s_compress_quad(make_uint2(qc.h0, qc.h1), word, qc, lv == log ? 16u : 64u, 0xffffffffu);
-                h = make_uint2(reduce_word_m31(h.x), reduce_word_m31(h.y));
-                c[0] = h.x;
-                c[4] = h.y;
-                asm volatile("bar.sync 1, %0;" ::"r"(meet) : "memory");
-                if (live) {
-                    o[0] = h.x;
-                    o[4] = h.y;
-                }
-                if (--lv < 0 || 8 * warp >= (1 << lv)) break;
-            }
-            below = side ? hb : ha;
-        }
+        const uint32_t* const below = hash_levels(ha, hb, hb, ev, TAIL_N, log, log, word, qc, [&](int lv) { return a.tree[k] + ((size_t)8 << lv); });
         // the root is in warp 0's below[0, 8): mix it in, draw the challenge
         if (tid < 32) {
             if (lane < 8) {
@@ -183,6 +192,105 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
     if (lane == 10) a.out[10] = 0xffffffffu;
 }
 
+// The layers above those, of up to 2^FRI_MID_LOG values, in one cooperative launch of up to 128 CTAs. A fold takes neighbouring values, so a CTA keeps its slice of
+// the values from layer to layer in shared memory and hashes the subtree above it; what goes round in a layer is the subtrees' roots, to CTA 0, and the
+// challenge back, both with a bit in every word that says that it is there (words of a hash and coordinates are below 2^31; the bit's value changes with
+// every use of the slot): neither waits for a fence or a count. CTA 0 hashes the levels above the subtrees and keeps the channel.
+//
+// As launches (fold and leaves, levels, top with the channel step) a layer of 2^11 ... 2^17 values took 16-33 us, whose chain of hashes is
+// 9-14. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
+// polls (a second) a CTA leaves; the channel's done word then stays zero.
+constexpr uint32_t MID_SPINS = 1u << 21;
+constexpr size_t MID_N = (size_t)1 << (FRI_MID_LOG - FRI_MID_CTAS_LOG), MID_PAIRS = MID_N / 2 * PAIR_WORDS, MID_SMEM = (2 * 4 * MID_N + 2 * MID_PAIRS) * 4;  // the largest slice
+static_assert(MID_N / 2 <= TAIL_THREADS && MID_N >= 256 && ((size_t)1 << FRI_MID_CTAS_LOG) <= MID_N, "a slice folds to at most a value a thread; quads and roots have room");
+__device__ __forceinline__ bool mid_wait(const uint32_t* slot, uint32_t there, uint32_t& w) {
+    for (uint32_t spin = 0; spin < MID_SPINS; spin++) {
+        w = *reinterpret_cast<const volatile uint32_t*>(slot);
+        if (w >> 31 == there) {
+            w &= 0x7fffffffu;
+            return true;
+        }
+    }
+    return false;
+}
+__global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_constant__ FriMidArgs a, const uint32_t* __restrict__ itw) {
+    extern __shared__ uint32_t dyn[];
+    __shared__ ChanSm ch;
+    __shared__ uint32_t alpha_w[4];
+    __shared__ bool gave_up;
+    uint32_t *ev = dyn, *ev_next = ev + 4 * MID_N, *const ha = ev_next + 4 * MID_N, *const hb = ha + MID_PAIRS;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, cta = blockIdx.x, ctas = 1u << a.log_ctas;
+    const QuadConst qc;
+    chan_make_schedule(ch, (int)tid, TAIL_THREADS);
+    if (tid == 0) gave_up = false;
+    if (cta == 0) {
+        if (tid < 32) ch.msg[tid] = tid < 8 ? a.chan[tid] : 0u;
+        if (tid == 0) ch.n_draws = a.chan[8];
+    }
+    int slice_log = a.first_log - a.log_ctas;
+    for (uint32_t i = tid; i < 4u << slice_log; i += TAIL_THREADS) {
+        const uint32_t c = i >> slice_log, r = i & ((1u << slice_log) - 1);
+        ev[c * MID_N + r] = a.src[c][((size_t)cta << slice_log) + r];
+    }
+    __syncthreads();
+    QuadWords word(ha + PAIR_WORDS * (tid >> 2), ch.sched);
+    for (int k = 0; k < a.n_layers; k++, slice_log--) {
+        const int log = a.first_log - k;
+        const uint32_t there = (k >> 1 & 1) ^ 1u;
+        uint32_t *const root_slots = a.sync + (size_t)(k & 1) * 8 * ctas, *const alpha_slot = a.sync + 16 * ctas + 4 * (k & 1);
+        const uint32_t half = 1u << (slice_log - 1), mine = tid < half ? tid : 0u, fold_at = (cta << (slice_log - 1)) + mine;
+        uint32_t t, ix;
+        if (a.circle && k == 0) half_coset_point(itw, log, fold_at, ix, t);
+        else t = itw[(1u << (log - 1)) + fold_at];
+        const uint32_t* below = hash_levels(ha, hb, hb, ev, MID_N, slice_log, slice_log, word, qc,
+                                            [&](int lv) { return a.tree[k] + ((size_t)8 << (lv + a.log_ctas)) + (((size_t)8 * cta) << lv); });
+        if (tid < 8) *reinterpret_cast<volatile uint32_t*>(root_slots + 8 * cta + tid) = below[tid] | there << 31;
+        if (cta == 0) {
+            __syncthreads();
+            for (uint32_t i = tid; i < 8 * ctas; i += TAIL_THREADS) {
+                uint32_t w = 0;
+                if (!mid_wait(root_slots + i, there, w)) gave_up = true;
+                ha[pair_at(i >> 3) + (i & 7u)] = w;
+            }
+            __syncthreads();
+            if (gave_up) return;
+            below = hash_levels(ha, hb, ha, ev, MID_N, a.log_ctas - 1, -1, word, qc, [&](int lv) { return a.tree[k] + ((size_t)8 << lv); });
+            if (tid < 32) {
+                if (lane < 8) {
+                    const uint32_t w = below[lane];
+                    ch.msg[8 + lane] = w;
+                    a.roots[8 * k + lane] = w;
+                }
+                chan_step(ch, 8, 1, alpha_w);
+                if (lane < 4) *reinterpret_cast<volatile uint32_t*>(alpha_slot + lane) = alpha_w[lane] | there << 31;
+            }
+        } else if (tid < 4) {
+            uint32_t w = 0;
+            if (!mid_wait(alpha_slot + tid, there, w)) gave_up = true;
+            alpha_w[tid] = w;
+        }
+        __syncthreads();
+        if (gave_up) return;
+        const qm31 alpha{{alpha_w[0], alpha_w[1], alpha_w[2], alpha_w[3]}};
+        if (tid < half) {
+            qm31 x, y;
+#pragma unroll
+            for (int c = 0; c < 4; c++) { x.c[c] = ev[c * MID_N + 2 * tid]; y.c[c] = ev[c * MID_N + 2 * tid + 1]; }
+            const qm31 r = qm31_add(qm31_add(x, y), qm31_mul(alpha, qm31_mul_m31(qm31_sub(x, y), t)));
+#pragma unroll
+            for (int c = 0; c < 4; c++) { ev_next[c * MID_N + tid] = r.c[c]; a.evals[k][((size_t)c << (log - 1)) + fold_at] = r.c[c]; }
+        }
+        uint32_t* const swap = ev;
+        ev = ev_next;
+        ev_next = swap;
+        __syncthreads();
+    }
+    if (cta || tid >= 32) return;
+    if (lane < 8) a.chan[lane] = ch.msg[lane];
+    if (lane == 8) a.chan[8] = ch.n_draws;
+    if (lane == FRI_MID_DONE) a.chan[FRI_MID_DONE] = 1u;
+}
+
 __global__ void __launch_bounds__(256) grind_first_kernel(const uint32_t* __restrict__ prefixed, int pow_bits, unsigned int* __restrict__ best) {
     const uint32_t lo = blockIdx.x * 256u + threadIdx.x;
     uint32_t h[8], m[16];
@@ -210,6 +318,35 @@ int fri_tail(zkb_ctx* ctx, const FriTailArgs& args) {
     ProfScope prof(ctx, "fri_tail_kernel");
     fri_tail_kernel<<<1, TAIL_THREADS, TAIL_SMEM, ctx->stream>>>(args, ctx->itw);
     ZKB_LAUNCH_CHECK(ctx);
+    return ZKB_OK;
+}
+
+int fri_mid(zkb_ctx* ctx, const FriMidArgs& args) {
+    ZKB_CHECK_ARG(ctx, args.n_layers >= 1 && args.n_layers <= FRI_MID_LOG - FRI_MID_END && args.first_log <= FRI_MID_LOG && args.first_log - args.n_layers >= FRI_MID_END);
+    ZKB_CHECK_ARG(ctx, args.first_log <= ctx->max_log - (args.circle ? 0 : 1));
+    ZKB_CHECK_ARG(ctx, args.log_ctas == fri_mid_ctas_log(args.first_log));
+    DeviceGuard g(ctx);
+    if (!ctx->fri_mid_ready) {
+        ZKB_CUDA(ctx, cudaFuncSetAttribute(fri_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MID_SMEM));
+        ctx->fri_mid_ready = true;
+    }
+    ProfScope prof(ctx, "fri_mid_kernel");
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails
+    attr[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1u << args.log_ctas);
+    cfg.blockDim = dim3(TAIL_THREADS);
+    cfg.dynamicSmemBytes = MID_SMEM;
+    cfg.stream = ctx->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, fri_mid_kernel, args, (const uint32_t*)ctx->itw);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        return FRI_MID_REFUSED;
+    }
+    ZKB_CUDA(ctx, e);
     return ZKB_OK;
 }
 

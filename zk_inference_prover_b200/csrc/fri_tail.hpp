@@ -7,7 +7,7 @@ struct zkb_ctx;
 
 namespace zk {
 
-constexpr int FRI_TAIL_LOG = 10;         // largest layer (log2) the launch takes
+constexpr int FRI_TAIL_LOG = 10;        // largest layer (log2) the launch takes
 constexpr int FRI_TAIL_MAX_LAST = 5;     // largest last layer (log2) it interpolates
 constexpr int FRI_TAIL_MAX_BOUND = 2;    // largest log2 of the last layer's coefficients it mixes into the channel
 
@@ -34,6 +34,26 @@ inline size_t fri_tail_out_words(int n_layers) { return FRI_TAIL_ROOTS + 8 * (si
 inline size_t fri_tail_stride(int log) { return log < 2 ? 4 : (size_t)1 << log; }
 
 int fri_tail(zkb_ctx* ctx, const FriTailArgs& args);
+
+// The layers above those in one launch of many CTAs. Where it runs it also takes the two largest that the other one could (a layer of 2^10 values takes one CTA 16 us,
+// sixteen of them 13); for those alone the launch does not pay: a proof of ten columns, domain 2^10: 236 us without it, 241 with; four columns, domain 2^14: 480
+// with neither, 437 with it down to 2^11, 423 down to 2^9.
+constexpr int FRI_MID_LOG = 17;        // largest layer (log2) it takes
+constexpr int FRI_MID_END = 8;         // what its last layer folds to is no smaller (log2)
+constexpr int FRI_MID_CTAS_LOG = 7;
+inline int fri_mid_ctas_log(int first_log) { return first_log - 6 < FRI_MID_CTAS_LOG ? first_log - 6 : FRI_MID_CTAS_LOG; }  // slices of 2^6 values and more
+constexpr int FRI_MID_DONE = 10;       // the word of the channel's sixteen that is one when the launch has ended well, zero before
+struct FriMidArgs {
+    const uint32_t* src[4];            // the first layer's coordinate columns
+    int first_log, n_layers, circle;   // as above; at least one layer, and the last one folds to no less than 2^FRI_MID_END values
+    int log_ctas;                      // fri_mid_ctas_log
+    uint32_t* tree[FRI_MID_LOG - FRI_MID_END];   // as above
+    uint32_t* evals[FRI_MID_LOG - FRI_MID_END];
+    uint32_t *chan, *roots, *sync;     // channel state, in and out; a root per layer; fri_mid_sync_words zeros
+};
+inline size_t fri_mid_sync_words(int log_ctas) { return ((size_t)16 << log_ctas) + 8; }
+constexpr int FRI_MID_REFUSED = -1001; // not all CTAs can be resident: nothing was launched
+int fri_mid(zkb_ctx* ctx, const FriMidArgs& args);
 // The first nonces (several times 2^pow_bits of them) tested against the digest at prefixed; the smallest that passes goes to *best.
 int grind_first(zkb_ctx* ctx, const uint32_t* prefixed, int pow_bits, uint32_t* best);
 // zkb_fold_circle_into_line_dalpha (leaves: ..._leaves, or null) into a line that counts as zero: it is neither cleared first nor read.

@@ -420,11 +420,42 @@ struct FriProver {
     MerkleProver first_tree;
     struct Inner { SecureColumnByCoords eval; MerkleProver tree; uint32_t fold_step; };
     std::vector<Inner> inner;
-    BaseColumn tail_slab;  // trees and layers of the launch that runs the last layers, which `inner` holds views of
+    BaseColumn mid_slab, tail_slab;  // trees and layers of the launches that run the middle and the last layers, which `inner` holds views of
     std::vector<qm31> last_layer_poly;
 
     bool have_nonce = false;  // the proof of work was searched for along with the commitment (grind_bits)
     uint64_t nonce = 0;
+
+    // Memory for n layers from 2^log on that one launch commits and folds: each one's tree and what it folds to (FriTailArgs).
+    static std::vector<std::pair<uint32_t*, uint32_t*>> layer_slab(const Device& d, BaseColumn& slab, uint32_t log, size_t n) {
+        size_t words = 0;
+        for (uint32_t k = 0; k < n; k++) words += ((size_t)16 << (log - k)) + 4 * zk::fri_tail_stride((int)(log - k) - 1);
+        slab = BaseColumn(d, words);
+        std::vector<std::pair<uint32_t*, uint32_t*>> places;
+        uint32_t* at = slab.ptr();
+        for (uint32_t k = 0; k < n; k++) {
+            uint32_t* const tree = at;
+            at += (size_t)16 << (log - k);
+            places.push_back({tree, at});
+            at += 4 * zk::fri_tail_stride((int)(log - k) - 1);
+        }
+        return places;
+    }
+    // Layers `first` and on, of 2^log values, which such a launch has committed; layer: the first of them, and what the last one folds to afterwards.
+    void adopt_layers(const Device& d, const SecureColumnByCoords& column, SecureColumnByCoords& layer, size_t first, uint32_t log,
+                      const std::vector<std::pair<uint32_t*, uint32_t*>>& places) {
+        for (size_t k = 0; k < places.size(); k++, log--) {
+            if (first + k == 0) first_tree = tree_view(d, places[k].first, log, column);
+            else {
+                Inner in{std::move(layer), {}, 1};
+                in.tree = tree_view(d, places[k].first, log, in.eval);
+                inner.push_back(std::move(in));
+            }
+            layer = SecureColumnByCoords();
+            for (int c = 0; c < 4; c++)
+                layer.columns[c] = BaseColumn::view(d, places[k].second + c * zk::fri_tail_stride((int)log - 1), (size_t)1 << (log - 1));
+        }
+    }
 
     // A tree in memory laid out as the tail's launch writes it (FriTailArgs::tree).
     static MerkleProver tree_view(const Device& d, uint32_t* tree, uint32_t log, const SecureColumnByCoords& eval) {
@@ -448,56 +479,85 @@ struct FriProver {
         if (config.line_fold_step == 1) {
             // Device-resident commit phase: every layer's tree, the channel step (mix the root, draw the
             // folding challenge) and the fold are enqueued back to back; the host reads all roots and the
-            // channel state once, after the last fold. Layers of at most 2^FRI_TAIL_LOG values run in one launch.
+            // channel state once, after the last fold. The last layers, of at most 2^FRI_TAIL_LOG values, run in one launch.
             const size_t n_layers = 1 + (inner_log > last_log ? inner_log - last_log : 0);
-            const size_t tail = first_log > (uint32_t)zk::FRI_TAIL_LOG ? std::min<size_t>(n_layers, first_log - zk::FRI_TAIL_LOG)
+            const size_t tail = first_log > (uint32_t)zk::FRI_TAIL_LOG ? std::min<size_t>(n_layers, first_log - zk::FRI_MID_END)
                                 : first_log >= 3 && inner_log >= last_log ? 0 : n_layers;  // the first layer of that launch
             const bool last_in_tail = tail < n_layers && last_log <= (uint32_t)zk::FRI_TAIL_MAX_LAST &&
                                       config.log_last_layer_degree_bound <= (uint32_t)zk::FRI_TAIL_MAX_BOUND;
-            // [channel 16 | challenges 4 each (16-byte aligned) | roots 8 each | the tail's results]
+            // Of the layers before that launch those of at most 2^FRI_MID_LOG values are one launch too; the others are launches of their own.
+            const size_t launched = first_log > (uint32_t)zk::FRI_MID_LOG ? std::min<size_t>(tail, first_log - zk::FRI_MID_LOG) : first_log > (uint32_t)zk::FRI_TAIL_LOG ? 0 : tail;
+            const size_t mid_layers = tail - launched;
+            const uint32_t mid_log = first_log - (uint32_t)launched;
+            // [the middle launch's meeting place | channel 16 | challenges 4 each (16-byte aligned) | roots 8 each | the tail's results]
+            const int mid_ctas_log = zk::fri_mid_ctas_log((int)mid_log);
+            const size_t sync_words = mid_layers ? zk::fri_mid_sync_words(mid_ctas_log) : 0;
             const size_t tail_at = 16 + 12 * tail, tail_layers = n_layers - tail;
-            BaseColumn fs(d, tail_at + zk::fri_tail_out_words((int)tail_layers));
-            uint32_t* chan = fs.ptr();
-            uint32_t* alphas = fs.ptr() + 16;
-            uint32_t* roots = fs.ptr() + 16 + 4 * tail;
+            BaseColumn fs(d, sync_words + tail_at + zk::fri_tail_out_words((int)tail_layers));
+            uint32_t* const sync = fs.ptr();
+            uint32_t* const chan = sync + sync_words;
+            uint32_t* alphas = chan + 16;
+            uint32_t* roots = chan + 16 + 4 * tail;
+            bool mid_done = false;
             if (tail > 0) {
-                uint32_t st[16] = {0};
-                for (int k = 0; k < 8; k++) st[k] = ch.digest()[k];
-                st[8] = ch.n_draws();
-                d.check(zk::upload_small(d.ctx(), chan, st, 16));
-                layer = SecureColumnByCoords(d, (size_t)1 << inner_log);
-                bool stepped = false;
-                MerkleProver::ChanStep step0{chan, alphas, roots};
-                fp.first_tree = MerkleProver::commit(d, column.refs(), nullptr, &step0, &stepped);
-                if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, fp.first_tree.layers[0].ptr(), alphas, roots));
-                // every fold but the last also hashes the leaves of the layer it produces: that layer is committed next
+                std::vector<uint32_t> st(sync_words + 16, 0u);
+                for (int k = 0; k < 8; k++) st[sync_words + k] = ch.digest()[k];
+                st[sync_words + 8] = ch.n_draws();
+                d.check(zk::upload_small(d.ctx(), sync, st.data(), st.size()));
                 HashColumn leaves;
-                bool have_leaves = tail > 1 && first_log >= 3;
-                B200Backend::fold_circle_into_line(d, layer, column, alphas, have_leaves ? &leaves : nullptr);
-                for (size_t k = 1; k < tail; k++) {
-                    Inner in{std::move(layer), {}, 1};
-                    std::vector<const BaseColumn*> refs = in.eval.refs();
-                    MerkleProver::ChanStep step{chan, alphas + 4 * k, roots + 8 * k};
-                    in.tree = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr, &step, &stepped);
-                    if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, in.tree.layers[0].ptr(), alphas + 4 * k, roots + 8 * k));
-                    have_leaves = k + 1 < tail;
-                    if (have_leaves) layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k, leaves);
-                    else layer = B200Backend::fold_line(d, in.eval, alphas + 4 * k);
-                    fp.inner.push_back(std::move(in));
+                bool have_leaves = false, stepped = false;
+                // Layers [k0, k1) as launches; every fold but the last also hashes the leaves of the layer it produces: that layer is committed next.
+                auto launch_layers = [&](size_t k0, size_t k1) {
+                    for (size_t k = k0; k < k1; k++) {
+                        MerkleProver::ChanStep step{chan, alphas + 4 * k, roots + 8 * k};
+                        Inner in{std::move(layer), {}, 1};
+                        std::vector<const BaseColumn*> refs = k ? in.eval.refs() : column.refs();
+                        MerkleProver tree = MerkleProver::commit(d, refs, have_leaves ? &leaves : nullptr, &step, &stepped);
+                        if (!stepped) d.check(zkb_channel_mix_root_draw(d.ctx(), chan, tree.layers[0].ptr(), alphas + 4 * k, roots + 8 * k));
+                        have_leaves = k + 1 < k1 && (k > 0 || first_log >= 3);
+                        if (k == 0) {
+                            layer = SecureColumnByCoords(d, (size_t)1 << inner_log);
+                            B200Backend::fold_circle_into_line(d, layer, column, alphas, have_leaves ? &leaves : nullptr);
+                            fp.first_tree = std::move(tree);
+                            continue;
+                        }
+                        layer = have_leaves ? B200Backend::fold_line(d, in.eval, alphas + 4 * k, leaves) : B200Backend::fold_line(d, in.eval, alphas + 4 * k);
+                        in.tree = std::move(tree);
+                        fp.inner.push_back(std::move(in));
+                    }
+                };
+                launch_layers(0, launched);
+                if (mid_layers) {
+                    zk::FriMidArgs ma;
+                    memset(&ma, 0, sizeof(ma));
+                    const std::vector<std::pair<uint32_t*, uint32_t*>> places = fp.layer_slab(d, fp.mid_slab, mid_log, mid_layers);
+                    for (size_t k = 0; k < mid_layers; k++) { ma.tree[k] = places[k].first; ma.evals[k] = places[k].second; }
+                    const auto src = launched ? layer.cptrs() : column.cptrs();
+                    for (int c = 0; c < 4; c++) ma.src[c] = src[c];
+                    ma.first_log = (int)mid_log;
+                    ma.n_layers = (int)mid_layers;
+                    ma.circle = launched == 0;
+                    ma.log_ctas = mid_ctas_log;
+                    ma.chan = chan;
+                    ma.roots = roots + 8 * launched;
+                    ma.sync = sync;
+                    const int rc = zk::fri_mid(d.ctx(), ma);
+                    if (rc == zk::FRI_MID_REFUSED) {
+                        fp.mid_slab = BaseColumn();
+                        launch_layers(launched, tail);
+                    } else {
+                        d.check(rc);
+                        mid_done = true;
+                        fp.adopt_layers(d, column, layer, launched, mid_log, places);
+                    }
                 }
             }
             if (tail_layers > 0) {
                 zk::FriTailArgs ta;
                 memset(&ta, 0, sizeof(ta));
                 const uint32_t log0 = first_log - (uint32_t)tail;
-                size_t words = 0;
-                for (uint32_t k = 0; k < tail_layers; k++) words += ((size_t)16 << (log0 - k)) + 4 * zk::fri_tail_stride((int)(log0 - k) - 1);
-                fp.tail_slab = BaseColumn(d, words);
-                uint32_t* at = fp.tail_slab.ptr();
-                for (uint32_t k = 0; k < tail_layers; k++) {
-                    ta.tree[k] = at; at += (size_t)16 << (log0 - k);
-                    ta.evals[k] = at; at += 4 * zk::fri_tail_stride((int)(log0 - k) - 1);
-                }
+                const std::vector<std::pair<uint32_t*, uint32_t*>> places = fp.layer_slab(d, fp.tail_slab, log0, tail_layers);
+                for (size_t k = 0; k < tail_layers; k++) { ta.tree[k] = places[k].first; ta.evals[k] = places[k].second; }
                 const auto src = tail ? layer.cptrs() : column.cptrs();
                 for (int c = 0; c < 4; c++) ta.src[c] = src[c];
                 ta.first_log = (int)log0;
@@ -506,32 +566,17 @@ struct FriProver {
                 if (tail) ta.chan = chan;
                 for (int k = 0; k < 8; k++) ta.digest[k] = ch.digest()[k];
                 ta.n_draws = ch.n_draws();
-                ta.out = fs.ptr() + tail_at;
+                ta.out = chan + tail_at;
                 ta.last_log = (int)last_log;
                 ta.last_bound = last_in_tail ? (int)config.log_last_layer_degree_bound : -1;
                 ta.pow_bits = grind_bits > 0 ? (uint32_t)grind_bits : 0u;
                 d.check(zk::fri_tail(d.ctx(), ta));
                 if (last_in_tail && grind_bits > 0) d.check(zk::grind_first(d.ctx(), ta.out + 16, grind_bits, ta.out + 10));
-                for (uint32_t k = 0; k < tail_layers; k++) {
-                    const uint32_t log = log0 - k;
-                    if (k > 0) {
-                        layer = SecureColumnByCoords();
-                        for (int c = 0; c < 4; c++)
-                            layer.columns[c] = BaseColumn::view(d, ta.evals[k - 1] + c * zk::fri_tail_stride((int)log), (size_t)1 << log);
-                    }
-                    if (tail + k == 0) fp.first_tree = tree_view(d, ta.tree[0], log, column);
-                    else {
-                        Inner in{std::move(layer), {}, 1};
-                        in.tree = tree_view(d, ta.tree[k], log, in.eval);
-                        fp.inner.push_back(std::move(in));
-                    }
-                }
-                layer = SecureColumnByCoords();
-                for (int c = 0; c < 4; c++)
-                    layer.columns[c] = BaseColumn::view(d, ta.evals[tail_layers - 1] + c * zk::fri_tail_stride((int)last_log), (size_t)1 << last_log);
+                fp.adopt_layers(d, column, layer, tail, log0, places);
             }
             const uint32_t* h = nullptr;  // one copy, one synchronisation
-            d.check(zk::read_small(d.ctx(), fs.ptr(), fs.len(), &h));
+            d.check(zk::read_small(d.ctx(), chan, fs.len() - sync_words, &h));
+            if (mid_done && h[zk::FRI_MID_DONE] != 1u) throw Error(ZKB_ETIMEOUT, "FRI: a layer's challenge did not arrive");
             const uint32_t* const state = tail_layers ? h + tail_at : h;
             HashWords dg;
             for (int k = 0; k < 8; k++) dg[k] = state[k];
