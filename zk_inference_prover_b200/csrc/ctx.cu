@@ -208,32 +208,41 @@ __global__ void gather_words_kernel(const uint32_t* const* __restrict__ addrs, s
     if (t < n) out[t] = *addrs[t];
 }
 
-// Everything a read plan asks for (gather_plan). Thread t < n_cells: cell t of the blocks (their out_off ascending, found by
-// bisection); then a word per word address; then eight words per hash address. The plan begins with the word addresses.
-struct PlanBlock { const uint32_t* const* cols; uint32_t ncols, idx, out_off, here; };  // idx: where its row indices start; here: cols is an offset into the plan
+// Everything a read plan asks for (gather_plan). Thread t < n_cells: cell t of the blocks (their out_off ascending; a CTA's first warp finds the block its
+// cells begin in, the threads go on from there); then a word per word address; then eight words per hash address. The plan begins with
+// the word addresses. With a launch a block beyond 2^20 cells, the 54 blocks of a micro segment took 119 us and as much in the gaps between them, now 14; 56 blocks of
+// 12 million cells 236 us and the gaps, now 120.
+struct PlanBlock { const uint32_t* const* cols; uint64_t out_off; uint32_t ncols, idx, here, pad; };  // idx: where its row indices start; here: cols is an offset into the plan
 __host__ __device__ __forceinline__ const uint32_t* const* plan_cols(const PlanBlock& b, const void* plan) {
     return b.here ? reinterpret_cast<const uint32_t* const*>(static_cast<const char*>(plan) + reinterpret_cast<uintptr_t>(b.cols)) : b.cols;
 }
-__global__ void __launch_bounds__(256) gather_plan_kernel(const PlanBlock* __restrict__ blocks, int n_blocks, const uint32_t* __restrict__ idx, uint32_t n_cells,
-                                                          const uint32_t* const* __restrict__ words, uint32_t n_words,
-                                                          const uint32_t* const* __restrict__ hashes, uint32_t n_hashes, uint32_t* __restrict__ out) {
-    uint32_t t = blockIdx.x * 256u + threadIdx.x;
-    if (t < n_cells) {
-        int lo = 0, hi = n_blocks - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (blocks[mid].out_off <= t) lo = mid; else hi = mid - 1;
+__global__ void __launch_bounds__(256) gather_plan_kernel(const PlanBlock* __restrict__ blocks, int n_blocks, const uint32_t* __restrict__ idx, uint64_t n_cells,
+                                                          const uint32_t* const* __restrict__ words, uint64_t n_words,
+                                                          const uint32_t* const* __restrict__ hashes, uint64_t n_hashes, uint32_t* __restrict__ out) {
+    __shared__ int first;
+    const uint64_t t0 = blockIdx.x * 256ull, t = t0 + threadIdx.x;
+    if (t0 < n_cells) {
+        if (threadIdx.x < 32) {  // the last block that begins at t0 or before, of all that have cells
+            int n = 0;
+            for (int b = threadIdx.x; b < n_blocks; b += 32) n += blocks[b].out_off <= t0;
+            n = __reduce_add_sync(0xffffffffu, n);
+            if (threadIdx.x == 0) first = n - 1;
         }
-        const PlanBlock b = blocks[lo];
-        const uint32_t e = t - b.out_off;
-        out[t] = plan_cols(b, words)[e % b.ncols][idx[b.idx + e / b.ncols]];
+        __syncthreads();
+    }
+    if (t < n_cells) {
+        int b = first;
+        while (b + 1 < n_blocks && blocks[b + 1].out_off <= t) b++;
+        const PlanBlock pb = blocks[b];
+        const uint32_t e = (uint32_t)(t - pb.out_off);
+        out[t] = plan_cols(pb, words)[e % pb.ncols][idx[pb.idx + e / pb.ncols]];
         return;
     }
     if (t < n_cells + n_words) {
         out[t] = *words[t - n_cells];
         return;
     }
-    const uint32_t h = t - n_cells - n_words;
+    const uint64_t h = t - n_cells - n_words;
     if (h < 8 * n_hashes) out[t] = hashes[h >> 3][h & 7];
 }
 
@@ -790,7 +799,7 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
             return rc;
         }
         if (g.nidx) memcpy(pi + first_idx, g.idx, 4 * (size_t)g.nidx);
-        pb[b] = {(const uint32_t* const*)cols, (uint32_t)g.ncols, (uint32_t)first_idx, (uint32_t)g.out_off, here ? 1u : 0u};
+        pb[b] = {(const uint32_t* const*)cols, g.out_off, (uint32_t)g.ncols, (uint32_t)first_idx, here ? 1u : 0u, 0u};
         first_idx += (size_t)g.nidx;
     }
     unsigned char *d_blob = nullptr, *d_own = nullptr;
@@ -810,21 +819,7 @@ int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t to
         const uint32_t* const* d_hashes = reinterpret_cast<const uint32_t* const*>(d_blob + at_hash);
         const PlanBlock* d_blocks = reinterpret_cast<const PlanBlock*>(d_blob + at_blocks);
         const uint32_t* d_idx = reinterpret_cast<const uint32_t*>(d_blob + at_idx);
-        // Up to 2^20 cells one launch reads everything; beyond, a launch per block, whose threads need no bisection.
-        const bool one = total_words <= ((size_t)1 << 20);
-        if (!one) {
-            for (int b = 0; b < n_blocks; b++) {
-                const size_t cells = (size_t)blocks[b].ncols * blocks[b].nidx;
-                if (cells)
-                    gather_multi_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, ctx->stream>>>(plan_cols(pb[b], d_blob), blocks[b].ncols, d_idx + pb[b].idx, blocks[b].nidx,
-                                                                                                  d_out + blocks[b].out_off);
-            }
-        }
-        const uint32_t cells = one ? (uint32_t)total_words : 0u;
-        const size_t threads = cells + n_words + 8 * n_hashes;
-        if (threads)
-            gather_plan_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(d_blocks, n_blocks, d_idx, cells, d_words, (uint32_t)n_words, d_hashes,
-                                                                                           (uint32_t)n_hashes, d_out + (one ? 0 : total_words));
+        gather_plan_kernel<<<(unsigned)((results + 255) / 256), 256, 0, ctx->stream>>>(d_blocks, n_blocks, d_idx, total_words, d_words, n_words, d_hashes, n_hashes, d_out);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, d_out, results * 4, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

@@ -8,7 +8,7 @@
 // 2^10 values 91 -> 86 us. As launches (fold and leaves, tree
 // top with channel step) a layer also paid two launches, the gaps around them and a dozen allocations for its arrays: a ten-column
 // proof of 2^8 rows spent 190 us of device time in them and as much on the host. Layers stay in shared memory; what the decommitment
-// reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs.
+// reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs: fri_mid_kernel below.
 #include "channel.cuh"
 #include "common.cuh"
 #include "fri_tail.hpp"
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
 // every use of the slot): neither waits for a fence or a count. CTA 0 hashes the levels above the subtrees and keeps the channel.
 //
 // As launches (fold and leaves, levels, top with the channel step) a layer of 2^11 ... 2^17 values took 16-33 us, whose chain of hashes is
-// 9-14. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
+// 9-14; the layers of 2^17 ... 2^9 values here and the rest in the tail's launch take 206 us, 298 before. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
 // polls (a second) a CTA leaves; the channel's done word then stays zero.
 constexpr uint32_t MID_SPINS = 1u << 21;
 constexpr size_t MID_N = (size_t)1 << (FRI_MID_LOG - FRI_MID_CTAS_LOG), MID_PAIRS = MID_N / 2 * PAIR_WORDS, MID_SMEM = (2 * 4 * MID_N + 2 * MID_PAIRS) * 4;  // the largest slice

@@ -26,8 +26,7 @@ struct GatherBlock {
 // Every cell of every block, every word of word_addrs and every hash (8 words) of hash_addrs, in one round trip: results go to
 // h_out as [blocks: total_words][one word per word address][eight words per hash address], which should be page-locked. A
 // decommitment's whole read plan (Column::batch_at and batch_at_multi, nitroo/crates/stwo/src/prover/backend/mod.rs:68-89, for all
-// the layers of all the trees at once): the addresses and indices travel in one staged block, and unless the blocks are wide one
-// launch reads everything.
+// the layers of all the trees at once): the addresses and indices travel in one staged block, and one launch reads everything.
 int gather_plan(zkb_ctx* ctx, const GatherBlock* blocks, int n_blocks, size_t total_words, const uint32_t* const* word_addrs, size_t n_words,
                 const uint32_t* const* hash_addrs, size_t n_hashes, uint32_t* h_out);
 
