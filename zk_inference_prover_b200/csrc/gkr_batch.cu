@@ -262,10 +262,10 @@ __device__ __forceinline__ void batch_step_open(GkrStepSm& sm, const GkrStepStat
     if (lane == 0) sm.ch.n_draws = st.n_draws;
     __syncwarp();
 }
-// The channel's state to where the next launch finds it.
-__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, GkrStepState* st, int lane) {
+// The channel's state (digest, n_draws) to where the next launch, or the host, finds it.
+__device__ __forceinline__ void batch_step_close(const GkrStepSm& sm, uint32_t* channel, int lane) {
     const uint32_t w = lane < 8 ? sm.ch.msg[lane] : lane == 8 ? sm.ch.n_draws : 0u;
-    if (lane < 12) reinterpret_cast<uint32_t*>(st)[lane] = w;
+    if (lane < 12) channel[lane] = w;
 }
 
 // What a layer brings back is written by its last launch into page-locked host memory (the masks by the threads that fix them; the
@@ -276,9 +276,8 @@ struct GkrLayerOut {
     volatile unsigned int* flag;
     unsigned int id;
 };
-__device__ __forceinline__ void layer_out_words(const GkrLayerOut& o, const uint32_t* records, int n_rounds, const GkrStepState* st, int i, int threads) {
-    for (int k = i; k < 6 * n_rounds; k += threads) reinterpret_cast<uint4*>(o.records)[k] = __ldcg(reinterpret_cast<const uint4*>(records) + k);
-    if (i < 3) reinterpret_cast<uint4*>(o.channel)[i] = __ldcg(reinterpret_cast<const uint4*>(st) + i);
+__device__ __forceinline__ void layer_out_words(const GkrLayerOut& o, const uint32_t* records, int n_rounds, int i, int threads) {
+    for (int k = i; k < 6 * n_rounds; k += threads) reinterpret_cast<uint4*>(o.records)[k] = reinterpret_cast<const uint4*>(records)[k];
 }
 __device__ __forceinline__ qm31 acc_value(const unsigned long long* a) { return {{m31_reduce64(a[0]), m31_reduce64(a[1]), m31_reduce64(a[2]), m31_reduce64(a[3])}}; }
 
@@ -607,7 +606,7 @@ __device__ __forceinline__ bool look_helpers(GkrStepSm& sm, const GkrStepConst* 
             if (lane < 16) sm.ahead[lane] = v;
         }
         look_met();
-        if (sends && lane < 4 && !gave_up) *reinterpret_cast<volatile uint32_t*>(&sync->slot[round + 1][lane]) = sm.look_r[round & 1].c[lane] | 0x80000000u;
+        if (sends && next && lane < 4 && !gave_up) *reinterpret_cast<volatile uint32_t*>(&sync->slot[round + 1][lane]) = sm.look_r[round & 1].c[lane] | 0x80000000u;
     }
     if (warp == 2) record(n_rounds - 1);
     return gave_up;
@@ -815,14 +814,14 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
         const GkrTable* const looks = tabs + n_rounds + 1;
         const qm31 half_lambda = qm31_mul_m31(lambda, 1u << 30);
         const uint32_t block = blockIdx.x - 1;
-        for (int t = look_from; t <= n_rounds; t++) {
-            const GkrTable tb = t < n_rounds ? looks[t] : tabs[n_rounds];
+        for (int t = look_from; t < n_rounds; t++) {
+            const GkrTable tb = looks[t];
             if (block >= tb.ctas) {
                 if (block >= tb.later) return;
                 continue;
             }
             const GkrBatchItem* const items = items_base + tb.first;
-            const int lanes_log = tb.form == 3 ? 3 : tb.form == 4 ? 2 : 0;  // lanes a term (form 3), an item (4), of two threads an item (2)
+            const int lanes_log = tb.form == 3 ? 3 : 2;  // lanes a term (form 3), an item (4)
             uint32_t chunk = block, term = 0;
             GkrBatchItem it{};
             bool live = false;
@@ -867,8 +866,7 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
                 } else if (tb.form == 3) {
                     if (!early || chunk != block) load();
                     look_term(sums, it, live, term, tb.terms_log, v0, v1, r, half_lambda, ea);
-                } else if (live && tb.form == 4) fix_entry(it, tid & 3, load_entry(it, tid & 3), load_entry(it, (tid & 3) + 4), r);
-                else if (live) fix_mask(it, (int)term, r, host.masks + 16 * (size_t)(uint32_t)it.slot);
+                } else if (live) fix_entry(it, tid & 3, load_entry(it, tid & 3), load_entry(it, (tid & 3) + 4), r);
                 chunk += tb.ctas;
                 if (chunk >= tb.chunks) break;
                 look_up();
@@ -881,24 +879,26 @@ __global__ void __launch_bounds__(GKR_THREADS, 1) gkr_batch_layer_kernel(const G
                     h[0] = h[1] = 0u;
                     if (v) atomicAdd(acc.at(t + 1, 0) + i, v);
                 }
-            if (t == n_rounds) __threadfence_system();
             __syncthreads();
-            if (tid == 0) { __threadfence(); atomicAdd(t < n_rounds ? &sync->look_count[t] : &sync->count[t], 1u); }
+            if (tid == 0) { __threadfence(); atomicAdd(&sync->look_count[t], 1u); }
         }
         return;
     }
     if (!lead) return;
     __syncthreads();
     if (gave_up) return;
+    // What the rounds ahead leave, four entries an oracle, is fixed here: the challenge is, and it goes to the host with the rest. (As one more pass of the
+    // CTAs, each with its fence for the host, the masks took 9,700 cycles of a layer, and the channel by way of memory 1,400.)
     if (look_from >= 0) {
-        if (tid == 0 && !wait_count(&sync->count[n_rounds], tabs[n_rounds].ctas)) gave_up = true;
-        __syncthreads();
-        if (gave_up) return;
+        const GkrTable& tb = tabs[n_rounds];
+        const qm31 r = sm.look_r[(n_rounds - 1) & 1];
+        for (uint32_t i = tid; i < 2 * tb.n_items; i += GKR_THREADS) {
+            const GkrBatchItem it = items_base[tb.first + (i >> 1)];
+            fix_mask(it, (int)(i & 1), r, host.masks + 16 * (size_t)(uint32_t)it.slot);
+        }
     }
-    if (warp == 0) batch_step_close(sm, st, lane);
-    __threadfence();
-    __syncthreads();
-    layer_out_words(host, records, n_rounds, st, tid, GKR_THREADS);
+    if (warp == 0) batch_step_close(sm, host.channel, lane);
+    layer_out_words(host, records, n_rounds, tid, GKR_THREADS);
     __threadfence_system();
     __syncthreads();
     if (tid == 0) *host.flag = host.id;
@@ -915,7 +915,8 @@ __global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, Gk
         __syncwarp();
     }
     if (t == n_rounds) {
-        layer_out_words(host, records, n_rounds, st, lane, 32);
+        layer_out_words(host, records, n_rounds, lane, 32);
+        if (lane < 12) host.channel[lane] = reinterpret_cast<const uint32_t*>(st)[lane];
         __threadfence_system();
         __syncwarp();
         if (lane == 0) *host.flag = host.id;
@@ -930,7 +931,7 @@ __global__ void __launch_bounds__(32) gkr_batch_step_kernel(GkrStepState* st, Gk
     batch_step_open(sm, *st, lane);
     batch_step(sm, *st, rc[t], acc_value(a), acc_value(a + 4), records + GKR_LAYER_OUT_WORDS * (size_t)t, [] {});
     if (lane < 4) sync->slot[t + 1][lane] = sm.r.c[lane] | 0x80000000u;
-    batch_step_close(sm, st, lane);
+    batch_step_close(sm, reinterpret_cast<uint32_t*>(st), lane);
 }
 
 // ---- a single round with its results to the host
@@ -1232,7 +1233,7 @@ static void plan_look(GkrLayerPlan& plan, uint32_t grid) {
         tb.run_log = LOOK_MIN_LOG;
         while (tb.run_log < GKR_THREADS_LOG && ((lanes + (1u << tb.run_log) - 1) >> tb.run_log) > grid - 1) tb.run_log++;
         tb.chunks = (uint32_t)((lanes + (1u << tb.run_log) - 1) >> tb.run_log);
-        tb.ctas = std::min(tb.chunks, grid - 1);
+        tb.ctas = j == n ? 0u : std::min(tb.chunks, grid - 1);  // (CTA 0 has the masks)
     }
     uint32_t later = 0;
     for (int j = n; j >= from; j--) {
