@@ -1,5 +1,5 @@
 """Proofs at the sizes where the library changes how it runs them, word for word against the oracle: FRI layers that fit the
-one-launch tail (2^10 values), those that many thread blocks take in one launch (2^17) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
+one-launch tail (2^10 values), those that many thread blocks take in one launch (2^15) and those above, last layers it interpolates and those it leaves to the host; GKR instances around
 the layer sizes one CTA takes (2^13 entries), passes of one term per lane, of several and of more than the small form's limit;
 batches whose towers take one launch (2^10 entries) and two; samples whose quotient lines are worked out on the host and on the
 device (from 512 on, in pieces of 1,024); trees hashed on a second stream, quotients planned on a second thread, decommitments of a few

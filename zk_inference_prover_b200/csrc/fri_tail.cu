@@ -192,13 +192,13 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
     if (lane == 10) a.out[10] = 0xffffffffu;
 }
 
-// The layers above those, of up to 2^FRI_MID_LOG values, in one cooperative launch of up to 128 CTAs. A fold takes neighbouring values, so a CTA keeps its slice of
+// The layers above those, of up to 2^FRI_MID_LOG values, in one cooperative launch of up to 32 CTAs. A fold takes neighbouring values, so a CTA keeps its slice of
 // the values from layer to layer in shared memory and hashes the subtree above it; what goes round in a layer is the subtrees' roots, to CTA 0, and the
 // challenge back, both with a bit in every word that says that it is there (words of a hash and coordinates are below 2^31; the bit's value changes with
 // every use of the slot): neither waits for a fence or a count. CTA 0 hashes the levels above the subtrees and keeps the channel.
 //
-// As launches (fold and leaves, levels, top with the channel step) a layer of 2^11 ... 2^17 values took 16-33 us, whose chain of hashes is
-// 9-14; the layers of 2^17 ... 2^9 values here and the rest in the tail's launch take 206 us, 298 before. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
+// As launches (fold and leaves, levels, top with the channel step) a layer of 2^11 ... 2^15 values took 16-24 us, whose chain of hashes is
+// 9-12; a proof of four columns, domain 2^14: 470 us before, 428 with this launch. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
 // polls (a second) a CTA leaves; the channel's done word then stays zero.
 constexpr uint32_t MID_SPINS = 1u << 21;
 constexpr size_t MID_N = (size_t)1 << (FRI_MID_LOG - FRI_MID_CTAS_LOG), MID_PAIRS = MID_N / 2 * PAIR_WORDS, MID_SMEM = (2 * 4 * MID_N + 2 * MID_PAIRS) * 4;  // the largest slice

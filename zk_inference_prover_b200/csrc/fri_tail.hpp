@@ -37,10 +37,12 @@ int fri_tail(zkb_ctx* ctx, const FriTailArgs& args);
 
 // The layers above those in one launch of many CTAs. Where it runs it also takes the two largest that the other one could (a layer of 2^10 values takes one CTA 16 us,
 // sixteen of them 13); for those alone the launch does not pay: a proof of ten columns, domain 2^10: 236 us without it, 241 with; four columns, domain 2^14: 480
-// with neither, 437 with it down to 2^11, 423 down to 2^9.
-constexpr int FRI_MID_LOG = 17;        // largest layer (log2) it takes
+// with neither, 437 with it down to 2^11, 425 down to 2^9. Not from larger layers on with more CTAs: 128 from 2^17 on save a STARK proof another 50 us, but a CTA wants its SM
+// to itself, and beside other proofs' long kernels (chains of narrow tree layers, a CTA on most SMs for milliseconds) a grid of 128 waits for all of them with
+// the SMs it has: eight proofs side by side took 1.85 s a decode step, 1.05 with 32 CTAs and with launches alone.
+constexpr int FRI_MID_LOG = 15;        // largest layer (log2) it takes
 constexpr int FRI_MID_END = 8;         // what its last layer folds to is no smaller (log2)
-constexpr int FRI_MID_CTAS_LOG = 7;
+constexpr int FRI_MID_CTAS_LOG = 5;
 inline int fri_mid_ctas_log(int first_log) { return first_log - 6 < FRI_MID_CTAS_LOG ? first_log - 6 : FRI_MID_CTAS_LOG; }  // slices of 2^6 values and more
 constexpr int FRI_MID_DONE = 10;       // the word of the channel's sixteen that is one when the launch has ended well, zero before
 struct FriMidArgs {
