@@ -73,6 +73,24 @@ def test_gkr_batch_around_what_a_launch_carries(ctx, oracle, log_n, n_inst):
     assert len(got) == len(want) and (got == want).all()
 
 
+@pytest.mark.parametrize("spec", [{16: 1, 13: 40}, {14: 1, 11: 120, 3: 2}, {15: 2, 12: 30, 9: 300}])
+def test_gkr_batch_with_rounds_that_grow(ctx, oracle, spec):
+    """Shorter instances that enter make a round large again: small rounds, large ones and small ones in a layer, those ahead of the transcript last."""
+    inst, dev, keep = [], [], []
+    for log_n, count in spec.items():
+        for i in range(count):
+            n, kind = 1 << log_n, (3, 0, 1, 2)[len(inst) % 4]
+            at = 7600 + 3 * len(inst)
+            den = qm31_array(at, n, nonzero=True)
+            num = qm31_array(at + 1, n) if kind == 1 else m31_column(at + 2, n) if kind == 2 else None
+            inst.append((kind, num, den))
+            keep += [ctx.upload(num) if num is not None else None, ctx.upload(den)]
+            dev.append((kind, keep[-2].ptr if num is not None else 0, keep[-1].ptr, n))
+    want = oracle.gkr_prove(inst, 0x5EED0018, verify=True)
+    got = ctx.gkr_prove_device(dev, 0x5EED0018)
+    assert len(got) == len(want) and (got == want).all()
+
+
 @pytest.mark.parametrize("log_n", [2, 9, 10, 11, 12])
 def test_gkr_batch_around_the_tower_launches(ctx, oracle, log_n):
     inst, dev, keep = [], [], []

@@ -302,8 +302,9 @@ __device__ __forceinline__ void item_sums_of(const GkrBatchItem& it, size_t firs
 }
 
 // The terms of `g` neighbouring lanes (a power of two up to 32) are one item's: they are added up, taken times the item's power of
-// alpha and added to its group's sums in shared memory, as 16-bit halves (32-bit adds, no carries to fold; 2^16 terms fit). By
-// whole warps; adds: the lane belongs to an item.
+// alpha and added to its group's sums in shared memory, as 16-bit halves (32-bit adds, no carries to fold; 2^16 additions
+// fit: a piece makes 16 to a counter for items of 32 terms and more, and the largest layer that 180 GB hold, 2^31 terms, is some 3,600 pieces for
+// each of 148 CTAs; smaller items, of which a launch has at most 2^13, are two pieces). By whole warps; adds: the lane belongs to an item.
 __device__ __forceinline__ void add_to_group(uint32_t (*acc)[2 * ACC_WORDS], int g, bool adds, uint32_t oracle, uint32_t group, const uint32_t* __restrict__ alpha_pow, qm31 s0, qm31 s2) {
     const int lane = threadIdx.x & 31, sub = lane & (g - 1);
     const qm31 a = adds ? ldqb(alpha_pow, oracle) : qm31_zero();
@@ -347,7 +348,7 @@ __device__ __forceinline__ void add_to_group(uint32_t (*acc)[2 * ACC_WORDS], int
 //
 // The waits end: every CTA is resident (the launch is refused otherwise), a CTA waits only for what the others do before they wait
 // themselves, and after SPIN_LIMIT polls (about a second) it gives up and leaves; the host then sees no layer number and reports it.
-constexpr int GKR_THREADS_LOG = 9, GKR_THREADS = 1 << GKR_THREADS_LOG;
+constexpr int GKR_THREADS = 1 << GKR_THREADS_LOG;
 constexpr int LOOK_MIN_LOG = 7;                  // the fewest threads (log2) that a CTA is given work for
 constexpr uint32_t SPIN_LIMIT = 1u << 21;
 
@@ -449,7 +450,8 @@ __device__ __forceinline__ entry fix_entry(const GkrBatchItem& it, size_t e, ent
 
 // Eight lanes a term of the next round, one for each of its entries: bit 2 the variable this round fixes, bit 1 the next round's, bit 0 the pair. A term is
 // n0 d1 + n1 d0 + lambda d0 d1 = m0 d1 + m1 d0 with m = n + k d, k = lambda / 2 (a grand product's d0 d1 with n = 0, k = 1 / 2). Lanes 0 and 2 end with the term at r
-// = 0, 4 and 6 with it at r = 1, 5 and 7 with its leading coefficient. ea: eq times the oracle's power of alpha.
+// = 0, 4 and 6 with it at r = 1, 5 and 7 with its leading coefficient. ea: eq times the oracle's power of alpha. The sums are 16-bit halves as in
+// add_to_group: at most 64 additions a piece to a counter, and gkr_look_from allows few pieces.
 __device__ __forceinline__ size_t look_entry(uint32_t term, int terms_log) {  // this lane's
     const int q = threadIdx.x & 7;
     const size_t nt = (size_t)1 << terms_log;
@@ -1184,19 +1186,16 @@ static LayerBlob layer_blob(const GkrLayerPlan& plan) {
 }
 static size_t open_words(const GkrLayerPlan& plan) { return open_alpha(plan.n_rounds) + 4 * plan.n_vars.size(); }
 
-// The rounds that are taken ahead of the transcript: from the first whose table takes four lanes a term. Larger ones are bound by their products, of which this
-// way has twice as many. Their tables go behind the others, and the items that are used into look_items.
+// The rounds that are taken ahead of the transcript (gkr_look_from). Their tables go behind the others, and the items that are used into look_items.
 static GkrTable* tables_of(GkrLayerPlan& plan) { return reinterpret_cast<GkrTable*>(plan.tables.data()); }
 static void plan_look(GkrLayerPlan& plan, uint32_t grid) {
     const int n = plan.n_rounds;
-    GkrTable* tables = tables_of(plan);
-    int from = 0;
-    while (from < n && tables[from].form != 1) from++;
-    plan.look_from = -1;
-    if (plan.launches || from + 2 > n || grid < 2) return;
-    plan.look_from = from;
+    size_t terms[GKR_LAYER_MAX_ROUNDS];
+    for (int j = 0; j < n; j++) terms[j] = (size_t)tables_of(plan)[j].n_items << tables_of(plan)[j].terms_log;
+    const int from = plan.look_from = plan.launches ? -1 : gkr_look_from(terms, n, grid);
+    if (from < 0) return;
     plan.tables.resize((sizeof(GkrTable) / 4) * (2 * (size_t)n + 1), 0u);
-    tables = tables_of(plan);
+    GkrTable* const tables = tables_of(plan);
     std::vector<GkrBatchItem>& out = plan.look_items;
     auto table = [&](int j) { return std::make_pair(plan.items.begin() + plan.table_at[j], plan.items.begin() + plan.table_at[j + 1]); };
     out.assign(plan.items.begin(), table(from).second);
@@ -1270,9 +1269,7 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
         // n_rounds - j variables are left: 2^(that - 1) terms an item; at the end two entries of a mask each
         tb.terms_log = j < n_rounds ? n_rounds - j - 1 : 1;
         const size_t terms = (size_t)nt << tb.terms_log;
-        // Four lanes a term while that is at most two passes of the whole grid: a pass of this form is a third of the other's latency,
-        // and a third more work.
-        tb.form = j == n_rounds ? 2 : 4 * terms <= 2 * (size_t)grid * GKR_THREADS ? 1 : 0;
+        tb.form = j == n_rounds ? 2 : gkr_four_lanes(terms, grid) ? 1 : 0;
         // Whole items of 2^GKR_THREADS_LOG terms and more: a thread takes up to eight terms for one reduction, as long as four pieces per CTA remain.
         tb.run_log = 0;
         if (tb.form == 0)

@@ -1,5 +1,6 @@
 // A layer's sum-check, or one round of it, for a GKR batch of any number of instances in one launch (gkr_batch.cu); internal to the library.
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -74,6 +75,32 @@ struct GkrLayerPlan {
     bool launches = false;           // the layer as a launch per table and one per transcript step
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
+
+// How a layer's rounds are taken, by their terms and the CTAs of the launch.
+constexpr int GKR_THREADS_LOG = 9;  // of a CTA
+// Four lanes a term while that is at most two passes of the whole grid: a pass of this form is a third of the other's latency,
+// and a third more work.
+inline bool gkr_four_lanes(size_t terms, uint32_t grid) { return 4 * terms <= 2 * ((size_t)grid << GKR_THREADS_LOG); }
+// The round from which on they are taken ahead of the transcript (gkr_batch.cu), or -1. terms[j]: round j's, of all the oracles that are active by then;
+// they fall by half from round to round, and grow where shorter oracles enter. A round ahead takes eight lanes for a term of the round after it: some
+// 4,500 cycles and 5,000 for 512 lanes a CTA, 9,500 at least, where an ordinary round takes 16,000 and for a large one less per term than this. So what all rounds
+// from a candidate on save has to make up for the large ones among them. One instance of 2^16 above 500 of 2^14: 5.2 ms with no round ahead, 7.3 from the first
+// small round on, 5.2 by this rule; of 2^14 above 300 of 2^13: 3.1, 3.3 and 2.8; 34 of 2^10 ... 2^13, whose rounds only fall: 1.10, 0.82 and 0.82. No pass has more than
+// 43 times 512 lanes a CTA then: 31 rounds do not save more (look_term's sums rest on it).
+inline int gkr_look_from(const size_t* terms, int n_rounds, uint32_t grid) {
+    constexpr int64_t ORDINARY = 16000, AHEAD = 9500, AHEAD_BASE = 4500, AHEAD_PIECE = 5000;
+    if (grid < 2) return -1;
+    int from = -1;
+    int64_t saved = 0, most = 0;
+    for (int j = n_rounds - 1; j >= 0; j--) {
+        const int64_t lanes = j + 1 < n_rounds ? 8 * (int64_t)terms[j + 1] : 0;
+        saved += ORDINARY - std::max(AHEAD, AHEAD_BASE + AHEAD_PIECE * lanes / ((int64_t)(grid - 1) << GKR_THREADS_LOG));
+        if (j + 2 > n_rounds || saved <= most || !gkr_four_lanes(terms[j], grid)) continue;
+        most = saved;
+        from = j;
+    }
+    return from;
+}
 
 // alpha_pow[k] = alpha^k; claims[k]: oracle k's claim before the first round (4 words each). chan: digest (8 words) and n_draws.
 // Enqueues the layer; gkr_batch_layer_end waits for it. Only gkr_batch_plan may come between the two. GKR_BATCH_AGAIN: the launch was refused and the plan is
