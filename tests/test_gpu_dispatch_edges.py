@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from util import m31_column, qm31_array
+from zk_inference_prover_b200 import ZkbError
 
 pytestmark = pytest.mark.gpu
 
@@ -329,4 +330,17 @@ def test_fri_layers_of_many_ctas(ctx, oracle, log_rows, kw):
     kw = dict(pow_bits=4, log_blowup=1, n_queries=9, **kw)
     want = oracle.pcs_prove(trees, **kw)
     got = ctx.pcs_prove_host(trees, **kw)
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("kw", [dict(log_last_layer=9), {}])
+def test_fri_reports_a_wait_that_ran_out(ctx, oracle, monkeypatch, kw):
+    """Thread blocks that give up their first wait: of one layer, after which nobody waits for them, and of several. The context proves on."""
+    trees, kw = [[m31_column(9400, 1 << 10)]], dict(pow_bits=4, log_blowup=1, n_queries=9, **kw)
+    monkeypatch.setenv("ZKB_FRI_MID", "impatient")
+    with pytest.raises(ZkbError) as e:
+        ctx.pcs_prove_host(trees, **kw)
+    assert e.value.code == -4
+    monkeypatch.delenv("ZKB_FRI_MID")
+    want, got = oracle.pcs_prove(trees, **kw), ctx.pcs_prove_host(trees, **kw)
     assert len(got) == len(want) and (got == want).all()

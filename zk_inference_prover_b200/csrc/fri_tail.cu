@@ -9,6 +9,9 @@
 // top with channel step) a layer also paid two launches, the gaps around them and a dozen allocations for its arrays: a ten-column
 // proof of 2^8 rows spent 190 us of device time in them and as much on the host. Layers stay in shared memory; what the decommitment
 // reads later (trees, folded layers) is written to memory on the side. Above 2^10 values a layer has enough hashes for more SMs: fri_mid_kernel below.
+#include <cstdlib>
+#include <cstring>
+
 #include "channel.cuh"
 #include "common.cuh"
 #include "fri_tail.hpp"
@@ -199,12 +202,12 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
 //
 // As launches (fold and leaves, levels, top with the channel step) a layer of 2^11 ... 2^15 values took 16-24 us, whose chain of hashes is
 // 9-12; a proof of four columns, domain 2^14: 470 us before, 428 with this launch. The waits end: every CTA is resident (the launch is refused otherwise), a wait is for what the others do before their own, and after MID_SPINS
-// polls (a second) a CTA leaves; the channel's done word then stays zero.
+// polls (a second) a CTA leaves, with the channel's failed word set: after the last challenge nobody waits for it any more, and CTA 0 may end well.
 constexpr uint32_t MID_SPINS = 1u << 21;
 constexpr size_t MID_N = (size_t)1 << (FRI_MID_LOG - FRI_MID_CTAS_LOG), MID_PAIRS = MID_N / 2 * PAIR_WORDS, MID_SMEM = (2 * 4 * MID_N + 2 * MID_PAIRS) * 4;  // the largest slice
 static_assert(MID_N / 2 <= TAIL_THREADS && MID_N >= 256 && ((size_t)1 << FRI_MID_CTAS_LOG) <= MID_N, "a slice folds to at most a value a thread; quads and roots have room");
-__device__ __forceinline__ bool mid_wait(const uint32_t* slot, uint32_t there, uint32_t& w) {
-    for (uint32_t spin = 0; spin < MID_SPINS; spin++) {
+__device__ __forceinline__ bool mid_wait(const uint32_t* slot, uint32_t there, uint32_t polls, uint32_t& w) {
+    for (uint32_t spin = 0; spin < polls; spin++) {
         w = *reinterpret_cast<const volatile uint32_t*>(slot);
         if (w >> 31 == there) {
             w &= 0x7fffffffu;
@@ -249,11 +252,11 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
             __syncthreads();
             for (uint32_t i = tid; i < 8 * ctas; i += TAIL_THREADS) {
                 uint32_t w = 0;
-                if (!mid_wait(root_slots + i, there, w)) gave_up = true;
+                if (!mid_wait(root_slots + i, there, MID_SPINS, w)) gave_up = true;
                 ha[pair_at(i >> 3) + (i & 7u)] = w;
             }
             __syncthreads();
-            if (gave_up) return;
+            if (gave_up) break;
             below = hash_levels(ha, hb, ha, ev, MID_N, a.log_ctas - 1, -1, word, qc, [&](int lv) { return a.tree[k] + ((size_t)8 << lv); });
             if (tid < 32) {
                 if (lane < 8) {
@@ -266,11 +269,11 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
             }
         } else if (tid < 4) {
             uint32_t w = 0;
-            if (!mid_wait(alpha_slot + tid, there, w)) gave_up = true;
+            if (!mid_wait(alpha_slot + tid, there, a.impatient ? 0u : MID_SPINS, w)) gave_up = true;
             alpha_w[tid] = w;
         }
         __syncthreads();
-        if (gave_up) return;
+        if (gave_up) break;
         const qm31 alpha{{alpha_w[0], alpha_w[1], alpha_w[2], alpha_w[3]}};
         if (tid < half) {
             qm31 x, y;
@@ -285,7 +288,8 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
         ev_next = swap;
         __syncthreads();
     }
-    if (cta || tid >= 32) return;
+    if (gave_up && tid == 0) a.chan[FRI_MID_FAILED] = 1u;
+    if (gave_up || cta || tid >= 32) return;
     if (lane < 8) a.chan[lane] = ch.msg[lane];
     if (lane == 8) a.chan[8] = ch.n_draws;
     if (lane == FRI_MID_DONE) a.chan[FRI_MID_DONE] = 1u;
@@ -321,10 +325,13 @@ int fri_tail(zkb_ctx* ctx, const FriTailArgs& args) {
     return ZKB_OK;
 }
 
-int fri_mid(zkb_ctx* ctx, const FriMidArgs& args) {
+int fri_mid(zkb_ctx* ctx, FriMidArgs args) {
     ZKB_CHECK_ARG(ctx, args.n_layers >= 1 && args.n_layers <= FRI_MID_LOG - FRI_MID_END && args.first_log <= FRI_MID_LOG && args.first_log - args.n_layers >= FRI_MID_END);
     ZKB_CHECK_ARG(ctx, args.first_log <= ctx->max_log - (args.circle ? 0 : 1));
     ZKB_CHECK_ARG(ctx, args.log_ctas == fri_mid_ctas_log(args.first_log));
+    const char* const env = getenv("ZKB_FRI_MID");  // to be tried: as though the launch were refused; CTAs that give up at once
+    if (env && !strcmp(env, "refused")) return FRI_MID_REFUSED;
+    args.impatient = env && !strcmp(env, "impatient");
     DeviceGuard g(ctx);
     if (!ctx->fri_mid_ready) {
         ZKB_CUDA(ctx, cudaFuncSetAttribute(fri_mid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MID_SMEM));

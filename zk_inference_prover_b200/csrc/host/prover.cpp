@@ -576,7 +576,7 @@ struct FriProver {
             }
             const uint32_t* h = nullptr;  // one copy, one synchronisation
             d.check(zk::read_small(d.ctx(), chan, fs.len() - sync_words, &h));
-            if (mid_done && h[zk::FRI_MID_DONE] != 1u) throw Error(ZKB_ETIMEOUT, "FRI: a layer's challenge did not arrive");
+            if (mid_done && (h[zk::FRI_MID_DONE] != 1u || h[zk::FRI_MID_FAILED] != 0u)) throw Error(ZKB_ETIMEOUT, "FRI: a layer's challenge did not arrive");
             const uint32_t* const state = tail_layers ? h + tail_at : h;
             HashWords dg;
             for (int k = 0; k < 8; k++) dg[k] = state[k];
