@@ -352,7 +352,10 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
         }
     };
     const uint32_t lanes = blockDim.x / (32u * a.teams), team = (threadIdx.x >> 5) / lanes, t = (threadIdx.x >> 5) - team * lanes;
-    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(team + 1u), "r"(32u * lanes) : "memory"); };
+    auto team_sync = [&] {
+        __syncwarp();  // lanes without a row come here by another way than those with one, and the barrier takes whole warps
+        asm volatile("bar.sync %0, %1;" ::"r"(team + 1u), "r"(32u * lanes) : "memory");
+    };
     uint32_t off = 0, bad_exp = 0, un_off = 0, top = 0, since_flush = 0;
     // (a CTA's first team takes its rows before any CTA's second: what is left for a last pass is one team's a CTA)
     for (uint32_t block = blockIdx.x + gridDim.x * team; (block << 5 >> a.log_rows) == 0; block += gridDim.x * a.teams) {
