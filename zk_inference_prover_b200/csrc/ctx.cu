@@ -746,16 +746,20 @@ int stage_tables(zkb_ctx* ctx, const std::pair<const uint32_t* const*, size_t>* 
     if (total > ctx->ring_cap / 2) return ZKB_OK;
     if (int rc = stage_reserve(ctx, total)) return rc;
     const size_t first = ctx->ring_pos;
+    size_t end = first;
+    std::vector<std::pair<size_t, size_t>> placed;  // remembered when the copy is on its way: a table that is found has to be there
     for (size_t k = 0; k < n_tables; k++) {
         const void* const* const p = (const void* const*)tables[k].first;
         const size_t n = tables[k].second;
         if (!n || find_staged(ctx, p, n)) continue;
-        memcpy(ctx->h_ring + ctx->ring_pos, p, n * sizeof(void*));
-        remember_staged(ctx, ctx->ring_pos, n);
-        ctx->ring_pos += n;
+        memcpy(ctx->h_ring + end, p, n * sizeof(void*));
+        placed.push_back({end, n});
+        end += n;
     }
-    if (ctx->ring_pos > first)
-        ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->d_ring + first, ctx->h_ring + first, (ctx->ring_pos - first) * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
+    if (placed.empty()) return ZKB_OK;
+    ZKB_CUDA(ctx, cudaMemcpyAsync(ctx->d_ring + first, ctx->h_ring + first, (end - first) * sizeof(void*), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->ring_pos = end;
+    for (const auto& t : placed) remember_staged(ctx, t.first, t.second);
     return ZKB_OK;
 }
 
