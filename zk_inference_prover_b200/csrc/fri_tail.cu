@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_tail_kernel(const __grid_
     if (lane == 10) a.out[10] = 0xffffffffu;
 }
 
-// The layers above those, of up to 2^FRI_MID_LOG values, in one cooperative launch of up to 32 CTAs. A fold takes neighbouring values, so a CTA keeps its slice of
+// The layers above those, of up to 2^FRI_MID_LOG values, in one cooperative launch of 32 CTAs. A fold takes neighbouring values, so a CTA keeps its slice of
 // the values from layer to layer in shared memory and hashes the subtree above it; what goes round in a layer is the subtrees' roots, to CTA 0, and the
 // challenge back, both with a bit in every word that says that it is there (words of a hash and coordinates are below 2^31; the bit's value changes with
 // every use of the slot): neither waits for a fence or a count. CTA 0 hashes the levels above the subtrees and keeps the channel.
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
     __shared__ uint32_t alpha_w[4];
     __shared__ bool gave_up;
     uint32_t *ev = dyn, *ev_next = ev + 4 * MID_N, *const ha = ev_next + 4 * MID_N, *const hb = ha + MID_PAIRS;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, cta = blockIdx.x, ctas = 1u << a.log_ctas;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, cta = blockIdx.x, ctas = 1u << FRI_MID_CTAS_LOG;
     const QuadConst qc;
     chan_make_schedule(ch, (int)tid, TAIL_THREADS);
     if (tid == 0) gave_up = false;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
         if (tid < 32) ch.msg[tid] = tid < 8 ? a.chan[tid] : 0u;
         if (tid == 0) ch.n_draws = a.chan[8];
     }
-    int slice_log = a.first_log - a.log_ctas;
+    int slice_log = a.first_log - FRI_MID_CTAS_LOG;
     for (uint32_t i = tid; i < 4u << slice_log; i += TAIL_THREADS) {
         const uint32_t c = i >> slice_log, r = i & ((1u << slice_log) - 1);
         ev[c * MID_N + r] = a.src[c][((size_t)cta << slice_log) + r];
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
         if (a.circle && k == 0) half_coset_point(itw, log, fold_at, ix, t);
         else t = itw[(1u << (log - 1)) + fold_at];
         const uint32_t* below = hash_levels(ha, hb, hb, ev, MID_N, slice_log, slice_log, word, qc,
-                                            [&](int lv) { return a.tree[k] + ((size_t)8 << (lv + a.log_ctas)) + (((size_t)8 * cta) << lv); });
+                                            [&](int lv) { return a.tree[k] + ((size_t)8 << (lv + FRI_MID_CTAS_LOG)) + (((size_t)8 * cta) << lv); });
         if (tid < 8) *reinterpret_cast<volatile uint32_t*>(root_slots + 8 * cta + tid) = below[tid] | there << 31;
         if (cta == 0) {
             __syncthreads();
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) fri_mid_kernel(const __grid_c
             }
             __syncthreads();
             if (gave_up) break;
-            below = hash_levels(ha, hb, ha, ev, MID_N, a.log_ctas - 1, -1, word, qc, [&](int lv) { return a.tree[k] + ((size_t)8 << lv); });
+            below = hash_levels(ha, hb, ha, ev, MID_N, FRI_MID_CTAS_LOG - 1, -1, word, qc, [&](int lv) { return a.tree[k] + ((size_t)8 << lv); });
             if (tid < 32) {
                 if (lane < 8) {
                     const uint32_t w = below[lane];
@@ -328,7 +328,6 @@ int fri_tail(zkb_ctx* ctx, const FriTailArgs& args) {
 int fri_mid(zkb_ctx* ctx, FriMidArgs args) {
     ZKB_CHECK_ARG(ctx, args.n_layers >= 1 && args.n_layers <= FRI_MID_LOG - FRI_MID_END && args.first_log <= FRI_MID_LOG && args.first_log - args.n_layers >= FRI_MID_END);
     ZKB_CHECK_ARG(ctx, args.first_log <= ctx->max_log - (args.circle ? 0 : 1));
-    ZKB_CHECK_ARG(ctx, args.log_ctas == fri_mid_ctas_log(args.first_log));
     const char* const env = getenv("ZKB_FRI_MID");  // to be tried: as though the launch were refused; CTAs that give up at once
     if (env && !strcmp(env, "refused")) return FRI_MID_REFUSED;
     args.impatient = env && !strcmp(env, "impatient");
@@ -342,7 +341,7 @@ int fri_mid(zkb_ctx* ctx, FriMidArgs args) {
     attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails
     attr[0].val.cooperative = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1u << args.log_ctas);
+    cfg.gridDim = dim3(1u << FRI_MID_CTAS_LOG);
     cfg.blockDim = dim3(TAIL_THREADS);
     cfg.dynamicSmemBytes = MID_SMEM;
     cfg.stream = ctx->stream;

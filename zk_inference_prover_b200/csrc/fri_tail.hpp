@@ -42,20 +42,18 @@ int fri_tail(zkb_ctx* ctx, const FriTailArgs& args);
 // the SMs it has: eight proofs side by side took 1.85 s a decode step, 1.05 with 32 CTAs and with launches alone.
 constexpr int FRI_MID_LOG = 15;        // largest layer (log2) it takes
 constexpr int FRI_MID_END = 8;         // what its last layer folds to is no smaller (log2)
-constexpr int FRI_MID_CTAS_LOG = 5;
-inline int fri_mid_ctas_log(int first_log) { return first_log - 6 < FRI_MID_CTAS_LOG ? first_log - 6 : FRI_MID_CTAS_LOG; }  // slices of 2^6 values and more
+constexpr int FRI_MID_CTAS_LOG = 5;    // slices of 2^6 values and more of a first layer, of 2^4 of the last
 constexpr int FRI_MID_DONE = 10;       // the word of the channel's sixteen that is one when the first CTA has ended well, zero before
 constexpr int FRI_MID_FAILED = 11;     // ... and that is one when a CTA has given up a wait
 struct FriMidArgs {
     const uint32_t* src[4];            // the first layer's coordinate columns
     int first_log, n_layers, circle;   // as above; at least one layer, and the last one folds to no less than 2^FRI_MID_END values
-    int log_ctas;                      // fri_mid_ctas_log
     uint32_t* tree[FRI_MID_LOG - FRI_MID_END];   // as above
     uint32_t* evals[FRI_MID_LOG - FRI_MID_END];
-    uint32_t *chan, *roots, *sync;     // channel state, in and out; a root per layer; fri_mid_sync_words zeros
+    uint32_t *chan, *roots, *sync;     // channel state, in and out; a root per layer; FRI_MID_SYNC_WORDS zeros
     int impatient;                     // filled by fri_mid
 };
-inline size_t fri_mid_sync_words(int log_ctas) { return ((size_t)16 << log_ctas) + 8; }
+constexpr size_t FRI_MID_SYNC_WORDS = ((size_t)16 << FRI_MID_CTAS_LOG) + 8;
 constexpr int FRI_MID_REFUSED = -1001; // not all CTAs can be resident: nothing was launched
 int fri_mid(zkb_ctx* ctx, FriMidArgs args);
 // The first nonces (several times 2^pow_bits of them) tested against the digest at prefixed; the smallest that passes goes to *best.

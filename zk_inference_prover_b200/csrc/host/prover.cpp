@@ -490,8 +490,7 @@ struct FriProver {
             const size_t mid_layers = tail - launched;
             const uint32_t mid_log = first_log - (uint32_t)launched;
             // [the middle launch's meeting place | channel 16 | challenges 4 each (16-byte aligned) | roots 8 each | the tail's results]
-            const int mid_ctas_log = zk::fri_mid_ctas_log((int)mid_log);
-            const size_t sync_words = mid_layers ? zk::fri_mid_sync_words(mid_ctas_log) : 0;
+            const size_t sync_words = mid_layers ? zk::FRI_MID_SYNC_WORDS : 0;
             const size_t tail_at = 16 + 12 * tail, tail_layers = n_layers - tail;
             BaseColumn fs(d, sync_words + tail_at + zk::fri_tail_out_words((int)tail_layers));
             uint32_t* const sync = fs.ptr();
@@ -537,7 +536,6 @@ struct FriProver {
                     ma.first_log = (int)mid_log;
                     ma.n_layers = (int)mid_layers;
                     ma.circle = launched == 0;
-                    ma.log_ctas = mid_ctas_log;
                     ma.chan = chan;
                     ma.roots = roots + 8 * launched;
                     ma.sync = sync;
