@@ -344,3 +344,36 @@ def test_fri_reports_a_wait_that_ran_out(ctx, oracle, monkeypatch, kw):
     monkeypatch.delenv("ZKB_FRI_MID")
     want, got = oracle.pcs_prove(trees, **kw), ctx.pcs_prove_host(trees, **kw)
     assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("spec", [{5: 2, 3: 1}, {12: 2, 9: 30}, {16: 1, 13: 40}, {6: 500, 2: 3}])
+def test_gkr_batch_whose_launch_is_refused(ctx, oracle, monkeypatch, spec):
+    """Layers whose thread blocks can not all be resident are planned again, as launches, after what was planned had been staged: rounds ahead of the
+    transcript from the first one on (no eq table there yet) and from a later one, words that the launch carries and words that are copied."""
+    inst, dev, keep = [], [], []
+    for log_n, count in spec.items():
+        for i in range(count):
+            n, kind = 1 << log_n, (3, 0, 1, 2)[len(inst) % 4]
+            at = 9500 + 3 * len(inst)
+            den = qm31_array(at, n, nonzero=True)
+            num = qm31_array(at + 1, n) if kind == 1 else m31_column(at + 2, n) if kind == 2 else None
+            inst.append((kind, num, den))
+            keep += [ctx.upload(num) if num is not None else None, ctx.upload(den)]
+            dev.append((kind, keep[-2].ptr if num is not None else 0, keep[-1].ptr, n))
+    want = oracle.gkr_prove(inst, 0x5EED0019, verify=True)
+    monkeypatch.setenv("ZKB_GKR_DRIVER", "batch")
+    monkeypatch.setenv("ZKB_GKR_ROUNDS", "refused")
+    ctx.profile_begin()
+    got = ctx.gkr_prove_device(dev, 0x5EED0019)
+    prof, layers = ctx.profile_end(), max(spec)
+    assert prof["gkr_batch_step_kernel"][1] == sum(r + 1 for r in range(1, layers))  # every layer went that way
+    assert len(got) == len(want) and (got == want).all()
+
+
+@pytest.mark.parametrize("log_rows,kw", [(10, {}), (10, dict(log_last_layer=9)), (11, dict(log_last_layer=2)), (15, {}), (16, dict(log_last_layer=12))])
+def test_fri_layers_of_many_ctas_refused(ctx, oracle, monkeypatch, log_rows, kw):
+    """The middle layers as launches, none before them and one, with and without last layers in a launch behind them."""
+    monkeypatch.setenv("ZKB_FRI_MID", "refused")
+    ctx.profile_begin()
+    test_fri_layers_of_many_ctas(ctx, oracle, log_rows, kw)
+    assert "fri_mid_kernel" not in ctx.profile_end()

@@ -1369,7 +1369,7 @@ int gkr_batch_layer_begin(zkb_ctx* ctx, GkrLayerPlan& plan, const uint32_t* alph
     GkrSync* const d_sync = reinterpret_cast<GkrSync*>(d_blob + at.sync);
     const GkrAcc acc{reinterpret_cast<unsigned long long*>(d_blob + at.acc), n_rounds};
     cudaError_t e = cudaErrorCooperativeLaunchTooLarge;
-    if (!plan.launches) {
+    if (!plan.launches && !plan.refused) {
         ProfScope prof(ctx, "gkr_batch_layer_kernel");
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeCooperative;  // every CTA is resident, or the launch fails

@@ -73,6 +73,7 @@ struct GkrLayerPlan {
     const GkrBatchItem* d_items = nullptr;  // staged by gkr_batch_plan, and what else does not depend on the transcript
     uint32_t* d_blob = nullptr;
     bool launches = false;           // the layer as a launch per table and one per transcript step
+    bool refused = false;            // to be tried: as though the one launch were refused
 };
 int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
 

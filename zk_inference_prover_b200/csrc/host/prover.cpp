@@ -1636,7 +1636,8 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
     std::vector<qm31> ood_point;
 
     // Whether the transcript of a layer's rounds stays on the device (gkr_batch_layer_begin; ZKB_GKR_ROUNDS=host: never;
-    // ZKB_GKR_ROUNDS=launches: with a launch per round and step instead of one for the layer). The layer's
+    // ZKB_GKR_ROUNDS=launches: with a launch per round and step instead of one for the layer; =refused: the same, as though the one launch had
+    // been refused). The layer's
     // description is staged as one block (an item per oracle and active round, 64 bytes each, and some 52 bytes per oracle): a batch of
     // thousands of tall instances would not fit the staging ring and takes the round-by-round path, which stages one round's items at a time.
     const char* rounds_env = getenv("ZKB_GKR_ROUNDS");
@@ -1648,6 +1649,7 @@ static std::vector<uint32_t> gkr_prove_batch(const Device& d, Channel& ch, const
     // A layer's tables depend on the towers' sizes only: they are made and staged while the layer before runs.
     zk::GkrLayerPlan plan, next_plan;
     plan.launches = next_plan.launches = rounds_env && !strcmp(rounds_env, "launches");
+    plan.refused = next_plan.refused = rounds_env && !strcmp(rounds_env, "refused");
     std::vector<size_t> inst, next_inst;
     auto make_next = [&](int layer) {
         HostClock hc_plan("gkr.layer.plan");
