@@ -21,6 +21,7 @@
 #include "../../../include/zkb200_prover.h"
 #include "../air_program.hpp"
 #include "b200_backend.hpp"
+#include "commit_groups.hpp"
 #include "../fft_internal.hpp"
 #include "../gkr_resident.hpp"
 #include "../gkr_batch.hpp"
@@ -939,7 +940,7 @@ struct CommitmentSchemeProver {
             }
             if (incremental) { hash_ready(true); have_leaves = true; }
         } else {
-            // From the tallest columns down, each size interpolated, extended and hashed before the next: a segment's short columns are tens of thousands,
+            // From the tallest columns down, each size (small ones together: commit_group) interpolated, extended and hashed before the next: a segment's short columns are tens of thousands,
             // which take the host longer to write down than the device to transform, and the device has the tall ones' hashes meanwhile.
             const uint32_t blowup = config.fri.log_blowup_factor;
             struct Size { uint32_t log; const std::vector<size_t>* of; std::vector<uint32_t*> coeffs, evals; };
@@ -950,34 +951,44 @@ struct CommitmentSchemeProver {
                 count[g->first + blowup] = g->second.size();
             }
             MerkleBuilder builder(d, count);
-            // The tables of several sizes of few columns go to the device in one copy: a copy between two kernels of a few microseconds costs as much as one.
-            size_t prepared = 0;
-            auto prepare = [&](size_t k) {
-                if (k < prepared) return;
+            // The tables of several sizes of few columns go to the device in one copy: a copy between two kernels of a few microseconds costs as much as one. Those of the
+            // extended columns go behind the interpolations, which need not wait for their allocations: three trees of 10 columns of 2^6 ... 2^4 rows 344 us with one copy for both,
+            // 338 with two; of 2^7 ... 2^4 rows 397 and 393; of 40 columns of 2^9 ... 2^4 rows 642 and 635, 709 with a copy a size and table.
+            auto run_end = [&](size_t first) {
+                size_t end = first;
+                for (size_t n = 0; end < sizes.size() && end < first + 12 && (end == first || n + sizes[end].of->size() <= 4096); end++) n += sizes[end].of->size();
+                return end;
+            };
+            auto stage = [&](std::vector<uint32_t*> Size::*table, size_t first, size_t end) {
                 std::vector<std::pair<const uint32_t* const*, size_t>> tables;
-                for (size_t n = 0; prepared < sizes.size() && (prepared == k || n + sizes[prepared].of->size() <= 4096) && tables.size() < 24; prepared++) {
-                    Size& g = sizes[prepared];
-                    const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup), stride = std::max<size_t>(n_out, 4);
-                    n += nc;
-                    // one allocation for the extended columns of a size (16-byte aligned each)
-                    t.eval_slabs.emplace_back(d, nc * stride);
-                    g.coeffs.resize(nc);
-                    g.evals.resize(nc);
-                    for (size_t c = 0; c < nc; c++) {
-                        g.coeffs[c] = columns[(*g.of)[c]].ptr();
-                        g.evals[c] = t.eval_slabs.back().ptr() + c * stride;
-                    }
-                    tables.push_back({g.coeffs.data(), nc});
-                    tables.push_back({g.evals.data(), nc});
-                }
+                for (size_t k = first; k < end; k++) tables.push_back({(sizes[k].*table).data(), (sizes[k].*table).size()});
                 d.check(zk::stage_tables(d.ctx(), tables.data(), tables.size()));
             };
+            size_t with_coeffs = 0, with_evals = 0;  // sizes whose tables are made
             auto interpolate = [&](size_t k) {
-                prepare(k);
+                if (k == with_coeffs) {
+                    for (const size_t end = run_end(k); with_coeffs < end; with_coeffs++) {
+                        Size& g = sizes[with_coeffs];
+                        g.coeffs.reserve(g.of->size());
+                        for (size_t c : *g.of) g.coeffs.push_back(columns[c].ptr());
+                    }
+                    stage(&Size::coeffs, k, with_coeffs);
+                }
                 if (are_coeffs) return;  // TreeBuilder::extend_polys (pcs/mod.rs:437-452): the columns are coefficients already
                 d.check(zkb_ifft_cols(d.ctx(), sizes[k].coeffs.data(), (int)sizes[k].coeffs.size(), (int)sizes[k].log));
             };
             auto extend = [&](size_t k) {
+                if (k == with_evals) {
+                    for (const size_t end = run_end(k); with_evals < end; with_evals++) {
+                        Size& g = sizes[with_evals];
+                        const size_t nc = g.of->size(), stride = std::max<size_t>((size_t)1 << (g.log + blowup), 4);
+                        // one allocation for the extended columns of a size (16-byte aligned each)
+                        t.eval_slabs.emplace_back(d, nc * stride);
+                        g.evals.resize(nc);
+                        for (size_t c = 0; c < nc; c++) g.evals[c] = t.eval_slabs.back().ptr() + c * stride;
+                    }
+                    stage(&Size::evals, k, with_evals);
+                }
                 Size& g = sizes[k];
                 const size_t nc = g.of->size(), n_out = (size_t)1 << (g.log + blowup);
                 d.check(zkb_lde_cols(d.ctx(), g.coeffs.data(), (int)nc, (int)g.log, g.evals.data(), (int)(g.log + blowup)));
@@ -992,11 +1003,17 @@ struct CommitmentSchemeProver {
                 while (builder.next >= 0) builder.hash_next();
             } else {
                 const bool fork = several && several->more && !several->forked && narrow(count);
-                size_t k = 0;
-                for (; k < sizes.size() && !(fork && sizes[k].log + blowup <= NARROW_LOG); k++) {
-                    interpolate(k);
-                    extend(k);
-                    builder.hash_to_columns();
+                size_t stop = 0, k = 0;  // from `stop` on: on the side
+                std::vector<size_t> words;
+                for (const Size& g : sizes) {
+                    words.push_back(g.of->size() << (g.log + blowup));
+                    if (!(fork && g.log + blowup <= NARROW_LOG)) stop++;
+                }
+                while (k < stop) {
+                    const size_t end = k + zk::commit_group(&words[k], stop - k);
+                    for (size_t j = k; j < end; j++) interpolate(j);
+                    for (size_t j = k; j < end; j++) extend(j);
+                    for (; k < end; k++) builder.hash_to_columns();
                 }
                 if (k < sizes.size()) {
                     several->forked = true;
