@@ -97,3 +97,14 @@ def test_dequant_tables_in_shared_memory(ctx, oracle, variant, per_row, kmax, wi
     want["want"][:] = 0
     for k in ("counts", "m_norm", "m_frac", "m_mul", "m_r8", "pre", "base"):
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("kmax", [14, 16, 19])
+def test_dequant_tables_beside_the_counters(ctx, oracle, kmax):
+    """Both tables in shared memory beside fraction counters that two and more rows share."""
+    case = dequant_case(40 + kmax, 1, 256, 256, 16, kmax, 1, 0, False)
+    got = run_dequant(ctx, case)
+    want = oracle.witness_dequant(case["acc"], case["jx"], case["jw"], case["sx"], case["sw"], case["norm3"], case["mul2"], case["n_base"], case["n_pre"], case["cfg"])
+    want["want"][:] = 0
+    for k in ("counts", "m_norm", "m_frac", "m_mul", "m_r8", "pre", "base"):
+        assert np.array_equal(got[k], want[k]), k

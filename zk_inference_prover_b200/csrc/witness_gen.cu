@@ -137,14 +137,16 @@ __global__ void tables_patch_kernel(const uint32_t* __restrict__ idx, const uint
 // shared-memory histogram, the three large tables go through counters in shared memory too (count_cache.cuh), so one CTA an
 // SM takes units until none are left. A random row of a table in memory is a line a lane, so the LSU's data path was what bounded it (79 % busy): where a CTA has slots
 // enough, the normalisation table is in shared memory, a word a row, and the product table, 16 bits a row. 2^17 rows of 16 slots: 230 us with the large
-// tables' counts as warp-merged atomics, 88 us with the counters, 67 us with the tables, a counter a row of the fraction table and 32-bit arithmetic.
+// tables' counts as warp-merged atomics, 88 us with the counters, 67 us with the tables and 32-bit arithmetic. Rows of the fraction table share 2^12 counters: 2^14 of
+// them, one a row at kmax 13, take 48 KB from the L1 and, from kmax 15 on, the product table's place (bf16-chain calls with 2^14 and with 2^12: kmax 13
+// 109 and 105 us, kmax 16 143 and 110, kmax 19 133 and 111; the other variant, at kmax 13 only, 72.6 and 73.5).
 // ---------------------------------------------------------------------------------------------------
-constexpr int DEQ_THREADS = 1024, DEQ_NORM_LOG = 13, DEQ_FRAC_LOG = 14, DEQ_MUL_LOG = 14;
+constexpr int DEQ_THREADS = 1024, DEQ_NORM_LOG = 13, DEQ_FRAC_LOG = 12, DEQ_MUL_LOG = 14;
 constexpr uint32_t DEQ_COUNT_WORDS = (1u << DEQ_NORM_LOG) + (1u << DEQ_FRAC_LOG), DEQ_CHAIN_WORDS = DEQ_COUNT_WORDS + (1u << DEQ_MUL_LOG);
 // From how many slots a CTA on the tables are brought to shared memory too, which takes some 3 us. 2^17 rows of 16 slots, 14,000 a CTA: 83 us without,
 // 70 with; of four, 3,500: 29.7, 27.9; 2^14 rows of 16, 1,800: 19.0, 20.7.
 constexpr uint32_t DEQ_STAGE_SLOTS = 3072;
-constexpr uint32_t DEQ_SMEM = 227 * 1024;  // counters first, then the normalisation table and the column addresses as far as there is room for each
+constexpr uint32_t DEQ_SMEM = 227 * 1024;  // counters first, then the column addresses and the tables as far as there is room for each
 struct DeqArgs {
     const int32_t *acc, *jx, *jw;
     const uint32_t *sx, *sw, *norm3, *mul2;
