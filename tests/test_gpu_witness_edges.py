@@ -108,3 +108,13 @@ def test_dequant_tables_beside_the_counters(ctx, oracle, kmax):
     want["want"][:] = 0
     for k in ("counts", "m_norm", "m_frac", "m_mul", "m_r8", "pre", "base"):
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("n", [11, 12])
+@pytest.mark.parametrize("kmax,sticky,even", [(13, True, None), (13, False, True), (16, True, False), (16, False, None)])
+def test_residual_stream_around_the_fraction_counters(ctx, oracle, n, kmax, sticky, even):
+    """352 and 384 additions a thread block: fewer and more counters of the fraction table, shared by several rows and one each."""
+    case = wc.residual_stream_case(90 + n + kmax, "pairs", n, 5, 32, kind=0, sticky=sticky, kmax=kmax, spread=9)
+    got, want = run_residual_stream(ctx if even is None else _EvenColumns(ctx, 32, case["n_cols"], even), case), oracle.witness_residual_stream(case)
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k

@@ -11,6 +11,7 @@
 // (deliberate defects for negative controls) are not part of the operators and are not built.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -324,9 +325,14 @@ __device__ __noinline__ void add_slot_wide(const RsArgs& a, RsOperand x, RsOpera
 // an access, 170 us as it is now (650 instructions a slot, issue slots at 46 %, the LSU's data path too). The normalisation table in shared memory, a word
 // a row, gained nothing (173). 2^13 rows: 53 -> 48 us; four teams of eight warps instead of two of sixteen: 193.
 constexpr uint32_t RS_LANES = 16, RS_TEAMS = 2, RS_LEAVES = 4;
-constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 14, RS_SMUL_LOG = 14;
-constexpr uint32_t RS_ADD_WORDS = (1u << RS_VAL_LOG) + (1u << RS_NORM_LOG) + (1u << RS_FRAC_LOG), RS_MUL_WORDS = (1u << RS_VAL_LOG) + (1u << RS_SMUL_LOG);
-template <bool MUL, bool STICKY, bool EVEN>
+constexpr int RS_VAL_LOG = 13, RS_NORM_LOG = 13, RS_FRAC_LOG = 14, RS_FRAC_FEW_LOG = 12, RS_SMUL_LOG = 14;
+constexpr uint32_t RS_MUL_WORDS = (1u << RS_VAL_LOG) + (1u << RS_SMUL_LOG);
+constexpr uint32_t rs_add_words(int frac_log) { return (1u << RS_VAL_LOG) + (1u << RS_NORM_LOG) + (1u << frac_log); }
+// From how many additions a CTA on the fraction table has 2^RS_FRAC_LOG counters: those are 48 KB more to clear and to look through at the end, a microsecond.
+// With 2^12 and with 2^14, kmax 13: 2^13 rows of 4 additions, 256 a CTA: 18.1 and 19.4 us; 2^14 rows, 443 a CTA: 25.0 and 24.1; 32 rows of 128, 4,096: 40.7 and 38.4;
+// 2^15 rows of 128: 179 and 176.
+constexpr uint64_t RS_FRAC_ADDITIONS = 384;
+template <bool MUL, bool STICKY, bool EVEN, int FRAC_LOG>
 __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_kernel(const __grid_constant__ RsArgs a) {
     // The power table has 273 rows and every addition hits row DMAX with its larger operand: that row is counted in a register, the others per CTA in
     // shared memory, and added to the global array once at the end.
@@ -334,12 +340,12 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
     extern __shared__ __align__(16) uint32_t counts_sm[];
     uint32_t *const val_counts = counts_sm, *const norm_counts = counts_sm + (1u << RS_VAL_LOG), *const frac_counts = norm_counts + (1u << RS_NORM_LOG);
     uint32_t* const smul_counts = norm_counts;  // a program adds or multiplies
-    const bool norm_whole = count_is_whole<RS_NORM_LOG>(a.m_norm), frac_whole = count_is_whole<RS_FRAC_LOG>(a.m_frac);
+    const bool norm_whole = count_is_whole<RS_NORM_LOG>(a.m_norm), frac_whole = count_is_whole<FRAC_LOG>(a.m_frac);
     count_clear<RS_VAL_LOG>(val_counts, false, threadIdx.x, blockDim.x);
     if (MUL) count_clear<RS_SMUL_LOG>(smul_counts, false, threadIdx.x, blockDim.x);
     else {
         count_clear<RS_NORM_LOG>(norm_counts, norm_whole, threadIdx.x, blockDim.x);
-        count_clear<RS_FRAC_LOG>(frac_counts, frac_whole, threadIdx.x, blockDim.x);
+        count_clear<FRAC_LOG>(frac_counts, frac_whole, threadIdx.x, blockDim.x);
     }
     for (uint32_t k = threadIdx.x; k < RS_POW_ROWS; k += blockDim.x) pow_hist[k] = 0;
     __syncthreads();
@@ -348,7 +354,7 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
         if (MUL) count_flush<RS_SMUL_LOG>(smul_counts, a.m_smul.m, thread, threads);
         else {
             count_flush<RS_NORM_LOG>(norm_counts, a.m_norm.m, thread, threads);
-            count_flush<RS_FRAC_LOG>(frac_counts, a.m_frac.m, thread, threads);
+            count_flush<FRAC_LOG>(frac_counts, a.m_frac.m, thread, threads);
         }
     };
     const uint32_t lanes = blockDim.x / (32u * a.teams), team = (threadIdx.x >> 5) / lanes, t = (threadIdx.x >> 5) - team * lanes;
@@ -450,7 +456,7 @@ __global__ void __launch_bounds__(32 * RS_LANES * RS_TEAMS, 1) residual_stream_k
                 else atomicAdd(pow_hist + u, 1u);
             }
             lookup<RS_NORM_LOG>(norm_counts, a.m_norm, o.ni, off, norm_whole);
-            lookup<RS_FRAC_LOG>(frac_counts, a.m_frac, o.frac, off, frac_whole);
+            lookup<FRAC_LOG>(frac_counts, a.m_frac, o.frac, off, frac_whole);
             lookup<RS_VAL_LOG>(val_counts, a.m_val, o.val, off);
         } else {
             // the signed significands' correctly rounded product and binade carry come from one table row
@@ -744,13 +750,18 @@ int zkb_witness_residual_stream(zkb_ctx* ctx, const zkb_rs_program* prog, const 
     ProfScope prof(ctx, "residual_stream_kernel");
     cudaError_t e = cudaSuccess;
     auto launch = [&](auto kernel, uint32_t words) {
-        // the most any call takes: another thread's call must not lower it in between
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * (p.kind == 1 ? RS_MUL_WORDS : RS_ADD_WORDS)));
+        // the most any call of the kernel takes: another thread's call must not lower it in between
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * words));
         if (e == cudaSuccess) kernel<<<grid, threads, 4 * words, ctx->stream>>>(a);
     };
-    if (p.kind == 1) even ? launch(residual_stream_kernel<true, false, true>, RS_MUL_WORDS) : launch(residual_stream_kernel<true, false, false>, RS_MUL_WORDS);
-    else if (p.sticky) even ? launch(residual_stream_kernel<false, true, true>, RS_ADD_WORDS) : launch(residual_stream_kernel<false, true, false>, RS_ADD_WORDS);
-    else even ? launch(residual_stream_kernel<false, false, true>, RS_ADD_WORDS) : launch(residual_stream_kernel<false, false, false>, RS_ADD_WORDS);
+    auto add = [&](auto frac_log) {
+        constexpr int LOG = decltype(frac_log)::value;
+        if (p.sticky) even ? launch(residual_stream_kernel<false, true, true, LOG>, rs_add_words(LOG)) : launch(residual_stream_kernel<false, true, false, LOG>, rs_add_words(LOG));
+        else even ? launch(residual_stream_kernel<false, false, true, LOG>, rs_add_words(LOG)) : launch(residual_stream_kernel<false, false, false, LOG>, rs_add_words(LOG));
+    };
+    if (p.kind == 1) even ? launch(residual_stream_kernel<true, false, true, 0>, RS_MUL_WORDS) : launch(residual_stream_kernel<true, false, false, 0>, RS_MUL_WORDS);
+    else if ((uint64_t)rows * p.n_slots < grid * RS_FRAC_ADDITIONS) add(std::integral_constant<int, RS_FRAC_FEW_LOG>{});
+    else add(std::integral_constant<int, RS_FRAC_LOG>{});
     ZKB_CUDA(ctx, e);
     ZKB_LAUNCH_CHECK(ctx);
     return ZKB_OK;
