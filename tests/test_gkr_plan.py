@@ -64,6 +64,14 @@ def test_what_is_saved_makes_up_for_the_large_rounds(look_from):
                 continue
             assert 0 <= first <= len(terms) - 2
             cost = sum(max(9500, 4500 + 5000 * _pieces(terms, j, grid)) for j in range(first, len(terms)))
-            assert cost <= 16000 * (len(terms) - first) + 1
+            assert cost <= 16000 * (len(terms) - first) + 1 + (10000 if first == 0 and len(terms) <= 16 else 0)  # (no table of eq then)
             # a sum of 16-bit halves takes 2^16 additions; a piece makes at most 64 of them to one counter
             assert all(64 * (_pieces(terms, j, grid) + 1) < 1 << 16 for j in range(first, len(terms)))
+
+
+def test_the_table_of_eq_counts(look_from):
+    """Ahead from the first round on a layer needs no table: worth a first round that alone is not, where the terms' indices are short enough."""
+    halves = lambda *first: list(first) + [max(1, first[-1] >> k) for k in range(1, 15 - len(first) + 1)]
+    assert look_from(halves(16384, 24576)) == 0 and look_from(halves(1024, 31232)) == 0
+    assert look_from(halves(32768, 49152)) == 2  # too large even so
+    assert look_from(halves(24576, 24576, 16384)) == 0

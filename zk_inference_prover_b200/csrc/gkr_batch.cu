@@ -352,7 +352,7 @@ constexpr int GKR_THREADS = 1 << GKR_THREADS_LOG;
 constexpr int LOOK_MIN_LOG = 7;                  // the fewest threads (log2) that a CTA is given work for
 constexpr uint32_t SPIN_LIMIT = 1u << 21;
 
-constexpr int EQ_TABLES = 3;                     // of five bits of a term's index each
+constexpr int EQ_TABLES = GKR_EQ_BITS / 5;       // of five bits of a term's index each
 
 struct alignas(16) GkrTable {
     uint32_t first, n_items;  // its items
@@ -1287,7 +1287,7 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan) {
     }
     plan_look(plan, grid);
     // Rounds that take four and eight lanes a term can work eq out: a term a thread would take two products more for each of its six.
-    plan.needs_eq = plan.look_from != 0 || tables_of(plan)[0].terms_log > 5 * EQ_TABLES;
+    plan.needs_eq = plan.look_from != 0 || tables_of(plan)[0].terms_log > GKR_EQ_BITS;
     const std::vector<GkrBatchItem>& items = plan.look_from >= 0 ? plan.look_items : plan.items;
     // What the launch stages later must not come to lie over this: room for both.
     const size_t item_words = items.size() * (sizeof(GkrBatchItem) / 4);

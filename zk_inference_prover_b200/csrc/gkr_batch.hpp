@@ -79,6 +79,7 @@ int gkr_batch_plan(zkb_ctx* ctx, GkrLayerPlan& plan);
 
 // How a layer's rounds are taken, by their terms and the CTAs of the launch.
 constexpr int GKR_THREADS_LOG = 9;  // of a CTA
+constexpr int GKR_EQ_BITS = 15;     // of a term's index, for eq without a table
 // Four lanes a term while that is at most two passes of the whole grid: a pass of this form is a third of the other's latency,
 // and a third more work.
 inline bool gkr_four_lanes(size_t terms, uint32_t grid) { return 4 * terms <= 2 * ((size_t)grid << GKR_THREADS_LOG); }
@@ -86,16 +87,18 @@ inline bool gkr_four_lanes(size_t terms, uint32_t grid) { return 4 * terms <= 2 
 // they fall by half from round to round, and grow where shorter oracles enter. A round ahead takes eight lanes for a term of the round after it: some
 // 4,500 cycles and 5,000 for 512 lanes a CTA, 9,500 at least, where an ordinary round takes 16,000 and for a large one less per term than this. So what all rounds
 // from a candidate on save has to make up for the large ones among them. One instance of 2^16 above 500 of 2^14: 5.2 ms with no round ahead, 7.3 from the first
-// small round on, 5.2 by this rule; of 2^14 above 300 of 2^13: 3.1, 3.3 and 2.8; 34 of 2^10 ... 2^13, whose rounds only fall: 1.10, 0.82 and 0.82. No pass has more than
-// 43 times 512 lanes a CTA then: 31 rounds do not save more (look_term's sums rest on it).
+// small round on, 5.2 by this rule; of 2^14 above 300 of 2^13: 3.1, 3.3 and 2.8; 34 of 2^10 ... 2^13, whose rounds only fall: 1.10, 0.82 and 0.82. A layer that is ahead from its
+// first round on works eq out from the point, and the launch that would write the table is saved: 13 instances of 2^11 ... 2^15 0.921 ms without that in the
+// sum, 0.908 with it. No pass has more than 45 times 512 lanes a CTA then: 31 rounds do not save more (look_term's sums rest on it).
 inline int gkr_look_from(const size_t* terms, int n_rounds, uint32_t grid) {
-    constexpr int64_t ORDINARY = 16000, AHEAD = 9500, AHEAD_BASE = 4500, AHEAD_PIECE = 5000;
+    constexpr int64_t ORDINARY = 16000, AHEAD = 9500, AHEAD_BASE = 4500, AHEAD_PIECE = 5000, EQ_TABLE = 10000;
     if (grid < 2) return -1;
     int from = -1;
     int64_t saved = 0, most = 0;
     for (int j = n_rounds - 1; j >= 0; j--) {
         const int64_t lanes = j + 1 < n_rounds ? 8 * (int64_t)terms[j + 1] : 0;
         saved += ORDINARY - std::max(AHEAD, AHEAD_BASE + AHEAD_PIECE * lanes / ((int64_t)(grid - 1) << GKR_THREADS_LOG));
+        if (j == 0 && n_rounds - 1 <= GKR_EQ_BITS) saved += EQ_TABLE;
         if (j + 2 > n_rounds || saved <= most || !gkr_four_lanes(terms[j], grid)) continue;
         most = saved;
         from = j;
