@@ -137,7 +137,7 @@ __global__ void tables_patch_kernel(const uint32_t* __restrict__ idx, const uint
 // shared-memory histogram, the three large tables go through counters in shared memory too (count_cache.cuh), so one CTA an
 // SM takes units until none are left. A random row of a table in memory is a line a lane, so the LSU's data path was what bounded it (79 % busy): where a CTA has slots
 // enough, the normalisation table is in shared memory, a word a row, and the product table, 16 bits a row. 2^17 rows of 16 slots: 230 us with the large
-// tables' counts as warp-merged atomics, 88 us with the counters, 67 us with the tables and 32-bit arithmetic. Rows of the fraction table share 2^12 counters: 2^14 of
+// tables' counts as warp-merged atomics, 88 us with the counters, 64 us with the tables and 32-bit arithmetic. Rows of the fraction table share 2^12 counters: 2^14 of
 // them, one a row at kmax 13, take 48 KB from the L1 and, from kmax 15 on, the product table's place (bf16-chain calls with 2^14 and with 2^12: kmax 13
 // 109 and 105 us, kmax 16 143 and 110, kmax 19 133 and 111; the other variant, at kmax 13 only, 72.6 and 73.5).
 // ---------------------------------------------------------------------------------------------------
