@@ -50,9 +50,7 @@ class _EvenColumns:
 
 @pytest.mark.parametrize("even", [None, False, True])
 @pytest.mark.parametrize("shape,n,log_rows,live_rows,kind,sticky,spread", [("pairs", 8, 13, 8000, 0, True, 130), ("pairs", 8, 13, 8192, 1, True, 30),
-                                                                         ("tree", 40, 12, 4096, 0, False, 100), ("pairs", 4, 3, 7, 0, True, 9),
-                                                                         # fewer rows than a warp has lanes, over several levels of additions
-                                                                         ("tree", 40, 4, 16, 0, True, 20), ("tree", 40, 2, 3, 0, False, 20), ("pairs", 8, 1, 2, 1, True, 9)])
+                                                                         ("tree", 40, 12, 4096, 0, False, 100), ("pairs", 4, 3, 7, 0, True, 9)])
 def test_residual_stream_edges(ctx, oracle, even, shape, n, log_rows, live_rows, kind, sticky, spread):
     pad = 64 if shape == "tree" else None
     case = wc.residual_stream_case(77 + n + log_rows, shape, n, log_rows, live_rows, pad=pad, un=(0, 0), kind=kind, sticky=sticky, kmax=13, spread=spread)
@@ -118,3 +116,10 @@ def test_residual_stream_around_the_fraction_counters(ctx, oracle, n, kmax, stic
     got, want = run_residual_stream(ctx if even is None else _EvenColumns(ctx, 32, case["n_cols"], even), case), oracle.witness_residual_stream(case)
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("even", [None, False, True])
+@pytest.mark.parametrize("shape,n,log_rows,live_rows,kind,sticky,spread", [("tree", 40, 4, 16, 0, True, 20), ("tree", 40, 2, 3, 0, False, 20), ("pairs", 8, 1, 2, 1, True, 9)])
+def test_residual_stream_of_fewer_rows_than_lanes(ctx, oracle, even, shape, n, log_rows, live_rows, kind, sticky, spread):
+    """Over several levels of additions, whose barriers take whole warps."""
+    test_residual_stream_edges(ctx, oracle, even, shape, n, log_rows, live_rows, kind, sticky, spread)
